@@ -113,7 +113,9 @@ int see_cuda_set_attention_one_walk(see_cuda_backend* h, int enabled);
  * accumulation.  The result is the f32 product to a few 2^-24 of sum|a_k b_k|
  * (the reference holds its own GEMMs to 2e-6 of that: test/runtime/executor/
  * kernels_test.cc:1803-1822), not the CPU's bits.  mode -1 (default): in lazy
- * coherence only; 0: never; 1: in strict coherence too. */
+ * coherence only, and there from 2^24 multiply-adds, with int8 and bf16 weights
+ * (one exact piece: three products) and any width; 0: never; 1: in strict
+ * coherence too. */
 int see_cuda_set_split_gemm(see_cuda_backend* h, int mode);
 /* Large tensor-core products run on CTA pairs (two SMs per 256 x 256 tile, each loading half of the
  * weight tile).  Default on; 0 = one CTA per 128 x 256 tile.  Results are identical either way (the same

@@ -410,7 +410,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
     }
   }
   umma::PlanRange(&umma_->ctx, program.data(), begin, std::min(end, program.size()));
-  if (SplitGemmOn()) umma::PlanSplitGemms(&umma_->ctx, program.data(), begin, std::min(end, program.size()));
+  if (SplitGemmOn()) umma::PlanSplitGemms(&umma_->ctx, program.data(), begin, std::min(end, program.size()), SplitGemmWide(), relaxed_allowed_);
   // Cached bf16 activation copies do not outlive a range: a range replayed as a
   // CUDA graph must contain every conversion it depends on.
   umma::InvalidateRange(&umma_->ctx, 0, arena_bytes_);
@@ -1890,13 +1890,12 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     ++counters_.kernel_launches;
     return {};
   }
-  // Large exact f32 products: bf16 pieces on the tensor cores where the bits are not observed.
-  if (SplitGemmOn() && (ins.opcode == kGemmNN || ins.opcode == kGemmNT || ins.opcode == kGemmTN) &&
-      umma::SplitGemmEligible(a)) {
+  // Exact f32 products: bf16 pieces on the tensor cores where the bits are not observed.
+  if (SplitGemmOn() && ins.opcode != kGemmAccNN && umma::SplitGemmEligible(a, SplitGemmWide())) {
     int launches = 0;
-    const std::string err = umma::TrySplitGemm(&umma_->ctx, a,
-                                               RefSpace(ins.in[1]) == kArena ? 0 : (RefSpace(ins.in[1]) == kRodata ? 1 : 2),
-                                               RefOffset(ins.in[1]), stream_, &launches);
+    auto space = [](uint64_t ref) { return RefSpace(ref) == kArena ? 0 : (RefSpace(ref) == kRodata ? 1 : 2); };
+    const std::string err = umma::TrySplitGemm(&umma_->ctx, a, SplitGemmWide(), space(ins.in[0]), RefOffset(ins.in[0]),
+                                               space(ins.in[1]), RefOffset(ins.in[1]), stream_, &launches);
     if (!err.empty()) return std::unexpected("cuda: " + err);
     if (launches > 0) {
       counters_.kernel_launches += launches;

@@ -453,3 +453,7 @@ class CudaBackend {
 }  // namespace see
 
 #endif  // SEE_CUDA_BACKEND_H_
+  // In lazy coherence every exact product above 2^24 multiply-adds, any width and weight type; asked for
+  // explicitly (mode 1), or with adapter products in the CPU's arithmetic, the documented domain of
+  // see_cuda_set_split_gemm alone.
+  bool SplitGemmWide() const { return split_gemm_mode_ < 0 && adapter_fma_; }

@@ -5,23 +5,25 @@
 //     C[M,N] = epilogue( A_bf16[M,K] . B_bf16[N,K]^T )       f32 accumulate
 //
 // Blackwell-native: operands arrive by TMA (cp.async.bulk.tensor, 128-byte
-// swizzle) into a 3-stage shared-memory ring, one elected thread issues
-// tcgen05.mma (cta_group::1, kind::f16, M=128 x N=128 x K=16) with the
-// accumulator in tensor memory, tcgen05.commit hands ring slots back to the
-// producer, and four epilogue warps read the accumulator with tcgen05.ld and
-// apply scale / addend / bias / activation on the way to HBM.  One CTA per
-// 128x128 output tile, two CTAs resident per SM so one tile's epilogue
-// overlaps another's main loop.  Tensor-pipe bound for long K; for K <= 1024
-// the f32 output write is a comparable term (the arena is f32 by contract).
+// swizzle) into a shared-memory ring, one elected thread issues tcgen05.mma
+// (kind::f16) with the accumulator in tensor memory, tcgen05.commit hands ring
+// slots back to the producer, and the epilogue warps read the accumulator with
+// tcgen05.ld and apply scale / addend / bias / activation on the way to HBM.
+// Two kernels: UmmaGemmTileKernel for products of about one tile per SM, whose
+// time is latency and operand delivery, and UmmaGemmPersistentKernel for those
+// with several tiles per SM.  The reduction may also be a list of segments of
+// bf16 pieces (UmmaEpilogue::seg_blocks), which makes either an f32-accurate
+// product.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out raises
 // DeviceStatus::wait_timeout, the CTA stops issuing work, frees its tensor
 // memory and returns, and the host reports the condition at its next flush.
 #include <cuda.h>
 
-#include <utility>
-
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
+#include <utility>
 
 #include "act_expr.cuh"
 #include "kernels.h"
@@ -36,14 +38,8 @@ namespace {
 constexpr uint32_t kBlockM = umma_cfg::kBlockM;
 constexpr uint32_t kBlockN = umma_cfg::kBlockN;
 constexpr uint32_t kBlockK = umma_cfg::kBlockK;   // 64 bf16 = one 128-byte swizzle row
-constexpr uint32_t kStages = umma_cfg::kStages;
 constexpr uint32_t kUmmaK = 16;
 constexpr uint32_t kATileBytes = kBlockM * kBlockK * 2;
-constexpr uint32_t kBTileBytes = kBlockN * kBlockK * 2;
-constexpr uint32_t kStageBytes = kATileBytes + kBTileBytes;
-constexpr uint32_t kTmemCols = kBlockN;           // f32 accumulator columns
-constexpr uint32_t kThreads = 192;                // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
-
 
 using namespace umma_dev;   // mbarriers with bounded waits, TMA loads, descriptors, MMA issue, TMEM loads
 
@@ -177,30 +173,103 @@ __device__ __forceinline__ void EpilogueStoreBiasGelu(const UmmaEpilogue& ep, si
   reinterpret_cast<uint2*>(ep.shadow_dst)[at >> 2] = r;
 }
 
-struct __align__(8) Barriers {
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
+// Four neighbouring columns of one row of an output whose width is no multiple of four (an odd vocabulary): rows
+// start at any 4-byte boundary, so everything moves one element at a time.  No absorbed activation, no copy.
+__device__ __forceinline__ void EpilogueStoreRagged(const UmmaEpilogue& ep, size_t row, uint32_t n, const float4& acc) {
+  const float a[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+  for (uint32_t e = 0; e < 4; ++e) {
+    if (n + e >= ep.N) continue;
+    const size_t at = row * ep.N + n + e;
+    float v = a[e] * (ep.col_scale ? ep.col_scale[n + e] : ep.alpha);
+    if (ep.addend && !ep.addend_last) v = ep.addend[at] + v;
+    if (ep.bias) v = v + ep.bias[n + e];
+    if (ep.addend && ep.addend_last) v = ep.addend[at] + v;
+    if (ep.act != kActNone) v = ApplyAct(v, ep.act);
+    ep.C[at] = v;
+  }
+}
+
+// Element offsets along K of reduction block kb's tiles of A and B.
+struct BlockAt { int32_t a, b; bool aux; };
+__device__ __forceinline__ BlockAt BlockCoord(const UmmaEpilogue& ep, uint32_t kb, uint32_t main_blocks) {
+  if (kb >= main_blocks) {
+    const int32_t x = static_cast<int32_t>((kb - main_blocks) * kBlockK);
+    return {x, x, true};
+  }
+  if (ep.seg_blocks == 0) return {static_cast<int32_t>(kb * kBlockK), static_cast<int32_t>(kb * kBlockK), false};
+  const uint32_t seg = kb / ep.seg_blocks, w = kb - seg * ep.seg_blocks;
+  return {static_cast<int32_t>((((ep.seg_a >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK),
+          static_cast<int32_t>((((ep.seg_b >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK), false};
+}
+
+// ---- about one tile per SM --------------------------------------------------------------
+// Such a product (a data-parallel rank's 4096 rows, a few hundred rows of a short fine-tune, a
+// 256-wide f32 decoder) is bound by operand latency and by the fixed cost of a launch, not by the
+// tensor pipe.  Hence
+//  * a ring as deep as shared memory is large (4 to 8 stages): the tile's epilogue has nothing to
+//    overlap with, so it takes the ring's memory for its staging;
+//  * a tile width from 64 to 256 and a reduction cut over `splits` CTAs of a cluster, so that the
+//    grid comes near 148 CTAs whatever the shape.  The partial tiles meet in distributed shared
+//    memory: each CTA dumps its accumulator, and after a cluster barrier each takes 1 / splits of
+//    the rows, adds the partials in split order (a fixed order) and stores them;
+//  * the second operand of the epilogue (an addend, an activation's input) asked into L2 at the
+//    start: from HBM, a round trip per group of rows was 12-17 us of such a launch.
+// CTA pairs (cta_group::2, a third fewer operand bytes) were slower here at every shape: the two
+// CTAs' operands must both be there before either SM's tensor core starts.
+// Measured on a B200 (weights from HBM, plain epilogue), one-tile kernel of three stages or the
+// persistent kernel / this one, us: 4096 x 256 x 1536 16.0 / 10.8; 4096 x 256 x 6144 42 / 18.9;
+// 4096 x 768 x 3072 28.5 / 22.0; 600 x 512 x 2048 18.7 / 9.2; 600 x 512 x 8000 66 / 16.3.
+constexpr uint32_t kTThreads = 320;      // warp 0 TMA, warp 1 MMA, eight epilogue warps
+constexpr uint32_t kTEpiThreads = 256;
+constexpr uint32_t kTMaxStages = 8;
+template <uint32_t kTN>
+struct TTile {
+  static constexpr uint32_t kStageBytes = kATileBytes + kTN * kBlockK * 2;
+  static constexpr uint32_t kFit = 208u * 1024u / kStageBytes;
+  static constexpr uint32_t kStages = kFit < kTMaxStages ? kFit : kTMaxStages;
+  static constexpr uint32_t kTmemCols = kTN <= 64 ? 64 : (kTN <= 128 ? 128 : 256);
+  static_assert(kStages * kStageBytes >= kBlockM * kTN * 4, "the epilogue stages the whole tile in the ring");
+};
+
+struct __align__(8) TBarriers {
+  uint64_t full[kTMaxStages];
+  uint64_t empty[kTMaxStages];
   uint64_t tmem_full;
   uint32_t tmem_base;
   volatile uint32_t abort;  // set by a role whose wait ran out; the epilogue then stores nothing
 };
 
-__global__ void __launch_bounds__(kThreads, 2)
-UmmaGemmKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
-               UmmaEpilogue ep) {
+__device__ __forceinline__ float4 LoadClusterF4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr));
+  return v;
+}
+
+template <uint32_t kTN>
+__global__ void __launch_bounds__(kTThreads, 1)
+UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                   const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
+                   UmmaEpilogue ep, uint32_t splits) {
+  using T = TTile<kTN>;
+  constexpr uint32_t kStages = T::kStages, kStageBytes = T::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: the swizzle pattern and the descriptors' base offset assume it.
   uint8_t* smem = smem_raw + ((1024u - (SmemAddr(smem_raw) & 1023u)) & 1023u);
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes);
+  TBarriers* bars = reinterpret_cast<TBarriers*>(smem + kStages * kStageBytes);
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t m0 = blockIdx.y * kBlockM, n0 = blockIdx.x * kBlockN;
+  const uint32_t split = ClusterCtaRank();   // (a cluster is one tile's splits)
+  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, tile = blockIdx.x / splits;
+  const uint32_t mb = tile / tiles_n, nb = tile - mb * tiles_n;
+  const uint32_t m0 = mb * kBlockM, n0 = nb * kTN;
   // The reduction runs over the main operands' K and then over aux_k_blocks more
   // 64-wide blocks taken from the second pair of maps (a low-rank term T . B'^T
   // accumulated into the same tile; see UmmaEpilogue::aux_k_blocks).
   const uint32_t main_blocks = (ep.K + kBlockK - 1) / kBlockK;
   const uint32_t k_blocks = main_blocks + ep.aux_k_blocks;
+  const uint32_t kb0 = k_blocks * split / splits, kb1 = k_blocks * (split + 1) / splits;
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < kStages; ++s) {
@@ -209,118 +278,186 @@ UmmaGemmKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     MbarInit(&bars->tmem_full, 1);
     bars->abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    MbarInitFence();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(SmemAddr(&bars->tmem_base)), "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    TmemAlloc(&bars->tmem_base, T::kTmemCols);
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  TcFenceBefore();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  TcFenceAfter();
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
     // ---- TMA producer ----
     if (lane == 0) {
-      for (uint32_t kb = 0; kb < k_blocks; ++kb) {
-        const uint32_t s = kb % kStages, round = kb / kStages;
+      for (uint32_t kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+        const uint32_t s = it % kStages, round = it / kStages;
         if (round > 0 && !MbarWait(&bars->empty[s], (round - 1) & 1)) {
           ep.status->wait_timeout = 1;
           bars->abort = 1;
           break;
         }
         uint8_t* a_dst = smem + s * kStageBytes;
-        uint8_t* b_dst = a_dst + kATileBytes;
+        const BlockAt at = BlockCoord(ep, kb, main_blocks);
+        const CUtensorMap* ma = at.aux ? &map_a2 : &map_a;
+        const CUtensorMap* mb_ = at.aux ? &map_b2 : &map_b;
         MbarExpectTx(&bars->full[s], kStageBytes);
-        const bool aux = kb >= main_blocks;
-        const int32_t kx = static_cast<int32_t>((aux ? kb - main_blocks : kb) * kBlockK);
-        TmaLoad2D(a_dst, aux ? &map_a2 : &map_a, &bars->full[s], kx, static_cast<int32_t>(m0));
-        TmaLoad2D(b_dst, aux ? &map_b2 : &map_b, &bars->full[s], kx, static_cast<int32_t>(n0));
+        TmaLoad2D(a_dst, ma, &bars->full[s], at.a, static_cast<int32_t>(m0));
+        TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], at.b, static_cast<int32_t>(n0));
       }
     }
   } else if (warp == 1) {
     // ---- MMA issuer ----
     if (lane == 0) {
-      const uint32_t idesc = MakeInstrDesc(kBlockM, kBlockN);
-      bool ok = true;
-      for (uint32_t kb = 0; kb < k_blocks && ok; ++kb) {
-        const uint32_t s = kb % kStages, round = kb / kStages;
+      const uint32_t idesc = MakeInstrDesc(kBlockM, kTN);
+      for (uint32_t kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+        const uint32_t s = it % kStages, round = it / kStages;
         if (!MbarWait(&bars->full[s], round & 1)) {
           ep.status->wait_timeout = 1;
           bars->abort = 1;
-          ok = false;
           break;
         }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        TcFenceAfter();
         const uint32_t a_addr = SmemAddr(smem + s * kStageBytes);
-        const uint64_t desc_a = MakeSmemDesc(a_addr);
-        const uint64_t desc_b = MakeSmemDesc(a_addr + kATileBytes);
+        const uint64_t desc_a = MakeSmemDesc(a_addr), desc_b = MakeSmemDesc(a_addr + kATileBytes);
 #pragma unroll
         for (uint32_t k = 0; k < kBlockK / kUmmaK; ++k) {
           // advance 16 bf16 = 32 bytes inside the 128-byte swizzle row: +2 in >>4 units
-          UmmaBf16(tmem_base, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+          UmmaBf16(tmem_base, desc_a + 2 * k, desc_b + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
         }
-        UmmaCommit(&bars->empty[s]);  // the slot is free once these MMAs have read it
+        UmmaCommit(&bars->empty[s]);   // the slot is free once these MMAs have read it
       }
-      UmmaCommit(&bars->tmem_full);   // accumulator complete (or abandoned on timeout)
+      UmmaCommit(&bars->tmem_full);    // accumulator complete (or abandoned on timeout)
     }
-  } else {
-    // ---- epilogue: warps 2..5, TMEM lane quarter = warp % 4 ----
-    const uint32_t quarter = warp & 3;
-    bool ok = MbarWait(&bars->tmem_full, 0);
+  }
+  __syncwarp();
+  const bool epilogue = warp >= 2;
+  const uint32_t et = threadIdx.x - 64;   // thread of the epilogue
+  const float* side_ptr = ep.fuse_mode == kFuseActBwd ? ep.fuse_x : ep.addend;
+  const bool ragged = (ep.N & 3u) != 0;
+  constexpr uint32_t kChunks = kTN / 4;
+  const uint32_t rows = kBlockM / splits, r0 = split * rows;   // the rows this CTA stores
+  bool ok = true;
+  if (epilogue) {
+    // The second operand of the epilogue is asked into L2 while the products run.
+    if (side_ptr && !ragged)
+      for (uint32_t i = et; i < rows * (kTN / 32); i += kTEpiThreads) {
+        const uint32_t row = m0 + r0 + i / (kTN / 32), n = n0 + i % (kTN / 32) * 32;
+        if (row < ep.M && n < ep.N)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(side_ptr + static_cast<size_t>(row) * ep.N + n));
+      }
+    const uint32_t quarter = warp & 3, columns = ((warp - 2) >> 2) * (kTN / 2);
+    ok = MbarWait(&bars->tmem_full, 0);
     if (!ok && lane == 0) ep.status->wait_timeout = 1;
     if (bars->abort) ok = false;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok && k_blocks > 0) {
-      // The accumulator arrives one row per thread; HBM wants one row per warp
-      // access.  Each warp turns its 32 x 128 slab through shared memory: the
-      // operand ring is idle by now (tmem_full fires after the last MMA has read
-      // it), so the slab lives there.  16-byte chunks are XOR-swizzled with the
-      // row so both the row-per-thread writes and the row-per-warp reads are
-      // bank-conflict free.  Only this warp touches its slab: __syncwarp suffices.
-      float* slab = reinterpret_cast<float*>(smem + quarter * (32 * kBlockN * 4));
+    ok = __all_sync(0xFFFFFFFFu, ok);
+    TcFenceAfter();
+    if (ok) {
+      // The accumulator arrives one row per thread; HBM wants whole rows.  All MMAs are complete, so
+      // the ring is free: the tile goes there as [128][kTN] f32, 16-byte chunks XOR-ed with the
+      // row so that neither side conflicts.
+      float* dump = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kTN;
 #pragma unroll 1
-      for (uint32_t c0 = 0; c0 < kBlockN; c0 += 32) {
+      for (uint32_t c0 = 0; c0 < kTN / 2; c0 += 32) {
         uint32_t r[32];
-        TmemLoad32(tmem_base + ((quarter * 32) << 16) + c0, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        TmemLoad32(tmem_base + ((quarter * 32) << 16) + columns + c0, r);
+        TmemWaitLd();
 #pragma unroll
-        for (uint32_t q = 0; q < 8; ++q) {
-          const uint32_t chunk = ((c0 >> 2) + q) ^ lane;   // 32 chunks of 4 floats per row
-          *reinterpret_cast<uint4*>(slab + lane * kBlockN + chunk * 4) =
+        for (uint32_t q = 0; q < 8; ++q)
+          *reinterpret_cast<uint4*>(dump + ((((columns + c0) >> 2) + q) ^ (lane & 7u)) * 4) =
               make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+      }
+    }
+    TcFenceBefore();
+  }
+  if (splits > 1) ClusterSync();
+  else if (epilogue) asm volatile("bar.sync 1, %0;" ::"n"(kTEpiThreads) : "memory");
+  if (epilogue && ok) {
+    const uint32_t dump = SmemAddr(smem);
+    // The tile's element of row r0 + lr, chunk: this CTA's, or the sum of the splits' partials.
+    auto element = [&](uint32_t lr, uint32_t chunk) {
+      const uint32_t off = (lr * kTN + (chunk ^ (lr & 7u)) * 4) * 4;
+      if (splits == 1) return *reinterpret_cast<const float4*>(smem + off);
+      float4 acc = LoadClusterF4(MapToCta(dump + off, 0));
+      for (uint32_t p = 1; p < splits; ++p) {
+        const float4 v = LoadClusterF4(MapToCta(dump + off, p));
+        acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+      }
+      return acc;
+    };
+    // Four elements per thread at a time, their operands loaded before the first is stored.  `store` is one form of
+    // the epilogue, chosen once: tests per element would cost more than the stores.
+    constexpr uint32_t kUnroll = 4;
+    auto each = [&](auto has_side, auto store) {
+      for (uint32_t i0 = et; i0 < rows * kChunks; i0 += kTEpiThreads * kUnroll) {
+        float4 acc[kUnroll], side[kUnroll];
+#pragma unroll
+        for (uint32_t u = 0; u < kUnroll; ++u) {
+          const uint32_t i = i0 + u * kTEpiThreads, lr = r0 + i / kChunks, chunk = i % kChunks;
+          const uint32_t row = m0 + lr, n = n0 + chunk * 4;
+          if (i >= rows * kChunks || row >= ep.M || n >= ep.N) continue;
+          if constexpr (decltype(has_side)::value)
+            side[u] = __ldg(reinterpret_cast<const float4*>(side_ptr + static_cast<size_t>(row) * ep.N + n));
+          acc[u] = element(lr, chunk);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kUnroll; ++u) {
+          const uint32_t i = i0 + u * kTEpiThreads, lr = r0 + i / kChunks, chunk = i % kChunks;
+          const uint32_t row = m0 + lr, n = n0 + chunk * 4;
+          if (i >= rows * kChunks || row >= ep.M || n >= ep.N) continue;
+          float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
+          if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
+          store(static_cast<size_t>(row) * ep.N + n, row, n, acc[u], scale, side[u]);
         }
       }
-      __syncwarp();
-      // Lane l owns columns n0 + 4l .. 4l+3 of every row: its scale / bias are loop invariants.
-      const uint32_t n = n0 + lane * 4;
-      if (n < ep.N) {   // N % 4 == 0: a float4 is all in or all out
-        float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
-        if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
-        float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ep.bias) bias = __ldg(reinterpret_cast<const float4*>(ep.bias + n));
-        const uint32_t row0 = m0 + quarter * 32;
-        const uint32_t rows = row0 < ep.M ? (ep.M - row0 < 32 ? ep.M - row0 : 32) : 0;
-#pragma unroll 4
-        for (uint32_t rr = 0; rr < rows; ++rr) {
-          const float4 acc = *reinterpret_cast<const float4*>(slab + rr * kBlockN + ((lane ^ rr) * 4));
-          const size_t at = static_cast<size_t>(row0 + rr) * ep.N + n;
-          EpilogueStore(ep, at, n, acc, scale, bias);
-        }
+    };
+    const float4 one = make_float4(1.f, 1.f, 1.f, 1.f), none = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto bias_at = [&](uint32_t n) { return ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : none; };
+    using Side = std::true_type;
+    using NoSide = std::false_type;
+    if (ragged) {
+      for (uint32_t i = et; i < rows * kChunks; i += kTEpiThreads) {
+        const uint32_t lr = r0 + i / kChunks, row = m0 + lr, n = n0 + i % kChunks * 4;
+        if (row < ep.M && n < ep.N) EpilogueStoreRagged(ep, row, n, element(lr, i % kChunks));
       }
+    } else if (IsPlainStore(ep)) {
+      each(NoSide{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4&) {
+        EpilogueStorePlain(ep, at, acc, scale);
+      });
+    } else if (IsAddendOnly(ep)) {
+      each(Side{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4& side) {
+        EpilogueStoreAddend(ep, at, acc, scale, side);
+      });
+    } else if (IsCopyOnly(ep)) {
+      each(NoSide{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4&) {
+        EpilogueStoreCopy(ep, at, acc, scale);
+      });
+    } else if (IsBiasGeluOnly(ep) && !ep.shadow_k_scale) {
+      each(NoSide{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4&) {
+        EpilogueStoreBiasGelu(ep, at, acc, scale, bias_at(n), one);
+      });
+    } else if (IsGeluGradOnly(ep) && !ep.shadow_k_scale) {
+      each(Side{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4& side) {
+        EpilogueStoreGeluGrad(ep, at, acc, scale, one, side);
+      });
+    } else if (side_ptr) {
+      each(Side{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4& side) {
+        EpilogueStore(ep, at, n, acc, scale, bias_at(n), false, one, true, side);
+      });
+    } else {
+      each(NoSide{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4&) {
+        EpilogueStore(ep, at, n, acc, scale, bias_at(n));
+      });
     }
   }
 
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  TcFenceBefore();
   __syncthreads();
+  if (splits > 1) ClusterSync();   // no CTA leaves while another may still read its memories
   if (warp == 1) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(kTmemCols)
-                 : "memory");
+    TcFenceAfter();
+    TmemFree(tmem_base, T::kTmemCols);
   }
 }
 
@@ -337,11 +474,7 @@ UmmaGemmKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // under tile i+1's main loop.  What the one-tile kernel pays per tile — barrier
 // set-up, tensor-memory allocation, the first TMA round trip, CTA launch and
 // retirement — is paid once per SM.
-// The tile width is a template parameter: 256 columns where the product has tiles
-// to spare, 128 where the wide tile would leave SMs without work (a shard of a
-// few thousand rows with a 768-wide output: 96 wide tiles for 148 SMs, against
-// 192 narrow ones; the narrow tile's shorter stage buys a fourth ring slot).
-constexpr uint32_t kPBlockN = 256;                     // the wide tile
+constexpr uint32_t kPBlockN = 256;
 constexpr uint32_t kPMaxStages = 5;
 constexpr uint32_t kPEpiWarps = 16;
 constexpr uint32_t kPThreads = 64 + 32 * kPEpiWarps;   // warp 0 TMA, warp 1 MMA, then the epilogue warps
@@ -354,14 +487,14 @@ constexpr uint32_t kSlabBytes = 32 * kSlabCols * 4;   // one epilogue warp's 32 
 // receives its own 128 rows.  A third less operand traffic from L2 per flop, and
 // the smaller stage leaves room for five ring slots: the K = 768 shapes of the
 // step were bound by bytes in flight per SM, not by the tensor pipe.
-template <uint32_t kTN, bool kPair>
+template <bool kPair>
 struct PTile {
-  static constexpr uint32_t kStages = kPair ? 5 : (kTN == 256 ? 3 : 4);
-  static constexpr uint32_t kBRows = kPair ? kTN / 2 : kTN;      // rows of B this CTA loads per k block
+  static constexpr uint32_t kStages = kPair ? 5 : 3;
+  static constexpr uint32_t kBRows = kPair ? kPBlockN / 2 : kPBlockN;      // rows of B this CTA loads per k block
   static constexpr uint32_t kBTileBytes = kBRows * kBlockK * 2;
   static constexpr uint32_t kStageBytes = kATileBytes + kBTileBytes;
-  static constexpr uint32_t kTmemCols = 2 * kTN;
-  static constexpr uint32_t kColsPerEpiWarp = kTN / (kPEpiWarps / 4);
+  static constexpr uint32_t kTmemCols = 2 * kPBlockN;
+  static constexpr uint32_t kColsPerEpiWarp = kPBlockN / (kPEpiWarps / 4);
   static constexpr uint32_t kEpiPasses = kColsPerEpiWarp / kSlabCols;
   static constexpr uint32_t kRowsPerTile = kPair ? 2 * kBlockM : kBlockM;
 };
@@ -402,14 +535,15 @@ struct __align__(8) PBarriers {
 // while this group is converted and stored, across passes and from before the
 // wait for the accumulator, so a memory round trip is not paid per group with
 // every warp of the CTA waiting on it.
-template <bool kSideLoads, uint32_t kTN, bool kPair>
+template <bool kSideLoads, bool kPair>
 __global__ void __launch_bounds__(kPThreads, 1)
 UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
                          const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_a2,
                          const __grid_constant__ CUtensorMap map_b2, UmmaEpilogue ep,
                          uint32_t band_blocks) {
-  using T = PTile<kTN, kPair>;
+  using T = PTile<kPair>;
+  constexpr uint32_t kTN = kPBlockN;
   constexpr uint32_t kPStages = T::kStages, kPStageBytes = T::kStageBytes, kPTmemCols = T::kTmemCols;
   constexpr uint32_t kColsPerEpiWarp = T::kColsPerEpiWarp, kEpiPasses = T::kEpiPasses;
   extern __shared__ uint8_t smem_raw[];
@@ -467,7 +601,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         const uint32_t m0 = mb * T::kRowsPerTile + cta_rank * kBlockM, n0 = nb * kTN;
         // Ask L2 for the A rows of this CTA's next tile now, so that its loads
         // find them there instead of paying an HBM round trip inside the ring.
-        if (t + units < total_tiles && k_blocks <= 64) {   // (a long K would only thrash L2)
+        if (t + units < total_tiles && k_blocks <= 64 && ep.seg_blocks == 0) {   // (a long K would only thrash L2)
           uint32_t next_mb, next_nb;
           TileCoord(t + units, tiles_m, tiles_n, band_blocks, &next_mb, &next_nb);
           const uint32_t next_m0 = next_mb * T::kRowsPerTile + cta_rank * kBlockM;
@@ -487,24 +621,22 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
             break;
           }
           uint8_t* a_dst = smem + s * kPStageBytes;
-          const bool aux = kb >= main_blocks;
-          const CUtensorMap* ma = aux ? &map_a2 : &map_a;
-          const CUtensorMap* mb_ = aux ? &map_b2 : &map_b;
-          const int32_t kx = static_cast<int32_t>((aux ? kb - main_blocks : kb) * kBlockK);
+          const BlockAt at = BlockCoord(ep, kb, main_blocks);
+          const CUtensorMap* ma = at.aux ? &map_a2 : &map_a;
+          const CUtensorMap* mb_ = at.aux ? &map_b2 : &map_b;
           if constexpr (kPair) {
             // Both CTAs' bytes are counted on the even CTA's barrier, which alone expects them.
             if (cta_rank == 0) MbarExpectTx(&bars->full[s], 2 * kPStageBytes);
             const uint32_t full_bar = MapToCta(SmemAddr(&bars->full[s]), 0);
-            TmaLoad2DPair(a_dst, ma, full_bar, kx, static_cast<int32_t>(m0));
-            TmaLoad2DPair(a_dst + kATileBytes, mb_, full_bar, kx, static_cast<int32_t>(n0 + cta_rank * kBlockN));
+            TmaLoad2DPair(a_dst, ma, full_bar, at.a, static_cast<int32_t>(m0));
+            TmaLoad2DPair(a_dst + kATileBytes, mb_, full_bar, at.b, static_cast<int32_t>(n0 + cta_rank * kBlockN));
           } else {
             MbarExpectTx(&bars->full[s], kPStageBytes);
-            TmaLoad2D(a_dst, ma, &bars->full[s], kx, static_cast<int32_t>(m0));
-            // B's rows as 128-row boxes, back to back: one [kTN][64] tile.
-            TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], kx, static_cast<int32_t>(n0));
-            if constexpr (kTN == 256)
-              TmaLoad2D(a_dst + kATileBytes + kBTileBytes, mb_, &bars->full[s], kx,
-                        static_cast<int32_t>(n0 + kBlockN));
+            TmaLoad2D(a_dst, ma, &bars->full[s], at.a, static_cast<int32_t>(m0));
+            // B's rows as 128-row boxes, back to back: one [256][64] tile.
+            TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], at.b, static_cast<int32_t>(n0));
+            TmaLoad2D(a_dst + kATileBytes + kBlockN * kBlockK * 2, mb_, &bars->full[s], at.b,
+                      static_cast<int32_t>(n0 + kBlockN));
           }
         }
       }
@@ -541,11 +673,11 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
             if constexpr (kPair) UmmaBf16Pair(acc, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
             else UmmaBf16(acc, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
           }
-          if constexpr (kPair) UmmaCommitPair(&bars->empty[s]);
+          if constexpr (kPair) UmmaCommitPair(&bars->empty[s], 0);
           else UmmaCommit(&bars->empty[s]);
         }
         // accumulator complete (or abandoned on timeout)
-        if constexpr (kPair) UmmaCommitPair(&bars->tmem_full[buf]);
+        if constexpr (kPair) UmmaCommitPair(&bars->tmem_full[buf], 0);
         else UmmaCommit(&bars->tmem_full[buf]);
       }
     }
@@ -590,6 +722,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
       [[maybe_unused]] const bool bias_gelu_only = IsBiasGeluOnly(ep);
       [[maybe_unused]] const bool copy_only = IsCopyOnly(ep);
       [[maybe_unused]] const bool plain_store = IsPlainStore(ep);
+      [[maybe_unused]] const bool ragged = (ep.N & 3u) != 0;   // (never with kSideLoads)
       [[maybe_unused]] float4 side_a[4], side_b[4];
       if constexpr (kSideLoads) {   // the first group's loads fly during the wait for the accumulator
         const uint32_t n_g = n0 + col_group * kColsPerEpiWarp + cl * 4;
@@ -636,7 +769,11 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
                 make_uint4(ra[4 * q], ra[4 * q + 1], ra[4 * q + 2], ra[4 * q + 3]);
           __syncwarp();
           const uint32_t n = n0 + col_group * kColsPerEpiWarp + pass * kSlabCols + cl * 4;
-          if (n < ep.N) {   // N % 4 == 0: a float4 is all in or all out
+          if (ragged) {
+            for (uint32_t rr = sub; rr < rows; rr += kRowsPerInstr)
+              EpilogueStoreRagged(ep, row0 + rr, n, *reinterpret_cast<const float4*>(
+                                                        slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4)));
+          } else if (n < ep.N) {   // N % 4 == 0: a float4 is all in or all out
             float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
             if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
             float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -799,21 +936,18 @@ __global__ void WeightToBf16Kernel(const T* __restrict__ src, uint16_t* __restri
 
 }  // namespace
 
-size_t UmmaSmemBytes() { return kStages * kStageBytes + sizeof(Barriers) + 1024; }
-template <uint32_t kTN, bool kPair>
+template <bool kPair>
 static size_t UmmaPersistentSmemBytes() {
-  using T = PTile<kTN, kPair>;
+  using T = PTile<kPair>;
   return T::kStages * T::kStageBytes + kPEpiWarps * kSlabBytes + sizeof(PBarriers) + 1024;
 }
-
-template <bool kSideLoads, uint32_t kTN, bool kPair>
-static cudaError_t ConfigurePersistent() {
-  return cudaFuncSetAttribute(UmmaGemmPersistentKernel<kSideLoads, kTN, kPair>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(UmmaPersistentSmemBytes<kTN, kPair>()));
+template <uint32_t kTN>
+static size_t UmmaTileSmemBytes() {
+  using T = TTile<kTN>;
+  return T::kStages * T::kStageBytes + sizeof(TBarriers) + 1024;
 }
 
-// A launch with an optional cluster dimension (2 for the CTA-pair form).
+// A launch with an optional cluster dimension.
 // (Programmatic dependent launches — the next kernel's set-up run beside this
 // one's tail — were measured on the whole step and cost 1 %: not used.)
 template <typename... KArgs, typename... Args>
@@ -834,34 +968,87 @@ static cudaError_t LaunchClustered(void (*kernel)(KArgs...), dim3 grid, dim3 blo
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-template <uint32_t kTN>
-static cudaError_t LaunchPersistent(uint32_t grid, bool side_loads, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                                    const CUtensorMap& map_a2, const CUtensorMap& map_b2, const UmmaEpilogue& ep,
-                                    uint32_t band, cudaStream_t s) {
-  const size_t smem = UmmaPersistentSmemBytes<kTN, false>();
-  if (side_loads)
-    return LaunchClustered(UmmaGemmPersistentKernel<true, kTN, false>, dim3(grid), dim3(kPThreads), smem, s, 1u, map_a,
-                           map_b, map_a2, map_b2, ep, band);
-  return LaunchClustered(UmmaGemmPersistentKernel<false, kTN, false>, dim3(grid), dim3(kPThreads), smem, s, 1u, map_a,
-                         map_b, map_a2, map_b2, ep, band);
-}
-
-// The CTA-pair form: clusters of two, an even grid.
-static cudaError_t LaunchPairs(uint32_t grid, bool side_loads, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                               const CUtensorMap& map_a2, const CUtensorMap& map_b2, const UmmaEpilogue& ep,
-                               uint32_t band, cudaStream_t s) {
-  const size_t smem = UmmaPersistentSmemBytes<256, true>();
-  if (side_loads)
-    return LaunchClustered(UmmaGemmPersistentKernel<true, 256, true>, dim3(grid & ~1u), dim3(kPThreads), smem, s, 2u,
-                           map_a, map_b, map_a2, map_b2, ep, band);
-  return LaunchClustered(UmmaGemmPersistentKernel<false, 256, true>, dim3(grid & ~1u), dim3(kPThreads), smem, s, 2u,
-                         map_a, map_b, map_a2, map_b2, ep, band);
+// Calls f(kernel, shared-memory bytes) with the tile kernel of this width.
+template <typename F>
+static cudaError_t WithTileKernel(uint32_t tn, F f) {
+  switch (tn) {
+    case 64: return f(UmmaGemmTileKernel<64>, UmmaTileSmemBytes<64>());
+    case 128: return f(UmmaGemmTileKernel<128>, UmmaTileSmemBytes<128>());
+    case 192: return f(UmmaGemmTileKernel<192>, UmmaTileSmemBytes<192>());
+    default: return f(UmmaGemmTileKernel<256>, UmmaTileSmemBytes<256>());
+  }
 }
 
 static std::atomic<bool> g_cta_pairs{true};
 void UmmaSetCtaPairs(bool on) { g_cta_pairs.store(on, std::memory_order_relaxed); }
 
-cudaError_t UmmaGemmLaunch(const CUtensorMap& map_a, const CUtensorMap& map_b,
+static cudaError_t Configure() {
+  auto allow = [](auto kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  };
+  cudaError_t e = cudaSuccess;
+  for (uint32_t tn : {64u, 128u, 192u, 256u})
+    if ((e = WithTileKernel(tn, allow)) != cudaSuccess) return e;
+  if ((e = allow(UmmaGemmPersistentKernel<false, false>, UmmaPersistentSmemBytes<false>())) != cudaSuccess) return e;
+  if ((e = allow(UmmaGemmPersistentKernel<true, false>, UmmaPersistentSmemBytes<false>())) != cudaSuccess) return e;
+  if ((e = allow(UmmaGemmPersistentKernel<false, true>, UmmaPersistentSmemBytes<true>())) != cudaSuccess) return e;
+  return allow(UmmaGemmPersistentKernel<true, true>, UmmaPersistentSmemBytes<true>());
+}
+
+UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, bool light, uint32_t sms) {
+  UmmaGemmPlan p;
+  const uint32_t ptiles_n = (N + kPBlockN - 1) / kPBlockN, tiles_m = (M + kBlockM - 1) / kBlockM;
+  const uint64_t wide = static_cast<uint64_t>(ptiles_n) * tiles_m;
+  const bool pairs_on = g_cta_pairs.load(std::memory_order_relaxed) && sms >= 2;
+  // The tile kernel, on the width and split of least estimated time (us): waves of CTAs, each a fixed part, its
+  // reduction blocks, its epilogue and, when the reduction is cut, the exchange.  The constants are a fit (10 %
+  // standard error) to a sweep of 32 to 4096 rows, widths 256 to 32000 and K 512 to 32000 on a B200; the persistent
+  // kernel's likewise.
+  double best = 1e30;
+  for (uint32_t tn : {64u, 128u, 192u, 256u})
+    for (uint32_t splits = 1; splits <= 4 && splits <= k_blocks; splits *= 2) {
+      const uint64_t ctas = static_cast<uint64_t>(tiles_m) * ((N + tn - 1) / tn) * splits;
+      const uint64_t room = splits <= 2 ? sms : sms * 9 / 10;   // clusters of four do not fill every GPC
+      const double waves = static_cast<double>((ctas + room - 1) / room);
+      const double block = std::max(0.165 + 0.00087 * tn, 0.267);
+      const double t = 0.8 + waves * (2.0 + block * ((k_blocks + splits - 1) / splits) + 0.02 * tn / splits + (splits > 1 ? 3.0 : 0.0));
+      if (t < best) {
+        best = t;
+        p.tn = tn;
+        p.splits = splits;
+        p.grid = static_cast<uint32_t>(ctas);
+        p.b_box = tn;
+      }
+    }
+  if (wide > sms) {
+    // Enough tiles for every SM to amortise its set-up over several: a round of the persistent kernel is its main
+    // loop (0.53 us per reduction block, 0.43 in CTA pairs, which load a third fewer bytes per flop) or its
+    // epilogue, whichever is longer.  At 32768 rows the epilogue is HBM's: plain and copy-only ones take 8.3 us a tile
+    // and 7.3 in pairs, those with a second operand or an activation about 10.5 and 11.5, for a pair's two epilogues
+    // must both finish before the accumulator is free again.  An output that stays in L2 takes about 2 us less.
+    const uint64_t pair_tiles = static_cast<uint64_t>(ptiles_n) * ((M + 2 * kBlockM - 1) / (2 * kBlockM));
+    const uint64_t pairs = sms / 2;
+    const double l2 = static_cast<uint64_t>(M) * N <= (1ull << 24) ? 2.0 : 0.0;
+    const double single = 7.0 + static_cast<double>((wide + sms - 1) / sms) * std::max(0.53 * k_blocks, (light ? 8.3 : 10.5) - l2);
+    const double paired = pairs_on && wide > 2ull * sms
+                              ? 7.5 + static_cast<double>((pair_tiles + pairs - 1) / pairs) *
+                                          std::max(0.43 * k_blocks, (light ? 7.3 : 11.5) - l2)
+                              : 1e30;
+    if (std::min(single, paired) < best) {
+      p = UmmaGemmPlan{};
+      p.persistent = true;
+      p.pair = paired < single;
+      p.tn = kPBlockN;
+      p.grid = p.pair ? sms & ~1u : sms;
+      const uint32_t band = ptiles_n >= kWideTilesN ? kWideBandBlocks : 1u;
+      p.band = p.pair && band > 1 ? band / 2 : band;
+      p.b_box = kBlockN;
+    }
+  }
+  return p;
+}
+
+cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const CUtensorMap& map_a, const CUtensorMap& map_b,
                            const UmmaEpilogue& ep, cudaStream_t s, const CUtensorMap* aux_a,
                            const CUtensorMap* aux_b) {
   // Without a low-rank term the second pair of maps is never dereferenced; the
@@ -871,54 +1058,29 @@ cudaError_t UmmaGemmLaunch(const CUtensorMap& map_a, const CUtensorMap& map_b,
   // The shared-memory limit of a kernel is a per-device attribute: one flag per
   // device, so a second backend on another GPU of the same process configures its own.
   static std::atomic<bool> configured_on[64] = {};
-  static int sm_count[64] = {};
-  const size_t smem = UmmaSmemBytes();
   int dev = 0;
   cudaGetDevice(&dev);
   const bool tracked = dev >= 0 && dev < 64;
   if (!tracked || !configured_on[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(UmmaGemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    if ((e = ConfigurePersistent<false, 256, false>()) != cudaSuccess) return e;
-    if ((e = ConfigurePersistent<true, 256, false>()) != cudaSuccess) return e;
-    if ((e = ConfigurePersistent<false, 128, false>()) != cudaSuccess) return e;
-    if ((e = ConfigurePersistent<true, 128, false>()) != cudaSuccess) return e;
-    if ((e = ConfigurePersistent<false, 256, true>()) != cudaSuccess) return e;
-    if ((e = ConfigurePersistent<true, 256, true>()) != cudaSuccess) return e;
+    if (cudaError_t e = Configure(); e != cudaSuccess) return e;
     if (tracked) configured_on[dev].store(true, std::memory_order_release);
   }
-  if (dev >= 0 && dev < 64 && sm_count[dev] == 0)
-    cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-  const uint32_t sms = (dev >= 0 && dev < 64 && sm_count[dev] > 0) ? sm_count[dev] : 148;
-  const uint32_t tiles_n = (ep.N + kBlockN - 1) / kBlockN, tiles_m = (ep.M + kBlockM - 1) / kBlockM;
-  const uint32_t ptiles_n = (ep.N + kPBlockN - 1) / kPBlockN;
-  const uint64_t wide = static_cast<uint64_t>(ptiles_n) * tiles_m, narrow = static_cast<uint64_t>(tiles_n) * tiles_m;
-  const bool side_loads = ep.addend != nullptr || ep.fuse_mode == kFuseActBwd;
-  if (wide > 2ull * sms) {
-    // Enough tiles for every SM to amortise its set-up over several.
-    const uint32_t band = ptiles_n >= kWideTilesN ? kWideBandBlocks : 1u;
-    // CTA pairs where the reduction is long: measured at 32768 rows, K = 3072 and 32000 gain 9-10 % (a third
-    // less operand traffic per flop), while at K = 768 the epilogue sets the pace and a pair's two epilogues,
-    // which must both finish before the accumulator buffer is free again, cost 5-15 % where they are heavy.
-    if (g_cta_pairs.load(std::memory_order_relaxed) && sms >= 2 && ep.K >= 1536)
-      return LaunchPairs(sms, side_loads, map_a, map_b, map_a2, map_b2, ep, band > 1 ? band / 2 : 1u, s);
-    return LaunchPersistent<256>(sms, side_loads, map_a, map_b, map_a2, map_b2, ep, band, s);
-  }
-  if (narrow >= sms / 2) {
-    // A shard-sized product: the persistent kernel's staged, coalesced epilogue on
-    // whichever tile width finishes first, counted in rounds of 128 columns (plus
-    // a quarter tile of fixed cost per round).
-    const uint64_t wide_cost = ((wide + sms - 1) / sms) * (256 + 32);
-    const uint64_t narrow_cost = ((narrow + sms - 1) / sms) * (128 + 32);
-    if (wide_cost <= narrow_cost)
-      return LaunchPersistent<256>(static_cast<uint32_t>(wide < sms ? wide : sms), side_loads, map_a, map_b, map_a2,
-                                   map_b2, ep, 1u, s);
-    return LaunchPersistent<128>(static_cast<uint32_t>(narrow < sms ? narrow : sms), side_loads, map_a, map_b, map_a2,
-                                 map_b2, ep, 1u, s);
-  }
-  dim3 grid(tiles_n, tiles_m);
-  return LaunchClustered(UmmaGemmKernel, grid, dim3(kThreads), smem, s, 1u, map_a, map_b, map_a2, map_b2, ep);
+  if (!plan.persistent)
+    return WithTileKernel(plan.tn, [&](auto kernel, size_t bytes) {
+      return LaunchClustered(kernel, dim3(plan.grid), dim3(kTThreads), bytes, s, plan.splits, map_a, map_b, map_a2,
+                             map_b2, ep, plan.splits);
+    });
+  // An addend or the x of an absorbed backward activation is software-pipelined (16 bytes at a time).
+  const bool side_loads = (ep.addend != nullptr || ep.fuse_mode == kFuseActBwd) && (ep.N & 3) == 0;
+  auto launch = [&](auto kernel, size_t bytes) {
+    return LaunchClustered(kernel, dim3(plan.grid), dim3(kPThreads), bytes, s, plan.pair ? 2u : 1u, map_a, map_b, map_a2,
+                           map_b2, ep, plan.band);
+  };
+  if (plan.pair)
+    return side_loads ? launch(UmmaGemmPersistentKernel<true, true>, UmmaPersistentSmemBytes<true>())
+                      : launch(UmmaGemmPersistentKernel<false, true>, UmmaPersistentSmemBytes<true>());
+  return side_loads ? launch(UmmaGemmPersistentKernel<true, false>, UmmaPersistentSmemBytes<false>())
+                    : launch(UmmaGemmPersistentKernel<false, false>, UmmaPersistentSmemBytes<false>());
 }
 
 void WeightToBf16(const void* src, BType type, uint16_t* dst, uint32_t N, uint32_t K,

@@ -80,79 +80,97 @@ __global__ void SplitWeightsKernel(const LoraWeight* __restrict__ table, int cou
 }
 
 // ---- whole matrices: an f32 GEMM on the bf16 tensor cores -------------------------------
-// dst [rows][6 * cols] bf16: six K segments of `cols` each, segment s holding
-// piece PieceOf(0, s) (the A side of a product) or PieceOf(1, s) (the B side) of
-// every element, so that A' B'^T over the long K axis is the six-product sum of
-// the header comment (in its order: small products first).  src is [rows][cols], or [cols][rows] when transposed
-// (then a 32 x 32 tile goes through shared memory so both sides stay coalesced).
-template <int kSide>
+// dst [rows][3 Kp] bf16, Kp = cols rounded up to 64: piece p of element c at column p Kp + c, zero padding after
+// cols.  src is [rows][cols], or [cols][rows] when transposed (then a 32 x 32 tile goes through shared memory so both
+// sides stay coalesced).  An element is multiplied by k_scale[c] first when that is given.  HBM-bound (4 bytes read,
+// 6 written per element); which pieces a product multiplies, and in which order, is the GEMM's segment list.
+// A thread takes eight columns: 32 bytes in, 16 bytes out per piece.
+template <bool kVec>
 __global__ void SplitMatrixKernel(const float* __restrict__ src, uint16_t* __restrict__ dst, uint32_t rows,
-                                  uint32_t cols) {
-  const size_t quads = static_cast<size_t>(rows) * (cols / 4);
+                                  uint32_t cols, uint32_t kp, const float* __restrict__ k_scale) {
+  const uint32_t per_row = kp / 8;
+  const size_t octs = static_cast<size_t>(rows) * per_row;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  for (size_t q = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; q < quads; q += stride) {
-    const uint32_t row = static_cast<uint32_t>(q / (cols / 4)), c4 = static_cast<uint32_t>(q % (cols / 4)) * 4;
-    const float4 v = *reinterpret_cast<const float4*>(src + static_cast<size_t>(row) * cols + c4);
-    uint16_t p[4][3];
-    Split3(v.x, p[0]); Split3(v.y, p[1]); Split3(v.z, p[2]); Split3(v.w, p[3]);
-    uint16_t* out = dst + static_cast<size_t>(row) * 6 * cols + c4;
+  for (size_t q = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; q < octs; q += stride) {
+    const uint32_t row = static_cast<uint32_t>(q / per_row), c = static_cast<uint32_t>(q % per_row) * 8;
+    const float* p = src + static_cast<size_t>(row) * cols + c;
+    float v[8];
+    if (kVec) {   // cols % 4 == 0: four elements are all in or all out
 #pragma unroll
-    for (int s = 0; s < 6; ++s) {
-      const int pc = PieceOf(kSide, s);
-      uint2 w;
-      w.x = static_cast<uint32_t>(p[0][pc]) | (static_cast<uint32_t>(p[1][pc]) << 16);
-      w.y = static_cast<uint32_t>(p[2][pc]) | (static_cast<uint32_t>(p[3][pc]) << 16);
-      *reinterpret_cast<uint2*>(out + static_cast<size_t>(s) * cols) = w;
+      for (uint32_t h = 0; h < 8; h += 4) {
+        const float4 f = c + h < cols ? *reinterpret_cast<const float4*>(p + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[h] = f.x; v[h + 1] = f.y; v[h + 2] = f.z; v[h + 3] = f.w;
+      }
+    } else {
+#pragma unroll
+      for (uint32_t e = 0; e < 8; ++e) v[e] = c + e < cols ? p[e] : 0.0f;
     }
+    if (k_scale) {
+#pragma unroll
+      for (uint32_t e = 0; e < 8; ++e)
+        if (c + e < cols) v[e] = v[e] * k_scale[c + e];
+    }
+    uint32_t w[3][4];
+#pragma unroll
+    for (uint32_t e = 0; e < 8; e += 2) {
+      uint16_t lo[3], hi[3];
+      Split3(v[e], lo);
+      Split3(v[e + 1], hi);
+#pragma unroll
+      for (uint32_t i = 0; i < 3; ++i) w[i][e / 2] = static_cast<uint32_t>(lo[i]) | (static_cast<uint32_t>(hi[i]) << 16);
+    }
+    uint16_t* out = dst + static_cast<size_t>(row) * 3 * kp + c;
+#pragma unroll
+    for (uint32_t i = 0; i < 3; ++i)
+      *reinterpret_cast<uint4*>(out + static_cast<size_t>(i) * kp) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
   }
 }
 
 // src [cols][rows] -> dst row r, column c = src[c][r].
-template <int kSide>
 __global__ void SplitMatrixTransposedKernel(const float* __restrict__ src, uint16_t* __restrict__ dst,
-                                            uint32_t rows, uint32_t cols) {
+                                            uint32_t rows, uint32_t cols, uint32_t kp, const float* __restrict__ k_scale) {
   __shared__ float tile[32][33];
   const uint32_t r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
   for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
     const uint32_t c = c0 + i, r = r0 + threadIdx.x;
-    tile[i][threadIdx.x] = c < cols && r < rows ? src[static_cast<size_t>(c) * rows + r] : 0.0f;
+    float v = c < cols && r < rows ? src[static_cast<size_t>(c) * rows + r] : 0.0f;
+    if (k_scale && c < cols) v = v * k_scale[c];
+    tile[i][threadIdx.x] = v;
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
-    const uint32_t r = r0 + i, c = c0 + threadIdx.x;
-    if (r >= rows || c >= cols) continue;
-    uint16_t p[3];
-    Split3(tile[threadIdx.x][i], p);
-    uint16_t* out = dst + static_cast<size_t>(r) * 6 * cols + c;
+  // Two neighbouring columns per thread: 4-byte stores, sixteen threads per row.
+  const uint32_t t = threadIdx.y * 32 + threadIdx.x, c2 = (t & 15) * 2;
+  for (uint32_t i = t >> 4; i < 32; i += blockDim.y * 2) {
+    const uint32_t r = r0 + i;
+    if (r >= rows) continue;
+    uint16_t lo[3], hi[3];
+    Split3(tile[c2][i], lo);
+    Split3(tile[c2 + 1][i], hi);
+    uint16_t* out = dst + static_cast<size_t>(r) * 3 * kp + c0 + c2;
 #pragma unroll
-    for (int s = 0; s < 6; ++s) out[static_cast<size_t>(s) * cols] = p[PieceOf(kSide, s)];
+    for (int p = 0; p < 3; ++p)
+      *reinterpret_cast<uint32_t*>(out + static_cast<size_t>(p) * kp) =
+          static_cast<uint32_t>(lo[p]) | (static_cast<uint32_t>(hi[p]) << 16);
   }
 }
 
 }  // namespace
 
-void SplitMatrix(const float* src, uint16_t* dst, size_t rows, size_t cols, bool transposed, int side,
+void SplitMatrix(const float* src, uint16_t* dst, size_t rows, size_t cols, bool transposed, const float* k_scale,
                  cudaStream_t s) {
   if (rows == 0 || cols == 0) return;
+  const uint32_t kp = static_cast<uint32_t>((cols + 63) / 64 * 64);
+  const uint32_t r = static_cast<uint32_t>(rows), c = static_cast<uint32_t>(cols);
   if (transposed) {
-    const dim3 grid(static_cast<unsigned>((rows + 31) / 32), static_cast<unsigned>((cols + 31) / 32));
-    const dim3 block(32, 8);
-    if (side == 0)
-      SplitMatrixTransposedKernel<0><<<grid, block, 0, s>>>(src, dst, static_cast<uint32_t>(rows),
-                                                            static_cast<uint32_t>(cols));
-    else
-      SplitMatrixTransposedKernel<1><<<grid, block, 0, s>>>(src, dst, static_cast<uint32_t>(rows),
-                                                            static_cast<uint32_t>(cols));
+    const dim3 grid((r + 31) / 32, kp / 32), block(32, 8);
+    SplitMatrixTransposedKernel<<<grid, block, 0, s>>>(src, dst, r, c, kp, k_scale);
     return;
   }
-  size_t blocks = (rows * (cols / 4) + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (side == 0)
-    SplitMatrixKernel<0><<<static_cast<unsigned>(blocks), 256, 0, s>>>(src, dst, static_cast<uint32_t>(rows),
-                                                                       static_cast<uint32_t>(cols));
-  else
-    SplitMatrixKernel<1><<<static_cast<unsigned>(blocks), 256, 0, s>>>(src, dst, static_cast<uint32_t>(rows),
-                                                                       static_cast<uint32_t>(cols));
+  size_t blocks = (rows * (kp / 8) + 255) / 256;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  const bool vec = cols % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  if (vec) SplitMatrixKernel<true><<<static_cast<unsigned>(blocks), 256, 0, s>>>(src, dst, r, c, kp, k_scale);
+  else SplitMatrixKernel<false><<<static_cast<unsigned>(blocks), 256, 0, s>>>(src, dst, r, c, kp, k_scale);
 }
 
 uint32_t LoraSplitColumns(uint32_t r) { return (6 * r + 63) / 64 * 64; }

@@ -250,12 +250,10 @@ bool LoraBackwardSupported(size_t M, size_t N, size_t K, size_t r);
 size_t LoraBackwardPartialFloats(size_t N, size_t K, size_t r);
 bool LoraBackward(const LoraBackwardArgs& args, cudaStream_t s);
 
-// A whole f32 matrix as its bf16 pieces, dst [rows][6 * cols] (six K segments of
-// `cols`): the operand layout that makes an f32 GEMM a bf16 tensor-core GEMM over
-// K' = 6 K (k_lora.cu).  side 0: the A operand's piece order; 1: the B operand's.
-// src is [rows][cols], or [cols][rows] when `transposed`.  cols % 4 == 0 and 16-byte
-// aligned pointers for the untransposed form.
-void SplitMatrix(const float* src, uint16_t* dst, size_t rows, size_t cols, bool transposed, int side,
+// A whole f32 matrix as its three bf16 pieces side by side along K, dst [rows][3 Kp] with Kp = cols rounded up to
+// 64 (zeros past cols): the operand of an f32-accurate tensor-core product (UmmaEpilogue::seg_blocks).  src is
+// [rows][cols], or [cols][rows] when `transposed`; k_scale (or null) multiplies column c by k_scale[c] first.
+void SplitMatrix(const float* src, uint16_t* dst, size_t rows, size_t cols, bool transposed, const float* k_scale,
                  cudaStream_t s);
 
 // ---- GEMM -------------------------------------------------------------------

@@ -180,14 +180,14 @@ __device__ __forceinline__ void UmmaBf16Pair(uint32_t tmem_d, uint64_t desc_a, u
       : "memory");
 }
 // One arrival on the barrier at this shared-memory offset in BOTH CTAs of the pair
-// once the MMAs issued so far are complete: one commit per CTA, each naming that
-// CTA's barrier by its shared::cluster address.
-__device__ __forceinline__ void UmmaCommitPair(uint64_t* bar) {
+// (cluster ranks even, even + 1) once the MMAs issued so far are complete: one commit
+// per CTA, each naming that CTA's barrier by its shared::cluster address.
+__device__ __forceinline__ void UmmaCommitPair(uint64_t* bar, uint32_t even) {
   const uint32_t local = SmemAddr(bar);
 #pragma unroll
   for (uint32_t rank = 0; rank < 2; ++rank)
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 ::"r"(MapToCta(local, rank))
+                 ::"r"(MapToCta(local, even + rank))
                  : "memory");
 }
 __device__ __forceinline__ void MbarArriveCluster(uint32_t bar_cluster_addr) {

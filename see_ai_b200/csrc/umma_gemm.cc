@@ -69,6 +69,10 @@ struct Impl {
   uint16_t* split_a = nullptr;
   uint16_t* split_b = nullptr;
   uint64_t split_a_capacity = 0, split_b_capacity = 0;   // elements
+  // What split_a holds: the pieces of the arena matrix at `off` (several products in a row read the same one);
+  // ended by any write into that range.
+  struct SplitTag { bool valid = false, transposed = false; uint64_t off = 0, M = 0, K = 0; const float* k_scale = nullptr; } split_tag;
+  uint32_t sms = 148;
   std::map<WeightKey, uint16_t*> split_weights;          // frozen B operands, once per binding
 };
 
@@ -83,6 +87,9 @@ std::string Init(Context* ctx, int device, k::DeviceStatus* status) {
     return "cuda: the driver does not provide cuTensorMapEncodeTiled (TMA descriptors)";
   }
   impl->encode = reinterpret_cast<EncodeTiledFn>(fn);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0)
+    impl->sms = static_cast<uint32_t>(sms);
   impl->status = status;
   ctx->impl = impl;
   return {};
@@ -107,6 +114,7 @@ void InvalidateAll(Context* ctx) {
   ctx->impl->split_weights.clear();
   for (auto& a : ctx->impl->acts) a.valid = false;
   for (auto& e : ctx->impl->packs) e.valid = false;
+  ctx->impl->split_tag.valid = false;
 }
 
 void InvalidateRange(Context* ctx, uint64_t off, uint64_t bytes) {
@@ -118,6 +126,8 @@ void InvalidateRange(Context* ctx, uint64_t off, uint64_t bytes) {
   }
   for (auto& e : ctx->impl->packs)
     if (e.valid && off < e.src_off + e.elems * 4 && e.src_off < off + bytes) e.valid = false;
+  auto& t = ctx->impl->split_tag;
+  if (t.valid && off < t.off + t.M * t.K * 4 && t.off < off + bytes) t.valid = false;
 }
 
 // Sizes every activation-copy slot for the largest relaxed GEMM of the range
@@ -247,6 +257,31 @@ std::string TryLoraBackward(Context* ctx, const k::LoraBackwardArgs& a, cudaStre
   return {};
 }
 
+static bool GemmShape(uint64_t M, uint64_t N, uint64_t K) {
+  return K % 8 == 0 && N % 4 == 0 && K >= 64 && N >= 16 && M >= 64 && M <= 0xFFFFFFFFull && N <= 0xFFFFFFFFull &&
+         K <= 0xFFFFFFFFull;
+}
+
+static bool LightEpilogue(const k::GemmArgs& a) {
+  return !a.addend && !a.bias && a.act == kActNone && a.fuse_mode == k::kFuseNone;
+}
+
+// The frozen weight as a K-major bf16 matrix [N][K], converted once per binding; with k_scale,
+// w[n][k] = bf16(W[n][k] * s[k]).  Null: no memory.
+static uint16_t* WeightCopy(Impl* impl, const k::GemmArgs& a, int b_space, uint64_t b_off, const float* k_scale,
+                            uint64_t scale_off, cudaStream_t stream, int* launches) {
+  const WeightKey key{b_space, b_off, a.N, a.K, !a.b_transposed, static_cast<int>(a.b_type), k_scale ? scale_off : ~0ull};
+  if (auto it = impl->weights.find(key); it != impl->weights.end()) return it->second;
+  void* p = nullptr;
+  if (cudaMalloc(&p, a.N * a.K * 2) != cudaSuccess) return nullptr;
+  uint16_t* w = static_cast<uint16_t*>(p);
+  k::WeightToBf16(a.B, a.b_type, w, static_cast<uint32_t>(a.N), static_cast<uint32_t>(a.K),
+                  /*transpose=*/!a.b_transposed, k_scale, stream);
+  ++*launches;
+  impl->weights.emplace(key, w);
+  return w;
+}
+
 std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_off,
                     uint64_t a_off, uint64_t a_scale_off, cudaStream_t stream, int* launches) {
   *launches = 0;
@@ -256,8 +291,7 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   // multiple of 4 (float4 stores), enough rows to fill a 128-row tile, no
   // transposed A, no accumulate form.  Anything else runs on the exact kernels.
   if (a.a_transposed || a.accumulate) return {};
-  if (a.K % 8 != 0 || a.N % 4 != 0 || a.K < 64 || a.N < 16 || a.M < 64) return {};
-  if (a.M > 0xFFFFFFFFull || a.N > 0xFFFFFFFFull || a.K > 0xFFFFFFFFull) return {};
+  if (!GemmShape(a.M, a.N, a.K)) return {};
   auto misaligned = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
   if (misaligned(a.C) || misaligned(a.addend) || misaligned(a.bias) || misaligned(a.b_col_scale))
     return {};   // the epilogue moves float4s
@@ -267,20 +301,8 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   // weight copy, w[n][k] = bf16(W[n][k] * s[k]), once per binding: the activation
   // copy is then plain bf16(A), which every producer can write without a table
   // look-up per element, and which any other consumer of the tensor can share.
-  const WeightKey key{b_space, b_off, a.N, a.K, !a.b_transposed, static_cast<int>(a.b_type),
-                      a.a_k_scale ? a_scale_off : ~0ull};
-  uint16_t* w = nullptr;
-  if (auto it = impl->weights.find(key); it != impl->weights.end()) {
-    w = it->second;
-  } else {
-    void* p = nullptr;
-    if (cudaMalloc(&p, a.N * a.K * 2) != cudaSuccess) return "tensor-core path: weight copy allocation failed";
-    w = static_cast<uint16_t*>(p);
-    k::WeightToBf16(a.B, a.b_type, w, static_cast<uint32_t>(a.N), static_cast<uint32_t>(a.K),
-                    /*transpose=*/!a.b_transposed, a.a_k_scale, stream);
-    ++*launches;
-    impl->weights.emplace(key, w);
-  }
+  uint16_t* w = WeightCopy(impl, a, b_space, b_off, a.a_k_scale, a_scale_off, stream, launches);
+  if (!w) return "tensor-core path: weight copy allocation failed";
 
   // ---- the activation, bf16 [M][K], reused while its arena range is unwritten ----
   ActCopy* slot = nullptr;
@@ -316,12 +338,15 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   slot->last_use = ++impl->tick;
 
   CUtensorMap map_a, map_b, aux_a, aux_b;
-  if (!EncodeBf16Map(impl, &map_a, slot->buf, a.M, a.K, k::umma_cfg::kBlockM) ||
-      !EncodeBf16Map(impl, &map_b, w, a.N, a.K, k::umma_cfg::kBlockN))
-    return "tensor-core path: cuTensorMapEncodeTiled refused the operand layout";
   const bool has_aux = a.aux_a && a.aux_b && a.aux_k >= 64 && a.aux_k % 64 == 0;
+  const uint32_t k_blocks = static_cast<uint32_t>((a.K + 63) / 64) + (has_aux ? a.aux_k / 64 : 0);
+  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks,
+                                                LightEpilogue(a), impl->sms);
+  if (!EncodeBf16Map(impl, &map_a, slot->buf, a.M, a.K, k::umma_cfg::kBlockM) ||
+      !EncodeBf16Map(impl, &map_b, w, a.N, a.K, plan.b_box))
+    return "tensor-core path: cuTensorMapEncodeTiled refused the operand layout";
   if (has_aux && (!EncodeBf16Map(impl, &aux_a, a.aux_a, a.M, a.aux_k, k::umma_cfg::kBlockM) ||
-                  !EncodeBf16Map(impl, &aux_b, a.aux_b, a.N, a.aux_k, k::umma_cfg::kBlockN)))
+                  !EncodeBf16Map(impl, &aux_b, a.aux_b, a.N, a.aux_k, plan.b_box)))
     return "tensor-core path: cuTensorMapEncodeTiled refused the low-rank operand layout";
 
   k::UmmaEpilogue ep{};
@@ -345,7 +370,7 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   ep.addend_last = a.addend_after_bias ? 1 : 0;
   ep.aux_k_blocks = has_aux ? a.aux_k / 64 : 0;
   if (impl->prof_before) cudaEventRecord(impl->prof_before, stream);
-  if (cudaError_t e = k::UmmaGemmLaunch(map_a, map_b, ep, stream, has_aux ? &aux_a : nullptr,
+  if (cudaError_t e = k::UmmaGemmLaunch(plan, map_a, map_b, ep, stream, has_aux ? &aux_a : nullptr,
                                         has_aux ? &aux_b : nullptr);
       e != cudaSuccess)
     return std::string("tensor-core GEMM launch: ") + cudaGetErrorString(e);
@@ -358,13 +383,35 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   return {};
 }
 
-bool SplitGemmEligible(const k::GemmArgs& a) {
-  if (a.b_type != k::BType::kF32 || a.accumulate || a.b_col_scale || a.a_k_scale) return false;
-  if (a.M < 128 || a.N < 64 || a.K < 64 || (a.N & 3) != 0 || (a.K & 3) != 0) return false;
-  if (a.M * a.N * a.K < (1ull << 26)) return false;   // below ~0.1 GFLOP a launch is latency either way
-  if (a.M > 0x7FFFFFFFull || a.N > 0x7FFFFFFFull || 6 * a.K > 0x7FFFFFFFull) return false;
+namespace {
+
+// The reduction as segments of bf16 pieces, small products first because the tensor core truncates toward zero at
+// the accumulator's magnitude.  f32 times f32: a2 b0, a1 b1, a0 b2, a1 b0, a0 b1, a0 b0.  f32 times a weight that
+// is a bf16 value exactly (int8 levels, bf16): a2 b, a1 b, a0 b.
+constexpr uint32_t kSegF32 = 6, kSegAF32 = 0x001012, kSegBF32 = 0x010210;
+constexpr uint32_t kSegExact = 3, kSegAExact = 0x012, kSegBExact = 0;
+
+uint64_t PaddedK(uint64_t K) { return (K + 63) / 64 * 64; }
+uint64_t SplitThreshold(bool wide) { return wide ? 1ull << 24 : 1ull << 26; }
+
+bool SplitShape(uint64_t M, uint64_t N, uint64_t K, bool wide) {
+  if (M * N * K < SplitThreshold(wide)) return false;
+  if (M > 0x7FFFFFFFull || N > 0x7FFFFFFFull || 6 * PaddedK(K) > 0x7FFFFFFFull) return false;
+  // (A rank-r product, narrow, flat or short, belongs to the streaming kernels.)
+  if (wide) return M > 16 && N >= 32 && K >= 32;
+  return M >= 128 && N >= 64 && K >= 64 && (N & 3) == 0 && (K & 3) == 0;
+}
+
+}  // namespace
+
+bool SplitGemmEligible(const k::GemmArgs& a, bool wide) {
+  if (a.accumulate || !SplitShape(a.M, a.N, a.K, wide)) return false;
+  if (!wide && (a.b_type != k::BType::kF32 || a.b_col_scale || a.a_k_scale)) return false;
+  // (a TMA operand's rows start on 16-byte boundaries: an exact weight is read where its copy lies, unpadded)
+  if (a.b_type != k::BType::kF32 && (a.K & 7) != 0) return false;
   auto misaligned = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
-  return !(misaligned(a.A) || misaligned(a.B) || misaligned(a.C) || misaligned(a.addend) || misaligned(a.bias));
+  return !(misaligned(a.A) || misaligned(a.B) || misaligned(a.C) || misaligned(a.addend) || misaligned(a.bias) ||
+           misaligned(a.b_col_scale) || misaligned(a.a_k_scale));
 }
 
 static bool GrowSplit(uint16_t** buf, uint64_t* cap, uint64_t need, cudaStream_t stream, bool whole_device = false) {
@@ -381,71 +428,99 @@ static bool GrowSplit(uint16_t** buf, uint64_t* cap, uint64_t need, cudaStream_t
   return true;
 }
 
-void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size_t end) {
+void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size_t end, bool wide, bool relaxed_allowed) {
   Impl* impl = ctx->impl;
   if (!impl) return;
   uint64_t need_a = 0, need_b = 0;
   for (size_t i = begin; i < end; ++i) {
     const Instruction& ins = program[i];
-    if (ins.opcode != kGemmNN && ins.opcode != kGemmNT && ins.opcode != kGemmTN) continue;
+    switch (ins.opcode) {
+      case kGemmNN: case kGemmNT: case kGemmTN: break;
+      case kGemmNNQ8: case kGemmNTQ8: case kGemmNNBF16: case kGemmNTBF16: if (wide) break; [[fallthrough]];
+      default: continue;
+    }
     const uint64_t M = ins.out[0], N = ins.out[1], K = ins.out[2];
-    if (M < 128 || N < 64 || K < 64 || M * N * K < (1ull << 26)) continue;
-    need_a = std::max(need_a, M * 6 * K);
-    if (RefSpace(ins.in[1]) == kArena) need_b = std::max(need_b, N * 6 * K);
+    if (!SplitShape(M, N, K, wide)) continue;
+    if (relaxed_allowed && (ins.flags & kFlagRelaxed) && RefSpace(ins.in[1]) != kArena && ins.opcode != kGemmTN &&
+        GemmShape(M, N, K))
+      continue;   // runs on plain bf16 operands
+    need_a = std::max(need_a, M * 3 * PaddedK(K));
+    if (RefSpace(ins.in[1]) == kArena) need_b = std::max(need_b, N * 3 * PaddedK(K));
   }
+  if (need_a > impl->split_a_capacity) impl->split_tag.valid = false;
   GrowSplit(&impl->split_a, &impl->split_a_capacity, need_a, nullptr, true);
   GrowSplit(&impl->split_b, &impl->split_b_capacity, need_b, nullptr, true);
 }
 
-std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_off,
-                         cudaStream_t stream, int* launches) {
+std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_space, uint64_t a_off, int b_space,
+                         uint64_t b_off, cudaStream_t stream, int* launches) {
   *launches = 0;
   Impl* impl = ctx->impl;
-  if (!impl || !SplitGemmEligible(a)) return {};
-  const uint64_t K6 = 6 * a.K;
-  if (!GrowSplit(&impl->split_a, &impl->split_a_capacity, a.M * K6, stream))
+  if (!impl || !SplitGemmEligible(a, wide)) return {};
+  const bool exact_b = a.b_type != k::BType::kF32;
+  if (exact_b && b_space == 0) return {};
+  const uint64_t Kp = PaddedK(a.K);
+  if (a.M * 3 * Kp > impl->split_a_capacity) impl->split_tag.valid = false;
+  if (!GrowSplit(&impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream))
     return "tensor-core path: operand-piece allocation failed";
   // A: [M, K], or [K, M] for the transposed-A form.
-  k::SplitMatrix(a.A, impl->split_a, a.M, a.K, a.a_transposed, 0, stream);
-  ++*launches;
+  auto& tag = impl->split_tag;
+  if (!(tag.valid && a_space == 0 && tag.off == a_off && tag.M == a.M && tag.K == a.K && tag.transposed == a.a_transposed &&
+        tag.k_scale == a.a_k_scale)) {
+    k::SplitMatrix(a.A, impl->split_a, a.M, a.K, a.a_transposed, a.a_k_scale, stream);
+    ++*launches;
+    tag.valid = a_space == 0;
+    tag.off = a_off; tag.M = a.M; tag.K = a.K; tag.transposed = a.a_transposed; tag.k_scale = a.a_k_scale;
+  }
   // B: wanted as [N][K]; stored [N, K] (NT) or [K, N] (NN, TN).
   uint16_t* b = nullptr;
-  if (b_space != 0) {   // frozen: once per binding
+  if (exact_b) {
+    b = WeightCopy(impl, a, b_space, b_off, nullptr, ~0ull, stream, launches);
+    if (!b) return "tensor-core path: weight copy allocation failed";
+  } else if (b_space != 0) {   // frozen: once per binding
     const WeightKey key{b_space, b_off, a.N, a.K, !a.b_transposed, 100, ~0ull};
     if (auto it = impl->split_weights.find(key); it != impl->split_weights.end()) {
       b = it->second;
     } else {
       void* p = nullptr;
-      if (cudaMalloc(&p, a.N * K6 * 2) != cudaSuccess) return "tensor-core path: weight-piece allocation failed";
+      if (cudaMalloc(&p, a.N * 3 * Kp * 2) != cudaSuccess) return "tensor-core path: weight-piece allocation failed";
       b = static_cast<uint16_t*>(p);
-      k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, 1, stream);
+      k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);
       ++*launches;
       impl->split_weights.emplace(key, b);
     }
   } else {
-    if (!GrowSplit(&impl->split_b, &impl->split_b_capacity, a.N * K6, stream))
+    if (!GrowSplit(&impl->split_b, &impl->split_b_capacity, a.N * 3 * Kp, stream))
       return "tensor-core path: operand-piece allocation failed";
     b = impl->split_b;
-    k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, 1, stream);
+    k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);
     ++*launches;
   }
+  const uint32_t segments = exact_b ? kSegExact : kSegF32;
+  const uint32_t k_blocks = static_cast<uint32_t>(segments * (Kp / 64));
+  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks,
+                                                LightEpilogue(a), impl->sms);
   CUtensorMap map_a, map_b;
-  if (!EncodeBf16Map(impl, &map_a, impl->split_a, a.M, K6, k::umma_cfg::kBlockM) ||
-      !EncodeBf16Map(impl, &map_b, b, a.N, K6, k::umma_cfg::kBlockN))
+  // An exact weight is [N][K]: past K its last block reads zeros, and so do A's padding columns.
+  if (!EncodeBf16Map(impl, &map_a, impl->split_a, a.M, 3 * Kp, k::umma_cfg::kBlockM) ||
+      !EncodeBf16Map(impl, &map_b, b, a.N, exact_b ? a.K : 3 * Kp, plan.b_box))
     return "tensor-core path: cuTensorMapEncodeTiled refused the operand-piece layout";
   k::UmmaEpilogue ep{};
   ep.C = a.C;
   ep.addend = a.addend;
   ep.bias = a.bias;
-  ep.col_scale = nullptr;
+  ep.col_scale = a.b_col_scale;
   ep.alpha = a.alpha;   // (the exact kernels fold alpha into A or the finished dot; here it scales the tile)
   ep.act = static_cast<int>(a.act);
   ep.M = static_cast<uint32_t>(a.M);
   ep.N = static_cast<uint32_t>(a.N);
-  ep.K = static_cast<uint32_t>(K6);
+  ep.K = k_blocks * 64;
+  ep.seg_blocks = static_cast<uint32_t>(Kp / 64);
+  ep.seg_a = exact_b ? kSegAExact : kSegAF32;
+  ep.seg_b = exact_b ? kSegBExact : kSegBF32;
   ep.status = impl->status;
   if (impl->prof_before) cudaEventRecord(impl->prof_before, stream);
-  if (cudaError_t e = k::UmmaGemmLaunch(map_a, map_b, ep, stream); e != cudaSuccess)
+  if (cudaError_t e = k::UmmaGemmLaunch(plan, map_a, map_b, ep, stream); e != cudaSuccess)
     return std::string("tensor-core GEMM launch: ") + cudaGetErrorString(e);
   if (impl->prof_after) {
     cudaEventRecord(impl->prof_after, stream);

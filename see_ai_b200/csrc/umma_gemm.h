@@ -46,21 +46,25 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& args, int b_space, uint64_t
 // *launches == 0 with an empty return value: not applicable, use k::LoraBackward.
 std::string TryLoraBackward(Context* ctx, const k::LoraBackwardArgs& args, cudaStream_t stream, int* launches);
 
-// An EXACT f32 product on the tensor cores: both operands cut into three bf16
-// pieces, the six largest piece products summed over a K axis six times as long
-// (k::SplitMatrix), f32 accumulation in tensor memory.  The result is the f32
-// product to a few 2^-24 of sum|a_k b_k| — the accuracy the exact CUDA-core
-// kernels have against a float64 sum, not their bits — at a sixth of the bf16
-// tensor rate instead of the FP32 pipe's.  Takes NN, NT and TN forms with f32
-// operands in any address space; epilogue addend / bias / activation as usual.
-// *launches == 0 with an empty return value: outside the domain (small or odd
-// shapes, narrow outputs), use the exact kernels.
-bool SplitGemmEligible(const k::GemmArgs& args);
-std::string TrySplitGemm(Context* ctx, const k::GemmArgs& args, int b_space, uint64_t b_off,
-                         cudaStream_t stream, int* launches);
+// An EXACT product on the tensor cores: f32 operands cut into three bf16 pieces
+// (k::SplitMatrix), the six largest piece products summed in tensor memory in f32;
+// an int8 or bf16 weight is one piece as it is, three products.  The result is the
+// f32 product to a few 2^-24 of sum|a_k b_k| — the accuracy the exact CUDA-core
+// kernels have against a float64 sum, not their bits — at a sixth (a third) of the
+// bf16 tensor rate instead of the FP32 pipe's.  Epilogue scale / addend / bias /
+// activation as usual.  `wide` takes every shape and weight type worth a launch;
+// without it the domain is NN, NT and TN products of f32 operands of at least 2^26
+// multiply-adds with N and K multiples of 4.  The threshold of the wide domain,
+// 2^24: at 128 x 512 x 256 the split costs what the CUDA-core kernel costs.
+// *launches == 0 with an empty return value: outside the domain, use the exact kernels.
+bool SplitGemmEligible(const k::GemmArgs& args, bool wide);
+// a_space / b_space: 0 = arena, 1 = rodata, 2 = source model.
+std::string TrySplitGemm(Context* ctx, const k::GemmArgs& args, bool wide, int a_space, uint64_t a_off, int b_space,
+                         uint64_t b_off, cudaStream_t stream, int* launches);
 // Sizes the two operand buffers for the largest eligible product of a range
 // (called with the other per-range sizing, before any capture).
-void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size_t end);
+void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size_t end, bool wide,
+                    bool relaxed_allowed);
 
 // Producer-side conversion: the instruction that writes a tensor a relaxed GEMM
 // reads next can emit the bf16 copy itself (k::Shadow) and spare the GEMM's
