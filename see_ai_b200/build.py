@@ -36,6 +36,7 @@ CU_SOURCES = {
     "k_no_alloc.cu": ["-fmad=false"],
     "k_lora.cu": [],
     "k_gemm_skinny_fast.cu": [],
+    "k_gemm_fast.cu": [],
     "k_lora_mma.cu": [],
     "k_lora_umma.cu": [],
 }

@@ -1767,7 +1767,7 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
         pieces_made = adapter_fma_ && lf->down.flags == 0 && d.N == lf->r && k::LoraDownSupported(d.M, d.K, d.N) &&
                       k::LoraDown(d.A, static_cast<const float*>(d.B), d.C, d.M, d.K, d.N, d.alpha, stream_,
                                   d_lora_t_);
-        if (!pieces_made) k::GemmExact(d, stream_);
+        if (!pieces_made && !(adapter_fma_ && k::FastGemm(d, stream_))) k::GemmExact(d, stream_);
         ++counters_.kernel_launches;
         umma::InvalidateRange(&umma_->ctx, RefOffset(lf->down.in[2]), d.M * d.N * 4);
       }
@@ -1979,6 +1979,13 @@ Status CudaBackend::DispatchOptimizer(const Instruction& ins, const StepParams& 
     if (capturing_)
       return std::unexpected("cuda: step scalars must be uploaded before a range is captured");
     if (auto r = UploadStepScalars(params); !r) return r;
+  // Small and narrow products likewise, but for the rank-r expand product of many rows: that one is a stream, and a
+  // following add may ride it.
+  const bool expand = !a.a_transposed && a.K <= 16 && a.K % 4 == 0 && a.M >= 64 && a.N >= 64;
+  if (coherence_ == Coherence::kLazy && adapter_fma_ && !expand && !a.accumulate && k::FastGemm(a, stream_)) {
+    ++counters_.kernel_launches;
+    return {};
+  }
   }
   if (range_index_ < adam_group_of_.size() && adam_group_of_[range_index_] != -1) {
     const int32_t gi = adam_group_of_[range_index_];

@@ -317,6 +317,11 @@ size_t SplitKChunks(size_t M, size_t N, size_t K);
 // bit-identical to the CPU executor for f32 / int8 / bf16 weights.
 bool GemmExact(const GemmArgs& a, cudaStream_t s);
 
+// The same products for f32 weights where the bits are not observed: fused multiply-adds, the reduction cut over the
+// CTAs of a cluster and the warps of a CTA (k_gemm_fast.cu).  For shapes too small or too narrow for the tensor cores.
+// False (nothing launched): another weight type, a per-element scale, the accumulate form.
+bool FastGemm(const GemmArgs& a, cudaStream_t s);
+
 }  // namespace see::k
 
 #endif  // SEE_CUDA_KERNELS_H_
