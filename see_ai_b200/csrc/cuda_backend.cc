@@ -417,6 +417,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
   range_index_ = 0;
   lora_rows_tag_.valid = false;
   PlanAdamGroups(program, begin, std::min(end, program.size()));
+  PlanMergeRuns(program, begin, std::min(end, program.size()));
   PlanAttentionKeeps(program, begin, std::min(end, program.size()));
   auto plan_fusions = [&] {
     PlanShadows(program, begin, std::min(end, program.size()));
@@ -534,6 +535,8 @@ void CudaBackend::EndRange() {
   shadow_plan_.clear();
   adam_group_of_.clear();
   adam_groups_.clear();
+  merge_run_of_.clear();
+  merge_runs_.clear();
 }
 
 // Consecutive AdamW instructions without a fused clip become one launch over a
@@ -602,6 +605,79 @@ void CudaBackend::PlanAdamGroups(std::span<const Instruction> program, size_t be
   // The previous range's launches may still be reading the table.
   cudaStreamSynchronize(stream_);
   cudaMemcpy(d_adam_table_, table.data(), table.size() * sizeof(k::AdamTensor), cudaMemcpyHostToDevice);
+}
+
+void CudaBackend::PlanMergeRuns(std::span<const Instruction> program, size_t begin, size_t end) {
+  merge_run_of_.assign(end > begin ? end - begin : 0, -1);
+  merge_runs_.clear();
+  merge_program_.clear();
+  if (coherence_ == Coherence::kStrict || !epilogue_fusion_ || end <= begin) return;
+  auto is_pair = [&](size_t i) {
+    if (i + 1 >= end || program[i].opcode != kFill || program[i + 1].opcode != kGemmAccNN) return false;
+    const Instruction &f = program[i], &g = program[i + 1];
+    Extents ext;
+    if (!DescribeInstruction(f, arena_bytes_, rodata_bytes_, source_bytes_, &ext).empty() ||
+        !DescribeInstruction(g, arena_bytes_, rodata_bytes_, source_bytes_, &ext).empty())
+      return false;
+    const uint64_t K = g.out[2];
+    auto aligned = [&](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    return static_cast<uint32_t>(f.in[1]) == 0 && g.in[2] == f.in[0] && g.out[0] * g.out[1] == f.out[0] && f.out[0] > 0 &&
+           (K == 4 || K == 8 || K == 12 || K == 16) && g.out[1] % 4 == 0 && g.out[0] < (1u << 30) && g.out[1] < (1u << 30) &&
+           aligned(Rd(g.in[1])) && aligned(Wr(g.in[2]));
+  };
+  // Every delta of a run is written at once: none may be read, or written again, by another of the run.
+  auto hits = [](uint64_t a, uint64_t a_bytes, uint64_t b, uint64_t b_bytes) { return a < b + b_bytes && b < a + a_bytes; };
+  auto apart = [&](const Instruction& x, const Instruction& y) {
+    const uint64_t c = RefOffset(x.in[2]), c_bytes = x.out[0] * x.out[1] * 4;
+    for (int j = 0; j < 3; ++j) {
+      if (j < 2 && RefSpace(y.in[j]) != kArena) continue;
+      const uint64_t elems = j == 0 ? y.out[0] * y.out[2] : (j == 1 ? y.out[2] * y.out[1] : y.out[0] * y.out[1]);
+      if (hits(c, c_bytes, RefOffset(y.in[j]), elems * 4)) return false;
+    }
+    return true;
+  };
+  for (size_t i = begin; i < end;) {
+    if (!is_pair(i)) { ++i; continue; }
+    MergeRun run{i - begin, 0};
+    size_t j = i;
+    for (; run.pairs < k::kMergeEntries && is_pair(j) && program[j + 1].out[2] == program[i + 1].out[2]; j += 2) {
+      bool ok = true;
+      for (size_t q = i; q < j && ok; q += 2) ok = apart(program[q + 1], program[j + 1]) && apart(program[j + 1], program[q + 1]);
+      for (int o = 0; o < 2 && ok; ++o) {   // (nor may a delta overlap its own factors)
+        const Instruction& g = program[j + 1];
+        if (RefSpace(g.in[o]) == kArena)
+          ok = !hits(RefOffset(g.in[2]), g.out[0] * g.out[1] * 4, RefOffset(g.in[o]),
+                     (o == 0 ? g.out[0] * g.out[2] : g.out[2] * g.out[1]) * 4);
+      }
+      if (!ok) break;
+      ++run.pairs;
+    }
+    if (run.pairs == 0) { ++i; continue; }
+    merge_run_of_[run.first] = static_cast<int32_t>(merge_runs_.size());
+    for (size_t q = run.first + 1; q < run.first + 2 * run.pairs; ++q) merge_run_of_[q] = -2;
+    merge_program_.insert(merge_program_.end(), program.begin() + static_cast<long>(i), program.begin() + static_cast<long>(j));
+    merge_runs_.push_back(run);
+    i = j;
+  }
+}
+
+Status CudaBackend::DispatchMergeRun(const MergeRun& run) {
+  size_t at = 0;   // the run's place in merge_program_
+  for (const MergeRun& r : merge_runs_) {
+    if (r.first == run.first) break;
+    at += 2 * r.pairs;
+  }
+  k::MergeTable table{};
+  for (size_t i = 0; i < run.pairs; ++i) {
+    const Instruction& g = merge_program_[at + 2 * i + 1];
+    table.entry[i] = {Rd(g.in[0]), Rd(g.in[1]), Wr(g.in[2]), static_cast<uint32_t>(g.out[0]), static_cast<uint32_t>(g.out[1]),
+                      BitsToF32(g.in[3])};
+  }
+  k::MergeDeltas(table, static_cast<int>(run.pairs), static_cast<uint32_t>(merge_program_[at + 1].out[2]), merge_tally_, stream_);
+  if (merge_tally_) merge_counted_ += run.pairs;
+  ++counters_.kernel_launches;
+  counters_.fused_dispatches += 2 * run.pairs - 1;
+  return {};
 }
 
 namespace {
@@ -1903,6 +1979,13 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
       return {};
     }
   }
+  // Small and narrow products likewise, but for the rank-r expand product of many rows: that one is a stream, and a
+  // following add may ride it.
+  const bool expand = !a.a_transposed && a.K <= 16 && a.K % 4 == 0 && a.M >= 64 && a.N >= 64;
+  if (coherence_ == Coherence::kLazy && adapter_fma_ && !expand && !a.accumulate && k::FastGemm(a, stream_)) {
+    ++counters_.kernel_launches;
+    return {};
+  }
   // The split-K scratch is sized per range (BeginRange); an instruction executed
   // outside any range simply runs unsplit.
   a.split_scratch = d_split_;
@@ -1979,13 +2062,6 @@ Status CudaBackend::DispatchOptimizer(const Instruction& ins, const StepParams& 
     if (capturing_)
       return std::unexpected("cuda: step scalars must be uploaded before a range is captured");
     if (auto r = UploadStepScalars(params); !r) return r;
-  // Small and narrow products likewise, but for the rank-r expand product of many rows: that one is a stream, and a
-  // following add may ride it.
-  const bool expand = !a.a_transposed && a.K <= 16 && a.K % 4 == 0 && a.M >= 64 && a.N >= 64;
-  if (coherence_ == Coherence::kLazy && adapter_fma_ && !expand && !a.accumulate && k::FastGemm(a, stream_)) {
-    ++counters_.kernel_launches;
-    return {};
-  }
   }
   if (range_index_ < adam_group_of_.size() && adam_group_of_[range_index_] != -1) {
     const int32_t gi = adam_group_of_[range_index_];
@@ -2038,6 +2114,10 @@ Status CudaBackend::DispatchOptimizer(const Instruction& ins, const StepParams& 
 Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, const Extents&) {
   cudaStream_t s = stream_;
   auto launched = [&](int n = 1) { counters_.kernel_launches += n; };
+  if (range_index_ < merge_run_of_.size() && merge_run_of_[range_index_] != -1) {
+    if (merge_run_of_[range_index_] == -2) return {};   // done by the run's first instruction
+    return DispatchMergeRun(merge_runs_[static_cast<size_t>(merge_run_of_[range_index_])]);
+  }
   switch (static_cast<Op>(ins.opcode)) {
     case kNop: break;
     case kGemmNN: case kGemmNT: case kGemmTN: case kGemmAccNN: case kGemmNNQ8: case kGemmNTQ8:

@@ -171,6 +171,11 @@ class CudaBackend {
   // arithmetic bit for bit (reference: compiler/backend/allocation/arena_binder.cc:129-190).
   Status QuantizeColumns(const float* w, uint64_t K, uint64_t N, int8_t* levels, float* scales);
 
+  // Merge deltas launched as a run add their non-finite results to *tally (device memory) from now on; null: they do
+  // not.  merge_counted(): how many deltas have been counted that way since the last call of this.
+  void SetMergeTally(unsigned long long* tally) { merge_tally_ = tally; merge_counted_ = 0; }
+  uint64_t merge_counted() const { return merge_counted_; }
+
   // Profile mode: every instruction is bracketed by CUDA events on the stream.
   void SetProfiling(bool on);
   std::vector<ProfileRecord> TakeProfile();
@@ -268,6 +273,18 @@ class CudaBackend {
   std::vector<AdamGroup> adam_groups_;
   k::AdamTensor* d_adam_table_ = nullptr;
   size_t adam_table_capacity_ = 0;
+
+  // A run of merge deltas (kFill with zero, kGemmAccNN over exactly that tensor), issued as one launch from the first
+  // kFill (engine / lazy coherence only): the filled tensor never goes through memory.  `first` is a range position;
+  // pairs follow one another from there.
+  struct MergeRun { size_t first = 0, pairs = 0; };
+  void PlanMergeRuns(std::span<const Instruction> program, size_t begin, size_t end);
+  Status DispatchMergeRun(const MergeRun& run);
+  std::vector<int32_t> merge_run_of_;    // per range position: -1 none, -2 member, else run index
+  std::vector<MergeRun> merge_runs_;
+  std::vector<Instruction> merge_program_;   // the instructions of all runs, kFill / kGemmAccNN pairs in order
+  unsigned long long* merge_tally_ = nullptr;
+  uint64_t merge_counted_ = 0;
 
   // A relaxed GEMM followed by the kAddBias that consumes its output, when the
   // un-biased product is provably dead afterwards: the GEMM's epilogue adds the
@@ -440,6 +457,10 @@ class CudaBackend {
   float* d_lora_partials_ = nullptr;
   uint64_t lora_partials_capacity_ = 0;   // floats
   int split_gemm_mode_ = -1;
+  // In lazy coherence every exact product above 2^24 multiply-adds, any width and weight type; asked for
+  // explicitly (mode 1), or with adapter products in the CPU's arithmetic, the documented domain of
+  // see_cuda_set_split_gemm alone.
+  bool SplitGemmWide() const { return split_gemm_mode_ < 0 && adapter_fma_; }
   bool SplitGemmOn() const { return split_gemm_mode_ > 0 || (split_gemm_mode_ < 0 && coherence_ == Coherence::kLazy); }
   Status PrepareLoraFolds(const Instruction* program, size_t begin, uint64_t max_rows);
   void FreeLoraRanges();
@@ -453,7 +474,3 @@ class CudaBackend {
 }  // namespace see
 
 #endif  // SEE_CUDA_BACKEND_H_
-  // In lazy coherence every exact product above 2^24 multiply-adds, any width and weight type; asked for
-  // explicitly (mode 1), or with adapter products in the CPU's arithmetic, the documented domain of
-  // see_cuda_set_split_gemm alone.
-  bool SplitGemmWide() const { return split_gemm_mode_ < 0 && adapter_fma_; }

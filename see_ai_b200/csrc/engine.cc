@@ -96,7 +96,7 @@ std::expected<std::unique_ptr<UpdateEngine>, std::string> UpdateEngine::Create(i
 }
 
 void UpdateEngine::DropGraphs() {
-  for (GraphSlot* g : {&g_fwdbwd_, &g_opt_, &g_eval_, &g_step_}) {
+  for (GraphSlot* g : {&g_fwdbwd_, &g_opt_, &g_eval_, &g_step_, &g_merge_}) {
     if (g->exec) cudaGraphExecDestroy(g->exec);
     g->exec = nullptr;
     g->runs = 0;
@@ -204,6 +204,16 @@ Status UpdateEngine::LoadFromMemory(const uint8_t* plan, uint64_t size) {
   step_prog_ = std::move(step);
   emit_.resize(h.emit_count);
   if (h.emit_count) std::memcpy(emit_.data(), plan + h.emit_table_offset, h.emit_count * sizeof(EmitEntry));
+  {   // the deltas the merge program accumulates, against the emit table
+    std::vector<std::pair<uint64_t, uint64_t>> made, leave;
+    for (const Instruction& ins : merge_)
+      if (ins.opcode == kGemmAccNN) made.push_back({RefOffset(ins.in[2]), ins.out[0] * ins.out[1] * 4});
+    for (const EmitEntry& e : emit_) leave.push_back({e.arena_offset, e.byte_size});
+    std::sort(made.begin(), made.end());
+    std::sort(leave.begin(), leave.end());
+    emits_are_merge_deltas_ = !made.empty() && made == leave;
+    merge_counts_ = false;
+  }
   phases_ = ScanPhases(train_);
   grad_off_ = g_lo == ~0ull ? 0 : g_lo;
   grad_bytes_ = g_lo == ~0ull ? 0 : g_hi - g_lo;
@@ -544,14 +554,23 @@ Status UpdateEngine::Evaluate(EvalResult* out, uint64_t real_rows) {
 }
 
 Status UpdateEngine::RunMerge(bool* all_finite) {
-  if (auto r = RunRange(merge_, 0, merge_.size(), nullptr, nullptr); !r) return r;
-  cudaStream_t s = backend_->stream();
-  cudaMemsetAsync(d_tally_, 0, 4 * sizeof(unsigned long long), s);
-  for (const EmitEntry& e : emit_) {
+  if (!loaded_) return std::unexpected("engine: no plan is loaded");
+  for (const EmitEntry& e : emit_)
     if (e.arena_offset > header_.arena_size || e.byte_size > header_.arena_size - e.arena_offset)
       return std::unexpected("engine: an emit entry lies outside the arena");
-    k::CountNonFinite(reinterpret_cast<const float*>(backend_->device_arena() + e.arena_offset),
-                      e.byte_size / 4, d_tally_, s);
+  cudaStream_t s = backend_->stream();
+  cudaMemsetAsync(d_tally_, 0, 4 * sizeof(unsigned long long), s);
+  // Where the deltas that leave are exactly the ones the merge program makes, its kernels count the non-finite values
+  // as they write them (a replay counts as its capture did).
+  const bool replay = use_graphs_ && g_merge_.exec;
+  if (!replay) backend_->SetMergeTally(emits_are_merge_deltas_ ? d_tally_ + 2 : nullptr);
+  if (auto r = RunRange(merge_, 0, merge_.size(), &g_merge_, nullptr); !r) return r;
+  if (!replay) merge_counts_ = emits_are_merge_deltas_ && backend_->merge_counted() == emit_.size();
+  if (!merge_counts_) {
+    cudaMemsetAsync(d_tally_, 0, 4 * sizeof(unsigned long long), s);
+    for (const EmitEntry& e : emit_)
+      k::CountNonFinite(reinterpret_cast<const float*>(backend_->device_arena() + e.arena_offset), e.byte_size / 4,
+                        d_tally_, s);
   }
   unsigned long long tally[4] = {0, 0, 0, 0};
   if (auto e = cudaMemcpyAsync(tally, d_tally_, sizeof(tally), cudaMemcpyDeviceToHost, s); e != cudaSuccess)

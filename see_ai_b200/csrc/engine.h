@@ -154,7 +154,9 @@ class UpdateEngine {
   uint64_t step_ = 0, horizon_ = 0;
   uint64_t grad_off_ = 0, grad_bytes_ = 0;
   bool use_graphs_ = false, phase_timing_ = false;
-  GraphSlot g_fwdbwd_, g_opt_, g_eval_, g_step_;
+  bool emits_are_merge_deltas_ = false;   // the emit table lists exactly the merge program's deltas
+  bool merge_counts_ = false;             // ... and the merge program's kernels count their non-finite values
+  GraphSlot g_fwdbwd_, g_opt_, g_eval_, g_step_, g_merge_;
   uint8_t* pinned_ = nullptr;        // staging double buffer
   uint64_t pinned_bytes_ = 0;
   int pinned_slot_ = 0;

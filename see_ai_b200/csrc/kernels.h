@@ -317,6 +317,18 @@ size_t SplitKChunks(size_t M, size_t N, size_t K);
 // bit-identical to the CPU executor for f32 / int8 / bf16 weights.
 bool GemmExact(const GemmArgs& a, cudaStream_t s);
 
+// Several deltas C = alpha A B (from zero, in the exact quad order) of one rank K in {4, 8, 12, 16} as one launch:
+// A [M, K], B [K, N], N % 4 == 0, 16-byte aligned B and C.  `nonfinite` (or null) += the results that are not finite.
+// The table travels as a kernel parameter.
+struct MergeEntry {
+  const float* A; const float* B; float* C;
+  uint32_t M, N;
+  float alpha;
+};
+constexpr int kMergeEntries = 96;
+struct MergeTable { MergeEntry entry[kMergeEntries]; };
+void MergeDeltas(const MergeTable& table, int count, uint32_t K, unsigned long long* nonfinite, cudaStream_t s);
+
 // The same products for f32 weights where the bits are not observed: fused multiply-adds, the reduction cut over the
 // CTAs of a cluster and the warps of a CTA (k_gemm_fast.cu).  For shapes too small or too narrow for the tensor cores.
 // False (nothing launched): another weight type, a per-element scale, the accumulate form.
