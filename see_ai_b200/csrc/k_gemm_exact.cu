@@ -18,7 +18,8 @@
 // parity anchor and the path for the rank-r adapter products, whose outputs are
 // 8-16 wide (or tall): the block tile comes in three shapes (64x64, 256x16,
 // 16x256 for the quad order; 64x32, 128x16, 16x128 for the lane order) picked
-// from the output shape, so a skinny product wastes no lanes.  A tile shape
+// from the output shape, so a skinny product wastes no lanes, and a flat form
+// (GemmFlatKernel) for outputs of too few tiles.  A tile shape
 // changes which thread owns an element, never the element's arithmetic.
 // Large frozen-weight products carrying the relaxed permission go to the
 // tensor cores instead.
@@ -367,11 +368,163 @@ __global__ void __launch_bounds__(kThreads) MergeDeltasKernel(const __grid_const
   if ((threadIdx.x & 31) == 0 && bad) atomicAdd(nonfinite, bad);
 }
 
+// ---- both orders, few outputs --------------------------------------------------------------
+// With fewer 64 x 64 (or skinny) tiles than SMs the kernels above are a serial chain of global loads: K / 16 steps of
+// about 1.4 us in one or two blocks.  Here a block owns 16 R x 16 R outputs, R x R per thread, so that there are blocks
+// to go round, and takes K 128 at a time with the next 128 already on their way in registers while these are
+// multiplied.  The same operations per output in the same order (57 x 8 x 784: 81.5 -> 5 us; 57 x 128 x 784: 76 -> 6 us).
+constexpr int kFlatK = 128;
+template <bool TA, bool TB, typename BT, int R>
+struct FlatLoader {
+  static constexpr int T = 16 * R, kPer = T * kFlatK / kThreads;   // elements per thread and operand
+  float a[kPer], b[kPer];
+  // Which (row, k) element i of this thread is: lanes along the operand's contiguous axis.
+  static __device__ __forceinline__ void At(int i, bool k_contiguous, int* row, int* k) {
+    const int idx = static_cast<int>(threadIdx.x) + i * kThreads;
+    if (k_contiguous) { *row = idx / kFlatK; *k = idx % kFlatK; }
+    else { *row = idx % T; *k = idx / T; }
+  }
+  __device__ __forceinline__ void Load(const Params& p, size_t m0, size_t n0, size_t k0) {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      int r, k;
+      At(i, !TA, &r, &k);
+      a[i] = LoadA<TA>(p, m0 + r, k0 + k);
+      if (p.a_k_scale && k0 + k < p.K) a[i] = a[i] * p.a_k_scale[k0 + k];
+      At(i, TB, &r, &k);
+      b[i] = LoadB<TB, BT>(p, k0 + k, n0 + r);
+      if (p.b_col_scale && n0 + r < p.N) b[i] = b[i] * p.b_col_scale[n0 + r];
+    }
+  }
+  // As [row][k] (a row's quads are 16-byte reads), Bs [row][k] likewise.
+  __device__ __forceinline__ void Store(float (*As)[kFlatK + 4], float (*Bs)[kFlatK + 4], float alpha) {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      int r, k;
+      At(i, !TA, &r, &k);
+      As[r][k] = alpha * a[i];
+      At(i, TB, &r, &k);
+      Bs[r][k] = b[i];
+    }
+  }
+};
+
+// Lane order when kLane, quad order otherwise.
+template <bool kLane, bool TA, bool TB, typename BT, int R>
+__global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
+  constexpr int T = 16 * R;
+  __shared__ __align__(16) float As[T][kFlatK + 4];
+  __shared__ __align__(16) float Bs[T][kFlatK + 4];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // outputs (ty + 16 i, tx + 16 j)
+  const size_t m0 = static_cast<size_t>(blockIdx.y) * T, n0 = static_cast<size_t>(blockIdx.x) * T;
+  float c[R][R][kLane ? 8 : 1];
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+#pragma unroll
+      for (int l = 0; l < (kLane ? 8 : 1); ++l) c[i][j][l] = 0.0f;
+      const size_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      if (!kLane && p.accumulate && m < p.M && n < p.N) c[i][j][0] = p.C[m * p.N + n];
+    }
+  const float alpha_a = kLane ? 1.0f : p.alpha;   // (x * 1 == x)
+  FlatLoader<TA, TB, BT, R> next;
+  next.Load(p, m0, n0, 0);
+  for (size_t k0 = 0; k0 < p.K; k0 += kFlatK) {
+    next.Store(As, Bs, alpha_a);
+    __syncthreads();
+    if (k0 + kFlatK < p.K) next.Load(p, m0, n0, k0 + kFlatK);
+    const int kmax = p.K - k0 < static_cast<size_t>(kFlatK) ? static_cast<int>(p.K - k0) : kFlatK;
+    int k = 0;
+    for (; k + 4 <= kmax; k += 4) {
+      float4 a[R], b[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4*>(&As[ty + 16 * i][k]);
+#pragma unroll
+      for (int j = 0; j < R; ++j) b[j] = *reinterpret_cast<const float4*>(&Bs[tx + 16 * j][k]);
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          if (kLane) {
+            // k0 and k are multiples of 4: the four products go to lanes 0-3 or 4-7.
+            float* l = c[i][j];
+            if ((k & 4) == 0) {
+              l[0] = l[0] + a[i].x * b[j].x; l[1] = l[1] + a[i].y * b[j].y;
+              l[2] = l[2] + a[i].z * b[j].z; l[3] = l[3] + a[i].w * b[j].w;
+            } else {
+              l[4 % (kLane ? 8 : 1)] = l[4 % (kLane ? 8 : 1)] + a[i].x * b[j].x;
+              l[5 % (kLane ? 8 : 1)] = l[5 % (kLane ? 8 : 1)] + a[i].y * b[j].y;
+              l[6 % (kLane ? 8 : 1)] = l[6 % (kLane ? 8 : 1)] + a[i].z * b[j].z;
+              l[7 % (kLane ? 8 : 1)] = l[7 % (kLane ? 8 : 1)] + a[i].w * b[j].w;
+            }
+          } else {
+            float t = a[i].x * b[j].x;
+            t = t + a[i].y * b[j].y;
+            t = t + a[i].z * b[j].z;
+            t = t + a[i].w * b[j].w;
+            c[i][j][0] = c[i][j][0] + t;
+          }
+        }
+    }
+    for (; k < kmax; ++k)   // the K % 4 tail, one term at a time
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          const float x = As[ty + 16 * i][k] * Bs[tx + 16 * j][k];
+#pragma unroll
+          for (int l = 0; l < (kLane ? 8 : 1); ++l)
+            if (!kLane || l == (k & 7)) c[i][j][l] = c[i][j][l] + x;
+        }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const size_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      if (m >= p.M || n >= p.N) continue;
+      float v = c[i][j][0];
+      if (kLane) {
+#pragma unroll
+        for (int l = 1; l < (kLane ? 8 : 1); ++l) v = v + c[i][j][l];
+        v = p.alpha * v;
+      }
+      if (p.addend) v = p.addend[m * p.N + n] + v;
+      if (p.bias) v = v + p.bias[n];
+      p.C[m * p.N + n] = ApplyAct(v, p.act);
+    }
+}
+
 unsigned Blocks(size_t extent, size_t tile) { return static_cast<unsigned>((extent + tile - 1) / tile); }
+
+size_t QuadTiles(size_t M, size_t N) {
+  if (N <= 16) return static_cast<size_t>(Blocks(M, 256)) * Blocks(N, 16);
+  if (M <= 16) return static_cast<size_t>(Blocks(N, 256)) * Blocks(M, 16);
+  return static_cast<size_t>(Blocks(M, 64)) * Blocks(N, 64);
+}
+size_t LaneTiles(size_t M, size_t N) {
+  if (N <= 16) return static_cast<size_t>(Blocks(M, 128)) * Blocks(N, 16);
+  if (M <= 16) return static_cast<size_t>(Blocks(N, 128)) * Blocks(M, 16);
+  return static_cast<size_t>(Blocks(M, 64)) * Blocks(N, 32);
+}
+
+// The flat kernel where the tile kernels would leave SMs idle: 32 x 32 outputs per block if that still makes a block
+// per SM, else 16 x 16.
+template <bool kLane, bool TA, bool TB, typename BT>
+void LaunchFlat(const Params& p, cudaStream_t s) {
+  if (static_cast<size_t>(Blocks(p.M, 32)) * Blocks(p.N, 32) >= 148)
+    GemmFlatKernel<kLane, TA, TB, BT, 2><<<dim3(Blocks(p.N, 32), Blocks(p.M, 32)), kThreads, 0, s>>>(p);
+  else
+    GemmFlatKernel<kLane, TA, TB, BT, 1><<<dim3(Blocks(p.N, 16), Blocks(p.M, 16)), kThreads, 0, s>>>(p);
+}
 
 template <bool TA, typename BT>
 void LaunchQuad(const Params& p, unsigned z, cudaStream_t s) {
-  if (p.N <= 16) {
+  if (z == 1 && !p.partials && QuadTiles(p.M, p.N) < 148) {
+    LaunchFlat<false, TA, false, BT>(p, s);
+  } else if (p.N <= 16) {
     GemmQuadKernel<TA, BT, 256, 16><<<dim3(Blocks(p.N, 16), Blocks(p.M, 256), z), kThreads, 0, s>>>(p);
   } else if (p.M <= 16) {
     GemmQuadKernel<TA, BT, 16, 256><<<dim3(Blocks(p.N, 256), Blocks(p.M, 16), z), kThreads, 0, s>>>(p);
@@ -382,19 +535,15 @@ void LaunchQuad(const Params& p, unsigned z, cudaStream_t s) {
 
 template <typename BT>
 void LaunchLane(const Params& p, cudaStream_t s) {
-  if (p.N <= 16) {
+  if (LaneTiles(p.M, p.N) < 148) {
+    LaunchFlat<true, false, true, BT>(p, s);
+  } else if (p.N <= 16) {
     GemmLaneKernel<BT, 128, 16><<<dim3(Blocks(p.N, 16), Blocks(p.M, 128)), kThreads, 0, s>>>(p);
   } else if (p.M <= 16) {
     GemmLaneKernel<BT, 16, 128><<<dim3(Blocks(p.N, 128), Blocks(p.M, 16)), kThreads, 0, s>>>(p);
   } else {
     GemmLaneKernel<BT, 64, 32><<<dim3(Blocks(p.N, 32), Blocks(p.M, 64)), kThreads, 0, s>>>(p);
   }
-}
-
-size_t QuadTiles(size_t M, size_t N) {
-  if (N <= 16) return static_cast<size_t>(Blocks(M, 256)) * Blocks(N, 16);
-  if (M <= 16) return static_cast<size_t>(Blocks(N, 256)) * Blocks(M, 16);
-  return static_cast<size_t>(Blocks(M, 64)) * Blocks(N, 64);
 }
 
 }  // namespace
