@@ -214,6 +214,11 @@ int see_engine_train_optimizer(see_engine* h);
 int see_engine_step_program(see_engine* h);
 /* LossValue — reference: update_engine.cc:366-368.  Also surfaces a refusal. */
 int see_engine_read_loss(see_engine* h, float* loss);
+/* One optimizer step of a plan without gradient accumulation: see_engine_stage_batch,
+ * see_engine_train_forward_backward(1), see_engine_train_optimizer and
+ * see_engine_read_loss as one call. */
+int see_engine_train_step(see_engine* h, const void* input, uint64_t input_bytes, const void* labels,
+                          uint64_t label_bytes, float* loss);
 /* Evaluate one staged batch: eval program, loss, and the accuracy tally
  * (rows judged, argmax hits; reference: update_engine.cc:432-580) on device. */
 int see_engine_evaluate(see_engine* h, float* loss, uint64_t* rows, uint64_t* correct);

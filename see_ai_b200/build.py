@@ -32,6 +32,7 @@ CU_SOURCES = {
     "k_gemm_skinny.cu": ["-fmad=false"],
     "k_gemm_umma.cu": ["-fmad=false"],
     "k_eval.cu": [],
+    "k_host.cu": [],
     "k_attn_umma.cu": [],
     "k_no_alloc.cu": ["-fmad=false"],
     "k_lora.cu": [],

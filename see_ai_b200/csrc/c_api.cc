@@ -284,6 +284,10 @@ int see_engine_train_forward_backward(see_engine* h, int advance_step) {
 }
 int see_engine_train_optimizer(see_engine* h) { return Done(h, h->engine->TrainOptimizer()); }
 int see_engine_step_program(see_engine* h) { return Done(h, h->engine->StepProgram()); }
+int see_engine_train_step(see_engine* h, const void* input, uint64_t input_bytes, const void* labels,
+                          uint64_t label_bytes, float* loss) {
+  return Done(h, h->engine->TrainStep(input, input_bytes, labels, label_bytes, loss));
+}
 int see_engine_read_loss(see_engine* h, float* loss) { return Done(h, h->engine->ReadLoss(loss)); }
 int see_engine_evaluate(see_engine* h, float* loss, uint64_t* rows, uint64_t* correct) {
   see::EvalResult r;

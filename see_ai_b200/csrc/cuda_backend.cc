@@ -10,8 +10,6 @@ namespace see {
 
 namespace {
 
-constexpr int kScalarSlots = 64;
-
 std::string CudaErr(cudaError_t e, const char* what) {
   return std::string("cuda: ") + what + ": " + cudaGetErrorString(e);
 }
@@ -78,15 +76,11 @@ Status CudaBackend::Init() {
   d_count_ = reinterpret_cast<unsigned long long*>(base + 192);
   d_scalars_ = reinterpret_cast<k::AdamScalars*>(base + 256);
   d_partials_ = reinterpret_cast<double*>(base + 4096);
-  if (auto r = Check(cudaMallocHost(reinterpret_cast<void**>(&h_scalars_),
-                                    kScalarSlots * sizeof(k::AdamScalars)), "pinned scalars"); !r)
+  // One pinned block: what a flush publishes, then the staging of a strict flush's downloads.
+  if (auto r = Check(cudaMallocHost(reinterpret_cast<void**>(&h_published_), kPublishedBytes + kFlushStaging), "pinned status");
+      !r)
     return r;
-  if (auto r = Check(cudaMallocHost(reinterpret_cast<void**>(&h_status_), 64), "pinned status"); !r)
-    return r;
-  std::memset(h_status_, 0, 64);
-  scalar_done_.assign(kScalarSlots, nullptr);
-  for (auto& ev : scalar_done_)
-    if (auto r = Check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "scalar events"); !r) return r;
+  h_flush_ = reinterpret_cast<uint8_t*>(h_published_) + kPublishedBytes;
   umma_ = std::make_unique<UmmaState>();
   if (std::string e = umma::Init(&umma_->ctx, device_, d_status_); !e.empty()) return std::unexpected(e);
   return {};
@@ -97,7 +91,6 @@ CudaBackend::~CudaBackend() {
   if (stream_) cudaStreamSynchronize(stream_);
   for (auto& ev : events_) { cudaEventDestroy(ev.first); cudaEventDestroy(ev.second); }
   for (auto& ev : kernel_events_) { cudaEventDestroy(ev.first); cudaEventDestroy(ev.second); }
-  for (auto& ev : scalar_done_) if (ev) cudaEventDestroy(ev);
   if (umma_) umma::Destroy(&umma_->ctx);
   cudaFree(d_arena_);
   cudaFree(d_rodata_);
@@ -112,8 +105,7 @@ CudaBackend::~CudaBackend() {
   cudaFree(d_lora_t_);
   for (float* p : attn_keep_pool_) cudaFree(p);
   cudaFree(d_lora_partials_);
-  if (h_scalars_) cudaFreeHost(h_scalars_);
-  if (h_status_) cudaFreeHost(h_status_);
+  if (h_published_) cudaFreeHost(h_published_);
   if (own_stream_ && stream_) cudaStreamDestroy(stream_);
 }
 
@@ -231,6 +223,22 @@ Status CudaBackend::WriteArena(uint64_t off, uint64_t bytes, const void* src) {
     return r;
   counters_.h2d_bytes += bytes;
   umma::InvalidateRange(&umma_->ctx, off, bytes);
+  return {};
+}
+
+Status CudaBackend::WriteArenaPinned(uint64_t off0, uint64_t bytes0, const void* src0, uint64_t off1, uint64_t bytes1,
+                                     const void* src1) {
+  if (!d_arena_) return std::unexpected("cuda: nothing is bound");
+  for (const auto& [off, bytes] : {std::pair{off0, bytes0}, std::pair{off1, bytes1}})
+    if (bytes && (off > arena_bytes_ || bytes > arena_bytes_ - off))
+      return std::unexpected("cuda: write: range outside the arena");
+  cudaSetDevice(device_);
+  k::StageFromHost({d_arena_ + off0, src0, bytes0}, {d_arena_ + off1, src1, bytes1}, stream_);
+  if (auto r = Check(cudaPeekAtLastError(), "write"); !r) return r;
+  ++counters_.kernel_launches;
+  counters_.h2d_bytes += bytes0 + bytes1;
+  if (bytes0) umma::InvalidateRange(&umma_->ctx, off0, bytes0);
+  if (bytes1) umma::InvalidateRange(&umma_->ctx, off1, bytes1);
   return {};
 }
 
@@ -1587,35 +1595,56 @@ const k::Shadow* CudaBackend::ShadowFor(uint64_t out_ref, uint64_t elems) const 
   return &cur_shadow_;
 }
 
-Status CudaBackend::Flush() {
+Status CudaBackend::FlushWith(std::initializer_list<k::PublishItem> items, uint32_t* out) {
   if (!d_arena_) return {};
   cudaSetDevice(device_);
-  if (coherence_ == Coherence::kStrict) {
-    for (const auto& [off, bytes] : device_dirty_) {
-      if (auto r = Check(cudaMemcpyAsync(host_arena_ + off, d_arena_ + off, bytes,
-                                         cudaMemcpyDeviceToHost, stream_), "flush download"); !r)
+  // Strict coherence: every range written since the last flush comes back.  Scattered over at most kFlushStaging bytes
+  // they come as ONE copy of the whole span into pinned memory, and the host takes just the written ranges from there (a
+  // copy and a wait of its own per range was 15 us each); wider spans go range by range.
+  uint64_t lo = ~0ull, hi = 0;
+  const bool strict = coherence_ == Coherence::kStrict && !device_dirty_.empty();
+  bool staged = false;
+  if (strict) {
+    for (const auto& [off, bytes] : device_dirty_) { lo = std::min(lo, off); hi = std::max(hi, off + bytes); }
+    staged = hi - lo <= kFlushStaging;
+    if (staged) {
+      if (auto r = Check(cudaMemcpyAsync(h_flush_, d_arena_ + lo, hi - lo, cudaMemcpyDeviceToHost, stream_),
+                         "flush download"); !r)
         return r;
-      counters_.d2h_bytes += bytes;
+      counters_.d2h_bytes += hi - lo;
+    } else {
+      for (const auto& [off, bytes] : device_dirty_) {
+        if (auto r = Check(cudaMemcpyAsync(host_arena_ + off, d_arena_ + off, bytes,
+                                           cudaMemcpyDeviceToHost, stream_), "flush download"); !r)
+          return r;
+        counters_.d2h_bytes += bytes;
+      }
     }
   }
-  device_dirty_.clear();
-  if (auto r = Check(cudaMemcpyAsync(h_status_, d_status_, sizeof(k::DeviceStatus),
-                                     cudaMemcpyDeviceToHost, stream_), "status"); !r)
-    return r;
+  constexpr uint32_t kStatusWords = sizeof(k::DeviceStatus) / 4;
+  k::PublishList list;
+  list.item[list.count++] = {reinterpret_cast<const uint32_t*>(d_status_), kStatusWords};
+  uint32_t words = 0;
+  for (const k::PublishItem& it : items) { list.item[list.count++] = it; words += it.words; }
+  k::PublishToHost(list, h_published_, stream_);
+  counters_.d2h_bytes += words * 4;
   // Completion is an error or a success, never a silent fallback.
   if (auto r = Check(cudaStreamSynchronize(stream_), "flush: device work did not complete"); !r)
     return r;
   if (auto e = cudaGetLastError(); e != cudaSuccess) return std::unexpected(CudaErr(e, "flush"));
+  if (staged)
+    for (const auto& [off, bytes] : device_dirty_) std::memcpy(host_arena_ + off, h_flush_ + (off - lo), bytes);
+  device_dirty_.clear();
+  if (words && out) std::memcpy(out, h_published_ + kStatusWords, words * 4);
   if (!deferred_error_.empty()) {
     std::string e;
     e.swap(deferred_error_);
     return std::unexpected(e);
   }
-  if (h_status_[0] || h_status_[1]) {
-    const bool refused = h_status_[0] != 0;
+  if (h_published_[0] || h_published_[1]) {
+    const bool refused = h_published_[0] != 0;
     cudaMemsetAsync(d_status_, 0, sizeof(k::DeviceStatus), stream_);
     cudaStreamSynchronize(stream_);
-    h_status_[0] = h_status_[1] = 0;
     return std::unexpected(refused ? std::string(kNonFiniteNormRefusal)
                                    : std::string("cuda: a bounded device-side wait ran out"));
   }
@@ -2022,15 +2051,9 @@ void CudaBackend::SetCapturing(bool on) { capturing_ = on; }
 
 Status CudaBackend::UploadStepScalars(const StepParams& params) {
   cudaSetDevice(device_);
-  scalar_slot_ = (scalar_slot_ + 1) % kScalarSlots;
-  // The slot's previous upload may still be queued behind device work when the
-  // host runs many steps ahead: its bytes must not change until that copy ran.
-  if (auto r = Check(cudaEventSynchronize(scalar_done_[scalar_slot_]), "step scalars: slot"); !r) return r;
-  h_scalars_[scalar_slot_] = ScalarsOf(params);
-  if (auto r = Check(cudaMemcpyAsync(d_scalars_, &h_scalars_[scalar_slot_], sizeof(k::AdamScalars),
-                                     cudaMemcpyHostToDevice, stream_), "step scalars"); !r)
-    return r;
-  if (auto r = Check(cudaEventRecord(scalar_done_[scalar_slot_], stream_), "step scalars: event"); !r) return r;
+  k::SetScalars(ScalarsOf(params), d_scalars_, stream_);
+  ++counters_.kernel_launches;
+  if (auto r = Check(cudaPeekAtLastError(), "step scalars"); !r) return r;
   last_params_ = params;
   scalars_valid_ = true;
   return {};

@@ -23,6 +23,7 @@
 
 #include <cstdint>
 #include <expected>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <span>
@@ -92,6 +93,9 @@ class CudaBackend {
   // Asynchronous src -> device on the backend's stream; `src` must stay valid
   // until the stream has passed the copy (pinned memory for true overlap).
   Status WriteArena(uint64_t off, uint64_t bytes, const void* src);
+  // Two small ranges (the second may be empty) out of pinned memory by one kernel of the stream; same ordering and
+  // lifetime rules as WriteArena.
+  Status WriteArenaPinned(uint64_t off0, uint64_t bytes0, const void* src0, uint64_t off1, uint64_t bytes1, const void* src1);
   void Configure() {}  // the CPU tile policy is throughput-only on its own backend; ignored here
 
   Status Execute(const Instruction& ins, const StepParams& params);
@@ -109,7 +113,10 @@ class CudaBackend {
   }
   void BeginRange(std::span<const Instruction> program, size_t begin, size_t end);
   void EndRange();
-  Status Flush();
+  Status Flush() { return FlushWith({}); }
+  // Flush, and read `items` (device words, at most kPublishWords in all) into `out` on the way: one launch and one wait.
+  static constexpr uint32_t kPublishWords = 48;
+  Status FlushWith(std::initializer_list<k::PublishItem> items, uint32_t* out = nullptr);
 
   uint64_t relaxed_executions() const { return counters_.relaxed_executions; }
   uint64_t fused_dispatches() const { return counters_.fused_dispatches; }
@@ -158,11 +165,10 @@ class CudaBackend {
 
   // CUDA-graph support for the engine.  The optimizer kernels read the step's
   // learning rate and bias corrections from a small device block.  A captured
-  // range contains no upload of that block: before it captures or replays a range
-  // with optimizer instructions the engine calls UploadStepScalars, an ordinary
-  // stream-ordered copy from a ring of pinned slots (a slot is rewritten only
-  // after the copy that last read it has completed), so every replay sees its own
-  // step's values however far the host runs ahead of the device.
+  // range contains no write of that block: before it captures or replays a range
+  // with optimizer instructions the engine calls UploadStepScalars, a one-thread
+  // kernel of the stream that carries the values as its parameters, so every replay
+  // sees its own step's values however far the host runs ahead of the device.
   void SetCapturing(bool on);
   Status UploadStepScalars(const StepParams& params);
   static k::AdamScalars ScalarsOf(const StepParams& params);
@@ -231,13 +237,12 @@ class CudaBackend {
   float* d_gsum_ = nullptr;       // summed gradient for fused clips under data parallelism
   uint64_t gsum_capacity_ = 0;
   k::AdamScalars* d_scalars_ = nullptr;
-  k::AdamScalars* h_scalars_ = nullptr;  // pinned ring
-  std::vector<cudaEvent_t> scalar_done_; // per slot: the upload that last read it
-  int scalar_slot_ = 0;
   StepParams last_params_{};
   bool scalars_valid_ = false;
   bool capturing_ = false;
-  int* h_status_ = nullptr;  // pinned mirror of the status words
+  uint32_t* h_published_ = nullptr;  // pinned: the status words, then what a FlushWith asked for
+  uint8_t* h_flush_ = nullptr;       // behind it: pinned staging of a strict flush's downloads
+  static constexpr uint64_t kPublishedBytes = 4096, kFlushStaging = 2ull << 20;
 
   Coherence coherence_ = Coherence::kStrict;
   std::vector<std::pair<uint64_t, uint64_t>> host_dirty_;

@@ -263,8 +263,9 @@ Status UpdateEngine::LoadFromMemory(const uint8_t* plan, uint64_t size) {
     d_eval_terms_ = static_cast<double*>(p);
     eval_terms_capacity_ = terms;
   }
-  const uint64_t stage = (h.input_ref == kNullRef ? 0 : h.input_floats * 4) +
-                         (h.label_ref == kNullRef ? 0 : h.label_bytes);
+  // (labels start on a 16-byte boundary behind the input, and a half on one behind the other)
+  const uint64_t stage = (h.input_ref == kNullRef ? 0 : (h.input_floats * 4 + 15) / 16 * 16) +
+                         (h.label_ref == kNullRef ? 0 : (h.label_bytes + 15) / 16 * 16);
   if (stage > pinned_bytes_) {
     if (pinned_) cudaFreeHost(pinned_);
     pinned_ = nullptr;
@@ -332,13 +333,23 @@ Status UpdateEngine::StageBatch(const void* input, uint64_t input_bytes, const v
   // half has been consumed, fill it, enqueue the async upload.
   uint8_t* buf = pinned_ + static_cast<uint64_t>(pinned_slot_) * pinned_bytes_;
   cudaEventSynchronize(staged_[pinned_slot_]);
+  uint8_t* lab_buf = buf + (want_in + 15) / 16 * 16;
   if (want_in) std::memcpy(buf, input, want_in);
-  if (want_lab) std::memcpy(buf + want_in, labels, want_lab);
-  if (want_in)
-    if (auto r = backend_->WriteArena(RefOffset(header_.input_ref), want_in, buf); !r) return r;
-  if (want_lab)
-    if (auto r = backend_->WriteArena(RefOffset(header_.label_ref), want_lab, buf + want_in); !r)
+  if (want_lab) std::memcpy(lab_buf, labels, want_lab);
+  // A small batch by a kernel that reads the pinned half itself, a large one by the copy engine: the kernel saves two
+  // engine hand-overs (about 20 us), the copy engine is faster from about a megabyte.
+  constexpr uint64_t kKernelBytes = 1 << 20;
+  if (want_in + want_lab <= kKernelBytes) {
+    if (auto r = backend_->WriteArenaPinned(want_in ? RefOffset(header_.input_ref) : 0, want_in, buf,
+                                            want_lab ? RefOffset(header_.label_ref) : 0, want_lab, lab_buf);
+        !r)
       return r;
+  } else {
+    if (want_in)
+      if (auto r = backend_->WriteArena(RefOffset(header_.input_ref), want_in, buf); !r) return r;
+    if (want_lab)
+      if (auto r = backend_->WriteArena(RefOffset(header_.label_ref), want_lab, lab_buf); !r) return r;
+  }
   cudaEventRecord(staged_[pinned_slot_], backend_->stream());
   pinned_slot_ ^= 1;
   return {};
@@ -497,8 +508,17 @@ StepTimings UpdateEngine::TakeTimings() {
 
 Status UpdateEngine::ReadLoss(float* loss) {
   if (header_.loss_ref == kNullRef) return std::unexpected("engine: the plan has no loss slot");
-  if (auto r = backend_->ReadArena(RefOffset(header_.loss_ref), 4, loss); !r) return r;
-  return backend_->Flush();  // surfaces a refusal raised on the device
+  if (!loaded_) return std::unexpected("engine: no plan is loaded");
+  const auto* slot = reinterpret_cast<const uint32_t*>(backend_->device_arena() + RefOffset(header_.loss_ref));
+  return backend_->FlushWith({{slot, 1}}, reinterpret_cast<uint32_t*>(loss));  // surfaces a refusal raised on the device
+}
+
+Status UpdateEngine::TrainStep(const void* input, uint64_t input_bytes, const void* labels, uint64_t label_bytes,
+                               float* loss) {
+  if (auto r = StageBatch(input, input_bytes, labels, label_bytes); !r) return r;
+  if (auto r = TrainForwardBackward(true); !r) return r;
+  if (auto r = TrainOptimizer(); !r) return r;
+  return ReadLoss(loss);
 }
 
 Status UpdateEngine::Evaluate(EvalResult* out, uint64_t real_rows) {
@@ -508,7 +528,6 @@ Status UpdateEngine::Evaluate(EvalResult* out, uint64_t real_rows) {
   const uint64_t real = std::min<uint64_t>(real_rows, header_.batch);
   cudaStream_t s = backend_->stream();
   cudaMemsetAsync(d_tally_, 0, 4 * sizeof(unsigned long long), s);
-  cudaMemsetAsync(d_eval_out_, 0, 2 * sizeof(double), s);
   auto at = [&](uint64_t ref) { return backend_->device_arena() + RefOffset(ref); };
   // Accuracy needs class labels in the label slot and a softmax whose rows cover
   // the batch (reference: update_engine.cc:458-466); real rows only, each once.
@@ -532,13 +551,16 @@ Status UpdateEngine::Evaluate(EvalResult* out, uint64_t real_rows) {
       break;
     case EvalTail::kWeighted: row_loss = false; break;
   }
-  unsigned long long tally[4] = {0, 0, 0, 0};
-  double sums[2] = {0, 0};
-  if (auto e = cudaMemcpyAsync(tally, d_tally_, sizeof(tally), cudaMemcpyDeviceToHost, s); e != cudaSuccess)
-    return std::unexpected(std::string("engine: tally read: ") + cudaGetErrorString(e));
-  if (auto e = cudaMemcpyAsync(sums, d_eval_out_, sizeof(sums), cudaMemcpyDeviceToHost, s); e != cudaSuccess)
-    return std::unexpected(std::string("engine: row-loss read: ") + cudaGetErrorString(e));
-  if (auto r = ReadLoss(&out->loss); !r) return r;   // synchronises the stream
+  if (header_.loss_ref == kNullRef) return std::unexpected("engine: the plan has no loss slot");
+  struct { unsigned long long tally[4]; double sums[2]; float loss; uint32_t pad; } got{};
+  const auto* slot = reinterpret_cast<const uint32_t*>(at(header_.loss_ref));
+  if (auto r = backend_->FlushWith({{reinterpret_cast<const uint32_t*>(d_tally_), 8},
+                                    {reinterpret_cast<const uint32_t*>(d_eval_out_), 4}, {slot, 1}},
+                                   reinterpret_cast<uint32_t*>(&got)); !r)
+    return r;
+  const auto& tally = got.tally;
+  const auto& sums = got.sums;
+  out->loss = got.loss;
   out->rows = tally[0];
   out->correct = tally[1];
   out->has_accuracy = track_accuracy;
@@ -573,9 +595,8 @@ Status UpdateEngine::RunMerge(bool* all_finite) {
                         d_tally_, s);
   }
   unsigned long long tally[4] = {0, 0, 0, 0};
-  if (auto e = cudaMemcpyAsync(tally, d_tally_, sizeof(tally), cudaMemcpyDeviceToHost, s); e != cudaSuccess)
-    return std::unexpected(std::string("engine: tally read: ") + cudaGetErrorString(e));
-  if (auto r = backend_->Flush(); !r) return r;
+  if (auto r = backend_->FlushWith({{reinterpret_cast<const uint32_t*>(d_tally_), 8}}, reinterpret_cast<uint32_t*>(tally)); !r)
+    return r;
   if (all_finite) *all_finite = tally[2] == 0;
   return {};
 }

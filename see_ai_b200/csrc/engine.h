@@ -89,6 +89,8 @@ class UpdateEngine {
   Status TrainOptimizer();                     // [opt_begin, end)
   Status StepProgram();
   Status ReadLoss(float* loss);
+  // StageBatch, TrainForwardBackward(true), TrainOptimizer, ReadLoss in one call.
+  Status TrainStep(const void* input, uint64_t input_bytes, const void* labels, uint64_t label_bytes, float* loss);
   // Evaluation of the staged batch: the eval program, its loss, and on the
   // device the accuracy tally and the real-row loss over the batch's first
   // `real_rows` rows (the whole batch when real_rows >= the plan's batch).

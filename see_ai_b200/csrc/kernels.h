@@ -160,6 +160,17 @@ void SgdStep(float* p, const float* g, size_t n, const AdamScalars* a,
 void SumCopies(const float* g, float* out, size_t n, int g_copies, size_t copy_stride,
                float inv_copies, cudaStream_t s);
 
+// ---- small transfers to and from pinned host memory, as kernels of the stream (k_host.cu) ----
+struct HostCopy { void* dst = nullptr; const void* src = nullptr; size_t bytes = 0; };
+// Two copies out of pinned host memory in one launch (either may be empty).
+void StageFromHost(const HostCopy& a, const HostCopy& b, cudaStream_t s);
+// The items' words, one after the other, into pinned host memory; visible once the stream has been waited for.
+constexpr int kPublishItems = 6;
+struct PublishItem { const uint32_t* src; uint32_t words; };
+struct PublishList { PublishItem item[kPublishItems]; int count = 0; };
+void PublishToHost(const PublishList& list, uint32_t* host, cudaStream_t s);
+void SetScalars(const AdamScalars& v, AdamScalars* dst, cudaStream_t s);
+
 // ---- attention (exact family; scores in double like the CPU executor) --------
 void AttnFwd(const float* q, const float* k, const float* v, float* o, float* probs,
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,

@@ -17,7 +17,7 @@ ENGINE_SYMBOLS = [
     "see_engine_create", "see_engine_destroy", "see_engine_last_error", "see_engine_backend",
     "see_engine_load", "see_engine_bind_source", "see_engine_header", "see_engine_stage_batch",
     "see_engine_train_forward_backward", "see_engine_train_optimizer", "see_engine_step_program",
-    "see_engine_read_loss", "see_engine_evaluate", "see_engine_evaluate_rows", "see_engine_run_merge",
+    "see_engine_read_loss", "see_engine_train_step", "see_engine_evaluate", "see_engine_evaluate_rows", "see_engine_run_merge",
     "see_engine_read_arena", "see_engine_write_arena", "see_engine_step", "see_engine_set_step",
     "see_engine_set_horizon", "see_engine_effective_lr", "see_engine_set_use_graphs",
     "see_engine_set_phase_timing", "see_engine_take_timings", "see_engine_gradient_block",
@@ -64,6 +64,7 @@ def _lib() -> ctypes.CDLL:
     lib.see_engine_train_forward_backward.argtypes = [vp, i32]
     lib.see_engine_train_optimizer.argtypes = [vp]
     lib.see_engine_step_program.argtypes = [vp]
+    lib.see_engine_train_step.argtypes = [vp, vp, u64, vp, u64, ctypes.POINTER(ctypes.c_float)]
     lib.see_engine_read_loss.argtypes = [vp, ctypes.POINTER(ctypes.c_float)]
     lib.see_engine_evaluate.argtypes = [vp, ctypes.POINTER(ctypes.c_float), ctypes.POINTER(u64),
                                         ctypes.POINTER(u64)]
@@ -174,10 +175,13 @@ class Engine:
 
     def train_step(self, x, y) -> float:
         """One optimizer step of a plan without gradient accumulation."""
-        self.stage_batch(x, y)
-        self.train_forward_backward(True)
-        self.train_optimizer()
-        return self.read_loss()
+        x = np.ascontiguousarray(x)
+        yb = np.ascontiguousarray(y) if y is not None else None
+        v = ctypes.c_float()
+        self._check(self.lib.see_engine_train_step(
+            self.h, x.ctypes.data, x.nbytes, yb.ctypes.data if yb is not None else None,
+            yb.nbytes if yb is not None else 0, ctypes.byref(v)))
+        return float(np.float32(v.value))
 
     def evaluate(self, x, y) -> Tuple[float, int, int]:
         self.stage_batch(x, y)
