@@ -2137,6 +2137,7 @@ Status CudaBackend::DispatchOptimizer(const Instruction& ins, const StepParams& 
 Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, const Extents&) {
   cudaStream_t s = stream_;
   auto launched = [&](int n = 1) { counters_.kernel_launches += n; };
+  const bool fused = coherence_ == Coherence::kLazy && adapter_fma_;   // (the exact attention family's output sums)
   if (range_index_ < merge_run_of_.size() && merge_run_of_[range_index_] != -1) {
     if (merge_run_of_[range_index_] == -2) return {};   // done by the run's first instruction
     return DispatchMergeRun(merge_runs_[static_cast<size_t>(merge_run_of_[range_index_])]);
@@ -2221,14 +2222,14 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
     case kLayerNormBwd: {
       const AddFusion* adf = range_index_ < add_fusion_.size() && add_fusion_[range_index_].fuse
                                  ? &add_fusion_[range_index_] : nullptr;
-      const int fused = k::LayerNormBwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Rd(ins.out[0]),
+      const int absorbed = k::LayerNormBwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Rd(ins.out[0]),
                                          Rd(ins.out[1]), Wr(ins.in[3]), Hi32(ins.out[2]), Lo32(ins.out[2]), s,
                                          adf ? Rd(adf->x_ref) : nullptr, adf ? Wr(adf->out_ref) : nullptr,
                                          adf ? ShadowFor(adf->out_ref, static_cast<uint64_t>(Hi32(ins.out[2])) *
                                                                            Lo32(ins.out[2])) : nullptr);
       launched();
-      if (fused) {   // the kAddEW after it has been done
-        shadow_written_ = fused == 2;
+      if (absorbed) {   // the kAddEW after it has been done
+        shadow_written_ = absorbed == 2;
         umma::InvalidateRange(&umma_->ctx, RefOffset(adf->out_ref),
                               static_cast<uint64_t>(Hi32(ins.out[2])) * Lo32(ins.out[2]) * 4);
         ++counters_.fused_dispatches;
@@ -2258,11 +2259,11 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
         fb.seed = lf->seed;
         fb.store_probs = lf->store_probs;
       }
-      const bool fused = k::SoftmaxXEntFwd(ins.opcode == kSoftmaxXEntMaskedFwd, Rd(ins.in[0]),
+      const bool with_bwd = k::SoftmaxXEntFwd(ins.opcode == kSoftmaxXEntMaskedFwd, Rd(ins.in[0]),
                                            Rd<int32_t>(ins.in[1]), Wr(ins.in[2]), Wr(ins.in[3]), ins.out[0],
                                            ins.out[1], d_rows_, d_count_, s, lf ? &fb : nullptr);
       launched(2);
-      if (fused) {   // the backward instruction two places on has been done
+      if (with_bwd) {   // the backward instruction two places on has been done
         shadow_written_ = true;
         skip_act_at_ = static_cast<int64_t>(lf->bwd_index);
         ++counters_.fused_dispatches;
@@ -2353,13 +2354,13 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
       break;
     case kAttnFwd:
       k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
-                 Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, s);
+                 Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
       launched();
       break;
     case kAttnFwdSeg: {
       const AttnGeom g = UnpackAttnGeom(ins.out[1]);
       k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
-                 g.B, g.S, g.H, g.d, Rd<int32_t>(ins.out[2]), s);
+                 g.B, g.S, g.H, g.d, Rd<int32_t>(ins.out[2]), fused, s);
       launched();
       break;
     }
@@ -2390,13 +2391,13 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
         }
       }
       k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
-                 Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, s);
+                 Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
       launched();
       break;
     case kAttnFwdTiledSeg: {
       const AttnGeom g = UnpackAttnGeom(ins.out[1]);
       k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
-                 g.B, g.S, g.H, g.d, Rd<int32_t>(ins.out[2]), s);
+                 g.B, g.S, g.H, g.d, Rd<int32_t>(ins.out[2]), fused, s);
       launched();
       break;
     }
@@ -2407,7 +2408,7 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
       break;
     case kAttnDV:
       k::AttnDV(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
-                Hi32(ins.out[1]), Lo32(ins.out[1]), s);
+                Hi32(ins.out[1]), Lo32(ins.out[1]), fused, s);
       launched();
       break;
     case kSoftmaxRowsBwd:
@@ -2417,12 +2418,12 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
       break;
     case kAttnDQ:
       k::AttnDQ(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
-                Hi32(ins.out[1]), Lo32(ins.out[1]), s);
+                Hi32(ins.out[1]), Lo32(ins.out[1]), fused, s);
       launched();
       break;
     case kAttnDK:
       k::AttnDK(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
-                Hi32(ins.out[1]), Lo32(ins.out[1]), s);
+                Hi32(ins.out[1]), Lo32(ins.out[1]), fused, s);
       launched();
       break;
     case kAttnDQTiled: case kAttnDKTiled: case kAttnDVTiled: {
@@ -2483,10 +2484,10 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
         return std::unexpected("cuda: tiled attention backward supports head widths up to 256");
       if (ins.opcode == kAttnDQTiled)
         k::AttnDQTiled(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Rd(ins.in[3]), Wr(ins.out[0]),
-                       Wr(ins.out[1]), g.B, g.S, g.H, g.d, s);
+                       Wr(ins.out[1]), g.B, g.S, g.H, g.d, fused, s);
       else
         k::AttnDKVTiled(ins.opcode == kAttnDKTiled, Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]),
-                        Rd(ins.in[3]), Rd(ins.out[0]), Wr(ins.out[1]), g.B, g.S, g.H, g.d, s);
+                        Rd(ins.in[3]), Rd(ins.out[0]), Wr(ins.out[1]), g.B, g.S, g.H, g.d, fused, s);
       launched();
       break;
     }

@@ -15,15 +15,16 @@
 // Two sets of kernels give the same bits.
 //
 // The tile kernels (AttnFwdTile, AttnDPTile, AttnRowTile, AttnColTile,
-// AttnDQTiledTile, AttnDKVTiledTile) are FP64-bound: a block owns 16, 32 or 64
+// AttnDQTiledTile, AttnDKVTiledTile) are FP64-bound: a block owns 8, 16 or 32
 // query (or key) rows of one (sequence, head) and takes the other axis 64 at a
-// time.  Both operands of a score tile are widened to double once, while they
-// are copied to shared memory (a conversion costs four FMA slots, so per use it
-// would be the bound), features slowest, and a thread accumulates RM x 4 pairs
-// in registers: RM + 4 shared doubles per 4 RM fused multiply-adds, each
-// accumulator one chain over ascending features.  The f32 output sums are the
-// same shape of product, 64 columns of the head at a time, RM x 4 outputs per
-// thread, each one chain over ascending keys.
+// time.  Both operands of a score tile are widened to double once, on their way
+// into shared memory (a conversion costs four FMA slots, so per use it would be
+// the bound): the block's own rows for good, the streamed ones 8 features at a
+// time with the next 8 already in registers; a thread accumulates RM x 4 pairs:
+// RM + 4 shared doubles per 4 RM fused multiply-adds, each accumulator one chain
+// over ascending features.  The f32 output sums are the same shape of product,
+// 64 columns of the head at a time, RM x 4 outputs per thread, each one chain over
+// ascending keys, the keys' rows arriving by asynchronous copies.
 // One warp per row with a strided K row per lane (the row kernels below) took
 // 3747 us for 8 x 512 positions of 12 heads of 64 features and 320 us for
 // 32 x 128 of 4 heads.
@@ -212,61 +213,95 @@ __global__ void AttnDQTiledKernel(const float* __restrict__ q, const float* __re
 }
 
 // ---- tile kernels ------------------------------------------------------------------
+// A block of eight warps owns R = 8 RM rows of one axis (its "own" rows) and streams the other axis 64 rows at a time: two
+// groups of four warps take alternate tiles, each with slice buffers and barriers of its own (the score rows leave room
+// for two blocks per SM; one group per block, eight warps on an SM, issued 1.9 instructions per cycle).
 
-constexpr int kTile = 64;      // keys (or queries) of the streamed axis per step
-constexpr int kSlice = 32;     // features of both operands in shared memory at a time
+constexpr int kTile = 64;      // rows of the streamed axis per step
+constexpr int kSlice = 8;      // features of a streamed tile in shared memory at a time
 constexpr int kTileThreads = 256;
+constexpr int kGroup = 128;            // threads of a group
+constexpr int kStreamLd = kTile + 2;   // doubles per feature of a streamed slice (a multiple of 16 bytes; 2-way store conflicts)
+constexpr int kChunkRows = 32;         // rows of an f32 tile in shared memory at a time
 
-// Rows [0, rows) of a [., stride] f32 matrix, features [c0, c0 + kSlice) of d, widened into
-// dst[feature][kRows]; what lies outside is zero (0 * 0 leaves a chain as it is).
-// Lanes take consecutive rows, so that the stores are conflict-free; a row's 128-byte slice is
-// read 16 bytes at a time and stays in L1 between them.
+__host__ __device__ constexpr int PaddedFeatures(int d) { return (d + kSlice - 1) / kSlice * kSlice; }
+
+__device__ __forceinline__ float4 LoadFour(const float* __restrict__ p, int left, bool vec) {   // left: elements there are
+  if (left <= 0) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (vec) return *reinterpret_cast<const float4*>(p);
+  return make_float4(p[0], left > 1 ? p[1] : 0.0f, left > 2 ? p[2] : 0.0f, left > 3 ? p[3] : 0.0f);
+}
+
+// The block's own rows, widened to double once: dst[feature][kRows], zero outside (0 * 0 leaves a chain as it is).
 template <int kRows, bool kVec>
-__device__ __forceinline__ void LoadSlice(double* dst, const float* __restrict__ src, size_t stride, int rows, int c0,
-                                          int d) {
-  for (int t = threadIdx.x; t < kRows * (kSlice / 4); t += kTileThreads) {
-    const int r = t % kRows, c = t / kRows * 4;
-    float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (r < rows && c0 + c < d) {
-      const float* p = src + static_cast<size_t>(r) * stride + c0 + c;
-      if (kVec) {
-        const float4 f = *reinterpret_cast<const float4*>(p);
-        x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (c0 + c + e < d) x[e] = p[e];
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) dst[(c + e) * kRows + r] = static_cast<double>(x[e]);
+__device__ __forceinline__ void LoadOwn(double* dst, const float* __restrict__ src, size_t stride, int rows, int d) {
+  const int quads = PaddedFeatures(d) / 4;
+  for (int t = threadIdx.x; t < kRows * quads; t += kTileThreads) {
+    const int r = t / quads, c = t % quads * 4;
+    const float4 f = LoadFour(src + static_cast<size_t>(min(r, rows - 1)) * stride + c, r < rows ? d - c : 0, kVec);
+    dst[c * kRows + r] = f.x;
+    dst[(c + 1) * kRows + r] = f.y;
+    dst[(c + 2) * kRows + r] = f.z;
+    dst[(c + 3) * kRows + r] = f.w;
   }
 }
 
-// acc[r][e] = row (ty RM + r) of `a` . row Col(e) of `b`, in double, ascending features.
-// Starts with a barrier (the slices may still be in use) and leaves none behind.
+__device__ __forceinline__ int GroupOf() { return static_cast<int>(threadIdx.x) / kGroup; }
+__device__ __forceinline__ int InGroup() { return static_cast<int>(threadIdx.x) % kGroup; }
+__device__ __forceinline__ void GroupSync() {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + GroupOf()), "n"(kGroup) : "memory");
+}
+// A multiply-add of an output sum: two roundings as the CPU executor makes them, or one where the bits are not observed.
+template <bool kFused>
+__device__ __forceinline__ float MulAdd(float a, float b, float c) {
+  return kFused ? fmaf(a, b, c) : c + a * b;
+}
+
+// A streamed tile's slice on its way: a row's four features per thread of the group.
+struct SliceRegs { float4 v; };
+template <bool kVec>
+__device__ __forceinline__ void FetchSlice(SliceRegs* s, const float* __restrict__ src, size_t stride, int rows, int c0,
+                                           int d) {
+  const int r = InGroup() >> 1, c = c0 + (InGroup() & 1) * 4;
+  s->v = LoadFour(src + static_cast<size_t>(min(r, rows - 1)) * stride + c, r < rows ? d - c : 0, kVec);
+}
+__device__ __forceinline__ void StoreSlice(double* dst, const SliceRegs& s) {
+  const int r = InGroup() >> 1, c = (InGroup() & 1) * 4;
+  dst[c * kStreamLd + r] = s.v.x;
+  dst[(c + 1) * kStreamLd + r] = s.v.y;
+  dst[(c + 2) * kStreamLd + r] = s.v.z;
+  dst[(c + 3) * kStreamLd + r] = s.v.w;
+}
+
+// acc[r][e] = own row (ty RM + r) . streamed row Col(e), in double, ascending features.  `regs` holds the tile's first
+// slice on entry and the first slice of `next` (rows of the same stride; null: nothing) on exit, so that a global load is
+// always a whole slice of arithmetic ahead of its use.  `turn` alternates the two slice buffers: one barrier per slice.
 template <int RM, bool kVec>
-__device__ __forceinline__ void DotTile(const float* a, int a_rows, const float* b, int b_rows, size_t stride, int d,
-                                        double* sa, double* sb, double (&acc)[RM][4]) {
-  constexpr int R = 16 * RM;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+__device__ __forceinline__ void DotTile(const double* own, const float* b, int rows, const float* next, int next_rows,
+                                        size_t stride, int d, double* slices, int* turn, SliceRegs* regs,
+                                        double (&acc)[RM][4]) {
+  constexpr int R = 8 * RM;
+  const int tx = threadIdx.x & 15, ty = InGroup() >> 4;
 #pragma unroll
   for (int r = 0; r < RM; ++r)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[r][e] = 0.0;
   for (int c0 = 0; c0 < d; c0 += kSlice) {
-    __syncthreads();
-    LoadSlice<R, kVec>(sa, a, stride, a_rows, c0, d);
-    LoadSlice<kTile, kVec>(sb, b, stride, b_rows, c0, d);
-    __syncthreads();
-#pragma unroll 8
-    for (int c = 0; c < kSlice; ++c) {
-      double x[RM], y[4];
-      const double2 y0 = *reinterpret_cast<const double2*>(sb + c * kTile + 2 * tx);
-      const double2 y1 = *reinterpret_cast<const double2*>(sb + c * kTile + 32 + 2 * tx);
-      y[0] = y0.x; y[1] = y0.y; y[2] = y1.x; y[3] = y1.y;
+    double* sb = slices + *turn * (kSlice * kStreamLd);
+    *turn ^= 1;
+    StoreSlice(sb, *regs);
+    GroupSync();
+    if (c0 + kSlice < d) FetchSlice<kVec>(regs, b, stride, rows, c0 + kSlice, d);
+    else if (next) FetchSlice<kVec>(regs, next, stride, next_rows, 0, d);
+    const double* sa = own + c0 * R + ty * RM;
 #pragma unroll
-      for (int r = 0; r < RM; ++r) x[r] = sa[c * R + ty * RM + r];
+    for (int c = 0; c < kSlice; ++c) {
+      const double2 y0 = *reinterpret_cast<const double2*>(sb + c * kStreamLd + 2 * tx);
+      const double2 y1 = *reinterpret_cast<const double2*>(sb + c * kStreamLd + 32 + 2 * tx);
+      const double y[4] = {y0.x, y0.y, y1.x, y1.y};
+      double x[RM];
+#pragma unroll
+      for (int r = 0; r < RM; ++r) x[r] = sa[c * R + r];
 #pragma unroll
       for (int r = 0; r < RM; ++r)
 #pragma unroll
@@ -274,29 +309,33 @@ __device__ __forceinline__ void DotTile(const float* a, int a_rows, const float*
     }
   }
 }
-// The tile column a thread's accumulator e stands for (pairs, so that 16 lanes read 256 contiguous bytes).
+// The tile row a thread's accumulator e stands for (pairs, so that 16 lanes read 256 contiguous bytes).
 __device__ __forceinline__ int Col(int e) { return 2 * static_cast<int>(threadIdx.x & 15) + (e & 1) + (e >> 1) * 32; }
 
-// Rows [0, rows) x columns [c0, c0 + 64) of a [., stride] f32 matrix into dst[64][64] (zero outside).
+__host__ __device__ constexpr size_t GroupBytes() { return 2 * sizeof(double) * kSlice * kStreamLd; }
+__host__ __device__ constexpr size_t StreamBytes() { return 2 * GroupBytes(); }
+__host__ __device__ constexpr size_t OwnBytes(int RM, int d) { return sizeof(double) * PaddedFeatures(d) * 8 * RM; }
+
+// Rows [0, rows) x columns [c0, c0 + 64) of a [., stride] f32 matrix into dst[32][64] by asynchronous copies (zero
+// outside); one commit group.
 template <bool kVec>
-__device__ __forceinline__ void LoadTileF(float* dst, const float* __restrict__ src, size_t stride, int rows, int c0,
+__device__ __forceinline__ void CopyChunk(float* dst, const float* __restrict__ src, size_t stride, int rows, int c0,
                                           int d) {
-  for (int t = threadIdx.x; t < kTile * 16; t += kTileThreads) {
+  for (int t = threadIdx.x; t < kChunkRows * 16; t += kTileThreads) {
     const int r = t >> 4, c = (t & 15) * 4;
-    float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (r < rows && c0 + c < d) {
-      const float* p = src + static_cast<size_t>(r) * stride + c0 + c;
-      if (kVec) {
-        f = *reinterpret_cast<const float4*>(p);
-      } else {
-        f.x = p[0];
-        if (c0 + c + 1 < d) f.y = p[1];
-        if (c0 + c + 2 < d) f.z = p[2];
-        if (c0 + c + 3 < d) f.w = p[3];
-      }
+    const int left = r < rows ? d - (c0 + c) : 0;
+    const float* p = src + static_cast<size_t>(r < rows ? r : 0) * stride + (left > 0 ? c0 + c : 0);
+    const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(dst + r * kTile + c));
+    if (kVec) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(p), "r"(left > 0 ? 16 : 0) : "memory");
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
+                     ::"r"(to + 4 * e), "l"(left > e ? p + e : src), "r"(left > e ? 4 : 0) : "memory");
     }
-    *reinterpret_cast<float4*>(dst + r * kTile + c) = f;
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
 __device__ __forceinline__ void StoreRow4(float* p, const float (&v)[4], int c, int d, bool vec) {
@@ -310,14 +349,14 @@ __device__ __forceinline__ void StoreRow4(float* p, const float (&v)[4], int c, 
   }
 }
 
-// acc[r][e] += w[row][j] * x[j][c + e] for j = 0 .. 63 in order; row's weights at w + r * ld.  A row takes
+// acc[r][e] += w[row][j] * x[j][c + e] for j = 0 .. 31 in order; row's weights at w + r * ld.  A row takes
 // j in [lo[r], hi[r]) only (a weight outside is not multiplied: x may hold anything there); kAll: every j.
-template <int RM, bool kAll>
+template <bool kFused, int RM, bool kAll>
 __device__ __forceinline__ void RowProduct(const float* w, int ld, const float* x, const int (&lo)[RM],
                                            const int (&hi)[RM], float (&acc)[RM][4]) {
   const int c = (threadIdx.x & 15) * 4;
 #pragma unroll 2
-  for (int j = 0; j < kTile; j += 4) {
+  for (int j = 0; j < kChunkRows; j += 4) {
     float p[RM][4];
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
@@ -332,15 +371,44 @@ __device__ __forceinline__ void RowProduct(const float* w, int ld, const float* 
       for (int r = 0; r < RM; ++r) {
         if (kAll || (j + jj >= lo[r] && j + jj < hi[r])) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[r][e] += p[r][jj] * xv[e];
+          for (int e = 0; e < 4; ++e) acc[r][e] = MulAdd<kFused>(p[r][jj], xv[e], acc[r][e]);
         }
       }
     }
   }
 }
 
-__host__ __device__ constexpr size_t SliceBytes(int RM) { return sizeof(double) * kSlice * (16 * RM + kTile); }
-// Score rows are stored with a stride of a whole number of key tiles plus 4 floats (a multiple of 16 bytes that
+// Row sums over a whole score row: acc = sum over keys [0, nkeys) of w[row][key] * x[key][c0 ..], keys ascending, 32
+// keys at a time through the two chunk buffers at `xt`.  Ends with a barrier.
+template <bool kFused, int RM, bool kVec>
+__device__ __forceinline__ void RowSum(const float* w, int ld, const float* __restrict__ x, size_t stride, int nkeys, int S,
+                                       int c0, int d, const int (&row_lo)[RM], const int (&row_hi)[RM], int all_below,
+                                       float* xt, float (&acc)[RM][4]) {
+  int buf = 0;
+  CopyChunk<kVec>(xt, x, stride, min(kChunkRows, S), c0, d);
+  for (int k0 = 0; k0 < nkeys; k0 += kChunkRows, buf ^= 1) {
+    if (k0 + kChunkRows < nkeys) {
+      CopyChunk<kVec>(xt + (buf ^ 1) * (kChunkRows * kTile), x + static_cast<size_t>(k0 + kChunkRows) * stride, stride,
+                      min(kChunkRows, S - k0 - kChunkRows), c0, d);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    int lo[RM], hi[RM];
+#pragma unroll
+    for (int r = 0; r < RM; ++r) { lo[r] = row_lo[r] - k0; hi[r] = row_hi[r] - k0; }
+    const float* xs = xt + buf * (kChunkRows * kTile);
+    if (k0 + kChunkRows <= all_below) RowProduct<kFused, RM, true>(w + k0, ld, xs, lo, hi, acc);
+    else RowProduct<kFused, RM, false>(w + k0, ld, xs, lo, hi, acc);
+    __syncthreads();   // the buffer is refilled two chunks on
+  }
+}
+
+// In the output sums all 256 threads share the block's rows: OutRows(RM) each, 16 groups of 16 column quads.
+__host__ __device__ constexpr int OutRows(int RM) { return RM > 1 ? RM / 2 : 1; }
+
+// Score rows are stored with a stride of a whole number of tiles plus 4 floats (a multiple of 16 bytes that
 // puts a thread column's rows in different banks).
 __host__ __device__ constexpr size_t RowStride(size_t S) { return (S + kTile - 1) / kTile * kTile + 4; }
 
@@ -354,34 +422,42 @@ __device__ __forceinline__ TileAt KeyTile(int BH) {
   return {static_cast<int>(blockIdx.x) / BH, static_cast<size_t>(static_cast<int>(blockIdx.x) % BH)};
 }
 
-// Forward.  Block: 16 RM query rows of one (sequence, head).  Score rows of the whole block stay in shared memory between the three phases.
-template <int RM, bool kVec>
+// Forward.  Block: 8 RM query rows of one (sequence, head).  Score rows of the whole block stay in shared memory
+// between the three phases.
+template <int RM, bool kFused, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnFwdTileKernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, float* __restrict__ o,
     float* __restrict__ probs, float* __restrict__ stats, int BH, int S, int H, int d,
     const int32_t* __restrict__ starts, float inv_sqrt_d) {
   extern __shared__ __align__(16) uint8_t raw[];
-  constexpr int R = 16 * RM;
-  double* sa = reinterpret_cast<double*>(raw);
-  double* sb = sa + kSlice * R;
-  float* xt = reinterpret_cast<float*>(sb);                       // the V tile, where the K slice was
-  float* rows = reinterpret_cast<float*>(raw + SliceBytes(RM));
+  constexpr int R = 8 * RM;
+  double* slices = reinterpret_cast<double*>(raw + GroupOf() * GroupBytes());
+  float* xt = reinterpret_cast<float*>(raw);                       // the V chunks, where the K slices were
+  double* own = reinterpret_cast<double*>(raw + StreamBytes());
+  float* rows = reinterpret_cast<float*>(raw + StreamBytes() + OwnBytes(RM, d));
   const int ld = static_cast<int>(RowStride(S));
   const TileAt tile = QueryTile((S + R - 1) / R, BH);
   const int i0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const int nrows = min(R, S - i0), nkeys = min(i0 + R, S);
-  const int ty = threadIdx.x >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ty = InGroup() >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t base = b * S * D + h * d;
   auto first_key = [&](int i) {
     if (!starts) return 0;
     const int32_t s0 = starts[b * S + i];
     return s0 <= 0 ? 0 : (s0 < i ? static_cast<int>(s0) : i);
   };
-  for (int k0 = 0; k0 < nkeys; k0 += kTile) {
+  SliceRegs regs;
+  int turn = 0;
+  const int first = GroupOf() * kTile;
+  if (first < nkeys) FetchSlice<kVec>(&regs, k + base + static_cast<size_t>(first) * D, D, min(kTile, S - first), 0, d);
+  LoadOwn<R, kVec>(own, q + base + static_cast<size_t>(i0) * D, D, nrows, d);
+  __syncthreads();
+  for (int k0 = first; k0 < nkeys; k0 += 2 * kTile) {
     double acc[RM][4];
-    DotTile<RM, kVec>(q + base + static_cast<size_t>(i0) * D, nrows, k + base + static_cast<size_t>(k0) * D,
-                      min(kTile, S - k0), D, d, sa, sb, acc);
+    const float* kb = k + base + static_cast<size_t>(k0) * D;
+    DotTile<RM, kVec>(own, kb, min(kTile, S - k0), k0 + 2 * kTile < nkeys ? kb + 2 * kTile * D : nullptr,
+                      min(kTile, S - k0 - 2 * kTile), D, d, slices, &turn, &regs, acc);
 #pragma unroll
     for (int r = 0; r < RM; ++r)
 #pragma unroll
@@ -419,116 +495,148 @@ __global__ __launch_bounds__(kTileThreads) void AttnFwdTileKernel(
       st[3] = static_cast<float>(j0);
     }
   }
-  const int c = (threadIdx.x & 15) * 4;
-  int row_lo[RM], row_hi[RM];
+  __syncthreads();
+  constexpr int OR = OutRows(RM);
+  const int r0 = (threadIdx.x >> 4) * OR;   // this thread's rows of the output sums
+  int row_lo[OR], row_hi[OR];
 #pragma unroll
-  for (int r = 0; r < RM; ++r) {
-    const int i = min(i0 + ty * RM + r, S - 1);
+  for (int r = 0; r < OR; ++r) {
+    const int i = min(i0 + r0 + r, S - 1);
     row_lo[r] = first_key(i);
     row_hi[r] = i + 1;
   }
   for (int c0 = 0; c0 < d; c0 += kTile) {
-    float acc[RM][4];
+    float acc[OR][4] = {};
+    RowSum<kFused, OR, kVec>(rows + min(r0, R - OR) * ld, ld, v + base, D, nkeys, S, c0, d, row_lo, row_hi,
+                             starts ? 0 : i0 + 1, xt, acc);
 #pragma unroll
-    for (int r = 0; r < RM; ++r)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[r][e] = 0.0f;
-    for (int k0 = 0; k0 < nkeys; k0 += kTile) {
-      __syncthreads();
-      LoadTileF<kVec>(xt, v + base + static_cast<size_t>(k0) * D, D, min(kTile, S - k0), c0, d);
-      __syncthreads();
-      int lo[RM], hi[RM];
-#pragma unroll
-      for (int r = 0; r < RM; ++r) { lo[r] = row_lo[r] - k0; hi[r] = row_hi[r] - k0; }
-      if (!starts && k0 + kTile <= i0 + 1)
-        RowProduct<RM, true>(rows + ty * RM * ld + k0, ld, xt, lo, hi, acc);
-      else
-        RowProduct<RM, false>(rows + ty * RM * ld + k0, ld, xt, lo, hi, acc);
-    }
-#pragma unroll
-    for (int r = 0; r < RM; ++r)
-      if (ty * RM + r < nrows)
-        StoreRow4(o + base + static_cast<size_t>(i0 + ty * RM + r) * D, acc[r], c0 + c, d, kVec);
+    for (int r = 0; r < OR; ++r)
+      if (r0 + r < nrows)
+        StoreRow4(o + base + static_cast<size_t>(i0 + r0 + r) * D, acc[r], c0 + (threadIdx.x & 15) * 4, d, kVec);
   }
 }
 
-// dP[i][j] = dO_i . v_j for j <= i, zero above the diagonal.  Block: one 64 x 64 tile.
-template <bool kVec>
+// dP for a head too wide for a tile block's own rows: a thread per pair.
+__global__ void AttnDPWideKernel(const float* __restrict__ dout, const float* __restrict__ v, float* __restrict__ dp,
+                                 size_t BH, size_t S, size_t H, size_t d) {
+  const size_t pairs = BH * S * S, D = H * d;
+  for (size_t t = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; t < pairs;
+       t += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    const size_t j = t % S, i = t / S % S, bh = t / (S * S), at = bh / H * S * D + bh % H * d;
+    dp[t] = j <= i ? static_cast<float>(DotD(dout + at + i * D, v + at + j * D, d)) : 0.0f;
+  }
+}
+
+// dP[i][j] = dO_i . v_j for j <= i, zero above the diagonal.  Block: 8 RM query rows, every key tile.
+template <int RM, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __restrict__ dout,
                                                                  const float* __restrict__ v, float* __restrict__ dp,
                                                                  int BH, int S, int H, int d) {
   extern __shared__ __align__(16) uint8_t raw[];
-  double* sa = reinterpret_cast<double*>(raw);
-  double* sb = sa + kSlice * kTile;
-  const TileAt tile = KeyTile(BH);
-  const int tiles = (S + kTile - 1) / kTile, k0 = tile.tile % tiles * kTile, i0 = tile.tile / tiles * kTile;
+  constexpr int R = 8 * RM;
+  double* slices = reinterpret_cast<double*>(raw + GroupOf() * GroupBytes());
+  double* own = reinterpret_cast<double*>(raw + StreamBytes());
+  const TileAt tile = QueryTile((S + R - 1) / R, BH);
+  const int i0 = tile.tile * R, nkeys = min(i0 + R, S);
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const size_t base = b * S * D + h * d;
-  const int ty = threadIdx.x >> 4;
-  double acc[4][4] = {};
-  if (k0 <= i0)
-    DotTile<4, kVec>(dout + base + static_cast<size_t>(i0) * D, min(kTile, S - i0),
-                     v + base + static_cast<size_t>(k0) * D, min(kTile, S - k0), D, d, sa, sb, acc);
+  const int ty = InGroup() >> 4;
+  SliceRegs regs;
+  int turn = 0;
+  const int first = GroupOf() * kTile;
+  if (first < nkeys) FetchSlice<kVec>(&regs, v + base + static_cast<size_t>(first) * D, D, min(kTile, S - first), 0, d);
+  LoadOwn<R, kVec>(own, dout + base + static_cast<size_t>(i0) * D, D, min(R, S - i0), d);
+  __syncthreads();
+  for (int k0 = first; k0 < S; k0 += 2 * kTile) {
+    double acc[RM][4] = {};
+    if (k0 < nkeys) {
+      const float* vb = v + base + static_cast<size_t>(k0) * D;
+      DotTile<RM, kVec>(own, vb, min(kTile, S - k0), k0 + 2 * kTile < nkeys ? vb + 2 * kTile * D : nullptr,
+                        min(kTile, S - k0 - 2 * kTile), D, d, slices, &turn, &regs, acc);
+    }
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ty * 4 + r;
-    if (i >= S) continue;
-    float* row = dp + (bh * S + i) * S;
+    for (int r = 0; r < RM; ++r) {
+      const int i = i0 + ty * RM + r;
+      if (i >= S) continue;
+      float* row = dp + (bh * S + i) * S;
 #pragma unroll
-    for (int e = 0; e < 4; e += 2) {
-      const int j = k0 + Col(e);
-      const float x0 = j <= i ? static_cast<float>(acc[r][e]) : 0.0f;
-      const float x1 = j + 1 <= i ? static_cast<float>(acc[r][e + 1]) : 0.0f;
-      if ((S & 1) == 0 && j + 1 < S) {
-        *reinterpret_cast<float2*>(row + j) = make_float2(x0, x1);
-      } else {
-        if (j < S) row[j] = x0;
-        if (j + 1 < S) row[j + 1] = x1;
+      for (int e = 0; e < 4; e += 2) {
+        const int j = k0 + Col(e);
+        const float x0 = j <= i ? static_cast<float>(acc[r][e]) : 0.0f;
+        const float x1 = j + 1 <= i ? static_cast<float>(acc[r][e + 1]) : 0.0f;
+        if ((S & 1) == 0 && j + 1 < S) {
+          *reinterpret_cast<float2*>(row + j) = make_float2(x0, x1);
+        } else {
+          if (j < S) row[j] = x0;
+          if (j + 1 < S) row[j + 1] = x1;
+        }
       }
     }
   }
 }
 
 // dQ_i[c] = sum over j <= i of (dS[i][j] / sqrt(d)) k_j[c].  Block: 16 RM rows, 64 columns of the head.
-template <int RM, bool kVec>
+template <int RM, bool kFused, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnRowTileKernel(const float* __restrict__ ds,
                                                                   const float* __restrict__ k, float* __restrict__ dq,
                                                                   int BH, int S, int H, int d, float inv_sqrt_d) {
-  constexpr int R = 16 * RM, kLd = kTile + 4;
-  __shared__ __align__(16) float xt[kTile * kTile];
-  __shared__ __align__(16) float wt[R * kLd];
+  constexpr int R = 16 * RM, kLd = kChunkRows + 4;
+  __shared__ __align__(16) float xt[2 * kChunkRows * kTile];
+  __shared__ __align__(16) float wt[2 * R * kLd];
   const TileAt tile = QueryTile((S + R - 1) / R, BH);
   const int i0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const size_t base = b * S * D + h * d;
   const int c0 = blockIdx.y * kTile, ty = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
   const int nkeys = min(i0 + R, S);
+  constexpr int kPer = R * kChunkRows / kTileThreads;   // weights a thread carries for the next chunk
+  float w[kPer];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      const int idx = static_cast<int>(threadIdx.x) + t * kTileThreads, r = idx / kChunkRows, j = idx % kChunkRows;
+      w[t] = i0 + r < S && k0 + j < S ? ds[(bh * S + i0 + r) * S + k0 + j] : 0.0f;
+    }
+  };
   float acc[RM][4] = {};
-  for (int k0 = 0; k0 < nkeys; k0 += kTile) {
-    __syncthreads();
-    LoadTileF<kVec>(xt, k + base + static_cast<size_t>(k0) * D, D, min(kTile, S - k0), c0, d);
-    for (int t = threadIdx.x; t < R * kTile; t += kTileThreads) {
-      const int r = t / kTile, j = t % kTile;
-      wt[r * kLd + j] = i0 + r < S && k0 + j < S ? ds[(bh * S + i0 + r) * S + k0 + j] * inv_sqrt_d : 0.0f;
+  fetch(0);
+  CopyChunk<kVec>(xt, k + base, D, min(kChunkRows, S), c0, d);
+  int buf = 0;
+  for (int k0 = 0; k0 < nkeys; k0 += kChunkRows, buf ^= 1) {
+    float* ws = wt + buf * (R * kLd);
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      const int idx = static_cast<int>(threadIdx.x) + t * kTileThreads;
+      ws[idx / kChunkRows * kLd + idx % kChunkRows] = w[t] * inv_sqrt_d;
+    }
+    if (k0 + kChunkRows < nkeys) {
+      fetch(k0 + kChunkRows);
+      CopyChunk<kVec>(xt + (buf ^ 1) * (kChunkRows * kTile), k + base + static_cast<size_t>(k0 + kChunkRows) * D, D,
+                      min(kChunkRows, S - k0 - kChunkRows), c0, d);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
     int lo[RM], hi[RM];
 #pragma unroll
     for (int r = 0; r < RM; ++r) { lo[r] = 0; hi[r] = i0 + ty * RM + r + 1 - k0; }
-    if (k0 + kTile <= i0 + 1) RowProduct<RM, true>(wt + ty * RM * kLd, kLd, xt, lo, hi, acc);
-    else RowProduct<RM, false>(wt + ty * RM * kLd, kLd, xt, lo, hi, acc);
+    const float* xs = xt + buf * (kChunkRows * kTile);
+    if (k0 + kChunkRows <= i0 + 1) RowProduct<kFused, RM, true>(ws + ty * RM * kLd, kLd, xs, lo, hi, acc);
+    else RowProduct<kFused, RM, false>(ws + ty * RM * kLd, kLd, xs, lo, hi, acc);
+    __syncthreads();   // xs is refilled two chunks on
   }
 #pragma unroll
   for (int r = 0; r < RM; ++r)
     if (i0 + ty * RM + r < S) StoreRow4(dq + base + static_cast<size_t>(i0 + ty * RM + r) * D, acc[r], c0 + c, d, kVec);
 }
 
-// acc[r][e] += w[i][ty RM + r] x[i][c + e] for i = 0 .. rows - 1 in order, where query i reaches key row r:
-// i >= lo[r], and key[r] >= start[i] when there are segment starts (kAll: every i reaches every key).
-template <int RM, bool kAll>
+// acc[r][e] += w[i][r] x[i][c + e] for i = 0 .. rows - 1 in order (w at this thread's first key), where query i reaches
+// key r: i >= lo[r], and key + r >= start[i] when there are segment starts (kAll: every i reaches every key).
+template <bool kFused, int RM, bool kAll>
 __device__ __forceinline__ void ColProduct(const float* w, int ldw, const float* x, int rows, const int (&lo)[RM],
                                            float (&acc)[RM][4], const int* start = nullptr, int key = 0) {
-  const int c = (threadIdx.x & 15) * 4, ty = threadIdx.x >> 4;
+  const int c = (threadIdx.x & 15) * 4;
 #pragma unroll 4
   for (int i = 0; i < rows; ++i) {
     const float4 f = *reinterpret_cast<const float4*>(x + i * kTile + c);
@@ -536,45 +644,62 @@ __device__ __forceinline__ void ColProduct(const float* w, int ldw, const float*
     const int first = kAll || !start ? 0 : start[i];
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
-      const float g = w[i * ldw + ty * RM + r];
+      const float g = w[i * ldw + r];
       if (kAll || (i >= lo[r] && key + r >= first)) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[r][e] += g * xv[e];
+        for (int e = 0; e < 4; ++e) acc[r][e] = MulAdd<kFused>(g, xv[e], acc[r][e]);
       }
     }
   }
 }
 
 // out_j[c] = sum over i >= j of w[i][j] (scale) x_i[c], i ascending.  Block: 16 RM keys, 64 columns.
-template <int RM, bool kScaled, bool kVec>
+template <int RM, bool kFused, bool kScaled, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnColTileKernel(const float* __restrict__ w,
                                                                   const float* __restrict__ x, float* __restrict__ out,
                                                                   int BH, int S, int H, int d, float inv_sqrt_d) {
   constexpr int R = 16 * RM;
-  __shared__ __align__(16) float xt[kTile * kTile];
-  __shared__ __align__(16) float wt[kTile * R];
+  __shared__ __align__(16) float xt[2 * kChunkRows * kTile];
+  __shared__ __align__(16) float wt[2 * kChunkRows * R];
   const TileAt tile = KeyTile(BH);
   const int j0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const size_t base = b * S * D + h * d;
   const int c0 = blockIdx.y * kTile, ty = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
+  constexpr int kPer = R * kChunkRows / kTileThreads;
+  float g[kPer];
+  auto fetch = [&](int i0) {
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      const int idx = static_cast<int>(threadIdx.x) + t * kTileThreads, i = idx / R, j = idx % R;
+      g[t] = i0 + i < S && j0 + j < S ? w[(bh * S + i0 + i) * S + j0 + j] : 0.0f;
+    }
+  };
   float acc[RM][4] = {};
-  for (int i0 = j0; i0 < S; i0 += kTile) {
-    const int rows = min(kTile, S - i0);
-    __syncthreads();
-    LoadTileF<kVec>(xt, x + base + static_cast<size_t>(i0) * D, D, rows, c0, d);
-    for (int t = threadIdx.x; t < kTile * R; t += kTileThreads) {
-      const int i = t / R, j = t % R;
-      float g = i < rows && j0 + j < S ? w[(bh * S + i0 + i) * S + j0 + j] : 0.0f;
-      if (kScaled) g = g * inv_sqrt_d;
-      wt[t] = g;
+  fetch(j0);
+  CopyChunk<kVec>(xt, x + base + static_cast<size_t>(j0) * D, D, min(kChunkRows, S - j0), c0, d);
+  int buf = 0;
+  for (int i0 = j0; i0 < S; i0 += kChunkRows, buf ^= 1) {
+    float* ws = wt + buf * (kChunkRows * R);
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) ws[threadIdx.x + t * kTileThreads] = kScaled ? g[t] * inv_sqrt_d : g[t];
+    if (i0 + kChunkRows < S) {
+      fetch(i0 + kChunkRows);
+      CopyChunk<kVec>(xt + (buf ^ 1) * (kChunkRows * kTile), x + base + static_cast<size_t>(i0 + kChunkRows) * D, D,
+                      min(kChunkRows, S - i0 - kChunkRows), c0, d);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
     int lo[RM];
 #pragma unroll
     for (int r = 0; r < RM; ++r) lo[r] = j0 + ty * RM + r - i0;
-    if (i0 >= j0 + R - 1) ColProduct<RM, true>(wt, R, xt, rows, lo, acc);
-    else ColProduct<RM, false>(wt, R, xt, rows, lo, acc);
+    const float* xs = xt + buf * (kChunkRows * kTile);
+    const int rows = min(kChunkRows, S - i0);
+    if (i0 >= j0 + R - 1) ColProduct<kFused, RM, true>(ws + ty * RM, R, xs, rows, lo, acc);
+    else ColProduct<kFused, RM, false>(ws + ty * RM, R, xs, rows, lo, acc);
+    __syncthreads();
   }
 #pragma unroll
   for (int r = 0; r < RM; ++r)
@@ -583,30 +708,39 @@ __global__ __launch_bounds__(kTileThreads) void AttnColTileKernel(const float* _
 
 // Tiled dQ: the rows' probabilities and dP recomputed into shared memory, delta written into the stats rows,
 // then dQ (reference: runtime/executor/attention.cc:492-531).
-template <int RM, bool kVec>
+template <int RM, bool kFused, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnDQTiledTileKernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
     const float* __restrict__ dout, float* __restrict__ stats, float* __restrict__ dq, int BH, int S, int H,
     int d, float inv_sqrt_d) {
   extern __shared__ __align__(16) uint8_t raw[];
-  constexpr int R = 16 * RM;
-  double* sa = reinterpret_cast<double*>(raw);
-  double* sb = sa + kSlice * R;
-  float* xt = reinterpret_cast<float*>(sb);
+  constexpr int R = 8 * RM;
+  double* slices = reinterpret_cast<double*>(raw + GroupOf() * GroupBytes());
+  float* xt = reinterpret_cast<float*>(raw);
+  double* own_q = reinterpret_cast<double*>(raw + StreamBytes());
+  double* own_do = reinterpret_cast<double*>(raw + StreamBytes() + OwnBytes(RM, d));
   const int ld = static_cast<int>(RowStride(S));
-  float* prows = reinterpret_cast<float*>(raw + SliceBytes(RM));
+  float* prows = reinterpret_cast<float*>(raw + StreamBytes() + 2 * OwnBytes(RM, d));
   float* dprows = prows + R * ld;
   const TileAt tile = QueryTile((S + R - 1) / R, BH);
   const int i0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const int nrows = min(R, S - i0), nkeys = min(i0 + R, S);
-  const int ty = threadIdx.x >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ty = InGroup() >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t base = b * S * D + h * d, at = base + static_cast<size_t>(i0) * D;
   float* st = stats + (bh * S + i0) * kAttnStatsWidth;
-  for (int k0 = 0; k0 < nkeys; k0 += kTile) {
-    const size_t kat = base + static_cast<size_t>(k0) * D;
+  SliceRegs regs;
+  int turn = 0;
+  const int first = GroupOf() * kTile;
+  if (first < nkeys) FetchSlice<kVec>(&regs, k + base + static_cast<size_t>(first) * D, D, min(kTile, S - first), 0, d);
+  LoadOwn<R, kVec>(own_q, q + at, D, nrows, d);
+  LoadOwn<R, kVec>(own_do, dout + at, D, nrows, d);
+  __syncthreads();
+  for (int k0 = first; k0 < nkeys; k0 += 2 * kTile) {
+    const float *kb = k + base + static_cast<size_t>(k0) * D, *vb = v + base + static_cast<size_t>(k0) * D;
+    const int rows = min(kTile, S - k0);
     double acc[RM][4];
-    DotTile<RM, kVec>(q + at, nrows, k + kat, min(kTile, S - k0), D, d, sa, sb, acc);
+    DotTile<RM, kVec>(own_q, kb, rows, vb, rows, D, d, slices, &turn, &regs, acc);
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
       const int row = min(ty * RM + r, nrows - 1);
@@ -615,7 +749,8 @@ __global__ __launch_bounds__(kTileThreads) void AttnDQTiledTileKernel(
       for (int e = 0; e < 4; ++e)
         prows[(ty * RM + r) * ld + k0 + Col(e)] = expf(static_cast<float>(acc[r][e]) * inv_sqrt_d - m) * inv_denom;
     }
-    DotTile<RM, kVec>(dout + at, nrows, v + kat, min(kTile, S - k0), D, d, sa, sb, acc);
+    DotTile<RM, kVec>(own_do, vb, rows, k0 + 2 * kTile < nkeys ? kb + 2 * kTile * D : nullptr, min(kTile, S - k0 - 2 * kTile), D, d,
+                      slices, &turn, &regs, acc);
 #pragma unroll
     for (int r = 0; r < RM; ++r)
 #pragma unroll
@@ -635,97 +770,117 @@ __global__ __launch_bounds__(kTileThreads) void AttnDQTiledTileKernel(
       prow[j] = dsv * inv_sqrt_d;
     }
   }
-  const int c = (threadIdx.x & 15) * 4;
-  int row_lo[RM], row_hi[RM];
+  __syncthreads();
+  constexpr int OR = OutRows(RM);
+  const int r0 = (threadIdx.x >> 4) * OR;
+  int row_lo[OR], row_hi[OR];
   bool whole = true;
 #pragma unroll
-  for (int r = 0; r < RM; ++r) {
-    const int row = min(ty * RM + r, nrows - 1);
+  for (int r = 0; r < OR; ++r) {
+    const int row = min(r0 + r, nrows - 1);
     row_lo[r] = static_cast<int>(StatsStart(st[row * kAttnStatsWidth + 3], i0 + row));
     row_hi[r] = i0 + row + 1;
     whole = whole && row_lo[r] == 0;
   }
   for (int c0 = 0; c0 < d; c0 += kTile) {
-    float acc[RM][4] = {};
-    for (int k0 = 0; k0 < nkeys; k0 += kTile) {
-      __syncthreads();
-      LoadTileF<kVec>(xt, k + base + static_cast<size_t>(k0) * D, D, min(kTile, S - k0), c0, d);
-      __syncthreads();
-      int lo[RM], hi[RM];
+    float acc[OR][4] = {};
+    RowSum<kFused, OR, kVec>(prows + min(r0, R - OR) * ld, ld, k + base, D, nkeys, S, c0, d, row_lo, row_hi,
+                             whole ? i0 + 1 : 0, xt, acc);
 #pragma unroll
-      for (int r = 0; r < RM; ++r) { lo[r] = row_lo[r] - k0; hi[r] = row_hi[r] - k0; }
-      if (whole && k0 + kTile <= i0 + 1) RowProduct<RM, true>(prows + ty * RM * ld + k0, ld, xt, lo, hi, acc);
-      else RowProduct<RM, false>(prows + ty * RM * ld + k0, ld, xt, lo, hi, acc);
-    }
-#pragma unroll
-    for (int r = 0; r < RM; ++r)
-      if (ty * RM + r < nrows) StoreRow4(dq + at + static_cast<size_t>(ty * RM + r) * D, acc[r], c0 + c, d, kVec);
+    for (int r = 0; r < OR; ++r)
+      if (r0 + r < nrows)
+        StoreRow4(dq + at + static_cast<size_t>(r0 + r) * D, acc[r], c0 + (threadIdx.x & 15) * 4, d, kVec);
   }
 }
 
-// Tiled dK (kWantDK) or dV over the query rows i >= j of 16 RM keys, 64 columns of the head per block (a wider
-// head repeats the scores; reference: runtime/executor/attention.cc:533-590).
-template <int RM, bool kWantDK, bool kVec>
+// Tiled dK (kWantDK) or dV over the query rows i >= j of 8 RM keys, 64 columns of the head per block (a wider
+// head repeats the scores; reference: runtime/executor/attention.cc:533-590).  The groups form the weights of two query
+// tiles at a time, then all threads add both, the earlier tile first.
+template <int RM, bool kWantDK, bool kFused, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnDKVTiledTileKernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
     const float* __restrict__ dout, const float* __restrict__ stats, float* __restrict__ out, int BH, int S, int H,
     int d, float inv_sqrt_d) {
   extern __shared__ __align__(16) uint8_t raw[];
-  constexpr int R = 16 * RM, kLd = R + 4;
-  double* sa = reinterpret_cast<double*>(raw);
-  double* sb = sa + kSlice * R;
-  float* xt = reinterpret_cast<float*>(sb);
-  float* wt = reinterpret_cast<float*>(raw + SliceBytes(RM));   // [64 queries][R keys]
-  __shared__ int first[kTile];                                   // the first key each query reaches
+  constexpr int R = 8 * RM, kLd = R + 4;
+  const int group = GroupOf();
+  double* slices = reinterpret_cast<double*>(raw + group * GroupBytes());
+  double* own_k = reinterpret_cast<double*>(raw + StreamBytes());
+  double* own_v = reinterpret_cast<double*>(raw + StreamBytes() + OwnBytes(RM, d));
+  float* xt = reinterpret_cast<float*>(raw + StreamBytes() + (kWantDK ? 2 : 1) * OwnBytes(RM, d));   // [128 queries][64]
+  float* wt = xt + 2 * kTile * kTile;                                                                 // [128 queries][kLd]
+  __shared__ int first[2 * kTile];   // the first key each query reaches
   const TileAt tile = KeyTile(BH);
   const int j0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const size_t base = b * S * D + h * d, at = base + static_cast<size_t>(j0) * D;
-  const int c0 = blockIdx.y * kTile, ty = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
+  const int c0 = blockIdx.y * kTile, ty = InGroup() >> 4, c = (threadIdx.x & 15) * 4;
   const int nkeys = min(R, S - j0);
-  float acc[RM][4] = {};
-  for (int i0 = j0 / kTile * kTile; i0 < S; i0 += kTile) {
-    const int rows = min(kTile, S - i0);
-    const size_t iat = base + static_cast<size_t>(i0) * D;
-    double sc[RM][4], dp[RM][4];
-    DotTile<RM, kVec>(k + at, nkeys, q + iat, rows, D, d, sa, sb, sc);
-    if (kWantDK) DotTile<RM, kVec>(v + at, nkeys, dout + iat, rows, D, d, sa, sb, dp);
-    __syncthreads();
-    LoadTileF<kVec>(xt, (kWantDK ? q : dout) + iat, D, rows, c0, d);
+  const float* x = kWantDK ? q : dout;
+  constexpr int OR = OutRows(RM);
+  const int r0 = (threadIdx.x >> 4) * OR, r_at = min(r0, R - OR);   // this thread's keys of the output sums
+  float acc[OR][4] = {};
+  SliceRegs regs;
+  int turn = 0;
+  const int i_first = j0 / kTile * kTile, mine = i_first + group * kTile;
+  if (mine < S) FetchSlice<kVec>(&regs, q + base + static_cast<size_t>(mine) * D, D, min(kTile, S - mine), 0, d);
+  LoadOwn<R, kVec>(own_k, k + at, D, nkeys, d);
+  if (kWantDK) LoadOwn<R, kVec>(own_v, v + at, D, nkeys, d);
+  __syncthreads();
+  for (int pair = i_first; pair < S; pair += 2 * kTile) {
+    // The rows of x these tiles need, on their way while the scores are formed.
+    for (int t = 0; t < 2 * kTile; t += kChunkRows) {
+      const int rows = min(kChunkRows, S - pair - t);
+      CopyChunk<kVec>(xt + t * kTile, x + base + static_cast<size_t>(rows > 0 ? pair + t : pair) * D, D, max(0, rows), c0, d);
+    }
+    const int i0 = pair + group * kTile;
     bool late = false;
+    if (i0 < S) {
+      const int rows = min(kTile, S - i0);
+      const size_t iat = base + static_cast<size_t>(i0) * D;
+      const float* q_next = i0 + 2 * kTile < S ? q + iat + 2 * kTile * D : nullptr;
+      const int next_rows = min(kTile, S - i0 - 2 * kTile);
+      double sc[RM][4], dp[RM][4];
+      DotTile<RM, kVec>(own_k, q + iat, rows, kWantDK ? dout + iat : q_next, kWantDK ? rows : next_rows, D, d, slices, &turn,
+                        &regs, sc);
+      if (kWantDK) DotTile<RM, kVec>(own_v, dout + iat, rows, q_next, next_rows, D, d, slices, &turn, &regs, dp);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = i0 + Col(e);
-      const float* st = stats + (bh * S + min(i, S - 1)) * kAttnStatsWidth;
-      const int start = static_cast<int>(StatsStart(st[3], static_cast<size_t>(i)));
-      late = late || (i < S && start > j0);
-      if (ty == 0) first[Col(e)] = start;
+      for (int e = 0; e < 4; ++e) {
+        const int i = i0 + Col(e);
+        const float* st = stats + (bh * S + min(i, S - 1)) * kAttnStatsWidth;
+        const int start = static_cast<int>(StatsStart(st[3], static_cast<size_t>(i)));
+        late = late || (i < S && start > j0);
+        if (ty == 0) first[group * kTile + Col(e)] = start;
 #pragma unroll
-      for (int r = 0; r < RM; ++r) {
-        const int j = j0 + ty * RM + r;
-        float g = 0.0f;
-        if (i < S && j <= i && j >= start) {
-          const float p = expf(static_cast<float>(sc[r][e]) * inv_sqrt_d - st[0]) * st[1];
-          if (kWantDK) {
-            const float dsv = p * (static_cast<float>(dp[r][e]) - st[2]);
-            g = dsv * inv_sqrt_d;
-          } else {
-            g = p;
+        for (int r = 0; r < RM; ++r) {
+          const int j = j0 + ty * RM + r;
+          float g = 0.0f;
+          if (i < S && j <= i && j >= start) {
+            const float p = expf(static_cast<float>(sc[r][e]) * inv_sqrt_d - st[0]) * st[1];
+            if (kWantDK) {
+              const float dsv = p * (static_cast<float>(dp[r][e]) - st[2]);
+              g = dsv * inv_sqrt_d;
+            } else {
+              g = p;
+            }
           }
+          wt[(group * kTile + Col(e)) * kLd + ty * RM + r] = g;
         }
-        wt[Col(e) * kLd + ty * RM + r] = g;
       }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     const bool segments = __syncthreads_or(late);
-    int lo[RM];
+    const int rows = min(2 * kTile, S - pair);
+    int lo[OR];
 #pragma unroll
-    for (int r = 0; r < RM; ++r) lo[r] = j0 + ty * RM + r - i0;
-    if (i0 >= j0 + R - 1 && !segments) ColProduct<RM, true>(wt, kLd, xt, rows, lo, acc);
-    else ColProduct<RM, false>(wt, kLd, xt, rows, lo, acc, first, j0 + ty * RM);
+    for (int r = 0; r < OR; ++r) lo[r] = j0 + r_at + r - pair;
+    if (pair >= j0 + R - 1 && !segments) ColProduct<kFused, OR, true>(wt + r_at, kLd, xt, rows, lo, acc);
+    else ColProduct<kFused, OR, false>(wt + r_at, kLd, xt, rows, lo, acc, first, j0 + r_at);
+    __syncthreads();   // wt, xt and first are rewritten for the next pair
   }
 #pragma unroll
-  for (int r = 0; r < RM; ++r)
-    if (ty * RM + r < nkeys) StoreRow4(out + at + static_cast<size_t>(ty * RM + r) * D, acc[r], c0 + c, d, kVec);
+  for (int r = 0; r < OR; ++r)
+    if (r0 + r < nkeys) StoreRow4(out + at + static_cast<size_t>(r0 + r) * D, acc[r], c0 + c, d, kVec);
 }
 
 inline unsigned UnitBlocks(size_t units) {
@@ -749,20 +904,22 @@ namespace {
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kTwoPerSm = 113 * 1024;
 
-// 16 RM rows per block: four rows per thread (the most arithmetic per shared-memory read) while the grid still has
-// four blocks per SM, else two while it has two, else one.
-inline int RowsPerThread(size_t BH, size_t S, size_t chunks = 1) {
+// Rows per thread (per_rm of them times 16 or 8 to a block): four, the most arithmetic per shared-memory read, while
+// the grid still has two blocks per SM, else two while it has one, else one.
+inline int RowsPerThread(size_t BH, size_t S, int rows_per_rm, size_t chunks = 1) {
   for (int rm : {4, 2})
-    if (BH * ((S + 16 * rm - 1) / (16 * rm)) * chunks >= (rm == 4 ? 4u : 2u) * 148u) return rm;
+    if (BH * ((S + rows_per_rm * rm - 1) / (rows_per_rm * rm)) * chunks >= (rm == 4 ? 2u : 1u) * 148u) return rm;
   return 1;
 }
-// The same for the kernels whose score rows (`arrays` f32 rows of S keys per query row) live in shared memory: no more
-// rows than let two blocks share an SM, or one block of 16 rows; 0: not even that fits.
-inline int RowsPerThreadWithScores(size_t BH, size_t S, int arrays) {
-  auto bytes = [&](int rm) { return SliceBytes(rm) + static_cast<size_t>(arrays) * 16 * rm * RowStride(S) * sizeof(float); };
-  for (int rm = RowsPerThread(BH, S); rm >= 1; rm /= 2)
-    if (bytes(rm) <= kTwoPerSm) return rm;
-  return bytes(1) <= kMaxSmem ? 1 : 0;
+// The same for the kernels whose score rows (`arrays` f32 rows of S keys, and as many own operands, per query row) live
+// in shared memory: no more rows than let two blocks share an SM, or one block of 8 rows; 0: not even that fits.
+inline size_t ScoreBytes(int rm, size_t S, size_t d, int arrays) {
+  return StreamBytes() + static_cast<size_t>(arrays) * (OwnBytes(rm, static_cast<int>(d)) + 8 * rm * RowStride(S) * sizeof(float));
+}
+inline int RowsPerThreadWithScores(size_t BH, size_t S, size_t d, int arrays) {
+  for (int rm = RowsPerThread(BH, S, 8); rm >= 1; rm /= 2)
+    if (ScoreBytes(rm, S, d, arrays) <= kTwoPerSm) return rm;
+  return ScoreBytes(1, S, d, arrays) <= kMaxSmem ? 1 : 0;
 }
 inline bool Vec(size_t d, std::initializer_list<const void*> ps) {
   if (d % 4 != 0) return false;
@@ -772,16 +929,20 @@ inline bool Vec(size_t d, std::initializer_list<const void*> ps) {
 }
 template <int RM>
 using RowsTag = std::integral_constant<int, RM>;
-// f(rows tag, vector tag) with the constants of this launch.
+// f(rows tag, fused tag, vector tag) with the constants of this launch.
 template <typename F>
-inline void WithTile(int rm, bool vec, F f) {
-  auto with_rows = [&](auto v) {
-    if (rm == 4) f(RowsTag<4>{}, v);
-    else if (rm == 2) f(RowsTag<2>{}, v);
-    else f(RowsTag<1>{}, v);
+inline void WithTile(int rm, bool fused, bool vec, F f) {
+  auto with_rows = [&](auto fu, auto v) {
+    if (rm == 4) f(RowsTag<4>{}, fu, v);
+    else if (rm == 2) f(RowsTag<2>{}, fu, v);
+    else f(RowsTag<1>{}, fu, v);
   };
-  if (vec) with_rows(std::true_type{});
-  else with_rows(std::false_type{});
+  auto with_fused = [&](auto v) {
+    if (fused) with_rows(std::true_type{}, v);
+    else with_rows(std::false_type{}, v);
+  };
+  if (vec) with_fused(std::true_type{});
+  else with_fused(std::false_type{});
 }
 inline dim3 TileGrid(size_t BH, size_t tiles, size_t d) {
   return dim3(static_cast<unsigned>(BH * tiles), static_cast<unsigned>((d + kTile - 1) / kTile));
@@ -795,16 +956,16 @@ inline dim3 TileGrid(size_t BH, size_t tiles, size_t d) {
 
 void AttnFwd(const float* q, const float* k, const float* v, float* o, float* probs,
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,
-             cudaStream_t s) {
+             bool fused, cudaStream_t s) {
   const size_t units = B * H * S;
   if (units == 0) return;
   const float inv_sqrt_d = 1.0f / sqrtf(static_cast<float>(d));
-  if (const int rm = RowsPerThreadWithScores(B * H, S, 1); rm > 0) {
-    WithTile(rm, Vec(d, {q, k, v, o}), [&](auto rows, auto vec) {
+  if (const int rm = RowsPerThreadWithScores(B * H, S, d, 1); rm > 0) {
+    WithTile(rm, fused, Vec(d, {q, k, v, o}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
       constexpr int RM = decltype(rows)::value;
-      const size_t bytes = SliceBytes(RM) + 16 * RM * RowStride(S) * sizeof(float);
-      AllowSmem(AttnFwdTileKernel<RM, decltype(vec)::value>, bytes);
-      AttnFwdTileKernel<RM, decltype(vec)::value><<<static_cast<unsigned>(B * H * ((S + 16 * RM - 1) / (16 * RM))), kTileThreads, bytes, s>>>(
+      const size_t bytes = ScoreBytes(RM, S, d, 1);
+      AllowSmem(AttnFwdTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, bytes);
+      AttnFwdTileKernel<RM, decltype(fu)::value, decltype(vec)::value><<<static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes, s>>>(
           q, k, v, o, probs, stats, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d),
           starts, inv_sqrt_d);
     });
@@ -819,26 +980,31 @@ void AttnFwd(const float* q, const float* k, const float* v, float* o, float* pr
 void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d,
             cudaStream_t s) {
   if (B * H * S == 0) return;
-  const size_t tiles = (S + kTile - 1) / kTile;
-  const unsigned blocks = static_cast<unsigned>(B * H * tiles * tiles);
-  const int BH = static_cast<int>(B * H);
-  auto launch = [&](auto kernel) {
-    kernel<<<blocks, kTileThreads, SliceBytes(4), s>>>(dout, v, dp, BH, static_cast<int>(S), static_cast<int>(H),
-                                                       static_cast<int>(d));
-  };
-  if (Vec(d, {dout, v})) launch(AttnDPTileKernel<true>);
-  else launch(AttnDPTileKernel<false>);
+  auto bytes = [&](int rm) { return StreamBytes() + OwnBytes(rm, static_cast<int>(d)); };
+  int rm = RowsPerThread(B * H, S, 8);
+  while (rm > 1 && bytes(rm) > kTwoPerSm) rm /= 2;
+  if (bytes(rm) > kMaxSmem) {
+    AttnDPWideKernel<<<148 * 8, 256, 0, s>>>(dout, v, dp, B * H, S, H, d);
+    return;
+  }
+  WithTile(rm, false, Vec(d, {dout, v}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
+    constexpr int RM = decltype(rows)::value;
+    AllowSmem(AttnDPTileKernel<RM, decltype(vec)::value>, bytes(RM));
+    AttnDPTileKernel<RM, decltype(vec)::value>
+        <<<static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes(RM), s>>>(
+            dout, v, dp, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d));
+  });
 }
 
 namespace {
 
 template <bool kScaled>
 void ColSum(const float* w, const float* x, float* out, size_t B, size_t S, size_t H, size_t d, float scale,
-            cudaStream_t s) {
+            bool fused, cudaStream_t s) {
   if (B * H * S == 0) return;
-  WithTile(RowsPerThread(B * H, S, (d + kTile - 1) / kTile), Vec(d, {x, out}), [&](auto rows, auto vec) {
+  WithTile(RowsPerThread(B * H, S, 16, (d + kTile - 1) / kTile), fused, Vec(d, {x, out}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
     constexpr int RM = decltype(rows)::value;
-    AttnColTileKernel<RM, kScaled, decltype(vec)::value>
+    AttnColTileKernel<RM, decltype(fu)::value, kScaled, decltype(vec)::value>
         <<<TileGrid(B * H, (S + 16 * RM - 1) / (16 * RM), d), kTileThreads, 0, s>>>(
             w, x, out, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d), scale);
   });
@@ -847,22 +1013,22 @@ void ColSum(const float* w, const float* x, float* out, size_t B, size_t S, size
 }  // namespace
 
 void AttnDV(const float* probs, const float* dout, float* dv, size_t B, size_t S, size_t H,
-            size_t d, cudaStream_t s) {
-  ColSum<false>(probs, dout, dv, B, S, H, d, 1.0f, s);
+            size_t d, bool fused, cudaStream_t s) {
+  ColSum<false>(probs, dout, dv, B, S, H, d, 1.0f, fused, s);
 }
 
-void AttnDK(const float* ds, const float* q, float* dk, size_t B, size_t S, size_t H, size_t d,
+void AttnDK(const float* ds, const float* q, float* dk, size_t B, size_t S, size_t H, size_t d, bool fused,
             cudaStream_t s) {
-  ColSum<true>(ds, q, dk, B, S, H, d, 1.0f / sqrtf(static_cast<float>(d)), s);
+  ColSum<true>(ds, q, dk, B, S, H, d, 1.0f / sqrtf(static_cast<float>(d)), fused, s);
 }
 
 void AttnDQ(const float* ds, const float* k, float* dq, size_t B, size_t S, size_t H, size_t d,
-            cudaStream_t s) {
+            bool fused, cudaStream_t s) {
   if (B * H * S == 0) return;
   const float inv_sqrt_d = 1.0f / sqrtf(static_cast<float>(d));
-  WithTile(RowsPerThread(B * H, S, (d + kTile - 1) / kTile), Vec(d, {k, dq}), [&](auto rows, auto vec) {
+  WithTile(RowsPerThread(B * H, S, 16, (d + kTile - 1) / kTile), fused, Vec(d, {k, dq}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
     constexpr int RM = decltype(rows)::value;
-    AttnRowTileKernel<RM, decltype(vec)::value>
+    AttnRowTileKernel<RM, decltype(fu)::value, decltype(vec)::value>
         <<<TileGrid(B * H, (S + 16 * RM - 1) / (16 * RM), d), kTileThreads, 0, s>>>(
             ds, k, dq, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d), inv_sqrt_d);
   });
@@ -875,17 +1041,17 @@ void SoftmaxRowsBwd(const float* probs, const float* dp, float* ds, size_t rows,
 }
 
 void AttnDQTiled(const float* q, const float* k, const float* v, const float* dout, float* stats,
-                 float* dq, size_t B, size_t S, size_t H, size_t d, cudaStream_t s) {
+                 float* dq, size_t B, size_t S, size_t H, size_t d, bool fused, cudaStream_t s) {
   const size_t units = B * H * S;
   if (units == 0) return;
   const float inv_sqrt_d = 1.0f / sqrtf(static_cast<float>(d));
-  if (const int rm = RowsPerThreadWithScores(B * H, S, 2); rm > 0) {
-    WithTile(rm, Vec(d, {q, k, v, dout, dq}), [&](auto rows, auto vec) {
+  if (const int rm = RowsPerThreadWithScores(B * H, S, d, 2); rm > 0) {
+    WithTile(rm, fused, Vec(d, {q, k, v, dout, dq}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
       constexpr int RM = decltype(rows)::value;
-      const size_t bytes = SliceBytes(RM) + 2 * 16 * RM * RowStride(S) * sizeof(float);
-      AllowSmem(AttnDQTiledTileKernel<RM, decltype(vec)::value>, bytes);
-      AttnDQTiledTileKernel<RM, decltype(vec)::value>
-          <<<static_cast<unsigned>(B * H * ((S + 16 * RM - 1) / (16 * RM))), kTileThreads, bytes, s>>>(
+      const size_t bytes = ScoreBytes(RM, S, d, 2);
+      AllowSmem(AttnDQTiledTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, bytes);
+      AttnDQTiledTileKernel<RM, decltype(fu)::value, decltype(vec)::value>
+          <<<static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes, s>>>(
               q, k, v, dout, stats, dq, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H),
               static_cast<int>(d), inv_sqrt_d);
     });
@@ -899,20 +1065,21 @@ void AttnDQTiled(const float* q, const float* k, const float* v, const float* do
 
 void AttnDKVTiled(bool want_dk, const float* q, const float* k, const float* v, const float* dout,
                   const float* stats, float* out, size_t B, size_t S, size_t H, size_t d,
-                  cudaStream_t s) {
+                  bool fused, cudaStream_t s) {
   if (B * H * S == 0) return;
   const float inv_sqrt_d = 1.0f / sqrtf(static_cast<float>(d));
-  WithTile(RowsPerThread(B * H, S, (d + kTile - 1) / kTile), Vec(d, {q, k, v, dout, out}), [&](auto rows, auto vec) {
+  WithTile(RowsPerThread(B * H, S, 8, (d + kTile - 1) / kTile), fused, Vec(d, {q, k, v, dout, out}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
     constexpr int RM = decltype(rows)::value;
-    const size_t bytes = SliceBytes(RM) + kTile * (16 * RM + 4) * sizeof(float);
+    const size_t bytes = StreamBytes() + (want_dk ? 2 : 1) * OwnBytes(RM, static_cast<int>(d)) +
+                         2 * kTile * (kTile + 8 * RM + 4) * sizeof(float);
     auto launch = [&](auto kernel) {
       AllowSmem(kernel, bytes);
-      kernel<<<TileGrid(B * H, (S + 16 * RM - 1) / (16 * RM), d), kTileThreads, bytes, s>>>(
+      kernel<<<TileGrid(B * H, (S + 8 * RM - 1) / (8 * RM), d), kTileThreads, bytes, s>>>(
           q, k, v, dout, stats, out, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H),
           static_cast<int>(d), inv_sqrt_d);
     };
-    if (want_dk) launch(AttnDKVTiledTileKernel<RM, true, decltype(vec)::value>);
-    else launch(AttnDKVTiledTileKernel<RM, false, decltype(vec)::value>);
+    if (want_dk) launch(AttnDKVTiledTileKernel<RM, true, decltype(fu)::value, decltype(vec)::value>);
+    else launch(AttnDKVTiledTileKernel<RM, false, decltype(fu)::value, decltype(vec)::value>);
   });
 }
 

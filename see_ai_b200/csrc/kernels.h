@@ -172,24 +172,25 @@ void PublishToHost(const PublishList& list, uint32_t* host, cudaStream_t s);
 void SetScalars(const AdamScalars& v, AdamScalars* dst, cudaStream_t s);
 
 // ---- attention (exact family; scores in double like the CPU executor) --------
+// fused: the f32 output sums may contract multiply-adds (engine mode; never through the strict seam).
 void AttnFwd(const float* q, const float* k, const float* v, float* o, float* probs,
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,
-             cudaStream_t s);  // probs != null: cached family; stats != null: tiled family
+             bool fused, cudaStream_t s);  // probs != null: cached family; stats != null: tiled family
 void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d,
             cudaStream_t s);
 void AttnDV(const float* probs, const float* dout, float* dv, size_t B, size_t S, size_t H,
-            size_t d, cudaStream_t s);
+            size_t d, bool fused, cudaStream_t s);
 void SoftmaxRowsBwd(const float* probs, const float* dp, float* ds, size_t rows, size_t cols,
                     cudaStream_t s);
 void AttnDQ(const float* ds, const float* k, float* dq, size_t B, size_t S, size_t H, size_t d,
-            cudaStream_t s);
+            bool fused, cudaStream_t s);
 void AttnDK(const float* ds, const float* q, float* dk, size_t B, size_t S, size_t H, size_t d,
-            cudaStream_t s);
+            bool fused, cudaStream_t s);
 void AttnDQTiled(const float* q, const float* k, const float* v, const float* dout, float* stats,
-                 float* dq, size_t B, size_t S, size_t H, size_t d, cudaStream_t s);
+                 float* dq, size_t B, size_t S, size_t H, size_t d, bool fused, cudaStream_t s);
 void AttnDKVTiled(bool want_dk, const float* q, const float* k, const float* v, const float* dout,
                   const float* stats, float* out, size_t B, size_t S, size_t H, size_t d,
-                  cudaStream_t s);
+                  bool fused, cudaStream_t s);
 
 // ---- evaluation / merge tails (integer tallies, exact) -------------------------
 // tally[0] += rows with label >= 0, tally[1] += those whose argmax == label.

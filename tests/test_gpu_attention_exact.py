@@ -1,6 +1,6 @@
-"""The exact attention family at the edges of its kernels' tiles (16, 32 or 64
-rows of one axis, 64 of the other, 32 features and 64 output columns at a time,
-16-byte and scalar access, rows too long for shared memory), instruction by
+"""The exact attention family at the edges of its kernels' tiles (8, 16 or 32
+rows of one axis, 64 of the other, 8 features and 64 output columns at a time,
+16-byte and scalar access, rows too long and heads too wide for shared memory), instruction by
 instruction from the CPU oracle's bytes: the cached family's products bit for
 bit, what holds a double row sum or expf to the 1e-5 of the tensor's scale the
 executor is held to everywhere."""
@@ -21,7 +21,8 @@ SHAPES = [   # B, S, H, d
     (10, 70, 10, 12),    # two rows per thread
     (20, 65, 16, 8),     # four
     (1, 700, 1, 16),     # the tiled backward's two score rows: 16-row blocks
-    (1, 3400, 1, 8),     # score rows too long for a tile block: one warp per row
+    (1, 40, 1, 3400),    # a head too wide for a tile block (the tiled backward of keys stops at 256 features)
+    (1, 6900, 1, 8),     # score rows too long for a tile block: one warp per row
 ]
 
 
@@ -63,7 +64,9 @@ def _program(Bq, S, H, d, segments, cached):
     args = (o["q"], o["k"], o["v"], o["do"])
     prog += [P.Instr(Op.ATTN_FWD_TILED_SEG, 0, 0, (o["q"], o["k"], o["v"], o["o2"]), (o["stats"], geo, o["starts"]))
              if segments else P.Instr(Op.ATTN_FWD_TILED, 0, 0, (o["q"], o["k"], o["v"], o["o2"]), (o["stats"], bs, hd)),
-             P.Instr(Op.ATTN_DQ_TILED, 0, 0, args, (o["stats"], o["dq2"], geo)),
+             P.Instr(Op.ATTN_DQ_TILED, 0, 0, args, (o["stats"], o["dq2"], geo))]
+    if d <= 256:
+        prog += [
              P.Instr(Op.ATTN_DK_TILED, 0, 0, args, (o["stats"], o["dk2"], geo)),
              P.Instr(Op.ATTN_DV_TILED, 0, 0, args, (o["stats"], o["dv2"], geo))]
     return prog, arena
