@@ -2009,9 +2009,13 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     }
   }
   // Small and narrow products likewise, but for the rank-r expand product of many rows: that one is a stream, and a
-  // following add may ride it.
+  // following add may ride it.  A forward layer of short reduction keeps the reference's order of sums: its
+  // 16 x 16-block kernel is as fast there (feed-forward step at a batch of 32: 100 us against 106), and a
+  // pre-activation on the other side of a ReLU's kink than the CPU's moves a whole row of gradients.
   const bool expand = !a.a_transposed && a.K <= 16 && a.K % 4 == 0 && a.M >= 64 && a.N >= 64;
-  if (coherence_ == Coherence::kLazy && adapter_fma_ && !expand && !a.accumulate && k::FastGemm(a, stream_)) {
+  const bool short_layer = !a.a_transposed && !a.b_transposed && a.M > 16 && a.N > 16 && a.K <= 256;
+  if (coherence_ == Coherence::kLazy && adapter_fma_ && !expand && !short_layer && !a.accumulate &&
+      k::FastGemm(a, stream_)) {
     ++counters_.kernel_launches;
     return {};
   }
