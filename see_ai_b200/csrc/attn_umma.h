@@ -15,6 +15,7 @@ namespace see::k {
 
 struct AttnUmmaArgs {
   uint32_t B, S, H, d;
+  uint32_t sms;     // the device's multiprocessors (grid of the persistent kernels)
   float inv_sqrt_d;
   float* out;       // O / dQ / dK / dV, f32 [B*S, H*d]
   float* stats;     // f32 [B*H*S, 4]: score max, 1/denominator, delta, start
@@ -43,7 +44,7 @@ cudaError_t AttnFwdUmma(const CUtensorMap& q, const CUtensorMap& k_half, const C
                         const AttnUmmaArgs& a, cudaStream_t s);
 cudaError_t AttnDQUmma(const CUtensorMap& q, const CUtensorMap& dout, const CUtensorMap& k_half,
                        const CUtensorMap& v_half, const AttnUmmaArgs& a, cudaStream_t s);
-// mode 0: dV (v ignored); 1: dK; 2: both in one walk (a.out = dK, a.out2 = dV; d = 64 only).
+// mode 0: dV (v ignored); 1: dK; 2: both in one walk (a.out = dK, a.out2 = dV).
 cudaError_t AttnDKVUmma(int mode, const CUtensorMap& k, const CUtensorMap& v, const CUtensorMap& q_half,
                         const CUtensorMap& dout_half, const AttnUmmaArgs& a, cudaStream_t s);
 

@@ -1100,7 +1100,7 @@ void CudaBackend::PlanActFusions(std::span<const Instruction> program, size_t be
       continue;
     const AttnGeom g = UnpackAttnGeom(dk.out[2]);
     const uint64_t bytes = g.B * g.S * g.H * g.d * 4;
-    if (g.d != 64 || !disjoint(RefOffset(dk.out[1]), RefOffset(dk.out[1]) + bytes, RefOffset(dv.out[1]),
+    if (!disjoint(RefOffset(dk.out[1]), RefOffset(dk.out[1]) + bytes, RefOffset(dv.out[1]),
                                RefOffset(dv.out[1]) + bytes))
       continue;
     // Neither output may lie over an operand the other instruction still reads.

@@ -26,6 +26,8 @@
 // that runs out raises DeviceStatus::wait_timeout and the CTA stores nothing.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "attn_umma.h"
 #include "kernels.h"
 #include "shadow.cuh"
@@ -79,6 +81,31 @@ __device__ __forceinline__ float Exp2Approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Two f32 operations per instruction, each rounded as the scalar one.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 Pair(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float Lo(F2 v) { return __uint_as_float(static_cast<uint32_t>(v)); }
+__device__ __forceinline__ float Hi(F2 v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+__device__ __forceinline__ F2 Fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ F2 Add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 Mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 // Loads [R positions][D] of head h of sequence b ({d, S, H, B} map with box {64, R, 1, 1}) as
@@ -365,9 +392,9 @@ AttnFwdUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 // ---- dQ (and delta) --------------------------------------------------------------------
 // Per 128 query rows, the keys 64 at a time.  Per step S = Q K_h^T (columns
 // 0..63) and dP = dO V_h^T (64..127); dS = P (dP - delta) / sqrt(d) goes to shared
-// memory as bf16 and dQ += dS K (columns 128..128+D).  delta_i = sum_j P_ij dP_ij:
-// with the forward's kept copy of O at hand it is dO_i . O_i, one row of each read
-// by the row's thread before the walk; without it a first walk over the keys sums it.
+// memory as bf16 and dQ += dS K (columns 128..128+D).  A first walk over the keys sums
+// delta_i = sum_j P_ij dP_ij; where the forward's kept copy of O is at hand the kernel
+// with dedicated warps below takes the instruction instead.
 template <int D>
 __global__ void __launch_bounds__(128)
 AttnDQUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
@@ -390,8 +417,7 @@ AttnDQUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const uint32_t bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
   const uint32_t all_h = (a.S + kHalf - 1) / kHalf;
   const uint32_t n_h = 2 * (it + 1) < all_h ? 2 * (it + 1) : all_h;
-  const bool one_walk = a.fwd_keep != nullptr;
-  const uint32_t total = one_walk ? n_h : 2 * n_h;
+  const uint32_t total = 2 * n_h;
 
   if (tid == 0) {
     MbarInit(&ctl->bar_a, 1); MbarInit(&ctl->bar_b, 1); MbarInit(&ctl->mma, 1);
@@ -423,24 +449,10 @@ AttnDQUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   float delta = 0.0f;
   int failed = 0;
   if (tid == 0) issue_a(0);
-  if (one_walk && live) {   // (under the first loads' flight)
-    const size_t at = (static_cast<size_t>(b) * a.S + row) * (static_cast<size_t>(a.H) * D) + static_cast<size_t>(h) * D;
-    const float4* orow = reinterpret_cast<const float4*>(a.fwd_keep + at);
-    const uint2* drow = reinterpret_cast<const uint2*>(a.dout_bf16 + at);   // four bf16 per load
-#pragma unroll 4
-    for (int c = 0; c < D / 4; ++c) {
-      const float4 o = orow[c];
-      const uint2 g = drow[c];
-      delta = fmaf(o.x, __uint_as_float(g.x << 16), delta);
-      delta = fmaf(o.y, __uint_as_float(g.x & 0xFFFF0000u), delta);
-      delta = fmaf(o.z, __uint_as_float(g.y << 16), delta);
-      delta = fmaf(o.w, __uint_as_float(g.y & 0xFFFF0000u), delta);
-    }
-  }
 
   for (uint32_t t = 0; t < total; ++t) {
     const uint32_t jh = t % n_h;
-    const bool second = one_walk || t >= n_h;
+    const bool second = t >= n_h;
     if (tid == 0) {
       if (!MbarWait(&ctl->bar_a, t & 1)) failed = 1;
       TcFenceAfter();
@@ -520,18 +532,13 @@ AttnDQUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 // number per query, M = max * log2(e) - log2(1/denominator), so that
 // P^T = 2^(s * log2(e)/sqrt(d) - M).  dV += P^T dO_h, or
 // dS^T = P^T (dP^T - delta) / sqrt(d) with dP^T = V dO_h^T and dK += dS^T Q_h.
-// kMode 0: dV alone; 1: dK alone; 2: both in one walk (the plan's kAttnDKTiled /
-// kAttnDVTiled pair on the same operands): S^T and P^T are formed once, dV's
-// product rides the step's second commit, and the second kernel's passes over K,
-// Q and the statistics disappear.  Tensor memory: S^T, dP^T, dK, dV = 4 x 64 columns
-// at d = 64 (the 256 the dK form occupies anyway).
-template <int D, int kMode>
+// (The plan's kAttnDKTiled / kAttnDVTiled pair on the same operands goes to the kernel with
+// dedicated warps below, which makes both in one walk.)
+template <int D, bool kWantDK>
 __global__ void __launch_bounds__(128)
 AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                   const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                   AttnUmmaArgs a) {
-  constexpr bool kWantDK = kMode >= 1;
-  constexpr bool kBoth = kMode == 2;
   extern __shared__ uint8_t smem_raw[];
   Ctl* ctl = reinterpret_cast<Ctl*>(smem_raw);
   uint8_t* smem = AlignSmem(smem_raw + sizeof(Ctl));
@@ -543,11 +550,9 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
   uint8_t* q_s = v_s + (kWantDK ? kFull : 0);
   uint8_t* do_s = q_s + 2 * kHalfRows;
   uint8_t* p_s = do_s + 2 * kHalfRows;
-  uint8_t* p2_s = p_s + kHalfTileBytes;                      // both: P^T beside dS^T
-  float* stat_s = reinterpret_cast<float*>(p2_s + (kBoth ? kHalfTileBytes : 0));   // M[64], delta[64]
+  float* stat_s = reinterpret_cast<float*>(p_s + kHalfTileBytes);   // M[64], delta[64]
   constexpr uint32_t kOutCol = kWantDK ? 128 : 64;
-  constexpr uint32_t kOutCol2 = kOutCol + D;                 // both: dV after dK
-  constexpr uint32_t kTmemCols = TmemColsFor(kOutCol + (kBoth ? 2 : 1) * D);
+  constexpr uint32_t kTmemCols = TmemColsFor(kOutCol + D);
 
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   const uint32_t jt = blockIdx.x;                          // key tile; low tiles have the most work
@@ -619,7 +624,6 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
       if (kWantDK) TmemLoad32(t_lane + 64 + c0, rp);
       TmemWaitLd();
       float v[32];
-      [[maybe_unused]] float pv[kBoth ? 32 : 1];
 #pragma unroll
       for (int j4 = 0; j4 < 32; j4 += 4) {
         const float4 M4 = *reinterpret_cast<const float4*>(&stat_s[c0 + j4]);
@@ -635,11 +639,9 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
           float p = Exp2Approx(fmaf(__uint_as_float(rs[j]), c1, -Mv[u]));
           if (diagonal && key > q0 + c0 + j) p = 0.0f;
           v[j] = kWantDK ? p * (__uint_as_float(rp[j]) - dv[u]) * a.inv_sqrt_d : p;
-          if (kBoth) pv[kBoth ? j : 0] = p;
         }
       }
       StoreRowChunk(p_s, tid, c0, v);
-      if constexpr (kBoth) StoreRowChunk(p2_s, tid, c0, pv);
     }
     FenceProxyAsync();
     TcFenceBefore();
@@ -649,7 +651,6 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
       const uint8_t* qh = q_s + (t & 1) * kHalfRows;
       const uint8_t* doh = do_s + (t & 1) * kHalfRows;
       MmaPRows<D>(tmem + kOutCol, p_s, kWantDK ? qh : doh, t != 0);   // dK += dS^T Q_h, or dV += P^T dO_h
-      if (kBoth) MmaPRows<D>(tmem + kOutCol2, p2_s, doh, t != 0);     // dV += P^T dO_h
     }
   }
   if (tid == 0) UmmaCommit(&ctl->mma);
@@ -666,11 +667,6 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
     const size_t flat0 = (static_cast<size_t>(b) * a.S + row0w) * HD + static_cast<size_t>(h) * D;
     StoreOutRows<D>(t_lane + kOutCol, reinterpret_cast<float*>(smem) + warp * 32 * D, tid & 31, 1.0f,
                     a.out + flat0, HD, rows_live, a.shadow, flat0, h * D);
-    if constexpr (kBoth) {
-      __syncwarp();   // the warp's staging slab is reused
-      StoreOutRows<D>(t_lane + kOutCol2, reinterpret_cast<float*>(smem) + warp * 32 * D, tid & 31, 1.0f,
-                      a.out2 + flat0, HD, rows_live, a.shadow2, flat0, h * D);
-    }
   }
   TcFenceBefore();
   __syncthreads();
@@ -680,13 +676,390 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
   }
 }
 
+
+// ---- backward on dedicated warps -----------------------------------------------------------
+// dQ (with delta from the forward's kept copy) and dK + dV in one walk, as one persistent CTA
+// per SM whose warps have one job each, so that the chain load -> product -> exponentials ->
+// product of one step overlaps the next step's and the next tile's:
+//   warp 13      TMA: a tile's own 128 rows (double-buffered at d = 64) and a ring of 64-row steps
+//   warp 12      first products: keeps two steps of S and dP in tensor memory ahead of the softmax
+//   warps 0-7    the elementwise part: thread = row x 32 of the step's 64 columns; P and dS go back
+//                to tensor memory as bf16, over the S and dP columns they came from, and are the A
+//                operand of the second products there (no shared-memory tile, no proxy fence)
+//   warp 14      second products, as soon as a step's P and dS are there
+//   warps 8-11   outputs of the finished tile, and for dQ the row statistics of the next one
+// Same products, operands and summation order as the kernels above, so the same bits.
+//
+// What bounds it: a 128 x 64 x 16 product holds the tensor pipe 62 cycles, so a step's twelve (dQ)
+// or sixteen (dK/dV) take 750 or 990; the exponentials of 64 columns x 128 rows 512 cycles of the
+// exp pipe.  A step takes about 1250 and 1350 cycles, the second products' commit on its way round
+// the chain; one 128-thread CTA that did everything in turn took 4200, two to an SM.
+// Measured: forward + dQ + dK/dV of 8 x 2048 positions of 16 heads 1031 -> 677 us.  Two issuing
+// warps because one spent as long waiting and issuing as the pipe worked (dQ of that size: 233 us
+// with one, 202 with two, 178 with the element arithmetic in pairs).
+template <int D, bool kKV>
+struct BwdShape {
+  static constexpr uint32_t kFix = 128 * D * 2;              // one own-row tile
+  static constexpr uint32_t kStep = 64 * D * 2;              // one 64-row step tile
+  static constexpr uint32_t kFixBufs = D == 64 ? 2 : 1;
+  static constexpr uint32_t kStages = D == 64 ? 4 : 3;
+  static constexpr uint32_t kOutCols = (kKV ? 2 : 1) * D;
+  static constexpr uint32_t kOutBufs = 2 * kOutCols <= 256 ? 2 : 1;
+  static constexpr uint32_t kOutCol = 256;                   // after two {S, dP} pairs of 64 + 64 columns
+  static constexpr uint32_t kSlab = 32 * 64 * 4;             // a storing warp's staging
+  static constexpr uint32_t kStats = 2 * 2 * 128 * 4 + 8 * 64 * 4;
+  static constexpr size_t kSmem = kFixBufs * 2 * kFix + kStages * 2 * kStep + 4 * kSlab + kStats + 512 + 1024;
+};
+
+struct BwdCtl {
+  uint64_t fix_full[2], fix_empty[2];
+  uint64_t full[4], empty[4];
+  uint64_t acc_full[2], p_full[2];
+  uint64_t out_full[2], out_empty[2];
+  uint64_t stat_full[2], stat_empty[2];
+  uint32_t tmem_base;
+  volatile uint32_t failed;   // some role's wait ran out: the others stop too
+};
+static_assert(sizeof(BwdCtl) <= 512, "control block");
+
+// A bounded wait that also ends when another role of the CTA has given up.
+__device__ __forceinline__ bool RoleWait(BwdCtl* ctl, uint64_t* bar, uint32_t parity) {
+  const uint32_t addr = SmemAddr(bar);
+  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((it & 255) == 255 && ctl->failed) return false;
+  }
+  ctl->failed = 1;
+  return false;
+}
+// The same by a whole warp, with one answer (a vote: what follows stays warp-uniform for the compiler).
+__device__ __forceinline__ bool WarpWait(BwdCtl* ctl, uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xFFFFFFFFu, RoleWait(ctl, bar, parity));
+}
+
+// The tiles of a CTA: heaviest first, dealt out in rounds that alternate direction (within 1.5 % of
+// an even load from S = 2048 on, 10 % at 384 tiles of S = 512).
+struct BwdTile { uint32_t row_tile, bh, steps, step0; };
+template <bool kKV>
+__device__ __forceinline__ bool BwdTileAt(uint32_t round, uint32_t S, uint32_t BH, BwdTile* t) {
+  const uint32_t n_t = (S + kTile - 1) / kTile, all_h = (S + kHalf - 1) / kHalf;
+  const uint32_t at = round * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+  if (at >= n_t * BH) return false;   // only in the last round
+  const uint32_t rank = at / BH;
+  t->bh = at - rank * BH;
+  t->row_tile = kKV ? rank : n_t - 1 - rank;
+  t->step0 = kKV ? 2 * rank : 0;      // dK/dV: queries from the diagonal on; dQ: keys up to it
+  const uint32_t upto = 2 * (t->row_tile + 1) < all_h ? 2 * (t->row_tile + 1) : all_h;
+  t->steps = kKV ? all_h - t->step0 : upto;
+  return true;
+}
+
+constexpr uint32_t kBwdThreads = 15 * 32;
+
+// kKV false: x, y = Q, dO rows; u, w = K, V steps; out = dQ.
+// kKV true:  x, y = K, V rows;  u, w = Q, dO steps; out = dK, out2 = dV (transposed frame).
+template <int D, bool kKV>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+AttnBwdKernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
+              const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_w,
+              AttnUmmaArgs a) {
+  using Sh = BwdShape<D, kKV>;
+  extern __shared__ uint8_t smem_raw[];
+  BwdCtl* ctl = reinterpret_cast<BwdCtl*>(smem_raw);
+  uint8_t* fix_s = AlignSmem(smem_raw + 512);
+  uint8_t* ring_s = fix_s + Sh::kFixBufs * 2 * Sh::kFix;
+  uint8_t* slab_s = ring_s + Sh::kStages * 2 * Sh::kStep;
+  float* row_stat_s = reinterpret_cast<float*>(slab_s + 4 * Sh::kSlab);   // dQ: [2][{M, delta}][128]
+  float* col_stat_s = row_stat_s + 2 * 2 * 128;                           // dK/dV: per warp {-M[32], -delta[32]}
+
+  const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t BH = a.B * a.H;
+
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      MbarInit(&ctl->fix_full[i], 1); MbarInit(&ctl->fix_empty[i], 1);
+      MbarInit(&ctl->acc_full[i], 1); MbarInit(&ctl->p_full[i], 8);
+      MbarInit(&ctl->out_full[i], 1); MbarInit(&ctl->out_empty[i], 4);
+      MbarInit(&ctl->stat_full[i], 4); MbarInit(&ctl->stat_empty[i], 8);
+    }
+    for (int i = 0; i < 4; ++i) { MbarInit(&ctl->full[i], 1); MbarInit(&ctl->empty[i], 1); }
+    ctl->failed = 0;
+    MbarInitFence();
+  }
+  if (warp == 12) TmemAlloc(&ctl->tmem_base, 512);
+  TcFenceBefore();
+  __syncthreads();
+  TcFenceAfter();
+  constexpr uint32_t tmem = 0;   // all 512 columns are this CTA's
+
+  if (warp == 13) {
+    // ---- loads ----
+    if (lane == 0) {
+      uint32_t g = 0, i = 0;
+      bool ok = true;
+      BwdTile tl;
+      for (; ok && BwdTileAt<kKV>(i, a.S, BH, &tl); ++i) {
+        const uint32_t b = tl.bh / a.H, h = tl.bh - b * a.H;
+        const uint32_t fb = i % Sh::kFixBufs;
+        if (!(ok = RoleWait(ctl, &ctl->fix_empty[fb], ((i / Sh::kFixBufs) & 1) ^ 1))) break;
+        uint8_t* fx = fix_s + fb * 2 * Sh::kFix;
+        MbarExpectTx(&ctl->fix_full[fb], 2 * Sh::kFix);
+        LoadRows<D, 128>(fx, &map_x, &ctl->fix_full[fb], tl.row_tile * kTile, h, b);
+        LoadRows<D, 128>(fx + Sh::kFix, &map_y, &ctl->fix_full[fb], tl.row_tile * kTile, h, b);
+        for (uint32_t t = 0; t < tl.steps; ++t, ++g) {
+          const uint32_t s = g % Sh::kStages;
+          if (!(ok = RoleWait(ctl, &ctl->empty[s], ((g / Sh::kStages) & 1) ^ 1))) break;
+          uint8_t* st = ring_s + s * 2 * Sh::kStep;
+          MbarExpectTx(&ctl->full[s], 2 * Sh::kStep);
+          LoadRows<D, 64>(st, &map_u, &ctl->full[s], (tl.step0 + t) * kHalf, h, b);
+          LoadRows<D, 64>(st + Sh::kStep, &map_w, &ctl->full[s], (tl.step0 + t) * kHalf, h, b);
+        }
+      }
+      // Every slot's last release has arrived before the CTA may end.
+      for (uint32_t k = 0; ok && k < Sh::kStages; ++k, ++g)
+        ok = RoleWait(ctl, &ctl->empty[g % Sh::kStages], ((g / Sh::kStages) & 1) ^ 1);
+      for (uint32_t k = 0; ok && k < Sh::kFixBufs; ++k, ++i)
+        ok = RoleWait(ctl, &ctl->fix_empty[i % Sh::kFixBufs], ((i / Sh::kFixBufs) & 1) ^ 1);
+    }
+  } else if (warp == 12) {
+    // ---- first products: S (or S^T) and dP of one step into its half of the accumulators ----
+    // (the whole warp walks and waits; one elected lane issues)
+    BwdTile tl;
+    uint32_t g = 0;
+    bool ok = true;
+    for (uint32_t i = 0; ok && BwdTileAt<kKV>(i, a.S, BH, &tl); ++i) {
+      const uint32_t fb = i % Sh::kFixBufs;
+      if (!(ok = WarpWait(ctl, &ctl->fix_full[fb], (i / Sh::kFixBufs) & 1))) break;
+      const uint8_t* fx = fix_s + fb * 2 * Sh::kFix;
+      for (uint32_t t = 0; t < tl.steps; ++t, ++g) {
+        const uint32_t s = g % Sh::kStages;
+        if (!(ok = WarpWait(ctl, &ctl->full[s], (g / Sh::kStages) & 1))) break;
+        // The accumulators' last reader: the second products two steps ago (which release their ring slot with it).
+        if (g >= 2 && !(ok = WarpWait(ctl, &ctl->empty[(g - 2) % Sh::kStages], ((g - 2) / Sh::kStages) & 1))) break;
+        TcFenceAfter();
+        const uint8_t* st = ring_s + s * 2 * Sh::kStep;
+        const uint32_t acc = tmem + (g & 1) * 128;
+        if (ElectOne()) {
+          MmaRowRow<D, 64>(acc, fx, st);
+          MmaRowRow<D, 64>(acc + 64, fx + Sh::kFix, st + Sh::kStep);
+          UmmaCommit(&ctl->acc_full[g & 1]);
+          if (t + 1 == tl.steps) UmmaCommit(&ctl->fix_empty[fb]);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == 14) {
+    // ---- second products: dQ += dS K_h, or dK += dS^T Q_h and dV += P^T dO_h ----
+    BwdTile tl;
+    uint32_t g = 0;
+    bool ok = true;
+    const uint32_t idesc = MakeInstrDesc(128, D) | kInstrDescBMnMajor;
+    for (uint32_t i = 0; ok && BwdTileAt<kKV>(i, a.S, BH, &tl); ++i) {
+      const uint32_t ob = i % Sh::kOutBufs;
+      const uint32_t out = tmem + Sh::kOutCol + ob * Sh::kOutCols;
+      if (!(ok = WarpWait(ctl, &ctl->out_empty[ob], ((i / Sh::kOutBufs) & 1) ^ 1))) break;
+      for (uint32_t t = 0; t < tl.steps; ++t, ++g) {
+        const uint32_t s = g % Sh::kStages;
+        if (!(ok = WarpWait(ctl, &ctl->p_full[g & 1], (g >> 1) & 1))) break;
+        TcFenceAfter();
+        const uint32_t acc = tmem + (g & 1) * 128;
+        const uint32_t u = SmemAddr(ring_s + s * 2 * Sh::kStep);
+        if (ElectOne()) {
+#pragma unroll
+          for (uint32_t k = 0; k < 4; ++k)   // 16 positions of the step: columns {0, 8} of each 32-column half
+            UmmaBf16TmemA(out, acc + (k >> 1) * 32 + (k & 1) * 8, MakeSmemDescMn(u + k * 2048, 64 * 128), idesc,
+                          (t | k) != 0 ? 1u : 0u);
+          if constexpr (kKV) {
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k)
+              UmmaBf16TmemA(out + D, acc + 64 + (k >> 1) * 32 + (k & 1) * 8,
+                            MakeSmemDescMn(u + Sh::kStep + k * 2048, 64 * 128), idesc, (t | k) != 0 ? 1u : 0u);
+          }
+          UmmaCommit(&ctl->empty[s]);
+          if (t + 1 == tl.steps) UmmaCommit(&ctl->out_full[ob]);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp < 8) {
+    // ---- P and dS ----
+    const uint32_t half = warp >> 2, quarter = warp & 3;
+    const uint32_t r_in = quarter * 32 + lane;
+    const uint32_t t_lane = tmem + ((quarter * 32) << 16) + half * 32;
+    const float c1 = a.inv_sqrt_d * kLog2e;
+    float* col_m = col_stat_s + warp * 64;
+    uint32_t g = 0;
+    bool ok = true;
+    BwdTile tl;
+    for (uint32_t i = 0; ok && BwdTileAt<kKV>(i, a.S, BH, &tl); ++i) {
+      const uint32_t row0 = tl.row_tile * kTile, row = row0 + r_in;
+      float m2l = 0.0f, delta = 0.0f;
+      [[maybe_unused]] float4 next = make_float4(INFINITY, 1.0f, 0.0f, 0.0f);
+      const float4* stats = reinterpret_cast<const float4*>(a.stats) + static_cast<size_t>(tl.bh) * a.S;
+      if constexpr (kKV) {
+        const uint32_t qi = tl.step0 * kHalf + half * 32 + lane;
+        if (qi < a.S) next = stats[qi];   // past the end of the sequence: P = 2^-inf = 0
+      } else {
+        if (!(ok = RoleWait(ctl, &ctl->stat_full[i & 1], (i >> 1) & 1))) break;
+        m2l = row_stat_s[(i & 1) * 256 + r_in];
+        delta = row_stat_s[(i & 1) * 256 + 128 + r_in];
+        __syncwarp();
+        if (lane == 0) MbarArrive(&ctl->stat_empty[i & 1]);
+      }
+      for (uint32_t t = 0; t < tl.steps; ++t, ++g) {
+        const uint32_t col0 = (tl.step0 + t) * kHalf + half * 32;   // this thread's first key (query)
+        if constexpr (kKV) {
+          __syncwarp();   // the previous step's readers
+          col_m[lane] = -(next.x * kLog2e - log2f(next.y));
+          col_m[32 + lane] = -next.z;
+          next = make_float4(INFINITY, 1.0f, 0.0f, 0.0f);
+          if (t + 1 < tl.steps && col0 + kHalf + lane < a.S) next = stats[col0 + kHalf + lane];
+          __syncwarp();
+        }
+        if (!(ok = RoleWait(ctl, &ctl->acc_full[g & 1], (g >> 1) & 1))) break;
+        TcFenceAfter();
+        const uint32_t acc = t_lane + (g & 1) * 128;
+        uint32_t rs[32], rp[32], w[16];
+        TmemLoad32(acc, rs);
+        TmemLoad32(acc + 64, rp);
+        TmemWaitLd();
+        [[maybe_unused]] uint32_t pw[16];
+        // P = 2^(s c1 - M), dS = P (dP - delta) / sqrt(d); kDiag: some of the step's pairs are masked.
+        auto elements = [&](auto diag) {
+          constexpr bool kDiag = decltype(diag)::value;
+#pragma unroll
+          for (int j4 = 0; j4 < 32; j4 += 4) {
+            F2 nm[2], nd[2];   // -M and -delta, of the row (dQ) or of the columns (dK/dV)
+            if constexpr (kKV) {
+              const float4 m4 = *reinterpret_cast<const float4*>(col_m + j4);
+              const float4 d4 = *reinterpret_cast<const float4*>(col_m + 32 + j4);
+              nm[0] = Pair(m4.x, m4.y); nm[1] = Pair(m4.z, m4.w);
+              nd[0] = Pair(d4.x, d4.y); nd[1] = Pair(d4.z, d4.w);
+            } else {
+              nm[0] = nm[1] = Pair(-m2l, -m2l);
+              nd[0] = nd[1] = Pair(-delta, -delta);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const int j = j4 + 2 * q;
+              const F2 x = Fma2(Pair(__uint_as_float(rs[j]), __uint_as_float(rs[j + 1])), Pair(c1, c1), nm[q]);
+              float p0 = Exp2Approx(Lo(x)), p1 = Exp2Approx(Hi(x));
+              if constexpr (kDiag) {
+                if (kKV ? row > col0 + j : col0 + j > row) p0 = 0.0f;
+                if (kKV ? row > col0 + j + 1 : col0 + j + 1 > row) p1 = 0.0f;
+              }
+              const F2 ds = Mul2(Mul2(Pair(p0, p1), Add2(Pair(__uint_as_float(rp[j]), __uint_as_float(rp[j + 1])), nd[q])),
+                                 Pair(a.inv_sqrt_d, a.inv_sqrt_d));
+              w[j / 2] = PackBf16x2(Lo(ds), Hi(ds));
+              if constexpr (kKV) pw[j / 2] = PackBf16x2(p0, p1);
+            }
+          }
+        };
+        if (kKV ? col0 < row0 + kTile : col0 + 32 > row0) elements(std::true_type{});
+        else elements(std::false_type{});
+        if constexpr (kKV) TmemStore16(acc + 64, pw);
+        TmemStore16(acc, w);
+        TmemWaitSt();
+        TcFenceBefore();
+        __syncwarp();
+        if (lane == 0) MbarArrive(&ctl->p_full[g & 1]);
+      }
+    }
+  } else {
+    // ---- outputs, and dQ's row statistics ----
+    const uint32_t quarter = warp & 3, r_in = quarter * 32 + lane;
+    float* slab = reinterpret_cast<float*>(slab_s + quarter * Sh::kSlab);
+    const size_t HD = static_cast<size_t>(a.H) * D;
+    bool ok = true;
+    // dQ: P = 2^(s * log2(e)/sqrt(d) - M) with M = max * log2(e) - log2(1/denominator), and
+    // delta_i = dO_i . O_i from the forward's kept copy of O.
+    auto row_stats = [&](uint32_t i) {
+      BwdTile tl;
+      if (!BwdTileAt<kKV>(i, a.S, BH, &tl)) return;
+      if (!(ok = RoleWait(ctl, &ctl->stat_empty[i & 1], ((i >> 1) & 1) ^ 1))) return;
+      const uint32_t row = tl.row_tile * kTile + r_in, b = tl.bh / a.H, h = tl.bh - b * a.H;
+      float m2l = 0.0f, delta = 0.0f;
+      if (row < a.S) {
+        float* st_row = a.stats + (static_cast<size_t>(tl.bh) * a.S + row) * kAttnStatsWidth;
+        m2l = st_row[0] * kLog2e - log2f(st_row[1]);
+        const size_t at = (static_cast<size_t>(b) * a.S + row) * HD + static_cast<size_t>(h) * D;
+        const float4* orow = reinterpret_cast<const float4*>(a.fwd_keep + at);
+        const uint2* drow = reinterpret_cast<const uint2*>(a.dout_bf16 + at);   // four bf16 per load
+#pragma unroll 8
+        for (int c = 0; c < D / 4; ++c) {
+          const float4 o = orow[c];
+          const uint2 e = drow[c];
+          delta = fmaf(o.x, __uint_as_float(e.x << 16), delta);
+          delta = fmaf(o.y, __uint_as_float(e.x & 0xFFFF0000u), delta);
+          delta = fmaf(o.z, __uint_as_float(e.y << 16), delta);
+          delta = fmaf(o.w, __uint_as_float(e.y & 0xFFFF0000u), delta);
+        }
+        st_row[2] = delta;
+      }
+      row_stat_s[(i & 1) * 256 + r_in] = m2l;
+      row_stat_s[(i & 1) * 256 + 128 + r_in] = delta;
+      __syncwarp();
+      if (lane == 0) MbarArrive(&ctl->stat_full[i & 1]);
+    };
+    if constexpr (!kKV) row_stats(0);
+    BwdTile tl;
+    for (uint32_t i = 0; ok && BwdTileAt<kKV>(i, a.S, BH, &tl); ++i) {
+      if constexpr (!kKV) {
+        row_stats(i + 1);
+        if (!ok) break;
+      }
+      const uint32_t ob = i % Sh::kOutBufs;
+      if (!(ok = RoleWait(ctl, &ctl->out_full[ob], (i / Sh::kOutBufs) & 1))) break;
+      TcFenceAfter();
+      const uint32_t b = tl.bh / a.H, h = tl.bh - b * a.H;
+      const uint32_t row0w = tl.row_tile * kTile + quarter * 32;
+      const uint32_t rows_live = row0w < a.S ? (a.S - row0w < 32 ? a.S - row0w : 32) : 0;
+      const size_t flat0 = (static_cast<size_t>(b) * a.S + row0w) * HD + static_cast<size_t>(h) * D;
+      const uint32_t t_out = tmem + ((quarter * 32) << 16) + Sh::kOutCol + ob * Sh::kOutCols;
+#pragma unroll 1
+      for (uint32_t c = 0; c < D; c += 64) {
+        StoreOutRows<64>(t_out + c, slab, lane, 1.0f, a.out + flat0 + c, HD, rows_live, a.shadow, flat0 + c, h * D + c);
+        __syncwarp();   // the staging slab is reused
+        if constexpr (kKV) {
+          StoreOutRows<64>(t_out + D + c, slab, lane, 1.0f, a.out2 + flat0 + c, HD, rows_live, a.shadow2, flat0 + c,
+                           h * D + c);
+          __syncwarp();
+        }
+      }
+      TcFenceBefore();
+      __syncwarp();
+      if (lane == 0) MbarArrive(&ctl->out_empty[ob]);
+    }
+  }
+  __syncwarp();
+  TcFenceBefore();
+  __syncthreads();
+  if (ctl->failed) {
+    if (tid == 0) a.status->wait_timeout = 1;
+    DrainDelay();
+    __syncthreads();
+  }
+  if (warp == 12) {
+    TcFenceAfter();
+    TmemFree(ctl->tmem_base, 512);
+  }
+}
+
 }  // namespace
 
 size_t AttnFwdSmem(int d) { return 128 * d * 2 + 64 * d * 2 + d * 128 + kHalfTileBytes + 1152; }
 size_t AttnDQSmem(int d) { return 2 * 128 * d * 2 + 3 * 64 * d * 2 + kHalfTileBytes + 1152; }
-size_t AttnDKVSmem(int d, int mode) {   // 0: dV, 1: dK, 2: both
+size_t AttnDKVSmem(int d, bool dk) {
   const size_t full = 128 * d * 2, half = 64 * d * 2;
-  return (mode >= 1 ? 2 : 1) * full + 4 * half + (mode == 2 ? 2 : 1) * kHalfTileBytes + 2 * kHalf * 4 + 1152;
+  return (dk ? 2 : 1) * full + 4 * half + kHalfTileBytes + 2 * kHalf * 4 + 1152;
 }
 
 template <typename Kernel>
@@ -715,8 +1088,21 @@ cudaError_t AttnFwdUmma(const CUtensorMap& q, const CUtensorMap& k_half, const C
   return cudaGetLastError();
 }
 
+template <int D, bool kKV>
+static cudaError_t LaunchBwd(const CUtensorMap& x, const CUtensorMap& y, const CUtensorMap& u, const CUtensorMap& w,
+                             const AttnUmmaArgs& a, cudaStream_t s) {
+  const size_t smem = BwdShape<D, kKV>::kSmem;
+  if (cudaError_t e = Configure(AttnBwdKernel<D, kKV>, smem); e != cudaSuccess) return e;
+  const uint32_t tiles = (a.S + kTile - 1) / kTile * a.B * a.H;
+  AttnBwdKernel<D, kKV><<<tiles < a.sms ? tiles : a.sms, kBwdThreads, smem, s>>>(x, y, u, w, a);
+  return cudaGetLastError();
+}
+
 cudaError_t AttnDQUmma(const CUtensorMap& q, const CUtensorMap& dout, const CUtensorMap& k_half,
                        const CUtensorMap& v_half, const AttnUmmaArgs& a, cudaStream_t s) {
+  if (a.fwd_keep)
+    return a.d == 64 ? LaunchBwd<64, false>(q, dout, k_half, v_half, a, s)
+                     : LaunchBwd<128, false>(q, dout, k_half, v_half, a, s);
   dim3 grid((a.S + kTile - 1) / kTile, a.B * a.H);
   const size_t smem = AttnDQSmem(a.d);
   cudaError_t e;
@@ -733,19 +1119,21 @@ cudaError_t AttnDQUmma(const CUtensorMap& q, const CUtensorMap& dout, const CUte
 cudaError_t AttnDKVUmma(int mode, const CUtensorMap& k, const CUtensorMap& v,
                         const CUtensorMap& q_half, const CUtensorMap& dout_half, const AttnUmmaArgs& a,
                         cudaStream_t s) {
+  if (mode == 2)
+    return a.d == 64 ? LaunchBwd<64, true>(k, v, q_half, dout_half, a, s)
+                     : LaunchBwd<128, true>(k, v, q_half, dout_half, a, s);
   dim3 grid((a.S + kTile - 1) / kTile, a.B * a.H);
   cudaError_t e;
-#define SEE_LAUNCH_DKV(D, MODE)                                                              \
+#define SEE_LAUNCH_DKV(D, DK)                                                                \
   do {                                                                                       \
-    const size_t smem = AttnDKVSmem(D, MODE);                                                \
-    if ((e = Configure(AttnDKVUmmaKernel<D, MODE>, smem)) != cudaSuccess) return e;          \
-    AttnDKVUmmaKernel<D, MODE><<<grid, 128, smem, s>>>(k, v, q_half, dout_half, a);   \
+    const size_t smem = AttnDKVSmem(D, DK);                                                  \
+    if ((e = Configure(AttnDKVUmmaKernel<D, DK>, smem)) != cudaSuccess) return e;          \
+    AttnDKVUmmaKernel<D, DK><<<grid, 128, smem, s>>>(k, v, q_half, dout_half, a);   \
   } while (0)
   if (a.d == 64) {
-    if (mode == 2) SEE_LAUNCH_DKV(64, 2); else if (mode == 1) SEE_LAUNCH_DKV(64, 1); else SEE_LAUNCH_DKV(64, 0);
-  } else {   // d = 128: both accumulators would need 384 columns beside S^T and dP^T; not offered
-    if (mode == 2) return cudaErrorInvalidValue;
-    if (mode == 1) SEE_LAUNCH_DKV(128, 1); else SEE_LAUNCH_DKV(128, 0);
+    if (mode == 1) SEE_LAUNCH_DKV(64, true); else SEE_LAUNCH_DKV(64, false);
+  } else {
+    if (mode == 1) SEE_LAUNCH_DKV(128, true); else SEE_LAUNCH_DKV(128, false);
   }
 #undef SEE_LAUNCH_DKV
   return cudaGetLastError();

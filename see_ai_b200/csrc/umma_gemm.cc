@@ -653,6 +653,7 @@ std::string TryAttention(Context* ctx, uint16_t opcode, const AttentionOperands&
   k::AttnUmmaArgs a{};
   a.B = static_cast<uint32_t>(op.B); a.S = static_cast<uint32_t>(op.S);
   a.H = static_cast<uint32_t>(op.H); a.d = static_cast<uint32_t>(op.d);
+  a.sms = impl->sms;
   a.inv_sqrt_d = 1.0f / std::sqrt(static_cast<float>(op.d));
   a.out = op.out;
   a.stats = op.stats;
@@ -673,8 +674,7 @@ std::string TryAttention(Context* ctx, uint16_t opcode, const AttentionOperands&
     a.fwd_keep = nullptr;
     a.dout_bf16 = nullptr;
   }
-  const bool both = dk && op.out2 != nullptr && op.d == 64 &&
-                    (reinterpret_cast<uintptr_t>(op.out2) & 15) == 0;
+  const bool both = dk && op.out2 != nullptr && (reinterpret_cast<uintptr_t>(op.out2) & 15) == 0;
   if (both) {
     a.out2 = op.out2;
     a.shadow2 = op.shadow2;

@@ -128,3 +128,46 @@ def test_longest_sweep_sequence_against_the_exact_family_on_the_device(geom):
         assert np.isfinite(got).all(), name
         err = np.max(np.abs(got - want)) / np.max(np.abs(want))
         assert err < 1e-2, f"{name}: {err:.3g} of scale"
+
+
+# The backward with dedicated warps: sequence ends inside a 64- and a 128-row tile, one tile, fewer and
+# more tiles than SMs (a CTA's second and later tiles), both head widths.
+BACKWARD_GEOMS = [(1, 16, 1, 64), (2, 72, 3, 64), (1, 136, 2, 128), (3, 200, 8, 64), (2, 520, 3, 128),
+                  (16, 256, 12, 64), (13, 264, 12, 64), (9, 264, 12, 128)]
+
+
+@pytest.mark.parametrize("geom", BACKWARD_GEOMS, ids=["B%dS%dH%dd%d" % g for g in BACKWARD_GEOMS])
+def test_one_walk_backward_against_the_separate_kernels(geom):
+    """In one range of lazy coherence dQ takes delta from the forward's kept O and dK, dV come from one
+    kernel; as one-instruction ranges each has its own.  dV has the same operands and order: the same bits.
+    dQ and dK see delta from O (P rounded to bf16) instead of from f32 P: 2^-9 of P, within the 1e-2 of
+    scale this file holds every output to."""
+    Bq, S, H, d = geom
+    rng = np.random.default_rng(S * 17 + d + Bq)
+    t, prog, arena, ro, td = build(rng, Bq, S, H, d)
+
+    def run(one_range):
+        got = arena.copy()
+        be = B.CudaBackend(0)
+        be.set_coherence(B.COHERENCE_LAZY)
+        be.bind(got, ro)
+        if one_range:
+            be.run(prog(REL))
+        else:
+            for ins in prog(REL):
+                be.run([ins])
+        assert be.counters().relaxed_executions == 4
+        out = {}
+        for name in ("o", "dq", "dk", "dv"):
+            be.host_needs(t[name], 4 * td)
+            out[name] = got[t[name]:t[name] + 4 * td].view(np.float32).copy()
+        be.close()
+        return out
+
+    one, separate = run(True), run(False)
+    assert np.array_equal(one["o"], separate["o"])
+    assert np.array_equal(one["dv"], separate["dv"])
+    for name in ("dq", "dk"):
+        assert np.isfinite(one[name]).all(), name
+        err = np.max(np.abs(one[name] - separate[name])) / np.max(np.abs(separate[name]))
+        assert err < 1e-2, f"{name}: {err:.3g} of scale"
