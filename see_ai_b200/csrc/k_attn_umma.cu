@@ -278,7 +278,7 @@ AttnFwdUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   if (tid == 0) issue_a(0);
 
   for (uint32_t t = 0; t < total; ++t) {
-    if (tid == 0) {   // only the issuing thread needs the operands' arrival
+    if (warp == 0 && ElectOne()) {   // only the issuing thread needs the operands' arrival
       if (!MbarWait(&ctl->bar_a, t & 1)) failed = 1;
       TcFenceAfter();
       if (!failed) MmaRowRow<D, 64>(tmem, q_s, k_s);
@@ -288,7 +288,7 @@ AttnFwdUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     // are all free again once it arrives, and O is at rest.
     if (!MbarWait(&ctl->mma, t & 1)) failed = 1;
     TcFenceAfter();
-    if (tid == 0 && !failed) {
+    if (warp == 0 && ElectOne() && !failed) {
       if (t + 1 < total) issue_a(t + 1);
       issue_b(t);
     }
@@ -351,13 +351,13 @@ AttnFwdUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     FenceProxyAsync();
     TcFenceBefore();
     if (__syncthreads_or(failed)) { failed = 1; break; }
-    if (tid == 0) {
+    if (warp == 0 && ElectOne()) {
       if (!MbarWait(&ctl->bar_b, t & 1)) failed = 1;
       TcFenceAfter();
       if (!failed) MmaPRows<D>(tmem + 64, p_s, v_s, t != 0);
     }
   }
-  if (tid == 0) UmmaCommit(&ctl->mma);
+  if (warp == 0 && ElectOne()) UmmaCommit(&ctl->mma);
   if (!failed && !MbarWait(&ctl->mma, total & 1)) failed = 1;
   TcFenceAfter();
   failed = __syncthreads_or(failed);

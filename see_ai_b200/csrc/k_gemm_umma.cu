@@ -309,7 +309,7 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
   } else if (warp == 1) {
     // ---- MMA issuer ----
-    if (lane == 0) {
+    if (ElectOne()) {
       const uint32_t idesc = MakeInstrDesc(kBlockM, kTN);
       for (uint32_t kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const uint32_t s = it % kStages, round = it / kStages;
@@ -643,7 +643,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
     }
   } else if (warp == 1) {
     // ---- MMA issuer ----
-    if (lane == 0 && cta_rank == 0) {   // (a pair's odd CTA issues nothing: its memories are read by the even one's MMAs)
+    if (ElectOne() && cta_rank == 0) {   // (a pair's odd CTA issues nothing: its memories are read by the even one's MMAs)
       const uint32_t idesc = MakeInstrDesc(T::kRowsPerTile, kTN);
       uint32_t it = 0, lt = 0;
       bool ok = true;

@@ -225,7 +225,7 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
     }
   } else if (warp == 1) {
     // ---- MMA issue ----
-    if (lane == 0) {
+    if (ElectOne()) {
       const uint32_t idesc_rows = MakeInstrDesc(kRows, kWide);                      // dT: rows x k
       const uint32_t idesc_cols = MakeInstrDesc(128, kWide) | kInstrDescAMnMajor;   // dB, dA: columns x rows
       uint32_t it = 0;
