@@ -4,8 +4,8 @@ Two executors with one Python face (`run(program, arena, rodata, ...)`):
 
 * `RefExecutor`    — the reference's own CPU executor (oracle/_ref/libseeml_ref.so,
                      compiled from the reference's sources by oracle/Makefile).
-* `OracleExecutor` — our C restatement of the same arithmetic
-                     (oracle/libsee_oracle.so from oracle/see_oracle.c).
+* `OracleExecutor` — our restatement of the same arithmetic
+                     (oracle/libsee_oracle.so from oracle/see_oracle.cc).
 
 Only tests, the smoke check and the bench's CPU-baseline leg may import this
 module.  The product package must never import it.

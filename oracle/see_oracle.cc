@@ -1,4 +1,4 @@
-/* TEST INFRASTRUCTURE — a plain-C restatement of the reference CPU executor's
+/* TEST INFRASTRUCTURE — a plain restatement of the reference CPU executor's
  * arithmetic, used only as a checker by tests, the smoke check and the bench's
  * CPU-baseline leg.  Nothing the product ships calls into this file.
  *
@@ -8,10 +8,12 @@
  * reference executor itself (oracle/_ref) on seeded instruction programs, and
  * to the reference's known-answer vectors (tests/test_oracle_known_answers.py).
  *
- * Everything is serial; reductions that the reference folds per parallel chunk
- * are folded here in the same shape-derived chunk geometry, so the bits do not
- * depend on a thread count on either side.  Build: -O2 -ffp-contract=off (no
- * fused multiply-add may appear; the reference's x86 build has none).
+ * Every output element is made by one thread, in the reference's order; the GEMMs and
+ * the attention rows are dealt out to several threads (a single one took twenty minutes
+ * over ten steps of the 12-layer decoder).  Reductions that the reference folds per
+ * parallel chunk are folded here in the same shape-derived chunk geometry, so the bits do
+ * not depend on a thread count on either side.  Build: -O3 -ffp-contract=off (no fused
+ * multiply-add may appear; the reference's x86 build has none).
  *
  * Each function cites the reference lines it follows.
  */
@@ -21,6 +23,31 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+
+#include <algorithm>
+#include <atomic>
+#include <thread>
+#include <vector>
+
+/* f(i) for every i < n, on several threads where `work` (operations, roughly) is worth starting them. */
+template <typename F>
+static void parallel_for(size_t n, double work, F f) {
+  const size_t threads = work < 2e6 ? 1 : std::min<size_t>({n, std::max(1u, std::thread::hardware_concurrency()), 32});
+  if (threads <= 1) {
+    for (size_t i = 0; i < n; ++i) f(i);
+    return;
+  }
+  const size_t grain = std::max<size_t>(1, n / (threads * 8));
+  std::atomic<size_t> next{0};
+  auto body = [&] {
+    for (size_t i; (i = next.fetch_add(grain)) < n;)
+      for (size_t j = i; j < std::min(n, i + grain); ++j) f(j);
+  };
+  std::vector<std::thread> pool;
+  for (size_t t = 1; t < threads; ++t) pool.emplace_back(body);
+  body();
+  for (auto& t : pool) t.join();
+}
 
 typedef struct {
   uint16_t opcode, flags;
@@ -101,52 +128,96 @@ static float widen(const void* B, int b_type, size_t idx) {
   return ((const float*)B)[idx];
 }
 
+/* Both orders are functions of one output element alone, so rows and columns may be taken in blocks and by several
+ * threads: the operations of an element, and their order, stay as they are. */
+enum { GEMM_ROWS = 8, GEMM_COLS = 256 };
+typedef float Lanes __attribute__((vector_size(32)));
+
+/* B widened to f32 (times col_scale of its column, N columns); NULL scale: the matrix itself where it is f32 already. */
+static const float* widen_all(const void* B, int b_type, size_t rows, size_t cols, const float* col_scale, float** owned) {
+  *owned = NULL;
+  if (b_type == 0 && !col_scale) return (const float*)B;
+  float* w = *owned = (float*)malloc((rows * cols + 1) * sizeof(float));
+  parallel_for(rows, 4.0 * rows * cols, [&](size_t r) {
+    for (size_t c = 0; c < cols; ++c) {
+      const float b = widen(B, b_type, r * cols + c);
+      w[r * cols + c] = col_scale ? b * col_scale[c] : b;
+    }
+  });
+  return w;
+}
+
 /* Quad order (gemm.cc:73-187): c += ((a0b0 + a1b1) + a2b2) + a3b3 over k-quads
  * from k = 0, then single terms; alpha folded into each A element, a column
  * scale into each widened B element.  a_t: A is [K, M]. */
 static void gemm_quad(const float* A, const void* B, int b_type, float* C, size_t M, size_t N,
                       size_t K, float alpha, int a_t, const float* col_scale, int accumulate) {
-  for (size_t m = 0; m < M; ++m) {
-    for (size_t n = 0; n < N; ++n) {
-      float c = accumulate ? C[m * N + n] : 0.0f;
-      size_t k = 0;
-      for (; k + 4 <= K; k += 4) {
-        float a[4], b[4];
-        for (int q = 0; q < 4; ++q) {
-          a[q] = alpha * (a_t ? A[(k + q) * M + m] : A[m * K + k + q]);
-          b[q] = widen(B, b_type, (k + q) * N + n);
-          if (col_scale) b[q] = b[q] * col_scale[n];
-        }
-        c += a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3];
+  float* owned;
+  const float* W = widen_all(B, b_type, K, N, col_scale, &owned);
+  const size_t mb = (M + GEMM_ROWS - 1) / GEMM_ROWS, nb = (N + GEMM_COLS - 1) / GEMM_COLS;
+  float* out = (float*)malloc((M * N + 1) * sizeof(float));
+  parallel_for(mb * nb, 1.0 * M * N * K, [&](size_t block) {
+    const size_t bm = block / nb, bn = block % nb, m0 = bm * GEMM_ROWS, rows = M - m0 < GEMM_ROWS ? M - m0 : GEMM_ROWS;
+    const size_t n0 = bn * GEMM_COLS, cols = N - n0 < GEMM_COLS ? N - n0 : GEMM_COLS;
+    float c[GEMM_ROWS][GEMM_COLS];
+    for (size_t r = 0; r < rows; ++r)
+      for (size_t n = 0; n < cols; ++n) c[r][n] = accumulate ? C[(m0 + r) * N + n0 + n] : 0.0f;
+    size_t k = 0;
+    for (; k + 4 <= K; k += 4) {
+      const float *b0 = W + k * N + n0, *b1 = b0 + N, *b2 = b1 + N, *b3 = b2 + N;
+      for (size_t r = 0; r < rows; ++r) {
+        float a[4];
+        for (int q = 0; q < 4; ++q) a[q] = alpha * (a_t ? A[(k + q) * M + m0 + r] : A[(m0 + r) * K + k + q]);
+        for (size_t n = 0; n < cols; ++n) c[r][n] += a[0] * b0[n] + a[1] * b1[n] + a[2] * b2[n] + a[3] * b3[n];
       }
-      for (; k < K; ++k) {
-        const float a = alpha * (a_t ? A[k * M + m] : A[m * K + k]);
-        float b = widen(B, b_type, k * N + n);
-        if (col_scale) b = b * col_scale[n];
-        c += a * b;
-      }
-      C[m * N + n] = c;
     }
-  }
+    for (; k < K; ++k)
+      for (size_t r = 0; r < rows; ++r) {
+        const float a = alpha * (a_t ? A[k * M + m0 + r] : A[(m0 + r) * K + k]);
+        for (size_t n = 0; n < cols; ++n) c[r][n] += a * W[k * N + n0 + n];
+      }
+    for (size_t r = 0; r < rows; ++r) memcpy(out + (m0 + r) * N + n0, c[r], cols * sizeof(float));
+  });
+  memcpy(C, out, M * N * sizeof(float));
+  free(out);
+  free(owned);
 }
 
 /* Lane order (gemm.cc:346-527): product k into lane k mod 8, lanes summed
  * 0..7, times alpha; a reduction-axis scale multiplies A first (gemm.cc:652-674). */
 static void gemm_lane(const float* A, const void* B, int b_type, float* C, size_t M, size_t N,
                       size_t K, float alpha, const float* k_scale) {
-  for (size_t m = 0; m < M; ++m) {
-    for (size_t n = 0; n < N; ++n) {
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (size_t k = 0; k < K; ++k) {
-        float a = A[m * K + k];
-        if (k_scale) a = a * k_scale[k];
-        acc[k % 8] += a * widen(B, b_type, n * K + k);
+  float *owned, *owned_a;
+  const float* W = widen_all(B, b_type, N, K, NULL, &owned);
+  const float* X = widen_all(A, 0, M, K, k_scale, &owned_a);
+  const size_t mb = (M + 3) / 4;
+  float* out = (float*)malloc((M * N + 1) * sizeof(float));
+  parallel_for(N, 1.0 * M * N * K, [&](size_t n) {
+    for (size_t bm = 0; bm < mb; ++bm) {
+      const size_t m0 = bm * 4, rows = M - m0 < 4 ? M - m0 : 4;
+      Lanes acc[4];
+      memset(acc, 0, sizeof(acc));
+      size_t k = 0;
+      for (; k + 8 <= K; k += 8) {
+        Lanes b, a;
+        memcpy(&b, W + n * K + k, sizeof(b));
+        for (size_t r = 0; r < rows; ++r) {
+          memcpy(&a, X + (m0 + r) * K + k, sizeof(a));
+          acc[r] += a * b;
+        }
       }
-      float s = acc[0];
-      for (int l = 1; l < 8; ++l) s += acc[l];
-      C[m * N + n] = alpha * s;
+      for (size_t r = 0; r < rows; ++r) {
+        for (size_t t = k; t < K; ++t) acc[r][t % 8] += X[(m0 + r) * K + t] * W[n * K + t];
+        float s = acc[r][0];
+        for (int l = 1; l < 8; ++l) s += acc[r][l];
+        out[(m0 + r) * N + n] = alpha * s;
+      }
     }
-  }
+  });
+  memcpy(C, out, M * N * sizeof(float));
+  free(out);
+  free(owned);
+  free(owned_a);
 }
 
 /* Epilogues (gemm.cc:536-578): addend d + s, then bias, then activation. */
@@ -485,10 +556,10 @@ static void attn_fwd(const float* q, const float* k, const float* v, float* o, f
                      float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts) {
   const size_t D = H * d;
   const float inv_sqrt_d = 1.0f / sqrtf((float)d);
-  float* scratch = (float*)malloc(S * sizeof(float));
-  for (size_t u = 0; u < B * H * S; ++u) {
+  parallel_for(B * H * S, 1.0 * B * H * S * S * d, [&](size_t u) {
     const size_t b = u / (H * S), h = (u / S) % H, i = u % S;
     const float* qi = q + (b * S + i) * D + h * d;
+    float* scratch = probs ? NULL : (float*)malloc(S * sizeof(float));
     float* prow = probs ? probs + u * S : scratch;
     size_t j0 = 0;
     if (starts) {
@@ -522,26 +593,26 @@ static void attn_fwd(const float* q, const float* k, const float* v, float* o, f
       float* st = stats + u * 4;
       st[0] = row_max; st[1] = inv_denom; st[2] = 0.0f; st[3] = (float)j0;
     }
-  }
-  free(scratch);
+    free(scratch);
+  });
 }
 static void attn_dp(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H,
                     size_t d) {
   const size_t D = H * d;
-  for (size_t u = 0; u < B * H * S; ++u) {
+  parallel_for(B * H * S, 1.0 * B * H * S * S * d, [&](size_t u) {
     const size_t b = u / (H * S), h = (u / S) % H, i = u % S;
     const float* doi = dout + (b * S + i) * D + h * d;
     float* row = dp + u * S;
     for (size_t j = 0; j <= i; ++j) row[j] = (float)dot_d(doi, v + (b * S + j) * D + h * d, d);
     for (size_t j = i + 1; j < S; ++j) row[j] = 0.0f;
-  }
+  });
 }
 /* out_j = sum_{i>=j} (w[i, j] [* scale]) * x_i : dV (w = P, x = dO) and dK (w = dS, x = Q). */
 static void attn_col(const float* w, const float* x, float* out, size_t B, size_t S, size_t H,
                      size_t d, int scaled) {
   const size_t D = H * d;
   const float inv_sqrt_d = 1.0f / sqrtf((float)d);
-  for (size_t u = 0; u < B * H * S; ++u) {
+  parallel_for(B * H * S, 1.0 * B * H * S * S * d, [&](size_t u) {
     const size_t b = u / (H * S), h = (u / S) % H, j = u % S;
     float* oj = out + (b * S + j) * D + h * d;
     for (size_t c = 0; c < d; ++c) oj[c] = 0.0f;
@@ -551,13 +622,13 @@ static void attn_col(const float* w, const float* x, float* out, size_t B, size_
       const float* xi = x + (b * S + i) * D + h * d;
       for (size_t c = 0; c < d; ++c) oj[c] += g * xi[c];
     }
-  }
+  });
 }
 static void attn_dq(const float* ds, const float* k, float* dq, size_t B, size_t S, size_t H,
                     size_t d) {
   const size_t D = H * d;
   const float inv_sqrt_d = 1.0f / sqrtf((float)d);
-  for (size_t u = 0; u < B * H * S; ++u) {
+  parallel_for(B * H * S, 1.0 * B * H * S * S * d, [&](size_t u) {
     const size_t b = u / (H * S), h = (u / S) % H, i = u % S;
     float* dqi = dq + (b * S + i) * D + h * d;
     for (size_t c = 0; c < d; ++c) dqi[c] = 0.0f;
@@ -566,7 +637,7 @@ static void attn_dq(const float* ds, const float* k, float* dq, size_t B, size_t
       const float* kj = k + (b * S + j) * D + h * d;
       for (size_t c = 0; c < d; ++c) dqi[c] += g * kj[c];
     }
-  }
+  });
 }
 static void softmax_rows_bwd(const float* probs, const float* dp, float* ds, size_t rows,
                              size_t cols) {
@@ -589,14 +660,14 @@ static void attn_dq_tiled(const float* q, const float* k, const float* v, const 
                           float* stats, float* dq, size_t B, size_t S, size_t H, size_t d) {
   const size_t D = H * d;
   const float inv_sqrt_d = 1.0f / sqrtf((float)d);
-  float* prow = (float*)malloc(2 * S * sizeof(float));
-  float* dprow = prow + S;
-  for (size_t u = 0; u < B * H * S; ++u) {
+  parallel_for(B * H * S, 1.0 * B * H * S * S * d, [&](size_t u) {
     const size_t b = u / (H * S), h = (u / S) % H, i = u % S;
     const float* qi = q + (b * S + i) * D + h * d;
     const float* doi = dout + (b * S + i) * D + h * d;
     float* st = stats + u * 4;
     const size_t j0 = stats_start(st[3], i);
+    float* prow = (float*)malloc(2 * S * sizeof(float));
+    float* dprow = prow + S;
     double dot = 0.0;
     for (size_t j = j0; j <= i; ++j)
       prow[j] = prob_of(qi, k + (b * S + j) * D + h * d, d, inv_sqrt_d, st[0], st[1]);
@@ -614,15 +685,15 @@ static void attn_dq_tiled(const float* q, const float* k, const float* v, const 
       const float* kj = k + (b * S + j) * D + h * d;
       for (size_t c = 0; c < d; ++c) dqi[c] += g * kj[c];
     }
-  }
-  free(prow);
+    free(prow);
+  });
 }
 static void attn_dkv_tiled(int want_dk, const float* q, const float* k, const float* v,
                            const float* dout, const float* stats, float* out, size_t B, size_t S,
                            size_t H, size_t d) {
   const size_t D = H * d;
   const float inv_sqrt_d = 1.0f / sqrtf((float)d);
-  for (size_t u = 0; u < B * H * S; ++u) {
+  parallel_for(B * H * S, 1.0 * B * H * S * S * d, [&](size_t u) {
     const size_t b = u / (H * S), h = (u / S) % H, j = u % S;
     const float* kj = k + (b * S + j) * D + h * d;
     const float* vj = v + (b * S + j) * D + h * d;
@@ -642,7 +713,7 @@ static void attn_dkv_tiled(int want_dk, const float* q, const float* k, const fl
         for (size_t c = 0; c < d; ++c) oj[c] += p * doi[c];
       }
     }
-  }
+  });
 }
 
 /* ---- dispatch: runtime/executor/cpu_backend.cc:260-646 -------------------------------- */
@@ -826,6 +897,7 @@ static int execute(Oracle* o, const Instr* ins, const StepParams* sp) {
 }
 
 /* ---- C face, same shape as the reference shim's ------------------------------------------ */
+extern "C" {
 void* seeo_create(void) { return calloc(1, sizeof(Oracle)); }
 void seeo_destroy(void* h) { free(h); }
 const char* seeo_last_error(void* h) { return ((Oracle*)h)->error; }
@@ -859,3 +931,4 @@ int64_t seeo_run(void* h, const void* instrs, uint64_t begin, uint64_t end, cons
   }
   return 0;
 }
+}  /* extern "C" */

@@ -1,6 +1,6 @@
 """Pins the CPU checkers.
 
-(a) Our C restatement (oracle/see_oracle.c) reproduces, bit for bit, every
+(a) Our C restatement (oracle/see_oracle.cc) reproduces, bit for bit, every
     extent of every instruction in the write traces the reference's own probe
     recorded for eight plans compiled by the reference compiler.
 (b) The reference executor built from the reference's sources (oracle/_ref),
