@@ -139,6 +139,7 @@ Status CudaBackend::Bind(uint8_t* arena, uint64_t arena_bytes, const uint8_t* ro
     cudaFree(new_arena); cudaFree(new_rodata);
     return std::unexpected(CudaErr(e, "bind: sync"));
   }
+  if (d_arena_) ++buffer_moves_;
   cudaFree(d_arena_);
   cudaFree(d_rodata_);
   d_arena_ = static_cast<uint8_t*>(new_arena);
@@ -183,6 +184,7 @@ Status CudaBackend::BindDeviceImage(uint64_t arena_bytes, const uint8_t* prefix,
       return fail(e, "bind: rodata upload");
   }
   if (auto e = cudaStreamSynchronize(stream_); e != cudaSuccess) return fail(e, "bind: sync");
+  if (d_arena_) ++buffer_moves_;
   cudaFree(d_arena_);
   cudaFree(d_rodata_);
   d_arena_ = static_cast<uint8_t*>(new_arena);
@@ -245,6 +247,7 @@ Status CudaBackend::WriteArenaPinned(uint64_t off0, uint64_t bytes0, const void*
 Status CudaBackend::BindSource(const uint8_t* data, uint64_t bytes) {
   cudaSetDevice(device_);
   cudaStreamSynchronize(stream_);
+  if (d_source_) ++buffer_moves_;
   cudaFree(d_source_);
   d_source_ = nullptr;
   source_bytes_ = 0;
@@ -345,6 +348,7 @@ Status CudaBackend::EnsureScratch(uint64_t row_doubles) {
   // Growing scratch replaces the buffer: drain the stream first so no queued
   // kernel still reads the old one.
   if (auto r = Check(cudaStreamSynchronize(stream_), "scratch sync"); !r) return r;
+  if (d_rows_) ++buffer_moves_;
   cudaFree(d_rows_);
   d_rows_ = nullptr;
   rows_capacity_ = 0;
@@ -397,6 +401,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
   if (rows) (void)EnsureScratch(rows);
   if (split > split_capacity_) {
     cudaStreamSynchronize(stream_);
+    if (d_split_) ++buffer_moves_;
     cudaFree(d_split_);
     d_split_ = nullptr;
     split_capacity_ = 0;
@@ -408,6 +413,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
   }
   if (gsum > gsum_capacity_) {
     cudaStreamSynchronize(stream_);
+    if (d_gsum_) ++buffer_moves_;
     cudaFree(d_gsum_);
     d_gsum_ = nullptr;
     gsum_capacity_ = 0;
@@ -442,6 +448,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
                                                                        program[begin + i].out[1]));
   if (partial_floats > lora_partials_capacity_) {
     cudaStreamSynchronize(stream_);
+    if (d_lora_partials_) ++buffer_moves_;
     cudaFree(d_lora_partials_);
     d_lora_partials_ = nullptr;
     lora_partials_capacity_ = 0;
@@ -483,6 +490,7 @@ Status CudaBackend::PrepareLoraFolds(const Instruction* program, size_t begin, u
     cudaStreamSynchronize(stream_);   // queued kernels may still read the old buffers
   auto grow = [&](void** buf, uint64_t* cap, uint64_t need, size_t elem) -> Status {
     if (need <= *cap) return {};
+    if (*buf) ++buffer_moves_;
     cudaFree(*buf);
     *buf = nullptr;
     *cap = 0;
@@ -508,6 +516,7 @@ Status CudaBackend::PrepareLoraFolds(const Instruction* program, size_t begin, u
 }
 
 void CudaBackend::FreeLoraRanges() {
+  buffer_moves_ += lora_ranges_.size();
   for (auto& [key, rb] : lora_ranges_) {
     cudaFree(rb.table);
     cudaFree(rb.weights);
@@ -597,9 +606,11 @@ void CudaBackend::PlanAdamGroups(std::span<const Instruction> program, size_t be
   if (table.empty()) return;
   if (table.size() > adam_table_capacity_) {
     cudaStreamSynchronize(stream_);
+    if (d_adam_table_) ++buffer_moves_;
     cudaFree(d_adam_table_);
     d_adam_table_ = nullptr;
     adam_table_capacity_ = 0;
+    adam_table_.clear();
     void* p = nullptr;
     if (cudaMalloc(&p, table.size() * sizeof(k::AdamTensor)) != cudaSuccess) {
       cudaGetLastError();
@@ -613,6 +624,10 @@ void CudaBackend::PlanAdamGroups(std::span<const Instruction> program, size_t be
   // The previous range's launches may still be reading the table.
   cudaStreamSynchronize(stream_);
   cudaMemcpy(d_adam_table_, table.data(), table.size() * sizeof(k::AdamTensor), cudaMemcpyHostToDevice);
+  if (!adam_table_.empty() && (adam_table_.size() != table.size() ||
+                               std::memcmp(adam_table_.data(), table.data(), table.size() * sizeof(k::AdamTensor)) != 0))
+    ++buffer_moves_;
+  adam_table_ = std::move(table);
 }
 
 void CudaBackend::PlanMergeRuns(std::span<const Instruction> program, size_t begin, size_t end) {
@@ -941,6 +956,7 @@ void CudaBackend::PlanAttentionKeeps(std::span<const Instruction> program, size_
   if (slots == 0) return;
   if (elems > attn_keep_elems_) {   // grow: every buffer anew
     cudaStreamSynchronize(stream_);
+    buffer_moves_ += attn_keep_pool_.size();
     for (float* p : attn_keep_pool_) cudaFree(p);
     attn_keep_pool_.clear();
     attn_keep_elems_ = elems;
@@ -2052,6 +2068,8 @@ k::AdamScalars CudaBackend::ScalarsOf(const StepParams& params) {
 }
 
 void CudaBackend::SetCapturing(bool on) { capturing_ = on; }
+
+uint64_t CudaBackend::BufferGeneration() const { return buffer_moves_ + umma::BufferMoves(&umma_->ctx); }
 
 Status CudaBackend::UploadStepScalars(const StepParams& params) {
   cudaSetDevice(device_);

@@ -170,6 +170,8 @@ class CudaBackend {
   // kernel of the stream that carries the values as its parameters, so every replay
   // sees its own step's values however far the host runs ahead of the device.
   void SetCapturing(bool on);
+  // Changes whenever a device buffer that captured launches may address is freed, or a table they read changes.
+  uint64_t BufferGeneration() const;
   Status UploadStepScalars(const StepParams& params);
   static k::AdamScalars ScalarsOf(const StepParams& params);
 
@@ -245,6 +247,7 @@ class CudaBackend {
   static constexpr uint64_t kPublishedBytes = 4096, kFlushStaging = 2ull << 20;
 
   Coherence coherence_ = Coherence::kStrict;
+  uint64_t buffer_moves_ = 0;   // this object's part of BufferGeneration
   std::vector<std::pair<uint64_t, uint64_t>> host_dirty_;
   std::vector<std::pair<uint64_t, uint64_t>> device_dirty_;
   std::string deferred_error_;
@@ -278,6 +281,7 @@ class CudaBackend {
   std::vector<AdamGroup> adam_groups_;
   k::AdamTensor* d_adam_table_ = nullptr;
   size_t adam_table_capacity_ = 0;
+  std::vector<k::AdamTensor> adam_table_;   // what d_adam_table_ holds
 
   // A run of merge deltas (kFill with zero, kGemmAccNN over exactly that tensor), issued as one launch from the first
   // kFill (engine / lazy coherence only): the filled tensor never goes through memory.  `first` is a range position;

@@ -103,6 +103,17 @@ void UpdateEngine::DropGraphs() {
   }
 }
 
+// Scratch is sized per range, so a later range that needs more (a training step after two evaluations) replaces
+// buffers that an earlier range's graph writes.  Such a range starts over: eager once, then captured again.
+bool UpdateEngine::Replayable(GraphSlot* slot) {
+  if (!use_graphs_ || !slot || !slot->exec) return false;
+  if (slot->buffers == backend_->BufferGeneration()) return true;
+  cudaGraphExecDestroy(slot->exec);
+  slot->exec = nullptr;
+  slot->runs = 0;
+  return false;
+}
+
 UpdateEngine::~UpdateEngine() {
   if (backend_) cudaStreamSynchronize(backend_->stream());
   DropGraphs();
@@ -366,7 +377,7 @@ Status UpdateEngine::RunRange(const std::vector<Instruction>& prog, size_t begin
   Status result{};
   bool has_opt = false;
   for (size_t i = begin; i < end; ++i) has_opt = has_opt || prog[i].opcode == kAdamWStep || prog[i].opcode == kSgdStep;
-  if (use_graphs_ && slot && slot->exec) {
+  if (Replayable(slot)) {
     if (has_opt)
       if (auto r = backend_->UploadStepScalars(params); !r) return r;
     if (auto e = cudaGraphLaunch(slot->exec, s); e != cudaSuccess)
@@ -401,6 +412,7 @@ Status UpdateEngine::RunRange(const std::vector<Instruction>& prog, size_t begin
           result = std::unexpected(std::string("engine: graph instantiate: ") + cudaGetErrorString(ie));
         } else {
           slot->exec = exec;
+          slot->buffers = backend_->BufferGeneration();
           if (auto le = cudaGraphLaunch(exec, s); le != cudaSuccess)
             result = std::unexpected(std::string("engine: graph launch: ") + cudaGetErrorString(le));
         }
@@ -584,7 +596,7 @@ Status UpdateEngine::RunMerge(bool* all_finite) {
   cudaMemsetAsync(d_tally_, 0, 4 * sizeof(unsigned long long), s);
   // Where the deltas that leave are exactly the ones the merge program makes, its kernels count the non-finite values
   // as they write them (a replay counts as its capture did).
-  const bool replay = use_graphs_ && g_merge_.exec;
+  const bool replay = Replayable(&g_merge_);
   if (!replay) backend_->SetMergeTally(emits_are_merge_deltas_ ? d_tally_ + 2 : nullptr);
   if (auto r = RunRange(merge_, 0, merge_.size(), &g_merge_, nullptr); !r) return r;
   if (!replay) merge_counts_ = emits_are_merge_deltas_ && backend_->merge_counted() == emit_.size();

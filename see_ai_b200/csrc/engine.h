@@ -142,7 +142,10 @@ class UpdateEngine {
   struct GraphSlot {
     cudaGraphExec_t exec = nullptr;
     int runs = 0;
+    uint64_t buffers = 0;   // CudaBackend::BufferGeneration at the capture
   };
+  // Whether the slot's graph can be replayed; drops it when a buffer it addresses has been replaced since.
+  bool Replayable(GraphSlot* slot);
   Status RunRange(const std::vector<Instruction>& prog, size_t begin, size_t end, GraphSlot* slot,
                   float* phase_ms);
   StepParams MakeParams() const;

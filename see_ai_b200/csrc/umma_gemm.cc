@@ -73,6 +73,7 @@ struct Impl {
   // ended by any write into that range.
   struct SplitTag { bool valid = false, transposed = false; uint64_t off = 0, M = 0, K = 0; const float* k_scale = nullptr; } split_tag;
   uint32_t sms = 148;
+  uint64_t moves = 0;   // device buffers of this context freed since it was made (BufferMoves)
   std::map<WeightKey, uint16_t*> split_weights;          // frozen B operands, once per binding
 };
 
@@ -106,8 +107,11 @@ void Destroy(Context* ctx) {
   ctx->impl = nullptr;
 }
 
+uint64_t BufferMoves(const Context* ctx) { return ctx->impl ? ctx->impl->moves : 0; }
+
 void InvalidateAll(Context* ctx) {
   if (!ctx->impl) return;
+  ctx->impl->moves += ctx->impl->weights.size() + ctx->impl->split_weights.size();
   for (auto& [key, buf] : ctx->impl->weights) cudaFree(buf);
   ctx->impl->weights.clear();
   for (auto& [key, buf] : ctx->impl->split_weights) cudaFree(buf);
@@ -176,6 +180,7 @@ void PlanRange(Context* ctx, const Instruction* program, size_t begin, size_t en
       cudaDeviceSynchronize();
       const uint64_t cap = std::max(attn, impl->pack_capacity);
       if (attn > impl->pack_capacity) {
+        impl->moves += impl->packs.size();
         for (auto& e : impl->packs) cudaFree(e.rows);
         impl->packs.clear();
       }
@@ -197,6 +202,7 @@ void PlanRange(Context* ctx, const Instruction* program, size_t begin, size_t en
   for (auto& slot : impl->acts) {
     if (slot.capacity >= need) continue;
     if (!drained) { cudaDeviceSynchronize(); drained = true; }
+    if (slot.buf) ++impl->moves;
     cudaFree(slot.buf);
     slot.buf = nullptr;
     slot.capacity = 0;
@@ -322,6 +328,7 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
     if (slot->capacity < need) {
       // Replacing the buffer: queued kernels may still read the old one.
       cudaStreamSynchronize(stream);
+      if (slot->buf) ++impl->moves;
       cudaFree(slot->buf);
       slot->buf = nullptr;
       slot->capacity = 0;
@@ -414,10 +421,12 @@ bool SplitGemmEligible(const k::GemmArgs& a, bool wide) {
            misaligned(a.b_col_scale) || misaligned(a.a_k_scale));
 }
 
-static bool GrowSplit(uint16_t** buf, uint64_t* cap, uint64_t need, cudaStream_t stream, bool whole_device = false) {
+static bool GrowSplit(Impl* impl, uint16_t** buf, uint64_t* cap, uint64_t need, cudaStream_t stream,
+                      bool whole_device = false) {
   if (need <= *cap) return true;
   // Queued kernels may still read the old buffer.
   if (whole_device) cudaDeviceSynchronize(); else cudaStreamSynchronize(stream);
+  if (*buf) ++impl->moves;
   cudaFree(*buf);
   *buf = nullptr;
   *cap = 0;
@@ -448,8 +457,8 @@ void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size
     if (RefSpace(ins.in[1]) == kArena) need_b = std::max(need_b, N * 3 * PaddedK(K));
   }
   if (need_a > impl->split_a_capacity) impl->split_tag.valid = false;
-  GrowSplit(&impl->split_a, &impl->split_a_capacity, need_a, nullptr, true);
-  GrowSplit(&impl->split_b, &impl->split_b_capacity, need_b, nullptr, true);
+  GrowSplit(impl, &impl->split_a, &impl->split_a_capacity, need_a, nullptr, true);
+  GrowSplit(impl, &impl->split_b, &impl->split_b_capacity, need_b, nullptr, true);
 }
 
 std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_space, uint64_t a_off, int b_space,
@@ -461,7 +470,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   if (exact_b && b_space == 0) return {};
   const uint64_t Kp = PaddedK(a.K);
   if (a.M * 3 * Kp > impl->split_a_capacity) impl->split_tag.valid = false;
-  if (!GrowSplit(&impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream))
+  if (!GrowSplit(impl, &impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream))
     return "tensor-core path: operand-piece allocation failed";
   // A: [M, K], or [K, M] for the transposed-A form.
   auto& tag = impl->split_tag;
@@ -490,7 +499,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
       impl->split_weights.emplace(key, b);
     }
   } else {
-    if (!GrowSplit(&impl->split_b, &impl->split_b_capacity, a.N * 3 * Kp, stream))
+    if (!GrowSplit(impl, &impl->split_b, &impl->split_b_capacity, a.N * 3 * Kp, stream))
       return "tensor-core path: operand-piece allocation failed";
     b = impl->split_b;
     k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);

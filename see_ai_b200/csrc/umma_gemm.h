@@ -31,6 +31,9 @@ void Destroy(Context* ctx);
 // an activation's bf16 copy is reused by every GEMM that reads the same arena
 // range until an instruction writes into that range.
 void InvalidateAll(Context* ctx);
+// How many device buffers of the context have been freed so far.  Captured launches hold their addresses: a graph
+// captured at another count must not be replayed.
+uint64_t BufferMoves(const Context* ctx);
 void InvalidateRange(Context* ctx, uint64_t arena_off, uint64_t bytes);
 void PlanRange(Context* ctx, const Instruction* program, size_t begin, size_t end);
 
