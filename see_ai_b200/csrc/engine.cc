@@ -73,6 +73,45 @@ PhaseBoundaries ScanPhases(const std::vector<Instruction>& train) {
   return p;
 }
 
+namespace {
+
+// Whether the bytes that leave are exactly the deltas the merge program accumulates, each one's last write being its
+// accumulation: the emit table lists the same ranges, none over another, and nothing but a delta's own zero fill, directly
+// before its accumulation, and that accumulation writes into any of them.
+bool EmitsAreMergeDeltas(const std::vector<Instruction>& merge, const std::vector<EmitEntry>& emit, const PlanHeader& h) {
+  using Range = std::pair<uint64_t, uint64_t>;   // offset, bytes
+  auto delta_of = [](const Instruction& ins) { return Range{RefOffset(ins.in[2]), ins.out[0] * ins.out[1] * 4}; };
+  std::vector<Range> made, leave;
+  for (const Instruction& ins : merge)
+    if (ins.opcode == kGemmAccNN) made.push_back(delta_of(ins));
+  for (const EmitEntry& e : emit) leave.push_back({e.arena_offset, e.byte_size});
+  std::sort(made.begin(), made.end());
+  std::sort(leave.begin(), leave.end());
+  if (made.empty() || made != leave) return false;
+  for (size_t i = 1; i < leave.size(); ++i)
+    if (leave[i].first < leave[i - 1].first + leave[i - 1].second) return false;
+  for (size_t i = 0; i < merge.size(); ++i) {
+    Extents ext;
+    if (!DescribeInstruction(merge[i], h.arena_size, h.rodata_size, uint64_t{1} << 48, &ext).empty()) return false;
+    for (size_t x = 0; x < ext.count; ++x) {
+      const Extent& e = ext.e[x];
+      if (!e.write) continue;
+      const Range w{e.off, e.bytes};
+      const auto first_after = std::upper_bound(leave.begin(), leave.end(), Range{e.off, ~0ull});
+      const bool hits = (first_after != leave.end() && first_after->first < e.off + e.bytes) ||
+                        (first_after != leave.begin() && std::prev(first_after)->first + std::prev(first_after)->second > e.off);
+      if (!hits) continue;
+      const bool own = merge[i].opcode == kGemmAccNN && w == delta_of(merge[i]);
+      const bool fill = merge[i].opcode == kFill && i + 1 < merge.size() && merge[i + 1].opcode == kGemmAccNN &&
+                        w == delta_of(merge[i + 1]);
+      if (!own && !fill) return false;
+    }
+  }
+  return true;
+}
+
+}  // namespace
+
 // ---- lifecycle ---------------------------------------------------------------------
 
 std::expected<std::unique_ptr<UpdateEngine>, std::string> UpdateEngine::Create(int device) {
@@ -215,16 +254,8 @@ Status UpdateEngine::LoadFromMemory(const uint8_t* plan, uint64_t size) {
   step_prog_ = std::move(step);
   emit_.resize(h.emit_count);
   if (h.emit_count) std::memcpy(emit_.data(), plan + h.emit_table_offset, h.emit_count * sizeof(EmitEntry));
-  {   // the deltas the merge program accumulates, against the emit table
-    std::vector<std::pair<uint64_t, uint64_t>> made, leave;
-    for (const Instruction& ins : merge_)
-      if (ins.opcode == kGemmAccNN) made.push_back({RefOffset(ins.in[2]), ins.out[0] * ins.out[1] * 4});
-    for (const EmitEntry& e : emit_) leave.push_back({e.arena_offset, e.byte_size});
-    std::sort(made.begin(), made.end());
-    std::sort(leave.begin(), leave.end());
-    emits_are_merge_deltas_ = !made.empty() && made == leave;
-    merge_counts_ = false;
-  }
+  emits_are_merge_deltas_ = EmitsAreMergeDeltas(merge_, emit_, h);
+  merge_counts_ = false;
   phases_ = ScanPhases(train_);
   grad_off_ = g_lo == ~0ull ? 0 : g_lo;
   grad_bytes_ = g_lo == ~0ull ? 0 : g_hi - g_lo;

@@ -47,3 +47,28 @@ def test_deltas_are_the_instructions_bits_and_counted(dims, rank):
     eng.write_arena(0, state)
     assert eng.run_merge() is True
     eng.close()
+
+
+@pytest.mark.parametrize("graphs", [False, True], ids=["eager", "graphs"])
+def test_a_later_write_over_a_delta_is_in_the_finiteness_scan(graphs):
+    """An instruction behind the accumulation doubles one delta: finite as accumulated, infinite as it leaves."""
+    plan = P.Plan(synth.build_mlp_plan(synth.MlpConfig(dims=(64, 260, 36), batch=4, rank=4)))
+    acc = next(i for i in plan.merge if i.opcode == P.Op.GEMM_ACC_NN)
+    delta, n = acc.ins[2], acc.out[0] * acc.out[1]
+    merge = list(plan.merge) + [P.Instr(P.Op.ADD_EW, 0, 0, (delta, delta, delta, P.NULL_REF), (n, 0, 0))]
+    persist = plan.persist_init
+    blob = P.write_plan(plan.header, plan.train, plan.eval, merge, plan.step, plan.rodata, persist, emit=plan.emit)
+    eng = Engine(0)
+    eng.load(blob)
+    eng.set_use_graphs(graphs)
+    state = np.zeros(plan.header["persistent_size"] // 4, np.float32)
+    M, N, K = acc.out
+    state[acc.ins[0] // 4:acc.ins[0] // 4 + M * K] = 1.0
+    b = state[acc.ins[1] // 4:acc.ins[1] // 4 + K * N]
+    for value, finite in ((1.0, True), (6e37, False), (1.0, True)):   # K = 4 terms: 2.4e38 times alpha, then twice that
+        b[:] = value / np.frombuffer(np.uint32(acc.ins[3] & 0xFFFFFFFF).tobytes(), np.float32)[0]
+        eng.write_arena(0, state)
+        for _ in range(3):
+            assert eng.run_merge() is finite
+            assert np.isfinite(eng.read_arena(delta, 4 * n).view(np.float32)).all() == finite
+    eng.close()
