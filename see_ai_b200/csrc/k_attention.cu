@@ -541,6 +541,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const size_t base = b * S * D + h * d;
   const int ty = InGroup() >> 4;
+  const bool pairs = (S & 1) == 0 && (reinterpret_cast<uintptr_t>(dp) & 7) == 0;   // (j is even: 8-byte stores)
   SliceRegs regs;
   int turn = 0;
   const int first = GroupOf() * kTile;
@@ -564,7 +565,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __
         const int j = k0 + Col(e);
         const float x0 = j <= i ? static_cast<float>(acc[r][e]) : 0.0f;
         const float x1 = j + 1 <= i ? static_cast<float>(acc[r][e + 1]) : 0.0f;
-        if ((S & 1) == 0 && j + 1 < S) {
+        if (pairs && j + 1 < S) {
           *reinterpret_cast<float2*>(row + j) = make_float2(x0, x1);
         } else {
           if (j < S) row[j] = x0;

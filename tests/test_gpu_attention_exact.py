@@ -31,7 +31,7 @@ def setup_module(_m):
         oracle.build("oracle")
 
 
-def _program(Bq, S, H, d, segments, cached):
+def _program(Bq, S, H, d, segments, cached, shift=0):
     rng = np.random.default_rng(S * 1000 + d + segments)
     td, ss = Bq * S * H * d, Bq * H * S * S
     refs, size = {}, 0
@@ -40,8 +40,8 @@ def _program(Bq, S, H, d, segments, cached):
     if cached:
         sizes.update(P=ss, dP=ss, dS=ss)
     for name, n in sizes.items():
-        refs[name] = size
-        size = (size + 4 * n + 63) // 64 * 64
+        refs[name] = size + shift
+        size = (size + shift + 4 * n + 63) // 64 * 64
     arena = np.zeros(size, dtype=np.uint8)
     for name in ("q", "k", "v", "do"):
         arena[refs[name]:refs[name] + 4 * td] = rng.standard_normal(td, dtype=np.float32).view(np.uint8)
@@ -75,7 +75,16 @@ def _program(Bq, S, H, d, segments, cached):
 @pytest.mark.parametrize("segments", [0, 1], ids=["causal", "segments"])
 @pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
 def test_every_instruction_from_the_oracles_bytes(shape, segments):
-    prog, arena = _program(*shape, segments, cached=shape[1] < 2000)
+    _compare(*_program(*shape, segments, cached=shape[1] < 2000))
+
+
+@pytest.mark.parametrize("shift", [4, 8, 12])
+@pytest.mark.parametrize("shape", [(1, 64, 2, 32), (2, 130, 1, 64), (1, 65, 1, 8)], ids=lambda s: "x".join(map(str, s)))
+def test_tensors_that_are_no_more_than_float_aligned(shape, shift):
+    _compare(*_program(*shape, 0, cached=True, shift=shift))
+
+
+def _compare(prog, arena):
     cpu, gpu = arena.copy(), arena.copy()
     ref = oracle.OracleExecutor()
     ref.bind(cpu, None)
