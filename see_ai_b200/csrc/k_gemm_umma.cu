@@ -198,7 +198,7 @@ __device__ __forceinline__ BlockAt BlockCoord(const UmmaEpilogue& ep, uint32_t k
     return {x, x, true};
   }
   if (ep.seg_blocks == 0) return {static_cast<int32_t>(kb * kBlockK), static_cast<int32_t>(kb * kBlockK), false};
-  const uint32_t seg = kb / ep.seg_blocks, w = kb - seg * ep.seg_blocks;
+  const uint32_t w = kb / ep.segs, seg = kb - w * ep.segs;
   return {static_cast<int32_t>((((ep.seg_a >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK),
           static_cast<int32_t>((((ep.seg_b >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK), false};
 }
@@ -235,7 +235,8 @@ struct TTile {
 struct __align__(8) TBarriers {
   uint64_t full[kTMaxStages];
   uint64_t empty[kTMaxStages];
-  uint64_t tmem_full;
+  uint64_t tmem_full[2];
+  uint64_t tmem_empty[2];   // piece products only
   uint32_t tmem_base;
   volatile uint32_t abort;  // set by a role whose wait ran out; the epilogue then stores nothing
 };
@@ -247,7 +248,7 @@ __device__ __forceinline__ float4 LoadClusterF4(uint32_t cluster_addr) {
   return v;
 }
 
-template <uint32_t kTN>
+template <uint32_t kTN, bool kSeg>
 __global__ void __launch_bounds__(kTThreads, 1)
 UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
@@ -269,19 +270,27 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   // accumulated into the same tile; see UmmaEpilogue::aux_k_blocks).
   const uint32_t main_blocks = (ep.K + kBlockK - 1) / kBlockK;
   const uint32_t k_blocks = main_blocks + ep.aux_k_blocks;
-  const uint32_t kb0 = k_blocks * split / splits, kb1 = k_blocks * (split + 1) / splits;
+  // Accumulators of the reduction, `group` blocks each: a plain product has one, piece products one per block of K.
+  const uint32_t all = kSeg ? ep.seg_blocks : k_blocks;
+  const uint32_t part0 = all * split / splits, part1 = all * (split + 1) / splits;
+  const uint32_t kb0 = kSeg ? part0 * ep.segs : part0, kb1 = kSeg ? part1 * ep.segs : part1;
+  const uint32_t group = kSeg ? ep.segs : kb1 - kb0, groups = kSeg ? part1 - part0 : 1u;
+  constexpr uint32_t kTmemCols = kSeg ? 2 * T::kTmemCols : T::kTmemCols;
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < kStages; ++s) {
       MbarInit(&bars->full[s], 1);
       MbarInit(&bars->empty[s], 1);
     }
-    MbarInit(&bars->tmem_full, 1);
+    for (uint32_t b = 0; b < 2; ++b) {
+      MbarInit(&bars->tmem_full[b], 1);
+      MbarInit(&bars->tmem_empty[b], kTEpiThreads / 32);
+    }
     bars->abort = 0;
     MbarInitFence();
   }
   if (warp == 1) {
-    TmemAlloc(&bars->tmem_base, T::kTmemCols);
+    TmemAlloc(&bars->tmem_base, kTmemCols);
   }
   TcFenceBefore();
   __syncthreads();
@@ -311,24 +320,35 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // ---- MMA issuer ----
     if (ElectOne()) {
       const uint32_t idesc = MakeInstrDesc(kBlockM, kTN);
-      for (uint32_t kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-        const uint32_t s = it % kStages, round = it / kStages;
-        if (!MbarWait(&bars->full[s], round & 1)) {
+      bool going = true;
+      for (uint32_t g = 0, it = 0; g < groups && going; ++g) {
+        const uint32_t buf = kSeg ? g & 1 : 0, use = g >> 1;
+        if (kSeg && use > 0 && !MbarWait(&bars->tmem_empty[buf], (use - 1) & 1)) {
           ep.status->wait_timeout = 1;
           bars->abort = 1;
           break;
         }
-        TcFenceAfter();
-        const uint32_t a_addr = SmemAddr(smem + s * kStageBytes);
-        const uint64_t desc_a = MakeSmemDesc(a_addr), desc_b = MakeSmemDesc(a_addr + kATileBytes);
+        const uint32_t acc = tmem_base + buf * T::kTmemCols;
+        for (uint32_t b = 0; b < group; ++b, ++it) {
+          const uint32_t s = it % kStages, round = it / kStages;
+          if (!MbarWait(&bars->full[s], round & 1)) {
+            ep.status->wait_timeout = 1;
+            bars->abort = 1;
+            going = false;
+            break;
+          }
+          TcFenceAfter();
+          const uint32_t a_addr = SmemAddr(smem + s * kStageBytes);
+          const uint64_t desc_a = MakeSmemDesc(a_addr), desc_b = MakeSmemDesc(a_addr + kATileBytes);
 #pragma unroll
-        for (uint32_t k = 0; k < kBlockK / kUmmaK; ++k) {
-          // advance 16 bf16 = 32 bytes inside the 128-byte swizzle row: +2 in >>4 units
-          UmmaBf16(tmem_base, desc_a + 2 * k, desc_b + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
+          for (uint32_t k = 0; k < kBlockK / kUmmaK; ++k) {
+            // advance 16 bf16 = 32 bytes inside the 128-byte swizzle row: +2 in >>4 units
+            UmmaBf16(acc, desc_a + 2 * k, desc_b + 2 * k, idesc, (b | k) != 0 ? 1u : 0u);
+          }
+          UmmaCommit(&bars->empty[s]);      // the slot is free once these MMAs have read it
         }
-        UmmaCommit(&bars->empty[s]);   // the slot is free once these MMAs have read it
+        UmmaCommit(&bars->tmem_full[buf]);  // accumulator complete (or abandoned on timeout)
       }
-      UmmaCommit(&bars->tmem_full);    // accumulator complete (or abandoned on timeout)
     }
   }
   __syncwarp();
@@ -348,25 +368,59 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           asm volatile("prefetch.global.L2 [%0];" ::"l"(side_ptr + static_cast<size_t>(row) * ep.N + n));
       }
     const uint32_t quarter = warp & 3, columns = ((warp - 2) >> 2) * (kTN / 2);
-    ok = MbarWait(&bars->tmem_full, 0);
-    if (!ok && lane == 0) ep.status->wait_timeout = 1;
-    if (bars->abort) ok = false;
-    ok = __all_sync(0xFFFFFFFFu, ok);
-    TcFenceAfter();
+    const uint32_t t_row = tmem_base + ((quarter * 32) << 16) + columns;
+    auto await = [&](uint32_t buf, uint32_t parity) {
+      bool there = MbarWait(&bars->tmem_full[buf], parity);
+      if (!there && lane == 0) ep.status->wait_timeout = 1;
+      if (bars->abort) there = false;
+      there = __all_sync(0xFFFFFFFFu, there);
+      TcFenceAfter();
+      return there;
+    };
+    // Piece products: the blocks' accumulators, added with f32's rounding while the next block's products run.
+    [[maybe_unused]] float sum[kSeg ? kTN / 2 : 1];
+    if constexpr (kSeg) {
+#pragma unroll
+      for (uint32_t j = 0; j < kTN / 2; ++j) sum[j] = 0.0f;
+      for (uint32_t g = 0; g < groups && ok; ++g) {
+        const uint32_t buf = g & 1;
+        if (!(ok = await(buf, (g >> 1) & 1))) break;
+#pragma unroll
+        for (uint32_t c0 = 0; c0 < kTN / 2; c0 += 16) {
+          uint32_t r[16];
+          TmemLoad16(t_row + buf * T::kTmemCols + c0, r);
+          TmemWaitLd();
+#pragma unroll
+          for (uint32_t j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(r[j]);
+        }
+        TcFenceBefore();
+        __syncwarp();
+        if (lane == 0) MbarArrive(&bars->tmem_empty[buf]);
+      }
+    } else {
+      ok = await(0, 0);
+    }
     if (ok) {
       // The accumulator arrives one row per thread; HBM wants whole rows.  All MMAs are complete, so
       // the ring is free: the tile goes there as [128][kTN] f32, 16-byte chunks XOR-ed with the
       // row so that neither side conflicts.
       float* dump = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kTN;
-#pragma unroll 1
-      for (uint32_t c0 = 0; c0 < kTN / 2; c0 += 32) {
-        uint32_t r[32];
-        TmemLoad32(tmem_base + ((quarter * 32) << 16) + columns + c0, r);
-        TmemWaitLd();
+      if constexpr (kSeg) {
 #pragma unroll
-        for (uint32_t q = 0; q < 8; ++q)
-          *reinterpret_cast<uint4*>(dump + ((((columns + c0) >> 2) + q) ^ (lane & 7u)) * 4) =
-              make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+        for (uint32_t q = 0; q < kTN / 8; ++q)
+          *reinterpret_cast<float4*>(dump + (((columns >> 2) + q) ^ (lane & 7u)) * 4) =
+              make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
+      } else {
+#pragma unroll 1
+        for (uint32_t c0 = 0; c0 < kTN / 2; c0 += 32) {
+          uint32_t r[32];
+          TmemLoad32(t_row + c0, r);
+          TmemWaitLd();
+#pragma unroll
+          for (uint32_t q = 0; q < 8; ++q)
+            *reinterpret_cast<uint4*>(dump + ((((columns + c0) >> 2) + q) ^ (lane & 7u)) * 4) =
+                make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+        }
       }
     }
     TcFenceBefore();
@@ -457,7 +511,7 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   if (splits > 1) ClusterSync();   // no CTA leaves while another may still read its memories
   if (warp == 1) {
     TcFenceAfter();
-    TmemFree(tmem_base, T::kTmemCols);
+    TmemFree(tmem_base, kTmemCols);
   }
 }
 
@@ -535,13 +589,16 @@ struct __align__(8) PBarriers {
 // while this group is converted and stored, across passes and from before the
 // wait for the accumulator, so a memory round trip is not paid per group with
 // every warp of the CTA waiting on it.
-template <bool kSideLoads, bool kPair>
+// kSeg: piece products (UmmaEpilogue::seg_blocks).  An accumulator buffer then holds one block of K, and the epilogue
+// warps add the blocks in registers, 64 outputs a thread, one block behind the products.
+template <bool kSideLoads, bool kPair, bool kSeg>
 __global__ void __launch_bounds__(kPThreads, 1)
 UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
                          const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_a2,
                          const __grid_constant__ CUtensorMap map_b2, UmmaEpilogue ep,
                          uint32_t band_blocks) {
+  static_assert(!(kSideLoads && kSeg), "the sums take the registers of the loads in flight");
   using T = PTile<kPair>;
   constexpr uint32_t kTN = kPBlockN;
   constexpr uint32_t kPStages = T::kStages, kPStageBytes = T::kStageBytes, kPTmemCols = T::kTmemCols;
@@ -557,6 +614,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
   const uint32_t tiles_n = (ep.N + kTN - 1) / kTN;
   const uint32_t tiles_m = (ep.M + T::kRowsPerTile - 1) / T::kRowsPerTile;
   const uint32_t total_tiles = tiles_m * tiles_n;
+  const uint32_t group = kSeg ? ep.segs : k_blocks, groups = kSeg ? ep.seg_blocks : 1u;   // blocks per accumulator
   // A work unit is a CTA, or a CTA pair: `unit` walks the tiles, `cta_rank` is this CTA's half of a pair's tile.
   const uint32_t cta_rank = kPair ? ClusterCtaRank() : 0u;
   const uint32_t unit = kPair ? blockIdx.x >> 1 : blockIdx.x, units = kPair ? gridDim.x >> 1 : gridDim.x;
@@ -645,9 +703,9 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
     // ---- MMA issuer ----
     if (ElectOne() && cta_rank == 0) {   // (a pair's odd CTA issues nothing: its memories are read by the even one's MMAs)
       const uint32_t idesc = MakeInstrDesc(T::kRowsPerTile, kTN);
-      uint32_t it = 0, lt = 0;
+      uint32_t it = 0, lt = 0;   // lt: accumulators so far
       bool ok = true;
-      for (uint32_t t = unit; t < total_tiles && ok; t += units, ++lt) {
+      for (uint32_t t = unit, g = 0; t < total_tiles && ok; ++lt, g = g + 1 < groups ? g + 1 : (t += units, 0u)) {
         const uint32_t buf = lt & 1, use = lt >> 1;
         if (use > 0 && !MbarWait(&bars->tmem_empty[buf], (use - 1) & 1)) {
           ep.status->wait_timeout = 1;
@@ -656,7 +714,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + buf * kTN;
-        for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
+        for (uint32_t kb = 0; kb < group; ++kb, ++it) {
           const uint32_t s = it % kPStages, round = it / kPStages;
           if (!MbarWait(&bars->full[s], round & 1)) {
             ep.status->wait_timeout = 1;
@@ -689,9 +747,9 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
     constexpr uint32_t kChunks = kSlabCols / 4;          // 16-byte chunks per slab row
     constexpr uint32_t kRowsPerInstr = 32 / kChunks;     // rows one store instruction covers
     const uint32_t sub = lane / kChunks, cl = lane % kChunks;
-    uint32_t lt = 0;
+    uint32_t lt = 0;   // accumulators so far
     for (uint32_t t = unit; t < total_tiles; t += units, ++lt) {
-      const uint32_t buf = lt & 1, use = lt >> 1;
+      uint32_t buf = lt & 1, use = lt >> 1;
       uint32_t mb, nb;
       TileCoord(t, tiles_m, tiles_n, band_blocks, &mb, &nb);
       const uint32_t m0 = mb * T::kRowsPerTile + cta_rank * kBlockM, n0 = nb * kTN;
@@ -734,35 +792,54 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
                           : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
-      bool ok = MbarWait(&bars->tmem_full[buf], use & 1);
-      if (!ok && lane == 0) { ep.status->wait_timeout = 1; bars->abort = 1; }
-      if (bars->abort) ok = false;
-      ok = __all_sync(0xFFFFFFFFu, ok);
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      auto await = [&] {
+        bool there = MbarWait(&bars->tmem_full[buf], use & 1);
+        if (!there && lane == 0) { ep.status->wait_timeout = 1; bars->abort = 1; }
+        if (bars->abort) there = false;
+        there = __all_sync(0xFFFFFFFFu, there);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        return there;
+      };
+      auto hand_back = [&] {   // the accumulator buffer is read out
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (kPair) MbarArriveCluster(MapToCta(SmemAddr(&bars->tmem_empty[buf]), 0));
+          else MbarArrive(&bars->tmem_empty[buf]);
+        }
+      };
+      [[maybe_unused]] float sum[kSeg ? kEpiPasses : 1][kSeg ? kSlabCols : 1];
+      if constexpr (kSeg) {
+#pragma unroll
+        for (uint32_t p = 0; p < kEpiPasses; ++p)
+#pragma unroll
+          for (uint32_t j = 0; j < kSlabCols; ++j) sum[p][j] = 0.0f;
+        bool ok = true;
+        for (uint32_t g = 0; g < groups; ++g) {
+          if (g > 0) { ++lt; buf = lt & 1; use = lt >> 1; }
+          if (!(ok = await())) break;
+          const uint32_t t_row = tmem_base + ((quarter * 32) << 16) + buf * kTN + col_group * kColsPerEpiWarp;
+#pragma unroll
+          for (uint32_t c = 0; c < kColsPerEpiWarp; c += 16) {   // (all 64 at once do not fit the registers)
+            uint32_t ra[16];
+            TmemLoad16(t_row + c, ra);
+            TmemWaitLd();
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) sum[c / kSlabCols][c % kSlabCols + j] += __uint_as_float(ra[j]);
+          }
+          hand_back();
+        }
+        if (!ok) break;
+      } else {
+        if (!await()) break;
+      }
       // 32 columns at a time through the slab.  A thread writes its accumulator
       // row as eight 16-byte chunks, chunk index XOR-ed with the row; the warp
       // then reads four rows per instruction (eight lanes each): whole 128-byte
       // lines of C per store instruction.  Conflict-free both ways.
       const uint32_t t_row = tmem_base + ((quarter * 32) << 16) + buf * kTN + col_group * kColsPerEpiWarp;
       if constexpr (!kSideLoads) {
-  #pragma unroll 1
-        for (uint32_t pass = 0; pass < kEpiPasses; ++pass) {
-          uint32_t ra[32];
-          TmemLoad32(t_row + pass * kSlabCols, ra);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (pass == kEpiPasses - 1) {
-            // The accumulator buffer is read out: hand it back before the slow part.
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-              if constexpr (kPair)
-                MbarArriveCluster(MapToCta(SmemAddr(&bars->tmem_empty[buf]), 0));
-              else
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];"
-                             ::"r"(SmemAddr(&bars->tmem_empty[buf])) : "memory");
-            }
-          }
+        auto store_pass = [&](uint32_t pass, const uint32_t (&ra)[32]) {
   #pragma unroll
           for (uint32_t q = 0; q < kChunks; ++q)
             *reinterpret_cast<uint4*>(slab + lane * kSlabCols + ((q ^ (lane & (kChunks - 1))) * 4)) =
@@ -797,6 +874,24 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
             }
           }
           __syncwarp();   // the slab is rewritten next
+        };
+        if constexpr (kSeg) {
+#pragma unroll
+          for (uint32_t pass = 0; pass < kEpiPasses; ++pass) {
+            uint32_t ra[32];
+#pragma unroll
+            for (uint32_t j = 0; j < kSlabCols; ++j) ra[j] = __float_as_uint(sum[pass][j]);
+            store_pass(pass, ra);
+          }
+        } else {
+  #pragma unroll 1
+          for (uint32_t pass = 0; pass < kEpiPasses; ++pass) {
+            uint32_t ra[32];
+            TmemLoad32(t_row + pass * kSlabCols, ra);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (pass == kEpiPasses - 1) hand_back();   // before the slow part
+            store_pass(pass, ra);
+          }
         }
       } else {
         // Groups of four row steps (two per pass); group g + 1's side operands are
@@ -816,17 +911,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
           uint32_t ra[32];
           TmemLoad32(t_row + pass * kSlabCols, ra);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (pass == kEpiPasses - 1) {
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-              if constexpr (kPair)
-                MbarArriveCluster(MapToCta(SmemAddr(&bars->tmem_empty[buf]), 0));
-              else
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];"
-                             ::"r"(SmemAddr(&bars->tmem_empty[buf])) : "memory");
-            }
-          }
+          if (pass == kEpiPasses - 1) hand_back();
 #pragma unroll
           for (uint32_t q = 0; q < kChunks; ++q)
             *reinterpret_cast<uint4*>(slab + lane * kSlabCols + ((q ^ (lane & (kChunks - 1))) * 4)) =
@@ -969,13 +1054,13 @@ static cudaError_t LaunchClustered(void (*kernel)(KArgs...), dim3 grid, dim3 blo
 }
 
 // Calls f(kernel, shared-memory bytes) with the tile kernel of this width.
-template <typename F>
+template <bool kSeg, typename F>
 static cudaError_t WithTileKernel(uint32_t tn, F f) {
   switch (tn) {
-    case 64: return f(UmmaGemmTileKernel<64>, UmmaTileSmemBytes<64>());
-    case 128: return f(UmmaGemmTileKernel<128>, UmmaTileSmemBytes<128>());
-    case 192: return f(UmmaGemmTileKernel<192>, UmmaTileSmemBytes<192>());
-    default: return f(UmmaGemmTileKernel<256>, UmmaTileSmemBytes<256>());
+    case 64: return f(UmmaGemmTileKernel<64, kSeg>, UmmaTileSmemBytes<64>());
+    case 128: return f(UmmaGemmTileKernel<128, kSeg>, UmmaTileSmemBytes<128>());
+    case 192: return f(UmmaGemmTileKernel<192, kSeg>, UmmaTileSmemBytes<192>());
+    default: return f(UmmaGemmTileKernel<256, kSeg>, UmmaTileSmemBytes<256>());
   }
 }
 
@@ -988,14 +1073,17 @@ static cudaError_t Configure() {
   };
   cudaError_t e = cudaSuccess;
   for (uint32_t tn : {64u, 128u, 192u, 256u})
-    if ((e = WithTileKernel(tn, allow)) != cudaSuccess) return e;
-  if ((e = allow(UmmaGemmPersistentKernel<false, false>, UmmaPersistentSmemBytes<false>())) != cudaSuccess) return e;
-  if ((e = allow(UmmaGemmPersistentKernel<true, false>, UmmaPersistentSmemBytes<false>())) != cudaSuccess) return e;
-  if ((e = allow(UmmaGemmPersistentKernel<false, true>, UmmaPersistentSmemBytes<true>())) != cudaSuccess) return e;
-  return allow(UmmaGemmPersistentKernel<true, true>, UmmaPersistentSmemBytes<true>());
+    if ((e = WithTileKernel<false>(tn, allow)) != cudaSuccess || (e = WithTileKernel<true>(tn, allow)) != cudaSuccess) return e;
+  const size_t one = UmmaPersistentSmemBytes<false>(), pair = UmmaPersistentSmemBytes<true>();
+  if ((e = allow(UmmaGemmPersistentKernel<false, false, false>, one)) != cudaSuccess) return e;
+  if ((e = allow(UmmaGemmPersistentKernel<true, false, false>, one)) != cudaSuccess) return e;
+  if ((e = allow(UmmaGemmPersistentKernel<false, false, true>, one)) != cudaSuccess) return e;
+  if ((e = allow(UmmaGemmPersistentKernel<false, true, false>, pair)) != cudaSuccess) return e;
+  if ((e = allow(UmmaGemmPersistentKernel<true, true, false>, pair)) != cudaSuccess) return e;
+  return allow(UmmaGemmPersistentKernel<false, true, true>, pair);
 }
 
-UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, bool light, uint32_t sms) {
+UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms) {
   UmmaGemmPlan p;
   const uint32_t ptiles_n = (N + kPBlockN - 1) / kPBlockN, tiles_m = (M + kBlockM - 1) / kBlockM;
   const uint64_t wide = static_cast<uint64_t>(ptiles_n) * tiles_m;
@@ -1006,7 +1094,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, bool light,
   // kernel's likewise.
   double best = 1e30;
   for (uint32_t tn : {64u, 128u, 192u, 256u})
-    for (uint32_t splits = 1; splits <= 4 && splits <= k_blocks; splits *= 2) {
+    for (uint32_t splits = 1; splits <= 4 && splits * group <= k_blocks; splits *= 2) {
       const uint64_t ctas = static_cast<uint64_t>(tiles_m) * ((N + tn - 1) / tn) * splits;
       const uint64_t room = splits <= 2 ? sms : sms * 9 / 10;   // clusters of four do not fill every GPC
       const double waves = static_cast<double>((ctas + room - 1) / room);
@@ -1065,22 +1153,28 @@ cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const CUtensorMap& map_a, c
     if (cudaError_t e = Configure(); e != cudaSuccess) return e;
     if (tracked) configured_on[dev].store(true, std::memory_order_release);
   }
-  if (!plan.persistent)
-    return WithTileKernel(plan.tn, [&](auto kernel, size_t bytes) {
+  const bool seg = ep.seg_blocks != 0;
+  if (!plan.persistent) {
+    auto launch = [&](auto kernel, size_t bytes) {
       return LaunchClustered(kernel, dim3(plan.grid), dim3(kTThreads), bytes, s, plan.splits, map_a, map_b, map_a2,
                              map_b2, ep, plan.splits);
-    });
+    };
+    return seg ? WithTileKernel<true>(plan.tn, launch) : WithTileKernel<false>(plan.tn, launch);
+  }
   // An addend or the x of an absorbed backward activation is software-pipelined (16 bytes at a time).
-  const bool side_loads = (ep.addend != nullptr || ep.fuse_mode == kFuseActBwd) && (ep.N & 3) == 0;
+  const bool side_loads = !seg && (ep.addend != nullptr || ep.fuse_mode == kFuseActBwd) && (ep.N & 3) == 0;
   auto launch = [&](auto kernel, size_t bytes) {
     return LaunchClustered(kernel, dim3(plan.grid), dim3(kPThreads), bytes, s, plan.pair ? 2u : 1u, map_a, map_b, map_a2,
                            map_b2, ep, plan.band);
   };
+  const size_t bytes = plan.pair ? UmmaPersistentSmemBytes<true>() : UmmaPersistentSmemBytes<false>();
   if (plan.pair)
-    return side_loads ? launch(UmmaGemmPersistentKernel<true, true>, UmmaPersistentSmemBytes<true>())
-                      : launch(UmmaGemmPersistentKernel<false, true>, UmmaPersistentSmemBytes<true>());
-  return side_loads ? launch(UmmaGemmPersistentKernel<true, false>, UmmaPersistentSmemBytes<false>())
-                    : launch(UmmaGemmPersistentKernel<false, false>, UmmaPersistentSmemBytes<false>());
+    return seg          ? launch(UmmaGemmPersistentKernel<false, true, true>, bytes)
+           : side_loads ? launch(UmmaGemmPersistentKernel<true, true, false>, bytes)
+                        : launch(UmmaGemmPersistentKernel<false, true, false>, bytes);
+  return seg          ? launch(UmmaGemmPersistentKernel<false, false, true>, bytes)
+         : side_loads ? launch(UmmaGemmPersistentKernel<true, false, false>, bytes)
+                      : launch(UmmaGemmPersistentKernel<false, false, false>, bytes);
 }
 
 void WeightToBf16(const void* src, BType type, uint16_t* dst, uint32_t N, uint32_t K,

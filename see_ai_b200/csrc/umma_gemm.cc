@@ -347,7 +347,7 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   CUtensorMap map_a, map_b, aux_a, aux_b;
   const bool has_aux = a.aux_a && a.aux_b && a.aux_k >= 64 && a.aux_k % 64 == 0;
   const uint32_t k_blocks = static_cast<uint32_t>((a.K + 63) / 64) + (has_aux ? a.aux_k / 64 : 0);
-  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks,
+  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks, 1,
                                                 LightEpilogue(a), impl->sms);
   if (!EncodeBf16Map(impl, &map_a, slot->buf, a.M, a.K, k::umma_cfg::kBlockM) ||
       !EncodeBf16Map(impl, &map_b, w, a.N, a.K, plan.b_box))
@@ -392,7 +392,7 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
 
 namespace {
 
-// The reduction as segments of bf16 pieces, small products first because the tensor core truncates toward zero at
+// The piece products of one block of the reduction, small ones first because the tensor core truncates toward zero at
 // the accumulator's magnitude.  f32 times f32: a2 b0, a1 b1, a0 b2, a1 b0, a0 b1, a0 b0.  f32 times a weight that
 // is a bf16 value exactly (int8 levels, bf16): a2 b, a1 b, a0 b.
 constexpr uint32_t kSegF32 = 6, kSegAF32 = 0x001012, kSegBF32 = 0x010210;
@@ -507,7 +507,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   }
   const uint32_t segments = exact_b ? kSegExact : kSegF32;
   const uint32_t k_blocks = static_cast<uint32_t>(segments * (Kp / 64));
-  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks,
+  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks, segments,
                                                 LightEpilogue(a), impl->sms);
   CUtensorMap map_a, map_b;
   // An exact weight is [N][K]: past K its last block reads zeros, and so do A's padding columns.
@@ -525,6 +525,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   ep.N = static_cast<uint32_t>(a.N);
   ep.K = k_blocks * 64;
   ep.seg_blocks = static_cast<uint32_t>(Kp / 64);
+  ep.segs = segments;
   ep.seg_a = exact_b ? kSegAExact : kSegAF32;
   ep.seg_b = exact_b ? kSegBExact : kSegBF32;
   ep.status = impl->status;

@@ -50,11 +50,19 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& args, int b_space, uint64_t
 std::string TryLoraBackward(Context* ctx, const k::LoraBackwardArgs& args, cudaStream_t stream, int* launches);
 
 // An EXACT product on the tensor cores: f32 operands cut into three bf16 pieces
-// (k::SplitMatrix), the six largest piece products summed in tensor memory in f32;
-// an int8 or bf16 weight is one piece as it is, three products.  The result is the
-// f32 product to a few 2^-24 of sum|a_k b_k| — the accuracy the exact CUDA-core
-// kernels have against a float64 sum, not their bits — at a sixth (a third) of the
-// bf16 tensor rate instead of the FP32 pipe's.  Epilogue scale / addend / bias /
+// (k::SplitMatrix), the six largest piece products of 64 k at a time summed in
+// tensor memory in f32; an int8 or bf16 weight is one piece as it is, three products.
+// The tensor core truncates each of a block's four steps at the accumulator's
+// magnitude; the blocks are added in f32 registers, rounded.  The result is the f32
+// product to about (1.5 + 0.3 sqrt(K / 64)) 2^-24 of its root mean square for terms of
+// either sign, and stays below 2e-6 of sum|a_k b_k| for same-signed ones: no further
+// from a float64 sum than the CUDA-core kernels in the reference's order, though not
+// their bits (normal operands, relative rms, those kernels / this: K = 768 2.6e-7 /
+// 1.0e-7, 3072 5.0e-7 / 1.5e-7, 32000 1.6e-6 / 2.2e-7; with one accumulator over all
+// of K it was 7.3e-7, 3.2e-6, 3.7e-5).  At a sixth (a third) of the bf16 tensor rate
+// instead of the FP32 pipe's; the sums cost, with int8 weights and 4096 rows, 34.1 ->
+// 34.4 us (768 x 768), 61 -> 78 (3072 x 768) and 442 -> 592 (32000 x 768), where a
+// tile's stores no longer hide behind a whole tile of products.  Epilogue scale / addend / bias /
 // activation as usual.  `wide` takes every shape and weight type worth a launch;
 // without it the domain is NN, NT and TN products of f32 operands of at least 2^26
 // multiply-adds with N and K multiples of 4.  The threshold of the wide domain,

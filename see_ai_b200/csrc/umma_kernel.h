@@ -49,10 +49,10 @@ struct UmmaEpilogue {
   // The stored value also as bf16 [M, N] (GemmArgs::pack_dst).
   uint16_t* pack_dst = nullptr;
   // An f32-accurate product out of bf16 pieces: the operands hold pieces side by side along K, each
-  // seg_blocks * 64 wide (zero-padded), and the reduction's segment s multiplies A's piece number
-  // (seg_a >> 4s) & 15 by B's piece number (seg_b >> 4s) & 15.  K = 64 * seg_blocks * (number of segments).
-  // 0: a plain product.
-  uint32_t seg_blocks = 0, seg_a = 0, seg_b = 0;
+  // seg_blocks * 64 wide (zero-padded).  64 wide block by block, piece product s = 0 .. segs - 1 multiplies A's
+  // piece number (seg_a >> 4s) & 15 by B's piece number (seg_b >> 4s) & 15; a block's products meet in one
+  // accumulator, the blocks' accumulators in f32 registers.  K = 64 * seg_blocks * segs.  0: a plain product.
+  uint32_t seg_blocks = 0, segs = 0, seg_a = 0, seg_b = 0;
 };
 
 // Which kernel takes a product, on which tiles (k_gemm_umma.cu).
@@ -63,9 +63,9 @@ struct UmmaGemmPlan {
   uint32_t grid = 0, band = 1;
   uint32_t b_box = 0;       // rows of B one TMA load brings: the box height of map_b and aux_b
 };
-// k_blocks: 64-wide blocks of the whole reduction, a low-rank term's included.  light: the epilogue only stores
-// (f32 or a bf16 copy), without a second operand, bias or activation.
-UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, bool light, uint32_t sms);
+// k_blocks: 64-wide blocks of the whole reduction, a low-rank term's included; `group` of them in a row (1: any) are
+// not cut.  light: the epilogue only stores (f32 or a bf16 copy), without a second operand, bias or activation.
+UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms);
 // map_a: bf16 [M, K] row-major, box {64, 128}, 128-byte swizzle; map_b: bf16 [N, K], box {64, plan.b_box}.
 cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const CUtensorMap& map_a, const CUtensorMap& map_b,
                            const UmmaEpilogue& ep, cudaStream_t s, const CUtensorMap* aux_a = nullptr,

@@ -72,3 +72,62 @@ def test_products_of_every_weight_type_match_float64(shape):
     ]
     worst = [float((np.abs(mat(off, M, N) - want) / (1.0 + mag)).max()) for off, (want, mag) in zip(outs, wants)]
     assert max(worst) < 2e-6, worst
+
+
+def _product(kind, M, N, K, nonneg, coherence):
+    """(result, float64 result, sum|a_k b_k|, split executions) of one product."""
+    rng = np.random.default_rng(M + 3 * N + 7 * K)
+    draw = (lambda *s: np.abs(rng.standard_normal(s)).astype(np.float32)) if nonneg else \
+        (lambda *s: rng.standard_normal(s).astype(np.float32))
+    a = Arena(rng)
+    A = a.alloc(M * K)
+    X = draw(*((K, M) if kind == "tn" else (M, K)))
+    shape = (N, K) if kind.startswith("nt") else (K, N)
+    if kind.endswith("q8"):
+        W = rng.integers(0 if nonneg else -127, 128, size=shape, dtype=np.int8)
+        scale = (rng.random(K if kind == "ntq8" else N) * 0.02 + 1e-3).astype(np.float32)
+        flags, last, op = P.FLAG_Q8_COL_SCALE, a.ro_alloc(scale), Op.GEMM_NT_Q8 if kind == "ntq8" else Op.GEMM_NN_Q8
+    else:
+        W, flags, last, op = draw(*shape), 0, P.NULL_REF, dict(nn=Op.GEMM_NN, nt=Op.GEMM_NT, tn=Op.GEMM_TN)[kind]
+    C = a.alloc(M * N)
+    ins = P.Instr(op, flags, 0, (A, a.ro_alloc(W), C, last), (M, N, K))
+    arena, ro = a.build()
+    arena[A:A + X.nbytes] = X.reshape(-1).view(np.uint8)
+    be = B.CudaBackend(0)
+    be.set_coherence(coherence)
+    be.bind(arena, ro)
+    be.run([ins])
+    taken = be.counters().split_executions
+    be.host_needs(C, 4 * M * N)
+    be.close()
+    x, w = X.astype(np.float64), W.astype(np.float64)
+    x, w = (x.T if kind == "tn" else x), (w.T if kind.startswith("nt") else w)
+    if kind == "nnq8":
+        w = w * scale
+    if kind == "ntq8":
+        x = x * scale
+    return arena[C:C + 4 * M * N].view(np.float32).astype(np.float64).reshape(M, N), x @ w, np.abs(x) @ np.abs(w), taken
+
+
+@pytest.mark.parametrize("kind", ["nn", "nt", "tn", "nnq8", "ntq8"])
+@pytest.mark.parametrize("shape", [(384, 640, 256), (1000, 768, 768), (600, 768, 3072), (4096, 3072, 256), (300, 256, 8192)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_no_further_from_float64_than_the_cuda_core_sums(kind, shape):
+    """The tensor core truncates at its accumulator's magnitude; blocks of 64 meet in rounded f32 sums so that
+    the whole is as accurate as the kernels in the reference's order, whatever K (rms over the output, 5 % for
+    the spread of a sample)."""
+    got, want, _, taken = _product(kind, *shape, False, B.COHERENCE_LAZY)
+    ref, _, _, none = _product(kind, *shape, False, B.COHERENCE_STRICT)
+    assert (taken, none) == (1, 0)
+    err, bar = np.sqrt(np.mean((got - want) ** 2)), np.sqrt(np.mean((ref - want) ** 2))
+    assert err <= 1.05 * bar, err / bar
+
+
+@pytest.mark.parametrize("kind", ["nn", "nt", "tn", "nnq8", "ntq8"])
+@pytest.mark.parametrize("shape", [(600, 512, 8192), (200, 136, 32000), (2100, 4096, 2048)], ids=lambda s: "x".join(map(str, s)))
+def test_same_signed_terms_over_a_long_reduction(kind, shape):
+    """Where every term adds up, truncation at the accumulator would grow with K (8e-5 at 32000 over one
+    accumulator).  Held to the reference's 2e-6 of sum|a_k b_k|."""
+    got, want, mag, taken = _product(kind, *shape, True, B.COHERENCE_LAZY)
+    assert taken == 1
+    assert (np.abs(got - want) / mag).max() < 2e-6
