@@ -190,6 +190,41 @@ __device__ __forceinline__ void EpilogueStoreRagged(const UmmaEpilogue& ep, size
   }
 }
 
+// Piece products whose sum is not finite (UmmaEpilogue::src_a).  A warp's lanes ask for neighbouring columns of a row,
+// so this walks A by broadcasts and B, stored [K, N], by whole lines; nothing calls it while all values are finite.
+__device__ __noinline__ float4 DotsFromSource(const UmmaEpilogue& ep, size_t row, uint32_t n) {
+  const size_t K = ep.src_k, N = ep.N;
+  float v[4];
+#pragma unroll
+  for (uint32_t e = 0; e < 4; ++e) v[e] = n + e < ep.N ? 0.0f : __uint_as_float(0x7FC00000u);
+  for (size_t k = 0; k < K; ++k) {
+    float a = ep.src_a[ep.src_a_t ? k * ep.M + row : row * K + k];
+    if (ep.src_a_scale) a = a * ep.src_a_scale[k];
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+      if (n + e >= ep.N) continue;
+      const size_t at = ep.src_b_t ? (n + e) * K + k : k * N + n + e;
+      const float b = ep.src_b_type == BType::kF32   ? static_cast<const float*>(ep.src_b)[at]
+                      : ep.src_b_type == BType::kI8 ? static_cast<float>(static_cast<const int8_t*>(ep.src_b)[at])
+                                                    : __uint_as_float(static_cast<uint32_t>(static_cast<const uint16_t*>(ep.src_b)[at]) << 16);
+      v[e] = v[e] + a * b;
+    }
+    if (v[0] != v[0] && v[1] != v[1] && v[2] != v[2] && v[3] != v[3]) break;   // NaN for good: a diverged run's rows end at once
+  }
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+// A wait for a part of the CTA that may be in there: as bounded as the others, only longer.
+template <bool kSeg>
+__device__ __forceinline__ bool PartnerWait(uint64_t* bar, uint32_t parity) {
+  for (int i = 0; i < (kSeg ? 64 : 1); ++i)
+    if (MbarWait(bar, parity)) return true;
+  return false;
+}
+__device__ __forceinline__ float4 Checked(const UmmaEpilogue& ep, size_t row, uint32_t n, const float4& acc) {
+  const float zero = (acc.x * 0.0f + acc.y * 0.0f) + (acc.z * 0.0f + acc.w * 0.0f);   // NaN unless all are finite
+  return zero == 0.0f ? acc : DotsFromSource(ep, row, n);
+}
+
 // Element offsets along K of reduction block kb's tiles of A and B.
 struct BlockAt { int32_t a, b; bool aux; };
 __device__ __forceinline__ BlockAt BlockCoord(const UmmaEpilogue& ep, uint32_t kb, uint32_t main_blocks) {
@@ -252,7 +287,7 @@ template <uint32_t kTN, bool kSeg>
 __global__ void __launch_bounds__(kTThreads, 1)
 UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
-                   UmmaEpilogue ep, uint32_t splits) {
+                   const __grid_constant__ UmmaEpilogue ep, uint32_t splits) {
   using T = TTile<kTN>;
   constexpr uint32_t kStages = T::kStages, kStageBytes = T::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
@@ -454,6 +489,7 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           if constexpr (decltype(has_side)::value)
             side[u] = __ldg(reinterpret_cast<const float4*>(side_ptr + static_cast<size_t>(row) * ep.N + n));
           acc[u] = element(lr, chunk);
+          if constexpr (kSeg) acc[u] = Checked(ep, row, n, acc[u]);
         }
 #pragma unroll
         for (uint32_t u = 0; u < kUnroll; ++u) {
@@ -473,7 +509,10 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (ragged) {
       for (uint32_t i = et; i < rows * kChunks; i += kTEpiThreads) {
         const uint32_t lr = r0 + i / kChunks, row = m0 + lr, n = n0 + i % kChunks * 4;
-        if (row < ep.M && n < ep.N) EpilogueStoreRagged(ep, row, n, element(lr, i % kChunks));
+        if (row >= ep.M || n >= ep.N) continue;
+        float4 acc = element(lr, i % kChunks);
+        if constexpr (kSeg) acc = Checked(ep, row, n, acc);
+        EpilogueStoreRagged(ep, row, n, acc);
       }
     } else if (IsPlainStore(ep)) {
       each(NoSide{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4&) {
@@ -596,7 +635,8 @@ __global__ void __launch_bounds__(kPThreads, 1)
 UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
                          const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_a2,
-                         const __grid_constant__ CUtensorMap map_b2, UmmaEpilogue ep,
+                         const __grid_constant__ CUtensorMap map_b2,
+                         const __grid_constant__ UmmaEpilogue ep,
                          uint32_t band_blocks) {
   static_assert(!(kSideLoads && kSeg), "the sums take the registers of the loads in flight");
   using T = PTile<kPair>;
@@ -672,7 +712,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         }
         for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
           const uint32_t s = it % kPStages, round = it / kPStages;
-          if (round > 0 && !MbarWait(&bars->empty[s], (round - 1) & 1)) {
+          if (round > 0 && !PartnerWait<kSeg>(&bars->empty[s], (round - 1) & 1)) {
             ep.status->wait_timeout = 1;
             bars->abort = 1;
             ok = false;
@@ -707,7 +747,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
       bool ok = true;
       for (uint32_t t = unit, g = 0; t < total_tiles && ok; ++lt, g = g + 1 < groups ? g + 1 : (t += units, 0u)) {
         const uint32_t buf = lt & 1, use = lt >> 1;
-        if (use > 0 && !MbarWait(&bars->tmem_empty[buf], (use - 1) & 1)) {
+        if (use > 0 && !PartnerWait<kSeg>(&bars->tmem_empty[buf], (use - 1) & 1)) {
           ep.status->wait_timeout = 1;
           bars->abort = 1;
           break;
@@ -716,7 +756,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         const uint32_t acc = tmem_base + buf * kTN;
         for (uint32_t kb = 0; kb < group; ++kb, ++it) {
           const uint32_t s = it % kPStages, round = it / kPStages;
-          if (!MbarWait(&bars->full[s], round & 1)) {
+          if (!PartnerWait<kSeg && kPair>(&bars->full[s], round & 1)) {
             ep.status->wait_timeout = 1;
             bars->abort = 1;
             ok = false;
@@ -793,7 +833,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         }
       }
       auto await = [&] {
-        bool there = MbarWait(&bars->tmem_full[buf], use & 1);
+        bool there = PartnerWait<kSeg>(&bars->tmem_full[buf], use & 1);
         if (!there && lane == 0) { ep.status->wait_timeout = 1; bars->abort = 1; }
         if (bars->abort) there = false;
         there = __all_sync(0xFFFFFFFFu, there);
@@ -847,9 +887,11 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
           __syncwarp();
           const uint32_t n = n0 + col_group * kColsPerEpiWarp + pass * kSlabCols + cl * 4;
           if (ragged) {
-            for (uint32_t rr = sub; rr < rows; rr += kRowsPerInstr)
-              EpilogueStoreRagged(ep, row0 + rr, n, *reinterpret_cast<const float4*>(
-                                                        slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4)));
+            for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr) {
+              float4 acc = *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
+              if constexpr (kSeg) acc = Checked(ep, row0 + rr, n, acc);
+              EpilogueStoreRagged(ep, row0 + rr, n, acc);
+            }
           } else if (n < ep.N) {   // N % 4 == 0: a float4 is all in or all out
             float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
             if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
@@ -860,8 +902,8 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
               kscale = __ldg(reinterpret_cast<const float4*>(ep.shadow_k_scale + n));
   #pragma unroll 4
             for (uint32_t rr = sub; rr < rows; rr += kRowsPerInstr) {
-              const float4 acc = *reinterpret_cast<const float4*>(
-                  slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
+              float4 acc = *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
+              if constexpr (kSeg) acc = Checked(ep, row0 + rr, n, acc);
               const size_t at = static_cast<size_t>(row0 + rr) * ep.N + n;
               if (plain_store)
                 EpilogueStorePlain(ep, at, acc, scale);

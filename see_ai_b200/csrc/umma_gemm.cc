@@ -526,6 +526,13 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   ep.K = k_blocks * 64;
   ep.seg_blocks = static_cast<uint32_t>(Kp / 64);
   ep.segs = segments;
+  ep.src_a = a.A;
+  ep.src_b = a.B;
+  ep.src_a_scale = a.a_k_scale;
+  ep.src_k = static_cast<uint32_t>(a.K);
+  ep.src_a_t = a.a_transposed ? 1 : 0;
+  ep.src_b_t = a.b_transposed ? 1 : 0;
+  ep.src_b_type = a.b_type;
   ep.seg_a = exact_b ? kSegAExact : kSegAF32;
   ep.seg_b = exact_b ? kSegBExact : kSegBF32;
   ep.status = impl->status;

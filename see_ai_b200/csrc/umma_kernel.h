@@ -53,6 +53,15 @@ struct UmmaEpilogue {
   // piece number (seg_a >> 4s) & 15 by B's piece number (seg_b >> 4s) & 15; a block's products meet in one
   // accumulator, the blocks' accumulators in f32 registers.  K = 64 * seg_blocks * segs.  0: a plain product.
   uint32_t seg_blocks = 0, segs = 0, seg_a = 0, seg_b = 0;
+  // The operands the pieces were cut from.  Pieces of a value that is not finite, or larger than the largest bf16,
+  // do not add up to it; an output that is not finite is therefore made again from these, one multiply-add after
+  // the other.
+  const float* src_a = nullptr;        // [M, src_k], or [src_k, M] (src_a_t)
+  const void* src_b = nullptr;         // [src_k, N], or [N, src_k] (src_b_t)
+  const float* src_a_scale = nullptr;  // of column k of A, or null
+  uint32_t src_k = 0;
+  int src_a_t = 0, src_b_t = 0;
+  BType src_b_type = BType::kF32;
 };
 
 // Which kernel takes a product, on which tiles (k_gemm_umma.cu).

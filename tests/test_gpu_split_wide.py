@@ -131,3 +131,57 @@ def test_same_signed_terms_over_a_long_reduction(kind, shape):
     got, want, mag, taken = _product(kind, *shape, True, B.COHERENCE_LAZY)
     assert taken == 1
     assert (np.abs(got - want) / mag).max() < 2e-6
+
+
+# A cluster's splits, one tile per SM, ragged widths, the persistent kernel with aligned and ragged rows.
+NONFINITE = [(600, 512, 2048), (257, 2003, 520), (4096, 4096, 256), (5000, 3001, 72)]
+
+
+@pytest.mark.parametrize("kind", ["nn", "nt", "tn", "nnq8", "ntq8"])
+@pytest.mark.parametrize("shape", NONFINITE, ids=["x".join(map(str, s)) for s in NONFINITE])
+def test_values_no_piece_holds(kind, shape):
+    """Infinities, NaNs and finite values above the largest bf16 in an activation (and in an f32 weight) leave what
+    the kernels in the reference's order leave: the same infinities and NaNs, finite results to 1e-5 of the row."""
+    M, N, K = shape
+    rng = np.random.default_rng(M + N)
+    a = Arena(rng)
+    A, C = a.alloc(M * K), a.alloc(M * N)
+    X = rng.standard_normal((M, K)).astype(np.float32)
+    X[3, 5], X[M // 2, K - 1], X[M - 1, 0] = np.inf, -np.inf, np.nan
+    X[7, 2], X[7, 9] = np.inf, -np.inf
+    X[11, :] = 0.0
+    X[11, 4] = np.float32(3.4e38)      # finite, above the largest bf16
+    shape_w = (N, K) if kind.startswith("nt") else (K, N)
+    flags, last = 0, P.NULL_REF
+    if kind.endswith("q8"):
+        W = rng.integers(-127, 128, size=shape_w, dtype=np.int8)
+        W[5 % shape_w[0], 5] = 0       # infinity times zero
+        flags, op = P.FLAG_Q8_COL_SCALE, Op.GEMM_NT_Q8 if kind == "ntq8" else Op.GEMM_NN_Q8
+        last = a.ro_alloc((rng.random(K if kind == "ntq8" else N) * 0.001 + 1e-3).astype(np.float32))
+    else:
+        W = (rng.standard_normal(shape_w) * 0.02).astype(np.float32)
+        (W if kind.startswith("nt") else W.T)[9, 1] = np.inf
+        op = dict(nn=Op.GEMM_NN, nt=Op.GEMM_NT, tn=Op.GEMM_TN)[kind]
+    ins = P.Instr(op, flags, 0, (A, a.ro_alloc(W), C, last), (M, N, K))
+    arena, ro = a.build()
+    arena[A:A + X.nbytes] = (X.T if kind == "tn" else X).reshape(-1).copy().view(np.uint8)
+
+    def run(coherence):
+        got = arena.copy()
+        be = B.CudaBackend(0)
+        be.set_coherence(coherence)
+        be.bind(got, ro)
+        be.run([ins])
+        taken = be.counters().split_executions
+        be.host_needs(C, 4 * M * N)
+        be.close()
+        return got[C:C + 4 * M * N].view(np.float32).astype(np.float64).reshape(M, N), taken
+
+    (got, taken), (want, _) = run(B.COHERENCE_LAZY), run(B.COHERENCE_STRICT)
+    assert taken == (0 if kind.endswith("q8") and K % 8 else 1)
+    assert not np.isfinite(want).all() and np.isfinite(want).any()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    ok = np.isfinite(want)
+    scale = np.max(np.abs(np.where(ok, want, 0.0)), axis=1, keepdims=True)
+    assert (np.abs(np.where(ok, got - want, 0.0)) <= 1e-5 * scale).all()
