@@ -98,24 +98,30 @@ int see_cuda_set_epilogue_fusion(see_cuda_backend* h, int enabled);
 /* 0: an adapter's rank-r expand product stays its own kernel instead of riding the
  * frozen product's tensor-core reduction (lazy coherence only); default 1. */
 int see_cuda_set_lora_fold(see_cuda_backend* h, int enabled);
-/* 0: the rank-r adapter products keep one rounding per operation (the CPU's
- * arithmetic, bit for bit) in lazy coherence too; default 1: fused multiply-adds
- * there.  Strict coherence is always bit-exact. */
+/* 0: the rank-r adapter products, the smaller f32 products and the exact attention
+ * family keep one rounding per operation in the CPU's order (bit for bit) in lazy
+ * coherence too, and see_cuda_set_split_gemm's default domain is that of its mode 1;
+ * default 1: fused multiply-adds there, in an order that depends on the shape alone
+ * (of the products other than rank-r ones and of attention only while
+ * see_cuda_set_split_gemm is not 0).  Strict coherence is always bit-exact. */
 int see_cuda_set_adapter_fma(see_cuda_backend* h, int enabled);
 /* Lazy coherence: the relaxed attention forward keeps a private f32 copy of its output, and the dQ
  * instruction of the same attention takes delta_i = sum_j P_ij dP_ij as dO_i . O_i from it and walks
  * the keys once instead of twice.  Same quantity, another rounding (tolerance class, like every relaxed
  * attention result).  Default on; 0 keeps the two-walk kernel. */
 int see_cuda_set_attention_one_walk(see_cuda_backend* h, int enabled);
-/* Exact f32 products (kGemmNN / kGemmNT / kGemmTN without the relaxed permission)
- * of at least 2^26 multiply-adds on the tensor cores: both operands cut into
- * three bf16 pieces, six piece products over a K axis six times as long, f32
- * accumulation.  The result is the f32 product to a few 2^-24 of sum|a_k b_k|
- * (the reference holds its own GEMMs to 2e-6 of that: test/runtime/executor/
- * kernels_test.cc:1803-1822), not the CPU's bits.  mode -1 (default): in lazy
- * coherence only, and there from 2^24 multiply-adds, with int8 and bf16 weights
- * (one exact piece: three products) and any width; 0: never; 1: in strict
- * coherence too. */
+/* Exact products (without the relaxed permission) on the tensor cores: f32 operands
+ * cut into three bf16 pieces, the six largest piece products of 64 k at a time in one
+ * accumulator, the blocks of 64 added in rounded f32.  The result is as close to a
+ * float64 product as the CPU's order of sums is (the reference holds its own GEMMs to
+ * 2e-6 of sum|a_k b_k|: test/runtime/executor/kernels_test.cc:1803-1822), not its
+ * bits; an output that is not finite is made in f32 multiply-adds.  mode -1 (default):
+ * in lazy coherence only, there for products of at least 2^24 multiply-adds with
+ * M > 16, N >= 32 and K >= 32, also by int8 and bf16 weights outside the arena where
+ * K % 8 == 0 (one exact piece: three products).  1: kGemmNN / kGemmNT / kGemmTN of f32
+ * operands from 2^26 multiply-adds with M >= 128, N and K >= 64 and multiples of 4, in
+ * strict coherence too.  0: never, and every f32 product but the rank-r ones, and the
+ * exact attention family, keep the CPU's order of sums in lazy coherence as well. */
 int see_cuda_set_split_gemm(see_cuda_backend* h, int mode);
 /* Large tensor-core products run on CTA pairs (two SMs per 256 x 256 tile, each loading half of the
  * weight tile).  Default on; 0 = one CTA per 128 x 256 tile.  Results are identical either way (the same

@@ -1888,7 +1888,7 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
         pieces_made = adapter_fma_ && lf->down.flags == 0 && d.N == lf->r && k::LoraDownSupported(d.M, d.K, d.N) &&
                       k::LoraDown(d.A, static_cast<const float*>(d.B), d.C, d.M, d.K, d.N, d.alpha, stream_,
                                   d_lora_t_);
-        if (!pieces_made && !(adapter_fma_ && k::FastGemm(d, stream_))) k::GemmExact(d, stream_);
+        if (!pieces_made && !(OwnOrder() && k::FastGemm(d, stream_))) k::GemmExact(d, stream_);
         ++counters_.kernel_launches;
         umma::InvalidateRange(&umma_->ctx, RefOffset(lf->down.in[2]), d.M * d.N * 4);
       }
@@ -2030,7 +2030,7 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
   // pre-activation on the other side of a ReLU's kink than the CPU's moves a whole row of gradients.
   const bool expand = !a.a_transposed && a.K <= 16 && a.K % 4 == 0 && a.M >= 64 && a.N >= 64;
   const bool short_layer = !a.a_transposed && !a.b_transposed && a.M > 16 && a.N > 16 && a.K <= 256;
-  if (coherence_ == Coherence::kLazy && adapter_fma_ && !expand && !short_layer && !a.accumulate &&
+  if (OwnOrder() && !expand && !short_layer && !a.accumulate &&
       k::FastGemm(a, stream_)) {
     ++counters_.kernel_launches;
     return {};
@@ -2159,7 +2159,7 @@ Status CudaBackend::DispatchOptimizer(const Instruction& ins, const StepParams& 
 Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, const Extents&) {
   cudaStream_t s = stream_;
   auto launched = [&](int n = 1) { counters_.kernel_launches += n; };
-  const bool fused = coherence_ == Coherence::kLazy && adapter_fma_;   // (the exact attention family's output sums)
+  const bool fused = OwnOrder();   // (the exact attention family's output sums)
   if (range_index_ < merge_run_of_.size() && merge_run_of_[range_index_] != -1) {
     if (merge_run_of_[range_index_] == -2) return {};   // done by the run's first instruction
     return DispatchMergeRun(merge_runs_[static_cast<size_t>(merge_run_of_[range_index_])]);

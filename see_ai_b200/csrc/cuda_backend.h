@@ -466,10 +466,13 @@ class CudaBackend {
   float* d_lora_partials_ = nullptr;
   uint64_t lora_partials_capacity_ = 0;   // floats
   int split_gemm_mode_ = -1;
-  // In lazy coherence every exact product above 2^24 multiply-adds, any width and weight type; asked for
+  // In lazy coherence the exact products of umma::SplitGemmEligible's wide domain; asked for
   // explicitly (mode 1), or with adapter products in the CPU's arithmetic, the documented domain of
   // see_cuda_set_split_gemm alone.
   bool SplitGemmWide() const { return split_gemm_mode_ < 0 && adapter_fma_; }
+  // f32 sums may be fused and in an order of the kernels' own: small and narrow products, the exact attention
+  // family's output sums.
+  bool OwnOrder() const { return coherence_ == Coherence::kLazy && adapter_fma_ && split_gemm_mode_ != 0; }
   bool SplitGemmOn() const { return split_gemm_mode_ > 0 || (split_gemm_mode_ < 0 && coherence_ == Coherence::kLazy); }
   Status PrepareLoraFolds(const Instruction* program, size_t begin, uint64_t max_rows);
   void FreeLoraRanges();

@@ -65,3 +65,45 @@ def test_products_match_float64_and_repeat(shape):
     ]
     for off, want, scale in wants:
         assert (np.abs(mat(got, off, M, N) - want) / (1.0 + scale)).max() < 2e-6
+
+
+@pytest.mark.parametrize("shape", [(57, 128, 784), (33, 33, 5), (40, 64, 1030), (300, 260, 512), (600, 512, 768)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_split_gemm_0_keeps_the_order_of_the_strict_seam(shape):
+    """With the switch off, lazy coherence leaves the bits of the strict seam, which are the CPU's: products of
+    every form (nothing here is rank-r), the exact attention chain."""
+    M, N, K = shape
+    rng = np.random.default_rng(M + N + K)
+    a = Arena(rng)
+    A = a.alloc(M * K, "normal"); At = a.alloc(K * M, "normal"); Bm = a.alloc(K * N, "normal"); Bt = a.alloc(N * K, "normal")
+    outs = [a.alloc(M * N) for _ in range(3)]
+    Bq, S, H, d = 2, 70, 2, 16
+    n = Bq * S * H * d
+    q, k, v, do = (a.alloc(n, "normal") for _ in range(4))
+    o, dq, dk, dv = (a.alloc(n) for _ in range(4))
+    stats = a.alloc(4 * Bq * H * S)
+    geo, bs, hd = P.pack_attn_geometry(Bq, S, H, d), P.pack2(Bq, S), P.pack2(H, d)
+    prog = [
+        P.Instr(Op.GEMM_NN, 0, P.f32_bits(0.5), (A, Bm, outs[0], P.NULL_REF), (M, N, K)),
+        P.Instr(Op.GEMM_NT, 0, 0, (A, Bt, outs[1], P.NULL_REF), (M, N, K)),
+        P.Instr(Op.GEMM_TN, 0, 0, (At, Bm, outs[2], P.NULL_REF), (M, N, K)),
+        P.Instr(Op.ATTN_FWD_TILED, 0, 0, (q, k, v, o), (stats, bs, hd)),
+        P.Instr(Op.ATTN_DQ_TILED, 0, 0, (q, k, v, do), (stats, dq, geo)),
+        P.Instr(Op.ATTN_DK_TILED, 0, 0, (q, k, v, do), (stats, dk, geo)),
+        P.Instr(Op.ATTN_DV_TILED, 0, 0, (q, k, v, do), (stats, dv, geo)),
+    ]
+    arena0, ro = a.build()
+
+    def run(lazy):
+        arena = arena0.copy()
+        be = B.CudaBackend(0)
+        if lazy:
+            be.set_coherence(B.COHERENCE_LAZY)
+            be.set_split_gemm(0)
+        be.bind(arena, ro)
+        be.run(prog)
+        be.host_needs(0, arena.size)
+        be.close()
+        return arena
+
+    assert np.array_equal(run(True), run(False))
