@@ -175,13 +175,14 @@ __device__ __forceinline__ void EpilogueStoreBiasGelu(const UmmaEpilogue& ep, si
 
 // Four neighbouring columns of one row of an output whose width is no multiple of four (an odd vocabulary): rows
 // start at any 4-byte boundary, so everything moves one element at a time.  No absorbed activation, no copy.
-__device__ __forceinline__ void EpilogueStoreRagged(const UmmaEpilogue& ep, size_t row, uint32_t n, const float4& acc) {
+__device__ __forceinline__ void EpilogueStoreRagged(const UmmaEpilogue& ep, size_t row, uint32_t n, const float4& acc,
+                                                    bool scaled) {
   const float a[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
   for (uint32_t e = 0; e < 4; ++e) {
     if (n + e >= ep.N) continue;
     const size_t at = row * ep.N + n + e;
-    float v = a[e] * (ep.col_scale ? ep.col_scale[n + e] : ep.alpha);
+    float v = scaled ? a[e] : a[e] * (ep.col_scale ? ep.col_scale[n + e] : ep.alpha);
     if (ep.addend && !ep.addend_last) v = ep.addend[at] + v;
     if (ep.bias) v = v + ep.bias[n + e];
     if (ep.addend && ep.addend_last) v = ep.addend[at] + v;
@@ -190,7 +191,8 @@ __device__ __forceinline__ void EpilogueStoreRagged(const UmmaEpilogue& ep, size
   }
 }
 
-// Piece products whose sum is not finite (UmmaEpilogue::src_a).  A warp's lanes ask for neighbouring columns of a row,
+// Piece products whose sum is not finite (UmmaEpilogue::src_a), scaled where the CUDA-core kernels scale: alpha on A's
+// elements and col_scale on B's, or alpha on the sum where B is [N, K].  A warp's lanes ask for neighbouring columns of a row,
 // so this walks A by broadcasts and B, stored [K, N], by whole lines; nothing calls it while all values are finite.
 __device__ __noinline__ float4 DotsFromSource(const UmmaEpilogue& ep, size_t row, uint32_t n) {
   const size_t K = ep.src_k, N = ep.N;
@@ -200,18 +202,21 @@ __device__ __noinline__ float4 DotsFromSource(const UmmaEpilogue& ep, size_t row
   for (size_t k = 0; k < K; ++k) {
     float a = ep.src_a[ep.src_a_t ? k * ep.M + row : row * K + k];
     if (ep.src_a_scale) a = a * ep.src_a_scale[k];
+    if (!ep.src_b_t && !ep.col_scale) a = ep.alpha * a;
 #pragma unroll
     for (uint32_t e = 0; e < 4; ++e) {
       if (n + e >= ep.N) continue;
       const size_t at = ep.src_b_t ? (n + e) * K + k : k * N + n + e;
-      const float b = ep.src_b_type == BType::kF32   ? static_cast<const float*>(ep.src_b)[at]
-                      : ep.src_b_type == BType::kI8 ? static_cast<float>(static_cast<const int8_t*>(ep.src_b)[at])
-                                                    : __uint_as_float(static_cast<uint32_t>(static_cast<const uint16_t*>(ep.src_b)[at]) << 16);
+      float b = ep.src_b_type == BType::kF32   ? static_cast<const float*>(ep.src_b)[at]
+                : ep.src_b_type == BType::kI8 ? static_cast<float>(static_cast<const int8_t*>(ep.src_b)[at])
+                                              : __uint_as_float(static_cast<uint32_t>(static_cast<const uint16_t*>(ep.src_b)[at]) << 16);
+      if (ep.col_scale) b = b * ep.col_scale[n + e];
       v[e] = v[e] + a * b;
     }
     if (v[0] != v[0] && v[1] != v[1] && v[2] != v[2] && v[3] != v[3]) break;   // NaN for good: a diverged run's rows end at once
   }
-  return make_float4(v[0], v[1], v[2], v[3]);
+  const float after = ep.src_b_t && !ep.col_scale ? ep.alpha : 1.0f;
+  return make_float4(after * v[0], after * v[1], after * v[2], after * v[3]);
 }
 // A wait for a part of the CTA that may be in there: as bounded as the others, only longer.
 template <bool kSeg>
@@ -220,9 +225,12 @@ __device__ __forceinline__ bool PartnerWait(uint64_t* bar, uint32_t parity) {
     if (MbarWait(bar, parity)) return true;
   return false;
 }
-__device__ __forceinline__ float4 Checked(const UmmaEpilogue& ep, size_t row, uint32_t n, const float4& acc) {
-  const float zero = (acc.x * 0.0f + acc.y * 0.0f) + (acc.z * 0.0f + acc.w * 0.0f);   // NaN unless all are finite
-  return zero == 0.0f ? acc : DotsFromSource(ep, row, n);
+// True: *acc held a value that is not finite and now holds the scaled products.
+__device__ __forceinline__ bool Remade(const UmmaEpilogue& ep, size_t row, uint32_t n, float4* acc) {
+  const float zero = (acc->x * 0.0f + acc->y * 0.0f) + (acc->z * 0.0f + acc->w * 0.0f);   // NaN unless all are finite
+  if (zero == 0.0f) return false;
+  *acc = DotsFromSource(ep, row, n);
+  return true;
 }
 
 // Element offsets along K of reduction block kb's tiles of A and B.
@@ -489,7 +497,6 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           if constexpr (decltype(has_side)::value)
             side[u] = __ldg(reinterpret_cast<const float4*>(side_ptr + static_cast<size_t>(row) * ep.N + n));
           acc[u] = element(lr, chunk);
-          if constexpr (kSeg) acc[u] = Checked(ep, row, n, acc[u]);
         }
 #pragma unroll
         for (uint32_t u = 0; u < kUnroll; ++u) {
@@ -498,6 +505,8 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           if (i >= rows * kChunks || row >= ep.M || n >= ep.N) continue;
           float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
           if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
+          if constexpr (kSeg)
+            if (Remade(ep, row, n, &acc[u])) scale = make_float4(1.f, 1.f, 1.f, 1.f);
           store(static_cast<size_t>(row) * ep.N + n, row, n, acc[u], scale, side[u]);
         }
       }
@@ -511,8 +520,9 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t lr = r0 + i / kChunks, row = m0 + lr, n = n0 + i % kChunks * 4;
         if (row >= ep.M || n >= ep.N) continue;
         float4 acc = element(lr, i % kChunks);
-        if constexpr (kSeg) acc = Checked(ep, row, n, acc);
-        EpilogueStoreRagged(ep, row, n, acc);
+        bool scaled = false;
+        if constexpr (kSeg) scaled = Remade(ep, row, n, &acc);
+        EpilogueStoreRagged(ep, row, n, acc, scaled);
       }
     } else if (IsPlainStore(ep)) {
       each(NoSide{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4&) {
@@ -889,8 +899,9 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
           if (ragged) {
             for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr) {
               float4 acc = *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
-              if constexpr (kSeg) acc = Checked(ep, row0 + rr, n, acc);
-              EpilogueStoreRagged(ep, row0 + rr, n, acc);
+              bool scaled = false;
+              if constexpr (kSeg) scaled = Remade(ep, row0 + rr, n, &acc);
+              EpilogueStoreRagged(ep, row0 + rr, n, acc, scaled);
             }
           } else if (n < ep.N) {   // N % 4 == 0: a float4 is all in or all out
             float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
@@ -903,16 +914,18 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
   #pragma unroll 4
             for (uint32_t rr = sub; rr < rows; rr += kRowsPerInstr) {
               float4 acc = *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
-              if constexpr (kSeg) acc = Checked(ep, row0 + rr, n, acc);
+              float4 by = scale;
+              if constexpr (kSeg)
+                if (Remade(ep, row0 + rr, n, &acc)) by = make_float4(1.f, 1.f, 1.f, 1.f);
               const size_t at = static_cast<size_t>(row0 + rr) * ep.N + n;
               if (plain_store)
-                EpilogueStorePlain(ep, at, acc, scale);
+                EpilogueStorePlain(ep, at, acc, by);
               else if (copy_only)
-                EpilogueStoreCopy(ep, at, acc, scale);
+                EpilogueStoreCopy(ep, at, acc, by);
               else if (bias_gelu_only)
-                EpilogueStoreBiasGelu(ep, at, acc, scale, bias, kscale);
+                EpilogueStoreBiasGelu(ep, at, acc, by, bias, kscale);
               else
-                EpilogueStore(ep, at, n, acc, scale, bias, true, kscale);
+                EpilogueStore(ep, at, n, acc, by, bias, true, kscale);
             }
           }
           __syncwarp();   // the slab is rewritten next
