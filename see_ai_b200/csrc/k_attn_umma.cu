@@ -740,7 +740,9 @@ __device__ __forceinline__ bool RoleWait(BwdCtl* ctl, uint64_t* bar, uint32_t pa
   ctl->failed = 1;
   return false;
 }
-// The same by a whole warp, with one answer (a vote: what follows stays warp-uniform for the compiler).
+// The same by a whole warp, with one answer: when another role gives up, lanes that still saw their barrier complete
+// leave with the others instead of issuing a warp-wide tensor-memory access alone (and what follows stays warp-uniform
+// for the compiler).
 __device__ __forceinline__ bool WarpWait(BwdCtl* ctl, uint64_t* bar, uint32_t parity) {
   return __all_sync(0xFFFFFFFFu, RoleWait(ctl, bar, parity));
 }
@@ -908,7 +910,7 @@ AttnBwdKernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
         const uint32_t qi = tl.step0 * kHalf + half * 32 + lane;
         if (qi < a.S) next = stats[qi];   // past the end of the sequence: P = 2^-inf = 0
       } else {
-        if (!(ok = RoleWait(ctl, &ctl->stat_full[i & 1], (i >> 1) & 1))) break;
+        if (!(ok = WarpWait(ctl, &ctl->stat_full[i & 1], (i >> 1) & 1))) break;
         m2l = row_stat_s[(i & 1) * 256 + r_in];
         delta = row_stat_s[(i & 1) * 256 + 128 + r_in];
         __syncwarp();
@@ -924,7 +926,7 @@ AttnBwdKernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
           if (t + 1 < tl.steps && col0 + kHalf + lane < a.S) next = stats[col0 + kHalf + lane];
           __syncwarp();
         }
-        if (!(ok = RoleWait(ctl, &ctl->acc_full[g & 1], (g >> 1) & 1))) break;
+        if (!(ok = WarpWait(ctl, &ctl->acc_full[g & 1], (g >> 1) & 1))) break;
         TcFenceAfter();
         const uint32_t acc = t_lane + (g & 1) * 128;
         uint32_t rs[32], rp[32], w[16];
@@ -984,7 +986,7 @@ AttnBwdKernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     auto row_stats = [&](uint32_t i) {
       BwdTile tl;
       if (!BwdTileAt<kKV>(i, a.S, BH, &tl)) return;
-      if (!(ok = RoleWait(ctl, &ctl->stat_empty[i & 1], ((i >> 1) & 1) ^ 1))) return;
+      if (!(ok = WarpWait(ctl, &ctl->stat_empty[i & 1], ((i >> 1) & 1) ^ 1))) return;
       const uint32_t row = tl.row_tile * kTile + r_in, b = tl.bh / a.H, h = tl.bh - b * a.H;
       float m2l = 0.0f, delta = 0.0f;
       if (row < a.S) {
@@ -1017,7 +1019,7 @@ AttnBwdKernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
         if (!ok) break;
       }
       const uint32_t ob = i % Sh::kOutBufs;
-      if (!(ok = RoleWait(ctl, &ctl->out_full[ob], (i / Sh::kOutBufs) & 1))) break;
+      if (!(ok = WarpWait(ctl, &ctl->out_full[ob], (i / Sh::kOutBufs) & 1))) break;
       TcFenceAfter();
       const uint32_t b = tl.bh / a.H, h = tl.bh - b * a.H;
       const uint32_t row0w = tl.row_tile * kTile + quarter * 32;
