@@ -409,13 +409,16 @@ bool SplitShape(uint64_t M, uint64_t N, uint64_t K, bool wide) {
   return M >= 128 && N >= 64 && K >= 64 && (N & 3) == 0 && (K & 3) == 0;
 }
 
+// An int8 or bf16 weight is read where its one bf16 copy lies, made once per binding and unpadded: outside the arena,
+// with rows that start on 16-byte boundaries, as TMA wants them.
+bool ExactWeightFits(uint64_t K, bool in_arena) { return (K & 7) == 0 && !in_arena; }
+
 }  // namespace
 
 bool SplitGemmEligible(const k::GemmArgs& a, bool wide) {
   if (a.accumulate || !SplitShape(a.M, a.N, a.K, wide)) return false;
   if (!wide && (a.b_type != k::BType::kF32 || a.b_col_scale || a.a_k_scale)) return false;
-  // (a TMA operand's rows start on 16-byte boundaries: an exact weight is read where its copy lies, unpadded)
-  if (a.b_type != k::BType::kF32 && (a.K & 7) != 0) return false;
+  if (a.b_type != k::BType::kF32 && !ExactWeightFits(a.K, false)) return false;
   auto misaligned = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
   return !(misaligned(a.A) || misaligned(a.B) || misaligned(a.C) || misaligned(a.addend) || misaligned(a.bias) ||
            misaligned(a.b_col_scale) || misaligned(a.a_k_scale));
@@ -443,18 +446,19 @@ void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size
   uint64_t need_a = 0, need_b = 0;
   for (size_t i = begin; i < end; ++i) {
     const Instruction& ins = program[i];
+    const bool in_arena = RefSpace(ins.in[1]) == kArena;
+    const uint64_t M = ins.out[0], N = ins.out[1], K = ins.out[2];
     switch (ins.opcode) {
       case kGemmNN: case kGemmNT: case kGemmTN: break;
-      case kGemmNNQ8: case kGemmNTQ8: case kGemmNNBF16: case kGemmNTBF16: if (wide) break; [[fallthrough]];
+      case kGemmNNQ8: case kGemmNTQ8: case kGemmNNBF16: case kGemmNTBF16: if (wide && ExactWeightFits(K, in_arena)) break; [[fallthrough]];
       default: continue;
     }
-    const uint64_t M = ins.out[0], N = ins.out[1], K = ins.out[2];
     if (!SplitShape(M, N, K, wide)) continue;
-    if (relaxed_allowed && (ins.flags & kFlagRelaxed) && RefSpace(ins.in[1]) != kArena && ins.opcode != kGemmTN &&
+    if (relaxed_allowed && (ins.flags & kFlagRelaxed) && !in_arena && ins.opcode != kGemmTN &&
         GemmShape(M, N, K))
       continue;   // runs on plain bf16 operands
     need_a = std::max(need_a, M * 3 * PaddedK(K));
-    if (RefSpace(ins.in[1]) == kArena) need_b = std::max(need_b, N * 3 * PaddedK(K));
+    if (in_arena) need_b = std::max(need_b, N * 3 * PaddedK(K));
   }
   if (need_a > impl->split_a_capacity) impl->split_tag.valid = false;
   GrowSplit(impl, &impl->split_a, &impl->split_a_capacity, need_a, nullptr, true);
@@ -467,7 +471,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   Impl* impl = ctx->impl;
   if (!impl || !SplitGemmEligible(a, wide)) return {};
   const bool exact_b = a.b_type != k::BType::kF32;
-  if (exact_b && b_space == 0) return {};
+  if (exact_b && !ExactWeightFits(a.K, b_space == 0)) return {};
   const uint64_t Kp = PaddedK(a.K);
   if (a.M * 3 * Kp > impl->split_a_capacity) impl->split_tag.valid = false;
   if (!GrowSplit(impl, &impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream))

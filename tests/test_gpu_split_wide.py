@@ -185,3 +185,24 @@ def test_values_no_piece_holds(kind, shape):
     ok = np.isfinite(want)
     scale = np.max(np.abs(np.where(ok, want, 0.0)), axis=1, keepdims=True)
     assert (np.abs(np.where(ok, got, 0.0) - np.where(ok, want, 0.0)) <= 1e-5 * scale).all()
+
+
+def test_no_piece_buffer_for_products_that_are_refused():
+    """An int8 weight whose rows TMA cannot take runs on the CUDA cores: its activation needs no pieces (123 MB)."""
+    import torch
+
+    M, N, K = 20000, 256, 1001
+    rng = np.random.default_rng(5)
+    a = Arena(rng)
+    A, C = a.alloc(M * K), a.alloc(M * N)
+    rq, rs = a.ro_alloc(rng.integers(-127, 128, size=(K, N), dtype=np.int8)), a.ro_alloc(np.ones(N, np.float32))
+    arena, ro = a.build()
+    be = B.CudaBackend(0)
+    be.set_coherence(B.COHERENCE_LAZY)
+    be.bind(arena, ro)
+    be.run([P.Instr(Op.GEMM_NN, 0, 0, (A, A, C, P.NULL_REF), (1, 1, 1))])   # (what a first run allocates)
+    before = torch.cuda.mem_get_info(0)[0]
+    be.run([P.Instr(Op.GEMM_NN_Q8, P.FLAG_Q8_COL_SCALE, 0, (A, rq, C, rs), (M, N, K))])
+    taken = before - torch.cuda.mem_get_info(0)[0]
+    be.close()
+    assert taken < 64 << 20, taken
