@@ -76,11 +76,7 @@ Status CudaBackend::Init() {
   d_count_ = reinterpret_cast<unsigned long long*>(base + 192);
   d_scalars_ = reinterpret_cast<k::AdamScalars*>(base + 256);
   d_partials_ = reinterpret_cast<double*>(base + 4096);
-  // One pinned block: what a flush publishes, then the staging of a strict flush's downloads.
-  if (auto r = Check(cudaMallocHost(reinterpret_cast<void**>(&h_published_), kPublishedBytes + kFlushStaging), "pinned status");
-      !r)
-    return r;
-  h_flush_ = reinterpret_cast<uint8_t*>(h_published_) + kPublishedBytes;
+  if (auto r = Check(cudaMallocHost(reinterpret_cast<void**>(&h_published_), kPublishedBytes), "pinned status"); !r) return r;
   umma_ = std::make_unique<UmmaState>();
   if (std::string e = umma::Init(&umma_->ctx, device_, d_status_); !e.empty()) return std::unexpected(e);
   return {};
@@ -106,6 +102,7 @@ CudaBackend::~CudaBackend() {
   for (float* p : attn_keep_pool_) cudaFree(p);
   cudaFree(d_lora_partials_);
   if (h_published_) cudaFreeHost(h_published_);
+  if (h_flush_) cudaFreeHost(h_flush_);
   if (own_stream_ && stream_) cudaStreamDestroy(stream_);
 }
 
@@ -1623,6 +1620,11 @@ Status CudaBackend::FlushWith(std::initializer_list<k::PublishItem> items, uint3
   if (strict) {
     for (const auto& [off, bytes] : device_dirty_) { lo = std::min(lo, off); hi = std::max(hi, off + bytes); }
     staged = hi - lo <= kFlushStaging;
+    if (staged && !h_flush_ && cudaMallocHost(reinterpret_cast<void**>(&h_flush_), kFlushStaging) != cudaSuccess) {
+      cudaGetLastError();   // no pinned memory to be had: range by range
+      h_flush_ = nullptr;
+      staged = false;
+    }
     if (staged) {
       if (auto r = Check(cudaMemcpyAsync(h_flush_, d_arena_ + lo, hi - lo, cudaMemcpyDeviceToHost, stream_),
                          "flush download"); !r)
