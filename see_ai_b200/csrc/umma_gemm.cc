@@ -75,6 +75,7 @@ struct Impl {
   uint32_t sms = 148;
   uint64_t moves = 0;   // device buffers of this context freed since it was made (BufferMoves)
   std::map<WeightKey, uint16_t*> split_weights;          // frozen B operands, once per binding
+  std::set<WeightKey> split_refused;                     // those there was no memory for
 };
 
 std::string Init(Context* ctx, int device, k::DeviceStatus* status) {
@@ -116,6 +117,7 @@ void InvalidateAll(Context* ctx) {
   ctx->impl->weights.clear();
   for (auto& [key, buf] : ctx->impl->split_weights) cudaFree(buf);
   ctx->impl->split_weights.clear();
+  ctx->impl->split_refused.clear();
   for (auto& a : ctx->impl->acts) a.valid = false;
   for (auto& e : ctx->impl->packs) e.valid = false;
   ctx->impl->split_tag.valid = false;
@@ -440,6 +442,14 @@ static bool GrowSplit(Impl* impl, uint16_t** buf, uint64_t* cap, uint64_t need, 
   return true;
 }
 
+// The same for a product outside any planned range; never while the stream is being captured.
+static bool RoomFor(Impl* impl, uint16_t** buf, uint64_t* cap, uint64_t need, cudaStream_t stream) {
+  if (need <= *cap) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) return false;
+  return GrowSplit(impl, buf, cap, need, stream);
+}
+
 void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size_t end, bool wide, bool relaxed_allowed) {
   Impl* impl = ctx->impl;
   if (!impl) return;
@@ -473,9 +483,35 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   const bool exact_b = a.b_type != k::BType::kF32;
   if (exact_b && !ExactWeightFits(a.K, b_space == 0)) return {};
   const uint64_t Kp = PaddedK(a.K);
+  // No memory for a copy or for pieces: the product stays on the CUDA cores, which need neither.
   if (a.M * 3 * Kp > impl->split_a_capacity) impl->split_tag.valid = false;
-  if (!GrowSplit(impl, &impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream))
-    return "tensor-core path: operand-piece allocation failed";
+  if (!RoomFor(impl, &impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream)) return {};
+  // B: wanted as [N][K]; stored [N, K] (NT) or [K, N] (NN, TN).
+  uint16_t* b = nullptr;
+  if (b_space != 0) {   // frozen: once per binding
+    const WeightKey key{b_space, b_off, a.N, a.K, !a.b_transposed, exact_b ? static_cast<int>(a.b_type) : 100, ~0ull};
+    if (impl->split_refused.count(key)) return {};
+    if (exact_b) {
+      b = WeightCopy(impl, a, b_space, b_off, nullptr, ~0ull, stream, launches);
+    } else if (auto it = impl->split_weights.find(key); it != impl->split_weights.end()) {
+      b = it->second;
+    } else if (void* p = nullptr; cudaMalloc(&p, a.N * 3 * Kp * 2) == cudaSuccess) {
+      b = static_cast<uint16_t*>(p);
+      k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);
+      ++*launches;
+      impl->split_weights.emplace(key, b);
+    }
+    if (!b) {   // (not asked for again under this binding: a captured range must take the way its eager pass took)
+      cudaGetLastError();
+      impl->split_refused.insert(key);
+      return {};
+    }
+  } else {
+    if (!RoomFor(impl, &impl->split_b, &impl->split_b_capacity, a.N * 3 * Kp, stream)) return {};
+    b = impl->split_b;
+    k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);
+    ++*launches;
+  }
   // A: [M, K], or [K, M] for the transposed-A form.
   auto& tag = impl->split_tag;
   if (!(tag.valid && a_space == 0 && tag.off == a_off && tag.M == a.M && tag.K == a.K && tag.transposed == a.a_transposed &&
@@ -484,30 +520,6 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
     ++*launches;
     tag.valid = a_space == 0;
     tag.off = a_off; tag.M = a.M; tag.K = a.K; tag.transposed = a.a_transposed; tag.k_scale = a.a_k_scale;
-  }
-  // B: wanted as [N][K]; stored [N, K] (NT) or [K, N] (NN, TN).
-  uint16_t* b = nullptr;
-  if (exact_b) {
-    b = WeightCopy(impl, a, b_space, b_off, nullptr, ~0ull, stream, launches);
-    if (!b) return "tensor-core path: weight copy allocation failed";
-  } else if (b_space != 0) {   // frozen: once per binding
-    const WeightKey key{b_space, b_off, a.N, a.K, !a.b_transposed, 100, ~0ull};
-    if (auto it = impl->split_weights.find(key); it != impl->split_weights.end()) {
-      b = it->second;
-    } else {
-      void* p = nullptr;
-      if (cudaMalloc(&p, a.N * 3 * Kp * 2) != cudaSuccess) return "tensor-core path: weight-piece allocation failed";
-      b = static_cast<uint16_t*>(p);
-      k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);
-      ++*launches;
-      impl->split_weights.emplace(key, b);
-    }
-  } else {
-    if (!GrowSplit(impl, &impl->split_b, &impl->split_b_capacity, a.N * 3 * Kp, stream))
-      return "tensor-core path: operand-piece allocation failed";
-    b = impl->split_b;
-    k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);
-    ++*launches;
   }
   const uint32_t segments = exact_b ? kSegExact : kSegF32;
   const uint32_t k_blocks = static_cast<uint32_t>(segments * (Kp / 64));
