@@ -10,6 +10,15 @@ namespace see {
 
 namespace {
 
+// A [rank x width] or [width x rank] gradient over so many rows that the kernel that streams them in chunks, split over
+// the grid, beats the clusters of k::FastGemm (us on a B200, clusters / stream, 768 wide, rank 8: [rank x width] 12.8 /
+// 14.7 at 4096 rows, 18.4 / 16.8 at 8192, 47.6 / 39.4 at 32768; [width x rank] 16.9 / 20.9 at 8192, 45.5 / 41.5 at
+// 32768; at 256 and 3072 wide the lines are the same within a few per cent).
+bool StreamedGradient(uint64_t M, uint64_t N, uint64_t K) {
+  const uint64_t r = std::min(M, N), width = std::max(M, N);
+  return r <= 16 && r % 4 == 0 && r > 0 && width >= 64 && width % 2 == 0 && K >= (M <= N ? 8192u : 16384u);
+}
+
 std::string CudaErr(cudaError_t e, const char* what) {
   return std::string("cuda: ") + what + ": " + cudaGetErrorString(e);
 }
@@ -382,6 +391,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
     const Instruction& ins = program[i];
     switch (ins.opcode) {
       case kGemmTN: {
+        if (OwnOrder() && !StreamedGradient(ins.out[0], ins.out[1], ins.out[2])) break;   // (nothing of it uses the scratch)
         const uint64_t chunks = k::SplitKChunks(ins.out[0], ins.out[1], ins.out[2]);
         if (chunks > 1) split = std::max(split, chunks * ins.out[0] * ins.out[1]);
         break;
@@ -2031,9 +2041,12 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
   // following add may ride it.  A forward layer of short reduction keeps the reference's order of sums: its
   // 16 x 16-block kernel is as fast there (feed-forward step at a batch of 32: 100 us against 106), and a
   // pre-activation on the other side of a ReLU's kink than the CPU's moves a whole row of gradients.
+  // The gradient of a rank-r factor over many rows is a stream as well: its chunks of rows go through scratch.
   const bool expand = !a.a_transposed && a.K <= 16 && a.K % 4 == 0 && a.M >= 64 && a.N >= 64;
+  const bool streamed = a.a_transposed && StreamedGradient(a.M, a.N, a.K) &&
+                        k::SplitKChunks(a.M, a.N, a.K) * a.M * a.N <= split_capacity_;
   const bool short_layer = !a.a_transposed && !a.b_transposed && a.M > 16 && a.N > 16 && a.K <= 256;
-  if (OwnOrder() && !expand && !short_layer && !a.accumulate &&
+  if (OwnOrder() && !expand && !streamed && !short_layer && !a.accumulate &&
       k::FastGemm(a, stream_)) {
     ++counters_.kernel_launches;
     return {};

@@ -107,3 +107,34 @@ def test_split_gemm_0_keeps_the_order_of_the_strict_seam(shape):
         return arena
 
     assert np.array_equal(run(True), run(False))
+
+
+@pytest.mark.parametrize("shape", [(16, 768, 8191), (16, 768, 8192), (8, 66, 20001), (768, 16, 16383), (768, 16, 16384), (256, 4, 17000)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_gradients_over_many_rows(shape):
+    """Both sides of the row counts at which a rank-r factor's gradient goes from clusters to chunks of rows, in a
+    run of its own and behind one that needs less scratch; the reference's bound for its GEMMs as above."""
+    M, N, K = shape
+    rng = np.random.default_rng(M + N + K)
+    a = Arena(rng)
+    At, Bm, C = a.alloc(K * M, "normal"), a.alloc(K * N, "normal"), a.alloc(M * N)
+    arena0, ro = a.build()
+    big = P.Instr(Op.GEMM_TN, 0, P.f32_bits(2.0), (At, Bm, C, P.NULL_REF), (M, N, K))
+    small = P.Instr(Op.GEMM_TN, 0, 0, (At, Bm, C, P.NULL_REF), (M, N, 300))
+
+    def run(progs):
+        arena = arena0.copy()
+        be = B.CudaBackend(0)
+        be.set_coherence(B.COHERENCE_LAZY)
+        be.bind(arena, ro)
+        for p in progs:
+            be.run(p)
+        be.host_needs(C, 4 * M * N)
+        be.close()
+        return arena[C:C + 4 * M * N].view(np.float32).astype(np.float64).reshape(M, N)
+
+    got = run([[big]])
+    assert np.array_equal(got, run([[small], [big], [small, big]]))
+    x = arena0[At:At + 4 * K * M].view(np.float32).astype(np.float64).reshape(K, M)
+    w = arena0[Bm:Bm + 4 * K * N].view(np.float32).astype(np.float64).reshape(K, N)
+    assert (np.abs(got - 2.0 * (x.T @ w)) / (1.0 + 2.0 * (np.abs(x).T @ np.abs(w)))).max() < 2e-6
