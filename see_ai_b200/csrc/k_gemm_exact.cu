@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kThreads) MergeDeltasKernel(const __grid_const
 // With fewer 64 x 64 (or skinny) tiles than SMs the kernels above are a serial chain of global loads: K / 16 steps of
 // about 1.4 us in one or two blocks.  Here a block owns 16 R x 16 R outputs, R x R per thread, so that there are blocks
 // to go round, and takes K 128 at a time with the next 128 already on their way in registers while these are
-// multiplied.  The same operations per output in the same order (57 x 8 x 784: 81.5 -> 5 us; 57 x 128 x 784: 76 -> 6 us).
+// multiplied.  The same operations per output in the same order (57 x 8 x 784: 81.5 -> 11.2 us; 57 x 128 x 784: 76 -> 12.5 us).
 constexpr int kFlatK = 128;
 template <bool TA, bool TB, typename BT, int R>
 struct FlatLoader {

@@ -11,15 +11,15 @@
 // of a cluster (up to eight, as many as bring the grid to one CTA per SM), and
 // inside a CTA over its eight warps.  A CTA's operand slices arrive by cp.async, 128 k
 // at a time in two buffers, in the layout they have in memory; each warp holds the
-// whole output tile in registers (RM x RN per lane) for its sixteenth-of-128 slice
-// of k.  The eight partial tiles are added in warp order through shared memory, the
+// whole output tile in registers (RM x RN per lane) for its eighth of the chunk's
+// k.  The eight partial tiles are added in warp order through shared memory, the
 // CTAs' in rank order through distributed shared memory.
 // Wide activations streamed through a narrow product (t = x A at thousands of rows)
 // are HBM-bound on the same kernel: one pass over x.
 //
 // Measured on a B200, us, before (one 64 x 64 or 256 x 16 tile per CTA, K serial) / now:
-// 32 x 1024 x 256 24.6 / 4; 32 x 64 x 1024 88.8 / 5; 600 x 8 x 512 10 / 5; 4096 x 8 x 4096
-// 944 / 25.
+// 32 x 1024 x 256 24.6 / 4; 32 x 64 x 1024 88.8 / 5.2; 600 x 8 x 512 70 / 4.3; 4096 x 8 x
+// 4096 944 / 26.  (Gradients of a rank-r factor over many rows stream: cuda_backend.cc.)
 #include <algorithm>
 #include <atomic>
 

@@ -11,9 +11,9 @@
 // tcgen05.ld and apply scale / addend / bias / activation on the way to HBM.
 // Two kernels: UmmaGemmTileKernel for products of about one tile per SM, whose
 // time is latency and operand delivery, and UmmaGemmPersistentKernel for those
-// with several tiles per SM.  The reduction may also be a list of segments of
-// bf16 pieces (UmmaEpilogue::seg_blocks), which makes either an f32-accurate
-// product.
+// with several tiles per SM.  The operands may also be bf16 pieces side by side
+// (UmmaEpilogue::seg_blocks), which makes either an f32-accurate product: 64 k of
+// piece products per accumulator, the accumulators added in registers.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out raises
 // DeviceStatus::wait_timeout, the CTA stops issuing work, frees its tensor
