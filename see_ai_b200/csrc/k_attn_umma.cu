@@ -202,12 +202,6 @@ __device__ __forceinline__ void StoreOutRows(uint32_t t_out, float* slab, uint32
   }
 }
 
-// After a wait ran out: give copies that may still be in flight towards this CTA's
-// shared memory a bounded time to land before the CTA retires.
-__device__ __forceinline__ void DrainDelay() {
-  for (int i = 0; i < 64; ++i) __nanosleep(2000);
-}
-
 constexpr uint32_t TmemColsFor(uint32_t need) { return need <= 128 ? 128 : (need <= 256 ? 256 : 512); }
 
 // ---- forward -------------------------------------------------------------------------

@@ -557,6 +557,7 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   TcFenceBefore();
   __syncthreads();
+  if (bars->abort) DrainDelay();
   if (splits > 1) ClusterSync();   // no CTA leaves while another may still read its memories
   if (warp == 1) {
     TcFenceAfter();
@@ -1011,6 +1012,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (bars->abort) DrainDelay();
   if constexpr (kPair) ClusterSync();   // neither CTA leaves while the other may still read its memories
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

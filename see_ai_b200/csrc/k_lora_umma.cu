@@ -474,6 +474,7 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
 
   TcFenceBefore();
   __syncthreads();
+  if (bars->abort) DrainDelay();
   if (warp == 1) {
     TcFenceAfter();
     TmemFree(tmem_base, kTmemCols);

@@ -14,6 +14,12 @@ namespace see::k::umma_dev {
 
 constexpr uint32_t kWaitLimit = 1u << 22;
 
+// After a wait ran out: give copies that may still be in flight towards this CTA's
+// shared memory a bounded time to land before the CTA retires.
+__device__ __forceinline__ void DrainDelay() {
+  for (int i = 0; i < 64; ++i) __nanosleep(2000);
+}
+
 __device__ __forceinline__ uint32_t SmemAddr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
