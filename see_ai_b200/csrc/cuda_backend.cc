@@ -2028,7 +2028,6 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     int launches = 0;
     auto space = [](uint64_t ref) { return RefSpace(ref) == kArena ? 0 : (RefSpace(ref) == kRodata ? 1 : 2); };
     const std::string err = umma::TrySplitGemm(&umma_->ctx, a, SplitGemmWide(), space(ins.in[0]), RefOffset(ins.in[0]),
-                                               !a.a_k_scale || RefSpace(ins.in[3]) != kArena,
                                                space(ins.in[1]), RefOffset(ins.in[1]), stream_, &launches);
     if (!err.empty()) return std::unexpected("cuda: " + err);
     if (launches > 0) {

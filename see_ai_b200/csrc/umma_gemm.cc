@@ -475,8 +475,8 @@ void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size
   GrowSplit(impl, &impl->split_b, &impl->split_b_capacity, need_b, nullptr, true);
 }
 
-std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_space, uint64_t a_off, bool scale_frozen,
-                         int b_space, uint64_t b_off, cudaStream_t stream, int* launches) {
+std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_space, uint64_t a_off, int b_space,
+                         uint64_t b_off, cudaStream_t stream, int* launches) {
   *launches = 0;
   Impl* impl = ctx->impl;
   if (!impl || !SplitGemmEligible(a, wide)) return {};
@@ -518,7 +518,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
         tag.k_scale == a.a_k_scale)) {
     k::SplitMatrix(a.A, impl->split_a, a.M, a.K, a.a_transposed, a.a_k_scale, stream);
     ++*launches;
-    tag.valid = a_space == 0 && (!a.a_k_scale || scale_frozen);
+    tag.valid = a_space == 0;
     tag.off = a_off; tag.M = a.M; tag.K = a.K; tag.transposed = a.a_transposed; tag.k_scale = a.a_k_scale;
   }
   const uint32_t segments = exact_b ? kSegExact : kSegF32;

@@ -69,9 +69,9 @@ std::string TryLoraBackward(Context* ctx, const k::LoraBackwardArgs& args, cudaS
 // 2^24: at 128 x 512 x 256 the split costs what the CUDA-core kernel costs.
 // *launches == 0 with an empty return value: outside the domain, use the exact kernels.
 bool SplitGemmEligible(const k::GemmArgs& args, bool wide);
-// a_space / b_space: 0 = arena, 1 = rodata, 2 = source model.  scale_frozen: args.a_k_scale, if any, lies outside the arena.
-std::string TrySplitGemm(Context* ctx, const k::GemmArgs& args, bool wide, int a_space, uint64_t a_off, bool scale_frozen,
-                         int b_space, uint64_t b_off, cudaStream_t stream, int* launches);
+// a_space / b_space: 0 = arena, 1 = rodata, 2 = source model.
+std::string TrySplitGemm(Context* ctx, const k::GemmArgs& args, bool wide, int a_space, uint64_t a_off, int b_space,
+                         uint64_t b_off, cudaStream_t stream, int* launches);
 // Sizes the two operand buffers for the largest eligible product of a range
 // (called with the other per-range sizing, before any capture).
 void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size_t end, bool wide,

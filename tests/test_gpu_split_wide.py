@@ -206,31 +206,3 @@ def test_no_piece_buffer_for_products_that_are_refused():
     taken = before - torch.cuda.mem_get_info(0)[0]
     be.close()
     assert taken < 64 << 20, taken
-
-
-def test_a_scale_rewritten_between_two_products_of_one_activation():
-    """The pieces of an activation serve the next product too; not where the scale cut into them has changed."""
-    M, N, K = 256, 512, 256
-    rng = np.random.default_rng(8)
-    a = Arena(rng)
-    A, C0, C1 = a.alloc(M * K, "normal"), a.alloc(M * N), a.alloc(M * N)
-    s, s2 = a.alloc(K, "normal"), a.alloc(K, "normal")
-    rq = a.ro_alloc(rng.integers(-127, 128, size=(N, K), dtype=np.int8))
-    arena0, ro = a.build()
-    prog = [P.Instr(Op.GEMM_NT_Q8, P.FLAG_Q8_COL_SCALE, 0, (A, rq, C0, s), (M, N, K)),
-            P.Instr(Op.COPY, 0, 0, (s2, s), (K,)),
-            P.Instr(Op.GEMM_NT_Q8, P.FLAG_Q8_COL_SCALE, 0, (A, rq, C1, s), (M, N, K))]
-
-    def run(coherence):
-        arena = arena0.copy()
-        be = B.CudaBackend(0)
-        be.set_coherence(coherence)
-        be.bind(arena, ro)
-        be.run(prog)
-        be.host_needs(C0, 4 * M * N)
-        be.host_needs(C1, 4 * M * N)
-        be.close()
-        return [arena[c:c + 4 * M * N].view(np.float32).copy() for c in (C0, C1)]
-
-    for got, want in zip(run(B.COHERENCE_LAZY), run(B.COHERENCE_STRICT)):
-        assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
