@@ -2037,9 +2037,10 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     }
   }
   // Small and narrow products likewise, but for the rank-r expand product of many rows: that one is a stream, and a
-  // following add may ride it.  A forward layer of short reduction keeps the reference's order of sums: its
-  // 16 x 16-block kernel is as fast there (feed-forward step at a batch of 32: 100 us against 106), and a
-  // pre-activation on the other side of a ReLU's kink than the CPU's moves a whole row of gradients.
+  // following add may ride it.  A forward layer of short reduction takes the kernel in the reference's order of
+  // sums, which is the faster one there (us, that / k::FastGemm, over 17 to 512 rows and widths of 32 to 1024: K = 64
+  // 6.6 - 8.7 / 8.8 - 10.8, K = 256 8.7 / 8.7 - 10.8, K = 384 10.7 / 8.7 - 12.4, K = 512 12.8 / 8.8 - 12.5, K = 1024 18.9 /
+  // 10.8) and keeps its pre-activations on the CPU's side of a ReLU's kink.
   // The gradient of a rank-r factor over many rows is a stream as well: its chunks of rows go through scratch.
   const bool expand = !a.a_transposed && a.K <= 16 && a.K % 4 == 0 && a.M >= 64 && a.N >= 64;
   const bool streamed = a.a_transposed && StreamedGradient(a.M, a.N, a.K) &&

@@ -194,7 +194,7 @@ __device__ __forceinline__ void EpilogueStoreRagged(const UmmaEpilogue& ep, size
 // Piece products whose sum is not finite (UmmaEpilogue::src_a), scaled where the CUDA-core kernels scale: alpha on A's
 // elements and col_scale on B's, or alpha on the sum where B is [N, K].  A warp's lanes ask for neighbouring columns of a row,
 // so this walks A by broadcasts and B, stored [K, N], by whole lines; nothing calls it while all values are finite.
-__device__ __noinline__ float4 DotsFromSource(const UmmaEpilogue& ep, size_t row, uint32_t n) {
+__device__ __forceinline__ float4 DotsFromSource(const UmmaEpilogue& ep, size_t row, uint32_t n) {
   const size_t K = ep.src_k, N = ep.N;
   float v[4];
 #pragma unroll
@@ -218,19 +218,36 @@ __device__ __noinline__ float4 DotsFromSource(const UmmaEpilogue& ep, size_t row
   const float after = ep.src_b_t && !ep.col_scale ? ep.alpha : 1.0f;
   return make_float4(after * v[0], after * v[1], after * v[2], after * v[3]);
 }
-// A wait for a part of the CTA that may be in there: as bounded as the others, only longer.
-template <bool kSeg>
-__device__ __forceinline__ bool PartnerWait(uint64_t* bar, uint32_t parity) {
-  for (int i = 0; i < (kSeg ? 64 : 1); ++i)
-    if (MbarWait(bar, parity)) return true;
-  return false;
-}
 // True: *acc held a value that is not finite and now holds the scaled products.
 __device__ __forceinline__ bool Remade(const UmmaEpilogue& ep, size_t row, uint32_t n, float4* acc) {
   const float zero = (acc->x * 0.0f + acc->y * 0.0f) + (acc->z * 0.0f + acc->w * 0.0f);   // NaN unless all are finite
   if (zero == 0.0f) return false;
   *acc = DotsFromSource(ep, row, n);
   return true;
+}
+// Four outputs of a tile in which some sum is not finite: made again where they are the ones.
+__device__ __noinline__ void StoreRemade(const UmmaEpilogue& ep, size_t row, uint32_t n, float4 acc) {
+  const bool made = Remade(ep, row, n, &acc);
+  if ((ep.N & 3u) != 0) { EpilogueStoreRagged(ep, row, n, acc, made); return; }
+  float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha), bias = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
+  if (made) scale = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (ep.bias) bias = __ldg(reinterpret_cast<const float4*>(ep.bias + n));
+  EpilogueStore(ep, row * ep.N + n, n, acc, scale, bias);
+}
+template <uint32_t kCount>
+__device__ __forceinline__ bool AllFinite(const float (&v)[kCount]) {
+  float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // NaN once something is not
+#pragma unroll
+  for (uint32_t j = 0; j < kCount; ++j) zero[j & 3] = fmaf(v[j], 0.0f, zero[j & 3]);
+  return (zero[0] + zero[1]) + (zero[2] + zero[3]) == 0.0f;
+}
+// A wait for a part of the CTA that may be in there: as bounded as the others, only longer.
+template <bool kSeg>
+__device__ __forceinline__ bool PartnerWait(uint64_t* bar, uint32_t parity) {
+  for (int i = 0; i < (kSeg ? 64 : 1); ++i)
+    if (MbarWait(bar, parity)) return true;
+  return false;
 }
 
 // Element offsets along K of reduction block kb's tiles of A and B.
@@ -281,9 +298,15 @@ struct __align__(8) TBarriers {
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];   // piece products only
   uint32_t tmem_base;
-  volatile uint32_t abort;  // set by a role whose wait ran out; the epilogue then stores nothing
+  volatile uint32_t abort;      // set by a role whose wait ran out; the epilogue then stores nothing
+  volatile uint32_t nonfinite;  // piece products: some sum of this CTA is not finite
 };
 
+__device__ __forceinline__ uint32_t LoadClusterU32(uint32_t cluster_addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr));
+  return v;
+}
 __device__ __forceinline__ float4 LoadClusterF4(uint32_t cluster_addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -330,6 +353,7 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       MbarInit(&bars->tmem_empty[b], kTEpiThreads / 32);
     }
     bars->abort = 0;
+    bars->nonfinite = 0;
     MbarInitFence();
   }
   if (warp == 1) {
@@ -449,6 +473,7 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       // row so that neither side conflicts.
       float* dump = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kTN;
       if constexpr (kSeg) {
+        if (!AllFinite(sum)) bars->nonfinite = 1;
 #pragma unroll
         for (uint32_t q = 0; q < kTN / 8; ++q)
           *reinterpret_cast<float4*>(dump + (((columns >> 2) + q) ^ (lane & 7u)) * 4) =
@@ -505,8 +530,6 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           if (i >= rows * kChunks || row >= ep.M || n >= ep.N) continue;
           float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
           if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
-          if constexpr (kSeg)
-            if (Remade(ep, row, n, &acc[u])) scale = make_float4(1.f, 1.f, 1.f, 1.f);
           store(static_cast<size_t>(row) * ep.N + n, row, n, acc[u], scale, side[u]);
         }
       }
@@ -515,14 +538,19 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     auto bias_at = [&](uint32_t n) { return ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : none; };
     using Side = std::true_type;
     using NoSide = std::false_type;
-    if (ragged) {
+    bool remake = false;   // (an element's splits lie in several CTAs)
+    if constexpr (kSeg)
+      for (uint32_t p = 0; p < splits; ++p)
+        remake = remake || (splits == 1 ? bars->nonfinite : LoadClusterU32(MapToCta(SmemAddr(const_cast<uint32_t*>(&bars->nonfinite)), p))) != 0;
+    if (remake) {
       for (uint32_t i = et; i < rows * kChunks; i += kTEpiThreads) {
         const uint32_t lr = r0 + i / kChunks, row = m0 + lr, n = n0 + i % kChunks * 4;
-        if (row >= ep.M || n >= ep.N) continue;
-        float4 acc = element(lr, i % kChunks);
-        bool scaled = false;
-        if constexpr (kSeg) scaled = Remade(ep, row, n, &acc);
-        EpilogueStoreRagged(ep, row, n, acc, scaled);
+        if (row < ep.M && n < ep.N) StoreRemade(ep, row, n, element(lr, i % kChunks));
+      }
+    } else if (ragged) {
+      for (uint32_t i = et; i < rows * kChunks; i += kTEpiThreads) {
+        const uint32_t lr = r0 + i / kChunks, row = m0 + lr, n = n0 + i % kChunks * 4;
+        if (row < ep.M && n < ep.N) EpilogueStoreRagged(ep, row, n, element(lr, i % kChunks), false);
       }
     } else if (IsPlainStore(ep)) {
       each(NoSide{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4&) {
@@ -860,6 +888,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         }
       };
       [[maybe_unused]] float sum[kSeg ? kEpiPasses : 1][kSeg ? kSlabCols : 1];
+      [[maybe_unused]] bool remake = false;   // some sum of this warp's is not finite
       if constexpr (kSeg) {
 #pragma unroll
         for (uint32_t p = 0; p < kEpiPasses; ++p)
@@ -881,6 +910,9 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
           hand_back();
         }
         if (!ok) break;
+#pragma unroll
+        for (uint32_t p = 0; p < kEpiPasses; ++p) remake = remake || !AllFinite(sum[p]);
+        remake = __any_sync(0xFFFFFFFFu, remake);
       } else {
         if (!await()) break;
       }
@@ -897,13 +929,14 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
                 make_uint4(ra[4 * q], ra[4 * q + 1], ra[4 * q + 2], ra[4 * q + 3]);
           __syncwarp();
           const uint32_t n = n0 + col_group * kColsPerEpiWarp + pass * kSlabCols + cl * 4;
-          if (ragged) {
-            for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr) {
-              float4 acc = *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
-              bool scaled = false;
-              if constexpr (kSeg) scaled = Remade(ep, row0 + rr, n, &acc);
-              EpilogueStoreRagged(ep, row0 + rr, n, acc, scaled);
-            }
+          auto staged = [&](uint32_t rr) {
+            return *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
+          };
+          if (kSeg && remake) {
+            for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr) StoreRemade(ep, row0 + rr, n, staged(rr));
+          } else if (ragged) {
+            for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr)
+              EpilogueStoreRagged(ep, row0 + rr, n, staged(rr), false);
           } else if (n < ep.N) {   // N % 4 == 0: a float4 is all in or all out
             float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
             if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
@@ -914,19 +947,16 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
               kscale = __ldg(reinterpret_cast<const float4*>(ep.shadow_k_scale + n));
   #pragma unroll 4
             for (uint32_t rr = sub; rr < rows; rr += kRowsPerInstr) {
-              float4 acc = *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
-              float4 by = scale;
-              if constexpr (kSeg)
-                if (Remade(ep, row0 + rr, n, &acc)) by = make_float4(1.f, 1.f, 1.f, 1.f);
+              const float4 acc = staged(rr);
               const size_t at = static_cast<size_t>(row0 + rr) * ep.N + n;
               if (plain_store)
-                EpilogueStorePlain(ep, at, acc, by);
+                EpilogueStorePlain(ep, at, acc, scale);
               else if (copy_only)
-                EpilogueStoreCopy(ep, at, acc, by);
+                EpilogueStoreCopy(ep, at, acc, scale);
               else if (bias_gelu_only)
-                EpilogueStoreBiasGelu(ep, at, acc, by, bias, kscale);
+                EpilogueStoreBiasGelu(ep, at, acc, scale, bias, kscale);
               else
-                EpilogueStore(ep, at, n, acc, by, bias, true, kscale);
+                EpilogueStore(ep, at, n, acc, scale, bias, true, kscale);
             }
           }
           __syncwarp();   // the slab is rewritten next
