@@ -115,6 +115,21 @@ CudaBackend::~CudaBackend() {
   if (own_stream_ && stream_) cudaStreamDestroy(stream_);
 }
 
+// False: no pinned memory to be had (downloads then go range by range).
+bool CudaBackend::EnsureFlushStaging(uint64_t bytes) {
+  if (bytes <= flush_capacity_) return true;
+  if (h_flush_) cudaFreeHost(h_flush_);   // (what was copied through it has been waited for)
+  h_flush_ = nullptr;
+  flush_capacity_ = 0;
+  if (cudaMallocHost(reinterpret_cast<void**>(&h_flush_), bytes) != cudaSuccess) {
+    cudaGetLastError();
+    h_flush_ = nullptr;
+    return false;
+  }
+  flush_capacity_ = bytes;
+  return true;
+}
+
 Status CudaBackend::Bind(uint8_t* arena, uint64_t arena_bytes, const uint8_t* rodata,
                          uint64_t rodata_bytes, uint64_t /*rodata_mapped_bytes*/) {
   if (!arena || arena_bytes == 0) return std::unexpected("cuda: bind: empty arena");
@@ -152,6 +167,7 @@ Status CudaBackend::Bind(uint8_t* arena, uint64_t arena_bytes, const uint8_t* ro
   d_rodata_ = static_cast<uint8_t*>(new_rodata);
   host_arena_ = arena;
   arena_bytes_ = arena_bytes;
+  if (coherence_ == Coherence::kStrict) (void)EnsureFlushStaging(std::min<uint64_t>(arena_bytes, kFlushStaging));
   rodata_bytes_ = rodata_bytes;
   counters_.h2d_bytes += arena_bytes + rodata_bytes;
   host_dirty_.clear();
@@ -1630,11 +1646,7 @@ Status CudaBackend::FlushWith(std::initializer_list<k::PublishItem> items, uint3
   if (strict) {
     for (const auto& [off, bytes] : device_dirty_) { lo = std::min(lo, off); hi = std::max(hi, off + bytes); }
     staged = hi - lo <= kFlushStaging;
-    if (staged && !h_flush_ && cudaMallocHost(reinterpret_cast<void**>(&h_flush_), kFlushStaging) != cudaSuccess) {
-      cudaGetLastError();   // no pinned memory to be had: range by range
-      h_flush_ = nullptr;
-      staged = false;
-    }
+    staged = staged && EnsureFlushStaging(hi - lo);
     if (staged) {
       if (auto r = Check(cudaMemcpyAsync(h_flush_, d_arena_ + lo, hi - lo, cudaMemcpyDeviceToHost, stream_),
                          "flush download"); !r)

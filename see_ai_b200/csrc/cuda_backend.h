@@ -243,7 +243,9 @@ class CudaBackend {
   bool scalars_valid_ = false;
   bool capturing_ = false;
   uint32_t* h_published_ = nullptr;  // pinned: the status words, then what a FlushWith asked for
-  uint8_t* h_flush_ = nullptr;       // pinned staging of a strict flush's downloads, from the first one on
+  uint8_t* h_flush_ = nullptr;       // pinned staging of a strict flush's downloads (from a strict Bind on)
+  uint64_t flush_capacity_ = 0;
+  bool EnsureFlushStaging(uint64_t bytes);
   static constexpr uint64_t kPublishedBytes = 4096, kFlushStaging = 2ull << 20;
 
   Coherence coherence_ = Coherence::kStrict;
