@@ -688,7 +688,7 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
 // or sixteen (dK/dV) take 750 or 990; the exponentials of 64 columns x 128 rows 512 cycles of the
 // exp pipe.  A step takes about 1250 and 1350 cycles, the second products' commit on its way round
 // the chain; one 128-thread CTA that did everything in turn took 4200, two to an SM.
-// Measured: forward + dQ + dK/dV of 8 x 2048 positions of 16 heads 1031 -> 677 us.  Two issuing
+// Measured: forward + dQ + dK/dV of 8 x 2048 positions of 16 heads 1024 -> 676 us (667 to 771 from run to run).  Two issuing
 // warps because one spent as long waiting and issuing as the pipe worked (dQ of that size: 233 us
 // with one, 202 with two, 178 with the element arithmetic in pairs).
 template <int D, bool kKV>
