@@ -318,54 +318,60 @@ __global__ void __launch_bounds__(kThreads) GemmLaneKernel(Params p) {
 
 // ---- merge: a run of deltas, each alpha A B from zero, in one launch -----------------------
 // delta [M, N] = 0 + (alpha A) B in the quad order, K = rank: what a kFill with zero followed by a kGemmAccNN leaves,
-// bit for bit, without the filled tensor's round trip through memory.  A block owns 32 rows x 256 columns of one
-// delta: four columns per thread with their K x 4 slice of B in registers, eight rows one after the other, A's rows
-// broadcast from shared memory.  Write-bound: 113 MB (48 deltas of 768 x 768, rank 16) in 28 us, against 48 x (2 + 4) us
-// and 96 launches before.  `nonfinite` (or null) counts the values that are not finite on their way out.
-constexpr int kMergeRows = 32;
+// bit for bit, without the filled tensor's round trip through memory.  A block owns 64 rows x 256 columns of one
+// delta: two columns per thread with their K x 2 slice of B in registers (asked for before A's rows are waited for),
+// 32 rows one after the other, A's rows broadcast from shared memory.  Bound by the f32 pipe: without fused
+// multiply-adds an output is 2 K operations, 25 us for the 113 MB (48 deltas of 768 x 768, rank 16) that take 17 us to
+// write.  Measured for those: 58.7 us with blocks of 32 rows and four columns a thread, whose B and A round trips lay
+// eight rows apart under sixteen warps to an SM; 42.5 so (0.86 instructions issued per cycle and scheduler); 45.8 with the operations as f32x2 pairs.
+// `nonfinite` (or null) counts the values that are not finite on their way out.
+constexpr int kMergeRows = 64;
 template <int K>
 __global__ void __launch_bounds__(kThreads) MergeDeltasKernel(const __grid_constant__ MergeTable table,
                                                               unsigned long long* __restrict__ nonfinite) {
   __shared__ __align__(16) float As[kMergeRows][K];
-  const MergeEntry e = table.entry[blockIdx.y];
+  const MergeEntry& e = table.entry[blockIdx.y];
   const int tiles_n = static_cast<int>((e.N + 255) / 256);
   const size_t m0 = static_cast<size_t>(blockIdx.x / tiles_n) * kMergeRows;
   if (m0 >= e.M) return;
-  const size_t n = static_cast<size_t>(blockIdx.x % tiles_n) * 256 + (threadIdx.x & 63) * 4;
+  const size_t n = static_cast<size_t>(blockIdx.x % tiles_n) * 256 + (threadIdx.x & 127) * 2;
   const size_t rows = e.M - m0 < kMergeRows ? e.M - m0 : kMergeRows;
+  float2 b[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    b[k] = n < e.N ? *reinterpret_cast<const float2*>(e.B + k * e.N + n) : make_float2(0.0f, 0.0f);   // N % 4 == 0
   for (size_t i = threadIdx.x; i < rows * K; i += kThreads) As[i / K][i % K] = e.alpha * e.A[m0 * K + i];
   __syncthreads();
-  unsigned long long bad = 0;
-  if (n < e.N) {   // N % 4 == 0
-    float4 b[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) b[k] = *reinterpret_cast<const float4*>(e.B + k * e.N + n);
-    for (size_t r = threadIdx.x >> 6; r < rows; r += 4) {
-      float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  unsigned bad = 0;
+  if (n < e.N) {
+    float zero = 0.0f;   // NaN once a value is not finite
+    const size_t step = 2 * static_cast<size_t>(e.N);
+    float* const c_first = e.C + (m0 + (threadIdx.x >> 7)) * e.N + n;
+    float* at = c_first;
+    const float* a_row = As[threadIdx.x >> 7];
+#pragma unroll 4
+    for (int left = (static_cast<int>(rows) + 1 - static_cast<int>(threadIdx.x >> 7)) / 2; left > 0; --left, at += step, a_row += 2 * K) {
+      float2 c = make_float2(0.0f, 0.0f);
 #pragma unroll
       for (int k = 0; k < K; k += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(&As[r][k]);
-        const float b0[4] = {b[k].x, b[k].y, b[k].z, b[k].w}, b1[4] = {b[k + 1].x, b[k + 1].y, b[k + 1].z, b[k + 1].w};
-        const float b2[4] = {b[k + 2].x, b[k + 2].y, b[k + 2].z, b[k + 2].w};
-        const float b3[4] = {b[k + 3].x, b[k + 3].y, b[k + 3].z, b[k + 3].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float t = a.x * b0[j];
-          t = t + a.y * b1[j];
-          t = t + a.z * b2[j];
-          t = t + a.w * b3[j];
-          c[j] = c[j] + t;
-        }
+        const float4 a = *reinterpret_cast<const float4*>(a_row + k);
+        float tx = a.x * b[k].x, ty = a.x * b[k].y;
+        tx = tx + a.y * b[k + 1].x; ty = ty + a.y * b[k + 1].y;
+        tx = tx + a.z * b[k + 2].x; ty = ty + a.z * b[k + 2].y;
+        tx = tx + a.w * b[k + 3].x; ty = ty + a.w * b[k + 3].y;
+        c.x = c.x + tx;
+        c.y = c.y + ty;
       }
-      *reinterpret_cast<float4*>(e.C + (m0 + r) * e.N + n) = make_float4(c[0], c[1], c[2], c[3]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bad += !isfinite(c[j]);
+      *reinterpret_cast<float2*>(at) = c;
+      zero = fmaf(c.x, 0.0f, zero);
+      zero = fmaf(c.y, 0.0f, zero);
     }
+    if (!(zero == 0.0f))   // count them, on what was written
+      for (const float* p = c_first; p < at; p += step) bad += !isfinite(p[0]) + !isfinite(p[1]);
   }
   if (!nonfinite) return;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xFFFFFFFFu, bad, o);
-  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(nonfinite, bad);
+  bad = __reduce_add_sync(0xFFFFFFFFu, bad);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(nonfinite, static_cast<unsigned long long>(bad));
 }
 
 // ---- both orders, few outputs --------------------------------------------------------------
