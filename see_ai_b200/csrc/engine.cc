@@ -287,7 +287,6 @@ Status UpdateEngine::LoadFromMemory(const uint8_t* plan, uint64_t size) {
       if (ins.in[2] == h.loss_ref && ins.out[0] == h.batch) {
         eval_tail_ = {ins.opcode == kSoftmaxXEntFwd ? EvalTail::kXent : EvalTail::kXentMasked, ins.in[3],
                       ins.in[1], ins.out[1]};
-        terms = std::max<uint64_t>(terms, h.batch);
       }
     } else if (ins.opcode == kMseFwd && ins.in[2] == h.loss_ref && h.batch > 0 && ins.out[0] % h.batch == 0) {
       eval_tail_ = {EvalTail::kMse, ins.in[0], ins.in[1], ins.out[0] / h.batch};
@@ -578,14 +577,15 @@ Status UpdateEngine::Evaluate(EvalResult* out, uint64_t real_rows) {
                               eval_probs_ref_ != kNullRef && eval_cols_ > 0 && eval_rows_ >= header_.batch;
   const int32_t* label_slot = header_.label_ref == kNullRef
                                   ? nullptr : reinterpret_cast<const int32_t*>(at(header_.label_ref));
-  if (track_accuracy)
-    k::ArgmaxTally(reinterpret_cast<const float*>(at(eval_probs_ref_)), label_slot, real, eval_cols_, d_tally_, s);
+  const bool xent = eval_tail_.kind == EvalTail::kXent || eval_tail_.kind == EvalTail::kXentMasked;
+  const float* arg_probs = track_accuracy ? reinterpret_cast<const float*>(at(eval_probs_ref_)) : nullptr;
+  if (arg_probs && !xent) k::ArgmaxTally(arg_probs, label_slot, real, eval_cols_, d_tally_, s);
   bool row_loss = true;
   switch (eval_tail_.kind) {
     case EvalTail::kXent: case EvalTail::kXentMasked:
       if (!label_slot) return std::unexpected("engine: a cross-entropy eval tail needs the label slot");
-      k::XentRealRowLoss(reinterpret_cast<const float*>(at(eval_tail_.a)), label_slot, real, eval_tail_.width,
-                         d_eval_terms_, d_eval_out_, d_tally_, s);
+      k::XentEvalTail(reinterpret_cast<const float*>(at(eval_tail_.a)), eval_tail_.width, arg_probs, eval_cols_,
+                      label_slot, real, d_eval_out_, d_tally_, s);
       break;
     case EvalTail::kMse:
       k::MseRealRowLoss(reinterpret_cast<const float*>(at(eval_tail_.a)),

@@ -112,36 +112,39 @@ __global__ void XEntRowsKernel(const float* __restrict__ logits, const int32_t* 
   }
 }
 
-// The same row softmax for wide rows (4096 <= C <= 32768, C % 4 == 0): one
-// 1024-thread block per row with the whole row in registers (eight 16-byte
-// vectors per thread), so the logits are read from HBM once and the
-// probabilities written once.  The next row is copied into shared memory
-// asynchronously (cp.async) while the current one is reduced, each thread
-// fetching exactly the chunks it will later read itself, so no barrier guards
-// the buffer.  Same expressions per element as RowSoftmaxBlock; the row sum is
-// folded as thread partials (ascending index), warp shuffles, then warps in order.
-constexpr int kWideThreads = 1024;
+// The same row softmax for wide rows (4096 <= C <= 32768, C % 4 == 0): a row lies whole in the registers of a block
+// (up to eight 16-byte vectors per thread), so the logits are read from HBM once and the probabilities written once.
+// The next row is copied into shared memory asynchronously (cp.async) while the current one is reduced, each thread
+// fetching exactly the chunks it will later read itself, so no barrier guards the buffer.  Same expressions per
+// element as RowSoftmaxBlock; the row sum is folded as thread partials (ascending index), warp shuffles, then warps in
+// order.
+// A row's two reductions are a chain of barriers that moves no bytes, so what counts is how many rows an SM has in
+// hand at once: four 256-thread blocks up to 8192 columns, two of 512 up to 16384, one of 1024 above.  (4096 rows of
+// 4096 columns: 82 us with 1024 threads to a row, 23 with 256.  The two halves of a 32000-wide row in a cluster of two,
+// with a second row resident on either SM, took 1770 us for 32768 rows; one block to a row and SM 1600.)
 constexpr int kWideVecs = 8;
+constexpr size_t kWideMaxColumns = 32768;
+constexpr size_t WideColumns(int threads) { return static_cast<size_t>(threads) * kWideVecs * 4; }
 
 __device__ __forceinline__ void CpAsync16(void* smem, const void* gmem) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
 
-__global__ void __launch_bounds__(kWideThreads, 1)
+template <int kThreads, int kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks)
 XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__ labels,
                    float* __restrict__ probs, double* __restrict__ row_loss, size_t N, size_t C,
                    bool masked, Shadow sh, float bwd_scale, bool store_probs) {
   extern __shared__ __align__(16) float4 row_smem[];
   __shared__ float smem_f[32];
-  __shared__ float label_prob;
   const int C4 = static_cast<int>(C / 4);
   const int tid = threadIdx.x;
   auto prefetch = [&](size_t n) {
     const float4* lrow = reinterpret_cast<const float4*>(logits + n * C);
 #pragma unroll
     for (int i = 0; i < kWideVecs; ++i) {
-      const int c4 = i * kWideThreads + tid;
+      const int c4 = i * kThreads + tid;
       if (c4 < C4) CpAsync16(&row_smem[c4], &lrow[c4]);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -153,15 +156,16 @@ XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < kWideVecs; ++i) {
-      const int c4 = i * kWideThreads + tid;
+      const int c4 = i * kThreads + tid;
       if (c4 < C4) {
         x[i] = row_smem[c4];
         mx = fmaxf(fmaxf(mx, x[i].x), fmaxf(x[i].y, fmaxf(x[i].z, x[i].w)));
       }
     }
     if (n + gridDim.x < N) prefetch(n + gridDim.x);
-    mx = BlockReduce<float>(mx, -INFINITY, smem_f, WarpMax,
-                            [](float a, float b) { return fmaxf(a, b); });
+    auto max2 = [](float a, float b) { return fmaxf(a, b); };
+    auto add2 = [](float a, float b) { return a + b; };
+    mx = BlockReduce<float>(mx, -INFINITY, smem_f, WarpMax, max2);
     // e^{x - mx} = 2^{x log2 e - mx log2 e} on the hardware exponential: one FMA and
     // one MUFU per element (libm expf is about twenty instructions, and a
     // vocabulary-wide row is instruction-bound with it).  Relative error about 1e-6
@@ -171,25 +175,27 @@ XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__
     float sum = 0.0f;
 #pragma unroll
     for (int i = 0; i < kWideVecs; ++i) {
-      if (i * kWideThreads + tid < C4) {
+      if (i * kThreads + tid < C4) {
         x[i].x = Ex2Approx(__fmaf_rn(x[i].x, kLog2E, shift)); sum += x[i].x;
         x[i].y = Ex2Approx(__fmaf_rn(x[i].y, kLog2E, shift)); sum += x[i].y;
         x[i].z = Ex2Approx(__fmaf_rn(x[i].z, kLog2E, shift)); sum += x[i].z;
         x[i].w = Ex2Approx(__fmaf_rn(x[i].w, kLog2E, shift)); sum += x[i].w;
       }
     }
-    sum = BlockReduce<float>(sum, 0.0f, smem_f, WarpSumF, [](float a, float b) { return a + b; });
+    sum = BlockReduce<float>(sum, 0.0f, smem_f, WarpSumF, add2);
     const float inv_sum = 1.0f / sum;
     float4* prow = reinterpret_cast<float4*>(probs + n * C);
     const int32_t lab = labels[n];
-    const int lab4 = lab >= 0 && static_cast<size_t>(lab) < C ? lab >> 2 : -1;
+    const bool valid = lab >= 0 && static_cast<size_t>(lab) < C;
+    const int lab4 = valid ? lab >> 2 : -1;
+    if (!valid && tid == 0) row_loss[n] = masked && lab < 0 ? 0.0 : NAN;
 #pragma unroll
     for (int i = 0; i < kWideVecs; ++i) {
-      const int c4 = i * kWideThreads + tid;
+      const int c4 = i * kThreads + tid;
       if (c4 < C4) {
         const float4 p = make_float4(x[i].x * inv_sum, x[i].y * inv_sum, x[i].z * inv_sum, x[i].w * inv_sum);
         if (store_probs) prow[c4] = p;
-        if (c4 == lab4) label_prob = (lab & 3) == 0 ? p.x : (lab & 3) == 1 ? p.y : (lab & 3) == 2 ? p.z : p.w;
+        if (c4 == lab4) row_loss[n] = NegLogSafe((lab & 3) == 0 ? p.x : (lab & 3) == 1 ? p.y : (lab & 3) == 2 ? p.z : p.w);
         if (sh.dst) {
           // The backward instruction's arithmetic on the value it would have read back.
           float4 v = make_float4(bwd_scale * p.x, bwd_scale * p.y, bwd_scale * p.z, bwd_scale * p.w);
@@ -205,15 +211,28 @@ XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__
         }
       }
     }
-    __syncthreads();  // label_prob is visible to thread 0 below; and the smem buffers are reused
-    if (tid == 0) {
-      double v;
-      if (masked && lab < 0) v = 0.0;
-      else if (lab < 0 || static_cast<size_t>(lab) >= C) v = NAN;
-      else v = NegLogSafe(label_prob);
-      row_loss[n] = v;
-    }
   }
+}
+
+template <int kThreads, int kMinBlocks>
+void LaunchXEntRowsWide(const float* logits, const int32_t* labels, float* probs, double* row_loss, size_t N, size_t C,
+                        bool masked, const Shadow& sh, float bwd_scale, bool store_probs, cudaStream_t s) {
+  auto kernel = XEntRowsWideKernel<kThreads, kMinBlocks>;
+  // Raising a kernel's dynamic shared-memory limit is a per-device setting of
+  // the function, not an allocation; done on first use per device.
+  // (Atomic flags: handle-free callers may make their first calls from two host
+  // threads at once; setting the attribute twice is harmless, a torn flag is not.)
+  static std::atomic<bool> configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kThreads * kWideVecs * 16);
+    if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+  }
+  // One round of resident blocks walks the rows, several apiece: their prefetches reach across rows.
+  const size_t blocks = 148 * kMinBlocks;
+  kernel<<<static_cast<unsigned>(N < blocks ? N : blocks), kThreads, C * sizeof(float), s>>>(
+      logits, labels, probs, row_loss, N, C, masked, sh, bwd_scale, store_probs);
 }
 
 // Folds row losses with the reference's chunk geometry: thread t owns chunk t
@@ -439,23 +458,10 @@ bool SoftmaxXEntFwd(bool masked, const float* logits, const int32_t* labels, flo
                     unsigned long long* count_scratch, cudaStream_t s, const XEntFusedBwd* fused_bwd) {
   if (N == 0) return false;
   bool fused = false;
-  const bool wide = C >= 4096 && C <= static_cast<size_t>(4 * kWideThreads * kWideVecs) &&
+  const bool wide = C >= 4096 && C <= kWideMaxColumns &&
                     (C & 3) == 0 && ((reinterpret_cast<uintptr_t>(logits) |
                                       reinterpret_cast<uintptr_t>(probs)) & 15) == 0;
   if (wide) {
-    // Raising a kernel's dynamic shared-memory limit is a per-device setting of
-    // the function, not an allocation; done on first use per device.
-    // (Atomic flags: handle-free callers may make their first calls from two host
-    // threads at once; setting the attribute twice is harmless, a torn flag is not.)
-    static std::atomic<bool> configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !configured[dev].load(std::memory_order_acquire)) {
-      cudaFuncSetAttribute(XEntRowsWideKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           4 * kWideThreads * kWideVecs * static_cast<int>(sizeof(float)));
-      configured[dev].store(true, std::memory_order_release);
-    }
-    const unsigned blocks = static_cast<unsigned>(N < 148 * 4 ? N : 148 * 4);
     Shadow sh{};
     float bwd_scale = 0.0f;
     bool store_probs = true;
@@ -465,8 +471,10 @@ bool SoftmaxXEntFwd(bool masked, const float* logits, const int32_t* labels, flo
       store_probs = fused_bwd->store_probs;
       fused = true;
     }
-    XEntRowsWideKernel<<<blocks, kWideThreads, C * sizeof(float), s>>>(logits, labels, probs, row_scratch, N, C,
-                                                                       masked, sh, bwd_scale, store_probs);
+    auto launch = [&](auto run) { run(logits, labels, probs, row_scratch, N, C, masked, sh, bwd_scale, store_probs, s); };
+    if (C <= WideColumns(256)) launch(LaunchXEntRowsWide<256, 4>);
+    else if (C <= WideColumns(512)) launch(LaunchXEntRowsWide<512, 2>);
+    else launch(LaunchXEntRowsWide<1024, 1>);
   } else {
     const int threads = C >= 1024 ? 256 : (C >= 128 ? 128 : 32);
     const unsigned blocks = static_cast<unsigned>(N < 148 * 16 ? N : 148 * 16);

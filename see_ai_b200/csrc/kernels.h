@@ -200,11 +200,12 @@ void ArgmaxTally(const float* probs, const int32_t* labels, size_t N, size_t C,
 void CountNonFinite(const float* x, size_t n, unsigned long long* tally, cudaStream_t s);
 // The real-row loss of the batch just evaluated: out[0] = the sum over the first
 // real_rows rows of each row's loss (-log max(p[label], 1e-12), NaN kept; rows
-// with label < 0 skipped), added in row order in double; tally[3] = the rows it
-// is over.  `terms` holds real_rows doubles.  The MSE form sums the squared
-// differences of real_rows * width elements in element order and divides by width.
-void XentRealRowLoss(const float* probs, const int32_t* labels, size_t real_rows, size_t width,
-                     double* terms, double* out, unsigned long long* tally, cudaStream_t s);
+// with label < 0 skipped), added in row order in double; tally[3] += the rows it
+// is over.  With arg_probs (rows of arg_cols) the same launch does ArgmaxTally over them.
+// The MSE form sums the squared differences of real_rows * width elements in element
+// order, in `terms` (as many doubles), and divides by width.
+void XentEvalTail(const float* probs, size_t width, const float* arg_probs, size_t arg_cols, const int32_t* labels,
+                  size_t real_rows, double* out, unsigned long long* tally, cudaStream_t s);
 void MseRealRowLoss(const float* pred, const float* target, size_t real_rows, size_t width, double* terms,
                     double* out, unsigned long long* tally, cudaStream_t s);
 // Symmetric per-column int8 quantisation of W [K, N] with the compiler's own
