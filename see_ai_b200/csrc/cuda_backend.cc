@@ -1781,7 +1781,7 @@ Status CudaBackend::Execute(const Instruction& ins, const StepParams& params) {
   }
 
   if (range_index_ == 0 && !lora_weights_.empty()) {   // every adapter matrix of the range, cut once
-    k::LoraSplitWeights(d_lora_table_, static_cast<int>(lora_weights_.size()), lora_max_n_, stream_);
+    k::LoraSplitWeights(d_lora_table_, static_cast<int>(lora_weights_.size()), lora_max_n_, lora_max_kx_, stream_);
     ++counters_.kernel_launches;
   }
   const uint64_t fused_before = counters_.fused_dispatches;

@@ -232,7 +232,7 @@ struct LoraWeight {
   uint32_t by_column;
 };
 // Every entry of a device-resident table in one launch.
-void LoraSplitWeights(const LoraWeight* table, int count, uint32_t max_n_out, cudaStream_t s);
+void LoraSplitWeights(const LoraWeight* table, int count, uint32_t max_n_out, uint32_t max_kx, cudaStream_t s);
 
 // ---- the activation-streaming adapter products on the tensor cores (k_lora_mma.cu) -----
 // t = alpha x A for x [M, K], A [K, r]; 3xTF32 (f32-class accuracy, not the CPU's
