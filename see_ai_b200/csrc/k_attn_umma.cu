@@ -717,7 +717,8 @@ struct BwdCtl {
 static_assert(sizeof(BwdCtl) <= 512, "control block");
 
 // A bounded wait that also ends when another role of the CTA has given up.
-__device__ __forceinline__ bool RoleWait(BwdCtl* ctl, uint64_t* bar, uint32_t parity) {
+template <typename Control>
+__device__ __forceinline__ bool RoleWait(Control* ctl, uint64_t* bar, uint32_t parity) {
   const uint32_t addr = SmemAddr(bar);
   for (uint32_t it = 0; it < kWaitLimit; ++it) {
     uint32_t done;
@@ -737,7 +738,8 @@ __device__ __forceinline__ bool RoleWait(BwdCtl* ctl, uint64_t* bar, uint32_t pa
 // The same by a whole warp, with one answer: when another role gives up, lanes that still saw their barrier complete
 // leave with the others instead of issuing a warp-wide tensor-memory access alone (and what follows stays warp-uniform
 // for the compiler).
-__device__ __forceinline__ bool WarpWait(BwdCtl* ctl, uint64_t* bar, uint32_t parity) {
+template <typename Control>
+__device__ __forceinline__ bool WarpWait(Control* ctl, uint64_t* bar, uint32_t parity) {
   return __all_sync(0xFFFFFFFFu, RoleWait(ctl, bar, parity));
 }
 
@@ -1049,6 +1051,334 @@ AttnBwdKernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   }
 }
 
+// ---- forward on dedicated warps ------------------------------------------------------------
+// From two query tiles a sequence on.  One persistent CTA per SM works two neighbouring query tiles of a (sequence,
+// head) at once, which share the keys' and values' steps of 64: a load warp, an issuing warp per tile, four warps per
+// tile that turn scores into probabilities (a row per thread) and four that store finished tiles.  A tile has two
+// score buffers, so the next step's scores are formed under this step's exponentials; P goes back to tensor memory as
+// the second product's operand, and O, double-buffered for d = 64, leaves under the next tile's steps.  What is left
+// is the exponentials: 8192 of them per step and tile on 16 lanes, 512 cycles, which the two tiles' warps keep busy
+// in turn, where the one-CTA-per-tile kernel above spent 3100 cycles a step with four CTAs to an SM.  Measured: 8 x 2048
+// positions of 16 heads 162 -> 115 us, 64 x 512 of 12 106 -> 83, 8 x 512 of 12 20.7 -> 15.4, 3 x 200 of 8 10.1 -> 9.7.  The row's
+// reference exponent, its lazy rescaling and the statistics are that kernel's.
+template <int D>
+struct FwdShape {
+  static constexpr uint32_t kQ = 128 * D * 2;                // one query tile
+  static constexpr uint32_t kStep = 64 * D * 2;              // one step of keys, or of values
+  static constexpr uint32_t kQBufs = D == 64 ? 2 : 1;        // of two tiles each
+  static constexpr uint32_t kStages = D == 64 ? 5 : 3;
+  static constexpr uint32_t kOutBufs = D == 64 ? 2 : 1;
+  static constexpr uint32_t kOutCol = 128;                   // of a tile's 256 columns: after two score buffers
+  static constexpr uint32_t kSlab = 32 * 64 * 4;
+  static constexpr size_t kSmem = kQBufs * 2 * kQ + kStages * 2 * kStep + 4 * kSlab + 2 * 2 * 128 * 4 + 512 + 1024;
+};
+struct FwdCtl {
+  uint64_t q_full[2], q_empty[2];
+  uint64_t full[5], empty[5];
+  uint64_t s_full[2][2], p_full[2][2], pv_done[2];   // [tile of the pair] ([score buffer])
+  uint64_t out_full[2][2], out_empty[2][2], stat_full[2][2];
+  uint32_t tmem_base;
+  volatile uint32_t failed;
+};
+static_assert(sizeof(FwdCtl) <= 512, "control block");
+
+// A CTA's pairs of tiles, heaviest first, dealt out in rounds that alternate direction.
+struct FwdPair {
+  uint32_t first_tile, bh, steps0, steps1, stream;
+  __device__ __forceinline__ uint32_t Steps(uint32_t tile) const { return tile == 0 ? steps0 : steps1; }
+};
+__device__ __forceinline__ bool FwdPairAt(uint32_t round, uint32_t S, uint32_t BH, FwdPair* u) {
+  const uint32_t n_t = (S + kTile - 1) / kTile, all_h = (S + kHalf - 1) / kHalf, n_u = (n_t + 1) / 2;
+  const uint32_t at = round * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+  if (at >= n_u * BH) return false;   // only in the last round
+  const uint32_t rank = at / BH;
+  u->bh = at - rank * BH;
+  u->first_tile = 2 * (n_u - 1 - rank);
+  auto steps = [&](uint32_t tile) { return tile >= n_t ? 0u : (2 * (tile + 1) < all_h ? 2 * (tile + 1) : all_h); };
+  u->steps0 = steps(u->first_tile);
+  u->steps1 = steps(u->first_tile + 1);
+  u->stream = u->steps1 > u->steps0 ? u->steps1 : u->steps0;
+  return true;
+}
+
+__device__ __forceinline__ float Max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+constexpr uint32_t kFwdThreads = 15 * 32;
+
+template <int D>
+__global__ void __launch_bounds__(kFwdThreads, 1)
+AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                  const __grid_constant__ CUtensorMap map_v, AttnUmmaArgs a) {
+  using Sh = FwdShape<D>;
+  extern __shared__ uint8_t smem_raw[];
+  FwdCtl* ctl = reinterpret_cast<FwdCtl*>(smem_raw);
+  uint8_t* q_s = AlignSmem(smem_raw + 512);
+  uint8_t* ring_s = q_s + Sh::kQBufs * 2 * Sh::kQ;
+  uint8_t* slab_s = ring_s + Sh::kStages * 2 * Sh::kStep;
+  float* stat_s = reinterpret_cast<float*>(slab_s + 4 * Sh::kSlab);   // [tile of the pair][output buffer][128]: 1 / sum
+
+  const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t BH = a.B * a.H;
+
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      MbarInit(&ctl->q_full[i], 1); MbarInit(&ctl->q_empty[i], 2); MbarInit(&ctl->pv_done[i], 1);
+      for (int j = 0; j < 2; ++j) {
+        MbarInit(&ctl->s_full[i][j], 1); MbarInit(&ctl->p_full[i][j], 4);
+        MbarInit(&ctl->out_full[i][j], 1); MbarInit(&ctl->out_empty[i][j], 4); MbarInit(&ctl->stat_full[i][j], 4);
+      }
+    }
+    for (int i = 0; i < 5; ++i) { MbarInit(&ctl->full[i], 1); MbarInit(&ctl->empty[i], 2); }
+    ctl->failed = 0;
+    MbarInitFence();
+  }
+  if (warp == 12) TmemAlloc(&ctl->tmem_base, 512);
+  TcFenceBefore();
+  __syncthreads();
+  TcFenceAfter();
+  constexpr uint32_t tmem = 0;   // all 512 columns are this CTA's: 256 per tile of the pair
+
+  if (warp == 14) {
+    // ---- loads ----
+    if (lane == 0) {
+      uint32_t g = 0, i = 0;
+      bool ok = true;
+      FwdPair u;
+      for (; ok && FwdPairAt(i, a.S, BH, &u); ++i) {
+        const uint32_t b = u.bh / a.H, h = u.bh - b * a.H;
+        const uint32_t qb = i % Sh::kQBufs;
+        if (!(ok = RoleWait(ctl, &ctl->q_empty[qb], ((i / Sh::kQBufs) & 1) ^ 1))) break;
+        uint8_t* q = q_s + qb * 2 * Sh::kQ;
+        MbarExpectTx(&ctl->q_full[qb], (u.steps1 ? 2 : 1) * Sh::kQ);
+        LoadRows<D, 128>(q, &map_q, &ctl->q_full[qb], u.first_tile * kTile, h, b);
+        if (u.steps1) LoadRows<D, 128>(q + Sh::kQ, &map_q, &ctl->q_full[qb], (u.first_tile + 1) * kTile, h, b);
+        for (uint32_t t = 0; t < u.stream; ++t, ++g) {
+          const uint32_t s = g % Sh::kStages;
+          if (!(ok = RoleWait(ctl, &ctl->empty[s], ((g / Sh::kStages) & 1) ^ 1))) break;
+          uint8_t* st = ring_s + s * 2 * Sh::kStep;
+          MbarExpectTx(&ctl->full[s], 2 * Sh::kStep);
+          LoadRows<D, 64>(st, &map_k, &ctl->full[s], t * kHalf, h, b);
+          LoadRows<D, 64>(st + Sh::kStep, &map_v, &ctl->full[s], t * kHalf, h, b);
+        }
+      }
+      // Every slot's last release has arrived before the CTA may end.
+      for (uint32_t k = 0; ok && k < Sh::kStages; ++k, ++g)
+        ok = RoleWait(ctl, &ctl->empty[g % Sh::kStages], ((g / Sh::kStages) & 1) ^ 1);
+      for (uint32_t k = 0; ok && k < Sh::kQBufs; ++k, ++i)
+        ok = RoleWait(ctl, &ctl->q_empty[i % Sh::kQBufs], ((i / Sh::kQBufs) & 1) ^ 1);
+    }
+  } else if (warp >= 12) {
+    // ---- products of one tile of the pair (the whole warp walks and waits; one elected lane issues) ----
+    const uint32_t tile = warp - 12;
+    const uint32_t base = tmem + tile * 256, idesc = MakeInstrDesc(128, D) | kInstrDescBMnMajor;
+    FwdPair u;
+    uint32_t g = 0, n = 0, j = 0;   // steps of the stream, of this tile's, finished tiles
+    bool ok = true;
+    for (uint32_t i = 0; ok && FwdPairAt(i, a.S, BH, &u); ++i) {
+      const uint32_t qb = i % Sh::kQBufs, steps = u.Steps(tile), ob = j % Sh::kOutBufs;
+      if (!(ok = WarpWait(ctl, &ctl->q_full[qb], (i / Sh::kQBufs) & 1))) break;
+      const uint8_t* q = q_s + qb * 2 * Sh::kQ + tile * Sh::kQ;
+      // The scores of step t (this tile's step m) into their buffer, whose last reader is P V two steps ago.  (A new
+      // tile's first step waits for the whole of the tile before: a parity tells one phase from the next only.)
+      auto scores = [&](uint32_t t, uint32_t m) {
+        const uint32_t at = g + t, s = at % Sh::kStages;
+        if (!WarpWait(ctl, &ctl->full[s], (at / Sh::kStages) & 1)) return false;
+        const uint32_t back = t == 0 ? 1 : 2;
+        if (m >= back && !WarpWait(ctl, &ctl->pv_done[tile], (m - back) & 1)) return false;
+        TcFenceAfter();
+        if (ElectOne()) {
+          MmaRowRow<D, 64>(base + (m & 1) * 64, q, ring_s + s * 2 * Sh::kStep);
+          UmmaCommit(&ctl->s_full[tile][m & 1]);
+          if (t + 1 == steps) UmmaCommit(&ctl->q_empty[qb]);
+        }
+        __syncwarp();
+        return true;
+      };
+      if (steps == 0) {
+        if (lane == 0) MbarArrive(&ctl->q_empty[qb]);
+      } else {
+        if (!(ok = scores(0, n))) break;
+        if (!(ok = WarpWait(ctl, &ctl->out_empty[tile][ob], ((j / Sh::kOutBufs) & 1) ^ 1))) break;
+        for (uint32_t t = 0; t < steps; ++t, ++n) {
+          if (t + 1 < steps && !(ok = scores(t + 1, n + 1))) break;
+          if (!(ok = WarpWait(ctl, &ctl->p_full[tile][n & 1], (n >> 1) & 1))) break;
+          TcFenceAfter();
+          const uint32_t s = (g + t) % Sh::kStages, v = SmemAddr(ring_s + s * 2 * Sh::kStep + Sh::kStep);
+          if (ElectOne()) {
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k)
+              UmmaBf16TmemA(base + Sh::kOutCol + ob * D, base + (n & 1) * 64 + k * 8, MakeSmemDescMn(v + k * 2048, 64 * 128),
+                            idesc, (t | k) != 0 ? 1u : 0u);
+            UmmaCommit(&ctl->pv_done[tile]);
+            UmmaCommit(&ctl->empty[s]);
+            if (t + 1 == steps) UmmaCommit(&ctl->out_full[tile][ob]);
+          }
+          __syncwarp();
+        }
+        if (!ok) break;
+        ++j;
+      }
+      for (uint32_t t = steps; t < u.stream; ++t) {   // steps that only the other tile takes
+        const uint32_t s = (g + t) % Sh::kStages;
+        if (!(ok = WarpWait(ctl, &ctl->full[s], ((g + t) / Sh::kStages) & 1))) break;
+        if (lane == 0) MbarArrive(&ctl->empty[s]);
+      }
+      g += u.stream;
+    }
+  } else if (warp < 8) {
+    // ---- probabilities ----
+    const uint32_t tile = warp >> 2, quarter = warp & 3, r_in = quarter * 32 + lane;
+    const uint32_t t_base = tmem + tile * 256 + ((quarter * 32) << 16);
+    const float c1 = a.inv_sqrt_d * kLog2e;
+    FwdPair u;
+    uint32_t n = 0, j = 0;
+    bool ok = true;
+    for (uint32_t i = 0; ok && FwdPairAt(i, a.S, BH, &u); ++i) {
+      const uint32_t steps = u.Steps(tile), ob = j % Sh::kOutBufs;
+      if (steps == 0) continue;
+      const uint32_t row0 = (u.first_tile + tile) * kTile, row = row0 + r_in;
+      const uint32_t t_o = t_base + Sh::kOutCol + ob * D;
+      float raw_max = -INFINITY;   // the row's true score maximum so far
+      float ref = -INFINITY;       // the exponent (log2 units) its p, sum and O are relative to
+      F2 sum = Pair(0.0f, 0.0f);
+      for (uint32_t t = 0; t < steps; ++t, ++n) {
+        if (!(ok = WarpWait(ctl, &ctl->s_full[tile][n & 1], (n >> 1) & 1))) break;
+        TcFenceAfter();
+        const uint32_t t_s = t_base + (n & 1) * 64, key0 = t * kHalf;
+        uint32_t lo[32], hi[32];
+        TmemLoad32(t_s, lo);
+        TmemLoad32(t_s + 32, hi);
+        TmemWaitLd();
+        if (key0 + kHalf > row0) {   // some keys of this step lie above the diagonal
+          constexpr uint32_t kMinusInf = 0xFF800000u;
+#pragma unroll
+          for (uint32_t e = 0; e < 32; ++e) {
+            if (key0 + e > row) lo[e] = kMinusInf;
+            if (key0 + 32 + e > row) hi[e] = kMinusInf;
+          }
+        }
+        float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          m[0] = Max3(m[0], __uint_as_float(lo[e]), __uint_as_float(lo[e + 1]));
+          m[1] = Max3(m[1], __uint_as_float(lo[e + 2]), __uint_as_float(lo[e + 3]));
+          m[2] = Max3(m[2], __uint_as_float(hi[e]), __uint_as_float(hi[e + 1]));
+          m[3] = Max3(m[3], __uint_as_float(hi[e + 2]), __uint_as_float(hi[e + 3]));
+        }
+        const float step_max = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+        raw_max = fmaxf(raw_max, step_max);
+        const float step_ref = step_max * c1;
+        const bool moves = step_ref > ref + kRescaleSlack;   // always at a row's first live key (ref = -inf)
+        float alpha = 1.0f;
+        if (moves) {
+          alpha = Exp2Approx(ref - step_ref);                // 0 the first time
+          sum = Mul2(sum, Pair(alpha, alpha));
+          ref = step_ref;
+        }
+        if (t > 0 && __any_sync(0xFFFFFFFFu, moves)) {       // the warp's rows rescale their O lanes together
+          if (!(ok = WarpWait(ctl, &ctl->pv_done[tile], (n - 1) & 1))) break;
+          TcFenceAfter();
+#pragma unroll 1
+          for (uint32_t c0 = 0; c0 < D; c0 += 16) {
+            uint32_t o[16];
+            TmemLoad16(t_o + c0, o);
+            TmemWaitLd();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+            TmemStore16(t_o + c0, o);
+          }
+          TmemWaitSt();
+        }
+        // p = 2^(s c1 - ref), packed over the scores' own registers.
+        const F2 scale = Pair(c1, c1), shift = Pair(-ref, -ref);
+        auto half = [&](uint32_t (&x)[32]) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            const F2 y = Fma2(Pair(__uint_as_float(x[e]), __uint_as_float(x[e + 1])), scale, shift);
+            const float p0 = Exp2Approx(Lo(y)), p1 = Exp2Approx(Hi(y));
+            sum = Add2(sum, Pair(p0, p1));
+            x[e / 2] = PackBf16x2(p0, p1);
+          }
+        };
+        half(lo);
+        half(hi);
+        uint32_t w[32];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) { w[e] = lo[e]; w[16 + e] = hi[e]; }
+        TmemStore32(t_s, w);
+        TmemWaitSt();
+        TcFenceBefore();
+        __syncwarp();
+        if (lane == 0) MbarArrive(&ctl->p_full[tile][n & 1]);
+      }
+      if (!ok) break;
+      const float l = Lo(sum) + Hi(sum);
+      if (row < a.S) {
+        // The stats row speaks of the true maximum: the sum relative to it is l 2^(ref - max c).
+        const float m = raw_max * a.inv_sqrt_d;
+        const float inv_l_at_max = 1.0f / (l * Exp2Approx(ref - raw_max * c1));
+        *reinterpret_cast<float4*>(a.stats + (static_cast<size_t>(u.bh) * a.S + row) * kAttnStatsWidth) =
+            make_float4(m, inv_l_at_max, 0.0f, 0.0f);
+      }
+      if (!(ok = WarpWait(ctl, &ctl->out_empty[tile][ob], ((j / Sh::kOutBufs) & 1) ^ 1))) break;
+      stat_s[(tile * 2 + ob) * 128 + r_in] = 1.0f / l;
+      __syncwarp();
+      if (lane == 0) MbarArrive(&ctl->stat_full[tile][ob]);
+      ++j;
+    }
+  } else {
+    // ---- outputs ----
+    const uint32_t quarter = warp & 3, r_in = quarter * 32 + lane;
+    float* slab = reinterpret_cast<float*>(slab_s + quarter * Sh::kSlab);
+    const size_t HD = static_cast<size_t>(a.H) * D;
+    uint32_t done0 = 0, done1 = 0;   // finished tiles of either place
+    bool ok = true;
+    FwdPair u;
+    for (uint32_t i = 0; ok && FwdPairAt(i, a.S, BH, &u); ++i) {
+      const uint32_t b = u.bh / a.H, h = u.bh - b * a.H;
+#pragma unroll
+      for (uint32_t tile = 0; tile < 2; ++tile) {
+        if (!ok || u.Steps(tile) == 0) continue;
+        uint32_t& j = tile == 0 ? done0 : done1;
+        const uint32_t ob = j % Sh::kOutBufs, parity = (j / Sh::kOutBufs) & 1;
+        if (!(ok = WarpWait(ctl, &ctl->out_full[tile][ob], parity) && WarpWait(ctl, &ctl->stat_full[tile][ob], parity))) break;
+        TcFenceAfter();
+        const float inv_l = stat_s[(tile * 2 + ob) * 128 + r_in];
+        const uint32_t row0w = (u.first_tile + tile) * kTile + quarter * 32;
+        const uint32_t rows_live = row0w < a.S ? (a.S - row0w < 32 ? a.S - row0w : 32) : 0;
+        const size_t flat0 = (static_cast<size_t>(b) * a.S + row0w) * HD + static_cast<size_t>(h) * D;
+        const uint32_t t_out = tmem + tile * 256 + ((quarter * 32) << 16) + Sh::kOutCol + ob * D;
+#pragma unroll 1
+        for (uint32_t c = 0; c < D; c += 64) {
+          StoreOutRows<64>(t_out + c, slab, lane, inv_l, a.out + flat0 + c, HD, rows_live, a.shadow, flat0 + c, h * D + c,
+                           a.keep);
+          __syncwarp();   // the staging slab is reused
+        }
+        TcFenceBefore();
+        __syncwarp();
+        if (lane == 0) MbarArrive(&ctl->out_empty[tile][ob]);
+        ++j;
+      }
+    }
+  }
+  __syncwarp();
+  TcFenceBefore();
+  __syncthreads();
+  if (ctl->failed) {
+    if (tid == 0) a.status->wait_timeout = 1;
+    DrainDelay();
+    __syncthreads();
+  }
+  if (warp == 12) {
+    TcFenceAfter();
+    TmemFree(ctl->tmem_base, 512);
+  }
+}
+
 }  // namespace
 
 size_t AttnFwdSmem(int d) { return 128 * d * 2 + 64 * d * 2 + d * 128 + kHalfTileBytes + 1152; }
@@ -1069,8 +1399,20 @@ void PackHeads(const float* x, uint16_t* rows, uint32_t B, uint32_t S, uint32_t 
   PackRowsKernel<<<static_cast<unsigned>(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(x, rows, quads);
 }
 
+template <int D>
+static cudaError_t LaunchFwdPair(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const AttnUmmaArgs& a,
+                                 cudaStream_t s) {
+  const size_t smem = FwdShape<D>::kSmem;
+  if (cudaError_t e = Configure(AttnFwdPairKernel<D>, smem); e != cudaSuccess) return e;
+  const uint32_t pairs = ((a.S + kTile - 1) / kTile + 1) / 2 * a.B * a.H;
+  AttnFwdPairKernel<D><<<pairs < a.sms ? pairs : a.sms, kFwdThreads, smem, s>>>(q, k, v, a);
+  return cudaGetLastError();
+}
+
 cudaError_t AttnFwdUmma(const CUtensorMap& q, const CUtensorMap& k_half, const CUtensorMap& v_half,
                         const AttnUmmaArgs& a, cudaStream_t s) {
+  // (A single tile a sequence has no neighbour to share its keys with: four small CTAs to an SM do better there.)
+  if (a.S > kTile) return a.d == 64 ? LaunchFwdPair<64>(q, k_half, v_half, a, s) : LaunchFwdPair<128>(q, k_half, v_half, a, s);
   dim3 grid((a.S + kTile - 1) / kTile, a.B * a.H);
   const size_t smem = AttnFwdSmem(a.d);
   cudaError_t e;
