@@ -453,6 +453,8 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
   umma::InvalidateRange(&umma_->ctx, 0, arena_bytes_);
   range_index_ = 0;
   lora_rows_tag_.valid = false;
+  waiting_products_.clear();   // (an earlier range that ended in an error)
+  umma::ReleaseProducts(&umma_->ctx);
   PlanAdamGroups(program, begin, std::min(end, program.size()));
   PlanMergeRuns(program, begin, std::min(end, program.size()));
   PlanAttentionKeeps(program, begin, std::min(end, program.size()));
@@ -461,6 +463,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
     PlanBiasFusions(program, begin, std::min(end, program.size()));
     PlanActFusions(program, begin, std::min(end, program.size()));
     PlanAttentionPacks(program, begin, std::min(end, program.size()));
+    PlanProductGroups(program, begin, std::min(end, program.size()));
   };
   plan_fusions();
   uint64_t partial_floats = 0;
@@ -508,7 +511,8 @@ Status CudaBackend::PrepareLoraFolds(const Instruction* program, size_t begin, u
   if (lora_weights_.empty()) return {};
   LoraRangeBuffers& rb = lora_ranges_[{program, begin}];
   const uint64_t w_need = static_cast<uint64_t>(lora_weights_.size()) * lora_max_n_ * lora_max_kx_;
-  const uint64_t t_need = max_rows * lora_max_kx_;
+  const uint64_t t_need = max_rows * lora_max_kx_ * k::kUmmaProducts;
+  lora_t_stride_ = max_rows * lora_max_kx_;
   if (w_need > rb.weights_capacity || t_need > lora_t_capacity_ || lora_weights_.size() > rb.table_capacity)
     cudaStreamSynchronize(stream_);   // queued kernels may still read the old buffers
   auto grow = [&](void** buf, uint64_t* cap, uint64_t need, size_t elem) -> Status {
@@ -551,6 +555,7 @@ void CudaBackend::FreeLoraRanges() {
 
 void CudaBackend::EndRange() {
   adapter_bwd_.clear();
+  product_group_.clear();
   lora_fold_.clear();
   lora_skip_.clear();
   lora_weights_.clear();
@@ -1567,6 +1572,7 @@ void CudaBackend::PlanActFusions(std::span<const Instruction> program, size_t be
       f.addend_ref = e.in[3];
       f.absorbed = 1;   // (the kAddEW is counted by the add fusion it already is)
       f.weight_slot = add_weight(g, e.in[1], f.r, static_cast<uint32_t>(N), GemmAlphaOf(e.imm), true);
+      f.expand_index = ea - begin;
       lora_skip_[ea - begin] = 2;
       lora_fold_[i - begin] = f;
       break;
@@ -1624,6 +1630,124 @@ void CudaBackend::PlanActFusions(std::span<const Instruction> program, size_t be
     adapter_bwd_[j - begin] = ab;
     lora_skip_[j + 1 - begin] = 1;
     lora_skip_[ja - begin] = 1;
+  }
+}
+
+void CudaBackend::PlanProductGroups(std::span<const Instruction> program, size_t begin, size_t end) {
+  product_group_.assign(end > begin ? end - begin : 0, ProductGroup{});
+  if (coherence_ == Coherence::kStrict || !relaxed_allowed_ || !epilogue_fusion_ || end < begin + 3) return;
+  if (act_fusion_.size() != end - begin || pack_plan_.size() != end - begin) return;
+  const bool whole = step_program_ != nullptr && program.data() == step_program_;
+  const size_t ext_base = whole ? 0 : begin, ext_end = whole ? program.size() : end;
+  std::vector<Extents> ext(ext_end - ext_base);
+  for (size_t i = ext_base; i < ext_end; ++i)
+    if (!DescribeInstruction(program[i], arena_bytes_, rodata_bytes_, source_bytes_, &ext[i - ext_base]).empty()) return;
+  auto overlap = [](uint64_t alo, uint64_t ahi, uint64_t blo, uint64_t bhi) { return alo < bhi && blo < ahi; };
+  auto touches = [&](size_t j, uint64_t lo, uint64_t hi) {
+    const Extents& e = ext[j - ext_base];
+    for (size_t x = 0; x < e.count; ++x)
+      if (e.e[x].space == kArena && overlap(e.e[x].off, e.e[x].off + e.e[x].bytes, lo, hi)) return true;
+    return false;
+  };
+  auto observed = [&](uint64_t lo, uint64_t hi) {
+    for (const auto& [off, bytes] : observed_)
+      if (overlap(lo, hi, off, off + bytes)) return true;
+    return gather_ranks_ > 1 && overlap(lo, hi, gather_off_, gather_off_ + gather_bytes_);
+  };
+  // What the dispatch of a relaxed frozen product at i comes to: its output, its epilogue's addend (and the
+  // instruction that reads it in the plan), and the last instruction it stands for.
+  struct Product { bool ok = false; uint64_t out = kNullRef, addend = kNullRef; size_t reader = 0, last = 0; };
+  auto aligned = [&](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  auto product_at = [&](size_t i) {
+    Product p;
+    const Instruction& g = program[i];
+    const size_t at = i - begin;
+    if (!IsRelaxedFrozenGemm(g) || RefSpace(g.in[2]) != kArena || RefSpace(g.in[0]) != kArena) return p;
+    if ((g.flags & (kFlagEpilogueBias | kFlagGemmAddend)) || ActOf(g.flags) != kActNone || bias_fusion_[at].fuse ||
+        act_fusion_[at].mode != 0 || lora_skip_[at] != 0 || shadow_plan_[at].want)
+      return p;
+    const LoraFold& f = lora_fold_[at];
+    const AddFusion& af = add_fusion_[at];
+    p.out = f.fuse ? f.out_ref : af.fuse ? af.out_ref : g.in[2];
+    p.last = i;
+    if (f.fuse && f.kind != 3) {
+      p.addend = f.addend_ref;
+      p.last = i + f.absorbed;
+      if (f.addend_ref != kNullRef) return p;   // (an absorbed residual add: no chain goes through it)
+    } else if (f.fuse) {
+      p.addend = f.addend_ref;
+      p.reader = begin + f.expand_index;
+      p.last = begin + af.add_index;
+    } else if (af.fuse) {
+      p.addend = af.x_ref;
+      p.reader = p.last = begin + af.add_index;
+    }
+    // The domain of the tensor-core kernels (umma::PrepareProduct), so that no member falls out of its group.
+    const uint64_t M = g.out[0], N = g.out[1], K = g.out[2];
+    p.ok = RefSpace(p.out) == kArena && K % 8 == 0 && N % 4 == 0 && K >= 64 && N >= 16 && M >= 64 && M <= 0xFFFFFFFFull &&
+           N <= 0xFFFFFFFFull && K <= 0xFFFFFFFFull && aligned(Wr(p.out)) && (p.addend == kNullRef || aligned(Rd(p.addend))) &&
+           aligned(GemmArgsOf(g).b_col_scale);
+    return p;
+  };
+  auto same_shape = [&](size_t i, size_t j) {
+    return program[i].out[0] == program[j].out[0] && program[i].out[1] == program[j].out[1] && program[i].out[2] == program[j].out[2];
+  };
+  constexpr size_t kWindow = 16;   // instructions a chain may reach across
+  for (size_t i = begin; i < end; ++i) {
+    if (product_group_[i - begin].member) continue;
+    Product p = product_at(i);
+    if (!p.ok || p.addend != kNullRef) continue;
+    size_t members[k::kUmmaProducts] = {i};
+    size_t count = 1;
+    if (pack_plan_[i - begin].S != 0) {
+      // side by side
+      if (!pack_plan_[i - begin].copy_only) continue;
+      for (size_t j = p.last + 1; count < k::kUmmaProducts && j < end; j = p.last + 1) {
+        p = product_at(j);
+        if (!p.ok || p.addend != kNullRef || !same_shape(i, j) || program[j].in[0] != program[i].in[0] ||
+            pack_plan_[j - begin].S == 0 || !pack_plan_[j - begin].copy_only)
+          break;
+        members[count++] = j;
+      }
+      if (count < 2) continue;
+      for (size_t m = 0; m < count; ++m) product_group_[members[m] - begin] = {true, m + 1 == count, false, 0, 0, 0};
+      continue;
+    }
+    // chained
+    uint64_t dead[k::kUmmaProducts][2] = {};
+    size_t after[k::kUmmaProducts] = {};
+    const uint64_t bytes = program[i].out[0] * program[i].out[1] * 4;
+    const k::GemmArgs first = GemmArgsOf(program[i]);
+    for (size_t j = p.last + 1; count < k::kUmmaProducts && j < end && j <= p.last + kWindow; ++j) {
+      const Product q = product_at(j);
+      if (!q.ok || q.addend != p.out || !same_shape(i, j) || pack_plan_[j - begin].S != 0) continue;
+      const k::GemmArgs next = GemmArgsOf(program[j]);
+      const uint64_t lo = RefOffset(p.out), hi = lo + bytes, q_lo = RefOffset(q.out), q_hi = q_lo + bytes;
+      bool ok = first.b_col_scale == nullptr && next.b_col_scale == nullptr && first.alpha == next.alpha && !observed(lo, hi);
+      // Nothing touches the sum up to there but the instruction that adds it, and then the product itself, whose own
+      // place (left unwritten) may be the sum's once that has been read.
+      const uint64_t x_lo = RefOffset(program[j].in[0]), x_hi = x_lo + program[j].out[0] * program[j].out[2] * 4;
+      const uint64_t z_lo = RefOffset(program[j].in[2]);
+      ok = ok && !overlap(lo, hi, x_lo, x_hi) && (q.reader < j || !overlap(lo, hi, z_lo, z_lo + bytes));
+      for (size_t w = p.last + 1; w < q.last && ok; ++w)
+        if (w != q.reader && w != j && touches(w, lo, hi)) ok = false;
+      if (ok && q_lo != lo) {
+        const DeadQuery query{lo, hi, false, ~0ull, 0, 0};
+        ok = !overlap(lo, hi, q_lo, q_hi) && DeadFrom(program, ext, ext_base, end, q.last + 1, whole, i, query);
+      }
+      if (!ok) break;
+      if (q_lo != lo) { dead[count - 1][0] = lo; dead[count - 1][1] = hi; }
+      after[count - 1] = p.last - begin;
+      members[count++] = j;
+      p = q;
+      j = p.last;
+    }
+    // (A chain rounds its sum once: only where a fold has given up the instructions' own rounding already.)
+    bool folds = false;
+    for (size_t m = 0; m < count; ++m) folds = folds || lora_fold_[members[m] - begin].fuse;
+    if (count < 2 || !folds) continue;
+    for (size_t m = 0; m < count; ++m)
+      product_group_[members[m] - begin] = {true, m + 1 == count, true, dead[m][0], dead[m][1], after[m]};
   }
 }
 
@@ -1911,7 +2035,7 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
         // (the tensor-core form of it leaves t's bf16 cut in the same launch)
         pieces_made = adapter_fma_ && lf->down.flags == 0 && d.N == lf->r && k::LoraDownSupported(d.M, d.K, d.N) &&
                       k::LoraDown(d.A, static_cast<const float*>(d.B), d.C, d.M, d.K, d.N, d.alpha, stream_,
-                                  d_lora_t_);
+                                  LoraRows());
         if (!pieces_made && !(OwnOrder() && k::FastGemm(d, stream_))) k::GemmExact(d, stream_);
         ++counters_.kernel_launches;
         umma::InvalidateRange(&umma_->ctx, RefOffset(lf->down.in[2]), d.M * d.N * 4);
@@ -1922,12 +2046,12 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
       else
         lora_rows_tag_.valid = false;   // the scratch is rewritten below (or was, by the down product)
       if (!pieces_made) {
-        if (!k::LoraSplitRows(Rd(lf->t_ref), d_lora_t_, a.M, lf->r, stream_))
+        if (!k::LoraSplitRows(Rd(lf->t_ref), LoraRows(), a.M, lf->r, stream_))
           return std::unexpected("cuda: low-rank fold: the factor cannot be split (rank or alignment)");
         ++counters_.kernel_launches;
       }
       const uint32_t kx = k::LoraSplitColumns(lf->r);
-      a.aux_a = d_lora_t_;
+      a.aux_a = LoraRows();
       a.aux_b = d_lora_w_ + static_cast<uint64_t>(lf->weight_slot) * lora_max_n_ * lora_max_kx_;
       a.aux_k = kx;
       a.C = Wr(lf->out_ref);
@@ -1946,12 +2070,35 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
       }
     }
     int launches = 0;
-    const std::string err = umma::TryGemm(&umma_->ctx, a, RefSpace(ins.in[1]) == kRodata ? 1 : 2,
-                                          RefOffset(ins.in[1]), RefOffset(ins.in[0]),
-                                          a.a_k_scale ? ins.in[3] : ~0ull,   // the whole ref: its address space is part of the key
-                                          stream_,
-                                          &launches);
-    if (err.empty() && launches > 0) {
+    bool launched = false;
+    const ProductGroup* group = range_index_ < product_group_.size() && product_group_[range_index_].member
+                                    ? &product_group_[range_index_] : nullptr;
+    // (without a copy buffer of its own a product leaves as f32, by itself)
+    const bool joins = group && (group->chained || (pack_rows && !a.store_c));
+    umma::PreparedProduct product;
+    std::string err = umma::PrepareProduct(&umma_->ctx, a, RefSpace(ins.in[1]) == kRodata ? 1 : 2, RefOffset(ins.in[1]),
+                                           RefOffset(ins.in[0]),
+                                           a.a_k_scale ? ins.in[3] : ~0ull,   // the whole ref: its address space is part of the key
+                                           joins && !group->last, &product, &launched, stream_, &launches);
+    if (err.empty() && launched) {
+      if (joins) {
+        if (group->chained) product.args.addend = nullptr;   // it is the sum of the products before this one
+        waiting_products_.push_back(product);
+        lora_rows_tag_.valid = false;   // (what it spoke of now belongs to the waiting product)
+      } else {
+        err = umma::LaunchProducts(&umma_->ctx, &product, 1, false, stream_, &launches);
+      }
+      if (err.empty() && group && group->last && !waiting_products_.empty()) {
+        err = umma::LaunchProducts(&umma_->ctx, waiting_products_.data(), static_cast<int>(waiting_products_.size()),
+                                   group->chained, stream_, &launches);
+        waiting_products_.clear();
+        umma::ReleaseProducts(&umma_->ctx);
+      }
+    }
+    if (err.empty() && group && !launched) return std::unexpected("cuda: the tensor-core path refused a product it was planned on");
+    if (err.empty() && group && group->dead_hi > group->dead_lo)
+      deferred_elided_.push_back({group->after, group->dead_lo, group->dead_hi});
+    if (err.empty() && launched) {
       ++counters_.relaxed_executions;
       counters_.kernel_launches += launches;
       skip_next_add_bias_ = fuse != nullptr;
@@ -1984,7 +2131,7 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     a.pack_dst = nullptr;
     if (!err.empty()) return std::unexpected("cuda: " + err);
     if (lf) return std::unexpected("cuda: low-rank fold: the tensor-core path refused a product it was planned on");
-    // launches == 0: the shape is outside the tensor-core kernel's domain.
+    // Not launched: the shape is outside the tensor-core kernel's domain.
     if (fuse) {
       a.bias = nullptr;
       a.C = Wr(ins.in[2]);
@@ -2013,8 +2160,8 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     b.alpha_dt = GemmAlphaOf(ins.imm); b.alpha_db = GemmAlphaOf(ab.db.imm); b.alpha_da = GemmAlphaOf(ab.da.imm);
     // dT's bf16 cut in the same pass, for the fold that takes dT A^T a few instructions on.
     const bool cut = lora_fold_enabled_ && d_lora_t_ != nullptr &&
-                     b.M * k::LoraSplitColumns(static_cast<uint32_t>(b.r)) <= lora_t_capacity_;
-    if (cut) b.dt_pieces = d_lora_t_;
+                     b.M * k::LoraSplitColumns(static_cast<uint32_t>(b.r)) <= lora_t_stride_;
+    if (cut) b.dt_pieces = LoraRows();
     lora_rows_tag_.valid = false;
     int tensor_launches = 0;
     if (const std::string err = umma::TryLoraBackward(&umma_->ctx, b, stream_, &tensor_launches); !err.empty())

@@ -34,6 +34,7 @@
 #include "extents.h"
 #include "kernels.h"
 #include "plan_abi.h"
+#include "umma_gemm.h"
 
 namespace see {
 
@@ -432,10 +433,26 @@ class CudaBackend {
     uint64_t out_ref = kNullRef;    // where the sum is written
     uint64_t addend_ref = kNullRef; // epilogue addend (the absorbed kAddEW's other operand, or kind 3's acc)
     uint32_t absorbed = 0;          // instructions this dispatch stands for besides G
+    size_t expand_index = 0;        // kind 3: range position of E, which alone reads acc
     uint64_t dead[3][2] = {{0, 0}, {0, 0}, {0, 0}};   // f32 ranges left unwritten
     int dead_count = 0;
   };
   std::vector<LoraFold> lora_fold_;          // per range position (of G)
+
+  // Relaxed products of one shape launched as one, from the last of them (umma::LaunchProducts): the dispatch of an
+  // earlier one makes its operands' copies and leaves the launch to the last.  Engine / lazy coherence only.
+  //   side by side: neighbours that read the same activation (Q, K and V), each leaving as its attention copy alone.
+  //     Nothing lies between them but what their own dispatches stand for.
+  //   chained: each adds its product to the one before it (the input gradients of Q, K and V), so that only the last sum
+  //     is stored.  The sums in between are proven dead; what an earlier product reads is copied, or frozen.
+  struct ProductGroup {
+    bool member = false, last = false, chained = false;
+    uint64_t dead_lo = 0, dead_hi = 0;   // chained, not the last: the sum left unwritten ...
+    size_t after = 0;                    // ... stale once the instruction at this range index has passed
+  };
+  void PlanProductGroups(std::span<const Instruction> program, size_t begin, size_t end);
+  std::vector<ProductGroup> product_group_;              // per range position
+  std::vector<umma::PreparedProduct> waiting_products_;  // prepared, not launched
   std::vector<uint8_t> lora_skip_;           // per range position: 1 done by an earlier dispatch, 2 never runs
   std::vector<k::LoraWeight> lora_weights_;  // the range's adapter matrices (host copy of the table)
   uint32_t lora_max_n_ = 0, lora_max_kx_ = 0;
@@ -451,8 +468,9 @@ class CudaBackend {
   std::map<std::pair<const Instruction*, size_t>, LoraRangeBuffers> lora_ranges_;
   k::LoraWeight* d_lora_table_ = nullptr;    // the current range's
   uint16_t* d_lora_w_ = nullptr;
-  uint16_t* d_lora_t_ = nullptr;             // [rows][kx] bf16, reused by every fold
-  uint64_t lora_t_capacity_ = 0;
+  uint16_t* d_lora_t_ = nullptr;             // [rows][kx] bf16, reused by every fold: one for each product of a group
+  uint64_t lora_t_capacity_ = 0, lora_t_stride_ = 0;
+  uint16_t* LoraRows() const { return d_lora_t_ ? d_lora_t_ + waiting_products_.size() * lora_t_stride_ : nullptr; }
   bool lora_fold_enabled_ = true;
   bool attn_one_walk_ = true;
   bool adapter_fma_ = true;

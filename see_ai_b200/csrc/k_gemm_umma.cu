@@ -136,12 +136,12 @@ __device__ __forceinline__ bool IsCopyOnly(const UmmaEpilogue& ep) {
   return ep.addend == nullptr && ep.bias == nullptr && ep.act == kActNone && ep.pack_dst != nullptr &&
          ep.fuse_mode == kFuseNone && !ep.store_c;
 }
-__device__ __forceinline__ void EpilogueStoreCopy(const UmmaEpilogue& ep, size_t at, const float4& acc,
+__device__ __forceinline__ void EpilogueStoreCopy(uint16_t* pack_dst, size_t at, const float4& acc,
                                                   const float4& scale) {
   uint32_t lo, hi;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(acc.y * scale.y), "f"(acc.x * scale.x));
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(acc.w * scale.w), "f"(acc.z * scale.z));
-  *reinterpret_cast<uint2*>(ep.pack_dst + at) = make_uint2(lo, hi);
+  *reinterpret_cast<uint2*>(pack_dst + at) = make_uint2(lo, hi);
 }
 // ... for a product stored as it is (the vocabulary head, the gradient products that carry nothing else) ...
 __device__ __forceinline__ bool IsPlainStore(const UmmaEpilogue& ep) {
@@ -250,17 +250,32 @@ __device__ __forceinline__ bool PartnerWait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
-// Element offsets along K of reduction block kb's tiles of A and B.
-struct BlockAt { int32_t a, b; bool aux; };
-__device__ __forceinline__ BlockAt BlockCoord(const UmmaEpilogue& ep, uint32_t kb, uint32_t main_blocks) {
+// Element offsets along K of reduction block kb's tiles of A and B, and which product's maps they come from (side by
+// side: `product`; chained: the one kb falls into).
+struct BlockAt { int32_t a, b; uint32_t product; bool aux; };
+__device__ __forceinline__ BlockAt BlockCoord(const UmmaEpilogue& ep, uint32_t kb, uint32_t main_blocks, uint32_t product) {
+  if (ep.chained)
+    for (uint32_t len; product + 1 < ep.products && kb >= (len = main_blocks + ep.product[product].aux_k_blocks); ++product)
+      kb -= len;
   if (kb >= main_blocks) {
     const int32_t x = static_cast<int32_t>((kb - main_blocks) * kBlockK);
-    return {x, x, true};
+    return {x, x, product, true};
   }
-  if (ep.seg_blocks == 0) return {static_cast<int32_t>(kb * kBlockK), static_cast<int32_t>(kb * kBlockK), false};
+  if (ep.seg_blocks == 0) return {static_cast<int32_t>(kb * kBlockK), static_cast<int32_t>(kb * kBlockK), product, false};
   const uint32_t w = kb / ep.segs, seg = kb - w * ep.segs;
   return {static_cast<int32_t>((((ep.seg_a >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK),
-          static_cast<int32_t>((((ep.seg_b >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK), false};
+          static_cast<int32_t>((((ep.seg_b >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK), product, false};
+}
+// Blocks of a tile's whole reduction.
+__device__ __forceinline__ uint32_t ReductionBlocks(const UmmaEpilogue& ep, uint32_t main_blocks, uint32_t product) {
+  uint32_t blocks = main_blocks + ep.product[product].aux_k_blocks;
+  if (ep.chained)
+    for (uint32_t p = 1; p < ep.products; ++p) blocks += main_blocks + ep.product[p].aux_k_blocks;
+  return blocks;
+}
+// Column tiles of all the outputs of a launch.
+__device__ __forceinline__ uint32_t ColumnTiles(const UmmaEpilogue& ep, uint32_t tiles_n) {
+  return ep.chained ? tiles_n : tiles_n * ep.products;
 }
 
 // ---- about one tile per SM --------------------------------------------------------------
@@ -316,9 +331,7 @@ __device__ __forceinline__ float4 LoadClusterF4(uint32_t cluster_addr) {
 
 template <uint32_t kTN, bool kSeg>
 __global__ void __launch_bounds__(kTThreads, 1)
-UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                   const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
-                   const __grid_constant__ UmmaEpilogue ep, uint32_t splits) {
+UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant__ UmmaEpilogue ep, uint32_t splits) {
   using T = TTile<kTN>;
   constexpr uint32_t kStages = T::kStages, kStageBytes = T::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
@@ -328,14 +341,14 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t split = ClusterCtaRank();   // (a cluster is one tile's splits)
-  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, tile = blockIdx.x / splits;
-  const uint32_t mb = tile / tiles_n, nb = tile - mb * tiles_n;
+  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, all_n = kSeg ? tiles_n : ColumnTiles(ep, tiles_n), tile = blockIdx.x / splits;
+  const uint32_t mb = tile / all_n, product = kSeg ? 0 : tile % all_n / tiles_n, nb = tile % all_n % tiles_n;
   const uint32_t m0 = mb * kBlockM, n0 = nb * kTN;
   // The reduction runs over the main operands' K and then over aux_k_blocks more
   // 64-wide blocks taken from the second pair of maps (a low-rank term T . B'^T
-  // accumulated into the same tile; see UmmaEpilogue::aux_k_blocks).
+  // accumulated into the same tile; see UmmaEpilogue::Product).
   const uint32_t main_blocks = (ep.K + kBlockK - 1) / kBlockK;
-  const uint32_t k_blocks = main_blocks + ep.aux_k_blocks;
+  const uint32_t k_blocks = ReductionBlocks(ep, main_blocks, product);
   // Accumulators of the reduction, `group` blocks each: a plain product has one, piece products one per block of K.
   const uint32_t all = kSeg ? ep.seg_blocks : k_blocks;
   const uint32_t part0 = all * split / splits, part1 = all * (split + 1) / splits;
@@ -375,9 +388,9 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           break;
         }
         uint8_t* a_dst = smem + s * kStageBytes;
-        const BlockAt at = BlockCoord(ep, kb, main_blocks);
-        const CUtensorMap* ma = at.aux ? &map_a2 : &map_a;
-        const CUtensorMap* mb_ = at.aux ? &map_b2 : &map_b;
+        const BlockAt at = BlockCoord(ep, kb, main_blocks, product);
+        const CUtensorMap* ma = at.aux ? &maps.a2[at.product] : &maps.a[at.product];
+        const CUtensorMap* mb_ = at.aux ? &maps.b2[at.product] : &maps.b[at.product];
         MbarExpectTx(&bars->full[s], kStageBytes);
         TmaLoad2D(a_dst, ma, &bars->full[s], at.a, static_cast<int32_t>(m0));
         TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], at.b, static_cast<int32_t>(n0));
@@ -511,6 +524,10 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // Four elements per thread at a time, their operands loaded before the first is stored.  `store` is one form of
     // the epilogue, chosen once: tests per element would cost more than the stores.
     constexpr uint32_t kUnroll = 4;
+    const bool side_by_side = !kSeg && ep.products > 1 && !ep.chained;
+    const float alpha = side_by_side ? ep.product[product].alpha : ep.alpha;
+    const float* col_scale = side_by_side ? ep.product[product].col_scale : ep.col_scale;
+    uint16_t* pack_dst = side_by_side ? ep.product[product].pack_dst : ep.pack_dst;
     auto each = [&](auto has_side, auto store) {
       for (uint32_t i0 = et; i0 < rows * kChunks; i0 += kTEpiThreads * kUnroll) {
         float4 acc[kUnroll], side[kUnroll];
@@ -528,8 +545,8 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           const uint32_t i = i0 + u * kTEpiThreads, lr = r0 + i / kChunks, chunk = i % kChunks;
           const uint32_t row = m0 + lr, n = n0 + chunk * 4;
           if (i >= rows * kChunks || row >= ep.M || n >= ep.N) continue;
-          float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
-          if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
+          float4 scale = make_float4(alpha, alpha, alpha, alpha);
+          if (col_scale) scale = __ldg(reinterpret_cast<const float4*>(col_scale + n));
           store(static_cast<size_t>(row) * ep.N + n, row, n, acc[u], scale, side[u]);
         }
       }
@@ -562,7 +579,7 @@ UmmaGemmTileKernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       });
     } else if (IsCopyOnly(ep)) {
       each(NoSide{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4&) {
-        EpilogueStoreCopy(ep, at, acc, scale);
+        EpilogueStoreCopy(pack_dst, at, acc, scale);
       });
     } else if (IsBiasGeluOnly(ep) && !ep.shadow_k_scale) {
       each(NoSide{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4&) {
@@ -671,11 +688,7 @@ struct __align__(8) PBarriers {
 // warps add the blocks in registers, 64 outputs a thread, one block behind the products.
 template <bool kSideLoads, bool kPair, bool kSeg>
 __global__ void __launch_bounds__(kPThreads, 1)
-UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
-                         const __grid_constant__ CUtensorMap map_b,
-                         const __grid_constant__ CUtensorMap map_a2,
-                         const __grid_constant__ CUtensorMap map_b2,
-                         const __grid_constant__ UmmaEpilogue ep,
+UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant__ UmmaEpilogue ep,
                          uint32_t band_blocks) {
   static_assert(!(kSideLoads && kSeg), "the sums take the registers of the loads in flight");
   using T = PTile<kPair>;
@@ -689,11 +702,11 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t main_blocks = (ep.K + kBlockK - 1) / kBlockK;
-  const uint32_t k_blocks = main_blocks + ep.aux_k_blocks;   // then the low-rank term's blocks
-  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN;
+  constexpr bool kSeveral = !kSeg && !kSideLoads;   // products side by side
+  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, all_n = kSeveral ? ColumnTiles(ep, tiles_n) : tiles_n;
   const uint32_t tiles_m = (ep.M + T::kRowsPerTile - 1) / T::kRowsPerTile;
-  const uint32_t total_tiles = tiles_m * tiles_n;
-  const uint32_t group = kSeg ? ep.segs : k_blocks, groups = kSeg ? ep.seg_blocks : 1u;   // blocks per accumulator
+  const uint32_t total_tiles = tiles_m * all_n;
+  const uint32_t groups = kSeg ? ep.seg_blocks : 1u;   // accumulators per tile
   // A work unit is a CTA, or a CTA pair: `unit` walks the tiles, `cta_rank` is this CTA's half of a pair's tile.
   const uint32_t cta_rank = kPair ? ClusterCtaRank() : 0u;
   const uint32_t unit = kPair ? blockIdx.x >> 1 : blockIdx.x, units = kPair ? gridDim.x >> 1 : gridDim.x;
@@ -734,20 +747,24 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
       bool ok = true;
       for (uint32_t t = unit; t < total_tiles && ok; t += units) {
         uint32_t mb, nb;
-        TileCoord(t, tiles_m, tiles_n, band_blocks, &mb, &nb);
+        TileCoord(t, tiles_m, all_n, band_blocks, &mb, &nb);
+        const uint32_t product = kSeveral ? nb / tiles_n : 0;
+        nb -= product * tiles_n;
         const uint32_t m0 = mb * T::kRowsPerTile + cta_rank * kBlockM, n0 = nb * kTN;
+        const uint32_t k_blocks = ReductionBlocks(ep, main_blocks, product);
         // Ask L2 for the A rows of this CTA's next tile now, so that its loads
         // find them there instead of paying an HBM round trip inside the ring.
         if (t + units < total_tiles && k_blocks <= 64 && ep.seg_blocks == 0) {   // (a long K would only thrash L2)
           uint32_t next_mb, next_nb;
-          TileCoord(t + units, tiles_m, tiles_n, band_blocks, &next_mb, &next_nb);
+          TileCoord(t + units, tiles_m, all_n, band_blocks, &next_mb, &next_nb);
           const uint32_t next_m0 = next_mb * T::kRowsPerTile + cta_rank * kBlockM;
           if (next_m0 != m0)
-            for (uint32_t kb = 0; kb < main_blocks; ++kb)
-              asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
-                           ::"l"(reinterpret_cast<uint64_t>(&map_a)),
-                             "r"(static_cast<int32_t>(kb * kBlockK)), "r"(static_cast<int32_t>(next_m0))
-                           : "memory");
+            for (uint32_t p = 0; p < (ep.chained ? ep.products : 1u); ++p)   // (side by side: they share A)
+              for (uint32_t kb = 0; kb < main_blocks; ++kb)
+                asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
+                             ::"l"(reinterpret_cast<uint64_t>(&maps.a[p])),
+                               "r"(static_cast<int32_t>(kb * kBlockK)), "r"(static_cast<int32_t>(next_m0))
+                             : "memory");
         }
         for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
           const uint32_t s = it % kPStages, round = it / kPStages;
@@ -758,9 +775,9 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
             break;
           }
           uint8_t* a_dst = smem + s * kPStageBytes;
-          const BlockAt at = BlockCoord(ep, kb, main_blocks);
-          const CUtensorMap* ma = at.aux ? &map_a2 : &map_a;
-          const CUtensorMap* mb_ = at.aux ? &map_b2 : &map_b;
+          const BlockAt at = BlockCoord(ep, kb, main_blocks, product);
+          const CUtensorMap* ma = at.aux ? &maps.a2[at.product] : &maps.a[at.product];
+          const CUtensorMap* mb_ = at.aux ? &maps.b2[at.product] : &maps.b[at.product];
           if constexpr (kPair) {
             // Both CTAs' bytes are counted on the even CTA's barrier, which alone expects them.
             if (cta_rank == 0) MbarExpectTx(&bars->full[s], 2 * kPStageBytes);
@@ -793,6 +810,14 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + buf * kTN;
+        uint32_t group;   // blocks of this accumulator
+        if constexpr (kSeg) {
+          group = ep.segs;
+        } else {
+          uint32_t mb, nb;
+          TileCoord(t, tiles_m, all_n, band_blocks, &mb, &nb);
+          group = ReductionBlocks(ep, main_blocks, kSeveral ? nb / tiles_n : 0);
+        }
         for (uint32_t kb = 0; kb < group; ++kb, ++it) {
           const uint32_t s = it % kPStages, round = it / kPStages;
           if (!PartnerWait<kSeg && kPair>(&bars->full[s], round & 1)) {
@@ -830,7 +855,9 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
     for (uint32_t t = unit; t < total_tiles; t += units, ++lt) {
       uint32_t buf = lt & 1, use = lt >> 1;
       uint32_t mb, nb;
-      TileCoord(t, tiles_m, tiles_n, band_blocks, &mb, &nb);
+      TileCoord(t, tiles_m, all_n, band_blocks, &mb, &nb);
+      const uint32_t product = kSeveral ? nb / tiles_n : 0;
+      nb -= product * tiles_n;
       const uint32_t m0 = mb * T::kRowsPerTile + cta_rank * kBlockM, n0 = nb * kTN;
       if (ep.fuse_mode == kFuseActBwd) {
         // The absorbed backward activation reads x[m, n] next to every output:
@@ -838,7 +865,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
         // lane and pass), a whole tile ahead of the loads that use them.
         auto prefetch_x = [&](uint32_t tile) {
           uint32_t pmb, pnb;
-          TileCoord(tile, tiles_m, tiles_n, band_blocks, &pmb, &pnb);
+          TileCoord(tile, tiles_m, all_n, band_blocks, &pmb, &pnb);   // (one product: nothing side by side has an x)
           const uint32_t prow = pmb * T::kRowsPerTile + cta_rank * kBlockM + quarter * 32 + lane;
           if (prow >= ep.M) return;
 #pragma unroll
@@ -859,6 +886,10 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
       [[maybe_unused]] const bool bias_gelu_only = IsBiasGeluOnly(ep);
       [[maybe_unused]] const bool copy_only = IsCopyOnly(ep);
       [[maybe_unused]] const bool plain_store = IsPlainStore(ep);
+      const bool side_by_side = kSeveral && ep.products > 1 && !ep.chained;
+      [[maybe_unused]] const float alpha = side_by_side ? ep.product[product].alpha : ep.alpha;
+      [[maybe_unused]] const float* col_scale = side_by_side ? ep.product[product].col_scale : ep.col_scale;
+      [[maybe_unused]] uint16_t* pack_dst = side_by_side ? ep.product[product].pack_dst : ep.pack_dst;
       [[maybe_unused]] const bool ragged = (ep.N & 3u) != 0;   // (never with kSideLoads)
       [[maybe_unused]] float4 side_a[4], side_b[4];
       if constexpr (kSideLoads) {   // the first group's loads fly during the wait for the accumulator
@@ -938,8 +969,8 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
             for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr)
               EpilogueStoreRagged(ep, row0 + rr, n, staged(rr), false);
           } else if (n < ep.N) {   // N % 4 == 0: a float4 is all in or all out
-            float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
-            if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
+            float4 scale = make_float4(alpha, alpha, alpha, alpha);
+            if (col_scale) scale = __ldg(reinterpret_cast<const float4*>(col_scale + n));
             float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
             if (ep.bias) bias = __ldg(reinterpret_cast<const float4*>(ep.bias + n));
             float4 kscale = make_float4(1.f, 1.f, 1.f, 1.f);   // the consumer's per-column factor (x * 1 == x)
@@ -952,7 +983,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ CUtensorMap map_a,
               if (plain_store)
                 EpilogueStorePlain(ep, at, acc, scale);
               else if (copy_only)
-                EpilogueStoreCopy(ep, at, acc, scale);
+                EpilogueStoreCopy(pack_dst, at, acc, scale);
               else if (bias_gelu_only)
                 EpilogueStoreBiasGelu(ep, at, acc, scale, bias, kscale);
               else
@@ -1170,9 +1201,10 @@ static cudaError_t Configure() {
   return allow(UmmaGemmPersistentKernel<false, true, true>, pair);
 }
 
-UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms) {
+UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms,
+                          uint32_t side_by_side) {
   UmmaGemmPlan p;
-  const uint32_t ptiles_n = (N + kPBlockN - 1) / kPBlockN, tiles_m = (M + kBlockM - 1) / kBlockM;
+  const uint32_t ptiles_n = (N + kPBlockN - 1) / kPBlockN * side_by_side, tiles_m = (M + kBlockM - 1) / kBlockM;
   const uint64_t wide = static_cast<uint64_t>(ptiles_n) * tiles_m;
   const bool pairs_on = g_cta_pairs.load(std::memory_order_relaxed) && sms >= 2;
   // The tile kernel, on the width and split of least estimated time (us): waves of CTAs, each a fixed part, its
@@ -1182,7 +1214,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
   double best = 1e30;
   for (uint32_t tn : {64u, 128u, 192u, 256u})
     for (uint32_t splits = 1; splits <= 4 && splits * group <= k_blocks; splits *= 2) {
-      const uint64_t ctas = static_cast<uint64_t>(tiles_m) * ((N + tn - 1) / tn) * splits;
+      const uint64_t ctas = static_cast<uint64_t>(tiles_m) * ((N + tn - 1) / tn) * side_by_side * splits;
       const uint64_t room = splits <= 2 ? sms : sms * 9 / 10;   // clusters of four do not fill every GPC
       const double waves = static_cast<double>((ctas + room - 1) / room);
       const double block = std::max(0.165 + 0.00087 * tn, 0.267);
@@ -1203,7 +1235,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
     // must both finish before the accumulator is free again.  An output that stays in L2 takes about 2 us less.
     const uint64_t pair_tiles = static_cast<uint64_t>(ptiles_n) * ((M + 2 * kBlockM - 1) / (2 * kBlockM));
     const uint64_t pairs = sms / 2;
-    const double l2 = static_cast<uint64_t>(M) * N <= (1ull << 24) ? 2.0 : 0.0;
+    const double l2 = static_cast<uint64_t>(M) * N * side_by_side <= (1ull << 24) ? 2.0 : 0.0;
     const double single = 7.0 + static_cast<double>((wide + sms - 1) / sms) * std::max(0.53 * k_blocks, (light ? 8.3 : 10.5) - l2);
     const double paired = pairs_on && wide > 2ull * sms
                               ? 7.5 + static_cast<double>((pair_tiles + pairs - 1) / pairs) *
@@ -1223,13 +1255,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
   return p;
 }
 
-cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                           const UmmaEpilogue& ep, cudaStream_t s, const CUtensorMap* aux_a,
-                           const CUtensorMap* aux_b) {
-  // Without a low-rank term the second pair of maps is never dereferenced; the
-  // main pair stands in so that the parameters are valid descriptors.
-  const CUtensorMap& map_a2 = ep.aux_k_blocks && aux_a ? *aux_a : map_a;
-  const CUtensorMap& map_b2 = ep.aux_k_blocks && aux_b ? *aux_b : map_b;
+cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const UmmaMaps& maps, const UmmaEpilogue& ep, cudaStream_t s) {
   // The shared-memory limit of a kernel is a per-device attribute: one flag per
   // device, so a second backend on another GPU of the same process configures its own.
   static std::atomic<bool> configured_on[64] = {};
@@ -1243,16 +1269,14 @@ cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const CUtensorMap& map_a, c
   const bool seg = ep.seg_blocks != 0;
   if (!plan.persistent) {
     auto launch = [&](auto kernel, size_t bytes) {
-      return LaunchClustered(kernel, dim3(plan.grid), dim3(kTThreads), bytes, s, plan.splits, map_a, map_b, map_a2,
-                             map_b2, ep, plan.splits);
+      return LaunchClustered(kernel, dim3(plan.grid), dim3(kTThreads), bytes, s, plan.splits, maps, ep, plan.splits);
     };
     return seg ? WithTileKernel<true>(plan.tn, launch) : WithTileKernel<false>(plan.tn, launch);
   }
   // An addend or the x of an absorbed backward activation is software-pipelined (16 bytes at a time).
   const bool side_loads = !seg && (ep.addend != nullptr || ep.fuse_mode == kFuseActBwd) && (ep.N & 3) == 0;
   auto launch = [&](auto kernel, size_t bytes) {
-    return LaunchClustered(kernel, dim3(plan.grid), dim3(kPThreads), bytes, s, plan.pair ? 2u : 1u, map_a, map_b, map_a2,
-                           map_b2, ep, plan.band);
+    return LaunchClustered(kernel, dim3(plan.grid), dim3(kPThreads), bytes, s, plan.pair ? 2u : 1u, maps, ep, plan.band);
   };
   const size_t bytes = plan.pair ? UmmaPersistentSmemBytes<true>() : UmmaPersistentSmemBytes<false>();
   if (plan.pair)

@@ -272,6 +272,7 @@ void SplitMatrix(const float* src, uint16_t* dst, size_t rows, size_t cols, bool
 // ---- GEMM -------------------------------------------------------------------
 enum class BType : uint8_t { kF32 = 0, kI8 = 1, kBf16 = 2 };
 constexpr int kFuseNone = 0, kFuseActFwd = 1, kFuseActBwd = 2;   // GemmArgs::fuse_mode
+constexpr uint32_t kUmmaProducts = 3;   // tensor-core products in one launch, at most
 struct GemmArgs {
   const float* A = nullptr;    // [M,K], or [K,M] when a_transposed
   const void* B = nullptr;     // [K,N], or [N,K] when b_transposed
@@ -301,7 +302,7 @@ struct GemmArgs {
   bool store_c = true;
   bool addend_after_bias = false;   // tensor-core path: v = addend + (product + bias)
   // Tensor-core path only: a low-rank term appended to the reduction (see
-  // UmmaEpilogue::aux_k_blocks): aux_a [M, aux_k] and aux_b [N, aux_k], bf16.
+  // UmmaEpilogue::Product): aux_a [M, aux_k] and aux_b [N, aux_k], bf16.
   const uint16_t* aux_a = nullptr;
   const uint16_t* aux_b = nullptr;
   uint32_t aux_k = 0;

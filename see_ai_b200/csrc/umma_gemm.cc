@@ -32,6 +32,7 @@ struct ActCopy {   // a bf16 copy of an arena activation [M, K]
   uint64_t a_off = ~0ull, scale_off = ~0ull, M = 0, K = 0;
   bool valid = false;
   bool reserved = false;   // handed to a producer (ReserveShadow) and not yet committed
+  bool kept = false;       // an operand of a product not launched yet (PrepareProduct): not to be reused
   uint16_t* buf = nullptr;
   uint64_t capacity = 0;  // elements
   uint64_t last_use = 0;
@@ -290,9 +291,10 @@ static uint16_t* WeightCopy(Impl* impl, const k::GemmArgs& a, int b_space, uint6
   return w;
 }
 
-std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_off,
-                    uint64_t a_off, uint64_t a_scale_off, cudaStream_t stream, int* launches) {
-  *launches = 0;
+std::string PrepareProduct(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_off, uint64_t a_off,
+                           uint64_t a_scale_off, bool keep, PreparedProduct* out, bool* ok, cudaStream_t stream,
+                           int* launches) {
+  *ok = false;
   Impl* impl = ctx->impl;
   if (!impl) return {};
   // The kernel's domain: K a multiple of 8 (16-byte global strides for TMA), N a
@@ -309,8 +311,9 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   // weight copy, w[n][k] = bf16(W[n][k] * s[k]), once per binding: the activation
   // copy is then plain bf16(A), which every producer can write without a table
   // look-up per element, and which any other consumer of the tensor can share.
-  uint16_t* w = WeightCopy(impl, a, b_space, b_off, a.a_k_scale, a_scale_off, stream, launches);
-  if (!w) return "tensor-core path: weight copy allocation failed";
+  out->args = a;
+  out->weight = WeightCopy(impl, a, b_space, b_off, a.a_k_scale, a_scale_off, stream, launches);
+  if (!out->weight) return "tensor-core path: weight copy allocation failed";
 
   // ---- the activation, bf16 [M][K], reused while its arena range is unwritten ----
   ActCopy* slot = nullptr;
@@ -321,7 +324,7 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
     // A slot a producer is writing (this product's own epilogue, when it has
     // absorbed a following activation) is not a candidate.
     for (auto& c : impl->acts) {
-      if (c.reserved) continue;
+      if (c.reserved || c.kept) continue;
       if (!c.valid) { slot = &c; break; }
       if (!slot || c.last_use < slot->last_use) slot = &c;
     }
@@ -345,20 +348,59 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
     slot->valid = true;
   }
   slot->last_use = ++impl->tick;
+  slot->kept = slot->kept || keep;
+  out->act = slot->buf;
+  *ok = true;
+  return {};
+}
 
-  CUtensorMap map_a, map_b, aux_a, aux_b;
-  const bool has_aux = a.aux_a && a.aux_b && a.aux_k >= 64 && a.aux_k % 64 == 0;
-  const uint32_t k_blocks = static_cast<uint32_t>((a.K + 63) / 64) + (has_aux ? a.aux_k / 64 : 0);
-  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks, 1,
-                                                LightEpilogue(a), impl->sms);
-  if (!EncodeBf16Map(impl, &map_a, slot->buf, a.M, a.K, k::umma_cfg::kBlockM) ||
-      !EncodeBf16Map(impl, &map_b, w, a.N, a.K, plan.b_box))
-    return "tensor-core path: cuTensorMapEncodeTiled refused the operand layout";
-  if (has_aux && (!EncodeBf16Map(impl, &aux_a, a.aux_a, a.M, a.aux_k, k::umma_cfg::kBlockM) ||
-                  !EncodeBf16Map(impl, &aux_b, a.aux_b, a.N, a.aux_k, plan.b_box)))
-    return "tensor-core path: cuTensorMapEncodeTiled refused the low-rank operand layout";
+void ReleaseProducts(Context* ctx) {
+  if (!ctx->impl) return;
+  for (auto& c : ctx->impl->acts) c.kept = false;
+}
 
+static bool HasLowRank(const k::GemmArgs& a) { return a.aux_a && a.aux_b && a.aux_k >= 64 && a.aux_k % 64 == 0; }
+
+std::string LaunchProducts(Context* ctx, const PreparedProduct* products, int count, bool chained, cudaStream_t stream,
+                           int* launches) {
+  Impl* impl = ctx->impl;
+  if (!impl || count < 1 || count > static_cast<int>(k::kUmmaProducts)) return "tensor-core path: no such launch";
+  const k::GemmArgs& a = products[count - 1].args;   // a chain's output
+  const uint32_t main_blocks = static_cast<uint32_t>((a.K + 63) / 64);
+  uint32_t longest = 0, all = 0;
+  for (int p = 0; p < count; ++p) {
+    const uint32_t blocks = main_blocks + (HasLowRank(products[p].args) ? products[p].args.aux_k / 64 : 0);
+    longest = std::max(longest, blocks);
+    all += blocks;
+  }
+  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), chained ? all : longest, 1,
+                                                LightEpilogue(a), impl->sms, chained ? 1u : static_cast<uint32_t>(count));
+  k::UmmaMaps maps;
   k::UmmaEpilogue ep{};
+  for (uint32_t p = 0; p < k::kUmmaProducts; ++p) {
+    if (static_cast<int>(p) >= count) {   // never read: the first product's maps stand in, as valid descriptors
+      maps.a[p] = maps.a2[p] = maps.a[0];
+      maps.b[p] = maps.b2[p] = maps.b[0];
+      continue;
+    }
+    const k::GemmArgs& g = products[p].args;
+    if (!EncodeBf16Map(impl, &maps.a[p], products[p].act, g.M, g.K, k::umma_cfg::kBlockM) ||
+        !EncodeBf16Map(impl, &maps.b[p], products[p].weight, g.N, g.K, plan.b_box))
+      return "tensor-core path: cuTensorMapEncodeTiled refused the operand layout";
+    maps.a2[p] = maps.a[p];
+    maps.b2[p] = maps.b[p];
+    if (HasLowRank(g)) {
+      if (!EncodeBf16Map(impl, &maps.a2[p], g.aux_a, g.M, g.aux_k, k::umma_cfg::kBlockM) ||
+          !EncodeBf16Map(impl, &maps.b2[p], g.aux_b, g.N, g.aux_k, plan.b_box))
+        return "tensor-core path: cuTensorMapEncodeTiled refused the low-rank operand layout";
+      ep.product[p].aux_k_blocks = g.aux_k / 64;
+    }
+    ep.product[p].pack_dst = g.pack_dst;
+    ep.product[p].col_scale = g.b_col_scale;
+    ep.product[p].alpha = g.alpha;
+  }
+  ep.products = static_cast<uint32_t>(count);
+  ep.chained = chained ? 1 : 0;
   ep.C = a.C;
   ep.addend = a.addend;
   ep.bias = a.bias;
@@ -377,11 +419,8 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   ep.pack_dst = a.pack_dst;
   ep.store_c = a.store_c ? 1 : 0;
   ep.addend_last = a.addend_after_bias ? 1 : 0;
-  ep.aux_k_blocks = has_aux ? a.aux_k / 64 : 0;
   if (impl->prof_before) cudaEventRecord(impl->prof_before, stream);
-  if (cudaError_t e = k::UmmaGemmLaunch(plan, map_a, map_b, ep, stream, has_aux ? &aux_a : nullptr,
-                                        has_aux ? &aux_b : nullptr);
-      e != cudaSuccess)
+  if (cudaError_t e = k::UmmaGemmLaunch(plan, maps, ep, stream); e != cudaSuccess)
     return std::string("tensor-core GEMM launch: ") + cudaGetErrorString(e);
   if (impl->prof_after) {
     cudaEventRecord(impl->prof_after, stream);
@@ -390,6 +429,17 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_
   }
   ++*launches;
   return {};
+}
+
+std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_off,
+                    uint64_t a_off, uint64_t a_scale_off, cudaStream_t stream, int* launches) {
+  *launches = 0;
+  PreparedProduct product;
+  bool ok = false;
+  if (std::string e = PrepareProduct(ctx, a, b_space, b_off, a_off, a_scale_off, false, &product, &ok, stream, launches);
+      !e.empty() || !ok)
+    return e;
+  return LaunchProducts(ctx, &product, 1, false, stream, launches);
 }
 
 namespace {
@@ -525,11 +575,15 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   const uint32_t k_blocks = static_cast<uint32_t>(segments * (Kp / 64));
   const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks, segments,
                                                 LightEpilogue(a), impl->sms);
-  CUtensorMap map_a, map_b;
+  k::UmmaMaps maps;
   // An exact weight is [N][K]: past K its last block reads zeros, and so do A's padding columns.
-  if (!EncodeBf16Map(impl, &map_a, impl->split_a, a.M, 3 * Kp, k::umma_cfg::kBlockM) ||
-      !EncodeBf16Map(impl, &map_b, b, a.N, exact_b ? a.K : 3 * Kp, plan.b_box))
+  if (!EncodeBf16Map(impl, &maps.a[0], impl->split_a, a.M, 3 * Kp, k::umma_cfg::kBlockM) ||
+      !EncodeBf16Map(impl, &maps.b[0], b, a.N, exact_b ? a.K : 3 * Kp, plan.b_box))
     return "tensor-core path: cuTensorMapEncodeTiled refused the operand-piece layout";
+  for (uint32_t p = 0; p < k::kUmmaProducts; ++p) {   // (never read: valid descriptors)
+    maps.a[p] = maps.a2[p] = maps.a[0];
+    maps.b[p] = maps.b2[p] = maps.b[0];
+  }
   k::UmmaEpilogue ep{};
   ep.C = a.C;
   ep.addend = a.addend;
@@ -553,7 +607,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   ep.seg_b = exact_b ? kSegBExact : kSegBF32;
   ep.status = impl->status;
   if (impl->prof_before) cudaEventRecord(impl->prof_before, stream);
-  if (cudaError_t e = k::UmmaGemmLaunch(plan, map_a, map_b, ep, stream); e != cudaSuccess)
+  if (cudaError_t e = k::UmmaGemmLaunch(plan, maps, ep, stream); e != cudaSuccess)
     return std::string("tensor-core GEMM launch: ") + cudaGetErrorString(e);
   if (impl->prof_after) {
     cudaEventRecord(impl->prof_after, stream);
@@ -586,7 +640,7 @@ uint16_t* ReserveShadow(Context* ctx, uint64_t elems, bool keep_reserved) {
   ActCopy* slot = nullptr;
   for (auto& c : impl->acts) {
     if (!keep_reserved) c.reserved = false;   // normally one reservation at a time
-    if (c.reserved || c.capacity < elems || !c.buf) continue;
+    if (c.reserved || c.kept || c.capacity < elems || !c.buf) continue;
     if (!c.valid) { slot = &c; break; }
     if (!slot || c.last_use < slot->last_use) slot = &c;
   }

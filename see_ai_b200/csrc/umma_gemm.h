@@ -44,6 +44,24 @@ void PlanRange(Context* ctx, const Instruction* program, size_t begin, size_t en
 std::string TryGemm(Context* ctx, const k::GemmArgs& args, int b_space, uint64_t b_off,
                     uint64_t a_off, uint64_t a_scale_off, cudaStream_t stream, int* launches);
 
+// Several products of one shape as one launch: side by side (they share the activation, each leaves as its attention
+// copy alone) or chained (their sum is the output; the operands of all but the last product are unread by then).
+// PrepareProduct checks the domain, makes the operands' bf16 copies as TryGemm does and fills *out; *ok = false with an
+// empty return value: not applicable.  `keep` holds the activation copy's slot, whatever happens to the activation's
+// range, until ReleaseProducts.  LaunchProducts takes one to kUmmaProducts prepared products; the epilogue of a chain is the
+// last one's.
+struct PreparedProduct {
+  k::GemmArgs args;
+  const uint16_t* weight = nullptr;   // [N][K]
+  const uint16_t* act = nullptr;      // [M][K]
+};
+std::string PrepareProduct(Context* ctx, const k::GemmArgs& args, int b_space, uint64_t b_off, uint64_t a_off,
+                           uint64_t a_scale_off, bool keep, PreparedProduct* out, bool* ok, cudaStream_t stream,
+                           int* launches);
+std::string LaunchProducts(Context* ctx, const PreparedProduct* products, int count, bool chained, cudaStream_t stream,
+                           int* launches);
+void ReleaseProducts(Context* ctx);
+
 // An adapter site's three backward products (k::LoraBackwardArgs) as 3xTF32 on the tcgen05
 // tensor cores, one pass over dY and x, when the shape is inside that kernel's domain.
 // *launches == 0 with an empty return value: not applicable, use k::LoraBackward.

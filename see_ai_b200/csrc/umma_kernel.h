@@ -39,13 +39,22 @@ struct UmmaEpilogue {
   const float* shadow_k_scale = nullptr;
   int store_c = 1;
   int addend_last = 0;
-  // A low-rank term folded into the product: after the main operands' K the
-  // reduction continues over aux_k_blocks blocks of 64 from a second operand
-  // pair, T' [M, 64 * aux_k_blocks] and B' [N, 64 * aux_k_blocks] (bf16, K-major),
+  // Up to kUmmaProducts products of one shape in one launch.  chained = 0: side by side, each with its own output
+  // (`products` > 1: they share A, and every one leaves as its attention copy alone, product[p].pack_dst).
+  // chained = 1: one output, the sum of the products; their reductions follow one another.
+  // Each may carry a low-rank term: after the main operands' K the reduction continues over aux_k_blocks blocks of
+  // 64 from a second operand pair, T' [M, 64 * aux_k_blocks] and B' [N, 64 * aux_k_blocks] (bf16, K-major),
   // so the tile holds A W^T + T' B'^T before the epilogue scales it.  With T' and
   // B' the three-way bf16 splits of f32 factors (LoraSplit* in kernels.h) the
   // added term is the f32 product t . b to about 2^-23 of |t| |b|.
-  uint32_t aux_k_blocks = 0;
+  uint32_t products = 1;
+  int chained = 0;
+  struct Product {
+    uint32_t aux_k_blocks = 0;
+    uint16_t* pack_dst = nullptr;      // side by side
+    const float* col_scale = nullptr;  // side by side: [N], or null and alpha
+    float alpha = 1.0f;
+  } product[kUmmaProducts];
   // The stored value also as bf16 [M, N] (GemmArgs::pack_dst).
   uint16_t* pack_dst = nullptr;
   // An f32-accurate product out of bf16 pieces: the operands hold pieces side by side along K, each
@@ -64,6 +73,10 @@ struct UmmaEpilogue {
   BType src_b_type = BType::kF32;
 };
 
+// The operands of a launch, per product: a, a2: bf16 [M, K] row-major, box {64, 128}, 128-byte swizzle; b, b2: bf16
+// [N, K], box {64, plan.b_box}; a2 and b2 the low-rank term's (any valid map where there is none).
+struct UmmaMaps { CUtensorMap a[kUmmaProducts], b[kUmmaProducts], a2[kUmmaProducts], b2[kUmmaProducts]; };
+
 // Which kernel takes a product, on which tiles (k_gemm_umma.cu).
 struct UmmaGemmPlan {
   bool persistent = false, pair = false;
@@ -74,11 +87,10 @@ struct UmmaGemmPlan {
 };
 // k_blocks: 64-wide blocks of the whole reduction, a low-rank term's included; `group` of them in a row (1: any) are
 // not cut.  light: the epilogue only stores (f32 or a bf16 copy), without a second operand, bias or activation.
-UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms);
-// map_a: bf16 [M, K] row-major, box {64, 128}, 128-byte swizzle; map_b: bf16 [N, K], box {64, plan.b_box}.
-cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const CUtensorMap& map_a, const CUtensorMap& map_b,
-                           const UmmaEpilogue& ep, cudaStream_t s, const CUtensorMap* aux_a = nullptr,
-                           const CUtensorMap* aux_b = nullptr);
+// side_by_side: outputs of this shape in the launch.
+UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms,
+                          uint32_t side_by_side = 1);
+cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const UmmaMaps& maps, const UmmaEpilogue& ep, cudaStream_t s);
 // Large products run on CTA pairs (cta_group::2) by default; off = one CTA per tile.  Process-wide.
 void UmmaSetCtaPairs(bool on);
 // dst[N][K] (bf16 bits) from src [K][N] (transpose) or [N][K]; int8 and bf16 widen exactly.
