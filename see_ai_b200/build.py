@@ -31,6 +31,7 @@ CU_SOURCES = {
     "k_gemm_exact.cu": ["-fmad=false"],
     "k_gemm_skinny.cu": ["-fmad=false"],
     "k_gemm_umma.cu": ["-fmad=false"],
+    "k_gemm_cut.cu": ["-fmad=false"],
     "k_eval.cu": [],
     "k_host.cu": [],
     "k_attn_umma.cu": [],

@@ -1,0 +1,385 @@
+// f32-accurate products of an f32 activation that lies row-major (A [M, K], K fastest) on the tensor cores, the
+// activation cut into its three bf16 pieces on the way into shared memory:
+//
+//     C[M,N] = epilogue( A[M,K] . B[N,K]^T )      B: three bf16 pieces of an f32 weight, or one that is it exactly
+//
+// The same piece products in the same order as the piece form of k_gemm_umma.cu (UmmaEpilogue::seg_blocks): 64 k at a
+// time in one accumulator, the blocks added in f32 registers.  There the pieces are a matrix of their own, made by a
+// launch of its own (six bytes written for four read, read back twice over), and every piece product loads both its
+// tiles anew: 6 x (16 + 32) KB per 64 k of a 128 x 256 tile.  Here 32 KB of f32 and each piece of B once: what a small
+// product (4096 x 256 x 256 of an f32 decoder, 4096 x 768 x 768 of an int8 one) waited for.
+//
+// One CTA a tile (or a cluster of `splits`, each a part of K): warp 0 brings B by TMA, warp 1 issues tcgen05.mma, and
+// sixteen working warps do the rest in turn, a block of 64 k at a time: cut block k (its f32 already in registers) into
+// the ring, ask for block k + 1, add the accumulator of block k - 1 into their registers while the tensor core
+// multiplies block k.  Then the tile goes through the ring's memory and leaves as whole rows.
+//
+// Every wait on an mbarrier is bounded; one that runs out raises DeviceStatus::wait_timeout and the CTA stores nothing.
+#include <cuda.h>
+
+#include <algorithm>
+#include <atomic>
+#include <type_traits>
+
+#include "lora_split.cuh"
+#include "umma_device.cuh"
+#include "umma_epilogue.cuh"
+#include "umma_kernel.h"
+
+namespace see::k {
+
+namespace {
+
+using namespace umma_dev;
+using namespace umma_epi;
+
+constexpr uint32_t kBlockM = umma_cfg::kBlockM, kBlockK = umma_cfg::kBlockK;
+constexpr uint32_t kPieceBytes = kBlockM * kBlockK * 2;   // one bf16 piece of a block of A
+constexpr uint32_t kWorkWarps = 16, kWorkThreads = 32 * kWorkWarps, kCutThreads = 64 + kWorkThreads;
+constexpr uint32_t kMaxStages = 3;
+
+template <uint32_t kTN, uint32_t kBPieces>
+struct CutShape {
+  static constexpr uint32_t kBBytes = kTN * kBlockK * 2;   // one piece of a block of B
+  static constexpr uint32_t kStageBytes = 3 * kPieceBytes + kBPieces * kBBytes;
+  static constexpr uint32_t kFit = 216u * 1024u / kStageBytes;
+  static constexpr uint32_t kStages = kFit < kMaxStages ? kFit : kMaxStages;
+  static constexpr uint32_t kAccCols = kTN <= 64 ? 64 : (kTN <= 128 ? 128 : 256);
+  static constexpr uint32_t kColsPerWarp = kTN / 4;        // a warp's share of a tile: 32 rows x a quarter of the columns
+  static constexpr size_t kSmem = kStages * kStageBytes + 512 + 1024;
+  static_assert(kStages >= 1 && kStages * kStageBytes >= kBlockM * kTN * 4, "the epilogue stages the whole tile in the ring");
+};
+
+struct __align__(8) CutBarriers {
+  uint64_t a_full[kMaxStages], b_full[kMaxStages], empty[kMaxStages];
+  uint64_t tmem_full[2], tmem_empty[2];
+  uint32_t tmem_base;
+  volatile uint32_t abort;
+  volatile uint32_t nonfinite;
+};
+
+// Sixteen of the 128 x 64 f32 elements of block kb: rows r and r + 4 of the warp's eight, eight columns of each.
+struct CutRegs { float4 v[4]; };
+__device__ __forceinline__ void FetchBlock(CutRegs* f, const UmmaEpilogue& ep, uint32_t m0, uint32_t kb, bool vec) {
+  const uint32_t work = (threadIdx.x - 64) >> 5, lane = threadIdx.x & 31;
+  const uint32_t k = kb * kBlockK + (lane & 7) * 8;
+#pragma unroll
+  for (uint32_t h = 0; h < 2; ++h) {
+    const uint32_t row = m0 + work * 8 + h * 4 + (lane >> 3);
+    const float* p = ep.src_a + static_cast<size_t>(row) * ep.src_k + k;
+#pragma unroll
+    for (uint32_t q = 0; q < 2; ++q) {
+      const uint32_t c = k + 4 * q;
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row < ep.M && c < ep.src_k) {
+        if (vec) {   // src_k % 4 == 0: four elements are all in or all out
+          x = __ldg(reinterpret_cast<const float4*>(p + 4 * q));
+        } else {
+          x.x = p[4 * q];
+          if (c + 1 < ep.src_k) x.y = p[4 * q + 1];
+          if (c + 2 < ep.src_k) x.z = p[4 * q + 2];
+          if (c + 3 < ep.src_k) x.w = p[4 * q + 3];
+        }
+        if (ep.src_a_scale) {
+          x.x = x.x * ep.src_a_scale[c];
+          if (c + 1 < ep.src_k) x.y = x.y * ep.src_a_scale[c + 1];
+          if (c + 2 < ep.src_k) x.z = x.z * ep.src_a_scale[c + 2];
+          if (c + 3 < ep.src_k) x.w = x.w * ep.src_a_scale[c + 3];
+        }
+      }
+      f->v[2 * h + q] = x;
+    }
+  }
+}
+// Two elements' pieces, packed (Split3's values).
+__device__ __forceinline__ void CutPair(float lo, float hi, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    p[i] = PackBf16x2(lo, hi);
+    lo = lo - __uint_as_float(p[i] << 16);
+    hi = hi - __uint_as_float(p[i] & 0xFFFF0000u);
+  }
+}
+__device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs& f) {
+  const uint32_t work = (threadIdx.x - 64) >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (uint32_t h = 0; h < 2; ++h) {
+    uint32_t w[3][4];
+#pragma unroll
+    for (uint32_t q = 0; q < 2; ++q) {
+      const float4 x = f.v[2 * h + q];
+      uint32_t a[3], b[3];
+      CutPair(x.x, x.y, a);
+      CutPair(x.z, x.w, b);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) { w[i][2 * q] = a[i]; w[i][2 * q + 1] = b[i]; }
+    }
+    const uint32_t at = Sw128Offset(work * 8 + h * 4 + (lane >> 3), lane & 7);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      *reinterpret_cast<uint4*>(pieces + i * kPieceBytes + at) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+  }
+}
+
+template <uint32_t kTN, uint32_t kBPieces>
+__global__ void __launch_bounds__(kCutThreads, 1)
+UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ UmmaEpilogue ep, uint32_t splits) {
+  using Sh = CutShape<kTN, kBPieces>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (SmemAddr(smem_raw) & 1023u)) & 1023u);
+  CutBarriers* bars = reinterpret_cast<CutBarriers*>(smem + Sh::kStages * Sh::kStageBytes);
+
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t split = ClusterCtaRank();   // (a cluster is one tile's splits)
+  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, tile = blockIdx.x / splits;
+  const uint32_t mb = tile / tiles_n, nb = tile - mb * tiles_n;
+  const uint32_t m0 = mb * kBlockM, n0 = nb * kTN;
+  const uint32_t groups = (ep.src_k + kBlockK - 1) / kBlockK;   // an accumulator each
+  const uint32_t g0 = groups * split / splits, g1 = groups * (split + 1) / splits;
+
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < Sh::kStages; ++s) {
+      MbarInit(&bars->a_full[s], kWorkWarps);
+      MbarInit(&bars->b_full[s], 1);
+      MbarInit(&bars->empty[s], 1);
+    }
+    for (uint32_t b = 0; b < 2; ++b) {
+      MbarInit(&bars->tmem_full[b], 1);
+      MbarInit(&bars->tmem_empty[b], kWorkWarps);
+    }
+    bars->abort = 0;
+    bars->nonfinite = 0;
+    MbarInitFence();
+  }
+  if (warp == 1) TmemAlloc(&bars->tmem_base, 2 * Sh::kAccCols);
+  TcFenceBefore();
+  __syncthreads();
+  TcFenceAfter();
+  const uint32_t tmem_base = bars->tmem_base;
+  auto give_up = [&] { ep.status->wait_timeout = 1; bars->abort = 1; };
+
+  const bool work = warp >= 2;
+  const uint32_t wt = threadIdx.x - 64;
+  constexpr uint32_t kChunks = kTN / 4;
+  const uint32_t rows = kBlockM / splits, r0 = split * rows;   // the rows this CTA stores
+  bool ok = true;
+  if (warp == 0) {
+    // ---- B ----
+    if (lane == 0)
+      for (uint32_t g = g0, it = 0; g < g1; ++g, ++it) {
+        const uint32_t s = it % Sh::kStages, round = it / Sh::kStages;
+        if (round > 0 && !MbarWait(&bars->empty[s], (round - 1) & 1)) { give_up(); break; }
+        uint8_t* b = smem + s * Sh::kStageBytes + 3 * kPieceBytes;
+        MbarExpectTx(&bars->b_full[s], kBPieces * Sh::kBBytes);
+#pragma unroll
+        for (uint32_t p = 0; p < kBPieces; ++p)
+          TmaLoad2D(b + p * Sh::kBBytes, &map_b, &bars->b_full[s], static_cast<int32_t>((p * groups + g) * kBlockK),
+                    static_cast<int32_t>(n0));
+      }
+  } else if (warp == 1) {
+    // ---- products: small ones first, for the tensor core truncates toward zero at the accumulator's magnitude ----
+    if (ElectOne()) {
+      const uint32_t idesc = MakeInstrDesc(kBlockM, kTN);
+      for (uint32_t g = g0, it = 0; g < g1; ++g, ++it) {
+        const uint32_t s = it % Sh::kStages, parity = (it / Sh::kStages) & 1, buf = it & 1, use = it >> 1;
+        if ((use > 0 && !MbarWait(&bars->tmem_empty[buf], (use - 1) & 1)) || !MbarWait(&bars->b_full[s], parity) ||
+            !MbarWait(&bars->a_full[s], parity)) {
+          give_up();
+          break;
+        }
+        TcFenceAfter();
+        const uint32_t acc = tmem_base + buf * Sh::kAccCols, a = SmemAddr(smem + s * Sh::kStageBytes), b = a + 3 * kPieceBytes;
+        auto product = [&](uint32_t pa, uint32_t pb, bool first) {
+          const uint64_t da = MakeSmemDesc(a + pa * kPieceBytes), db = MakeSmemDesc(b + pb * Sh::kBBytes);
+#pragma unroll
+          for (uint32_t k = 0; k < 4; ++k) UmmaBf16(acc, da + 2 * k, db + 2 * k, idesc, first && k == 0 ? 0u : 1u);
+        };
+        if constexpr (kBPieces == 3) {
+          product(2, 0, true);
+          product(1, 1, false);
+          product(0, 2, false);
+          product(1, 0, false);
+          product(0, 1, false);
+          product(0, 0, false);
+        } else {
+          product(2, 0, true);
+          product(1, 0, false);
+          product(0, 0, false);
+        }
+        UmmaCommit(&bars->empty[s]);
+        UmmaCommit(&bars->tmem_full[buf]);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---- cut, and add ----
+    const uint32_t quarter = warp & 3, columns = ((warp - 2) >> 2) * Sh::kColsPerWarp;
+    const uint32_t t_row = tmem_base + ((quarter * 32) << 16) + columns;
+    const bool vec = (ep.src_k & 3u) == 0 && (reinterpret_cast<uintptr_t>(ep.src_a) & 15) == 0;
+    float sum[Sh::kColsPerWarp];
+#pragma unroll
+    for (uint32_t j = 0; j < Sh::kColsPerWarp; ++j) sum[j] = 0.0f;
+    auto add = [&](uint32_t it) {   // the accumulator of this CTA's group number `it`
+      const uint32_t buf = it & 1;
+      bool there = MbarWait(&bars->tmem_full[buf], (it >> 1) & 1);
+      if (!there && lane == 0) give_up();
+      if (bars->abort) there = false;
+      there = __all_sync(0xFFFFFFFFu, there);
+      TcFenceAfter();
+      if (!there) return false;
+#pragma unroll
+      for (uint32_t c = 0; c < Sh::kColsPerWarp; c += 16) {
+        uint32_t r[16];
+        TmemLoad16(t_row + buf * Sh::kAccCols + c, r);
+        TmemWaitLd();
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) sum[c + j] += __uint_as_float(r[j]);
+      }
+      TcFenceBefore();
+      __syncwarp();
+      if (lane == 0) MbarArrive(&bars->tmem_empty[buf]);
+      return true;
+    };
+    CutRegs f;
+    FetchBlock(&f, ep, m0, g0, vec);
+    for (uint32_t g = g0, it = 0; g < g1 && ok; ++g, ++it) {
+      const uint32_t s = it % Sh::kStages, round = it / Sh::kStages;
+      bool free = round == 0 || MbarWait(&bars->empty[s], (round - 1) & 1);
+      if (!free && lane == 0) give_up();
+      if (bars->abort) free = false;
+      if (!(ok = __all_sync(0xFFFFFFFFu, free))) break;
+      StoreBlock(smem + s * Sh::kStageBytes, f);
+      if (g + 1 < g1) FetchBlock(&f, ep, m0, g + 1, vec);
+      FenceProxyAsync();
+      __syncwarp();
+      if (lane == 0) MbarArrive(&bars->a_full[s]);
+      if (it > 0) ok = add(it - 1);
+    }
+    if (ok && g1 > g0) ok = add(g1 - g0 - 1);
+    if (ok) {
+      // All products are complete, so the ring is free: the tile goes there as [128][kTN] f32, 16-byte chunks XOR-ed
+      // with the row so that neither side conflicts.
+      if (!AllFinite(sum)) bars->nonfinite = 1;
+      float* dump = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kTN;
+#pragma unroll
+      for (uint32_t q = 0; q < Sh::kColsPerWarp / 4; ++q)
+        *reinterpret_cast<float4*>(dump + (((columns >> 2) + q) ^ (lane & 7u)) * 4) =
+            make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
+    }
+    TcFenceBefore();
+  }
+  if (splits > 1) ClusterSync();
+  else if (work) asm volatile("bar.sync 1, %0;" ::"n"(kWorkThreads) : "memory");
+  if (work && ok) {
+    const uint32_t dump = SmemAddr(smem);
+    auto element = [&](uint32_t lr, uint32_t chunk) {
+      const uint32_t off = (lr * kTN + (chunk ^ (lr & 7u)) * 4) * 4;
+      if (splits == 1) return *reinterpret_cast<const float4*>(smem + off);
+      float4 acc = LoadClusterF4(MapToCta(dump + off, 0));
+      for (uint32_t p = 1; p < splits; ++p) {
+        const float4 v = LoadClusterF4(MapToCta(dump + off, p));
+        acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+      }
+      return acc;
+    };
+    bool remake = false;   // (an element's splits lie in several CTAs)
+    for (uint32_t p = 0; p < splits; ++p)
+      remake = remake || (splits == 1 ? bars->nonfinite : LoadClusterU32(MapToCta(SmemAddr(const_cast<uint32_t*>(&bars->nonfinite)), p))) != 0;
+    const bool ragged = (ep.N & 3u) != 0, plain = IsPlainStore(ep);
+    for (uint32_t i = wt; i < rows * kChunks; i += kWorkThreads) {
+      const uint32_t lr = r0 + i / kChunks, chunk = i % kChunks, row = m0 + lr, n = n0 + chunk * 4;
+      if (row >= ep.M || n >= ep.N) continue;
+      const float4 acc = element(lr, chunk);
+      if (remake) { StoreRemade(ep, row, n, acc); continue; }
+      if (ragged) { EpilogueStoreRagged(ep, row, n, acc, false); continue; }
+      float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
+      if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
+      const size_t at = static_cast<size_t>(row) * ep.N + n;
+      if (plain) {
+        EpilogueStorePlain(ep, at, acc, scale);
+      } else {
+        const float4 bias = ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        EpilogueStore(ep, at, n, acc, scale, bias);
+      }
+    }
+  }
+
+  TcFenceBefore();
+  __syncthreads();
+  if (bars->abort) DrainDelay();
+  if (splits > 1) ClusterSync();   // no CTA leaves while another may still read its memories
+  if (warp == 1) {
+    TcFenceAfter();
+    TmemFree(tmem_base, 2 * Sh::kAccCols);
+  }
+}
+
+template <uint32_t kTN, uint32_t kBPieces>
+cudaError_t Launch(const UmmaCutPlan& plan, const CUtensorMap& map_b, const UmmaEpilogue& ep, cudaStream_t s) {
+  auto kernel = UmmaGemmCutKernel<kTN, kBPieces>;
+  constexpr size_t kSmem = CutShape<kTN, kBPieces>::kSmem;
+  static std::atomic<bool> configured[64] = {};   // (a per-device setting of the function)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)); e != cudaSuccess)
+      return e;
+    if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(plan.grid);
+  cfg.blockDim = dim3(kCutThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = plan.splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = plan.splits > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, map_b, ep, plan.splits);
+}
+
+}  // namespace
+
+UmmaCutPlan UmmaPlanCut(uint32_t M, uint32_t N, uint32_t groups, bool exact_b, uint32_t sms) {
+  // One round of CTAs only, and for an f32 weight at most sixteen blocks of 64 k: beyond that the working warps, which
+  // take about 1.2 us to cut a block and add one (1.4 at a tile width of 128 or 192), fall behind the piece form's
+  // tensor time, and every further column tile cuts A again.  Measured on a B200, the piece form's kernel (+ its cut of A) / this,
+  // us, f32 weights: 4096 x 256 x 256 14.0 (+2.8) / 9.7, 1024 x 256 x 256 8.4 (+2.0) / 8.0, 600 x 512 x 512 12.3 (+2.1) / 10.7,
+  // 128 x 1024 x 1024 14.7 (+2.0) / 11.1, 300 x 5000 x 256 15.1 (+1.9) / 11.8, 4096 x 256 x 1024 21.7 (+5.9) / 23.6; past the line
+  // 2048 x 512 x 2048 32.1 (+5.9) / 42.0, 4096 x 1024 x 256 18.8 (+2.7) / 22.4, 4096 x 4096 x 256 57.9 (+4.0) / 77.1; int8 weights:
+  // 4096 x 768 x 768 24.5 (+4.8) / 23.6, 4096 x 768 x 3072 71.1 (+19.4) / 68.0, 2048 x 512 x 2048 22.3 (+5.9) / 25.0; past it 4096 x
+  // 3072 x 768 67.3 (+6.1) / 87.9.
+  UmmaCutPlan best;
+  if (!exact_b && groups > 16) return best;
+  double least = 1e30;
+  const uint32_t tiles_m = (M + kBlockM - 1) / kBlockM;
+  for (uint32_t tn : {64u, 128u, 192u}) {
+    if (!exact_b && tn > 128) continue;   // (a block of three 192-wide pieces leaves room for one stage)
+    for (uint32_t splits = 1; splits <= 4 && splits <= groups; splits *= 2) {
+      const uint64_t ctas = static_cast<uint64_t>(tiles_m) * ((N + tn - 1) / tn) * splits;
+      if (ctas > (splits <= 2 ? sms : sms * 9 / 10)) continue;   // clusters of four do not fill every GPC
+      const double group = exact_b ? 1.1 + 0.001 * tn : 0.9 + 0.004 * tn;
+      const double t = group * ((groups + splits - 1) / splits) + 0.015 * tn / splits + (splits > 1 ? 2.0 : 0.0);
+      if (t < least) {
+        least = t;
+        best = {tn, splits, static_cast<uint32_t>(ctas)};
+      }
+    }
+  }
+  return best;
+}
+
+cudaError_t UmmaCutLaunch(const UmmaCutPlan& plan, bool exact_b, const CUtensorMap& map_b, const UmmaEpilogue& ep, cudaStream_t s) {
+  if (exact_b) {
+    switch (plan.tn) {
+      case 64: return Launch<64, 1>(plan, map_b, ep, s);
+      case 128: return Launch<128, 1>(plan, map_b, ep, s);
+      default: return Launch<192, 1>(plan, map_b, ep, s);
+    }
+  }
+  return plan.tn == 64 ? Launch<64, 3>(plan, map_b, ep, s) : Launch<128, 3>(plan, map_b, ep, s);
+}
+
+}  // namespace see::k

@@ -533,9 +533,22 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   const bool exact_b = a.b_type != k::BType::kF32;
   if (exact_b && !ExactWeightFits(a.K, b_space == 0)) return {};
   const uint64_t Kp = PaddedK(a.K);
+  const uint32_t segments = exact_b ? kSegExact : kSegF32;
+  const uint32_t k_blocks = static_cast<uint32_t>(segments * (Kp / 64));
+  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks, segments,
+                                                LightEpilogue(a), impl->sms);
+  auto& tag = impl->split_tag;
+  const bool have_pieces = tag.valid && a_space == 0 && tag.off == a_off && tag.M == a.M && tag.K == a.K &&
+                           tag.transposed == a.a_transposed && tag.k_scale == a.a_k_scale;
+  // Where A lies row by row and the product is small its pieces need no matrix of their own.
+  const k::UmmaCutPlan cut = k::UmmaPlanCut(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N),
+                                            static_cast<uint32_t>(Kp / 64), exact_b, impl->sms);
+  const bool cuts = !a.a_transposed && cut.grid != 0;
   // No memory for a copy or for pieces: the product stays on the CUDA cores, which need neither.
-  if (a.M * 3 * Kp > impl->split_a_capacity) impl->split_tag.valid = false;
-  if (!RoomFor(impl, &impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream)) return {};
+  if (!cuts) {
+    if (a.M * 3 * Kp > impl->split_a_capacity) impl->split_tag.valid = false;
+    if (!RoomFor(impl, &impl->split_a, &impl->split_a_capacity, a.M * 3 * Kp, stream)) return {};
+  }
   // B: wanted as [N][K]; stored [N, K] (NT) or [K, N] (NN, TN).
   uint16_t* b = nullptr;
   if (b_space != 0) {   // frozen: once per binding
@@ -562,27 +575,11 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
     k::SplitMatrix(static_cast<const float*>(a.B), b, a.N, a.K, !a.b_transposed, nullptr, stream);
     ++*launches;
   }
-  // A: [M, K], or [K, M] for the transposed-A form.
-  auto& tag = impl->split_tag;
-  if (!(tag.valid && a_space == 0 && tag.off == a_off && tag.M == a.M && tag.K == a.K && tag.transposed == a.a_transposed &&
-        tag.k_scale == a.a_k_scale)) {
+  if (!cuts && !have_pieces) {   // A: [M, K], or [K, M] for the transposed-A form
     k::SplitMatrix(a.A, impl->split_a, a.M, a.K, a.a_transposed, a.a_k_scale, stream);
     ++*launches;
     tag.valid = a_space == 0;
     tag.off = a_off; tag.M = a.M; tag.K = a.K; tag.transposed = a.a_transposed; tag.k_scale = a.a_k_scale;
-  }
-  const uint32_t segments = exact_b ? kSegExact : kSegF32;
-  const uint32_t k_blocks = static_cast<uint32_t>(segments * (Kp / 64));
-  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), k_blocks, segments,
-                                                LightEpilogue(a), impl->sms);
-  k::UmmaMaps maps;
-  // An exact weight is [N][K]: past K its last block reads zeros, and so do A's padding columns.
-  if (!EncodeBf16Map(impl, &maps.a[0], impl->split_a, a.M, 3 * Kp, k::umma_cfg::kBlockM) ||
-      !EncodeBf16Map(impl, &maps.b[0], b, a.N, exact_b ? a.K : 3 * Kp, plan.b_box))
-    return "tensor-core path: cuTensorMapEncodeTiled refused the operand-piece layout";
-  for (uint32_t p = 0; p < k::kUmmaProducts; ++p) {   // (never read: valid descriptors)
-    maps.a[p] = maps.a2[p] = maps.a[0];
-    maps.b[p] = maps.b2[p] = maps.b[0];
   }
   k::UmmaEpilogue ep{};
   ep.C = a.C;
@@ -606,9 +603,26 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   ep.seg_a = exact_b ? kSegAExact : kSegAF32;
   ep.seg_b = exact_b ? kSegBExact : kSegBF32;
   ep.status = impl->status;
+  cudaError_t launched = cudaSuccess;
   if (impl->prof_before) cudaEventRecord(impl->prof_before, stream);
-  if (cudaError_t e = k::UmmaGemmLaunch(plan, maps, ep, stream); e != cudaSuccess)
-    return std::string("tensor-core GEMM launch: ") + cudaGetErrorString(e);
+  if (cuts) {
+    CUtensorMap map_b;
+    if (!EncodeBf16Map(impl, &map_b, b, a.N, exact_b ? a.K : 3 * Kp, cut.tn))
+      return "tensor-core path: cuTensorMapEncodeTiled refused the operand-piece layout";
+    launched = k::UmmaCutLaunch(cut, exact_b, map_b, ep, stream);
+  } else {
+    k::UmmaMaps maps;
+    // An exact weight is [N][K]: past K its last block reads zeros, and so do A's padding columns.
+    if (!EncodeBf16Map(impl, &maps.a[0], impl->split_a, a.M, 3 * Kp, k::umma_cfg::kBlockM) ||
+        !EncodeBf16Map(impl, &maps.b[0], b, a.N, exact_b ? a.K : 3 * Kp, plan.b_box))
+      return "tensor-core path: cuTensorMapEncodeTiled refused the operand-piece layout";
+    for (uint32_t p = 0; p < k::kUmmaProducts; ++p) {   // (never read: valid descriptors)
+      maps.a[p] = maps.a2[p] = maps.a[0];
+      maps.b[p] = maps.b2[p] = maps.b[0];
+    }
+    launched = k::UmmaGemmLaunch(plan, maps, ep, stream);
+  }
+  if (launched != cudaSuccess) return std::string("tensor-core GEMM launch: ") + cudaGetErrorString(launched);
   if (impl->prof_after) {
     cudaEventRecord(impl->prof_after, stream);
     impl->prof_used = true;

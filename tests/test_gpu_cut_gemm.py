@@ -1,0 +1,76 @@
+"""Exact products whose activation is cut into bf16 pieces inside the kernel (a single round of tiles, A row by row):
+edges of the 128-row tiles, the column tiles and the 64-wide blocks of K, reductions shared by a cluster, ragged widths,
+rows of A off the 16-byte grid's multiples, every weight type and epilogue, and operands that are not finite."""
+
+import numpy as np
+import pytest
+
+from see_ai_b200 import backend as B
+from see_ai_b200 import plan as P
+from tests.test_oracle_pinned import Arena
+
+pytestmark = pytest.mark.gpu
+Op = P.Op
+
+
+def _run(prog, arena0, ro, mode):
+    arena = arena0.copy()
+    be = B.CudaBackend(0)
+    be.set_coherence(B.COHERENCE_LAZY)
+    be.set_split_gemm(mode)
+    be.bind(arena, ro)
+    be.run(prog)
+    be.host_needs(0, arena.size)
+    be.flush()
+    taken = be.counters().split_executions
+    be.close()
+    return arena, taken
+
+
+SHAPES = [(1023, 256, 256), (4096, 256, 256), (129, 1024, 1021), (640, 514, 320), (300, 5000, 256), (4096, 192, 1000), (2000, 385, 96)]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
+@pytest.mark.parametrize("bad", [False, True], ids=["finite", "infinite"])
+def test_against_double(shape, bad):
+    M, N, K = shape
+    rng = np.random.default_rng(M + N + K)
+    a = Arena(rng)
+    x = a.alloc(M * K, "normal"); d = a.alloc(M * N, "normal")
+    w = rng.standard_normal(K * N).astype(np.float32)
+    q = rng.integers(-127, 128, size=K * N, dtype=np.int8)
+    rw, rq = a.ro_alloc(w), a.ro_alloc(q)
+    sc, ks = (rng.random(N) * 0.01 + 1e-3).astype(np.float32), (rng.random(K) * 0.01 + 1e-3).astype(np.float32)
+    rs, rk = a.ro_alloc(sc), a.ro_alloc(ks)
+    bias = rng.standard_normal(N).astype(np.float32)
+    rb = a.ro_alloc(bias)
+    outs = [a.alloc(M * N) for _ in range(4)]
+    dims, f = (M, N, K), P.f32_bits
+    prog = [
+        P.Instr(Op.GEMM_NN, P.FLAG_EPILOGUE_BIAS | (P.ACT_RELU << 1), f(0.5), (x, rw, outs[0], rb), dims),
+        P.Instr(Op.GEMM_NT, P.FLAG_GEMM_ADDEND, f(2.0), (x, rw, outs[1], d), dims),
+        P.Instr(Op.GEMM_NN_Q8, P.FLAG_Q8_COL_SCALE, 0, (x, rq, outs[2], rs), dims),
+        P.Instr(Op.GEMM_NT_Q8, P.FLAG_Q8_COL_SCALE, 0, (x, rq, outs[3], rk), dims),
+    ]
+    arena, ro = a.build()
+    A = arena[x:x + 4 * M * K].view(np.float32).reshape(M, K)
+    if bad:
+        A[M // 2, K // 3] = np.inf
+    got, taken = _run(prog, arena, ro, -1)
+    assert taken >= 2
+    D = arena[d:d + 4 * M * N].view(np.float32).reshape(M, N).astype(np.float64)
+    A64 = A.astype(np.float64)
+    wn, wt, qn, qt = (m.astype(np.float64) for m in (w.reshape(K, N), w.reshape(N, K).T, q.reshape(K, N), q.reshape(N, K).T))
+    with np.errstate(invalid="ignore"):
+        want = [np.maximum(0.5 * (A64 @ wn) + bias, 0), D + 2.0 * (A64 @ wt), (A64 @ qn) * sc, (A64 * ks) @ qt]
+    for k, (off, ref) in enumerate(zip(outs, want)):
+        g = got[off:off + 4 * M * N].view(np.float32).reshape(M, N).astype(np.float64)
+        rows = np.ones(M, bool)
+        if bad:
+            rows[M // 2] = False
+            assert not np.isfinite(g[M // 2]).all()
+        # (1.5 + 0.3 sqrt(K / 64)) 2^-24 of the product's root mean square, eight times that at the worst element
+        rms = np.sqrt(np.mean(ref[rows] ** 2))
+        err = np.abs(g[rows] - ref[rows])
+        assert np.sqrt(np.mean(err ** 2)) <= 4e-7 * rms, k
+        assert err.max() <= 8e-6 * rms, k
