@@ -2600,7 +2600,7 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
     }
     case kAttnDP:
       k::AttnDP(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
-                Hi32(ins.out[1]), Lo32(ins.out[1]), s);
+                Hi32(ins.out[1]), Lo32(ins.out[1]), OwnOrder(), s);
       launched();
       break;
     case kAttnDV:

@@ -221,7 +221,9 @@ constexpr int kTile = 64;      // rows of the streamed axis per step
 constexpr int kSlice = 8;      // features of a streamed tile in shared memory at a time
 constexpr int kTileThreads = 256;
 constexpr int kGroup = 128;            // threads of a group
-constexpr int kStreamLd = kTile + 2;   // doubles per feature of a streamed slice (a multiple of 16 bytes; 2-way store conflicts)
+constexpr int kStreamLd = kTile + 4;   // doubles per feature of a streamed slice: a multiple of 16 bytes, and four features' rows
+                                       // in four different quarters of the banks, as the tensor instruction's fragments want them
+__host__ __device__ constexpr int OwnLd(int rows) { return rows + 4; }   // likewise of the block's own rows
 constexpr int kChunkRows = 32;         // rows of an f32 tile in shared memory at a time
 
 __host__ __device__ constexpr int PaddedFeatures(int d) { return (d + kSlice - 1) / kSlice * kSlice; }
@@ -232,17 +234,17 @@ __device__ __forceinline__ float4 LoadFour(const float* __restrict__ p, int left
   return make_float4(p[0], left > 1 ? p[1] : 0.0f, left > 2 ? p[2] : 0.0f, left > 3 ? p[3] : 0.0f);
 }
 
-// The block's own rows, widened to double once: dst[feature][kRows], zero outside (0 * 0 leaves a chain as it is).
+// The block's own rows, widened to double once: dst[feature][OwnLd(kRows)], zero outside (0 * 0 leaves a chain as it is).
 template <int kRows, bool kVec>
 __device__ __forceinline__ void LoadOwn(double* dst, const float* __restrict__ src, size_t stride, int rows, int d) {
   const int quads = PaddedFeatures(d) / 4;
   for (int t = threadIdx.x; t < kRows * quads; t += kTileThreads) {
     const int r = t / quads, c = t % quads * 4;
     const float4 f = LoadFour(src + static_cast<size_t>(min(r, rows - 1)) * stride + c, r < rows ? d - c : 0, kVec);
-    dst[c * kRows + r] = f.x;
-    dst[(c + 1) * kRows + r] = f.y;
-    dst[(c + 2) * kRows + r] = f.z;
-    dst[(c + 3) * kRows + r] = f.w;
+    dst[c * OwnLd(kRows) + r] = f.x;
+    dst[(c + 1) * OwnLd(kRows) + r] = f.y;
+    dst[(c + 2) * OwnLd(kRows) + r] = f.z;
+    dst[(c + 3) * OwnLd(kRows) + r] = f.w;
   }
 }
 
@@ -273,14 +275,42 @@ __device__ __forceinline__ void StoreSlice(double* dst, const SliceRegs& s) {
   dst[(c + 3) * kStreamLd + r] = s.v.w;
 }
 
-// acc[r][e] = own row (ty RM + r) . streamed row Col(e), in double, ascending features.  `regs` holds the tile's first
+// Which pair (row of the block's own, row of the streamed tile) a thread's accumulator acc[r][e] stands for; e and e + 1
+// (e even) are neighbours.  kMma: the fragments of the tensor instruction, a warp to 16 streamed rows; else the thread
+// grid of 8 x 16 (16 lanes read 256 contiguous bytes).
+template <bool kMma, int RM>
+__device__ __forceinline__ int RowAt(int r) {
+  return kMma ? r * 8 + static_cast<int>(threadIdx.x & 31) / 4 : (InGroup() >> 4) * RM + r;
+}
+template <bool kMma>
+__device__ __forceinline__ int Col(int e) {
+  return kMma ? (InGroup() >> 5) * 16 + (e >> 1) * 8 + 2 * static_cast<int>(threadIdx.x & 3) + (e & 1)
+              : 2 * static_cast<int>(threadIdx.x & 15) + (e & 1) + (e >> 1) * 32;
+}
+
+// c += a b in double: 16 x 8 += 16 x 8 . 8 x 8 (8 x 8 += 8 x 4 . 4 x 8).
+__device__ __forceinline__ void DMma16(double (&c0)[4], double (&c1)[4], int e, const double (&a)[4], const double (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+d"(c0[e]), "+d"(c0[e + 1]), "+d"(c1[e]), "+d"(c1[e + 1])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+__device__ __forceinline__ void DMma8(double (&c)[4], int e, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[e]), "+d"(c[e + 1]) : "d"(a), "d"(b));
+}
+
+// acc[r][e] = own row RowAt(r) . streamed row Col(e), in double.  `regs` holds the tile's first
 // slice on entry and the first slice of `next` (rows of the same stride; null: nothing) on exit, so that a global load is
 // always a whole slice of arithmetic ahead of its use.  `turn` alternates the two slice buffers: one barrier per slice.
-template <int RM, bool kVec>
+// kMma false: every accumulator one chain over ascending features, the CPU's.  kMma true (where the bits are not
+// observed): the FP64 tensor instruction, whose sums of eight are doubles all the same.  Both run at the FP64 pipe's
+// rate at best; a thread grid of RM x 4 pairs reads RM + 4 doubles of shared memory for 4 RM multiply-adds, the fragments
+// 2 RM + 4 for 64 RM of a warp's.
+template <int RM, bool kVec, bool kMma>
 __device__ __forceinline__ void DotTile(const double* own, const float* b, int rows, const float* next, int next_rows,
                                         size_t stride, int d, double* slices, int* turn, SliceRegs* regs,
                                         double (&acc)[RM][4]) {
-  constexpr int R = 8 * RM;
+  constexpr int R = 8 * RM, kLd = OwnLd(R);
   const int tx = threadIdx.x & 15, ty = InGroup() >> 4;
 #pragma unroll
   for (int r = 0; r < RM; ++r)
@@ -293,28 +323,53 @@ __device__ __forceinline__ void DotTile(const double* own, const float* b, int r
     GroupSync();
     if (c0 + kSlice < d) FetchSlice<kVec>(regs, b, stride, rows, c0 + kSlice, d);
     else if (next) FetchSlice<kVec>(regs, next, stride, next_rows, 0, d);
-    const double* sa = own + c0 * R + ty * RM;
+    if constexpr (kMma) {
+      const int g = static_cast<int>(threadIdx.x & 31) / 4, t = threadIdx.x & 3;
+      const double* sa = own + (c0 + t) * kLd + g;
+      const double* bb = sb + t * kStreamLd + (InGroup() >> 5) * 16 + g;
+      double y[2][2];
 #pragma unroll
-    for (int c = 0; c < kSlice; ++c) {
-      const double2 y0 = *reinterpret_cast<const double2*>(sb + c * kStreamLd + 2 * tx);
-      const double2 y1 = *reinterpret_cast<const double2*>(sb + c * kStreamLd + 32 + 2 * tx);
-      const double y[4] = {y0.x, y0.y, y1.x, y1.y};
-      double x[RM];
+      for (int n = 0; n < 2; ++n) {
+        y[n][0] = bb[8 * n];
+        y[n][1] = bb[4 * kStreamLd + 8 * n];
+      }
+      if constexpr (RM == 1) {
+        const double x0 = sa[0], x1 = sa[4 * kLd];
 #pragma unroll
-      for (int r = 0; r < RM; ++r) x[r] = sa[c * R + r];
+        for (int n = 0; n < 2; ++n) {
+          DMma8(acc[0], 2 * n, x0, y[n][0]);
+          DMma8(acc[0], 2 * n, x1, y[n][1]);
+        }
+      } else {
 #pragma unroll
-      for (int r = 0; r < RM; ++r)
+        for (int m = 0; m + 1 < RM; m += 2) {
+          const double x[4] = {sa[8 * m], sa[8 * m + 8], sa[4 * kLd + 8 * m], sa[4 * kLd + 8 * m + 8]};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[r][e] = fma(x[r], y[e], acc[r][e]);
+          for (int n = 0; n < 2; ++n) DMma16(acc[m], acc[m + 1], 2 * n, x, y[n]);
+        }
+      }
+    } else {
+      const double* sa = own + c0 * kLd + ty * RM;
+#pragma unroll
+      for (int c = 0; c < kSlice; ++c) {
+        const double2 y0 = *reinterpret_cast<const double2*>(sb + c * kStreamLd + 2 * tx);
+        const double2 y1 = *reinterpret_cast<const double2*>(sb + c * kStreamLd + 32 + 2 * tx);
+        const double y[4] = {y0.x, y0.y, y1.x, y1.y};
+        double x[RM];
+#pragma unroll
+        for (int r = 0; r < RM; ++r) x[r] = sa[c * kLd + r];
+#pragma unroll
+        for (int r = 0; r < RM; ++r)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[r][e] = fma(x[r], y[e], acc[r][e]);
+      }
     }
   }
 }
-// The tile row a thread's accumulator e stands for (pairs, so that 16 lanes read 256 contiguous bytes).
-__device__ __forceinline__ int Col(int e) { return 2 * static_cast<int>(threadIdx.x & 15) + (e & 1) + (e >> 1) * 32; }
 
 __host__ __device__ constexpr size_t GroupBytes() { return 2 * sizeof(double) * kSlice * kStreamLd; }
 __host__ __device__ constexpr size_t StreamBytes() { return 2 * GroupBytes(); }
-__host__ __device__ constexpr size_t OwnBytes(int RM, int d) { return sizeof(double) * PaddedFeatures(d) * 8 * RM; }
+__host__ __device__ constexpr size_t OwnBytes(int RM, int d) { return sizeof(double) * PaddedFeatures(d) * OwnLd(8 * RM); }
 
 // Rows [0, rows) x columns [c0, c0 + 64) of a [., stride] f32 matrix into dst[32][64] by asynchronous copies (zero
 // outside); one commit group.
@@ -440,7 +495,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnFwdTileKernel(
   const int i0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const int nrows = min(R, S - i0), nkeys = min(i0 + R, S);
-  const int ty = InGroup() >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t base = b * S * D + h * d;
   auto first_key = [&](int i) {
     if (!starts) return 0;
@@ -456,13 +511,13 @@ __global__ __launch_bounds__(kTileThreads) void AttnFwdTileKernel(
   for (int k0 = first; k0 < nkeys; k0 += 2 * kTile) {
     double acc[RM][4];
     const float* kb = k + base + static_cast<size_t>(k0) * D;
-    DotTile<RM, kVec>(own, kb, min(kTile, S - k0), k0 + 2 * kTile < nkeys ? kb + 2 * kTile * D : nullptr,
-                      min(kTile, S - k0 - 2 * kTile), D, d, slices, &turn, &regs, acc);
+    DotTile<RM, kVec, kFused>(own, kb, min(kTile, S - k0), k0 + 2 * kTile < nkeys ? kb + 2 * kTile * D : nullptr,
+                              min(kTile, S - k0 - 2 * kTile), D, d, slices, &turn, &regs, acc);
 #pragma unroll
     for (int r = 0; r < RM; ++r)
 #pragma unroll
       for (int e = 0; e < 4; e += 2)
-        *reinterpret_cast<float2*>(rows + (ty * RM + r) * ld + k0 + Col(e)) =
+        *reinterpret_cast<float2*>(rows + RowAt<kFused, RM>(r) * ld + k0 + Col<kFused>(e)) =
             make_float2(static_cast<float>(acc[r][e]) * inv_sqrt_d, static_cast<float>(acc[r][e + 1]) * inv_sqrt_d);
   }
   __syncthreads();
@@ -528,7 +583,7 @@ __global__ void AttnDPWideKernel(const float* __restrict__ dout, const float* __
 }
 
 // dP[i][j] = dO_i . v_j for j <= i, zero above the diagonal.  Block: 8 RM query rows, every key tile.
-template <int RM, bool kVec>
+template <int RM, bool kMma, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __restrict__ dout,
                                                                  const float* __restrict__ v, float* __restrict__ dp,
                                                                  int BH, int S, int H, int d) {
@@ -540,7 +595,6 @@ __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __
   const int i0 = tile.tile * R, nkeys = min(i0 + R, S);
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const size_t base = b * S * D + h * d;
-  const int ty = InGroup() >> 4;
   const bool pairs = (S & 1) == 0 && (reinterpret_cast<uintptr_t>(dp) & 7) == 0;   // (j is even: 8-byte stores)
   SliceRegs regs;
   int turn = 0;
@@ -552,17 +606,17 @@ __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __
     double acc[RM][4] = {};
     if (k0 < nkeys) {
       const float* vb = v + base + static_cast<size_t>(k0) * D;
-      DotTile<RM, kVec>(own, vb, min(kTile, S - k0), k0 + 2 * kTile < nkeys ? vb + 2 * kTile * D : nullptr,
-                        min(kTile, S - k0 - 2 * kTile), D, d, slices, &turn, &regs, acc);
+      DotTile<RM, kVec, kMma>(own, vb, min(kTile, S - k0), k0 + 2 * kTile < nkeys ? vb + 2 * kTile * D : nullptr,
+                              min(kTile, S - k0 - 2 * kTile), D, d, slices, &turn, &regs, acc);
     }
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
-      const int i = i0 + ty * RM + r;
+      const int i = i0 + RowAt<kMma, RM>(r);
       if (i >= S) continue;
       float* row = dp + (bh * S + i) * S;
 #pragma unroll
       for (int e = 0; e < 4; e += 2) {
-        const int j = k0 + Col(e);
+        const int j = k0 + Col<kMma>(e);
         const float x0 = j <= i ? static_cast<float>(acc[r][e]) : 0.0f;
         const float x1 = j + 1 <= i ? static_cast<float>(acc[r][e + 1]) : 0.0f;
         if (pairs && j + 1 < S) {
@@ -727,7 +781,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDQTiledTileKernel(
   const int i0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const int nrows = min(R, S - i0), nkeys = min(i0 + R, S);
-  const int ty = InGroup() >> 4, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t base = b * S * D + h * d, at = base + static_cast<size_t>(i0) * D;
   float* st = stats + (bh * S + i0) * kAttnStatsWidth;
   SliceRegs regs;
@@ -741,21 +795,21 @@ __global__ __launch_bounds__(kTileThreads) void AttnDQTiledTileKernel(
     const float *kb = k + base + static_cast<size_t>(k0) * D, *vb = v + base + static_cast<size_t>(k0) * D;
     const int rows = min(kTile, S - k0);
     double acc[RM][4];
-    DotTile<RM, kVec>(own_q, kb, rows, vb, rows, D, d, slices, &turn, &regs, acc);
+    DotTile<RM, kVec, kFused>(own_q, kb, rows, vb, rows, D, d, slices, &turn, &regs, acc);
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
-      const int row = min(ty * RM + r, nrows - 1);
+      const int row = min(RowAt<kFused, RM>(r), nrows - 1);
       const float m = st[row * kAttnStatsWidth], inv_denom = st[row * kAttnStatsWidth + 1];
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        prows[(ty * RM + r) * ld + k0 + Col(e)] = expf(static_cast<float>(acc[r][e]) * inv_sqrt_d - m) * inv_denom;
+        prows[RowAt<kFused, RM>(r) * ld + k0 + Col<kFused>(e)] = expf(static_cast<float>(acc[r][e]) * inv_sqrt_d - m) * inv_denom;
     }
-    DotTile<RM, kVec>(own_do, vb, rows, k0 + 2 * kTile < nkeys ? kb + 2 * kTile * D : nullptr, min(kTile, S - k0 - 2 * kTile), D, d,
+    DotTile<RM, kVec, kFused>(own_do, vb, rows, k0 + 2 * kTile < nkeys ? kb + 2 * kTile * D : nullptr, min(kTile, S - k0 - 2 * kTile), D, d,
                       slices, &turn, &regs, acc);
 #pragma unroll
     for (int r = 0; r < RM; ++r)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) dprows[(ty * RM + r) * ld + k0 + Col(e)] = static_cast<float>(acc[r][e]);
+      for (int e = 0; e < 4; ++e) dprows[RowAt<kFused, RM>(r) * ld + k0 + Col<kFused>(e)] = static_cast<float>(acc[r][e]);
   }
   __syncthreads();
   for (int r = warp; r < nrows; r += kTileThreads / 32) {
@@ -815,7 +869,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDKVTiledTileKernel(
   const int j0 = tile.tile * R;
   const size_t bh = tile.bh, b = bh / H, h = bh % H, D = static_cast<size_t>(H) * d;
   const size_t base = b * S * D + h * d, at = base + static_cast<size_t>(j0) * D;
-  const int c0 = blockIdx.y * kTile, ty = InGroup() >> 4, c = (threadIdx.x & 15) * 4;
+  const int c0 = blockIdx.y * kTile, c = (threadIdx.x & 15) * 4;
   const int nkeys = min(R, S - j0);
   const float* x = kWantDK ? q : dout;
   constexpr int OR = OutRows(RM);
@@ -842,19 +896,19 @@ __global__ __launch_bounds__(kTileThreads) void AttnDKVTiledTileKernel(
       const float* q_next = i0 + 2 * kTile < S ? q + iat + 2 * kTile * D : nullptr;
       const int next_rows = min(kTile, S - i0 - 2 * kTile);
       double sc[RM][4], dp[RM][4];
-      DotTile<RM, kVec>(own_k, q + iat, rows, kWantDK ? dout + iat : q_next, kWantDK ? rows : next_rows, D, d, slices, &turn,
+      DotTile<RM, kVec, kFused>(own_k, q + iat, rows, kWantDK ? dout + iat : q_next, kWantDK ? rows : next_rows, D, d, slices, &turn,
                         &regs, sc);
-      if (kWantDK) DotTile<RM, kVec>(own_v, dout + iat, rows, q_next, next_rows, D, d, slices, &turn, &regs, dp);
+      if (kWantDK) DotTile<RM, kVec, kFused>(own_v, dout + iat, rows, q_next, next_rows, D, d, slices, &turn, &regs, dp);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int i = i0 + Col(e);
+        const int i = i0 + Col<kFused>(e);
         const float* st = stats + (bh * S + min(i, S - 1)) * kAttnStatsWidth;
         const int start = static_cast<int>(StatsStart(st[3], static_cast<size_t>(i)));
         late = late || (i < S && start > j0);
-        if (ty == 0) first[group * kTile + Col(e)] = start;
+        if (RowAt<kFused, RM>(0) == 0) first[group * kTile + Col<kFused>(e)] = start;
 #pragma unroll
         for (int r = 0; r < RM; ++r) {
-          const int j = j0 + ty * RM + r;
+          const int j = j0 + RowAt<kFused, RM>(r);
           float g = 0.0f;
           if (i < S && j <= i && j >= start) {
             const float p = expf(static_cast<float>(sc[r][e]) * inv_sqrt_d - st[0]) * st[1];
@@ -865,7 +919,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDKVTiledTileKernel(
               g = p;
             }
           }
-          wt[(group * kTile + Col(e)) * kLd + ty * RM + r] = g;
+          wt[(group * kTile + Col<kFused>(e)) * kLd + RowAt<kFused, RM>(r)] = g;
         }
       }
     }
@@ -978,7 +1032,7 @@ void AttnFwd(const float* q, const float* k, const float* v, float* o, float* pr
                                                              starts, inv_sqrt_d);
 }
 
-void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d,
+void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, bool own_order,
             cudaStream_t s) {
   if (B * H * S == 0) return;
   auto bytes = [&](int rm) { return StreamBytes() + OwnBytes(rm, static_cast<int>(d)); };
@@ -988,10 +1042,10 @@ void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, si
     AttnDPWideKernel<<<148 * 8, 256, 0, s>>>(dout, v, dp, B * H, S, H, d);
     return;
   }
-  WithTile(rm, false, Vec(d, {dout, v}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
+  WithTile(rm, own_order, Vec(d, {dout, v}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
     constexpr int RM = decltype(rows)::value;
-    AllowSmem(AttnDPTileKernel<RM, decltype(vec)::value>, bytes(RM));
-    AttnDPTileKernel<RM, decltype(vec)::value>
+    AllowSmem(AttnDPTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, bytes(RM));
+    AttnDPTileKernel<RM, decltype(fu)::value, decltype(vec)::value>
         <<<static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes(RM), s>>>(
             dout, v, dp, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d));
   });

@@ -176,7 +176,7 @@ void SetScalars(const AdamScalars& v, AdamScalars* dst, cudaStream_t s);
 void AttnFwd(const float* q, const float* k, const float* v, float* o, float* probs,
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,
              bool fused, cudaStream_t s);  // probs != null: cached family; stats != null: tiled family
-void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d,
+void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, bool own_order,
             cudaStream_t s);
 void AttnDV(const float* probs, const float* dout, float* dv, size_t B, size_t S, size_t H,
             size_t d, bool fused, cudaStream_t s);
