@@ -29,6 +29,10 @@
 // operand: dA_chunk += x_chunk^T dT in the same accumulator columns, stored the same way.
 // The partial sums have the layout the fold kernel of k_lora_mma.cu adds up in block order.
 //
+// With few rows (two blocks for every tile fit the chip) a cluster of two works a tile, each block half of dY's and half of
+// x's columns: the halves of dT cross through the peer's shared memory and are added there, everything else is apart.
+// A 4096-row launch had 64 blocks on 148 SMs, twelve stages each one after the other: 20.3 us, 16.4 in pairs.
+//
 // Every wait is bounded: a wait that runs out raises the status flag, and the block
 // stops issuing work and frees its tensor memory.
 #include <cuda.h>
@@ -70,10 +74,14 @@ constexpr int kMaxChunks = (kTmemCols - 2 * kWide) / kWide;     // 8
 struct Bars {
   uint64_t raw_full[kRawStages], raw_empty[kRawStages], pc_full[kStages], pc_empty[kStages];
   uint64_t small_ready[2], dt_full[2], dt_free[2], acc_full, acc_free;
+  uint64_t peer_dt;   // the other half of dT has arrived in `exchange`
   uint32_t tmem_base;
   volatile uint32_t abort;
 };
-constexpr size_t kSmemBytes = 1024 + kRawStages * kRawBytes + kStages * kPieceBytes + 2 * kSmallBytes + sizeof(Bars);
+constexpr uint32_t kExchangeBytes = kRows * kR * 4;             // dT of a tile, f32
+constexpr size_t kSmemBytes =
+    1024 + kRawStages * kRawBytes + kStages * kPieceBytes + 2 * kSmallBytes + kExchangeBytes + sizeof(Bars);
+static_assert(kSmemBytes <= 227 * 1024, "shared memory of a block");
 
 constexpr uint32_t kInstrDescAMnMajor = 1u << 15;
 
@@ -97,6 +105,22 @@ __device__ __forceinline__ void LoadSummed(uint32_t taddr, float (&v)[kR]) {
 }
 __device__ __forceinline__ void MbarArrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemAddr(bar)) : "memory");
+}
+// A bounded wait for what a peer block of the cluster wrote here.
+__device__ __forceinline__ bool MbarWaitCluster(uint64_t* bar, uint32_t parity) {
+  const uint32_t addr = SmemAddr(bar);
+  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
 }
 // A descriptor whose start address lies `bytes` further on (the address field holds bytes / 16).
 __device__ __forceinline__ uint64_t Advance(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
@@ -139,18 +163,22 @@ __global__ void __launch_bounds__(kThreads, 1)
 LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_constant__ CUtensorMap map_x,
                        const __grid_constant__ CUtensorMap map_b, const float* __restrict__ t,
                        float* dt, float* __restrict__ partials, uint32_t M, uint32_t N, uint32_t K,
-                       float alpha_dt, uint16_t* __restrict__ pieces, uint32_t piece_cols, DeviceStatus* status) {
+                       float alpha_dt, uint16_t* __restrict__ pieces, uint32_t piece_cols, DeviceStatus* status,
+                       uint32_t halves) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (SmemAddr(smem_raw) & 1023u)) & 1023u);
   uint8_t* pc = smem;                                   // the pieces' ring first: its tiles want 1024-byte alignment
   uint8_t* small = pc + kStages * kPieceBytes;          // two buffers of the small operand's pieces
   uint8_t* raw = small + 2 * kSmallBytes;
-  Bars* bars = reinterpret_cast<Bars*>(raw + kRawStages * kRawBytes);
+  float* exchange = reinterpret_cast<float*>(raw + kRawStages * kRawBytes);
+  Bars* bars = reinterpret_cast<Bars*>(raw + kRawStages * kRawBytes + kExchangeBytes);
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t nc = N / kChunk, kc = K / kChunk;
+  // halves == 1: a block walks its tiles.  halves == 2: a cluster of two has one tile, a block half of its chunks.
+  const uint32_t half = halves == 2 ? ClusterCtaRank() : 0u, walker = blockIdx.x / halves, walkers = gridDim.x / halves;
+  const uint32_t nc = N / kChunk / halves, kc = K / kChunk / halves, n_first = half * nc, k_first = half * kc;
   const uint32_t tiles = (M + kRows - 1) / kRows;
-  const uint32_t mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;   // this block's tiles
+  const uint32_t mine = walker < tiles ? (tiles - walker + walkers - 1) / walkers : 0u;   // this block's tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kRawStages; ++s) {
@@ -168,12 +196,14 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
     }
     MbarInit(&bars->acc_full, 1);
     MbarInit(&bars->acc_free, kWorkerWarps);
+    MbarInit(&bars->peer_dt, 4);
     bars->abort = 0;
     MbarInitFence();
   }
   if (warp == 1) TmemAlloc(&bars->tmem_base, kTmemCols);
   TcFenceBefore();
   __syncthreads();
+  if (halves == 2) ClusterSync();   // the peer's barriers exist before anything signals them
   TcFenceAfter();
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_acc = tmem_base, tmem_dt = tmem_base + kWide * kMaxChunks;   // dT: two buffers of 48 columns
@@ -205,22 +235,22 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
         if (q >= total) return;
         const bool dy = q < first_walk;
         const uint32_t per = dy ? nc : kc, i = dy ? q : q - first_walk;
-        const uint32_t v = i / per, c = i - v * per;
+        const uint32_t v = i / per, c = i - v * per + (dy ? n_first : k_first);
         asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
                      ::"l"(reinterpret_cast<uint64_t>(dy ? &map_dy : &map_x)), "r"(static_cast<int32_t>(c * kChunk)),
-                       "r"(static_cast<int32_t>((blockIdx.x + v * gridDim.x) * kRows))
+                       "r"(static_cast<int32_t>((walker + v * walkers) * kRows))
                      : "memory");
       };
       for (uint32_t q = 0; q < kAhead; ++q) prefetch(q);
       for (uint32_t v = 0; v < mine && ok; ++v)
         for (uint32_t c = 0; c < nc && ok; ++c) {
           prefetch(it + kAhead);
-          stage(&map_dy, c, (blockIdx.x + v * gridDim.x) * kRows, true);
+          stage(&map_dy, n_first + c, (walker + v * walkers) * kRows, true);
         }
       for (uint32_t v = 0; v < mine && ok; ++v)
         for (uint32_t c = 0; c < kc && ok; ++c) {
           prefetch(it + kAhead);
-          stage(&map_x, c, (blockIdx.x + v * gridDim.x) * kRows, false);
+          stage(&map_x, k_first + c, (walker + v * walkers) * kRows, false);
         }
     }
   } else if (warp == 1) {
@@ -380,13 +410,39 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
       if (!MbarWait(&bars->dt_full[v & 1], (v >> 1) & 1)) { give_up(); return; }
       TcFenceAfter();
       if (w < 4) {   // one warp per lane quadrant: its lanes 0 .. 15 hold rows 16 quad .. 16 quad + 15
-        const uint32_t row0 = (blockIdx.x + v * gridDim.x) * kRows;
+        const uint32_t row0 = (walker + v * walkers) * kRows;
         float val[kR];
         LoadSummed(tmem_dt + (v & 1) * kWide + ((quad * 32u) << 16), val);
         const uint32_t r = quad * 16u + lane;
-        if (lane < 16 && row0 + r < M) {
+        float4* here = reinterpret_cast<float4*>(exchange + r * kR);
+        if (halves == 2) {   // this block's half of the sum to the peer, the peer's half from it
+          if (lane < 16) {
+            const uint32_t there = MapToCta(SmemAddr(here), half ^ 1u);
 #pragma unroll
-          for (int n = 0; n < kR; ++n) val[n] *= alpha_dt;
+            for (uint32_t q = 0; q < kR / 4; ++q)
+              asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(there + 16 * q), "f"(val[4 * q]),
+                           "f"(val[4 * q + 1]), "f"(val[4 * q + 2]), "f"(val[4 * q + 3]) : "memory");
+          }
+          __syncwarp();
+          if (lane == 0) MbarArriveCluster(MapToCta(SmemAddr(&bars->peer_dt), half ^ 1u));
+          const bool there = MbarWaitCluster(&bars->peer_dt, 0);
+          if (!__all_sync(0xFFFFFFFFu, there)) { give_up(); return; }
+          if (lane < 16) {
+#pragma unroll
+            for (int q = 0; q < kR / 4; ++q) {
+              const float4 o = here[q];
+              val[4 * q] += o.x; val[4 * q + 1] += o.y; val[4 * q + 2] += o.z; val[4 * q + 3] += o.w;
+            }
+          }
+        }
+#pragma unroll
+        for (int n = 0; n < kR; ++n) val[n] *= alpha_dt;
+        if (halves == 2 && lane < 16) {   // both blocks' walk over x takes it from here
+#pragma unroll
+          for (int q = 0; q < kR / 4; ++q)
+            here[q] = make_float4(val[4 * q], val[4 * q + 1], val[4 * q + 2], val[4 * q + 3]);
+        }
+        if (half == 0 && lane < 16 && row0 + r < M) {
           float4* dst = reinterpret_cast<float4*>(dt + static_cast<size_t>(row0 + r) * kR);
 #pragma unroll
           for (int q = 0; q < kR / 4; ++q)
@@ -417,11 +473,11 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
       if (lane == 0) MbarArrive(&bars->dt_free[v & 1]);
     };
     // The accumulator columns as this block's partial sums; `by_column`: [16][width] (dB), else [width][16] (dA).
-    auto store_partials = [&](float* out, uint32_t chunks, uint32_t width, bool by_column) {
+    auto store_partials = [&](float* out, uint32_t first, uint32_t chunks, uint32_t width, bool by_column) {
       for (uint32_t c = w >> 2; c < chunks; c += kWorkerWarps / 4) {   // the warps of a quadrant take chunks in turn
         float val[kR];
         LoadSummed(tmem_acc + kWide * c + ((quad * 32u) << 16), val);
-        const uint32_t f = c * kChunk + quad * 32u + lane;
+        const uint32_t f = (first + c) * kChunk + quad * 32u + lane;
         if (by_column) {
 #pragma unroll
           for (int n = 0; n < kR; ++n) out[static_cast<size_t>(n) * width + f] = val[n];
@@ -433,14 +489,14 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
         }
       }
     };
-    float* pb = partials + static_cast<size_t>(blockIdx.x) * (static_cast<size_t>(kR) * N + static_cast<size_t>(K) * kR);
+    float* pb = partials + static_cast<size_t>(walker) * (static_cast<size_t>(kR) * N + static_cast<size_t>(K) * kR);
     float* pa = pb + static_cast<size_t>(kR) * N;
 
     // ---- over dY ----
-    float4 ahead = mine > 0 ? small_load(t, blockIdx.x * kRows) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 ahead = mine > 0 ? small_load(t, walker * kRows) : make_float4(0.f, 0.f, 0.f, 0.f);
     for (uint32_t v = 0; v < mine && ok; ++v) {
       const float4 now = ahead;
-      if (v + 1 < mine) ahead = small_load(t, (blockIdx.x + (v + 1) * gridDim.x) * kRows);
+      if (v + 1 < mine) ahead = small_load(t, (walker + (v + 1) * walkers) * kRows);
       small_store(now, v);
       cut_stage(true);
       if (ok && v > 0) dt_out(v - 1);   // one tile behind: its products have had a stage's time to complete
@@ -450,7 +506,7 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
     if (ok && mine > 0 && !MbarWait(&bars->acc_full, 0)) give_up();
     if (ok && mine > 0) {
       TcFenceAfter();
-      store_partials(pb, nc, N, true);
+      store_partials(pb, n_first, nc, N, true);
       TcFenceBefore();
       __threadfence_block();   // this block's dT rows, written by two of the warps, are read back by all of them
       __syncwarp();
@@ -458,23 +514,27 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
       if (!MbarWait(&bars->acc_free, 0)) give_up();   // every worker warp has stored its rows
     }
     // ---- over x ----
-    if (ok && mine > 0) ahead = small_load(dt, blockIdx.x * kRows);
+    if (ok && mine > 0) {
+      if (halves == 1) ahead = small_load(dt, walker * kRows);
+      else if (wt < 4 * kRows) ahead = *reinterpret_cast<const float4*>(exchange + (wt >> 2) * kR + (wt & 3u) * 4u);
+    }
     for (uint32_t v = 0; v < mine && ok; ++v) {
       const float4 now = ahead;
-      if (v + 1 < mine) ahead = small_load(dt, (blockIdx.x + (v + 1) * gridDim.x) * kRows);
+      if (v + 1 < mine) ahead = small_load(dt, (walker + (v + 1) * walkers) * kRows);
       small_store(now, mine + v);
       for (uint32_t c = 0; c < kc && ok; ++c) cut_stage(false);
     }
     if (ok && mine > 0 && !MbarWait(&bars->acc_full, 1)) give_up();
     if (ok && mine > 0) {
       TcFenceAfter();
-      store_partials(pa, kc, K, false);
+      store_partials(pa, k_first, kc, K, false);
     }
   }
 
   TcFenceBefore();
   __syncthreads();
   if (bars->abort) DrainDelay();
+  if (halves == 2) ClusterSync();   // neither block leaves while the other may still write here
   if (warp == 1) {
     TcFenceAfter();
     TmemFree(tmem_base, kTmemCols);
@@ -510,10 +570,24 @@ cudaError_t LoraBackwardUmmaLaunch(const CUtensorMap& map_dy, const CUtensorMap&
     if (e != cudaSuccess) return e;
     if (tracked) configured[dev].store(true, std::memory_order_release);
   }
-  LoraBackwardUmmaKernel<<<blocks, kThreads, kSmemBytes, s>>>(
-      map_dy, map_x, map_b, a.t, a.dt, a.partials, static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N),
-      static_cast<uint32_t>(a.K), a.alpha_dt, a.dt_pieces, LoraSplitColumns(static_cast<uint32_t>(a.r)), status);
-  return cudaGetLastError();
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // Two blocks to a tile where every block of the launch still has an SM of its own (`blocks` is then the tiles).
+  const bool split = 2 * blocks <= sms && static_cast<size_t>(blocks) * kRows >= a.M && a.N % (2 * kChunk) == 0 && a.K % (2 * kChunk) == 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(split ? 2 * blocks : blocks));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = split ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, LoraBackwardUmmaKernel, map_dy, map_x, map_b, a.t, a.dt, a.partials,
+                            static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), static_cast<uint32_t>(a.K), a.alpha_dt,
+                            a.dt_pieces, LoraSplitColumns(static_cast<uint32_t>(a.r)), status, split ? 2u : 1u);
 }
 
 }  // namespace see::k
