@@ -182,11 +182,6 @@ LoraDownKernel(const float* __restrict__ x, const float* __restrict__ A, float* 
   uint32_t* a_hi = reinterpret_cast<uint32_t*>(smem);
   uint32_t* a_lo = a_hi + static_cast<size_t>(R) * S::kStride;
   float* part = smem + S::kWeightFloats;   // [warp][lane][kLaneFloats]
-  for (int idx = threadIdx.x; idx < K * R; idx += kDownThreads) {   // A [K][R] -> a[n][k], k fastest (bank-free stores)
-    const int n = idx / K, k = idx - n * K;
-    SplitTf32(__ldg(A + k * R + n), &a_hi[n * S::kStride + k], &a_lo[n * S::kStride + k]);
-  }
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   constexpr int kBlocks = K / 16;
   const size_t tiles = (M + kTileRows - 1) / kTileRows;
@@ -201,6 +196,41 @@ LoraDownKernel(const float* __restrict__ x, const float* __restrict__ A, float* 
   const size_t stride = static_cast<size_t>(gridDim.x) * groups;
   const size_t trips = kSplitK ? (tiles + stride - 1) / stride : 0;
   size_t trip = 0;
+  // A tile's first blocks of x: the first tile's on their way during the prologue, every other's during the stores of
+  // the tile before.
+  float4 va[kDownAhead], vb[kDownAhead];
+  auto load_first = [&](size_t tile) {
+    const size_t row = tile * kTileRows + g;
+    const float* xa = x + (tile < tiles && row < M ? row : 0) * K + 4 * t;
+    const float* xb = x + (tile < tiles && row + 8 < M ? row + 8 : 0) * K + 4 * t;
+#pragma unroll
+    for (int p = 0; p < kDownAhead; ++p) {
+      if (tile >= tiles || (kSplitK && kb0 + p >= kb1)) continue;
+      va[p] = __ldg(reinterpret_cast<const float4*>(xa + 16 * (kb0 + p)));
+      vb[p] = __ldg(reinterpret_cast<const float4*>(xb + 16 * (kb0 + p)));
+    }
+  };
+  load_first(static_cast<size_t>(group) * gridDim.x + blockIdx.x);
+  // A [K][R] -> a[n][k], k fastest over the lanes (bank-free stores), four n per load (A is 16-byte aligned) and every
+  // load of the thread in flight at once; with few rows this prologue is most of the launch (4096 x 768, r 16: 9.8 us with
+  // one element a load and x asked for after it, 7.0 to 7.6 so).
+  constexpr int kQuads = K * R / 4, kLoads = (kQuads + kDownThreads - 1) / kDownThreads;
+  float4 f[kLoads];
+#pragma unroll
+  for (int i = 0; i < kLoads; ++i) {
+    const int idx = static_cast<int>(threadIdx.x) + i * kDownThreads, q = idx / K, k = idx - q * K;
+    f[i] = idx < kQuads ? __ldg(reinterpret_cast<const float4*>(A + k * R + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < kLoads; ++i) {
+    const int idx = static_cast<int>(threadIdx.x) + i * kDownThreads, q = idx / K, k = idx - q * K;
+    if (idx >= kQuads) continue;
+    const float v[4] = {f[i].x, f[i].y, f[i].z, f[i].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      SplitTf32(v[e], &a_hi[(4 * q + e) * S::kStride + k], &a_lo[(4 * q + e) * S::kStride + k]);
+  }
+  __syncthreads();
   for (size_t tile = static_cast<size_t>(group) * gridDim.x + blockIdx.x; kSplitK ? trip < trips : tile < tiles;
        tile += stride, ++trip) {
     const bool live = tile < tiles;
@@ -213,13 +243,6 @@ LoraDownKernel(const float* __restrict__ x, const float* __restrict__ A, float* 
     for (int j = 0; j < R / 8; ++j)
 #pragma unroll
       for (int term = 0; term < 3; ++term) c[j][term][0] = c[j][term][1] = c[j][term][2] = c[j][term][3] = 0.0f;
-    float4 va[kDownAhead], vb[kDownAhead];
-#pragma unroll
-    for (int p = 0; p < kDownAhead; ++p) {
-      if (kSplitK && (!live || kb0 + p >= kb1)) continue;
-      va[p] = __ldg(reinterpret_cast<const float4*>(xa + 16 * (kb0 + p)));
-      vb[p] = __ldg(reinterpret_cast<const float4*>(xb + 16 * (kb0 + p)));
-    }
 #pragma unroll 1
     for (int s0 = kb0; s0 < (kSplitK && !live ? kb0 : kb1); s0 += kDownAhead) {
 #pragma unroll
@@ -254,6 +277,7 @@ LoraDownKernel(const float* __restrict__ x, const float* __restrict__ A, float* 
         }
       }
     }
+    load_first(tile + stride);
     // This lane holds rows g and g + 8, columns 8 j + 2 t and + 1.
     if (kSplitK) {
       float* mine = part + (static_cast<size_t>(warp) * 32 + lane) * S::kLaneFloats;
