@@ -14,8 +14,11 @@
 //
 // Two sets of kernels give the same bits.
 //
+// (Where the bits are not observed the tile kernels take their double dots on the FP64 tensor instruction and contract
+// the output sums: DotTile and MulAdd.)
+//
 // The tile kernels (AttnFwdTile, AttnDPTile, AttnRowTile, AttnColTile,
-// AttnDQTiledTile, AttnDKVTiledTile) are FP64-bound: a block owns 8, 16 or 32
+// AttnDQTiledTile, AttnDKVTiledTile) are bound by FP64 and shared memory: a block owns 8, 16 or 32
 // query (or key) rows of one (sequence, head) and takes the other axis 64 at a
 // time.  Both operands of a score tile are widened to double once, on their way
 // into shared memory (a conversion costs four FMA slots, so per use it would be
@@ -305,7 +308,9 @@ __device__ __forceinline__ void DMma8(double (&c)[4], int e, double a, double b)
 // kMma false: every accumulator one chain over ascending features, the CPU's.  kMma true (where the bits are not
 // observed): the FP64 tensor instruction, whose sums of eight are doubles all the same.  Both run at the FP64 pipe's
 // rate at best; a thread grid of RM x 4 pairs reads RM + 4 doubles of shared memory for 4 RM multiply-adds, the fragments
-// 2 RM + 4 for 64 RM of a warp's.
+// 2 RM + 4 a lane for 64 RM a lane of a slice.  Measured, thread grid / tensor instruction: forward of 8 x 512 positions
+// of 12 heads of 64 226 / 176 us (shared memory 68 % busy, the FP64 pipe 29), of 32 x 128 of 4 heads 37.3 / 30.5, dP of those
+// 21.4 / 16.6.
 template <int RM, bool kVec, bool kMma>
 __device__ __forceinline__ void DotTile(const double* own, const float* b, int rows, const float* next, int next_rows,
                                         size_t stride, int d, double* slices, int* turn, SliceRegs* regs,

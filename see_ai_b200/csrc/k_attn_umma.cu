@@ -17,7 +17,8 @@
 // reductions of the bf16 products: two walks over the keys (first the row
 // statistics, then the products), so no accumulator is ever rescaled.
 //
-// A CTA is 128 threads, one query row (or key row) per thread, and takes the
+// Sequences of several tiles and a step's backward run on dedicated warps (AttnFwdPairKernel, AttnBwdKernel, with their
+// own comments below).  In the other kernels a CTA is 128 threads, one query row (or key row) per thread, and takes the
 // other axis 64 positions per step, which keeps its footprint at 48-72 KB of
 // shared memory and 128-256 columns of tensor memory: two to four CTAs share an
 // SM and fill each other's load, MMA and exp latencies.  Thread 0 issues TMA
