@@ -1693,8 +1693,9 @@ void CudaBackend::PlanProductGroups(std::span<const Instruction> program, size_t
     return program[i].out[0] == program[j].out[0] && program[i].out[1] == program[j].out[1] && program[i].out[2] == program[j].out[2];
   };
   constexpr size_t kWindow = 16;   // instructions a chain may reach across
+  // The products that wait for a launch are one list, so a group begins behind the last member of the one before:
+  // nothing inside a chain's window starts another.
   for (size_t i = begin; i < end; ++i) {
-    if (product_group_[i - begin].member) continue;
     Product p = product_at(i);
     if (!p.ok || p.addend != kNullRef) continue;
     size_t members[k::kUmmaProducts] = {i};
@@ -1711,6 +1712,7 @@ void CudaBackend::PlanProductGroups(std::span<const Instruction> program, size_t
       }
       if (count < 2) continue;
       for (size_t m = 0; m < count; ++m) product_group_[members[m] - begin] = {true, m + 1 == count, false, 0, 0, 0};
+      i = members[count - 1];
       continue;
     }
     // chained
@@ -1748,6 +1750,7 @@ void CudaBackend::PlanProductGroups(std::span<const Instruction> program, size_t
     if (count < 2 || !folds) continue;
     for (size_t m = 0; m < count; ++m)
       product_group_[members[m] - begin] = {true, m + 1 == count, true, dead[m][0], dead[m][1], after[m]};
+    i = members[count - 1];
   }
 }
 

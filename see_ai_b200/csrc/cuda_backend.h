@@ -440,7 +440,8 @@ class CudaBackend {
   std::vector<LoraFold> lora_fold_;          // per range position (of G)
 
   // Relaxed products of one shape launched as one, from the last of them (umma::LaunchProducts): the dispatch of an
-  // earlier one makes its operands' copies and leaves the launch to the last.  Engine / lazy coherence only.
+  // earlier one makes its operands' copies and leaves the launch to the last.  Engine / lazy coherence only.  Groups do
+  // not interleave: from the first member to the last no product belongs to another group.
   //   side by side: neighbours that read the same activation (Q, K and V), each leaving as its attention copy alone.
   //     Nothing lies between them but what their own dispatches stand for.
   //   chained: each adds its product to the one before it (the input gradients of Q, K and V), so that only the last sum

@@ -1,0 +1,115 @@
+"""Input gradients that several relaxed products add up to, launched together (a chain), where something else that is
+launched together lies between the members: a second chain, or Q, K and V side by side.  A program run as ONE range is
+compared with the same program run one instruction per range: the frozen products are the same bf16 computation both
+ways, so the sums differ by the arithmetic of the low-rank terms and of the additions, held to 2e-6 of the terms'
+magnitudes as the folds are."""
+
+import numpy as np
+import pytest
+
+from see_ai_b200 import backend as B
+from see_ai_b200 import plan as P
+from tests.test_oracle_pinned import Arena
+
+pytestmark = pytest.mark.gpu
+Op = P.Op
+REL, CS, ADDEND = P.FLAG_RELAXED, P.FLAG_Q8_COL_SCALE, P.FLAG_GEMM_ADDEND
+SIZES = [(256, 128, 192), (4864, 128, 2048)]   # (M, K, N): one-tile kernel; persistent kernel
+
+
+class Chain:
+    """s_p = s_(p-1) + dT_p A_p^T + dY_p W_p^T, p = 0 .. n - 1: the instructions of each member, and what is scratch."""
+
+    def __init__(self, a, rng, M, N, K, r, n):
+        self.M, self.N, self.K, self.r = M, N, K, r
+        self.members, self.scratch, self.terms = [], [], []
+        total = None
+        for p in range(n):
+            dy, dt, A = a.alloc(M * K, "normal"), a.alloc(M * r, "normal"), a.alloc(N * r, "normal", scale=0.05)
+            levels = rng.integers(-127, 128, size=(N, K), dtype=np.int8)
+            scale = (rng.random(K) * 0.01 + 1e-3).astype(np.float32)
+            w, sk = a.ro_alloc(levels), a.ro_alloc(scale)
+            z, part, out = a.alloc(M * N), a.alloc(M * N), a.alloc(M * N)
+            g = P.Instr(Op.GEMM_NT_Q8, REL | CS, 0, (dy, w, z, sk), (M, N, K))
+            if p == 0:
+                self.members.append([g, P.Instr(Op.GEMM_NT, ADDEND, 0, (dt, A, out, z), (M, N, r))])
+            else:
+                self.members.append([P.Instr(Op.GEMM_NT, ADDEND, 0, (dt, A, part, total), (M, N, r)), g,
+                                     P.Instr(Op.ADD_EW, 0, 0, (part, z, out, P.NULL_REF), (M * N, 0, 0))])
+                self.scratch.append(part)
+                self.scratch.append(total)
+            self.scratch.append(z)
+            self.terms.append((dy, levels * scale, dt, A))
+            total = out
+        self.out = total
+
+    def fills(self):
+        return [P.Instr(Op.FILL, 0, 0, (s, P.f32_bits(0.0)), (self.M * self.N, 0, 0)) for s in self.scratch]
+
+    def check(self, one, split, arena0):
+        M, N, K, r = self.M, self.N, self.K, self.r
+        got, want = _f32(one, self.out, M * N), _f32(split, self.out, M * N)
+        mag = np.ones((M, N))
+        for dy, w, dt, A in self.terms:
+            mag += np.abs(_f32(arena0, dy, M * K).reshape(M, K) @ w.T)
+            mag += np.abs(_f32(arena0, dt, M * r).reshape(M, r)) @ np.abs(_f32(arena0, A, N * r).reshape(N, r)).T
+        mag = mag.reshape(-1)
+        err = np.abs(got - want) / mag
+        assert np.isfinite(got).all() and err.max() < 2e-6, err.max()
+
+
+def _f32(arena, off, n):
+    return arena[off:off + 4 * n].view(np.float32).astype(np.float64)
+
+
+def _run(prog, arena0, ro, one_range=True):
+    arena = arena0.copy()
+    be = B.CudaBackend(0)
+    be.set_coherence(B.COHERENCE_LAZY)
+    be.bind(arena, ro)
+    be.set_program(prog)
+    for i, end in [(0, len(prog))] if one_range else [(i, i + 1) for i in range(len(prog))]:
+        be.run(None, None, i, end)
+    be.host_needs(0, arena.size)
+    be.flush()
+    launches = be.counters().kernel_launches
+    be.close()
+    return arena, launches
+
+
+@pytest.mark.parametrize("size", SIZES, ids=["one-tile", "persistent"])
+@pytest.mark.parametrize("n", [2, 3])
+def test_two_interleaved_chains(size, n):
+    M, K, N = size
+    rng = np.random.default_rng(M + n)
+    a = Arena(rng)
+    one, two = (Chain(a, rng, M, N, K, 16, n) for _ in range(2))
+    prog = [ins for p in range(n) for c in (one, two) for ins in c.members[p]] + one.fills() + two.fills()
+    arena0, ro = a.build()
+    got, _ = _run(prog, arena0, ro)
+    want, _ = _run(prog, arena0, ro, one_range=False)
+    one.check(got, want, arena0)
+    two.check(got, want, arena0)
+
+
+@pytest.mark.parametrize("M", [256, 4864])
+def test_side_by_side_products_inside_a_chain(M):
+    S, H, d, K, r = 64, 2, 64, 128, 16
+    N = H * d
+    rng = np.random.default_rng(M)
+    a = Arena(rng)
+    chain = Chain(a, rng, M, N, K, r, 2)
+    x = a.alloc(M * K, "normal")
+    q, k, v, o = (a.alloc(M * N) for _ in range(4))
+    stats = a.alloc(M * H * 4)
+    qkv = [P.Instr(Op.GEMM_NN_Q8, REL | CS, 0,
+                   (x, a.ro_alloc(rng.integers(-127, 128, size=K * N, dtype=np.int8)), out,
+                    a.ro_alloc((rng.random(N) * 0.001 + 1e-3).astype(np.float32))), (M, N, K)) for out in (q, k, v)]
+    attention = P.Instr(Op.ATTN_FWD_TILED, REL, 0, (q, k, v, o), (stats, P.pack2(M // S, S), P.pack2(H, d)))
+    clear = [P.Instr(Op.FILL, 0, 0, (t, P.f32_bits(0.0)), (M * N, 0, 0)) for t in (q, k, v)]
+    prog = chain.members[0] + qkv + [attention] + clear + chain.members[1] + chain.fills()
+    arena0, ro = a.build()
+    got, _ = _run(prog, arena0, ro)
+    want, _ = _run(prog, arena0, ro, one_range=False)
+    chain.check(got, want, arena0)
+    assert np.array_equal(got[o:o + 4 * M * N], want[o:o + 4 * M * N])
