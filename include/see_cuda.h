@@ -98,6 +98,9 @@ int see_cuda_set_epilogue_fusion(see_cuda_backend* h, int enabled);
 /* 0: an adapter's rank-r expand product stays its own kernel instead of riding the
  * frozen product's tensor-core reduction (lazy coherence only); default 1. */
 int see_cuda_set_lora_fold(see_cuda_backend* h, int enabled);
+/* 0: relaxed products of one shape (Q, K and V side by side, their input gradients
+ * as one sum) are launched one by one (lazy coherence only; the same bits); default 1. */
+int see_cuda_set_product_groups(see_cuda_backend* h, int enabled);
 /* 0: the rank-r adapter products, the smaller f32 products and the exact attention
  * family keep one rounding per operation in the CPU's order (bit for bit) in lazy
  * coherence too, and see_cuda_set_split_gemm's default domain is that of its mode 1;

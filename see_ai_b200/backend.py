@@ -32,7 +32,7 @@ EXPORTED_SYMBOLS = [
     "see_cuda_set_gradient_gather",
     "see_cuda_set_profiling", "see_cuda_take_profile",
     "see_cuda_xent_forward_static", "see_cuda_static_max_rows", "see_cuda_static_last_error",
-    "see_cuda_quantize_columns", "see_cuda_set_lora_fold", "see_cuda_set_adapter_fma", "see_cuda_set_split_gemm", "see_cuda_set_cta_pairs", "see_cuda_set_adapter_tensor_backward", "see_cuda_set_attention_one_walk",
+    "see_cuda_quantize_columns", "see_cuda_set_lora_fold", "see_cuda_set_product_groups", "see_cuda_set_adapter_fma", "see_cuda_set_split_gemm", "see_cuda_set_cta_pairs", "see_cuda_set_adapter_tensor_backward", "see_cuda_set_attention_one_walk",
 ]
 
 
@@ -105,6 +105,7 @@ def load_library() -> ctypes.CDLL:
     lib.see_cuda_take_profile.restype = ctypes.c_int64
     lib.see_cuda_quantize_columns.argtypes = [vp, vp, u64, u64, vp, vp]
     lib.see_cuda_set_lora_fold.argtypes = [vp, i32]
+    lib.see_cuda_set_product_groups.argtypes = [vp, i32]
     lib.see_cuda_set_adapter_fma.argtypes = [vp, i32]
     lib.see_cuda_set_split_gemm.argtypes = [vp, i32]
     lib.see_cuda_set_cta_pairs.argtypes = [i32]
@@ -247,6 +248,9 @@ class CudaBackend:
 
     def set_epilogue_fusion(self, enabled: bool):
         self._check(self.lib.see_cuda_set_epilogue_fusion(self.h, int(enabled)))
+
+    def set_product_groups(self, enabled: bool):
+        self._check(self.lib.see_cuda_set_product_groups(self.h, int(enabled)))
 
     def set_lora_fold(self, enabled: bool):
         self._check(self.lib.see_cuda_set_lora_fold(self.h, int(enabled)))

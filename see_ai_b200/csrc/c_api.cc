@@ -116,6 +116,11 @@ int see_cuda_end_range(see_cuda_backend* h) {
   return SEE_OK;
 }
 
+int see_cuda_set_product_groups(see_cuda_backend* h, int enabled) {
+  h->backend->SetProductGroups(enabled != 0);
+  return SEE_OK;
+}
+
 int see_cuda_set_lora_fold(see_cuda_backend* h, int enabled) {
   h->backend->SetLoraFold(enabled != 0);
   return SEE_OK;

@@ -1635,7 +1635,7 @@ void CudaBackend::PlanActFusions(std::span<const Instruction> program, size_t be
 
 void CudaBackend::PlanProductGroups(std::span<const Instruction> program, size_t begin, size_t end) {
   product_group_.assign(end > begin ? end - begin : 0, ProductGroup{});
-  if (coherence_ == Coherence::kStrict || !relaxed_allowed_ || !epilogue_fusion_ || end < begin + 3) return;
+  if (coherence_ == Coherence::kStrict || !relaxed_allowed_ || !epilogue_fusion_ || !product_groups_ || end < begin + 3) return;
   if (act_fusion_.size() != end - begin || pack_plan_.size() != end - begin) return;
   const bool whole = step_program_ != nullptr && program.data() == step_program_;
   const size_t ext_base = whole ? 0 : begin, ext_end = whole ? program.size() : end;
@@ -1744,8 +1744,7 @@ void CudaBackend::PlanProductGroups(std::span<const Instruction> program, size_t
       p = q;
       j = p.last;
     }
-    // (A chain rounds its sum once: only where a fold has given up the instructions' own rounding already.)
-    bool folds = false;
+    bool folds = false;   // (measured with a low-rank fold among them; other sums stay instructions of their own)
     for (size_t m = 0; m < count; ++m) folds = folds || lora_fold_[members[m] - begin].fuse;
     if (count < 2 || !folds) continue;
     for (size_t m = 0; m < count; ++m)
@@ -2085,7 +2084,6 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
                                            joins && !group->last, &product, &launched, stream_, &launches);
     if (err.empty() && launched) {
       if (joins) {
-        if (group->chained) product.args.addend = nullptr;   // it is the sum of the products before this one
         waiting_products_.push_back(product);
         lora_rows_tag_.valid = false;   // (what it spoke of now belongs to the waiting product)
       } else {

@@ -152,6 +152,8 @@ class CudaBackend {
   // Off: the rank-r expand product of an adapter stays its own kernel instead of
   // riding the frozen product's reduction (takes effect at the next BeginRange).
   void SetLoraFold(bool enabled) { lora_fold_enabled_ = enabled; }
+  // Off: relaxed products are launched one by one (takes effect at the next BeginRange).
+  void SetProductGroups(bool enabled) { product_groups_ = enabled; }
   void SetAttentionOneWalk(bool enabled) { attn_one_walk_ = enabled; }
 
   // Off: the rank-r adapter products keep the CPU's one-rounding-per-operation
@@ -473,6 +475,7 @@ class CudaBackend {
   uint64_t lora_t_capacity_ = 0, lora_t_stride_ = 0;
   uint16_t* LoraRows() const { return d_lora_t_ ? d_lora_t_ + waiting_products_.size() * lora_t_stride_ : nullptr; }
   bool lora_fold_enabled_ = true;
+  bool product_groups_ = true;
   bool attn_one_walk_ = true;
   bool adapter_fma_ = true;
   // The three backward products of an adapter site (dT = a dY B^T, dB = a t^T dY,

@@ -53,32 +53,27 @@ __device__ __forceinline__ bool PartnerWait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
-// Element offsets along K of reduction block kb's tiles of A and B, and which product's maps they come from (side by
-// side: `product`; chained: the one kb falls into).
-struct BlockAt { int32_t a, b; uint32_t product; bool aux; };
-__device__ __forceinline__ BlockAt BlockCoord(const UmmaEpilogue& ep, uint32_t kb, uint32_t main_blocks, uint32_t product) {
-  if (ep.chained)
-    for (uint32_t len; product + 1 < ep.products && kb >= (len = main_blocks + ep.product[product].aux_k_blocks); ++product)
-      kb -= len;
+// What a launch's accumulators are.
+//   kPlain  one per tile (of one product, or of each of several side by side)
+//   kPieces piece products (UmmaEpilogue::seg_blocks): one per block of K
+//   kChain  the products of a chain: one each
+enum class Sums { kPlain, kPieces, kChain };
+
+// Element offsets along K of reduction block kb's tiles of A and B of a product.
+struct BlockAt { int32_t a, b; bool aux; };
+__device__ __forceinline__ BlockAt BlockCoord(const UmmaEpilogue& ep, uint32_t kb, uint32_t main_blocks) {
   if (kb >= main_blocks) {
     const int32_t x = static_cast<int32_t>((kb - main_blocks) * kBlockK);
-    return {x, x, product, true};
+    return {x, x, true};
   }
-  if (ep.seg_blocks == 0) return {static_cast<int32_t>(kb * kBlockK), static_cast<int32_t>(kb * kBlockK), product, false};
+  if (ep.seg_blocks == 0) return {static_cast<int32_t>(kb * kBlockK), static_cast<int32_t>(kb * kBlockK), false};
   const uint32_t w = kb / ep.segs, seg = kb - w * ep.segs;
   return {static_cast<int32_t>((((ep.seg_a >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK),
-          static_cast<int32_t>((((ep.seg_b >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK), product, false};
+          static_cast<int32_t>((((ep.seg_b >> (4 * seg)) & 15u) * ep.seg_blocks + w) * kBlockK), false};
 }
-// Blocks of a tile's whole reduction.
+// Blocks of a product's whole reduction.
 __device__ __forceinline__ uint32_t ReductionBlocks(const UmmaEpilogue& ep, uint32_t main_blocks, uint32_t product) {
-  uint32_t blocks = main_blocks + ep.product[product].aux_k_blocks;
-  if (ep.chained)
-    for (uint32_t p = 1; p < ep.products; ++p) blocks += main_blocks + ep.product[p].aux_k_blocks;
-  return blocks;
-}
-// Column tiles of all the outputs of a launch.
-__device__ __forceinline__ uint32_t ColumnTiles(const UmmaEpilogue& ep, uint32_t tiles_n) {
-  return ep.chained ? tiles_n : tiles_n * ep.products;
+  return main_blocks + ep.product[product].aux_k_blocks;
 }
 
 // ---- about one tile per SM --------------------------------------------------------------
@@ -114,16 +109,25 @@ struct __align__(8) TBarriers {
   uint64_t full[kTMaxStages];
   uint64_t empty[kTMaxStages];
   uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];   // piece products only
+  uint64_t tmem_empty[2];   // where accumulators take turns (piece products, wide chains)
   uint32_t tmem_base;
   volatile uint32_t abort;      // set by a role whose wait ran out; the epilogue then stores nothing
   volatile uint32_t nonfinite;  // piece products: some sum of this CTA is not finite
 };
 
-template <uint32_t kTN, bool kSeg>
+// A chain (kChain) is the sum of its products as separate launches would leave it, bit for bit: every product has an
+// accumulator of its own, cut over the same splits, and their scaled sums meet in f32 in the products' order.  (One
+// accumulator for all truncates at the sum's magnitude: rms error 3.2e-6 at K = 3072 where 768 at a time leave 7.3e-7.)
+// Up to 128 columns all accumulators stay in tensor memory until the end (3 x 128 of 512 columns); wider tiles, never cut,
+// take turns in two buffers and are added in registers.
+template <uint32_t kTN, Sums kSums>
 __global__ void __launch_bounds__(kTThreads, 1)
 UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant__ UmmaEpilogue ep, uint32_t splits) {
   using T = TTile<kTN>;
+  constexpr bool kSeg = kSums == Sums::kPieces, kChain = kSums == Sums::kChain;
+  constexpr bool kResident = kChain && kTN <= 128;       // the accumulators lie side by side until the end
+  constexpr bool kTurns = (kSeg || kChain) && !kResident; // ... take turns and are added in registers
+  static_assert(!kResident || T::kStages * T::kStageBytes >= kUmmaProducts * kBlockM * kTN * 4, "a chain's tiles are staged together");
   constexpr uint32_t kStages = T::kStages, kStageBytes = T::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: the swizzle pattern and the descriptors' base offset assume it.
@@ -132,20 +136,23 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t split = ClusterCtaRank();   // (a cluster is one tile's splits)
-  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, all_n = kSeg ? tiles_n : ColumnTiles(ep, tiles_n), tile = blockIdx.x / splits;
-  const uint32_t mb = tile / all_n, product = kSeg ? 0 : tile % all_n / tiles_n, nb = tile % all_n % tiles_n;
+  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, all_n = kSums == Sums::kPlain ? tiles_n * ep.products : tiles_n, tile = blockIdx.x / splits;
+  const uint32_t mb = tile / all_n, product = kSums == Sums::kPlain ? tile % all_n / tiles_n : 0, nb = tile % all_n % tiles_n;
   const uint32_t m0 = mb * kBlockM, n0 = nb * kTN;
   // The reduction runs over the main operands' K and then over aux_k_blocks more
   // 64-wide blocks taken from the second pair of maps (a low-rank term T . B'^T
   // accumulated into the same tile; see UmmaEpilogue::Product).
   const uint32_t main_blocks = (ep.K + kBlockK - 1) / kBlockK;
-  const uint32_t k_blocks = ReductionBlocks(ep, main_blocks, product);
-  // Accumulators of the reduction, `group` blocks each: a plain product has one, piece products one per block of K.
-  const uint32_t all = kSeg ? ep.seg_blocks : k_blocks;
-  const uint32_t part0 = all * split / splits, part1 = all * (split + 1) / splits;
-  const uint32_t kb0 = kSeg ? part0 * ep.segs : part0, kb1 = kSeg ? part1 * ep.segs : part1;
-  const uint32_t group = kSeg ? ep.segs : kb1 - kb0, groups = kSeg ? part1 - part0 : 1u;
-  constexpr uint32_t kTmemCols = kSeg ? 2 * T::kTmemCols : T::kTmemCols;
+  // This CTA's accumulators: of one product, of each block of K of piece products, of each product of a chain.
+  const uint32_t part0 = kSeg ? ep.seg_blocks * split / splits : 0, part1 = kSeg ? ep.seg_blocks * (split + 1) / splits : 0;
+  const uint32_t groups = kSeg ? part1 - part0 : (kChain ? ep.products : 1u);
+  struct Blocks { uint32_t product, begin, end; };
+  auto blocks_of = [&](uint32_t g) -> Blocks {
+    if (kSeg) return {0, (part0 + g) * ep.segs, (part0 + g + 1) * ep.segs};
+    const uint32_t p = kChain ? g : product, all = ReductionBlocks(ep, main_blocks, p);
+    return {p, all * split / splits, all * (split + 1) / splits};
+  };
+  constexpr uint32_t kTmemCols = kTurns ? 2 * T::kTmemCols : (kResident ? 4 * T::kTmemCols : T::kTmemCols);
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < kStages; ++s) {
@@ -171,20 +178,25 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
   if (warp == 0) {
     // ---- TMA producer ----
     if (lane == 0) {
-      for (uint32_t kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-        const uint32_t s = it % kStages, round = it / kStages;
-        if (round > 0 && !MbarWait(&bars->empty[s], (round - 1) & 1)) {
-          ep.status->wait_timeout = 1;
-          bars->abort = 1;
-          break;
+      bool going = true;
+      for (uint32_t g = 0, it = 0; g < groups && going; ++g) {
+        const Blocks part = blocks_of(g);
+        for (uint32_t kb = part.begin; kb < part.end; ++kb, ++it) {
+          const uint32_t s = it % kStages, round = it / kStages;
+          if (round > 0 && !MbarWait(&bars->empty[s], (round - 1) & 1)) {
+            ep.status->wait_timeout = 1;
+            bars->abort = 1;
+            going = false;
+            break;
+          }
+          uint8_t* a_dst = smem + s * kStageBytes;
+          const BlockAt at = BlockCoord(ep, kb, main_blocks);
+          const CUtensorMap* ma = at.aux ? &maps.a2[part.product] : &maps.a[part.product];
+          const CUtensorMap* mb_ = at.aux ? &maps.b2[part.product] : &maps.b[part.product];
+          MbarExpectTx(&bars->full[s], kStageBytes);
+          TmaLoad2D(a_dst, ma, &bars->full[s], at.a, static_cast<int32_t>(m0));
+          TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], at.b, static_cast<int32_t>(n0));
         }
-        uint8_t* a_dst = smem + s * kStageBytes;
-        const BlockAt at = BlockCoord(ep, kb, main_blocks, product);
-        const CUtensorMap* ma = at.aux ? &maps.a2[at.product] : &maps.a[at.product];
-        const CUtensorMap* mb_ = at.aux ? &maps.b2[at.product] : &maps.b[at.product];
-        MbarExpectTx(&bars->full[s], kStageBytes);
-        TmaLoad2D(a_dst, ma, &bars->full[s], at.a, static_cast<int32_t>(m0));
-        TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], at.b, static_cast<int32_t>(n0));
       }
     }
   } else if (warp == 1) {
@@ -193,14 +205,15 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
       const uint32_t idesc = MakeInstrDesc(kBlockM, kTN);
       bool going = true;
       for (uint32_t g = 0, it = 0; g < groups && going; ++g) {
-        const uint32_t buf = kSeg ? g & 1 : 0, use = g >> 1;
-        if (kSeg && use > 0 && !MbarWait(&bars->tmem_empty[buf], (use - 1) & 1)) {
+        const uint32_t buf = kTurns ? g & 1 : (kResident ? g : 0), use = g >> 1;
+        if (kTurns && use > 0 && !MbarWait(&bars->tmem_empty[buf], (use - 1) & 1)) {
           ep.status->wait_timeout = 1;
           bars->abort = 1;
           break;
         }
         const uint32_t acc = tmem_base + buf * T::kTmemCols;
-        for (uint32_t b = 0; b < group; ++b, ++it) {
+        const Blocks part = blocks_of(g);
+        for (uint32_t b = 0; b < part.end - part.begin; ++b, ++it) {
           const uint32_t s = it % kStages, round = it / kStages;
           if (!MbarWait(&bars->full[s], round & 1)) {
             ep.status->wait_timeout = 1;
@@ -218,7 +231,9 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
           }
           UmmaCommit(&bars->empty[s]);      // the slot is free once these MMAs have read it
         }
-        UmmaCommit(&bars->tmem_full[buf]);  // accumulator complete (or abandoned on timeout)
+        // accumulator complete (or abandoned on timeout); of resident ones the last, with all before it
+        if (kTurns) UmmaCommit(&bars->tmem_full[buf]);
+        else if (g + 1 == groups || !going) UmmaCommit(&bars->tmem_full[0]);
       }
     }
   }
@@ -248,11 +263,11 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
       TcFenceAfter();
       return there;
     };
-    // Piece products: the blocks' accumulators, added with f32's rounding while the next block's products run.
-    [[maybe_unused]] float sum[kSeg ? kTN / 2 : 1];
-    if constexpr (kSeg) {
+    // Accumulators that take turns are added with f32's rounding while the next one's products run.
+    [[maybe_unused]] float sum[kTurns ? kTN / 2 : 1];
+    if constexpr (kTurns) {
 #pragma unroll
-      for (uint32_t j = 0; j < kTN / 2; ++j) sum[j] = 0.0f;
+      for (uint32_t j = 0; j < kTN / 2; ++j) sum[j] = kChain ? -0.0f : 0.0f;   // (-0 + x is x, -0 included)
       for (uint32_t g = 0; g < groups && ok; ++g) {
         const uint32_t buf = g & 1;
         if (!(ok = await(buf, (g >> 1) & 1))) break;
@@ -262,7 +277,7 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
           TmemLoad16(t_row + buf * T::kTmemCols + c0, r);
           TmemWaitLd();
 #pragma unroll
-          for (uint32_t j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(r[j]);
+          for (uint32_t j = 0; j < 16; ++j) sum[c0 + j] += kChain ? __uint_as_float(r[j]) * ep.alpha : __uint_as_float(r[j]);
         }
         TcFenceBefore();
         __syncwarp();
@@ -276,22 +291,24 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
       // the ring is free: the tile goes there as [128][kTN] f32, 16-byte chunks XOR-ed with the
       // row so that neither side conflicts.
       float* dump = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kTN;
-      if constexpr (kSeg) {
-        if (!AllFinite(sum)) bars->nonfinite = 1;
+      if constexpr (kTurns) {
+        if (kSeg && !AllFinite(sum)) bars->nonfinite = 1;
 #pragma unroll
         for (uint32_t q = 0; q < kTN / 8; ++q)
           *reinterpret_cast<float4*>(dump + (((columns >> 2) + q) ^ (lane & 7u)) * 4) =
               make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
       } else {
+        for (uint32_t g = 0; g < (kResident ? groups : 1u); ++g) {   // (a chain's tiles one behind the other)
 #pragma unroll 1
-        for (uint32_t c0 = 0; c0 < kTN / 2; c0 += 32) {
-          uint32_t r[32];
-          TmemLoad32(t_row + c0, r);
-          TmemWaitLd();
+          for (uint32_t c0 = 0; c0 < kTN / 2; c0 += 32) {
+            uint32_t r[32];
+            TmemLoad32(t_row + g * T::kTmemCols + c0, r);
+            TmemWaitLd();
 #pragma unroll
-          for (uint32_t q = 0; q < 8; ++q)
-            *reinterpret_cast<uint4*>(dump + ((((columns + c0) >> 2) + q) ^ (lane & 7u)) * 4) =
-                make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+            for (uint32_t q = 0; q < 8; ++q)
+              *reinterpret_cast<uint4*>(dump + g * (kBlockM * kTN) + ((((columns + c0) >> 2) + q) ^ (lane & 7u)) * 4) =
+                  make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+          }
         }
       }
     }
@@ -302,8 +319,7 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
   if (epilogue && ok) {
     const uint32_t dump = SmemAddr(smem);
     // The tile's element of row r0 + lr, chunk: this CTA's, or the sum of the splits' partials.
-    auto element = [&](uint32_t lr, uint32_t chunk) {
-      const uint32_t off = (lr * kTN + (chunk ^ (lr & 7u)) * 4) * 4;
+    auto partials = [&](uint32_t off) {
       if (splits == 1) return *reinterpret_cast<const float4*>(smem + off);
       float4 acc = LoadClusterF4(MapToCta(dump + off, 0));
       for (uint32_t p = 1; p < splits; ++p) {
@@ -312,11 +328,24 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
       }
       return acc;
     };
+    auto element = [&](uint32_t lr, uint32_t chunk) {
+      const uint32_t off = (lr * kTN + (chunk ^ (lr & 7u)) * 4) * 4;
+      float4 acc = partials(off);
+      if constexpr (kResident) {   // the products' scaled sums, in order
+        const float s = ep.alpha;
+        acc = make_float4(acc.x * s, acc.y * s, acc.z * s, acc.w * s);
+        for (uint32_t g = 1; g < groups; ++g) {
+          const float4 v = partials(off + g * (kBlockM * kTN * 4));
+          acc = make_float4(acc.x + v.x * s, acc.y + v.y * s, acc.z + v.z * s, acc.w + v.w * s);
+        }
+      }
+      return acc;
+    };
     // Four elements per thread at a time, their operands loaded before the first is stored.  `store` is one form of
     // the epilogue, chosen once: tests per element would cost more than the stores.
     constexpr uint32_t kUnroll = 4;
-    const bool side_by_side = !kSeg && ep.products > 1 && !ep.chained;
-    const float alpha = side_by_side ? ep.product[product].alpha : ep.alpha;
+    const bool side_by_side = kSums == Sums::kPlain && ep.products > 1;
+    const float alpha = kChain ? 1.0f : (side_by_side ? ep.product[product].alpha : ep.alpha);
     const float* col_scale = side_by_side ? ep.product[product].col_scale : ep.col_scale;
     uint16_t* pack_dst = side_by_side ? ep.product[product].pack_dst : ep.pack_dst;
     auto each = [&](auto has_side, auto store) {
@@ -350,7 +379,11 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
     if constexpr (kSeg)
       for (uint32_t p = 0; p < splits; ++p)
         remake = remake || (splits == 1 ? bars->nonfinite : LoadClusterU32(MapToCta(SmemAddr(const_cast<uint32_t*>(&bars->nonfinite)), p))) != 0;
-    if (remake) {
+    if (kChain) {   // (stored as it is: nothing else is part of a chain)
+      each(NoSide{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4&) {
+        EpilogueStorePlain(ep, at, acc, scale);
+      });
+    } else if (remake) {
       for (uint32_t i = et; i < rows * kChunks; i += kTEpiThreads) {
         const uint32_t lr = r0 + i / kChunks, row = m0 + lr, n = n0 + i % kChunks * 4;
         if (row < ep.M && n < ep.N) StoreRemade(ep, row, n, element(lr, i % kChunks));
@@ -475,13 +508,14 @@ struct __align__(8) PBarriers {
 // while this group is converted and stored, across passes and from before the
 // wait for the accumulator, so a memory round trip is not paid per group with
 // every warp of the CTA waiting on it.
-// kSeg: piece products (UmmaEpilogue::seg_blocks).  An accumulator buffer then holds one block of K, and the epilogue
-// warps add the blocks in registers, 64 outputs a thread, one block behind the products.
-template <bool kSideLoads, bool kPair, bool kSeg>
+// Piece products and chains: an accumulator buffer holds one block of K, or one product, and the epilogue warps add them
+// in registers, 64 outputs a thread, one buffer behind the products.
+template <bool kSideLoads, bool kPair, Sums kSums>
 __global__ void __launch_bounds__(kPThreads, 1)
 UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant__ UmmaEpilogue ep,
                          uint32_t band_blocks) {
-  static_assert(!(kSideLoads && kSeg), "the sums take the registers of the loads in flight");
+  constexpr bool kSeg = kSums == Sums::kPieces, kChain = kSums == Sums::kChain, kAdds = kSeg || kChain;
+  static_assert(!(kSideLoads && kAdds), "the sums take the registers of the loads in flight");
   using T = PTile<kPair>;
   constexpr uint32_t kTN = kPBlockN;
   constexpr uint32_t kPStages = T::kStages, kPStageBytes = T::kStageBytes, kPTmemCols = T::kTmemCols;
@@ -493,11 +527,11 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t main_blocks = (ep.K + kBlockK - 1) / kBlockK;
-  constexpr bool kSeveral = !kSeg && !kSideLoads;   // products side by side
-  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, all_n = kSeveral ? ColumnTiles(ep, tiles_n) : tiles_n;
+  constexpr bool kSeveral = !kAdds && !kSideLoads;   // products side by side
+  const uint32_t tiles_n = (ep.N + kTN - 1) / kTN, all_n = kSeveral ? tiles_n * ep.products : tiles_n;
   const uint32_t tiles_m = (ep.M + T::kRowsPerTile - 1) / T::kRowsPerTile;
   const uint32_t total_tiles = tiles_m * all_n;
-  const uint32_t groups = kSeg ? ep.seg_blocks : 1u;   // accumulators per tile
+  const uint32_t groups = kSeg ? ep.seg_blocks : (kChain ? ep.products : 1u);   // accumulators per tile
   // A work unit is a CTA, or a CTA pair: `unit` walks the tiles, `cta_rank` is this CTA's half of a pair's tile.
   const uint32_t cta_rank = kPair ? ClusterCtaRank() : 0u;
   const uint32_t unit = kPair ? blockIdx.x >> 1 : blockIdx.x, units = kPair ? gridDim.x >> 1 : gridDim.x;
@@ -542,46 +576,51 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
         const uint32_t product = kSeveral ? nb / tiles_n : 0;
         nb -= product * tiles_n;
         const uint32_t m0 = mb * T::kRowsPerTile + cta_rank * kBlockM, n0 = nb * kTN;
-        const uint32_t k_blocks = ReductionBlocks(ep, main_blocks, product);
         // Ask L2 for the A rows of this CTA's next tile now, so that its loads
         // find them there instead of paying an HBM round trip inside the ring.
-        if (t + units < total_tiles && k_blocks <= 64 && ep.seg_blocks == 0) {   // (a long K would only thrash L2)
+        uint32_t ahead = 0;   // blocks of a tile
+        for (uint32_t p = kChain ? 0 : product; p <= (kChain ? groups - 1 : product); ++p) ahead += ReductionBlocks(ep, main_blocks, p);
+        if (t + units < total_tiles && ahead <= 64 && !kSeg) {   // (a long K would only thrash L2)
           uint32_t next_mb, next_nb;
           TileCoord(t + units, tiles_m, all_n, band_blocks, &next_mb, &next_nb);
           const uint32_t next_m0 = next_mb * T::kRowsPerTile + cta_rank * kBlockM;
           if (next_m0 != m0)
-            for (uint32_t p = 0; p < (ep.chained ? ep.products : 1u); ++p)   // (side by side: they share A)
+            for (uint32_t p = 0; p < (kChain ? groups : 1u); ++p)   // (side by side: they share A)
               for (uint32_t kb = 0; kb < main_blocks; ++kb)
                 asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
                              ::"l"(reinterpret_cast<uint64_t>(&maps.a[p])),
                                "r"(static_cast<int32_t>(kb * kBlockK)), "r"(static_cast<int32_t>(next_m0))
                              : "memory");
         }
-        for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
-          const uint32_t s = it % kPStages, round = it / kPStages;
-          if (round > 0 && !PartnerWait<kSeg>(&bars->empty[s], (round - 1) & 1)) {
-            ep.status->wait_timeout = 1;
-            bars->abort = 1;
-            ok = false;
-            break;
-          }
-          uint8_t* a_dst = smem + s * kPStageBytes;
-          const BlockAt at = BlockCoord(ep, kb, main_blocks, product);
-          const CUtensorMap* ma = at.aux ? &maps.a2[at.product] : &maps.a[at.product];
-          const CUtensorMap* mb_ = at.aux ? &maps.b2[at.product] : &maps.b[at.product];
-          if constexpr (kPair) {
-            // Both CTAs' bytes are counted on the even CTA's barrier, which alone expects them.
-            if (cta_rank == 0) MbarExpectTx(&bars->full[s], 2 * kPStageBytes);
-            const uint32_t full_bar = MapToCta(SmemAddr(&bars->full[s]), 0);
-            TmaLoad2DPair(a_dst, ma, full_bar, at.a, static_cast<int32_t>(m0));
-            TmaLoad2DPair(a_dst + kATileBytes, mb_, full_bar, at.b, static_cast<int32_t>(n0 + cta_rank * kBlockN));
-          } else {
-            MbarExpectTx(&bars->full[s], kPStageBytes);
-            TmaLoad2D(a_dst, ma, &bars->full[s], at.a, static_cast<int32_t>(m0));
-            // B's rows as 128-row boxes, back to back: one [256][64] tile.
-            TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], at.b, static_cast<int32_t>(n0));
-            TmaLoad2D(a_dst + kATileBytes + kBlockN * kBlockK * 2, mb_, &bars->full[s], at.b,
-                      static_cast<int32_t>(n0 + kBlockN));
+        for (uint32_t g = 0; g < (kChain ? groups : 1u) && ok; ++g) {
+          const uint32_t p = kChain ? g : product;
+          const uint32_t k_blocks = kSeg ? groups * ep.segs : ReductionBlocks(ep, main_blocks, p);
+          for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
+            const uint32_t s = it % kPStages, round = it / kPStages;
+            if (round > 0 && !PartnerWait<kSeg>(&bars->empty[s], (round - 1) & 1)) {
+              ep.status->wait_timeout = 1;
+              bars->abort = 1;
+              ok = false;
+              break;
+            }
+            uint8_t* a_dst = smem + s * kPStageBytes;
+            const BlockAt at = BlockCoord(ep, kb, main_blocks);
+            const CUtensorMap* ma = at.aux ? &maps.a2[p] : &maps.a[p];
+            const CUtensorMap* mb_ = at.aux ? &maps.b2[p] : &maps.b[p];
+            if constexpr (kPair) {
+              // Both CTAs' bytes are counted on the even CTA's barrier, which alone expects them.
+              if (cta_rank == 0) MbarExpectTx(&bars->full[s], 2 * kPStageBytes);
+              const uint32_t full_bar = MapToCta(SmemAddr(&bars->full[s]), 0);
+              TmaLoad2DPair(a_dst, ma, full_bar, at.a, static_cast<int32_t>(m0));
+              TmaLoad2DPair(a_dst + kATileBytes, mb_, full_bar, at.b, static_cast<int32_t>(n0 + cta_rank * kBlockN));
+            } else {
+              MbarExpectTx(&bars->full[s], kPStageBytes);
+              TmaLoad2D(a_dst, ma, &bars->full[s], at.a, static_cast<int32_t>(m0));
+              // B's rows as 128-row boxes, back to back: one [256][64] tile.
+              TmaLoad2D(a_dst + kATileBytes, mb_, &bars->full[s], at.b, static_cast<int32_t>(n0));
+              TmaLoad2D(a_dst + kATileBytes + kBlockN * kBlockK * 2, mb_, &bars->full[s], at.b,
+                        static_cast<int32_t>(n0 + kBlockN));
+            }
           }
         }
       }
@@ -604,6 +643,8 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
         uint32_t group;   // blocks of this accumulator
         if constexpr (kSeg) {
           group = ep.segs;
+        } else if constexpr (kChain) {
+          group = ReductionBlocks(ep, main_blocks, g);
         } else {
           uint32_t mb, nb;
           TileCoord(t, tiles_m, all_n, band_blocks, &mb, &nb);
@@ -677,7 +718,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
       [[maybe_unused]] const bool bias_gelu_only = IsBiasGeluOnly(ep);
       [[maybe_unused]] const bool copy_only = IsCopyOnly(ep);
       [[maybe_unused]] const bool plain_store = IsPlainStore(ep);
-      const bool side_by_side = kSeveral && ep.products > 1 && !ep.chained;
+      const bool side_by_side = kSeveral && ep.products > 1;
       [[maybe_unused]] const float alpha = side_by_side ? ep.product[product].alpha : ep.alpha;
       [[maybe_unused]] const float* col_scale = side_by_side ? ep.product[product].col_scale : ep.col_scale;
       [[maybe_unused]] uint16_t* pack_dst = side_by_side ? ep.product[product].pack_dst : ep.pack_dst;
@@ -709,13 +750,13 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
           else MbarArrive(&bars->tmem_empty[buf]);
         }
       };
-      [[maybe_unused]] float sum[kSeg ? kEpiPasses : 1][kSeg ? kSlabCols : 1];
+      [[maybe_unused]] float sum[kAdds ? kEpiPasses : 1][kAdds ? kSlabCols : 1];
       [[maybe_unused]] bool remake = false;   // some sum of this warp's is not finite
-      if constexpr (kSeg) {
+      if constexpr (kAdds) {
 #pragma unroll
         for (uint32_t p = 0; p < kEpiPasses; ++p)
 #pragma unroll
-          for (uint32_t j = 0; j < kSlabCols; ++j) sum[p][j] = 0.0f;
+          for (uint32_t j = 0; j < kSlabCols; ++j) sum[p][j] = kChain ? -0.0f : 0.0f;   // (-0 + x is x, -0 included)
         bool ok = true;
         for (uint32_t g = 0; g < groups; ++g) {
           if (g > 0) { ++lt; buf = lt & 1; use = lt >> 1; }
@@ -727,14 +768,20 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
             TmemLoad16(t_row + c, ra);
             TmemWaitLd();
 #pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) sum[c / kSlabCols][c % kSlabCols + j] += __uint_as_float(ra[j]);
+            for (uint32_t j = 0; j < 16; ++j) {
+              float& to = sum[c / kSlabCols][c % kSlabCols + j];
+              if constexpr (kChain) to += __uint_as_float(ra[j]) * alpha;   // as the products' own epilogues, one after the other
+              else to += __uint_as_float(ra[j]);
+            }
           }
           hand_back();
         }
         if (!ok) break;
+        if constexpr (kSeg) {
 #pragma unroll
-        for (uint32_t p = 0; p < kEpiPasses; ++p) remake = remake || !AllFinite(sum[p]);
-        remake = __any_sync(0xFFFFFFFFu, remake);
+          for (uint32_t p = 0; p < kEpiPasses; ++p) remake = remake || !AllFinite(sum[p]);
+          remake = __any_sync(0xFFFFFFFFu, remake);
+        }
       } else {
         if (!await()) break;
       }
@@ -754,7 +801,11 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
           auto staged = [&](uint32_t rr) {
             return *reinterpret_cast<const float4*>(slab + rr * kSlabCols + ((cl ^ (rr & (kChunks - 1))) * 4));
           };
-          if (kSeg && remake) {
+          if constexpr (kChain) {   // scaled already, and nothing else is part of a chain
+  #pragma unroll 4
+            for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr)
+              *reinterpret_cast<float4*>(ep.C + static_cast<size_t>(row0 + rr) * ep.N + n) = staged(rr);
+          } else if (kSeg && remake) {
             for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr) StoreRemade(ep, row0 + rr, n, staged(rr));
           } else if (ragged) {
             for (uint32_t rr = sub; rr < rows && n < ep.N; rr += kRowsPerInstr)
@@ -783,7 +834,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
           }
           __syncwarp();   // the slab is rewritten next
         };
-        if constexpr (kSeg) {
+        if constexpr (kAdds) {
 #pragma unroll
           for (uint32_t pass = 0; pass < kEpiPasses; ++pass) {
             uint32_t ra[32];
@@ -963,14 +1014,36 @@ static cudaError_t LaunchClustered(void (*kernel)(KArgs...), dim3 grid, dim3 blo
 }
 
 // Calls f(kernel, shared-memory bytes) with the tile kernel of this width.
-template <bool kSeg, typename F>
+template <Sums kSums, typename F>
 static cudaError_t WithTileKernel(uint32_t tn, F f) {
   switch (tn) {
-    case 64: return f(UmmaGemmTileKernel<64, kSeg>, UmmaTileSmemBytes<64>());
-    case 128: return f(UmmaGemmTileKernel<128, kSeg>, UmmaTileSmemBytes<128>());
-    case 192: return f(UmmaGemmTileKernel<192, kSeg>, UmmaTileSmemBytes<192>());
-    default: return f(UmmaGemmTileKernel<256, kSeg>, UmmaTileSmemBytes<256>());
+    case 64: return f(UmmaGemmTileKernel<64, kSums>, UmmaTileSmemBytes<64>());
+    case 128: return f(UmmaGemmTileKernel<128, kSums>, UmmaTileSmemBytes<128>());
+    case 192: return f(UmmaGemmTileKernel<192, kSums>, UmmaTileSmemBytes<192>());
+    default: return f(UmmaGemmTileKernel<256, kSums>, UmmaTileSmemBytes<256>());
   }
+}
+template <typename F>
+static cudaError_t WithTileKernel(Sums sums, uint32_t tn, F f) {
+  return sums == Sums::kPieces  ? WithTileKernel<Sums::kPieces>(tn, f)
+         : sums == Sums::kChain ? WithTileKernel<Sums::kChain>(tn, f)
+                                : WithTileKernel<Sums::kPlain>(tn, f);
+}
+// ... with the persistent one.  (Only a plain product has side loads.)
+template <typename F>
+static cudaError_t WithPersistentKernel(Sums sums, bool side_loads, bool pair, F f) {
+  const size_t bytes = pair ? UmmaPersistentSmemBytes<true>() : UmmaPersistentSmemBytes<false>();
+  if (sums == Sums::kPieces)
+    return pair ? f(UmmaGemmPersistentKernel<false, true, Sums::kPieces>, bytes)
+                : f(UmmaGemmPersistentKernel<false, false, Sums::kPieces>, bytes);
+  if (sums == Sums::kChain)
+    return pair ? f(UmmaGemmPersistentKernel<false, true, Sums::kChain>, bytes)
+                : f(UmmaGemmPersistentKernel<false, false, Sums::kChain>, bytes);
+  if (side_loads)
+    return pair ? f(UmmaGemmPersistentKernel<true, true, Sums::kPlain>, bytes)
+                : f(UmmaGemmPersistentKernel<true, false, Sums::kPlain>, bytes);
+  return pair ? f(UmmaGemmPersistentKernel<false, true, Sums::kPlain>, bytes)
+              : f(UmmaGemmPersistentKernel<false, false, Sums::kPlain>, bytes);
 }
 
 static std::atomic<bool> g_cta_pairs{true};
@@ -981,19 +1054,18 @@ static cudaError_t Configure() {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   };
   cudaError_t e = cudaSuccess;
-  for (uint32_t tn : {64u, 128u, 192u, 256u})
-    if ((e = WithTileKernel<false>(tn, allow)) != cudaSuccess || (e = WithTileKernel<true>(tn, allow)) != cudaSuccess) return e;
-  const size_t one = UmmaPersistentSmemBytes<false>(), pair = UmmaPersistentSmemBytes<true>();
-  if ((e = allow(UmmaGemmPersistentKernel<false, false, false>, one)) != cudaSuccess) return e;
-  if ((e = allow(UmmaGemmPersistentKernel<true, false, false>, one)) != cudaSuccess) return e;
-  if ((e = allow(UmmaGemmPersistentKernel<false, false, true>, one)) != cudaSuccess) return e;
-  if ((e = allow(UmmaGemmPersistentKernel<false, true, false>, pair)) != cudaSuccess) return e;
-  if ((e = allow(UmmaGemmPersistentKernel<true, true, false>, pair)) != cudaSuccess) return e;
-  return allow(UmmaGemmPersistentKernel<false, true, true>, pair);
+  for (Sums sums : {Sums::kPlain, Sums::kPieces, Sums::kChain}) {
+    for (uint32_t tn : {64u, 128u, 192u, 256u})
+      if ((e = WithTileKernel(sums, tn, allow)) != cudaSuccess) return e;
+    for (bool pair : {false, true})
+      for (bool side_loads : {false, true})
+        if ((e = WithPersistentKernel(sums, side_loads, pair, allow)) != cudaSuccess) return e;
+  }
+  return e;
 }
 
 UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms,
-                          uint32_t side_by_side) {
+                          uint32_t side_by_side, uint32_t only_splits, bool chained) {
   UmmaGemmPlan p;
   const uint32_t ptiles_n = (N + kPBlockN - 1) / kPBlockN * side_by_side, tiles_m = (M + kBlockM - 1) / kBlockM;
   const uint64_t wide = static_cast<uint64_t>(ptiles_n) * tiles_m;
@@ -1005,6 +1077,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
   double best = 1e30;
   for (uint32_t tn : {64u, 128u, 192u, 256u})
     for (uint32_t splits = 1; splits <= 4 && splits * group <= k_blocks; splits *= 2) {
+      if ((only_splits != 0 && splits != only_splits) || (chained && splits > 1 && tn > 128)) continue;
       const uint64_t ctas = static_cast<uint64_t>(tiles_m) * ((N + tn - 1) / tn) * side_by_side * splits;
       const uint64_t room = splits <= 2 ? sms : sms * 9 / 10;   // clusters of four do not fill every GPC
       const double waves = static_cast<double>((ctas + room - 1) / room);
@@ -1018,7 +1091,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
         p.b_box = tn;
       }
     }
-  if (wide > sms) {
+  if (wide > sms && only_splits <= 1) {
     // Enough tiles for every SM to amortise its set-up over several: a round of the persistent kernel is its main
     // loop (0.53 us per reduction block, 0.43 in CTA pairs, which load a third fewer bytes per flop) or its
     // epilogue, whichever is longer.  At 32768 rows the epilogue is HBM's: plain and copy-only ones take 8.3 us a tile
@@ -1033,6 +1106,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
                                           std::max(0.43 * k_blocks, (light ? 7.3 : 11.5) - l2)
                               : 1e30;
     if (std::min(single, paired) < best) {
+      best = std::min(single, paired);
       p = UmmaGemmPlan{};
       p.persistent = true;
       p.pair = paired < single;
@@ -1043,6 +1117,7 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
       p.b_box = kBlockN;
     }
   }
+  p.us = best;
   return p;
 }
 
@@ -1057,26 +1132,16 @@ cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const UmmaMaps& maps, const
     if (cudaError_t e = Configure(); e != cudaSuccess) return e;
     if (tracked) configured_on[dev].store(true, std::memory_order_release);
   }
-  const bool seg = ep.seg_blocks != 0;
-  if (!plan.persistent) {
-    auto launch = [&](auto kernel, size_t bytes) {
+  const Sums sums = ep.seg_blocks != 0 ? Sums::kPieces : ep.chained ? Sums::kChain : Sums::kPlain;
+  if (!plan.persistent)
+    return WithTileKernel(sums, plan.tn, [&](auto kernel, size_t bytes) {
       return LaunchClustered(kernel, dim3(plan.grid), dim3(kTThreads), bytes, s, plan.splits, maps, ep, plan.splits);
-    };
-    return seg ? WithTileKernel<true>(plan.tn, launch) : WithTileKernel<false>(plan.tn, launch);
-  }
+    });
   // An addend or the x of an absorbed backward activation is software-pipelined (16 bytes at a time).
-  const bool side_loads = !seg && (ep.addend != nullptr || ep.fuse_mode == kFuseActBwd) && (ep.N & 3) == 0;
-  auto launch = [&](auto kernel, size_t bytes) {
+  const bool side_loads = (ep.addend != nullptr || ep.fuse_mode == kFuseActBwd) && (ep.N & 3) == 0;
+  return WithPersistentKernel(sums, side_loads, plan.pair, [&](auto kernel, size_t bytes) {
     return LaunchClustered(kernel, dim3(plan.grid), dim3(kPThreads), bytes, s, plan.pair ? 2u : 1u, maps, ep, plan.band);
-  };
-  const size_t bytes = plan.pair ? UmmaPersistentSmemBytes<true>() : UmmaPersistentSmemBytes<false>();
-  if (plan.pair)
-    return seg          ? launch(UmmaGemmPersistentKernel<false, true, true>, bytes)
-           : side_loads ? launch(UmmaGemmPersistentKernel<true, true, false>, bytes)
-                        : launch(UmmaGemmPersistentKernel<false, true, false>, bytes);
-  return seg          ? launch(UmmaGemmPersistentKernel<false, false, true>, bytes)
-         : side_loads ? launch(UmmaGemmPersistentKernel<true, false, false>, bytes)
-                      : launch(UmmaGemmPersistentKernel<false, false, false>, bytes);
+  });
 }
 
 void WeightToBf16(const void* src, BType type, uint16_t* dst, uint32_t N, uint32_t K,

@@ -361,20 +361,14 @@ void ReleaseProducts(Context* ctx) {
 
 static bool HasLowRank(const k::GemmArgs& a) { return a.aux_a && a.aux_b && a.aux_k >= 64 && a.aux_k % 64 == 0; }
 
-std::string LaunchProducts(Context* ctx, const PreparedProduct* products, int count, bool chained, cudaStream_t stream,
-                           int* launches) {
-  Impl* impl = ctx->impl;
-  if (!impl || count < 1 || count > static_cast<int>(k::kUmmaProducts)) return "tensor-core path: no such launch";
-  const k::GemmArgs& a = products[count - 1].args;   // a chain's output
-  const uint32_t main_blocks = static_cast<uint32_t>((a.K + 63) / 64);
-  uint32_t longest = 0, all = 0;
-  for (int p = 0; p < count; ++p) {
-    const uint32_t blocks = main_blocks + (HasLowRank(products[p].args) ? products[p].args.aux_k / 64 : 0);
-    longest = std::max(longest, blocks);
-    all += blocks;
-  }
-  const k::UmmaGemmPlan plan = k::UmmaPlanGemm(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), chained ? all : longest, 1,
-                                                LightEpilogue(a), impl->sms, chained ? 1u : static_cast<uint32_t>(count));
+static uint32_t ProductBlocks(const k::GemmArgs& a) {
+  return static_cast<uint32_t>((a.K + 63) / 64) + (HasLowRank(a) ? a.aux_k / 64 : 0);
+}
+
+// One launch on `plan`: a product, several side by side or a chain, whose output and epilogue are the last one's.
+static std::string LaunchOnce(Impl* impl, const PreparedProduct* products, int count, bool chained, const k::UmmaGemmPlan& plan,
+                              cudaStream_t stream, int* launches) {
+  const k::GemmArgs& a = products[count - 1].args;
   k::UmmaMaps maps;
   k::UmmaEpilogue ep{};
   for (uint32_t p = 0; p < k::kUmmaProducts; ++p) {
@@ -402,7 +396,7 @@ std::string LaunchProducts(Context* ctx, const PreparedProduct* products, int co
   ep.products = static_cast<uint32_t>(count);
   ep.chained = chained ? 1 : 0;
   ep.C = a.C;
-  ep.addend = a.addend;
+  ep.addend = chained ? nullptr : a.addend;   // (a chain's is the sum of the products before it)
   ep.bias = a.bias;
   ep.col_scale = a.b_col_scale;
   ep.alpha = a.alpha;
@@ -419,15 +413,55 @@ std::string LaunchProducts(Context* ctx, const PreparedProduct* products, int co
   ep.pack_dst = a.pack_dst;
   ep.store_c = a.store_c ? 1 : 0;
   ep.addend_last = a.addend_after_bias ? 1 : 0;
-  if (impl->prof_before) cudaEventRecord(impl->prof_before, stream);
   if (cudaError_t e = k::UmmaGemmLaunch(plan, maps, ep, stream); e != cudaSuccess)
     return std::string("tensor-core GEMM launch: ") + cudaGetErrorString(e);
+  ++*launches;
+  return {};
+}
+
+std::string LaunchProducts(Context* ctx, const PreparedProduct* products, int count, bool chained, cudaStream_t stream,
+                           int* launches) {
+  Impl* impl = ctx->impl;
+  if (!impl || count < 1 || count > static_cast<int>(k::kUmmaProducts)) return "tensor-core path: no such launch";
+  const uint32_t M = static_cast<uint32_t>(products[0].args.M), N = static_cast<uint32_t>(products[0].args.N);
+  // Each as it would run alone, and all in one launch that cuts every reduction as those do: the same sums, so the same
+  // bits.  The shorter by the planner's estimates is taken: 600 x 768 x 768 alone is cut in four, and three of it side by
+  // side cut in four no longer fit one round.
+  k::UmmaGemmPlan alone[k::kUmmaProducts], together;
+  uint32_t longest = 0, all = 0;
+  double one_by_one = 0.0;
+  for (int p = 0; p < count; ++p) {
+    const uint32_t blocks = ProductBlocks(products[p].args);
+    alone[p] = k::UmmaPlanGemm(M, N, blocks, 1, LightEpilogue(products[p].args), impl->sms);
+    longest = std::max(longest, blocks);
+    all += blocks;
+    one_by_one += alone[p].us;
+  }
+  bool one_launch = count > 1;
+  for (int p = 1; p < count; ++p) one_launch = one_launch && alone[p].splits == alone[0].splits;
+  if (one_launch) {
+    together = k::UmmaPlanGemm(M, N, chained ? all : longest, 1, true, impl->sms, chained ? 1u : static_cast<uint32_t>(count),
+                               alone[0].splits, chained);
+    one_launch = together.us < one_by_one;
+  }
+  if (impl->prof_before) cudaEventRecord(impl->prof_before, stream);
+  if (one_launch) {
+    if (std::string e = LaunchOnce(impl, products, count, chained, together, stream, launches); !e.empty()) return e;
+  } else {
+    for (int p = 0; p < count; ++p) {
+      PreparedProduct one = products[p];
+      if (chained) {   // the running sum in the last one's output: where the ones before it went may be in use again
+        one.args.C = products[count - 1].args.C;
+        one.args.addend = p > 0 ? one.args.C : nullptr;
+      }
+      if (std::string e = LaunchOnce(impl, &one, 1, false, alone[p], stream, launches); !e.empty()) return e;
+    }
+  }
   if (impl->prof_after) {
     cudaEventRecord(impl->prof_after, stream);
     impl->prof_used = true;
     impl->prof_before = impl->prof_after = nullptr;
   }
-  ++*launches;
   return {};
 }
 

@@ -49,7 +49,8 @@ std::string TryGemm(Context* ctx, const k::GemmArgs& args, int b_space, uint64_t
 // PrepareProduct checks the domain, makes the operands' bf16 copies as TryGemm does and fills *out; *ok = false with an
 // empty return value: not applicable.  `keep` holds the activation copy's slot, whatever happens to the activation's
 // range, until ReleaseProducts.  LaunchProducts takes one to kUmmaProducts prepared products; the epilogue of a chain is the
-// last one's.
+// last one's.  The bits are those of the products launched one after the other; where one launch would have to sum in another
+// way, or takes longer by the planner's estimates, that is what it does.
 struct PreparedProduct {
   k::GemmArgs args;
   const uint16_t* weight = nullptr;   // [N][K]

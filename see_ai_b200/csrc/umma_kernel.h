@@ -41,7 +41,8 @@ struct UmmaEpilogue {
   int addend_last = 0;
   // Up to kUmmaProducts products of one shape in one launch.  chained = 0: side by side, each with its own output
   // (`products` > 1: they share A, and every one leaves as its attention copy alone, product[p].pack_dst).
-  // chained = 1: one output, the sum of the products; their reductions follow one another.
+  // chained = 1: one output, the sum of the products: an accumulator each, scaled and added in f32 in the products' order,
+  // what launches one after the other leave.
   // Each may carry a low-rank term: after the main operands' K the reduction continues over aux_k_blocks blocks of
   // 64 from a second operand pair, T' [M, 64 * aux_k_blocks] and B' [N, 64 * aux_k_blocks] (bf16, K-major),
   // so the tile holds A W^T + T' B'^T before the epilogue scales it.  With T' and
@@ -84,12 +85,14 @@ struct UmmaGemmPlan {
   uint32_t splits = 1;      // tile kernel: CTAs that share a tile's reduction
   uint32_t grid = 0, band = 1;
   uint32_t b_box = 0;       // rows of B one TMA load brings: the box height of map_b and aux_b
+  double us = 0.0;          // the estimate it was chosen by
 };
 // k_blocks: 64-wide blocks of the whole reduction, a low-rank term's included; `group` of them in a row (1: any) are
 // not cut.  light: the epilogue only stores (f32 or a bf16 copy), without a second operand, bias or activation.
-// side_by_side: outputs of this shape in the launch.
+// side_by_side: outputs of this shape in the launch.  only_splits != 0: with the reduction cut that often.  chained: k_blocks are
+// a chain's, whose reductions are each cut (tn up to 128 only where they are).  No such plan: us = 1e30.
 UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t group, bool light, uint32_t sms,
-                          uint32_t side_by_side = 1);
+                          uint32_t side_by_side = 1, uint32_t only_splits = 0, bool chained = false);
 cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const UmmaMaps& maps, const UmmaEpilogue& ep, cudaStream_t s);
 // Piece products of an f32 activation that the kernel cuts itself (k_gemm_cut.cu; UmmaEpilogue::src_a, src_k and
 // src_a_scale are its operand): groups = blocks of 64 k.  grid == 0: the piece form is the faster one.

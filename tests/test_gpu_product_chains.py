@@ -1,8 +1,8 @@
-"""Input gradients that several relaxed products add up to, launched together (a chain), where something else that is
-launched together lies between the members: a second chain, or Q, K and V side by side.  A program run as ONE range is
-compared with the same program run one instruction per range: the frozen products are the same bf16 computation both
-ways, so the sums differ by the arithmetic of the low-rank terms and of the additions, held to 2e-6 of the terms'
-magnitudes as the folds are."""
+"""Input gradients that several relaxed products add up to, launched together (a chain), alone and where something else
+that is launched together lies between the members: a second chain, or Q, K and V side by side.  A program run as ONE
+range is compared with the same program run one instruction per range: the frozen products are the same bf16 computation
+both ways, so the sums differ by the arithmetic of the low-rank terms and of the additions, held to 2e-6 of the terms'
+magnitudes as the folds are.  And with the same range whose products are launched one by one: the same bits."""
 
 import numpy as np
 import pytest
@@ -62,10 +62,11 @@ def _f32(arena, off, n):
     return arena[off:off + 4 * n].view(np.float32).astype(np.float64)
 
 
-def _run(prog, arena0, ro, one_range=True):
+def _run(prog, arena0, ro, one_range=True, groups=True):
     arena = arena0.copy()
     be = B.CudaBackend(0)
     be.set_coherence(B.COHERENCE_LAZY)
+    be.set_product_groups(groups)
     be.bind(arena, ro)
     be.set_program(prog)
     for i, end in [(0, len(prog))] if one_range else [(i, i + 1) for i in range(len(prog))]:
@@ -113,3 +114,61 @@ def test_side_by_side_products_inside_a_chain(M):
     want, _ = _run(prog, arena0, ro, one_range=False)
     chain.check(got, want, arena0)
     assert np.array_equal(got[o:o + 4 * M * N], want[o:o + 4 * M * N])
+
+
+# (M, N, K, rank, members): the one-tile kernel at each width and cut, the persistent one, CTA pairs; ragged
+# last tiles in both directions; one and two low-rank blocks.
+CHAINS = [
+    (64, 64, 64, 4, 2), (200, 128, 128, 16, 3), (600, 512, 512, 8, 3), (600, 768, 768, 16, 3), (300, 768, 768, 8, 2),
+    (1000, 516, 520, 16, 3), (2000, 256, 256, 16, 3), (4096, 768, 768, 16, 3), (4001, 768, 768, 16, 2),
+    (4864, 2048, 192, 16, 3), (20000, 768, 320, 8, 3), (20000, 1028, 768, 16, 2),
+]
+
+
+@pytest.mark.parametrize("shape", CHAINS, ids=["x".join(map(str, c)) for c in CHAINS])
+def test_a_chain_has_the_separate_launches_bits(shape):
+    M, N, K, r, n = shape
+    rng = np.random.default_rng(M + N + K)
+    a = Arena(rng)
+    chain = Chain(a, rng, M, N, K, r, n)
+    prog = [ins for m in chain.members for ins in m] + chain.fills()
+    arena0, ro = a.build()
+    got, launches = _run(prog, arena0, ro)
+    want, launches_one_by_one = _run(prog, arena0, ro, groups=False)
+    assert np.array_equal(got[chain.out:chain.out + 4 * M * N], want[chain.out:chain.out + 4 * M * N])
+    assert np.isfinite(_f32(got, chain.out, M * N)).all()
+    assert launches_one_by_one - launches in (0, n - 1)   # (0: the planner found one by one the shorter)
+    if M >= 4000:
+        assert launches_one_by_one - launches == n - 1
+
+
+# The one-tile kernel with and without a cut, the persistent one, CTA pairs; rows that end inside a tile.
+QKV = [(192, 64, 128, 128), (600, 200, 512, 512), (600, 200, 768, 768), (304, 304, 768, 768), (512, 128, 768, 768),
+       (4096, 512, 768, 768), (20000, 160, 256, 192)]
+
+
+@pytest.mark.parametrize("shape", QKV, ids=["x".join(map(str, c)) for c in QKV])
+@pytest.mark.parametrize("n", [2, 3])
+def test_products_side_by_side_have_the_separate_launches_bits(shape, n):
+    M, S, N, K = shape
+    d, H = 64, N // 64
+    rng = np.random.default_rng(M + N + K + n)
+    a = Arena(rng)
+    x = a.alloc(M * K, "normal")
+    q, k, v, o = (a.alloc(M * N, "normal") for _ in range(4))
+    stats = a.alloc(M * H * 4)
+    outs = (q, k, v)[:n]
+    products = [P.Instr(Op.GEMM_NN_Q8, REL | CS, 0,
+                        (x, a.ro_alloc(rng.integers(-127, 128, size=K * N, dtype=np.int8)), out,
+                         a.ro_alloc((rng.random(N) * 0.001 + 1e-3).astype(np.float32))), (M, N, K)) for out in outs]
+    attention = P.Instr(Op.ATTN_FWD_TILED, REL, 0, (q, k, v, o), (stats, P.pack2(M // S, S), P.pack2(H, d)))
+    clear = [P.Instr(Op.FILL, 0, 0, (t, P.f32_bits(0.0)), (M * N, 0, 0)) for t in outs]
+    prog = products + [attention] + clear
+    arena0, ro = a.build()
+    got, launches = _run(prog, arena0, ro)
+    want, launches_one_by_one = _run(prog, arena0, ro, groups=False)
+    assert np.array_equal(got[o:o + 4 * M * N], want[o:o + 4 * M * N])
+    assert np.array_equal(got[stats:stats + 16 * M * H], want[stats:stats + 16 * M * H])
+    assert launches_one_by_one - launches in (0, n - 1)
+    if M >= 4000:
+        assert launches_one_by_one - launches == n - 1

@@ -12,7 +12,7 @@ from see_ai_b200.engine import Engine
 pytestmark = pytest.mark.gpu
 
 
-def _steps(cfg, grouped, steps=1):
+def _steps(cfg, grouped, steps=1, groups=True):
     blob = synth.build_decoder_plan(cfg)
     plan = P.Plan(blob)
     spans = [(i.ins[1], i.ins[1] + 4 * i.out[0]) for i in plan.train if i.opcode == P.Op.ADAMW_STEP]
@@ -20,6 +20,7 @@ def _steps(cfg, grouped, steps=1):
     rng = np.random.default_rng(9)
     eng = Engine(0)
     eng.backend.set_epilogue_fusion(grouped)   # (off: no group, no fold, every instruction's f32 output stored)
+    eng.backend.set_product_groups(groups)
     eng.load(blob)
     eng.set_use_graphs(True)
     state = np.frombuffer(plan.persist_init, dtype=np.uint8).copy().view(np.float32)
@@ -54,3 +55,16 @@ def test_grouped_products_give_the_separate_products_gradients(d_model, seq, seq
     assert np.isfinite(g1).all() and np.linalg.norm(g1 - g2) <= 1e-2 * np.linalg.norm(g2), np.linalg.norm(g1 - g2) / np.linalg.norm(g2)
     for (l1, _), (l2, _) in zip(got, want):
         assert abs(l1 - l2) <= 1e-3 * abs(l2)
+
+
+@pytest.mark.parametrize("targets,rank", [("qkvo", 16), ("qv", 8), ("q", 4), ("k", 8), ("qkv", 12)])
+@pytest.mark.parametrize("d_model,seq,seqs", [(128, 72, 3), (512, 200, 3), (768, 128, 4), (512, 512, 40)],
+                         ids=["one-tile", "ragged", "cut", "persistent"])
+def test_grouping_alone_leaves_every_bit(d_model, seq, seqs, targets, rank):
+    cfg = synth.DecoderConfig(layers=2, d_model=d_model, heads=d_model // 64, ffn=256, vocab=512, seq=seq, batch_seqs=seqs,
+                              rank=rank, alpha=2.0 * rank, targets=tuple(targets), quantized=True, attention="tiled", seed=3)
+    got, n_grouped = _steps(cfg, True, 4)
+    want, n_single = _steps(cfg, True, 4, groups=False)
+    assert n_grouped < n_single or d_model < 512
+    for (l1, g1), (l2, g2) in zip(got, want):
+        assert l1 == l2 and np.array_equal(g1, g2)
