@@ -1076,7 +1076,7 @@ struct FwdShape {
 struct FwdCtl {
   uint64_t q_full[2], q_empty[2];
   uint64_t full[5], empty[5];
-  uint64_t s_full[2][2], p_full[2][2], pv_done[2];   // [tile of the pair] ([score buffer])
+  uint64_t s_full[2][2], p_full[2][2], pv_done[2][2];   // [tile of the pair][score buffer]
   uint64_t out_full[2][2], out_empty[2][2], stat_full[2][2];
   uint32_t tmem_base;
   volatile uint32_t failed;
@@ -1127,9 +1127,9 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
-      MbarInit(&ctl->q_full[i], 1); MbarInit(&ctl->q_empty[i], 2); MbarInit(&ctl->pv_done[i], 1);
+      MbarInit(&ctl->q_full[i], 1); MbarInit(&ctl->q_empty[i], 2);
       for (int j = 0; j < 2; ++j) {
-        MbarInit(&ctl->s_full[i][j], 1); MbarInit(&ctl->p_full[i][j], 4);
+        MbarInit(&ctl->s_full[i][j], 1); MbarInit(&ctl->p_full[i][j], 4); MbarInit(&ctl->pv_done[i][j], 1);
         MbarInit(&ctl->out_full[i][j], 1); MbarInit(&ctl->out_empty[i][j], 4); MbarInit(&ctl->stat_full[i][j], 4);
       }
     }
@@ -1183,13 +1183,13 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       const uint32_t qb = i % Sh::kQBufs, steps = u.Steps(tile), ob = j % Sh::kOutBufs;
       if (!(ok = WarpWait(ctl, &ctl->q_full[qb], (i / Sh::kQBufs) & 1))) break;
       const uint8_t* q = q_s + qb * 2 * Sh::kQ + tile * Sh::kQ;
-      // The scores of step t (this tile's step m) into their buffer, whose last reader is P V two steps ago.  (A new
-      // tile's first step waits for the whole of the tile before: a parity tells one phase from the next only.)
+      // The scores of step t (this tile's step m) into their buffer, whose last reader is P V two steps ago.  (A parity
+      // tells one phase from the next only, so either buffer has a barrier of its own: its step m - 4 was waited for
+      // before m - 2 was issued, also where a tile ended in between.)
       auto scores = [&](uint32_t t, uint32_t m) {
         const uint32_t at = g + t, s = at % Sh::kStages;
         if (!WarpWait(ctl, &ctl->full[s], (at / Sh::kStages) & 1)) return false;
-        const uint32_t back = t == 0 ? 1 : 2;
-        if (m >= back && !WarpWait(ctl, &ctl->pv_done[tile], (m - back) & 1)) return false;
+        if (m >= 2 && !WarpWait(ctl, &ctl->pv_done[tile][m & 1], ((m >> 1) - 1) & 1)) return false;
         TcFenceAfter();
         if (ElectOne()) {
           MmaRowRow<D, 64>(base + (m & 1) * 64, q, ring_s + s * 2 * Sh::kStep);
@@ -1214,7 +1214,7 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             for (uint32_t k = 0; k < 4; ++k)
               UmmaBf16TmemA(base + Sh::kOutCol + ob * D, base + (n & 1) * 64 + k * 8, MakeSmemDescMn(v + k * 2048, 64 * 128),
                             idesc, (t | k) != 0 ? 1u : 0u);
-            UmmaCommit(&ctl->pv_done[tile]);
+            UmmaCommit(&ctl->pv_done[tile][n & 1]);
             UmmaCommit(&ctl->empty[s]);
             if (t + 1 == steps) UmmaCommit(&ctl->out_full[tile][ob]);
           }
@@ -1281,7 +1281,7 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           ref = step_ref;
         }
         if (t > 0 && __any_sync(0xFFFFFFFFu, moves)) {       // the warp's rows rescale their O lanes together
-          if (!(ok = WarpWait(ctl, &ctl->pv_done[tile], (n - 1) & 1))) break;
+          if (!(ok = WarpWait(ctl, &ctl->pv_done[tile][(n - 1) & 1], ((n - 1) >> 1) & 1))) break;
           TcFenceAfter();
 #pragma unroll 1
           for (uint32_t c0 = 0; c0 < D; c0 += 16) {
