@@ -1245,7 +1245,7 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       const uint32_t t_o = t_base + Sh::kOutCol + ob * D;
       float raw_max = -INFINITY;   // the row's true score maximum so far
       float ref = -INFINITY;       // the exponent (log2 units) its p, sum and O are relative to
-      F2 sum = Pair(0.0f, 0.0f);
+      float l = 0.0f;              // the row's sum: one chain, the order of the kernel above
       for (uint32_t t = 0; t < steps; ++t, ++n) {
         if (!(ok = WarpWait(ctl, &ctl->s_full[tile][n & 1], (n >> 1) & 1))) break;
         TcFenceAfter();
@@ -1277,7 +1277,7 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         float alpha = 1.0f;
         if (moves) {
           alpha = Exp2Approx(ref - step_ref);                // 0 the first time
-          sum = Mul2(sum, Pair(alpha, alpha));
+          l *= alpha;
           ref = step_ref;
         }
         if (t > 0 && __any_sync(0xFFFFFFFFu, moves)) {       // the warp's rows rescale their O lanes together
@@ -1301,7 +1301,8 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           for (int e = 0; e < 32; e += 2) {
             const F2 y = Fma2(Pair(__uint_as_float(x[e]), __uint_as_float(x[e + 1])), scale, shift);
             const float p0 = Exp2Approx(Lo(y)), p1 = Exp2Approx(Hi(y));
-            sum = Add2(sum, Pair(p0, p1));
+            l += p0;
+            l += p1;
             x[e / 2] = PackBf16x2(p0, p1);
           }
         };
@@ -1317,7 +1318,6 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         if (lane == 0) MbarArrive(&ctl->p_full[tile][n & 1]);
       }
       if (!ok) break;
-      const float l = Lo(sum) + Hi(sum);
       if (row < a.S) {
         // The stats row speaks of the true maximum: the sum relative to it is l 2^(ref - max c).
         const float m = raw_max * a.inv_sqrt_d;

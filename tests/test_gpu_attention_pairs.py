@@ -63,3 +63,14 @@ def test_several_pairs_to_a_cta_against_float64(geom):
         inv = 1.0 / torch.exp(s - m[..., None]).sum(dim=-1)
         assert np.abs(stats[b, :, :, 0] - m.cpu().numpy()).max() <= 1e-4
         assert np.abs(stats[b, :, :, 1] / inv.cpu().numpy() - 1.0).max() <= 2e-4
+
+
+@pytest.mark.parametrize("geom", [(6, 136, 12, 64), (3, 520, 8, 64), (5, 264, 6, 128)], ids=lambda g: "B%dS%dH%dd%d" % g)
+def test_the_first_tile_has_the_bits_of_a_sequence_that_is_only_that(geom):
+    """Causal: the first 128 positions know nothing of the rest, and a sequence of 128 has the one-tile kernel."""
+    Bq, S, H, d = geom
+    x = _inputs(np.random.default_rng(S + d), *geom)
+    o, stats = _forward({n: v.reshape(-1) for n, v in x.items()}, *geom)
+    one, one_stats = _forward({n: np.ascontiguousarray(v[:, :128]).reshape(-1) for n, v in x.items()}, Bq, 128, H, d)
+    assert np.array_equal(o[:, :128], one)
+    assert np.array_equal(stats[:, :, :128], one_stats)
