@@ -116,8 +116,8 @@ __global__ void XEntRowsKernel(const float* __restrict__ logits, const int32_t* 
 // (up to eight 16-byte vectors per thread), so the logits are read from HBM once and the probabilities written once.
 // The next row is copied into shared memory asynchronously (cp.async) while the current one is reduced, each thread
 // fetching exactly the chunks it will later read itself, so no barrier guards the buffer.  Same expressions per
-// element as RowSoftmaxBlock; the row sum is folded as thread partials (ascending index), warp shuffles, then warps in
-// order.
+// element as RowSoftmaxBlock; the row sum is folded as the partials of 1024 threads (ascending index), warp shuffles, then
+// the 32 warps in order, whatever the block's size: a thread of a smaller block holds the partials of several.
 // A row's two reductions are a chain of barriers that moves no bytes, so what counts is how many rows an SM has in
 // hand at once: four 256-thread blocks up to 8192 columns, two of 512 up to 16384, one of 1024 above.  (4096 rows of
 // 4096 columns: 82 us with 1024 threads to a row, 23 with 256.  The two halves of a 32000-wide row in a cluster of two,
@@ -164,7 +164,6 @@ XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__
     }
     if (n + gridDim.x < N) prefetch(n + gridDim.x);
     auto max2 = [](float a, float b) { return fmaxf(a, b); };
-    auto add2 = [](float a, float b) { return a + b; };
     mx = BlockReduce<float>(mx, -INFINITY, smem_f, WarpMax, max2);
     // e^{x - mx} = 2^{x log2 e - mx log2 e} on the hardware exponential: one FMA and
     // one MUFU per element (libm expf is about twenty instructions, and a
@@ -172,9 +171,11 @@ XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__
     // at the far end of the row, inside the 1e-5 these rows are held to.
     constexpr float kLog2E = 1.4426950408889634f;
     const float shift = -mx * kLog2E;
-    float sum = 0.0f;
+    constexpr int kParts = 1024 / kThreads;   // column quad i of this thread is one of thread (i % kParts) kThreads + tid's
+    float part[kParts] = {};
 #pragma unroll
     for (int i = 0; i < kWideVecs; ++i) {
+      float& sum = part[i % kParts];
       if (i * kThreads + tid < C4) {
         x[i].x = Ex2Approx(__fmaf_rn(x[i].x, kLog2E, shift)); sum += x[i].x;
         x[i].y = Ex2Approx(__fmaf_rn(x[i].y, kLog2E, shift)); sum += x[i].y;
@@ -182,7 +183,17 @@ XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__
         x[i].w = Ex2Approx(__fmaf_rn(x[i].w, kLog2E, shift)); sum += x[i].w;
       }
     }
-    sum = BlockReduce<float>(sum, 0.0f, smem_f, WarpSumF, add2);
+#pragma unroll
+    for (int v = 0; v < kParts; ++v) part[v] = WarpSumF(part[v]);
+    __syncthreads();
+    if ((tid & 31) == 0) {
+#pragma unroll
+      for (int v = 0; v < kParts; ++v) smem_f[v * (kThreads / 32) + (tid >> 5)] = part[v];
+    }
+    __syncthreads();
+    float sum = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) sum += smem_f[w];
     const float inv_sum = 1.0f / sum;
     float4* prow = reinterpret_cast<float4*>(probs + n * C);
     const int32_t lab = labels[n];

@@ -57,6 +57,30 @@ def test_wide_rows_against_double(rows, classes, masked):
     assert abs(float(arena[loss:loss + 4].view(np.float32)[0]) - want) <= 1e-5 * abs(want)
 
 
+@pytest.mark.parametrize("rows,classes", [(1, 4096), (600, 5000), (700, 8000), (3, 8192), (300, 8196), (5, 16384)])
+def test_the_bits_do_not_depend_on_the_threads_to_a_row(rows, classes):
+    """A row padded with -inf to 32768 columns (1024 threads to a row) has the same sums, with zeros added."""
+    rng = np.random.default_rng(rows + classes)
+    x = (rng.standard_normal((rows, classes)) * 4.0).astype(np.float32)
+    y = rng.integers(0, classes, size=rows, dtype=np.int32)
+
+    def run(width):
+        a = Arena(rng)
+        logits = a.alloc(rows * width, np.pad(x, ((0, 0), (0, width - classes)), constant_values=-np.inf))
+        labels = a.alloc(rows, y.view(np.float32))
+        loss, probs = a.alloc(1), a.alloc(rows * width)
+        arena, ro = a.build()
+        be = B.CudaBackend(0)
+        be.bind(arena, ro)
+        be.run([P.Instr(Op.XENT_FWD, 0, 0, (logits, labels, loss, probs), (rows, width, 0))])
+        be.close()
+        return (arena[probs:probs + 4 * rows * width].view(np.float32).reshape(rows, width)[:, :classes].copy(),
+                arena[loss:loss + 4].view(np.float32)[0])
+
+    (p, l), (q, m) = run(classes), run(32768)
+    assert np.array_equal(p, q) and l == m
+
+
 @pytest.mark.parametrize("rows,classes", [(223, 128), (224, 132), (225, 1024), (700, 131)])
 def test_eval_tail_over_several_chunks_of_rows(rows, classes):
     rng = np.random.default_rng(rows)
