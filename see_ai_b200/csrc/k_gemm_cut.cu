@@ -268,6 +268,7 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
     }
     TcFenceBefore();
   }
+  __syncwarp();   // (one lane of the loading and of the issuing warp has walked the blocks: the barriers want whole warps)
   if (splits > 1) ClusterSync();
   else if (work) asm volatile("bar.sync 1, %0;" ::"n"(kWorkThreads) : "memory");
   if (work && ok) {

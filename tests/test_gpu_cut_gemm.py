@@ -7,6 +7,7 @@ import pytest
 
 from see_ai_b200 import backend as B
 from see_ai_b200 import plan as P
+from tests.test_gpu_umma import bf16_round
 from tests.test_oracle_pinned import Arena
 
 pytestmark = pytest.mark.gpu
@@ -74,3 +75,64 @@ def test_against_double(shape, bad):
         err = np.abs(g[rows] - ref[rows])
         assert np.sqrt(np.mean(err ** 2)) <= 4e-7 * rms, k
         assert err.max() <= 8e-6 * rms, k
+
+
+# Each kernel of the form, by the planner's choice on 148 SMs: (M, N, K), weight, the tile width and the CTAs that share a
+# tile's K.
+FORMS = [
+    ((4096, 256, 256), "f32", 64, 1), ((1023, 256, 256), "f32", 64, 4), ((600, 2048, 512), "f32", 128, 1),
+    ((256, 4096, 512), "f32", 128, 2), ((640, 514, 320), "f32", 128, 4),
+    ((2000, 385, 96), "int8", 64, 1), ((128, 1024, 1024), "bf16", 64, 4), ((300, 5000, 256), "bf16", 128, 1),
+    ((4096, 256, 256), "int8", 128, 2), ((640, 514, 320), "bf16", 128, 4), ((4096, 768, 768), "int8", 192, 1),
+    ((2048, 768, 1024), "bf16", 192, 2), ((1000, 768, 3072), "int8", 192, 4), ((600, 2048, 512), "bf16", 192, 2),
+]
+
+
+@pytest.mark.parametrize("form", FORMS, ids=["%dx%dx%d-%s-w%d-c%d" % (*f[0], *f[1:]) for f in FORMS])
+def test_each_kernel_of_the_form(form):
+    (M, N, K), kind, _, _ = form
+    rng = np.random.default_rng(M + N + K)
+    a = Arena(rng)
+    x = a.alloc(M * K, "normal")
+    out = a.alloc(M * N)
+    if kind == "int8":
+        w = rng.integers(-127, 128, size=(K, N), dtype=np.int8)
+        scale = (rng.random(N) * 0.01 + 1e-3).astype(np.float32)
+        ins = P.Instr(Op.GEMM_NN_Q8, P.FLAG_Q8_COL_SCALE, 0, (x, a.ro_alloc(w), out, a.ro_alloc(scale)), (M, N, K))
+        w64 = w.astype(np.float64) * scale
+    else:
+        w = rng.standard_normal((K, N)).astype(np.float32)
+        if kind == "bf16":
+            w = bf16_round(w.reshape(-1)).reshape(K, N)
+        stored = (w.view(np.uint32) >> 16).astype(np.uint16) if kind == "bf16" else w
+        ins = P.Instr(Op.GEMM_NN_BF16 if kind == "bf16" else Op.GEMM_NN, 0, 0, (x, a.ro_alloc(stored), out, P.NULL_REF), (M, N, K))
+        w64 = w.astype(np.float64)
+    arena0, ro = a.build()
+    A = arena0[x:x + 4 * M * K].view(np.float32).reshape(M, K)
+    bad_row, bad_k = M - 1, K // 3
+    finite = A.copy()
+    A[bad_row, bad_k] = np.inf
+    arena = arena0.copy()
+    be = B.CudaBackend(0)
+    be.set_coherence(B.COHERENCE_LAZY)
+    be.bind(arena, ro)
+    be.set_program([ins])
+    results, launches = [], []
+    for _ in range(3):
+        be.run(None)
+        be.host_needs(out, 4 * M * N)
+        be.flush()
+        launches.append(be.counters().kernel_launches)
+        results.append(arena[out:out + 4 * M * N].view(np.float32).reshape(M, N).copy())
+    assert be.counters().split_executions == 3
+    be.close()
+    # the weight's pieces are made once; a matrix of A's pieces would be a launch of its own each time
+    assert launches[2] - launches[1] == launches[1] - launches[0] == 1
+    assert np.array_equal(results[0], results[1], equal_nan=True) and np.array_equal(results[1], results[2], equal_nan=True)
+    got = results[0].astype(np.float64)
+    with np.errstate(invalid="ignore"):
+        assert np.array_equal(results[0][bad_row], (np.inf * w64[bad_k]).astype(np.float32), equal_nan=True)
+    want = finite.astype(np.float64)[:bad_row] @ w64
+    rms = np.sqrt(np.mean(want ** 2))
+    err = np.abs(got[:bad_row] - want)
+    assert np.sqrt(np.mean(err ** 2)) <= 4e-7 * rms and err.max() <= 8e-6 * rms   # as above
