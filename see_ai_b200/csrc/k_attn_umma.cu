@@ -1410,10 +1410,32 @@ static cudaError_t LaunchFwdPair(const CUtensorMap& q, const CUtensorMap& k, con
   return cudaGetLastError();
 }
 
+// Which forward takes a geometry (both give the same bits).  Pairs share the keys' steps and keep the exponentials' pipe
+// busy, but an SM works one pair at a time in whole rounds, and a short walk does not repay its longer set-up; the
+// one-tile form has four CTAs to an SM (two for d = 128), started at once.  Measured on a B200, pairs / one tile, us, d = 64:
+//   3 steps of keys: 24 heads of 192 positions 9.9 / 9.5, 192 of them (1.3 rounds) 15.2 / 12.1, 256 15.1 / 14.0; once the one-tile
+//     CTAs are no longer all resident, 384, 18.6 / 19.4
+//   4 steps: 48 of 256 10.2 / 11.2, 192 (1.3 rounds) 16.2 / 14.5, 256 (1.73) 16.0 / 16.9, 384 20.7 / 22.2
+//   5 steps, three tiles, the last with a CTA of pairs to itself: 48 of 320 10.8 / 12.7, 96 (1.3 rounds) 15.6 / 14.0, 144 (1.95)
+//     15.5 / 16.1, 192 (2.59) 19.5 / 18.0, 256 (3.46, not all resident) 24.1 / 24.8
+//   6 steps: 96 of 384 15.5 / 15.6, 192 20.4 / 20.0, others 0.72 to 0.92; from 7 on pairs always
+// and d = 128: 3 steps, 64 of 192 13.1 / 11.5, 128 15.1 / 13.5, 192 (not all resident) 21.3 / 21.2; 4 steps, 8 of 256 12.9 / 12.6,
+// 128 15.3 / 15.9.
+static bool PairsForward(const AttnUmmaArgs& a) {
+  const uint64_t steps = (a.S + kHalf - 1) / kHalf, tiles = (a.S + kTile - 1) / kTile, heads = static_cast<uint64_t>(a.B) * a.H;
+  const uint64_t ctas = tiles * heads, units = (tiles + 1) / 2 * heads, sms = a.sms;
+  const bool resident = ctas <= (a.d == 64 ? 4u : 2u) * sms;
+  if (steps <= 2) return false;   // a single tile has no neighbour to share its keys with
+  if (steps == 3) return !resident;
+  if (a.d == 128) return steps > 4 || ctas > sms;
+  if (steps > 5 || !resident || units <= sms) return true;
+  const uint64_t rounds = (units + sms - 1) / sms;
+  return units * 10 >= rounds * sms * (steps == 4 ? 8 : 9);   // the last round is nearly full
+}
+
 cudaError_t AttnFwdUmma(const CUtensorMap& q, const CUtensorMap& k_half, const CUtensorMap& v_half,
                         const AttnUmmaArgs& a, cudaStream_t s) {
-  // (A single tile a sequence has no neighbour to share its keys with: four small CTAs to an SM do better there.)
-  if (a.S > kTile) return a.d == 64 ? LaunchFwdPair<64>(q, k_half, v_half, a, s) : LaunchFwdPair<128>(q, k_half, v_half, a, s);
+  if (PairsForward(a)) return a.d == 64 ? LaunchFwdPair<64>(q, k_half, v_half, a, s) : LaunchFwdPair<128>(q, k_half, v_half, a, s);
   dim3 grid((a.S + kTile - 1) / kTile, a.B * a.H);
   const size_t smem = AttnFwdSmem(a.d);
   cudaError_t e;

@@ -40,7 +40,7 @@ def _inputs(rng, Bq, S, H, d):
 
 # 3 rounds of a CTA's pairs and an odd number of tiles; one pair a sequence; two rounds at d = 128 (one output buffer);
 # a last tile of one step, of two.
-GEOMS = [(8, 520, 20, 64), (37, 136, 12, 64), (9, 264, 20, 128), (20, 200, 16, 128), (2, 1160, 40, 64)]
+GEOMS = [(8, 520, 20, 64), (56, 136, 12, 64), (9, 264, 20, 128), (20, 200, 16, 128), (2, 1160, 40, 64)]
 
 
 @pytest.mark.parametrize("geom", GEOMS, ids=["B%dS%dH%dd%d" % g for g in GEOMS])
@@ -65,7 +65,7 @@ def test_several_pairs_to_a_cta_against_float64(geom):
         assert np.abs(stats[b, :, :, 1] / inv.cpu().numpy() - 1.0).max() <= 2e-4
 
 
-@pytest.mark.parametrize("geom", [(6, 136, 12, 64), (3, 520, 8, 64), (5, 264, 6, 128)], ids=lambda g: "B%dS%dH%dd%d" % g)
+@pytest.mark.parametrize("geom", [(32, 136, 12, 64), (3, 520, 8, 64), (5, 264, 6, 128)], ids=lambda g: "B%dS%dH%dd%d" % g)
 def test_the_first_tile_has_the_bits_of_a_sequence_that_is_only_that(geom):
     """Causal: the first 128 positions know nothing of the rest, and a sequence of 128 has the one-tile kernel."""
     Bq, S, H, d = geom
@@ -74,3 +74,17 @@ def test_the_first_tile_has_the_bits_of_a_sequence_that_is_only_that(geom):
     one, one_stats = _forward({n: np.ascontiguousarray(v[:, :128]).reshape(-1) for n, v in x.items()}, Bq, 128, H, d)
     assert np.array_equal(o[:, :128], one)
     assert np.array_equal(stats[:, :, :128], one_stats)
+
+
+# (batches of the same sequences, S, H, d): either side of each line between the two kernels.
+LINES = [((2, 26), 192, 12, 64), ((16, 22), 256, 12, 64), ((8, 12, 16, 22), 320, 12, 64), ((4, 22), 136, 8, 128), ((2, 22), 256, 8, 128)]
+
+
+@pytest.mark.parametrize("line", LINES, ids=lambda l: "S%dH%dd%d" % l[1:])
+def test_a_sequence_has_the_same_bits_in_every_batch(line):
+    batches, S, H, d = line
+    x = _inputs(np.random.default_rng(S + d), max(batches), S, H, d)
+    o, stats = _forward({n: v.reshape(-1) for n, v in x.items()}, max(batches), S, H, d)
+    for b in batches[:-1]:
+        few, few_stats = _forward({n: np.ascontiguousarray(v[:b]).reshape(-1) for n, v in x.items()}, b, S, H, d)
+        assert np.array_equal(few, o[:b]) and np.array_equal(few_stats, stats[:b])
