@@ -224,9 +224,20 @@ constexpr int kTile = 64;      // rows of the streamed axis per step
 constexpr int kSlice = 8;      // features of a streamed tile in shared memory at a time
 constexpr int kTileThreads = 256;
 constexpr int kGroup = 128;            // threads of a group
-constexpr int kStreamLd = kTile + 4;   // doubles per feature of a streamed slice: a multiple of 16 bytes, and four features' rows
-                                       // in four different quarters of the banks, as the tensor instruction's fragments want them
-__host__ __device__ constexpr int OwnLd(int rows) { return rows + 4; }   // likewise of the block's own rows
+constexpr int kStreamLd = kTile + 2;   // doubles per feature of a streamed slice (a multiple of 16 bytes; 2-way store conflicts)
+// Where row r of feature c lies in a streamed slice, and among the block's own rows.  kMma: the tensor instruction's
+// fragments are four features of the same rows at once, so these turn the rows into four different quarters of the banks.
+// (Padding did that too, at an eighth to a half more shared memory, and fewer rows fitted a block: forward of 8 x 480
+// positions of 12 heads of 128 406 us, 284 turned; dQ of 8 x 448 of those 903 and 556, of 8 x 600 of 12 heads of 64 798 and 500;
+// 8 x 512 of 12 heads of 64 185 and 184.)
+template <bool kMma>
+__device__ __forceinline__ int StreamAt(int c, int r) {
+  return kMma ? c * kTile + (r ^ ((c & 3) << 2) ^ ((c & 4) << 1)) : c * kStreamLd + r;
+}
+template <bool kMma, int kRows>
+__device__ __forceinline__ int OwnAt(int c, int r) {
+  return c * kRows + (kMma ? r ^ (kRows == 8 ? (c & 2) << 1 : (c & 3) << 2) : r);
+}
 constexpr int kChunkRows = 32;         // rows of an f32 tile in shared memory at a time
 
 __host__ __device__ constexpr int PaddedFeatures(int d) { return (d + kSlice - 1) / kSlice * kSlice; }
@@ -237,17 +248,17 @@ __device__ __forceinline__ float4 LoadFour(const float* __restrict__ p, int left
   return make_float4(p[0], left > 1 ? p[1] : 0.0f, left > 2 ? p[2] : 0.0f, left > 3 ? p[3] : 0.0f);
 }
 
-// The block's own rows, widened to double once: dst[feature][OwnLd(kRows)], zero outside (0 * 0 leaves a chain as it is).
-template <int kRows, bool kVec>
+// The block's own rows, widened to double once: dst[feature][kRows], zero outside (0 * 0 leaves a chain as it is).
+template <int kRows, bool kVec, bool kMma>
 __device__ __forceinline__ void LoadOwn(double* dst, const float* __restrict__ src, size_t stride, int rows, int d) {
   const int quads = PaddedFeatures(d) / 4;
   for (int t = threadIdx.x; t < kRows * quads; t += kTileThreads) {
     const int r = t / quads, c = t % quads * 4;
     const float4 f = LoadFour(src + static_cast<size_t>(min(r, rows - 1)) * stride + c, r < rows ? d - c : 0, kVec);
-    dst[c * OwnLd(kRows) + r] = f.x;
-    dst[(c + 1) * OwnLd(kRows) + r] = f.y;
-    dst[(c + 2) * OwnLd(kRows) + r] = f.z;
-    dst[(c + 3) * OwnLd(kRows) + r] = f.w;
+    dst[OwnAt<kMma, kRows>(c, r)] = f.x;
+    dst[OwnAt<kMma, kRows>(c + 1, r)] = f.y;
+    dst[OwnAt<kMma, kRows>(c + 2, r)] = f.z;
+    dst[OwnAt<kMma, kRows>(c + 3, r)] = f.w;
   }
 }
 
@@ -270,12 +281,13 @@ __device__ __forceinline__ void FetchSlice(SliceRegs* s, const float* __restrict
   const int r = InGroup() >> 1, c = c0 + (InGroup() & 1) * 4;
   s->v = LoadFour(src + static_cast<size_t>(min(r, rows - 1)) * stride + c, r < rows ? d - c : 0, kVec);
 }
+template <bool kMma>
 __device__ __forceinline__ void StoreSlice(double* dst, const SliceRegs& s) {
   const int r = InGroup() >> 1, c = (InGroup() & 1) * 4;
-  dst[c * kStreamLd + r] = s.v.x;
-  dst[(c + 1) * kStreamLd + r] = s.v.y;
-  dst[(c + 2) * kStreamLd + r] = s.v.z;
-  dst[(c + 3) * kStreamLd + r] = s.v.w;
+  dst[StreamAt<kMma>(c, r)] = s.v.x;
+  dst[StreamAt<kMma>(c + 1, r)] = s.v.y;
+  dst[StreamAt<kMma>(c + 2, r)] = s.v.z;
+  dst[StreamAt<kMma>(c + 3, r)] = s.v.w;
 }
 
 // Which pair (row of the block's own, row of the streamed tile) a thread's accumulator acc[r][e] stands for; e and e + 1
@@ -315,31 +327,33 @@ template <int RM, bool kVec, bool kMma>
 __device__ __forceinline__ void DotTile(const double* own, const float* b, int rows, const float* next, int next_rows,
                                         size_t stride, int d, double* slices, int* turn, SliceRegs* regs,
                                         double (&acc)[RM][4]) {
-  constexpr int R = 8 * RM, kLd = OwnLd(R);
+  constexpr int R = 8 * RM;
   const int tx = threadIdx.x & 15, ty = InGroup() >> 4;
 #pragma unroll
   for (int r = 0; r < RM; ++r)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[r][e] = 0.0;
+  // kMma: this lane's fragments in a slice and among the own rows, the even and the odd eights of rows; four features on,
+  // own rows lie as they did and a slice's eights have changed places.
+  [[maybe_unused]] const int g = static_cast<int>(threadIdx.x & 31) / 4, t = threadIdx.x & 3, w = (InGroup() >> 5) * 16 + g;
+  [[maybe_unused]] const int f0 = StreamAt<true>(t, w), f1 = StreamAt<true>(t, w + 8);
+  [[maybe_unused]] const int e0 = OwnAt<true, R>(t, g), e1 = OwnAt<true, R>(t, g + 8);
   for (int c0 = 0; c0 < d; c0 += kSlice) {
     double* sb = slices + *turn * (kSlice * kStreamLd);
     *turn ^= 1;
-    StoreSlice(sb, *regs);
+    StoreSlice<kMma>(sb, *regs);
     GroupSync();
     if (c0 + kSlice < d) FetchSlice<kVec>(regs, b, stride, rows, c0 + kSlice, d);
     else if (next) FetchSlice<kVec>(regs, next, stride, next_rows, 0, d);
     if constexpr (kMma) {
-      const int g = static_cast<int>(threadIdx.x & 31) / 4, t = threadIdx.x & 3;
-      const double* sa = own + (c0 + t) * kLd + g;
-      const double* bb = sb + t * kStreamLd + (InGroup() >> 5) * 16 + g;
+      const double* sa = own + c0 * R;
       double y[2][2];
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        y[n][0] = bb[8 * n];
-        y[n][1] = bb[4 * kStreamLd + 8 * n];
-      }
+      y[0][0] = sb[f0];
+      y[1][0] = sb[f1];
+      y[0][1] = sb[f1 + 4 * kTile];
+      y[1][1] = sb[f0 + 4 * kTile];
       if constexpr (RM == 1) {
-        const double x0 = sa[0], x1 = sa[4 * kLd];
+        const double x0 = sa[e0], x1 = sa[e0 + 4 * R];
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           DMma8(acc[0], 2 * n, x0, y[n][0]);
@@ -348,13 +362,13 @@ __device__ __forceinline__ void DotTile(const double* own, const float* b, int r
       } else {
 #pragma unroll
         for (int m = 0; m + 1 < RM; m += 2) {
-          const double x[4] = {sa[8 * m], sa[8 * m + 8], sa[4 * kLd + 8 * m], sa[4 * kLd + 8 * m + 8]};
+          const double x[4] = {sa[e0 + 8 * m], sa[e1 + 8 * m], sa[e0 + 4 * R + 8 * m], sa[e1 + 4 * R + 8 * m]};
 #pragma unroll
           for (int n = 0; n < 2; ++n) DMma16(acc[m], acc[m + 1], 2 * n, x, y[n]);
         }
       }
     } else {
-      const double* sa = own + c0 * kLd + ty * RM;
+      const double* sa = own + c0 * R + ty * RM;
 #pragma unroll
       for (int c = 0; c < kSlice; ++c) {
         const double2 y0 = *reinterpret_cast<const double2*>(sb + c * kStreamLd + 2 * tx);
@@ -362,7 +376,7 @@ __device__ __forceinline__ void DotTile(const double* own, const float* b, int r
         const double y[4] = {y0.x, y0.y, y1.x, y1.y};
         double x[RM];
 #pragma unroll
-        for (int r = 0; r < RM; ++r) x[r] = sa[c * kLd + r];
+        for (int r = 0; r < RM; ++r) x[r] = sa[c * R + r];
 #pragma unroll
         for (int r = 0; r < RM; ++r)
 #pragma unroll
@@ -374,7 +388,7 @@ __device__ __forceinline__ void DotTile(const double* own, const float* b, int r
 
 __host__ __device__ constexpr size_t GroupBytes() { return 2 * sizeof(double) * kSlice * kStreamLd; }
 __host__ __device__ constexpr size_t StreamBytes() { return 2 * GroupBytes(); }
-__host__ __device__ constexpr size_t OwnBytes(int RM, int d) { return sizeof(double) * PaddedFeatures(d) * OwnLd(8 * RM); }
+__host__ __device__ constexpr size_t OwnBytes(int RM, int d) { return sizeof(double) * PaddedFeatures(d) * 8 * RM; }
 
 // Rows [0, rows) x columns [c0, c0 + 64) of a [., stride] f32 matrix into dst[32][64] by asynchronous copies (zero
 // outside); one commit group.
@@ -511,7 +525,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnFwdTileKernel(
   int turn = 0;
   const int first = GroupOf() * kTile;
   if (first < nkeys) FetchSlice<kVec>(&regs, k + base + static_cast<size_t>(first) * D, D, min(kTile, S - first), 0, d);
-  LoadOwn<R, kVec>(own, q + base + static_cast<size_t>(i0) * D, D, nrows, d);
+  LoadOwn<R, kVec, kFused>(own, q + base + static_cast<size_t>(i0) * D, D, nrows, d);
   __syncthreads();
   for (int k0 = first; k0 < nkeys; k0 += 2 * kTile) {
     double acc[RM][4];
@@ -605,7 +619,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __
   int turn = 0;
   const int first = GroupOf() * kTile;
   if (first < nkeys) FetchSlice<kVec>(&regs, v + base + static_cast<size_t>(first) * D, D, min(kTile, S - first), 0, d);
-  LoadOwn<R, kVec>(own, dout + base + static_cast<size_t>(i0) * D, D, min(R, S - i0), d);
+  LoadOwn<R, kVec, kMma>(own, dout + base + static_cast<size_t>(i0) * D, D, min(R, S - i0), d);
   __syncthreads();
   for (int k0 = first; k0 < S; k0 += 2 * kTile) {
     double acc[RM][4] = {};
@@ -793,8 +807,8 @@ __global__ __launch_bounds__(kTileThreads) void AttnDQTiledTileKernel(
   int turn = 0;
   const int first = GroupOf() * kTile;
   if (first < nkeys) FetchSlice<kVec>(&regs, k + base + static_cast<size_t>(first) * D, D, min(kTile, S - first), 0, d);
-  LoadOwn<R, kVec>(own_q, q + at, D, nrows, d);
-  LoadOwn<R, kVec>(own_do, dout + at, D, nrows, d);
+  LoadOwn<R, kVec, kFused>(own_q, q + at, D, nrows, d);
+  LoadOwn<R, kVec, kFused>(own_do, dout + at, D, nrows, d);
   __syncthreads();
   for (int k0 = first; k0 < nkeys; k0 += 2 * kTile) {
     const float *kb = k + base + static_cast<size_t>(k0) * D, *vb = v + base + static_cast<size_t>(k0) * D;
@@ -884,8 +898,8 @@ __global__ __launch_bounds__(kTileThreads) void AttnDKVTiledTileKernel(
   int turn = 0;
   const int i_first = j0 / kTile * kTile, mine = i_first + group * kTile;
   if (mine < S) FetchSlice<kVec>(&regs, q + base + static_cast<size_t>(mine) * D, D, min(kTile, S - mine), 0, d);
-  LoadOwn<R, kVec>(own_k, k + at, D, nkeys, d);
-  if (kWantDK) LoadOwn<R, kVec>(own_v, v + at, D, nkeys, d);
+  LoadOwn<R, kVec, kFused>(own_k, k + at, D, nkeys, d);
+  if (kWantDK) LoadOwn<R, kVec, kFused>(own_v, v + at, D, nkeys, d);
   __syncthreads();
   for (int pair = i_first; pair < S; pair += 2 * kTile) {
     // The rows of x these tiles need, on their way while the scores are formed.

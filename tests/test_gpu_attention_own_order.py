@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
 SHAPES = [   # B, S, H, d: one, two and four rows per thread; remainders of 8 features, 16 and 64 rows
     (1, 1, 1, 8), (1, 65, 3, 64), (1, 130, 1, 66), (2, 64, 1, 20), (1, 257, 1, 33), (10, 70, 10, 12), (20, 65, 16, 8), (8, 129, 12, 64),
 ]
+FULL_BLOCKS = [(5, 480, 4, 128), (5, 600, 2, 64)]   # score rows and operands that fill what shared memory two blocks of 32 or 16 rows have
 
 
 def setup_module(_m):
@@ -24,7 +25,7 @@ def setup_module(_m):
 
 
 @pytest.mark.parametrize("segments", [0, 1], ids=["causal", "segments"])
-@pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
+@pytest.mark.parametrize("shape", SHAPES + FULL_BLOCKS, ids=["x".join(map(str, s)) for s in SHAPES + FULL_BLOCKS])
 def test_every_instruction_from_the_oracles_bytes(shape, segments):
     prog, arena = _program(*shape, segments, cached=True)
     cpu, gpu = arena.copy(), arena.copy()
