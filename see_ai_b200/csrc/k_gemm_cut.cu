@@ -348,9 +348,9 @@ UmmaCutPlan UmmaPlanCut(uint32_t M, uint32_t N, uint32_t groups, bool exact_b, u
   // take about 1.2 us to cut a block and add one (1.4 at a tile width of 128 or 192), fall behind the piece form's
   // tensor time, and every further column tile cuts A again.  Measured on a B200, the piece form's kernel (+ its cut of A) / this,
   // us, f32 weights: 4096 x 256 x 256 14.0 (+2.8) / 9.7, 1024 x 256 x 256 8.4 (+2.0) / 8.0, 600 x 512 x 512 12.3 (+2.1) / 10.7,
-  // 128 x 1024 x 1024 14.7 (+2.0) / 11.1, 300 x 5000 x 256 15.1 (+1.9) / 11.8, 4096 x 256 x 1024 21.7 (+5.9) / 23.6; past the line
+  // 128 x 1024 x 1024 14.7 (+2.0) / 11.1, 300 x 5000 x 256 15.1 (+1.9) / 11.8, 4096 x 256 x 1024 21.7 (+5.9) / 18.5; past the line
   // 2048 x 512 x 2048 32.1 (+5.9) / 42.0, 4096 x 1024 x 256 18.8 (+2.7) / 22.4, 4096 x 4096 x 256 57.9 (+4.0) / 77.1; int8 weights:
-  // 4096 x 768 x 768 24.5 (+4.8) / 23.6, 4096 x 768 x 3072 71.1 (+19.4) / 68.0, 2048 x 512 x 2048 22.3 (+5.9) / 25.0; past it 4096 x
+  // 4096 x 768 x 768 24.8 (+4.2) / 23.1, 4096 x 768 x 3072 69.0 (+20.9) / 67.9, 2048 x 512 x 2048 22.2 (+6.2) / 25.0; past it 4096 x
   // 3072 x 768 67.3 (+6.1) / 87.9.
   UmmaCutPlan best;
   if (!exact_b && groups > 16) return best;

@@ -577,7 +577,11 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   // Where A lies row by row and the product is small its pieces need no matrix of their own.
   const k::UmmaCutPlan cut = k::UmmaPlanCut(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N),
                                             static_cast<uint32_t>(Kp / 64), exact_b, impl->sms);
-  const bool cuts = !a.a_transposed && cut.grid != 0;
+  // (Pieces that are there already are worth it where the kernel's working warps would take a long walk alone: int8 2048 x
+  // 512 x 2048 25.0 us, 22.2 from pieces, 4096 x 512 x 2048 41.9 and 33.8; up to 16 blocks of 64 k, and with 192-wide tiles,
+  // cutting is the shorter all the same, 4096 x 768 x 3072 67.9 and 69.0.)
+  const bool long_walk = exact_b && cut.tn <= 128 && Kp / 64 > 16 * cut.splits;
+  const bool cuts = !a.a_transposed && cut.grid != 0 && !(have_pieces && long_walk);
   // No memory for a copy or for pieces: the product stays on the CUDA cores, which need neither.
   if (!cuts) {
     if (a.M * 3 * Kp > impl->split_a_capacity) impl->split_tag.valid = false;

@@ -136,3 +136,29 @@ def test_each_kernel_of_the_form(form):
     rms = np.sqrt(np.mean(want ** 2))
     err = np.abs(got[:bad_row] - want)
     assert np.sqrt(np.mean(err ** 2)) <= 4e-7 * rms and err.max() <= 8e-6 * rms   # as above
+
+
+def test_pieces_that_are_there_are_used_on_a_long_walk():
+    """A wide product cuts the activation into a piece matrix; the narrow one after it, which would cut it inside its
+    kernel, takes that."""
+    M, K = 2048, 2048
+    rng = np.random.default_rng(11)
+    a = Arena(rng)
+    x = a.alloc(M * K, "normal")
+    prog, want = [], []
+    for N in (2048, 512):
+        w = rng.integers(-127, 128, size=(K, N), dtype=np.int8)
+        scale = (rng.random(N) * 0.01 + 1e-3).astype(np.float32)
+        out = a.alloc(M * N)
+        prog.append(P.Instr(Op.GEMM_NN_Q8, P.FLAG_Q8_COL_SCALE, 0, (x, a.ro_alloc(w), out, a.ro_alloc(scale)), (M, N, K)))
+        want.append((out, N, w * scale.astype(np.float64)))
+    arena, ro = a.build()
+    A = arena[x:x + 4 * M * K].view(np.float32).reshape(M, K).astype(np.float64)
+    both, taken = _run(prog, arena, ro, -1)
+    alone, _ = _run(prog[1:], arena, ro, -1)
+    assert taken == 2
+    for got, (out, N, w) in ((both, want[0]), (both, want[1]), (alone, want[1])):
+        ref = A @ w
+        err = np.abs(got[out:out + 4 * M * N].view(np.float32).reshape(M, N) - ref)
+        rms = np.sqrt(np.mean(ref ** 2))
+        assert np.sqrt(np.mean(err ** 2)) <= 4e-7 * rms and err.max() <= 8e-6 * rms
