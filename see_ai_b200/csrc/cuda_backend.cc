@@ -767,7 +767,7 @@ void CudaBackend::PlanShadows(std::span<const Instruction> program, size_t begin
         RefSpace(g.in[0]) != kArena)
       continue;
     const uint64_t M = g.out[0], N = g.out[1], K = g.out[2];
-    if (K % 8 != 0 || N % 4 != 0 || K < 64 || N < 16 || M < 64) continue;   // TryGemm's domain
+    if (K % 8 != 0 || N % 4 != 0 || K < 64 || N < 16 || M < 64) continue;   // PrepareProduct's domain
     ShadowPlan want;
     want.want = true;
     want.a_off = RefOffset(g.in[0]);
@@ -817,7 +817,7 @@ void CudaBackend::PlanBiasFusions(std::span<const Instruction> program, size_t b
         RefSpace(ab.in[2]) != kArena)
       continue;
     const uint64_t M = g.out[0], N = g.out[1], K = g.out[2];
-    if (K % 8 != 0 || N % 4 != 0 || K < 64 || N < 16 || M < 64) continue;   // TryGemm's domain
+    if (K % 8 != 0 || N % 4 != 0 || K < 64 || N < 16 || M < 64) continue;   // PrepareProduct's domain
     if (ab.in[0] != g.in[2] || ab.out[0] != M || ab.out[1] != N) continue;
     const uint64_t r_lo = RefOffset(g.in[2]), r_hi = r_lo + M * N * 4;
     const uint64_t z_lo = RefOffset(ab.in[2]), z_hi = z_lo + M * N * 4;
@@ -868,7 +868,7 @@ bool IsRelaxedFrozenGemm(const Instruction& g) {
   if (!gemm || !(g.flags & kFlagRelaxed) || RefSpace(g.in[1]) == kArena || RefSpace(g.in[0]) != kArena)
     return false;
   const uint64_t M = g.out[0], N = g.out[1], K = g.out[2];
-  return K % 8 == 0 && N % 4 == 0 && K >= 64 && N >= 16 && M >= 64;   // TryGemm's domain
+  return K % 8 == 0 && N % 4 == 0 && K >= 64 && N >= 16 && M >= 64;   // PrepareProduct's domain
 }
 
 uint64_t GemmScaleKey(const Instruction& g) {

@@ -162,32 +162,27 @@ __global__ void SquaredDiffTermsKernel(const float* __restrict__ pred, const flo
   }
 }
 
-// out[0] = sum (sign = -1: minus the terms; +1: plus), divided by the divisor
-// (MSE: the row width); tally[3] = rows counted.  One warp: 32 terms per load, two
+// out[0] = the sum of the terms over the divisor (the row width of a mean squared
+// error); tally[3] = n.  One warp: 32 terms per load, two
 // loads ahead, and every lane makes the same chain of additions over the terms
 // the shuffles bring it in row order, so a step costs one dependent double add
 // (one thread that also loads: 190 us for 4096 rows; this: 35).
-__global__ void OrderedFoldKernel(const double* __restrict__ terms, const int32_t* __restrict__ labels,
-                                  size_t n, double sign, double divisor, double* __restrict__ out,
+__global__ void OrderedFoldKernel(const double* __restrict__ terms, size_t n, double divisor, double* __restrict__ out,
                                   unsigned long long* __restrict__ tally) {
   const size_t lane = threadIdx.x;
   double sum = 0.0;
-  unsigned long long counted = 0;
-  // A skipped row's term is 0: adding it leaves the sum as it is.
   auto load = [&](size_t i0) { return i0 + lane < n ? terms[i0 + lane] : 0.0; };
   double next0 = load(0), next1 = load(32);
   for (size_t i0 = 0; i0 < n; i0 += 32) {
-    const double t = sign * next0;   // x + (-t) and x - t are the same IEEE operation
+    const double t = next0;
     next0 = next1;
     next1 = load(i0 + 64);
-    const bool in = i0 + lane < n && !(labels && labels[i0 + lane] < 0);
-    counted += __popc(__ballot_sync(0xFFFFFFFFu, in));
 #pragma unroll
     for (int j = 0; j < 32; ++j) sum += __shfl_sync(0xFFFFFFFFu, t, j);
   }
   if (lane != 0) return;
   out[0] = divisor != 0.0 ? sum / divisor : sum;
-  tally[3] = counted;
+  tally[3] = n;
 }
 
 // ---- per-column int8 quantiser ----------------------------------------------------------
@@ -247,7 +242,7 @@ void MseRealRowLoss(const float* pred, const float* target, size_t real_rows, si
     if (blocks > 148 * 8) blocks = 148 * 8;
     SquaredDiffTermsKernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(pred, target, n, terms);
   }
-  OrderedFoldKernel<<<1, 32, 0, s>>>(terms, nullptr, n, 1.0, static_cast<double>(width), out, tally);
+  OrderedFoldKernel<<<1, 32, 0, s>>>(terms, n, static_cast<double>(width), out, tally);
 }
 
 void QuantizeColumns(const float* w, size_t K, size_t N, int8_t* levels, float* scales,

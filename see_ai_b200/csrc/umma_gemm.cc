@@ -465,17 +465,6 @@ std::string LaunchProducts(Context* ctx, const PreparedProduct* products, int co
   return {};
 }
 
-std::string TryGemm(Context* ctx, const k::GemmArgs& a, int b_space, uint64_t b_off,
-                    uint64_t a_off, uint64_t a_scale_off, cudaStream_t stream, int* launches) {
-  *launches = 0;
-  PreparedProduct product;
-  bool ok = false;
-  if (std::string e = PrepareProduct(ctx, a, b_space, b_off, a_off, a_scale_off, false, &product, &ok, stream, launches);
-      !e.empty() || !ok)
-    return e;
-  return LaunchProducts(ctx, &product, 1, false, stream, launches);
-}
-
 namespace {
 
 // The piece products of one block of the reduction, small ones first because the tensor core truncates toward zero at

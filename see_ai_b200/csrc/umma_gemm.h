@@ -37,17 +37,12 @@ uint64_t BufferMoves(const Context* ctx);
 void InvalidateRange(Context* ctx, uint64_t arena_off, uint64_t bytes);
 void PlanRange(Context* ctx, const Instruction* program, size_t begin, size_t end);
 
-// Runs C = epilogue(A @ B) on the tensor cores when the shape is inside the
-// kernel's domain.  *launches is the number of kernels enqueued; 0 with an
-// empty return value means "not applicable — use the exact kernel".
-// b_space: 1 = rodata, 2 = source model; offsets identify operands for caching.
-std::string TryGemm(Context* ctx, const k::GemmArgs& args, int b_space, uint64_t b_off,
-                    uint64_t a_off, uint64_t a_scale_off, cudaStream_t stream, int* launches);
-
-// Several products of one shape as one launch: side by side (they share the activation, each leaves as its attention
-// copy alone) or chained (their sum is the output; the operands of all but the last product are unread by then).
-// PrepareProduct checks the domain, makes the operands' bf16 copies as TryGemm does and fills *out; *ok = false with an
-// empty return value: not applicable.  `keep` holds the activation copy's slot, whatever happens to the activation's
+// C = epilogue(A @ B) on the tensor cores, one product a launch or several of one shape: side by side (they share the
+// activation, each leaves as its attention copy alone) or chained (their sum is the output; the operands of all but the
+// last product are unread by then).
+// PrepareProduct checks the kernels' domain, makes the operands' bf16 copies and fills *out; *ok = false with an
+// empty return value: not applicable, use the exact kernel.  *launches grows by the kernels enqueued.  b_space: 1 = rodata,
+// 2 = source model; offsets identify operands for caching.  `keep` holds the activation copy's slot, whatever happens to the activation's
 // range, until ReleaseProducts.  LaunchProducts takes one to kUmmaProducts prepared products; the epilogue of a chain is the
 // last one's.  The bits are those of the products launched one after the other; where one launch would have to sum in another
 // way, or takes longer by the planner's estimates, that is what it does.
@@ -101,7 +96,7 @@ void PlanSplitGemms(Context* ctx, const Instruction* program, size_t begin, size
 // conversion pass the f32 re-read.  ReserveShadow picks an activation slot and
 // returns its buffer (null when none can hold M x K); after the producing
 // instruction's own write extents have gone through InvalidateRange, CommitShadow
-// publishes the slot under the key TryGemm looks up (arena offset, scale offset,
+// publishes the slot under the key PrepareProduct looks up (arena offset, scale offset,
 // M, K).  A reservation that is not committed is simply reused later.
 // keep_reserved: a second reservation beside the one already held (an instruction
 // that writes two tensors).
