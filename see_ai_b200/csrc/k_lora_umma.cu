@@ -31,7 +31,9 @@
 //
 // With few rows (two blocks for every tile fit the chip) a cluster of two works a tile, each block half of dY's and half of
 // x's columns: the halves of dT cross through the peer's shared memory and are added there, everything else is apart.
-// A 4096-row launch had 64 blocks on 148 SMs, twelve stages each one after the other: 20.3 us, 16.4 in pairs.
+// A 4096-row launch had 64 blocks on 148 SMs, twelve stages each one after the other: 20.3 us, 16.4 in pairs.  dT's two
+// accumulators truncate over half the columns each and meet in a rounded sum: rms error against float64 at width 768 2.9e-6 one
+// block to a tile, 2.6e-6 in pairs (2.3e-6 and 1.0e-6 for terms of one sign); dB is the same bits, dA follows dT.
 //
 // Every wait is bounded: a wait that runs out raises the status flag, and the block
 // stops issuing work and frees its tensor memory.

@@ -1,6 +1,6 @@
 """The adapter backward with two blocks to a 64-row tile (as many rows as give every block an SM of its own) and, one tile
 past that line, with blocks that walk: a single tile, ragged last tiles, against float64; the same bits
-run to run.  The tcgen05 kernel's bound: every term within 2^-17 of itself (two bf16 pieces of the streamed operand), with
+run to run.  768 wide: the only sites that are planned onto that kernel.  Its bound: every term within 2^-17 of itself (two bf16 pieces of the streamed operand), with
 errors of either sign, so 2e-6 of 1 + sum|a_k b_k| once a sum has a few hundred terms; dB and dA sum M of them."""
 
 import numpy as np

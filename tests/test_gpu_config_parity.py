@@ -18,8 +18,8 @@ What each comparison uses:
     the learning rate, so no element-wise 1e-5 can hold after a step);
   * the accept / reject verdict of the gate: equal.
 
-Every measured figure is also written to gpurun_out/config_parity.json when
-that folder exists.
+Every measured figure is also written to the JSON file that SEE_PARITY_FIGURES
+names, if it is set.
 """
 
 import json
@@ -37,16 +37,15 @@ from tests.util import compare
 
 pytestmark = pytest.mark.gpu
 Op = P.Op
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 _METRICS = {}
 
 
 def _record(name, **kv):
     _METRICS.setdefault(name, {}).update({k: (float(v) if isinstance(v, (np.floating, float)) else v)
                                           for k, v in kv.items()})
-    out = os.path.join(ROOT, "gpurun_out")
-    if os.path.isdir(out):
-        with open(os.path.join(out, "config_parity.json"), "w") as f:
+    out = os.environ.get("SEE_PARITY_FIGURES")
+    if out:
+        with open(out, "w") as f:
             json.dump(_METRICS, f, indent=1)
 
 

@@ -1,6 +1,7 @@
 """Exact products whose activation is cut into bf16 pieces inside the kernel (a single round of tiles, A row by row):
 edges of the 128-row tiles, the column tiles and the 64-wide blocks of K, reductions shared by a cluster, ragged widths,
-rows of A off the 16-byte grid's multiples, every weight type and epilogue, and operands that are not finite."""
+rows of A off the 16-byte grid's multiples, f32 and int8 weights with every epilogue, operands that are not finite; and
+each kernel of the form, bf16 weights among them."""
 
 import numpy as np
 import pytest

@@ -1,5 +1,6 @@
 """Relaxed products launched together (Q, K and V side by side; their input gradients chained into one sum) against the
-same step with every product a launch of its own: the one-tile kernel, the persistent one and CTA pairs, sites with and
+same step without any fusion, to what bf16 operands leave, and against the same step with every product a launch of its
+own, bit for bit: the one-tile kernel, the persistent one and CTA pairs, sites with and
 without an adapter, ranks with one and two low-rank blocks; eager, captured and replayed."""
 
 import numpy as np
