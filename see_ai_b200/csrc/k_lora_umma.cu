@@ -29,11 +29,11 @@
 // operand: dA_chunk += x_chunk^T dT in the same accumulator columns, stored the same way.
 // The partial sums have the layout the fold kernel of k_lora_mma.cu adds up in block order.
 //
-// With few rows (two blocks for every tile fit the chip) a cluster of two works a tile, each block half of dY's and half of
-// x's columns: the halves of dT cross through the peer's shared memory and are added there, everything else is apart.
-// A 4096-row launch had 64 blocks on 148 SMs, twelve stages each one after the other: 20.3 us, 16.4 in pairs.  dT's two
-// accumulators truncate over half the columns each and meet in a rounded sum: rms error against float64 at width 768 2.9e-6 one
-// block to a tile, 2.6e-6 in pairs (2.3e-6 and 1.0e-6 for terms of one sign); dB is the same bits, dA follows dT.
+// With few rows (two blocks for every tile fit the chip) two blocks work a tile: each walks all of dY for dT, which either
+// needs whole and as one sum, and takes half of the columns of dB and of x.  A 4096-row launch had 64 blocks on 148 SMs,
+// twelve stages each one after the other; these take nine: 23.0 -> 19.0 us at width 768 with the inputs in HBM, 22.7 -> 18.4
+// for 64 rows.  The bits are one block's.  (A cluster of two that walks half of dY each and adds its halves of dT in
+// distributed shared memory takes six, and 19.4 and 19.2 us.)
 //
 // Every wait is bounded: a wait that runs out raises the status flag, and the block
 // stops issuing work and frees its tensor memory.
@@ -76,13 +76,12 @@ constexpr int kMaxChunks = (kTmemCols - 2 * kWide) / kWide;     // 8
 struct Bars {
   uint64_t raw_full[kRawStages], raw_empty[kRawStages], pc_full[kStages], pc_empty[kStages];
   uint64_t small_ready[2], dt_full[2], dt_free[2], acc_full, acc_free;
-  uint64_t peer_dt;   // the other half of dT has arrived in `exchange`
   uint32_t tmem_base;
   volatile uint32_t abort;
 };
-constexpr uint32_t kExchangeBytes = kRows * kR * 4;             // dT of a tile, f32
+constexpr uint32_t kTileDtBytes = kRows * kR * 4;               // dT of a tile, f32
 constexpr size_t kSmemBytes =
-    1024 + kRawStages * kRawBytes + kStages * kPieceBytes + 2 * kSmallBytes + kExchangeBytes + sizeof(Bars);
+    1024 + kRawStages * kRawBytes + kStages * kPieceBytes + 2 * kSmallBytes + kTileDtBytes + sizeof(Bars);
 static_assert(kSmemBytes <= 227 * 1024, "shared memory of a block");
 
 constexpr uint32_t kInstrDescAMnMajor = 1u << 15;
@@ -107,22 +106,6 @@ __device__ __forceinline__ void LoadSummed(uint32_t taddr, float (&v)[kR]) {
 }
 __device__ __forceinline__ void MbarArrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemAddr(bar)) : "memory");
-}
-// A bounded wait for what a peer block of the cluster wrote here.
-__device__ __forceinline__ bool MbarWaitCluster(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = SmemAddr(bar);
-  for (uint32_t it = 0; it < kWaitLimit; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
 }
 // A descriptor whose start address lies `bytes` further on (the address field holds bytes / 16).
 __device__ __forceinline__ uint64_t Advance(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
@@ -172,13 +155,13 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
   uint8_t* pc = smem;                                   // the pieces' ring first: its tiles want 1024-byte alignment
   uint8_t* small = pc + kStages * kPieceBytes;          // two buffers of the small operand's pieces
   uint8_t* raw = small + 2 * kSmallBytes;
-  float* exchange = reinterpret_cast<float*>(raw + kRawStages * kRawBytes);
-  Bars* bars = reinterpret_cast<Bars*>(raw + kRawStages * kRawBytes + kExchangeBytes);
+  float* tile_dt = reinterpret_cast<float*>(raw + kRawStages * kRawBytes);   // halves == 2
+  Bars* bars = reinterpret_cast<Bars*>(raw + kRawStages * kRawBytes + kTileDtBytes);
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // halves == 1: a block walks its tiles.  halves == 2: a cluster of two has one tile, a block half of its chunks.
-  const uint32_t half = halves == 2 ? ClusterCtaRank() : 0u, walker = blockIdx.x / halves, walkers = gridDim.x / halves;
-  const uint32_t nc = N / kChunk / halves, kc = K / kChunk / halves, n_first = half * nc, k_first = half * kc;
+  // halves == 1: a block walks its tiles.  halves == 2: two blocks have one tile, dB and dA of half of its chunks each.
+  const uint32_t walker = blockIdx.x / halves, walkers = gridDim.x / halves, half = blockIdx.x - walker * halves;
+  const uint32_t nd = N / kChunk, nc = nd / halves, kc = K / kChunk / halves, n_first = half * nc, k_first = half * kc;
   const uint32_t tiles = (M + kRows - 1) / kRows;
   const uint32_t mine = walker < tiles ? (tiles - walker + walkers - 1) / walkers : 0u;   // this block's tiles
 
@@ -198,14 +181,12 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
     }
     MbarInit(&bars->acc_full, 1);
     MbarInit(&bars->acc_free, kWorkerWarps);
-    MbarInit(&bars->peer_dt, 4);
     bars->abort = 0;
     MbarInitFence();
   }
   if (warp == 1) TmemAlloc(&bars->tmem_base, kTmemCols);
   TcFenceBefore();
   __syncthreads();
-  if (halves == 2) ClusterSync();   // the peer's barriers exist before anything signals them
   TcFenceAfter();
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_acc = tmem_base, tmem_dt = tmem_base + kWide * kMaxChunks;   // dT: two buffers of 48 columns
@@ -232,12 +213,12 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
       // The ring holds two stages, too little to cover the latency of HBM: position q of the stage
       // stream is asked into L2 kAhead stages before its load.
       constexpr uint32_t kAhead = 8;
-      const uint32_t first_walk = mine * nc, total = first_walk + mine * kc;
+      const uint32_t first_walk = mine * nd, total = first_walk + mine * kc;
       auto prefetch = [&](uint32_t q) {
         if (q >= total) return;
         const bool dy = q < first_walk;
-        const uint32_t per = dy ? nc : kc, i = dy ? q : q - first_walk;
-        const uint32_t v = i / per, c = i - v * per + (dy ? n_first : k_first);
+        const uint32_t per = dy ? nd : kc, i = dy ? q : q - first_walk;
+        const uint32_t v = i / per, c = i - v * per + (dy ? 0u : k_first);
         asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
                      ::"l"(reinterpret_cast<uint64_t>(dy ? &map_dy : &map_x)), "r"(static_cast<int32_t>(c * kChunk)),
                        "r"(static_cast<int32_t>((walker + v * walkers) * kRows))
@@ -245,9 +226,9 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
       };
       for (uint32_t q = 0; q < kAhead; ++q) prefetch(q);
       for (uint32_t v = 0; v < mine && ok; ++v)
-        for (uint32_t c = 0; c < nc && ok; ++c) {
+        for (uint32_t c = 0; c < nd && ok; ++c) {
           prefetch(it + kAhead);
-          stage(&map_dy, n_first + c, (walker + v * walkers) * kRows, true);
+          stage(&map_dy, c, (walker + v * walkers) * kRows, true);
         }
       for (uint32_t v = 0; v < mine && ok; ++v)
         for (uint32_t c = 0; c < kc && ok; ++c) {
@@ -285,7 +266,7 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
         if (v >= 2 && !MbarWait(&bars->dt_free[v & 1], ((v >> 1) - 1) & 1)) { fail(); break; }
         TcFenceAfter();
         const uint32_t tmem_t = tmem_dt + (v & 1) * kWide;
-        for (uint32_t c = 0; c < nc && ok; ++c, ++it) {
+        for (uint32_t c = 0; c < nd && ok; ++c, ++it) {
           const uint32_t s = it % kStages, round = it / kStages;
           if (!MbarWait(&bars->pc_full[s], round & 1)) { fail(); break; }
           TcFenceAfter();
@@ -299,7 +280,8 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
               UmmaBf16(tmem_t, Advance(a0, (2 * p + h) * kTileBytes + off), Advance(b0, 3 * h * kWTileBytes + off),
                        idesc_rows, (c == 0 && kk == 0 && p == 0) ? 0u : 1u);
           }
-          columns_times_small(act, SmemAddr(small + (v & 1) * kSmallBytes), tmem_acc + kWide * c, v == 0);
+          if (c - n_first < nc)
+            columns_times_small(act, SmemAddr(small + (v & 1) * kSmallBytes), tmem_acc + kWide * (c - n_first), v == 0);
           UmmaCommit(&bars->pc_empty[s]);
         }
         if (ok) UmmaCommit(&bars->dt_full[v & 1]);
@@ -416,33 +398,12 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
         float val[kR];
         LoadSummed(tmem_dt + (v & 1) * kWide + ((quad * 32u) << 16), val);
         const uint32_t r = quad * 16u + lane;
-        float4* here = reinterpret_cast<float4*>(exchange + r * kR);
-        if (halves == 2) {   // this block's half of the sum to the peer, the peer's half from it
-          if (lane < 16) {
-            const uint32_t there = MapToCta(SmemAddr(here), half ^ 1u);
-#pragma unroll
-            for (uint32_t q = 0; q < kR / 4; ++q)
-              asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(there + 16 * q), "f"(val[4 * q]),
-                           "f"(val[4 * q + 1]), "f"(val[4 * q + 2]), "f"(val[4 * q + 3]) : "memory");
-          }
-          __syncwarp();
-          if (lane == 0) MbarArriveCluster(MapToCta(SmemAddr(&bars->peer_dt), half ^ 1u));
-          const bool there = MbarWaitCluster(&bars->peer_dt, 0);
-          if (!__all_sync(0xFFFFFFFFu, there)) { give_up(); return; }
-          if (lane < 16) {
-#pragma unroll
-            for (int q = 0; q < kR / 4; ++q) {
-              const float4 o = here[q];
-              val[4 * q] += o.x; val[4 * q + 1] += o.y; val[4 * q + 2] += o.z; val[4 * q + 3] += o.w;
-            }
-          }
-        }
 #pragma unroll
         for (int n = 0; n < kR; ++n) val[n] *= alpha_dt;
-        if (halves == 2 && lane < 16) {   // both blocks' walk over x takes it from here
+        if (halves == 2 && lane < 16) {   // this block's walk over x takes it from here
 #pragma unroll
           for (int q = 0; q < kR / 4; ++q)
-            here[q] = make_float4(val[4 * q], val[4 * q + 1], val[4 * q + 2], val[4 * q + 3]);
+            reinterpret_cast<float4*>(tile_dt + r * kR)[q] = make_float4(val[4 * q], val[4 * q + 1], val[4 * q + 2], val[4 * q + 3]);
         }
         if (half == 0 && lane < 16 && row0 + r < M) {
           float4* dst = reinterpret_cast<float4*>(dt + static_cast<size_t>(row0 + r) * kR);
@@ -502,7 +463,7 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
       small_store(now, v);
       cut_stage(true);
       if (ok && v > 0) dt_out(v - 1);   // one tile behind: its products have had a stage's time to complete
-      for (uint32_t c = 1; c < nc && ok; ++c) cut_stage(true);
+      for (uint32_t c = 1; c < nd && ok; ++c) cut_stage(true);
     }
     if (ok && mine > 0) dt_out(mine - 1);
     if (ok && mine > 0 && !MbarWait(&bars->acc_full, 0)) give_up();
@@ -518,7 +479,7 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
     // ---- over x ----
     if (ok && mine > 0) {
       if (halves == 1) ahead = small_load(dt, walker * kRows);
-      else if (wt < 4 * kRows) ahead = *reinterpret_cast<const float4*>(exchange + (wt >> 2) * kR + (wt & 3u) * 4u);
+      else if (wt < 4 * kRows) ahead = *reinterpret_cast<const float4*>(tile_dt + (wt >> 2) * kR + (wt & 3u) * 4u);
     }
     for (uint32_t v = 0; v < mine && ok; ++v) {
       const float4 now = ahead;
@@ -536,7 +497,6 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
   TcFenceBefore();
   __syncthreads();
   if (bars->abort) DrainDelay();
-  if (halves == 2) ClusterSync();   // neither block leaves while the other may still write here
   if (warp == 1) {
     TcFenceAfter();
     TmemFree(tmem_base, kTmemCols);
@@ -576,20 +536,10 @@ cudaError_t LoraBackwardUmmaLaunch(const CUtensorMap& map_dy, const CUtensorMap&
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // Two blocks to a tile where every block of the launch still has an SM of its own (`blocks` is then the tiles).
   const bool split = 2 * blocks <= sms && static_cast<size_t>(blocks) * kRows >= a.M && a.N % (2 * kChunk) == 0 && a.K % (2 * kChunk) == 0;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(split ? 2 * blocks : blocks));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = split ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, LoraBackwardUmmaKernel, map_dy, map_x, map_b, a.t, a.dt, a.partials,
-                            static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N), static_cast<uint32_t>(a.K), a.alpha_dt,
-                            a.dt_pieces, LoraSplitColumns(static_cast<uint32_t>(a.r)), status, split ? 2u : 1u);
+  LoraBackwardUmmaKernel<<<static_cast<unsigned>(split ? 2 * blocks : blocks), kThreads, kSmemBytes, s>>>(
+      map_dy, map_x, map_b, a.t, a.dt, a.partials, static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N),
+      static_cast<uint32_t>(a.K), a.alpha_dt, a.dt_pieces, LoraSplitColumns(static_cast<uint32_t>(a.r)), status, split ? 2u : 1u);
+  return cudaGetLastError();
 }
 
 }  // namespace see::k

@@ -55,3 +55,35 @@ def test_site_gradients_against_float64(M):
                                  ("dB", f(one, gB, r, N), s * T.T @ DY, s * np.abs(T.T) @ np.abs(DY)),
                                  ("dA", f(one, gA, K, r), X.T @ DT, np.abs(X.T) @ np.abs(DT))):
         assert (np.abs(got - want) / (1.0 + mag)).max() < (2e-6 if name == "dT" or M >= 500 else 2.0 ** -17), name
+
+
+def test_dt_has_the_bits_of_blocks_that_walk():
+    """dT of a row is one sum over the row whatever shares its tile: the first rows of a batch that walks, alone."""
+    N, K, r, M = 768, 768, 16, 4800
+    rng = np.random.default_rng(5)
+    x, dy, t = (rng.standard_normal((M, n)).astype(np.float32) for n in (K, N, r))
+    Bm = (rng.standard_normal((r, N)) * 0.05).astype(np.float32)
+
+    def run(rows):
+        a = Arena(rng)
+        refs = [a.alloc(v.size, v) for v in (x[:rows], dy[:rows], t[:rows], Bm)]
+        dt, gB, gA = a.alloc(rows * r), a.alloc(r * N), a.alloc(K * r)
+        arena, ro = a.build()
+        be = B.CudaBackend(0)
+        be.set_coherence(B.COHERENCE_LAZY)
+        be.bind(arena, ro)
+        be.set_program([
+            P.Instr(Op.GEMM_NT, 0, P.f32_bits(2.0), (refs[1], refs[3], dt, P.NULL_REF), (rows, r, N)),
+            P.Instr(Op.GEMM_TN, 0, P.f32_bits(2.0), (refs[2], refs[1], gB, P.NULL_REF), (r, N, rows)),
+            P.Instr(Op.GEMM_TN, 0, 0, (refs[0], dt, gA, P.NULL_REF), (K, r, rows)),
+        ])
+        be.run(None)
+        be.host_needs(0, arena.size)
+        be.flush()
+        assert be.counters().fused_dispatches == 2
+        be.close()
+        return arena[dt:dt + 4 * rows * r].view(np.float32).reshape(rows, r).copy()
+
+    whole = run(M)
+    for rows in (64, 1000, 4096):
+        assert np.array_equal(run(rows), whole[:rows])
