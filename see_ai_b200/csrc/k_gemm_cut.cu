@@ -121,10 +121,13 @@ __device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs& f) {
   }
 }
 
-template <uint32_t kTN, uint32_t kBPieces>
+// kParts: a CTA's blocks are summed in several parts.
+template <uint32_t kTN, uint32_t kBPieces, bool kParts>
 __global__ void __launch_bounds__(kCutThreads, 1)
-UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ UmmaEpilogue ep, uint32_t splits) {
+UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ UmmaEpilogue ep, uint32_t splits,
+                  uint32_t parts) {
   using Sh = CutShape<kTN, kBPieces>;
+  constexpr uint32_t kTmemCols = (kParts ? 4 : 2) * Sh::kAccCols;   // two accumulators, and the parts so far
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (SmemAddr(smem_raw) & 1023u)) & 1023u);
   CutBarriers* bars = reinterpret_cast<CutBarriers*>(smem + Sh::kStages * Sh::kStageBytes);
@@ -151,7 +154,7 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
     bars->nonfinite = 0;
     MbarInitFence();
   }
-  if (warp == 1) TmemAlloc(&bars->tmem_base, 2 * Sh::kAccCols);
+  if (warp == 1) TmemAlloc(&bars->tmem_base, kTmemCols);
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
@@ -216,9 +219,13 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
     const uint32_t quarter = warp & 3, columns = ((warp - 2) >> 2) * Sh::kColsPerWarp;
     const uint32_t t_row = tmem_base + ((quarter * 32) << 16) + columns;
     const bool vec = (ep.src_k & 3u) == 0 && (reinterpret_cast<uintptr_t>(ep.src_a) & 15) == 0;
+    // The blocks of a part of K are one chain of additions and the parts meet after that, as the piece form's CTAs do
+    // where it cuts K more often than this kernel: no chain is longer than there.
     float sum[Sh::kColsPerWarp];
 #pragma unroll
     for (uint32_t j = 0; j < Sh::kColsPerWarp; ++j) sum[j] = 0.0f;
+    [[maybe_unused]] const uint32_t first_part = parts / splits * split;
+    [[maybe_unused]] uint32_t part = first_part, part_end = groups * (part + 1) / parts;
     auto add = [&](uint32_t it) {   // the accumulator of this CTA's group number `it`
       const uint32_t buf = it & 1;
       bool there = MbarWait(&bars->tmem_full[buf], (it >> 1) & 1);
@@ -238,6 +245,31 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
       TcFenceBefore();
       __syncwarp();
       if (lane == 0) MbarArrive(&bars->tmem_empty[buf]);
+      if constexpr (kParts) {
+        if (g0 + it + 1 == part_end) {   // the parts so far wait in tensor memory: the registers are full
+#pragma unroll
+          for (uint32_t c = 0; c < Sh::kColsPerWarp; c += 16) {
+            uint32_t r[16];
+            if (part > first_part) {
+              TmemLoad16(t_row + 2 * Sh::kAccCols + c, r);
+              TmemWaitLd();
+#pragma unroll
+              for (uint32_t j = 0; j < 16; ++j) sum[c + j] = __uint_as_float(r[j]) + sum[c + j];
+            }
+            if (part_end < g1) {
+#pragma unroll
+              for (uint32_t j = 0; j < 16; ++j) {
+                r[j] = __float_as_uint(sum[c + j]);
+                sum[c + j] = 0.0f;
+              }
+              TmemStore16(t_row + 2 * Sh::kAccCols + c, r);
+            }
+          }
+          TmemWaitSt();
+          ++part;
+          part_end = groups * (part + 1) / parts;
+        }
+      }
       return true;
     };
     CutRegs f;
@@ -311,13 +343,13 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
   if (splits > 1) ClusterSync();   // no CTA leaves while another may still read its memories
   if (warp == 1) {
     TcFenceAfter();
-    TmemFree(tmem_base, 2 * Sh::kAccCols);
+    TmemFree(tmem_base, kTmemCols);
   }
 }
 
-template <uint32_t kTN, uint32_t kBPieces>
+template <uint32_t kTN, uint32_t kBPieces, bool kParts = false>
 cudaError_t Launch(const UmmaCutPlan& plan, const CUtensorMap& map_b, const UmmaEpilogue& ep, cudaStream_t s) {
-  auto kernel = UmmaGemmCutKernel<kTN, kBPieces>;
+  auto kernel = UmmaGemmCutKernel<kTN, kBPieces, kParts>;
   constexpr size_t kSmem = CutShape<kTN, kBPieces>::kSmem;
   static std::atomic<bool> configured[64] = {};   // (a per-device setting of the function)
   int dev = 0;
@@ -338,7 +370,7 @@ cudaError_t Launch(const UmmaCutPlan& plan, const CUtensorMap& map_b, const Umma
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = plan.splits > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, map_b, ep, plan.splits);
+  return cudaLaunchKernelEx(&cfg, kernel, map_b, ep, plan.splits, plan.parts);
 }
 
 }  // namespace
@@ -373,6 +405,10 @@ UmmaCutPlan UmmaPlanCut(uint32_t M, uint32_t N, uint32_t groups, bool exact_b, u
 }
 
 cudaError_t UmmaCutLaunch(const UmmaCutPlan& plan, bool exact_b, const CUtensorMap& map_b, const UmmaEpilogue& ep, cudaStream_t s) {
+  if (plan.parts > plan.splits && plan.tn <= 128) {   // (192-wide tiles leave no tensor memory for it, and are cut at least as often)
+    if (exact_b) return plan.tn == 64 ? Launch<64, 1, true>(plan, map_b, ep, s) : Launch<128, 1, true>(plan, map_b, ep, s);
+    return plan.tn == 64 ? Launch<64, 3, true>(plan, map_b, ep, s) : Launch<128, 3, true>(plan, map_b, ep, s);
+  }
   if (exact_b) {
     switch (plan.tn) {
       case 64: return Launch<64, 1>(plan, map_b, ep, s);

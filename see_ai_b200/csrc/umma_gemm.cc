@@ -564,8 +564,12 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   const bool have_pieces = tag.valid && a_space == 0 && tag.off == a_off && tag.M == a.M && tag.K == a.K &&
                            tag.transposed == a.a_transposed && tag.k_scale == a.a_k_scale;
   // Where A lies row by row and the product is small its pieces need no matrix of their own.
-  const k::UmmaCutPlan cut = k::UmmaPlanCut(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N),
+  k::UmmaCutPlan cut = k::UmmaPlanCut(static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N),
                                             static_cast<uint32_t>(Kp / 64), exact_b, impl->sms);
+  // Sums no longer than the piece form's, where more than four blocks in a row would make them so: rms error against
+  // float64 at int8 2048 x 512 x 2048 1.03e-7 in one chain a CTA, 9.3e-8 in parts (piece form 9.4e-8), f32 4096 x 256 x 1024 1.00e-7 and
+  // 9.6e-8 (9.7e-8), for 2 to 3 % of the time; up to four blocks the errors are the same.
+  cut.parts = Kp / 64 > 4 * cut.splits ? plan.splits : cut.splits;
   // (Pieces that are there already are worth it where the kernel's working warps would take a long walk alone: int8 2048 x
   // 512 x 2048 25.0 us, 22.2 from pieces, 4096 x 512 x 2048 41.9 and 33.8; up to 16 blocks of 64 k, and with 192-wide tiles,
   // cutting is the shorter all the same, 4096 x 768 x 3072 67.9 and 69.0.)

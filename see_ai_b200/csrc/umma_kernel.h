@@ -96,7 +96,8 @@ UmmaGemmPlan UmmaPlanGemm(uint32_t M, uint32_t N, uint32_t k_blocks, uint32_t gr
 cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const UmmaMaps& maps, const UmmaEpilogue& ep, cudaStream_t s);
 // Piece products of an f32 activation that the kernel cuts itself (k_gemm_cut.cu; UmmaEpilogue::src_a, src_k and
 // src_a_scale are its operand): groups = blocks of 64 k.  grid == 0: the piece form is the faster one.
-struct UmmaCutPlan { uint32_t tn = 64, splits = 1, grid = 0; };
+// parts: chains of additions that K is summed in (a multiple of splits, or fewer).
+struct UmmaCutPlan { uint32_t tn = 64, splits = 1, grid = 0, parts = 1; };
 UmmaCutPlan UmmaPlanCut(uint32_t M, uint32_t N, uint32_t groups, bool exact_b, uint32_t sms);
 // map_b: bf16 [N, 3 Kp] or, exact, [N, K], box {64, plan.tn}.
 cudaError_t UmmaCutLaunch(const UmmaCutPlan& plan, bool exact_b, const CUtensorMap& map_b, const UmmaEpilogue& ep, cudaStream_t s);

@@ -86,6 +86,9 @@ FORMS = [
     ((2000, 385, 96), "int8", 64, 1), ((128, 1024, 1024), "bf16", 64, 4), ((300, 5000, 256), "bf16", 128, 1),
     ((4096, 256, 256), "int8", 128, 2), ((640, 514, 320), "bf16", 128, 4), ((4096, 768, 768), "int8", 192, 1),
     ((2048, 768, 1024), "bf16", 192, 2), ((1000, 768, 3072), "int8", 192, 4), ((600, 2048, 512), "bf16", 192, 2),
+    # ... where a CTA sums its blocks in two parts, or in four
+    ((512, 3072, 320), "f32", 128, 1), ((300, 2048, 640), "f32", 128, 2), ((600, 1024, 320), "f32", 64, 1),
+    ((1024, 2048, 1088), "int8", 128, 1), ((512, 2048, 1000), "bf16", 128, 2),
 ]
 
 
