@@ -521,6 +521,7 @@ Status CudaBackend::PrepareLoraFolds(const Instruction* program, size_t begin, u
     cudaFree(*buf);
     *buf = nullptr;
     *cap = 0;
+    rb.uploaded.clear();
     if (auto r = Check(cudaMalloc(buf, need * elem), "low-rank fold operands"); !r) return r;
     *cap = need;
     return {};
@@ -536,10 +537,17 @@ Status CudaBackend::PrepareLoraFolds(const Instruction* program, size_t begin, u
   d_lora_w_ = rb.weights;
   for (size_t i = 0; i < lora_weights_.size(); ++i)
     lora_weights_[i].dst = d_lora_w_ + static_cast<uint64_t>(i) * lora_max_n_ * lora_max_kx_;
-  // An earlier pass over this range may still be reading the table.
+  // A pass over the same range mostly finds its table there: an upload waits for the device first, since an earlier
+  // pass may still be reading the table.
+  const size_t bytes = lora_weights_.size() * sizeof(k::LoraWeight);
+  if (rb.uploaded.size() == bytes && std::memcmp(rb.uploaded.data(), lora_weights_.data(), bytes) == 0) return {};
+  rb.uploaded.clear();
   cudaStreamSynchronize(stream_);
-  return Check(cudaMemcpy(d_lora_table_, lora_weights_.data(), lora_weights_.size() * sizeof(k::LoraWeight),
-                          cudaMemcpyHostToDevice), "low-rank fold table");
+  if (auto r = Check(cudaMemcpy(d_lora_table_, lora_weights_.data(), bytes, cudaMemcpyHostToDevice), "low-rank fold table"); !r)
+    return r;
+  rb.uploaded.resize(bytes);
+  std::memcpy(rb.uploaded.data(), lora_weights_.data(), bytes);
+  return {};
 }
 
 void CudaBackend::FreeLoraRanges() {
@@ -632,6 +640,9 @@ void CudaBackend::PlanAdamGroups(std::span<const Instruction> program, size_t be
     i = j;
   }
   if (table.empty()) return;
+  // (Found as it was uploaded, the table stays: an upload waits for the device.)
+  if (adam_table_.size() == table.size() && std::memcmp(adam_table_.data(), table.data(), table.size() * sizeof(k::AdamTensor)) == 0)
+    return;
   if (table.size() > adam_table_capacity_) {
     cudaStreamSynchronize(stream_);
     if (d_adam_table_) ++buffer_moves_;
@@ -651,11 +662,10 @@ void CudaBackend::PlanAdamGroups(std::span<const Instruction> program, size_t be
   }
   // The previous range's launches may still be reading the table.
   cudaStreamSynchronize(stream_);
-  cudaMemcpy(d_adam_table_, table.data(), table.size() * sizeof(k::AdamTensor), cudaMemcpyHostToDevice);
-  if (!adam_table_.empty() && (adam_table_.size() != table.size() ||
-                               std::memcmp(adam_table_.data(), table.data(), table.size() * sizeof(k::AdamTensor)) != 0))
-    ++buffer_moves_;
+  const cudaError_t uploaded = cudaMemcpy(d_adam_table_, table.data(), table.size() * sizeof(k::AdamTensor), cudaMemcpyHostToDevice);
+  if (!adam_table_.empty()) ++buffer_moves_;
   adam_table_ = std::move(table);
+  if (uploaded != cudaSuccess) adam_table_.clear();   // (asked for again by the next range)
 }
 
 void CudaBackend::PlanMergeRuns(std::span<const Instruction> program, size_t begin, size_t end) {

@@ -467,6 +467,7 @@ class CudaBackend {
     size_t table_capacity = 0;
     uint16_t* weights = nullptr;   // [entries][max n_out][max kx] bf16
     uint64_t weights_capacity = 0;
+    std::vector<uint8_t> uploaded;   // the table's bytes as the device has them
   };
   std::map<std::pair<const Instruction*, size_t>, LoraRangeBuffers> lora_ranges_;
   k::LoraWeight* d_lora_table_ = nullptr;    // the current range's
