@@ -38,6 +38,7 @@
 #include <type_traits>
 
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace see::k {
 
@@ -85,6 +86,7 @@ __global__ void AttnFwdKernel(const float* __restrict__ q, const float* __restri
                               float* __restrict__ probs, float* __restrict__ stats, size_t B,
                               size_t S, size_t H, size_t d, const int32_t* __restrict__ starts,
                               float inv_sqrt_d) {
+  AwaitPrevious();
   extern __shared__ float smem[];
   float* qs = WarpSmem(smem, d, S, 1);
   float* prow = qs + d;
@@ -145,6 +147,7 @@ __global__ void AttnFwdKernel(const float* __restrict__ q, const float* __restri
 // dS = P * (dP - rowsum(dP * P)), the rowsum in double.
 __global__ void SoftmaxRowsBwdKernel(const float* __restrict__ probs, const float* __restrict__ dp,
                                      float* __restrict__ ds, size_t rows, size_t cols) {
+  AwaitPrevious();
   const int lane = threadIdx.x & 31;
   for (size_t r = blockIdx.x * static_cast<size_t>(kWarps) + (threadIdx.x >> 5); r < rows;
        r += static_cast<size_t>(gridDim.x) * kWarps) {
@@ -165,6 +168,7 @@ __global__ void AttnDQTiledKernel(const float* __restrict__ q, const float* __re
                                   const float* __restrict__ v, const float* __restrict__ dout,
                                   float* __restrict__ stats, float* __restrict__ dq, size_t B,
                                   size_t S, size_t H, size_t d, float inv_sqrt_d) {
+  AwaitPrevious();
   extern __shared__ float smem[];
   // per warp: q row (d), dO row (d) packed as 2d, then prow (S), dprow (S)
   float* base = smem + (threadIdx.x >> 5) * (2 * d + 2 * S);
@@ -503,6 +507,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnFwdTileKernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, float* __restrict__ o,
     float* __restrict__ probs, float* __restrict__ stats, int BH, int S, int H, int d,
     const int32_t* __restrict__ starts, float inv_sqrt_d) {
+  AwaitPrevious();
   extern __shared__ __align__(16) uint8_t raw[];
   constexpr int R = 8 * RM;
   double* slices = reinterpret_cast<double*>(raw + GroupOf() * GroupBytes());
@@ -593,6 +598,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnFwdTileKernel(
 // dP for a head too wide for a tile block's own rows: a thread per pair.
 __global__ void AttnDPWideKernel(const float* __restrict__ dout, const float* __restrict__ v, float* __restrict__ dp,
                                  size_t BH, size_t S, size_t H, size_t d) {
+  AwaitPrevious();
   const size_t pairs = BH * S * S, D = H * d;
   for (size_t t = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; t < pairs;
        t += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -606,6 +612,7 @@ template <int RM, bool kMma, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnDPTileKernel(const float* __restrict__ dout,
                                                                  const float* __restrict__ v, float* __restrict__ dp,
                                                                  int BH, int S, int H, int d) {
+  AwaitPrevious();
   extern __shared__ __align__(16) uint8_t raw[];
   constexpr int R = 8 * RM;
   double* slices = reinterpret_cast<double*>(raw + GroupOf() * GroupBytes());
@@ -654,6 +661,7 @@ template <int RM, bool kFused, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnRowTileKernel(const float* __restrict__ ds,
                                                                   const float* __restrict__ k, float* __restrict__ dq,
                                                                   int BH, int S, int H, int d, float inv_sqrt_d) {
+  AwaitPrevious();
   constexpr int R = 16 * RM, kLd = kChunkRows + 4;
   __shared__ __align__(16) float xt[2 * kChunkRows * kTile];
   __shared__ __align__(16) float wt[2 * R * kLd];
@@ -732,6 +740,7 @@ template <int RM, bool kFused, bool kScaled, bool kVec>
 __global__ __launch_bounds__(kTileThreads) void AttnColTileKernel(const float* __restrict__ w,
                                                                   const float* __restrict__ x, float* __restrict__ out,
                                                                   int BH, int S, int H, int d, float inv_sqrt_d) {
+  AwaitPrevious();
   constexpr int R = 16 * RM;
   __shared__ __align__(16) float xt[2 * kChunkRows * kTile];
   __shared__ __align__(16) float wt[2 * kChunkRows * R];
@@ -787,6 +796,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDQTiledTileKernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
     const float* __restrict__ dout, float* __restrict__ stats, float* __restrict__ dq, int BH, int S, int H,
     int d, float inv_sqrt_d) {
+  AwaitPrevious();
   extern __shared__ __align__(16) uint8_t raw[];
   constexpr int R = 8 * RM;
   double* slices = reinterpret_cast<double*>(raw + GroupOf() * GroupBytes());
@@ -875,6 +885,7 @@ __global__ __launch_bounds__(kTileThreads) void AttnDKVTiledTileKernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
     const float* __restrict__ dout, const float* __restrict__ stats, float* __restrict__ out, int BH, int S, int H,
     int d, float inv_sqrt_d) {
+  AwaitPrevious();
   extern __shared__ __align__(16) uint8_t raw[];
   constexpr int R = 8 * RM, kLd = R + 4;
   const int group = GroupOf();
@@ -1039,7 +1050,7 @@ void AttnFwd(const float* q, const float* k, const float* v, float* o, float* pr
       constexpr int RM = decltype(rows)::value;
       const size_t bytes = ScoreBytes(RM, S, d, 1);
       AllowSmem(AttnFwdTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, bytes);
-      AttnFwdTileKernel<RM, decltype(fu)::value, decltype(vec)::value><<<static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes, s>>>(
+      Next(AttnFwdTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes, s)(
           q, k, v, o, probs, stats, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d),
           starts, inv_sqrt_d);
     });
@@ -1047,7 +1058,7 @@ void AttnFwd(const float* q, const float* k, const float* v, float* o, float* pr
   }
   const size_t bytes = kWarps * (d + S) * sizeof(float);
   AllowSmem(AttnFwdKernel, bytes);
-  AttnFwdKernel<<<UnitBlocks(units), kWarps * 32, bytes, s>>>(q, k, v, o, probs, stats, B, S, H, d,
+  Next(AttnFwdKernel, UnitBlocks(units), kWarps * 32, bytes, s)(q, k, v, o, probs, stats, B, S, H, d,
                                                              starts, inv_sqrt_d);
 }
 
@@ -1058,14 +1069,13 @@ void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, si
   int rm = RowsPerThread(B * H, S, 8);
   while (rm > 1 && bytes(rm) > kTwoPerSm) rm /= 2;
   if (bytes(rm) > kMaxSmem) {
-    AttnDPWideKernel<<<148 * 8, 256, 0, s>>>(dout, v, dp, B * H, S, H, d);
+    Next(AttnDPWideKernel, 148 * 8, 256, 0, s)(dout, v, dp, B * H, S, H, d);
     return;
   }
   WithTile(rm, own_order, Vec(d, {dout, v}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
     constexpr int RM = decltype(rows)::value;
     AllowSmem(AttnDPTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, bytes(RM));
-    AttnDPTileKernel<RM, decltype(fu)::value, decltype(vec)::value>
-        <<<static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes(RM), s>>>(
+    Next(AttnDPTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes(RM), s)(
             dout, v, dp, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d));
   });
 }
@@ -1078,8 +1088,7 @@ void ColSum(const float* w, const float* x, float* out, size_t B, size_t S, size
   if (B * H * S == 0) return;
   WithTile(RowsPerThread(B * H, S, 16, (d + kTile - 1) / kTile), fused, Vec(d, {x, out}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
     constexpr int RM = decltype(rows)::value;
-    AttnColTileKernel<RM, decltype(fu)::value, kScaled, decltype(vec)::value>
-        <<<TileGrid(B * H, (S + 16 * RM - 1) / (16 * RM), d), kTileThreads, 0, s>>>(
+    Next(AttnColTileKernel<RM, decltype(fu)::value, kScaled, decltype(vec)::value>, TileGrid(B * H, (S + 16 * RM - 1) / (16 * RM), d), kTileThreads, 0, s)(
             w, x, out, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d), scale);
   });
 }
@@ -1102,8 +1111,7 @@ void AttnDQ(const float* ds, const float* k, float* dq, size_t B, size_t S, size
   const float inv_sqrt_d = 1.0f / sqrtf(static_cast<float>(d));
   WithTile(RowsPerThread(B * H, S, 16, (d + kTile - 1) / kTile), fused, Vec(d, {k, dq}), [&](auto rows, [[maybe_unused]] auto fu, auto vec) {
     constexpr int RM = decltype(rows)::value;
-    AttnRowTileKernel<RM, decltype(fu)::value, decltype(vec)::value>
-        <<<TileGrid(B * H, (S + 16 * RM - 1) / (16 * RM), d), kTileThreads, 0, s>>>(
+    Next(AttnRowTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, TileGrid(B * H, (S + 16 * RM - 1) / (16 * RM), d), kTileThreads, 0, s)(
             ds, k, dq, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H), static_cast<int>(d), inv_sqrt_d);
   });
 }
@@ -1111,7 +1119,7 @@ void AttnDQ(const float* ds, const float* k, float* dq, size_t B, size_t S, size
 void SoftmaxRowsBwd(const float* probs, const float* dp, float* ds, size_t rows, size_t cols,
                     cudaStream_t s) {
   if (rows == 0) return;
-  SoftmaxRowsBwdKernel<<<UnitBlocks(rows), kWarps * 32, 0, s>>>(probs, dp, ds, rows, cols);
+  Next(SoftmaxRowsBwdKernel, UnitBlocks(rows), kWarps * 32, 0, s)(probs, dp, ds, rows, cols);
 }
 
 void AttnDQTiled(const float* q, const float* k, const float* v, const float* dout, float* stats,
@@ -1124,8 +1132,7 @@ void AttnDQTiled(const float* q, const float* k, const float* v, const float* do
       constexpr int RM = decltype(rows)::value;
       const size_t bytes = ScoreBytes(RM, S, d, 2);
       AllowSmem(AttnDQTiledTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, bytes);
-      AttnDQTiledTileKernel<RM, decltype(fu)::value, decltype(vec)::value>
-          <<<static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes, s>>>(
+      Next(AttnDQTiledTileKernel<RM, decltype(fu)::value, decltype(vec)::value>, static_cast<unsigned>(B * H * ((S + 8 * RM - 1) / (8 * RM))), kTileThreads, bytes, s)(
               q, k, v, dout, stats, dq, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H),
               static_cast<int>(d), inv_sqrt_d);
     });
@@ -1133,7 +1140,7 @@ void AttnDQTiled(const float* q, const float* k, const float* v, const float* do
   }
   const size_t bytes = kWarps * (2 * d + 2 * S) * sizeof(float);
   AllowSmem(AttnDQTiledKernel, bytes);
-  AttnDQTiledKernel<<<UnitBlocks(units), kWarps * 32, bytes, s>>>(q, k, v, dout, stats, dq, B, S, H,
+  Next(AttnDQTiledKernel, UnitBlocks(units), kWarps * 32, bytes, s)(q, k, v, dout, stats, dq, B, S, H,
                                                                  d, inv_sqrt_d);
 }
 
@@ -1148,7 +1155,7 @@ void AttnDKVTiled(bool want_dk, const float* q, const float* k, const float* v, 
                          2 * kTile * (kTile + 8 * RM + 4) * sizeof(float);
     auto launch = [&](auto kernel) {
       AllowSmem(kernel, bytes);
-      kernel<<<TileGrid(B * H, (S + 8 * RM - 1) / (8 * RM), d), kTileThreads, bytes, s>>>(
+      Next(kernel, TileGrid(B * H, (S + 8 * RM - 1) / (8 * RM), d), kTileThreads, bytes, s)(
           q, k, v, dout, stats, out, static_cast<int>(B * H), static_cast<int>(S), static_cast<int>(H),
           static_cast<int>(d), inv_sqrt_d);
     };

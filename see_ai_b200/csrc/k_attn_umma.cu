@@ -31,6 +31,7 @@
 
 #include "attn_umma.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "shadow.cuh"
 #include "umma_device.cuh"
 
@@ -58,6 +59,7 @@ __device__ __forceinline__ uint32_t Bf16Bits(float f) {   // round to nearest ev
 
 __global__ void __launch_bounds__(256)
 PackRowsKernel(const float* __restrict__ x, uint16_t* __restrict__ rows, size_t quads) {
+  AwaitPrevious();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t q = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; q < quads; q += stride) {
     const float4 f = reinterpret_cast<const float4*>(x)[q];
@@ -250,6 +252,7 @@ AttnFwdUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   const uint32_t tmem = ctl->tmem_base;
   const uint32_t t_s = tmem + ((warp * 32) << 16);
   const uint32_t t_o = t_s + 64;
@@ -422,6 +425,7 @@ AttnDQUmmaKernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   const uint32_t tmem = ctl->tmem_base;
   const uint32_t t_lane = tmem + ((warp * 32) << 16);
 
@@ -564,6 +568,7 @@ AttnDKVUmmaKernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   const uint32_t tmem = ctl->tmem_base;
   const uint32_t t_lane = tmem + ((warp * 32) << 16);
 
@@ -797,6 +802,7 @@ AttnBwdKernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   constexpr uint32_t tmem = 0;   // all 512 columns are this CTA's
 
   if (warp == 13) {
@@ -1141,6 +1147,7 @@ AttnFwdPairKernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   constexpr uint32_t tmem = 0;   // all 512 columns are this CTA's: 256 per tile of the pair
 
   if (warp == 14) {
@@ -1397,7 +1404,7 @@ static cudaError_t Configure(Kernel kernel, size_t smem) {
 void PackHeads(const float* x, uint16_t* rows, uint32_t B, uint32_t S, uint32_t H, uint32_t d, cudaStream_t s) {
   const size_t quads = static_cast<size_t>(B) * S * H * d / 4;
   const size_t blocks = (quads + 255) / 256;
-  PackRowsKernel<<<static_cast<unsigned>(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(x, rows, quads);
+  Next(PackRowsKernel, static_cast<unsigned>(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s)(x, rows, quads);
 }
 
 template <int D>
@@ -1406,7 +1413,7 @@ static cudaError_t LaunchFwdPair(const CUtensorMap& q, const CUtensorMap& k, con
   const size_t smem = FwdShape<D>::kSmem;
   if (cudaError_t e = Configure(AttnFwdPairKernel<D>, smem); e != cudaSuccess) return e;
   const uint32_t pairs = ((a.S + kTile - 1) / kTile + 1) / 2 * a.B * a.H;
-  AttnFwdPairKernel<D><<<pairs < a.sms ? pairs : a.sms, kFwdThreads, smem, s>>>(q, k, v, a);
+  Next(AttnFwdPairKernel<D>, pairs < a.sms ? pairs : a.sms, kFwdThreads, smem, s)(q, k, v, a);
   return cudaGetLastError();
 }
 
@@ -1441,10 +1448,10 @@ cudaError_t AttnFwdUmma(const CUtensorMap& q, const CUtensorMap& k_half, const C
   cudaError_t e;
   if (a.d == 64) {
     if ((e = Configure(AttnFwdUmmaKernel<64>, smem)) != cudaSuccess) return e;
-    AttnFwdUmmaKernel<64><<<grid, 128, smem, s>>>(q, k_half, v_half, a);
+    Next(AttnFwdUmmaKernel<64>, grid, 128, smem, s)(q, k_half, v_half, a);
   } else {
     if ((e = Configure(AttnFwdUmmaKernel<128>, smem)) != cudaSuccess) return e;
-    AttnFwdUmmaKernel<128><<<grid, 128, smem, s>>>(q, k_half, v_half, a);
+    Next(AttnFwdUmmaKernel<128>, grid, 128, smem, s)(q, k_half, v_half, a);
   }
   return cudaGetLastError();
 }
@@ -1455,7 +1462,7 @@ static cudaError_t LaunchBwd(const CUtensorMap& x, const CUtensorMap& y, const C
   const size_t smem = BwdShape<D, kKV>::kSmem;
   if (cudaError_t e = Configure(AttnBwdKernel<D, kKV>, smem); e != cudaSuccess) return e;
   const uint32_t tiles = (a.S + kTile - 1) / kTile * a.B * a.H;
-  AttnBwdKernel<D, kKV><<<tiles < a.sms ? tiles : a.sms, kBwdThreads, smem, s>>>(x, y, u, w, a);
+  Next(AttnBwdKernel<D, kKV>, tiles < a.sms ? tiles : a.sms, kBwdThreads, smem, s)(x, y, u, w, a);
   return cudaGetLastError();
 }
 
@@ -1469,10 +1476,10 @@ cudaError_t AttnDQUmma(const CUtensorMap& q, const CUtensorMap& dout, const CUte
   cudaError_t e;
   if (a.d == 64) {
     if ((e = Configure(AttnDQUmmaKernel<64>, smem)) != cudaSuccess) return e;
-    AttnDQUmmaKernel<64><<<grid, 128, smem, s>>>(q, dout, k_half, v_half, a);
+    Next(AttnDQUmmaKernel<64>, grid, 128, smem, s)(q, dout, k_half, v_half, a);
   } else {
     if ((e = Configure(AttnDQUmmaKernel<128>, smem)) != cudaSuccess) return e;
-    AttnDQUmmaKernel<128><<<grid, 128, smem, s>>>(q, dout, k_half, v_half, a);
+    Next(AttnDQUmmaKernel<128>, grid, 128, smem, s)(q, dout, k_half, v_half, a);
   }
   return cudaGetLastError();
 }
@@ -1489,7 +1496,7 @@ cudaError_t AttnDKVUmma(int mode, const CUtensorMap& k, const CUtensorMap& v,
   do {                                                                                       \
     const size_t smem = AttnDKVSmem(D, DK);                                                  \
     if ((e = Configure(AttnDKVUmmaKernel<D, DK>, smem)) != cudaSuccess) return e;          \
-    AttnDKVUmmaKernel<D, DK><<<grid, 128, smem, s>>>(k, v, q_half, dout_half, a);   \
+    Next(AttnDKVUmmaKernel<D, DK>, grid, 128, smem, s)(k, v, q_half, dout_half, a);   \
   } while (0)
   if (a.d == 64) {
     if (mode == 1) SEE_LAUNCH_DKV(64, true); else SEE_LAUNCH_DKV(64, false);

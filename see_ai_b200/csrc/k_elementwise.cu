@@ -7,6 +7,7 @@
 // to libm-vs-CUDA-libm differences (a few ulp).
 #include "act_expr.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "shadow.cuh"
 
 namespace see::k {
@@ -30,6 +31,7 @@ inline bool Aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 template <typename F>
 __global__ void Map1(const float* __restrict__ x, float* __restrict__ out, size_t n, bool vec, F f,
                      Shadow sh) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   if (vec) {
@@ -52,6 +54,7 @@ __global__ void Map1(const float* __restrict__ x, float* __restrict__ out, size_
 // out may alias x or y exactly (in-place accumulate); never partially.
 template <typename F>
 __global__ void Map2(const float* x, const float* y, float* out, size_t n, bool vec, F f, Shadow sh) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   if (vec) {
@@ -90,7 +93,7 @@ bool LaunchMap1(const float* x, float* out, size_t n, cudaStream_t s, F f,
   if (n == 0) return false;
   const bool vec = Aligned16(x) && Aligned16(out);
   const bool shadowed = vec && ShadowUsable(shadow, out, n);
-  Map1<<<BlocksFor(vec ? (n + 3) / 4 : n), kThreads, 0, s>>>(x, out, n, vec, f,
+  Next(Map1<F>, BlocksFor(vec ? (n + 3) / 4 : n), kThreads, 0, s)(x, out, n, vec, f,
                                                               shadowed ? *shadow : Shadow{});
   return shadowed;
 }
@@ -100,12 +103,13 @@ bool LaunchMap2(const float* x, const float* y, float* out, size_t n, cudaStream
   if (n == 0) return false;
   const bool vec = Aligned16(x) && Aligned16(y) && Aligned16(out);
   const bool shadowed = vec && ShadowUsable(shadow, out, n);
-  Map2<<<BlocksFor(vec ? (n + 3) / 4 : n), kThreads, 0, s>>>(x, y, out, n, vec, f,
+  Next(Map2<F>, BlocksFor(vec ? (n + 3) / 4 : n), kThreads, 0, s)(x, y, out, n, vec, f,
                                                               shadowed ? *shadow : Shadow{});
   return shadowed;
 }
 
 __global__ void FillKernel(float* __restrict__ dst, float value, size_t n, bool vec) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   if (vec) {
@@ -122,6 +126,7 @@ __global__ void FillKernel(float* __restrict__ dst, float value, size_t n, bool 
 // out[r, c] = x[r, c] + b[c]   (reference: runtime/executor/elementwise.cc:28-36)
 __global__ void AddBiasKernel(const float* __restrict__ x, const float* __restrict__ b,
                               float* __restrict__ out, size_t rows, size_t cols, bool vec) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   if (vec) {  // cols % 4 == 0
@@ -167,6 +172,7 @@ __device__ __forceinline__ float RunStages(float v, float y1, float y2, uint32_t
 __global__ void FusedMapKernel(const float* __restrict__ x, const float* __restrict__ o1,
                                const float* __restrict__ o2, float* __restrict__ out, size_t n,
                                uint32_t stages, float imm0, float imm1) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = tid; i < n; i += stride) {
@@ -182,6 +188,7 @@ __global__ void FusedMapKernel(const float* __restrict__ x, const float* __restr
 __global__ void EmbedKernel(const int32_t* __restrict__ tokens, const float* __restrict__ table,
                             float* __restrict__ out, size_t rows, size_t dim, size_t vocab,
                             bool vec) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   if (vec) {
@@ -210,6 +217,7 @@ __global__ void EmbedKernel(const int32_t* __restrict__ tokens, const float* __r
 // runtime/executor/elementwise.cc:162-187): one thread per column.
 __global__ void ReduceRowsKernel(const float* __restrict__ dy, float* __restrict__ db,
                                  size_t rows, size_t cols) {
+  AwaitPrevious();
   const size_t c = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (c >= cols) return;
   float acc = 0.0f;
@@ -222,6 +230,7 @@ __global__ void ReduceRowsKernel(const float* __restrict__ dy, float* __restrict
 __global__ void SegmentStartsKernel(const int32_t* __restrict__ tokens,
                                     int32_t* __restrict__ starts, size_t B, size_t S,
                                     int32_t eos) {
+  AwaitPrevious();
   const size_t b = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (b >= B) return;
   int32_t start = 0;
@@ -234,6 +243,7 @@ __global__ void SegmentStartsKernel(const int32_t* __restrict__ tokens,
 // table[s, c, 0..1] = cos, sin(s * freq_c), freq by the f32 recurrence
 // freq *= step (reference: runtime/executor/attention.cc:157-174).
 __global__ void RopeTableKernel(float* __restrict__ table, size_t S, size_t half, float step) {
+  AwaitPrevious();
   const size_t s = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (s >= S) return;
   float* row = table + s * half * 2;
@@ -252,6 +262,7 @@ template <bool kBackward>
 __global__ void RopeKernel(const float* __restrict__ x, float* __restrict__ y, size_t units,
                            size_t S, size_t H, size_t d, float step,
                            const float* __restrict__ table) {
+  AwaitPrevious();
   const size_t u = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (u >= units) return;
   const size_t D = H * d, half = d / 2;
@@ -286,6 +297,7 @@ __device__ __forceinline__ uint16_t Bf16Rne(float f) { return static_cast<uint16
 
 __global__ void ToBf16Kernel(const float* __restrict__ x, uint16_t* __restrict__ out, size_t rows,
                              size_t cols, const float* __restrict__ col_scale, bool vec) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const size_t n = rows * cols;
@@ -334,13 +346,13 @@ void Copy(const float* src, float* dst, size_t n, cudaStream_t s) {
 void Fill(float* dst, float value, size_t n, cudaStream_t s) {
   if (n == 0) return;
   const bool vec = Aligned16(dst);
-  FillKernel<<<BlocksFor(vec ? (n + 3) / 4 : n), kThreads, 0, s>>>(dst, value, n, vec);
+  Next(FillKernel, BlocksFor(vec ? (n + 3) / 4 : n), kThreads, 0, s)(dst, value, n, vec);
 }
 void AddBias(const float* x, const float* b, float* out, size_t rows, size_t cols,
              cudaStream_t s) {
   if (rows * cols == 0) return;
   const bool vec = (cols % 4 == 0) && Aligned16(x) && Aligned16(b) && Aligned16(out);
-  AddBiasKernel<<<BlocksFor(vec ? rows * cols / 4 : rows * cols), kThreads, 0, s>>>(
+  Next(AddBiasKernel, BlocksFor(vec ? rows * cols / 4 : rows * cols), kThreads, 0, s)(
       x, b, out, rows, cols, vec);
 }
 bool ActFwd(Act act, const float* x, float* out, size_t n, cudaStream_t s, const Shadow* shadow) {
@@ -365,27 +377,27 @@ bool ActBwd(Act act, const float* dy, const float* x, float* dx, size_t n, cudaS
 void FusedMap(const float* x, const float* o1, const float* o2, float* out, size_t n,
               uint32_t stages, float imm0, float imm1, cudaStream_t s) {
   if (n == 0) return;
-  FusedMapKernel<<<BlocksFor(n), kThreads, 0, s>>>(x, o1, o2, out, n, stages, imm0, imm1);
+  Next(FusedMapKernel, BlocksFor(n), kThreads, 0, s)(x, o1, o2, out, n, stages, imm0, imm1);
 }
 void EmbedFwd(const int32_t* tokens, const float* table, float* out, size_t rows, size_t dim,
               size_t vocab, cudaStream_t s) {
   if (rows * dim == 0) return;
   const bool vec = (dim % 4 == 0) && Aligned16(table) && Aligned16(out);
-  EmbedKernel<<<BlocksFor(vec ? rows * dim / 4 : rows * dim), kThreads, 0, s>>>(
+  Next(EmbedKernel, BlocksFor(vec ? rows * dim / 4 : rows * dim), kThreads, 0, s)(
       tokens, table, out, rows, dim, vocab, vec);
 }
 void ReduceRows(const float* dy, float* db, size_t rows, size_t cols, cudaStream_t s) {
   if (cols == 0) return;
-  ReduceRowsKernel<<<static_cast<unsigned>((cols + 127) / 128), 128, 0, s>>>(dy, db, rows, cols);
+  Next(ReduceRowsKernel, static_cast<unsigned>((cols + 127) / 128), 128, 0, s)(dy, db, rows, cols);
 }
 void SegmentStarts(const int32_t* tokens, int32_t* starts, size_t B, size_t S, int32_t eos,
                    cudaStream_t s) {
   if (B == 0) return;
-  SegmentStartsKernel<<<static_cast<unsigned>((B + 63) / 64), 64, 0, s>>>(tokens, starts, B, S, eos);
+  Next(SegmentStartsKernel, static_cast<unsigned>((B + 63) / 64), 64, 0, s)(tokens, starts, B, S, eos);
 }
 void RopeTable(float* table, size_t S, size_t d, float step, cudaStream_t s) {
   if (S == 0) return;
-  RopeTableKernel<<<static_cast<unsigned>((S + 127) / 128), 128, 0, s>>>(table, S, d / 2, step);
+  Next(RopeTableKernel, static_cast<unsigned>((S + 127) / 128), 128, 0, s)(table, S, d / 2, step);
 }
 void Rope(bool backward, const float* x, float* y, size_t B, size_t S, size_t H, size_t d,
           float step, const float* table, cudaStream_t s) {
@@ -393,9 +405,9 @@ void Rope(bool backward, const float* x, float* y, size_t B, size_t S, size_t H,
   if (units == 0) return;
   const unsigned blocks = static_cast<unsigned>((units + 127) / 128);
   if (backward)
-    RopeKernel<true><<<blocks, 128, 0, s>>>(x, y, units, S, H, d, step, table);
+    Next(RopeKernel<true>, blocks, 128, 0, s)(x, y, units, S, H, d, step, table);
   else
-    RopeKernel<false><<<blocks, 128, 0, s>>>(x, y, units, S, H, d, step, table);
+    Next(RopeKernel<false>, blocks, 128, 0, s)(x, y, units, S, H, d, step, table);
 }
 void ToBf16(const float* x, uint16_t* out, size_t rows, size_t cols, const float* col_scale,
             cudaStream_t s) {
@@ -403,7 +415,7 @@ void ToBf16(const float* x, uint16_t* out, size_t rows, size_t cols, const float
   const bool vec = (cols % 4 == 0) && Aligned16(x) &&
                    (reinterpret_cast<uintptr_t>(out) & 7) == 0 &&
                    (!col_scale || Aligned16(col_scale));
-  ToBf16Kernel<<<BlocksFor((rows * cols + 3) / 4), kThreads, 0, s>>>(x, out, rows, cols, col_scale,
+  Next(ToBf16Kernel, BlocksFor((rows * cols + 3) / 4), kThreads, 0, s)(x, out, rows, cols, col_scale,
                                                                      vec);
 }
 

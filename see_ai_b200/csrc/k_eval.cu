@@ -6,6 +6,7 @@
 // same integer results are produced here and only three counters come back.
 // Integer tallies: exact whatever the order of the atomic adds.
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace see::k {
 
@@ -78,6 +79,7 @@ __device__ __forceinline__ bool ArgmaxVec(const float* probs, size_t C) {
 
 __global__ void ArgmaxTallyKernel(const float* __restrict__ probs, const int32_t* __restrict__ labels,
                                   size_t N, size_t C, unsigned long long* __restrict__ tally) {
+  AwaitPrevious();
   const size_t warps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
   const size_t warp = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
   if (ArgmaxVec(probs, C)) ArgmaxRows<true>(probs, labels, N, C, tally, warp, warps);
@@ -86,6 +88,7 @@ __global__ void ArgmaxTallyKernel(const float* __restrict__ probs, const int32_t
 
 __global__ void CountNonFiniteKernel(const float* __restrict__ x, size_t n,
                                      unsigned long long* __restrict__ tally) {
+  AwaitPrevious();
   unsigned long long bad = 0;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
@@ -113,6 +116,7 @@ __global__ void __launch_bounds__(kTailThreads)
 XentEvalTailKernel(const float* __restrict__ probs, const float* __restrict__ arg_probs, size_t arg_cols,
                    const int32_t* __restrict__ labels, size_t rows, size_t width, double* __restrict__ out,
                    unsigned long long* __restrict__ tally) {
+  AwaitPrevious();
   if (blockIdx.x > 0) {
     const size_t warps = static_cast<size_t>(gridDim.x - 1) * (kTailThreads / 32);
     const size_t warp = static_cast<size_t>(blockIdx.x - 1) * (kTailThreads / 32) + (threadIdx.x >> 5);
@@ -155,6 +159,7 @@ XentEvalTailKernel(const float* __restrict__ probs, const float* __restrict__ ar
 
 __global__ void SquaredDiffTermsKernel(const float* __restrict__ pred, const float* __restrict__ target,
                                        size_t n, double* __restrict__ terms) {
+  AwaitPrevious();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += stride) {
     const double d = static_cast<double>(pred[i]) - target[i];
@@ -169,6 +174,7 @@ __global__ void SquaredDiffTermsKernel(const float* __restrict__ pred, const flo
 // (one thread that also loads: 190 us for 4096 rows; this: 35).
 __global__ void OrderedFoldKernel(const double* __restrict__ terms, size_t n, double divisor, double* __restrict__ out,
                                   unsigned long long* __restrict__ tally) {
+  AwaitPrevious();
   const size_t lane = threadIdx.x;
   double sum = 0.0;
   auto load = [&](size_t i0) { return i0 + lane < n ? terms[i0 + lane] : 0.0; };
@@ -194,6 +200,7 @@ __global__ void OrderedFoldKernel(const double* __restrict__ terms, size_t n, do
 // (non-negative floats order like their bits) give the reference's scales exactly.
 __global__ void ColumnAbsMaxKernel(const float* __restrict__ w, size_t K, size_t N,
                                    unsigned int* __restrict__ maxbits) {
+  AwaitPrevious();
   const size_t n = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (n >= N) return;
   const size_t rows_per = (K + gridDim.y - 1) / gridDim.y;
@@ -207,6 +214,7 @@ __global__ void ColumnAbsMaxKernel(const float* __restrict__ w, size_t K, size_t
 }
 
 __global__ void ColumnScaleKernel(const unsigned int* __restrict__ maxbits, size_t N, float* __restrict__ scales) {
+  AwaitPrevious();
   const size_t n = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (n >= N) return;
   const float m = __uint_as_float(maxbits[n]);
@@ -216,6 +224,7 @@ __global__ void ColumnScaleKernel(const unsigned int* __restrict__ maxbits, size
 
 __global__ void QuantizeLevelsKernel(const float* __restrict__ w, const float* __restrict__ scales, size_t count,
                                      size_t N, int8_t* __restrict__ q) {
+  AwaitPrevious();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count; i += stride) {
     float r = roundf(__fdiv_rn(w[i], scales[i % N]));   // roundf: halves away from zero, as std::round
@@ -230,7 +239,7 @@ void XentEvalTail(const float* probs, size_t width, const float* arg_probs, size
                   size_t real_rows, double* out, unsigned long long* tally, cudaStream_t s) {
   size_t blocks = arg_probs ? (real_rows + 7) / 8 : 0;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  XentEvalTailKernel<<<static_cast<unsigned>(blocks + 1), kTailThreads, 0, s>>>(probs, arg_probs, arg_cols, labels,
+  Next(XentEvalTailKernel, static_cast<unsigned>(blocks + 1), kTailThreads, 0, s)(probs, arg_probs, arg_cols, labels,
                                                                                real_rows, width, out, tally);
 }
 
@@ -240,9 +249,9 @@ void MseRealRowLoss(const float* pred, const float* target, size_t real_rows, si
   if (n) {
     size_t blocks = (n + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
-    SquaredDiffTermsKernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(pred, target, n, terms);
+    Next(SquaredDiffTermsKernel, static_cast<unsigned>(blocks), 256, 0, s)(pred, target, n, terms);
   }
-  OrderedFoldKernel<<<1, 32, 0, s>>>(terms, n, static_cast<double>(width), out, tally);
+  Next(OrderedFoldKernel, 1, 32, 0, s)(terms, n, static_cast<double>(width), out, tally);
 }
 
 void QuantizeColumns(const float* w, size_t K, size_t N, int8_t* levels, float* scales,
@@ -252,11 +261,11 @@ void QuantizeColumns(const float* w, size_t K, size_t N, int8_t* levels, float* 
   unsigned slices = static_cast<unsigned>((K + 63) / 64);
   if (slices > 1024) slices = 1024;
   const dim3 grid(static_cast<unsigned>((N + 127) / 128), slices);
-  ColumnAbsMaxKernel<<<grid, 128, 0, s>>>(w, K, N, maxbits_scratch);
-  ColumnScaleKernel<<<static_cast<unsigned>((N + 127) / 128), 128, 0, s>>>(maxbits_scratch, N, scales);
+  Next(ColumnAbsMaxKernel, grid, 128, 0, s)(w, K, N, maxbits_scratch);
+  Next(ColumnScaleKernel, static_cast<unsigned>((N + 127) / 128), 128, 0, s)(maxbits_scratch, N, scales);
   size_t blocks = (K * N + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  QuantizeLevelsKernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(w, scales, K * N, N, levels);
+  Next(QuantizeLevelsKernel, static_cast<unsigned>(blocks), 256, 0, s)(w, scales, K * N, N, levels);
 }
 
 void ArgmaxTally(const float* probs, const int32_t* labels, size_t N, size_t C,
@@ -264,14 +273,14 @@ void ArgmaxTally(const float* probs, const int32_t* labels, size_t N, size_t C,
   if (N == 0) return;
   size_t blocks = (N + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  ArgmaxTallyKernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(probs, labels, N, C, tally);
+  Next(ArgmaxTallyKernel, static_cast<unsigned>(blocks), 256, 0, s)(probs, labels, N, C, tally);
 }
 
 void CountNonFinite(const float* x, size_t n, unsigned long long* tally, cudaStream_t s) {
   if (n == 0) return;
   size_t blocks = (n + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  CountNonFiniteKernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(x, n, tally);
+  Next(CountNonFiniteKernel, static_cast<unsigned>(blocks), 256, 0, s)(x, n, tally);
 }
 
 }  // namespace see::k

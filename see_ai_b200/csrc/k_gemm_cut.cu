@@ -21,6 +21,7 @@
 #include <atomic>
 #include <type_traits>
 
+#include "launch.cuh"
 #include "lora_split.cuh"
 #include "umma_device.cuh"
 #include "umma_epilogue.cuh"
@@ -158,6 +159,7 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   const uint32_t tmem_base = bars->tmem_base;
   auto give_up = [&] { ep.status->wait_timeout = 1; bars->abort = 1; };
 
@@ -359,18 +361,7 @@ cudaError_t Launch(const UmmaCutPlan& plan, const CUtensorMap& map_b, const Umma
       return e;
     if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(plan.grid);
-  cfg.blockDim = dim3(kCutThreads);
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = plan.splits;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = plan.splits > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, map_b, ep, plan.splits, plan.parts);
+  return Next(kernel, plan.grid, kCutThreads, kSmem, s, plan.splits)(map_b, ep, plan.splits, plan.parts);
 }
 
 }  // namespace

@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "gemm_exact_common.cuh"
+#include "launch.cuh"
 
 namespace see::k {
 
@@ -51,6 +52,7 @@ __device__ __forceinline__ float LoadB(const Params& p, size_t k, size_t n) {
 // ---- quad order: BM x BN tile (BM * BN = 4096), 256 threads, 4x4 outputs per thread ----
 template <bool TA, typename BT, int BM, int BN>
 __global__ void __launch_bounds__(kThreads) GemmQuadKernel(Params p) {
+  AwaitPrevious();
   static_assert(BM * BN == 16 * kThreads, "4x4 outputs per thread");
   __shared__ __align__(16) float As[BK][BM + 4];
   __shared__ __align__(16) float Bs[BK][BN + 4];
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(kThreads) GemmQuadKernel(Params p) {
 // grouping is a function of the chunk count alone.
 constexpr int kFoldGroups = 8;
 __global__ void __launch_bounds__(32 * kFoldGroups) SplitKFoldKernel(Params p, size_t chunks) {
+  AwaitPrevious();
   __shared__ float group_sum[kFoldGroups][32];
   const size_t total = p.M * p.N;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -217,6 +220,7 @@ __global__ void __launch_bounds__(32 * kFoldGroups) SplitKFoldKernel(Params p, s
 // ---- lane order: BM x BN tile (BM * BN = 2048), 256 threads, 4x2 outputs x 8 lanes -----
 template <typename BT, int BM, int BN>
 __global__ void __launch_bounds__(kThreads) GemmLaneKernel(Params p) {
+  AwaitPrevious();
   static_assert(BM * BN == 8 * kThreads, "4x2 outputs per thread");
   __shared__ __align__(16) float As[BK][BM + 4];
   __shared__ __align__(16) float Bs[BK][BN + 4];
@@ -329,6 +333,7 @@ constexpr int kMergeRows = 64;
 template <int K>
 __global__ void __launch_bounds__(kThreads) MergeDeltasKernel(const __grid_constant__ MergeTable table,
                                                               unsigned long long* __restrict__ nonfinite) {
+  AwaitPrevious();
   __shared__ __align__(16) float As[kMergeRows][K];
   const MergeEntry& e = table.entry[blockIdx.y];
   const int tiles_n = static_cast<int>((e.N + 255) / 256);
@@ -418,6 +423,7 @@ struct FlatLoader {
 // Lane order when kLane, quad order otherwise.
 template <bool kLane, bool TA, bool TB, typename BT, int R>
 __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
+  AwaitPrevious();
   constexpr int T = 16 * R;
   __shared__ __align__(16) float As[T][kFlatK + 4];
   __shared__ __align__(16) float Bs[T][kFlatK + 4];
@@ -521,9 +527,9 @@ size_t LaneTiles(size_t M, size_t N) {
 template <bool kLane, bool TA, bool TB, typename BT>
 void LaunchFlat(const Params& p, cudaStream_t s) {
   if (static_cast<size_t>(Blocks(p.M, 32)) * Blocks(p.N, 32) >= 148)
-    GemmFlatKernel<kLane, TA, TB, BT, 2><<<dim3(Blocks(p.N, 32), Blocks(p.M, 32)), kThreads, 0, s>>>(p);
+    Next(GemmFlatKernel<kLane, TA, TB, BT, 2>, dim3(Blocks(p.N, 32), Blocks(p.M, 32)), kThreads, 0, s)(p);
   else
-    GemmFlatKernel<kLane, TA, TB, BT, 1><<<dim3(Blocks(p.N, 16), Blocks(p.M, 16)), kThreads, 0, s>>>(p);
+    Next(GemmFlatKernel<kLane, TA, TB, BT, 1>, dim3(Blocks(p.N, 16), Blocks(p.M, 16)), kThreads, 0, s)(p);
 }
 
 template <bool TA, typename BT>
@@ -531,11 +537,11 @@ void LaunchQuad(const Params& p, unsigned z, cudaStream_t s) {
   if (z == 1 && !p.partials && QuadTiles(p.M, p.N) < 148) {
     LaunchFlat<false, TA, false, BT>(p, s);
   } else if (p.N <= 16) {
-    GemmQuadKernel<TA, BT, 256, 16><<<dim3(Blocks(p.N, 16), Blocks(p.M, 256), z), kThreads, 0, s>>>(p);
+    Next(GemmQuadKernel<TA, BT, 256, 16>, dim3(Blocks(p.N, 16), Blocks(p.M, 256), z), kThreads, 0, s)(p);
   } else if (p.M <= 16) {
-    GemmQuadKernel<TA, BT, 16, 256><<<dim3(Blocks(p.N, 256), Blocks(p.M, 16), z), kThreads, 0, s>>>(p);
+    Next(GemmQuadKernel<TA, BT, 16, 256>, dim3(Blocks(p.N, 256), Blocks(p.M, 16), z), kThreads, 0, s)(p);
   } else {
-    GemmQuadKernel<TA, BT, 64, 64><<<dim3(Blocks(p.N, 64), Blocks(p.M, 64), z), kThreads, 0, s>>>(p);
+    Next(GemmQuadKernel<TA, BT, 64, 64>, dim3(Blocks(p.N, 64), Blocks(p.M, 64), z), kThreads, 0, s)(p);
   }
 }
 
@@ -544,11 +550,11 @@ void LaunchLane(const Params& p, cudaStream_t s) {
   if (LaneTiles(p.M, p.N) < 148) {
     LaunchFlat<true, false, true, BT>(p, s);
   } else if (p.N <= 16) {
-    GemmLaneKernel<BT, 128, 16><<<dim3(Blocks(p.N, 16), Blocks(p.M, 128)), kThreads, 0, s>>>(p);
+    Next(GemmLaneKernel<BT, 128, 16>, dim3(Blocks(p.N, 16), Blocks(p.M, 128)), kThreads, 0, s)(p);
   } else if (p.M <= 16) {
-    GemmLaneKernel<BT, 16, 128><<<dim3(Blocks(p.N, 128), Blocks(p.M, 16)), kThreads, 0, s>>>(p);
+    Next(GemmLaneKernel<BT, 16, 128>, dim3(Blocks(p.N, 128), Blocks(p.M, 16)), kThreads, 0, s)(p);
   } else {
-    GemmLaneKernel<BT, 64, 32><<<dim3(Blocks(p.N, 32), Blocks(p.M, 64)), kThreads, 0, s>>>(p);
+    Next(GemmLaneKernel<BT, 64, 32>, dim3(Blocks(p.N, 32), Blocks(p.M, 64)), kThreads, 0, s)(p);
   }
 }
 
@@ -573,10 +579,10 @@ void MergeDeltas(const MergeTable& table, int count, uint32_t K, unsigned long l
     blocks = std::max<size_t>(blocks, ((table.entry[i].M + kMergeRows - 1) / kMergeRows) * ((table.entry[i].N + 255) / 256));
   const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(count));
   switch (K) {
-    case 4: MergeDeltasKernel<4><<<grid, kThreads, 0, s>>>(table, nonfinite); break;
-    case 8: MergeDeltasKernel<8><<<grid, kThreads, 0, s>>>(table, nonfinite); break;
-    case 12: MergeDeltasKernel<12><<<grid, kThreads, 0, s>>>(table, nonfinite); break;
-    default: MergeDeltasKernel<16><<<grid, kThreads, 0, s>>>(table, nonfinite); break;
+    case 4: Next(MergeDeltasKernel<4>, grid, kThreads, 0, s)(table, nonfinite); break;
+    case 8: Next(MergeDeltasKernel<8>, grid, kThreads, 0, s)(table, nonfinite); break;
+    case 12: Next(MergeDeltasKernel<12>, grid, kThreads, 0, s)(table, nonfinite); break;
+    default: Next(MergeDeltasKernel<16>, grid, kThreads, 0, s)(table, nonfinite); break;
   }
 }
 
@@ -616,7 +622,7 @@ bool GemmExact(const GemmArgs& a, cudaStream_t s) {
       p.partials = a.split_scratch;
       if (!tn_partials(p, chunks, s)) LaunchQuad<true, float>(p, static_cast<unsigned>(chunks), s);
       const size_t blocks = (a.M * a.N + 31) / 32;
-      SplitKFoldKernel<<<static_cast<unsigned>(blocks), 32 * kFoldGroups, 0, s>>>(p, chunks);
+      Next(SplitKFoldKernel, static_cast<unsigned>(blocks), 32 * kFoldGroups, 0, s)(p, chunks);
       return false;
     }
     LaunchQuad<true, float>(p, 1, s);

@@ -24,6 +24,7 @@
 #include <atomic>
 
 #include "gemm_exact_common.cuh"
+#include "launch.cuh"
 #include "umma_device.cuh"
 
 namespace see::k {
@@ -93,6 +94,7 @@ struct FastTile {
 
 template <int kMode, int LM, int LN, int RM, int RN>
 __global__ void __launch_bounds__(kThreads) FastGemmKernel(FastParams p) {
+  AwaitPrevious();
   using T = FastTile<kMode, LM, LN, RM, RN>;
   constexpr int TM = T::TM, TN = T::TN;
   extern __shared__ __align__(16) float smem[];
@@ -245,18 +247,7 @@ bool Launch(FastParams p, cudaStream_t s) {
   int splits = 1;
   while (splits < 8 && tiles * splits * 2 <= 148 + 74 && p.K >= splits * 2 * 32) splits *= 2;
   p.per_split = ((p.K + splits - 1) / splits + 3) / 4 * 4;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = splits > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, FastGemmKernel<kMode, LM, LN, RM, RN>, p) == cudaSuccess;
+  return Next(FastGemmKernel<kMode, LM, LN, RM, RN>, static_cast<unsigned>(tiles * splits), kThreads, smem, s, static_cast<unsigned>(splits))(p) == cudaSuccess;
 }
 
 // The tile whose narrow side fits the output's: 64 x 8 and 64 x 16 for rank-wide results, 8 x 64 and 16 x 64 for

@@ -19,6 +19,7 @@
 #include <atomic>
 
 #include "gemm_exact_common.cuh"
+#include "launch.cuh"
 
 #ifndef SEE_SKINNY_NAMESPACE
 #define SEE_SKINNY_NAMESPACE exact
@@ -83,6 +84,7 @@ constexpr size_t kReduceMaxK = 3072;
 
 template <int G, bool kLane, int R, int Q, int kReduceThreads>
 __global__ void __launch_bounds__(kReduceThreads) ReduceKernel(Params p) {
+  AwaitPrevious();
   constexpr int N = 4 * G;
   constexpr int kRowsPerWarp = 32 / G;  // per row slot; a warp covers R of these
   constexpr int kRowsPerBlock = R * kRowsPerWarp * (kReduceThreads / 32);
@@ -242,7 +244,7 @@ bool LaunchReduceAs(const Params& p, cudaStream_t s) {
     if (tracked) configured_on[dev].store(true, std::memory_order_release);
   }
   const unsigned blocks = static_cast<unsigned>((p.M + kRowsPerBlock - 1) / kRowsPerBlock);
-  ReduceKernel<G, kLane, R, Q, kReduceThreads><<<blocks, kReduceThreads, smem, s>>>(p);
+  Next(ReduceKernel<G, kLane, R, Q, kReduceThreads>, blocks, kReduceThreads, smem, s)(p);
   return true;
 }
 
@@ -282,6 +284,7 @@ __host__ __device__ inline size_t StagedSmemFloats(size_t K) {
 
 template <int G, bool kLane>
 __global__ void __launch_bounds__(StagedShape<G>::kThreads) ReduceStagedKernel(Params p) {
+  AwaitPrevious();
   constexpr int N = 4 * G;
   constexpr int kThreads = StagedShape<G>::kThreads, kRows = StagedShape<G>::kRows;
   constexpr int kRowsPerWarp = 32 / G;
@@ -413,7 +416,7 @@ bool LaunchReduceStaged(const Params& p, cudaStream_t s) {
   }
   constexpr int kRows = StagedShape<G>::kRows;
   const unsigned blocks = static_cast<unsigned>((p.M + kRows - 1) / kRows);
-  ReduceStagedKernel<G, kLane><<<blocks, StagedShape<G>::kThreads, smem, s>>>(p);
+  Next(ReduceStagedKernel<G, kLane>, blocks, StagedShape<G>::kThreads, smem, s)(p);
   return true;
 }
 
@@ -463,6 +466,7 @@ constexpr int kExpandBatch = 4;
 
 template <int K, bool kLane, bool kTail>
 __global__ void __launch_bounds__(kExpandThreads) ExpandKernel(Params p) {
+  AwaitPrevious();
   __shared__ __align__(16) float As[kExpandRows][K];
   const size_t r0 = static_cast<size_t>(blockIdx.y) * kExpandRows;
   const int rows = p.M - r0 < static_cast<size_t>(kExpandRows) ? static_cast<int>(p.M - r0) : kExpandRows;
@@ -581,11 +585,11 @@ void LaunchExpand(const Params& p, bool lane_order, cudaStream_t s) {
   const dim3 grid(static_cast<unsigned>((p.N / 4 + kExpandThreads - 1) / kExpandThreads),
                   static_cast<unsigned>((p.M + kExpandRows - 1) / kExpandRows));
   if (p.tail_out) {
-    if (lane_order) ExpandKernel<K, true, true><<<grid, kExpandThreads, 0, s>>>(p);
-    else ExpandKernel<K, false, true><<<grid, kExpandThreads, 0, s>>>(p);
+    if (lane_order) Next(ExpandKernel<K, true, true>, grid, kExpandThreads, 0, s)(p);
+    else Next(ExpandKernel<K, false, true>, grid, kExpandThreads, 0, s)(p);
   } else {
-    if (lane_order) ExpandKernel<K, true, false><<<grid, kExpandThreads, 0, s>>>(p);
-    else ExpandKernel<K, false, false><<<grid, kExpandThreads, 0, s>>>(p);
+    if (lane_order) Next(ExpandKernel<K, true, false>, grid, kExpandThreads, 0, s)(p);
+    else Next(ExpandKernel<K, false, false>, grid, kExpandThreads, 0, s)(p);
   }
 }
 
@@ -626,6 +630,7 @@ static_assert(kTnChunk == kSplitKChunk, "the staging buffer holds the largest ch
 
 template <bool kWideA, int R, int kChunk>
 __global__ void __launch_bounds__(kTnThreads) TnPartialKernel(Params p) {
+  AwaitPrevious();
   __shared__ __align__(16) float Ns[R][kChunk + 4];
   const size_t W = kWideA ? p.M : p.N;
   const float* wide = kWideA ? p.A : static_cast<const float*>(p.B);
@@ -712,10 +717,10 @@ __global__ void __launch_bounds__(kTnThreads) TnPartialKernel(Params p) {
 template <bool kWideA, int kChunk>
 bool LaunchTnChunk(const Params& p, int R, dim3 grid, cudaStream_t s) {
   switch (R) {
-    case 4: TnPartialKernel<kWideA, 4, kChunk><<<grid, kTnThreads, 0, s>>>(p); return true;
-    case 8: TnPartialKernel<kWideA, 8, kChunk><<<grid, kTnThreads, 0, s>>>(p); return true;
-    case 12: TnPartialKernel<kWideA, 12, kChunk><<<grid, kTnThreads, 0, s>>>(p); return true;
-    case 16: TnPartialKernel<kWideA, 16, kChunk><<<grid, kTnThreads, 0, s>>>(p); return true;
+    case 4: Next(TnPartialKernel<kWideA, 4, kChunk>, grid, kTnThreads, 0, s)(p); return true;
+    case 8: Next(TnPartialKernel<kWideA, 8, kChunk>, grid, kTnThreads, 0, s)(p); return true;
+    case 12: Next(TnPartialKernel<kWideA, 12, kChunk>, grid, kTnThreads, 0, s)(p); return true;
+    case 16: Next(TnPartialKernel<kWideA, 16, kChunk>, grid, kTnThreads, 0, s)(p); return true;
     default: return false;
   }
 }

@@ -27,6 +27,7 @@
 
 #include "act_expr.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "shadow.cuh"
 #include "umma_device.cuh"
 #include "umma_epilogue.cuh"
@@ -173,6 +174,7 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
@@ -563,6 +565,7 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
   __syncthreads();
   if constexpr (kPair) ClusterSync();   // the peer's barriers exist before anything signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  AwaitPrevious();
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
@@ -957,6 +960,7 @@ __device__ __forceinline__ uint16_t WeightBits(T v, const float* k_scale, uint32
 template <typename T>
 __global__ void WeightToBf16Kernel(const T* __restrict__ src, uint16_t* __restrict__ dst, uint32_t N,
                                    uint32_t K, bool transpose, const float* __restrict__ k_scale) {
+  AwaitPrevious();
   __shared__ uint16_t tile[32][33];
   const uint32_t bx = blockIdx.x * 32, by = blockIdx.y * 32;
   if (!transpose) {  // src [N][K] -> dst [N][K]
@@ -990,27 +994,6 @@ template <uint32_t kTN>
 static size_t UmmaTileSmemBytes() {
   using T = TTile<kTN>;
   return T::kStages * T::kStageBytes + sizeof(TBarriers) + 1024;
-}
-
-// A launch with an optional cluster dimension.
-// (Programmatic dependent launches — the next kernel's set-up run beside this
-// one's tail — were measured on the whole step and cost 1 %: not used.)
-template <typename... KArgs, typename... Args>
-static cudaError_t LaunchClustered(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                   unsigned cluster, Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 // Calls f(kernel, shared-memory bytes) with the tile kernel of this width.
@@ -1135,12 +1118,12 @@ cudaError_t UmmaGemmLaunch(const UmmaGemmPlan& plan, const UmmaMaps& maps, const
   const Sums sums = ep.seg_blocks != 0 ? Sums::kPieces : ep.chained ? Sums::kChain : Sums::kPlain;
   if (!plan.persistent)
     return WithTileKernel(sums, plan.tn, [&](auto kernel, size_t bytes) {
-      return LaunchClustered(kernel, dim3(plan.grid), dim3(kTThreads), bytes, s, plan.splits, maps, ep, plan.splits);
+      return Next(kernel, plan.grid, kTThreads, bytes, s, plan.splits)(maps, ep, plan.splits);
     });
   // An addend or the x of an absorbed backward activation is software-pipelined (16 bytes at a time).
   const bool side_loads = (ep.addend != nullptr || ep.fuse_mode == kFuseActBwd) && (ep.N & 3) == 0;
   return WithPersistentKernel(sums, side_loads, plan.pair, [&](auto kernel, size_t bytes) {
-    return LaunchClustered(kernel, dim3(plan.grid), dim3(kPThreads), bytes, s, plan.pair ? 2u : 1u, maps, ep, plan.band);
+    return Next(kernel, plan.grid, kPThreads, bytes, s, plan.pair ? 2u : 1u)(maps, ep, plan.band);
   });
 }
 
@@ -1150,13 +1133,13 @@ void WeightToBf16(const void* src, BType type, uint16_t* dst, uint32_t N, uint32
   dim3 grid = transpose ? dim3((N + 31) / 32, (K + 31) / 32) : dim3((K + 31) / 32, (N + 31) / 32);
   switch (type) {
     case BType::kI8:
-      WeightToBf16Kernel<int8_t><<<grid, block, 0, s>>>(static_cast<const int8_t*>(src), dst, N, K, transpose, k_scale);
+      Next(WeightToBf16Kernel<int8_t>, grid, block, 0, s)(static_cast<const int8_t*>(src), dst, N, K, transpose, k_scale);
       break;
     case BType::kBf16:
-      WeightToBf16Kernel<uint16_t><<<grid, block, 0, s>>>(static_cast<const uint16_t*>(src), dst, N, K, transpose, k_scale);
+      Next(WeightToBf16Kernel<uint16_t>, grid, block, 0, s)(static_cast<const uint16_t*>(src), dst, N, K, transpose, k_scale);
       break;
     case BType::kF32:
-      WeightToBf16Kernel<float><<<grid, block, 0, s>>>(static_cast<const float*>(src), dst, N, K, transpose, k_scale);
+      Next(WeightToBf16Kernel<float>, grid, block, 0, s)(static_cast<const float*>(src), dst, N, K, transpose, k_scale);
       break;
   }
 }

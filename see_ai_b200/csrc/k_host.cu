@@ -7,6 +7,7 @@
 // the feed-forward plan's 121 us.  A kernel that reads or writes pinned host memory
 // itself costs one launch.  Scalars travel as kernel parameters.
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace see::k {
 
@@ -27,6 +28,7 @@ __device__ __forceinline__ void CopyBytes(uint8_t* dst, const uint8_t* src, size
 }
 
 __global__ void StageKernel(HostCopy a, HostCopy b) {
+  AwaitPrevious();
   const size_t t = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t threads = static_cast<size_t>(gridDim.x) * blockDim.x;
   if (a.bytes) CopyBytes(static_cast<uint8_t*>(a.dst), static_cast<const uint8_t*>(a.src), a.bytes, t, threads);
@@ -34,6 +36,7 @@ __global__ void StageKernel(HostCopy a, HostCopy b) {
 }
 
 __global__ void PublishKernel(PublishList list, uint32_t* __restrict__ host) {
+  AwaitPrevious();
   uint32_t at = 0;
   for (int i = 0; i < list.count; ++i) {
     for (uint32_t w = threadIdx.x; w < list.item[i].words; w += blockDim.x) host[at + w] = list.item[i].src[w];
@@ -41,18 +44,18 @@ __global__ void PublishKernel(PublishList list, uint32_t* __restrict__ host) {
   }
 }
 
-__global__ void SetScalarsKernel(AdamScalars v, AdamScalars* dst) { *dst = v; }
+__global__ void SetScalarsKernel(AdamScalars v, AdamScalars* dst) { AwaitPrevious(); *dst = v; }
 
 }  // namespace
 
 void StageFromHost(const HostCopy& a, const HostCopy& b, cudaStream_t s) {
   const size_t quads = (a.bytes + b.bytes) / 16 + 1;
   const size_t blocks = quads < 64 * 256 ? (quads + 255) / 256 : 64;
-  StageKernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(a, b);
+  Next(StageKernel, static_cast<unsigned>(blocks), 256, 0, s)(a, b);
 }
 
-void PublishToHost(const PublishList& list, uint32_t* host, cudaStream_t s) { PublishKernel<<<1, 32, 0, s>>>(list, host); }
+void PublishToHost(const PublishList& list, uint32_t* host, cudaStream_t s) { Next(PublishKernel, 1, 32, 0, s)(list, host); }
 
-void SetScalars(const AdamScalars& v, AdamScalars* dst, cudaStream_t s) { SetScalarsKernel<<<1, 1, 0, s>>>(v, dst); }
+void SetScalars(const AdamScalars& v, AdamScalars* dst, cudaStream_t s) { Next(SetScalarsKernel, 1, 1, 0, s)(v, dst); }
 
 }  // namespace see::k

@@ -29,6 +29,7 @@
 // a range into its [N, KX] operand in one launch.  Compiled WITH fused
 // multiply-add: nothing here reproduces a CPU rounding sequence bit for bit.
 #include "kernels.h"
+#include "launch.cuh"
 #include "lora_split.cuh"
 
 namespace see::k {
@@ -39,6 +40,7 @@ namespace {
 // segments; the threads of a row also zero its padding columns [6 R, KX).
 template <int R>
 __global__ void SplitRowsKernel(const float* __restrict__ t, uint16_t* __restrict__ out, uint32_t M, uint32_t KX) {
+  AwaitPrevious();
   constexpr uint32_t kQuads = R / 4;
   const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t row = idx / kQuads, j = (idx - row * kQuads) * 4;
@@ -63,6 +65,7 @@ __global__ void SplitRowsKernel(const float* __restrict__ t, uint16_t* __restric
 // [N, KX] operand.  (A thread per row, two bytes at a time, took 82 us for the 96 matrices of twelve layers of
 // 768 x 16; cutting every value once per segment costs less than its stores did.)
 __global__ void SplitWeightsKernel(const LoraWeight* __restrict__ table, int count) {
+  AwaitPrevious();
   const LoraWeight e = table[blockIdx.y];
   const uint32_t quads = e.kx / 4, idx = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t n = idx / quads, c = (idx - n * quads) * 4;
@@ -97,6 +100,7 @@ __global__ void SplitWeightsKernel(const LoraWeight* __restrict__ table, int cou
 template <bool kVec>
 __global__ void SplitMatrixKernel(const float* __restrict__ src, uint16_t* __restrict__ dst, uint32_t rows,
                                   uint32_t cols, uint32_t kp, const float* __restrict__ k_scale) {
+  AwaitPrevious();
   const uint32_t per_row = kp / 8;
   const size_t octs = static_cast<size_t>(rows) * per_row;
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
@@ -138,6 +142,7 @@ __global__ void SplitMatrixKernel(const float* __restrict__ src, uint16_t* __res
 // src [cols][rows] -> dst row r, column c = src[c][r].
 __global__ void SplitMatrixTransposedKernel(const float* __restrict__ src, uint16_t* __restrict__ dst,
                                             uint32_t rows, uint32_t cols, uint32_t kp, const float* __restrict__ k_scale) {
+  AwaitPrevious();
   __shared__ float tile[32][33];
   const uint32_t r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
   for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
@@ -172,14 +177,14 @@ void SplitMatrix(const float* src, uint16_t* dst, size_t rows, size_t cols, bool
   const uint32_t r = static_cast<uint32_t>(rows), c = static_cast<uint32_t>(cols);
   if (transposed) {
     const dim3 grid((r + 31) / 32, kp / 32), block(32, 8);
-    SplitMatrixTransposedKernel<<<grid, block, 0, s>>>(src, dst, r, c, kp, k_scale);
+    Next(SplitMatrixTransposedKernel, grid, block, 0, s)(src, dst, r, c, kp, k_scale);
     return;
   }
   size_t blocks = (rows * (kp / 8) + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   const bool vec = cols % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  if (vec) SplitMatrixKernel<true><<<static_cast<unsigned>(blocks), 256, 0, s>>>(src, dst, r, c, kp, k_scale);
-  else SplitMatrixKernel<false><<<static_cast<unsigned>(blocks), 256, 0, s>>>(src, dst, r, c, kp, k_scale);
+  if (vec) Next(SplitMatrixKernel<true>, static_cast<unsigned>(blocks), 256, 0, s)(src, dst, r, c, kp, k_scale);
+  else Next(SplitMatrixKernel<false>, static_cast<unsigned>(blocks), 256, 0, s)(src, dst, r, c, kp, k_scale);
 }
 
 uint32_t LoraSplitColumns(uint32_t r) { return (6 * r + 63) / 64 * 64; }
@@ -189,10 +194,10 @@ bool LoraSplitRows(const float* t, uint16_t* out, size_t M, uint32_t r, cudaStre
   const uint32_t KX = LoraSplitColumns(r);
   const unsigned blocks = static_cast<unsigned>((M * (r / 4) + 255) / 256);
   switch (r) {
-    case 4: SplitRowsKernel<4><<<blocks, 256, 0, s>>>(t, out, static_cast<uint32_t>(M), KX); return true;
-    case 8: SplitRowsKernel<8><<<blocks, 256, 0, s>>>(t, out, static_cast<uint32_t>(M), KX); return true;
-    case 12: SplitRowsKernel<12><<<blocks, 256, 0, s>>>(t, out, static_cast<uint32_t>(M), KX); return true;
-    case 16: SplitRowsKernel<16><<<blocks, 256, 0, s>>>(t, out, static_cast<uint32_t>(M), KX); return true;
+    case 4: Next(SplitRowsKernel<4>, blocks, 256, 0, s)(t, out, static_cast<uint32_t>(M), KX); return true;
+    case 8: Next(SplitRowsKernel<8>, blocks, 256, 0, s)(t, out, static_cast<uint32_t>(M), KX); return true;
+    case 12: Next(SplitRowsKernel<12>, blocks, 256, 0, s)(t, out, static_cast<uint32_t>(M), KX); return true;
+    case 16: Next(SplitRowsKernel<16>, blocks, 256, 0, s)(t, out, static_cast<uint32_t>(M), KX); return true;
     default: return false;
   }
 }
@@ -201,7 +206,7 @@ void LoraSplitWeights(const LoraWeight* table, int count, uint32_t max_n_out, ui
   if (count <= 0 || max_n_out == 0) return;
   const size_t quads = static_cast<size_t>(max_n_out) * (max_kx / 4);
   const dim3 grid(static_cast<unsigned>((quads + 255) / 256), static_cast<unsigned>(count));
-  SplitWeightsKernel<<<grid, 256, 0, s>>>(table, count);
+  Next(SplitWeightsKernel, grid, 256, 0, s)(table, count);
 }
 
 }  // namespace see::k

@@ -33,6 +33,7 @@
 #include <atomic>
 
 #include "kernels.h"
+#include "launch.cuh"
 #include "lora_split.cuh"
 #include "lora_umma.h"
 
@@ -177,6 +178,7 @@ template <int K, int R, bool kSplitK>
 __global__ void __launch_bounds__(kDownThreads, 1)
 LoraDownKernel(const float* __restrict__ x, const float* __restrict__ A, float* __restrict__ out,
                uint16_t* __restrict__ pieces, uint32_t piece_cols, size_t M, float alpha, int ksplit) {
+  AwaitPrevious();
   using S = DownSmem<K, R>;
   extern __shared__ __align__(16) float smem[];
   uint32_t* a_hi = reinterpret_cast<uint32_t*>(smem);
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 LoraBackwardKernel(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ t,
                    const float* __restrict__ B, float* __restrict__ dt, float* __restrict__ partials, size_t M,
                    float alpha_dt, uint16_t* __restrict__ pieces, uint32_t piece_cols) {
+  AwaitPrevious();
   using S = BackSmem<N, K, R>;
   extern __shared__ __align__(16) float smem[];
   float* dy_s = smem;
@@ -499,6 +502,7 @@ LoraBackwardKernel(const float* __restrict__ dy, const float* __restrict__ x, co
 __global__ void FoldPartialsKernel(const float* __restrict__ partials, size_t stride, int blocks, size_t n_db,
                                    size_t n_da, float alpha_db, float alpha_da, float* __restrict__ dB,
                                    float* __restrict__ dA) {
+  AwaitPrevious();
   const size_t tid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t i = tid >> 2;
   const int q = static_cast<int>(tid & 3);
@@ -574,9 +578,9 @@ bool LaunchDown(const float* x, const float* A, float* out, uint16_t* pieces, ui
   int ksplit = 1;
   while (ksplit < kDownWarps && (K / 16) % (2 * ksplit) == 0 && tiles * (2 * ksplit) <= sms * kDownWarps) ksplit *= 2;
   if (ksplit > 1)
-    LoraDownKernel<K, R, true><<<grid, kDownThreads, smem, s>>>(x, A, out, pieces, piece_cols, M, alpha, ksplit);
+    Next(LoraDownKernel<K, R, true>, grid, kDownThreads, smem, s)(x, A, out, pieces, piece_cols, M, alpha, ksplit);
   else
-    LoraDownKernel<K, R, false><<<grid, kDownThreads, smem, s>>>(x, A, out, pieces, piece_cols, M, alpha, 1);
+    Next(LoraDownKernel<K, R, false>, grid, kDownThreads, smem, s)(x, A, out, pieces, piece_cols, M, alpha, 1);
   return true;
 }
 
@@ -589,9 +593,9 @@ bool LaunchBackward(const LoraBackwardArgs& a, cudaStream_t s) {
   const int blocks = static_cast<int>(tiles < static_cast<size_t>(SmCount()) ? tiles : SmCount());
   const size_t stride = static_cast<size_t>(R) * N + static_cast<size_t>(K) * R;
   if (static_cast<size_t>(blocks) * stride > a.partials_floats) return false;
-  LoraBackwardKernel<N, K, R><<<blocks, kThreads, smem, s>>>(a.dy, a.x, a.t, a.B, a.dt, a.partials, a.M, a.alpha_dt,
+  Next(LoraBackwardKernel<N, K, R>, blocks, kThreads, smem, s)(a.dy, a.x, a.t, a.B, a.dt, a.partials, a.M, a.alpha_dt,
                                                              a.dt_pieces, LoraSplitColumns(static_cast<uint32_t>(R)));
-  FoldPartialsKernel<<<static_cast<unsigned>((4 * stride + 255) / 256), 256, 0, s>>>(
+  Next(FoldPartialsKernel, static_cast<unsigned>((4 * stride + 255) / 256), 256, 0, s)(
       a.partials, stride, blocks, static_cast<size_t>(R) * N, static_cast<size_t>(K) * R, a.alpha_db, a.alpha_da, a.dB,
       a.dA);
   return true;
@@ -621,7 +625,7 @@ bool LoraDown(const float* x, const float* A, float* out, size_t M, size_t K, si
 
 void LoraFoldPartials(const LoraBackwardArgs& a, int blocks, cudaStream_t s) {
   const size_t stride = a.r * a.N + a.K * a.r;
-  FoldPartialsKernel<<<static_cast<unsigned>((4 * stride + 255) / 256), 256, 0, s>>>(
+  Next(FoldPartialsKernel, static_cast<unsigned>((4 * stride + 255) / 256), 256, 0, s)(
       a.partials, stride, blocks, a.r * a.N, a.K * a.r, a.alpha_db, a.alpha_da, a.dB, a.dA);
 }
 

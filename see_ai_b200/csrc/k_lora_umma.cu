@@ -44,6 +44,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "launch.cuh"
 #include "lora_split.cuh"
 #include "lora_umma.h"
 #include "umma_device.cuh"
@@ -188,6 +189,7 @@ LoraBackwardUmmaKernel(const __grid_constant__ CUtensorMap map_dy, const __grid_
   TcFenceBefore();
   __syncthreads();
   TcFenceAfter();
+  AwaitPrevious();
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_acc = tmem_base, tmem_dt = tmem_base + kWide * kMaxChunks;   // dT: two buffers of 48 columns
 
@@ -536,7 +538,7 @@ cudaError_t LoraBackwardUmmaLaunch(const CUtensorMap& map_dy, const CUtensorMap&
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // Two blocks to a tile where every block of the launch still has an SM of its own (`blocks` is then the tiles).
   const bool split = 2 * blocks <= sms && static_cast<size_t>(blocks) * kRows >= a.M && a.N % (2 * kChunk) == 0 && a.K % (2 * kChunk) == 0;
-  LoraBackwardUmmaKernel<<<static_cast<unsigned>(split ? 2 * blocks : blocks), kThreads, kSmemBytes, s>>>(
+  Next(LoraBackwardUmmaKernel, static_cast<unsigned>(split ? 2 * blocks : blocks), kThreads, kSmemBytes, s)(
       map_dy, map_x, map_b, a.t, a.dt, a.partials, static_cast<uint32_t>(a.M), static_cast<uint32_t>(a.N),
       static_cast<uint32_t>(a.K), a.alpha_dt, a.dt_pieces, LoraSplitColumns(static_cast<uint32_t>(a.r)), status, split ? 2u : 1u);
   return cudaGetLastError();

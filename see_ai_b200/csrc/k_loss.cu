@@ -10,6 +10,7 @@
 #include <atomic>
 #include "act_expr.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "shadow.cuh"
 
 namespace see::k {
@@ -98,6 +99,7 @@ __device__ __forceinline__ double NegLogSafe(float p) {
 __global__ void XEntRowsKernel(const float* __restrict__ logits, const int32_t* __restrict__ labels,
                                float* __restrict__ probs, double* __restrict__ row_loss, size_t N,
                                size_t C, bool masked) {
+  AwaitPrevious();
   __shared__ float smem_f[32];
   for (size_t n = blockIdx.x; n < N; n += gridDim.x) {
     RowSoftmaxBlock(logits + n * C, probs + n * C, C, 1.0f, smem_f);
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 XEntRowsWideKernel(const float* __restrict__ logits, const int32_t* __restrict__ labels,
                    float* __restrict__ probs, double* __restrict__ row_loss, size_t N, size_t C,
                    bool masked, Shadow sh, float bwd_scale, bool store_probs) {
+  AwaitPrevious();
   extern __shared__ __align__(16) float4 row_smem[];
   __shared__ float smem_f[32];
   const int C4 = static_cast<int>(C / 4);
@@ -242,7 +245,7 @@ void LaunchXEntRowsWide(const float* logits, const int32_t* labels, float* probs
   }
   // One round of resident blocks walks the rows, several apiece: their prefetches reach across rows.
   const size_t blocks = 148 * kMinBlocks;
-  kernel<<<static_cast<unsigned>(N < blocks ? N : blocks), kThreads, C * sizeof(float), s>>>(
+  Next(kernel, static_cast<unsigned>(N < blocks ? N : blocks), kThreads, C * sizeof(float), s)(
       logits, labels, probs, row_loss, N, C, masked, sh, bwd_scale, store_probs);
 }
 
@@ -253,6 +256,7 @@ __global__ void XEntFoldKernel(const double* __restrict__ row_loss,
                                const int32_t* __restrict__ labels, float* __restrict__ loss,
                                size_t N, size_t grain, bool masked,
                                unsigned long long* __restrict__ count_out) {
+  AwaitPrevious();
   __shared__ double partial[kMaxChunks];
   __shared__ unsigned long long targets[kMaxChunks];
   const size_t chunk = threadIdx.x;
@@ -289,6 +293,7 @@ __global__ void XEntFoldKernel(const double* __restrict__ row_loss,
 
 __global__ void CountTargetsKernel(const int32_t* __restrict__ labels, size_t N,
                                    unsigned long long* __restrict__ count_out) {
+  AwaitPrevious();
   __shared__ unsigned long long smem[32];
   unsigned long long t = 0;
   for (size_t n = threadIdx.x; n < N; n += blockDim.x) t += labels[n] >= 0;
@@ -310,6 +315,7 @@ __global__ void XEntBwdKernel(const float* __restrict__ probs, const int32_t* __
                               const float* __restrict__ seed, float* __restrict__ dlogits, size_t N,
                               size_t C, bool masked,
                               const unsigned long long* __restrict__ count) {
+  AwaitPrevious();
   float scale;
   if (masked) {
     const unsigned long long T = *count;
@@ -340,6 +346,7 @@ __global__ void XEntBwdRowsKernel(const float* __restrict__ probs, const int32_t
                                   const float* __restrict__ seed, float* __restrict__ dlogits,
                                   size_t N, size_t C, bool masked,
                                   const unsigned long long* __restrict__ count, Shadow sh) {
+  AwaitPrevious();
   float scale;
   if (masked) {
     const unsigned long long T = *count;
@@ -379,6 +386,7 @@ __global__ void XEntBwdRowsKernel(const float* __restrict__ probs, const int32_t
 // chunks), chunks folded in order (reference: runtime/executor/loss.cc:128-152).
 __global__ void MsePartialKernel(const float* __restrict__ pred, const float* __restrict__ target,
                                  size_t n, size_t grain, double* __restrict__ partials) {
+  AwaitPrevious();
   __shared__ double smem[32];
   const size_t b = blockIdx.x * grain;
   const size_t e = b + grain < n ? b + grain : n;
@@ -392,12 +400,14 @@ __global__ void MsePartialKernel(const float* __restrict__ pred, const float* __
 }
 __global__ void MseFoldKernel(const double* __restrict__ partials, size_t chunks, size_t n,
                               float* __restrict__ loss) {
+  AwaitPrevious();
   double total = 0.0;
   for (size_t c = 0; c < chunks; ++c) total += partials[c];
   *loss = static_cast<float>(total / static_cast<double>(n));
 }
 __global__ void MseBwdKernel(const float* __restrict__ pred, const float* __restrict__ target,
                              const float* __restrict__ seed, float* __restrict__ dpred, size_t n) {
+  AwaitPrevious();
   const float scale = 2.0f * *seed / static_cast<float>(n);
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
@@ -408,6 +418,7 @@ __global__ void MseBwdKernel(const float* __restrict__ pred, const float* __rest
 __global__ void KLRowsKernel(const float* __restrict__ s_logits, const float* __restrict__ t_logits,
                              float* __restrict__ p_s, float* __restrict__ p_t,
                              double* __restrict__ row_loss, size_t N, size_t C, float inv_T) {
+  AwaitPrevious();
   __shared__ float smem_f[32];
   __shared__ double smem_d[32];
   for (size_t n = blockIdx.x; n < N; n += gridDim.x) {
@@ -429,6 +440,7 @@ __global__ void KLRowsKernel(const float* __restrict__ s_logits, const float* __
 }
 __global__ void KLFoldKernel(const double* __restrict__ row_loss, float* __restrict__ loss,
                              size_t N, size_t grain, float loss_scale) {
+  AwaitPrevious();
   __shared__ double partial[kMaxChunks];
   const size_t r0 = threadIdx.x * grain;
   double total = 0.0;
@@ -448,6 +460,7 @@ __global__ void KLFoldKernel(const double* __restrict__ row_loss, float* __restr
 __global__ void KLBwdKernel(const float* __restrict__ p_s, const float* __restrict__ p_t,
                             const float* __restrict__ seed, float* __restrict__ dlogits,
                             size_t total, float n_rows, float T, float loss_scale) {
+  AwaitPrevious();
   const float scale = (*seed * loss_scale) / (n_rows * T);
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -489,10 +502,10 @@ bool SoftmaxXEntFwd(bool masked, const float* logits, const int32_t* labels, flo
   } else {
     const int threads = C >= 1024 ? 256 : (C >= 128 ? 128 : 32);
     const unsigned blocks = static_cast<unsigned>(N < 148 * 16 ? N : 148 * 16);
-    XEntRowsKernel<<<blocks, threads, 0, s>>>(logits, labels, probs, row_scratch, N, C, masked);
+    Next(XEntRowsKernel, blocks, threads, 0, s)(logits, labels, probs, row_scratch, N, C, masked);
   }
   const size_t grain = ChunkGrain(N, RowGrain(C, kGrainMath));
-  XEntFoldKernel<<<1, kMaxChunks, 0, s>>>(row_scratch, labels, loss, N, grain, masked,
+  Next(XEntFoldKernel, 1, kMaxChunks, 0, s)(row_scratch, labels, loss, N, grain, masked,
                                          count_scratch);
   return fused;
 }
@@ -501,7 +514,7 @@ bool SoftmaxXEntBwd(bool masked, const float* probs, const int32_t* labels, cons
                     float* dlogits, size_t N, size_t C, unsigned long long* count_scratch,
                     cudaStream_t s, const Shadow* shadow) {
   if (N * C == 0) return false;
-  if (masked) CountTargetsKernel<<<1, 256, 0, s>>>(labels, N, count_scratch);
+  if (masked) Next(CountTargetsKernel, 1, 256, 0, s)(labels, N, count_scratch);
   if (C >= 1024 && (C & 3) == 0 &&
       ((reinterpret_cast<uintptr_t>(probs) | reinterpret_cast<uintptr_t>(dlogits)) & 15) == 0) {
     const size_t per_row = (C / 4 + 255) / 256;
@@ -510,10 +523,10 @@ bool SoftmaxXEntBwd(bool masked, const float* probs, const int32_t* labels, cons
     const bool shadowed = ShadowUsable(shadow, dlogits, N * C) && shadow->cols == C;
     Shadow sh = shadowed ? *shadow : Shadow{};
     if (!shadowed) sh.only = false;
-    XEntBwdRowsKernel<<<grid, 256, 0, s>>>(probs, labels, seed, dlogits, N, C, masked, count_scratch, sh);
+    Next(XEntBwdRowsKernel, grid, 256, 0, s)(probs, labels, seed, dlogits, N, C, masked, count_scratch, sh);
     return shadowed;
   }
-  XEntBwdKernel<<<GridFor(N * C, 256, 148 * 8), 256, 0, s>>>(probs, labels, seed, dlogits, N, C,
+  Next(XEntBwdKernel, GridFor(N * C, 256, 148 * 8), 256, 0, s)(probs, labels, seed, dlogits, N, C,
                                                             masked, count_scratch);
   return false;
 }
@@ -523,14 +536,14 @@ void MseFwd(const float* pred, const float* target, float* loss, size_t n, doubl
   if (n == 0) return;
   const size_t grain = ChunkGrain(n, kGrainCheap);
   const size_t chunks = (n + grain - 1) / grain;
-  MsePartialKernel<<<static_cast<unsigned>(chunks), 256, 0, s>>>(pred, target, n, grain, scratch);
-  MseFoldKernel<<<1, 1, 0, s>>>(scratch, chunks, n, loss);
+  Next(MsePartialKernel, static_cast<unsigned>(chunks), 256, 0, s)(pred, target, n, grain, scratch);
+  Next(MseFoldKernel, 1, 1, 0, s)(scratch, chunks, n, loss);
 }
 
 void MseBwd(const float* pred, const float* target, const float* seed, float* dpred, size_t n,
             cudaStream_t s) {
   if (n == 0) return;
-  MseBwdKernel<<<GridFor(n, 256, 148 * 8), 256, 0, s>>>(pred, target, seed, dpred, n);
+  Next(MseBwdKernel, GridFor(n, 256, 148 * 8), 256, 0, s)(pred, target, seed, dpred, n);
 }
 
 void KLDistillFwd(const float* s_logits, const float* t_logits, float* loss, float* p_s,
@@ -540,15 +553,15 @@ void KLDistillFwd(const float* s_logits, const float* t_logits, float* loss, flo
   const float inv_T = 1.0f / T;
   const int threads = C >= 1024 ? 256 : (C >= 128 ? 128 : 32);
   const unsigned blocks = static_cast<unsigned>(N < 148 * 16 ? N : 148 * 16);
-  KLRowsKernel<<<blocks, threads, 0, s>>>(s_logits, t_logits, p_s, p_t, row_scratch, N, C, inv_T);
+  Next(KLRowsKernel, blocks, threads, 0, s)(s_logits, t_logits, p_s, p_t, row_scratch, N, C, inv_T);
   const size_t grain = ChunkGrain(N, RowGrain(C, kGrainMath));
-  KLFoldKernel<<<1, kMaxChunks, 0, s>>>(row_scratch, loss, N, grain, loss_scale);
+  Next(KLFoldKernel, 1, kMaxChunks, 0, s)(row_scratch, loss, N, grain, loss_scale);
 }
 
 void KLDistillBwd(const float* p_s, const float* p_t, const float* seed, float* dlogits,
                   size_t N, size_t C, float T, float loss_scale, cudaStream_t s) {
   if (N * C == 0) return;
-  KLBwdKernel<<<GridFor(N * C, 256, 148 * 8), 256, 0, s>>>(p_s, p_t, seed, dlogits, N * C,
+  Next(KLBwdKernel, GridFor(N * C, 256, 148 * 8), 256, 0, s)(p_s, p_t, seed, dlogits, N * C,
                                                           static_cast<float>(N), T, loss_scale);
 }
 

@@ -8,6 +8,7 @@
 // survives the cast to float.  Compiled with -fmad=false so the output
 // expressions round like the reference's.
 #include "kernels.h"
+#include "launch.cuh"
 #include "shadow.cuh"
 
 namespace see::k {
@@ -26,6 +27,7 @@ __global__ void LayerNormFwdKernel(const float* __restrict__ x, const float* __r
                                    const float* __restrict__ beta, float* __restrict__ y,
                                    float* __restrict__ mean, float* __restrict__ rstd,
                                    size_t rows, size_t cols, float eps, Shadow sh) {
+  AwaitPrevious();
   const size_t r = blockIdx.x * static_cast<size_t>(kWarpsPerBlock) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
@@ -58,6 +60,7 @@ __global__ void LayerNormBwdKernel(const float* __restrict__ dy, const float* __
                                    const float* __restrict__ gamma, const float* __restrict__ mean,
                                    const float* __restrict__ rstd, float* __restrict__ dx,
                                    size_t rows, size_t cols) {
+  AwaitPrevious();
   const size_t r = blockIdx.x * static_cast<size_t>(kWarpsPerBlock) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
@@ -94,6 +97,7 @@ LayerNormFwdVecKernel(const float* __restrict__ x, const float* __restrict__ gam
                       const float* __restrict__ beta, float* __restrict__ y,
                       float* __restrict__ mean, float* __restrict__ rstd, size_t rows, float eps,
                       Shadow sh) {
+  AwaitPrevious();
   constexpr size_t cols = 128 * V;
   const size_t r = blockIdx.x * static_cast<size_t>(kWarpsPerBlock) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
@@ -148,6 +152,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 LayerNormBwdVecKernel(const float* __restrict__ dy, const float* __restrict__ x,
                       const float* __restrict__ gamma, const float* __restrict__ mean,
                       const float* __restrict__ rstd, float* dx, size_t rows, const float* addend, Shadow sh) {
+  AwaitPrevious();
   constexpr size_t cols = 128 * V;
   const size_t r = blockIdx.x * static_cast<size_t>(kWarpsPerBlock) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
@@ -197,6 +202,7 @@ inline bool Vec16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) 
 __global__ void RmsNormFwdKernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                  float* __restrict__ y, float* __restrict__ rstd, size_t rows,
                                  size_t cols, float eps) {
+  AwaitPrevious();
   const size_t r = blockIdx.x * static_cast<size_t>(kWarpsPerBlock) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
@@ -214,6 +220,7 @@ __global__ void RmsNormFwdKernel(const float* __restrict__ x, const float* __res
 __global__ void RmsNormBwdKernel(const float* __restrict__ dy, const float* __restrict__ x,
                                  const float* __restrict__ gamma, const float* __restrict__ rstd,
                                  float* __restrict__ dx, size_t rows, size_t cols) {
+  AwaitPrevious();
   const size_t r = blockIdx.x * static_cast<size_t>(kWarpsPerBlock) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
@@ -247,7 +254,7 @@ bool LayerNormFwd(const float* x, const float* gamma, const float* beta, float* 
       (!shadowed || ShadowUsable(shadow, y, rows * cols))) {
     const unsigned blocks = RowBlocks(rows);
 #define SEE_LN_FWD(V) \
-    case V: LayerNormFwdVecKernel<V><<<blocks, kWarpsPerBlock * 32, 0, s>>>(x, gamma, beta, y, mean, rstd, rows, eps, sh); break
+    case V: Next(LayerNormFwdVecKernel<V>, blocks, kWarpsPerBlock * 32, 0, s)(x, gamma, beta, y, mean, rstd, rows, eps, sh); break
     switch (cols / 128) {
       SEE_LN_FWD(1); SEE_LN_FWD(2); SEE_LN_FWD(3); SEE_LN_FWD(4);
       SEE_LN_FWD(5); SEE_LN_FWD(6); SEE_LN_FWD(7); SEE_LN_FWD(8);
@@ -255,7 +262,7 @@ bool LayerNormFwd(const float* x, const float* gamma, const float* beta, float* 
 #undef SEE_LN_FWD
     return shadowed;
   }
-  LayerNormFwdKernel<<<RowBlocks(rows), kWarpsPerBlock * 32, 0, s>>>(x, gamma, beta, y, mean, rstd,
+  Next(LayerNormFwdKernel, RowBlocks(rows), kWarpsPerBlock * 32, 0, s)(x, gamma, beta, y, mean, rstd,
                                                                      rows, cols, eps, sh);
   return shadowed;
 }
@@ -272,7 +279,7 @@ int LayerNormBwd(const float* dy, const float* x, const float* gamma, const floa
     const Shadow sh = fused && ShadowUsable(sum_shadow, sum_out, rows * cols) && sum_shadow->cols == cols
                           ? *sum_shadow : Shadow{};
 #define SEE_LN_BWD(V) \
-    case V: LayerNormBwdVecKernel<V><<<blocks, kWarpsPerBlock * 32, 0, s>>>(dy, x, gamma, mean, rstd, dx, rows, addend, sh); break
+    case V: Next(LayerNormBwdVecKernel<V>, blocks, kWarpsPerBlock * 32, 0, s)(dy, x, gamma, mean, rstd, dx, rows, addend, sh); break
     switch (cols / 128) {
       SEE_LN_BWD(1); SEE_LN_BWD(2); SEE_LN_BWD(3); SEE_LN_BWD(4);
       SEE_LN_BWD(5); SEE_LN_BWD(6); SEE_LN_BWD(7); SEE_LN_BWD(8);
@@ -280,20 +287,20 @@ int LayerNormBwd(const float* dy, const float* x, const float* gamma, const floa
 #undef SEE_LN_BWD
     return fused ? (sh.dst ? 2 : 1) : 0;
   }
-  LayerNormBwdKernel<<<RowBlocks(rows), kWarpsPerBlock * 32, 0, s>>>(dy, x, gamma, mean, rstd, dx,
+  Next(LayerNormBwdKernel, RowBlocks(rows), kWarpsPerBlock * 32, 0, s)(dy, x, gamma, mean, rstd, dx,
                                                                      rows, cols);
   return 0;
 }
 void RmsNormFwd(const float* x, const float* gamma, float* y, float* rstd, size_t rows,
                 size_t cols, float eps, cudaStream_t s) {
   if (rows == 0) return;
-  RmsNormFwdKernel<<<RowBlocks(rows), kWarpsPerBlock * 32, 0, s>>>(x, gamma, y, rstd, rows, cols,
+  Next(RmsNormFwdKernel, RowBlocks(rows), kWarpsPerBlock * 32, 0, s)(x, gamma, y, rstd, rows, cols,
                                                                    eps);
 }
 void RmsNormBwd(const float* dy, const float* x, const float* gamma, const float* rstd,
                 float* dx, size_t rows, size_t cols, cudaStream_t s) {
   if (rows == 0) return;
-  RmsNormBwdKernel<<<RowBlocks(rows), kWarpsPerBlock * 32, 0, s>>>(dy, x, gamma, rstd, dx, rows,
+  Next(RmsNormBwdKernel, RowBlocks(rows), kWarpsPerBlock * 32, 0, s)(dy, x, gamma, rstd, dx, rows,
                                                                    cols);
 }
 

@@ -15,6 +15,7 @@
 // rank, gathered into local memory) that are summed in rank order and scaled
 // by 1 / copies before the update — identical bits on every rank.
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace see::k {
 
@@ -36,6 +37,7 @@ __device__ __forceinline__ double WarpSumD(double v) {
 
 __global__ void SqPartialKernel(const float* __restrict__ g, size_t n, size_t grain,
                                 double* __restrict__ partials) {
+  AwaitPrevious();
   __shared__ double smem[8];
   const size_t b = blockIdx.x * grain;
   const size_t e = b + grain < n ? b + grain : n;
@@ -54,6 +56,7 @@ __global__ void SqPartialKernel(const float* __restrict__ g, size_t n, size_t gr
 
 __global__ void SqFoldKernel(const double* __restrict__ partials, size_t chunks,
                              double* __restrict__ sq) {
+  AwaitPrevious();
   double t = 0.0;
   for (size_t c = 0; c < chunks; ++c) t += partials[c];
   *sq = t;
@@ -62,6 +65,7 @@ __global__ void SqFoldKernel(const double* __restrict__ partials, size_t chunks,
 // reference: runtime/executor/optimizer.cc:42-50 (ClipScale)
 __global__ void ClipScaleKernel(const double* __restrict__ sq, float max_norm,
                                 float* __restrict__ scale, DeviceStatus* status) {
+  AwaitPrevious();
   float s = 1.0f;
   if (max_norm > 0.0f) {
     const double norm = sqrt(*sq);
@@ -77,6 +81,7 @@ __global__ void ClipScaleKernel(const double* __restrict__ sq, float max_norm,
 // reference: runtime/executor/optimizer.cc:70-85 (ClipGlobal's factor)
 __global__ void ClipGlobalScaleKernel(const float* __restrict__ acc, float max_norm,
                                       float* __restrict__ scale, DeviceStatus* status) {
+  AwaitPrevious();
   float s = 1.0f;
   const double norm = sqrt(static_cast<double>(acc[0]));
   if (!isfinite(norm)) {
@@ -88,12 +93,14 @@ __global__ void ClipGlobalScaleKernel(const float* __restrict__ acc, float max_n
 }
 
 __global__ void SqNormAccumKernel(const double* __restrict__ sq, float* __restrict__ acc) {
+  AwaitPrevious();
   acc[0] = static_cast<float>(static_cast<double>(acc[0]) + *sq);
 }
 
 // g *= s only when s != 1 (the reference leaves g untouched below the threshold).
 __global__ void ScaleInPlaceKernel(float* __restrict__ g, size_t n, const float* __restrict__ scale,
                                    const DeviceStatus* __restrict__ status) {
+  AwaitPrevious();
   if (status->refused) return;
   const float s = *scale;
   if (s == 1.0f) return;
@@ -116,6 +123,7 @@ __global__ void AdamWKernel(float* __restrict__ p, const float* __restrict__ g,
                             const float* __restrict__ clip_scale,
                             const DeviceStatus* __restrict__ status, int copies, size_t cstride,
                             float inv_copies) {
+  AwaitPrevious();
   if (status->refused) return;
   const AdamScalars a = *scalars;
   const float s = clip_scale ? *clip_scale : 1.0f;
@@ -138,6 +146,7 @@ __global__ void AdamWKernel(float* __restrict__ p, const float* __restrict__ g,
 __global__ void AdamWMultiKernel(const AdamTensor* __restrict__ table,
                                  const AdamScalars* __restrict__ scalars,
                                  const DeviceStatus* __restrict__ status, float inv_copies) {
+  AwaitPrevious();
   if (status->refused) return;
   const AdamTensor t = table[blockIdx.y];
   const AdamScalars a = *scalars;
@@ -163,6 +172,7 @@ __global__ void SgdKernel(float* __restrict__ p, const float* __restrict__ g, si
                           const float* __restrict__ clip_scale,
                           const DeviceStatus* __restrict__ status, int copies, size_t cstride,
                           float inv_copies) {
+  AwaitPrevious();
   if (status->refused) return;
   const float lr = scalars->lr, weight_decay = scalars->weight_decay;
   const float s = clip_scale ? *clip_scale : 1.0f;
@@ -175,6 +185,7 @@ __global__ void SgdKernel(float* __restrict__ p, const float* __restrict__ g, si
 
 __global__ void SumCopiesKernel(const float* __restrict__ g, float* __restrict__ out, size_t n,
                                 int copies, size_t cstride, float inv_copies) {
+  AwaitPrevious();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
     out[i] = GatherGrad(g, i, copies, cstride, inv_copies);
@@ -193,35 +204,35 @@ void L2Squared(const float* g, size_t n, double* partials, double* sq, cudaStrea
   const size_t grain = ChunkGrain(n, kGrainCheap);
   const size_t chunks = n == 0 ? 0 : (n + grain - 1) / grain;
   if (chunks)
-    SqPartialKernel<<<static_cast<unsigned>(chunks), 256, 0, s>>>(g, n, grain, partials);
-  SqFoldKernel<<<1, 1, 0, s>>>(partials, chunks, sq);
+    Next(SqPartialKernel, static_cast<unsigned>(chunks), 256, 0, s)(g, n, grain, partials);
+  Next(SqFoldKernel, 1, 1, 0, s)(partials, chunks, sq);
 }
 
 void ClipScaleFromSq(const double* sq, float max_norm, float* scale, DeviceStatus* status,
                      cudaStream_t s) {
-  ClipScaleKernel<<<1, 1, 0, s>>>(sq, max_norm, scale, status);
+  Next(ClipScaleKernel, 1, 1, 0, s)(sq, max_norm, scale, status);
 }
 
 void ScaleInPlaceBy(float* g, size_t n, const float* scale, const DeviceStatus* status,
                     cudaStream_t s) {
   if (n == 0) return;
-  ScaleInPlaceKernel<<<GridFor(n), 256, 0, s>>>(g, n, scale, status);
+  Next(ScaleInPlaceKernel, GridFor(n), 256, 0, s)(g, n, scale, status);
 }
 
 void SqNormAccum(const double* sq, float* acc, cudaStream_t s) {
-  SqNormAccumKernel<<<1, 1, 0, s>>>(sq, acc);
+  Next(SqNormAccumKernel, 1, 1, 0, s)(sq, acc);
 }
 
 void ClipGlobalScale(const float* acc, float max_norm, float* scale, DeviceStatus* status,
                      cudaStream_t s) {
-  ClipGlobalScaleKernel<<<1, 1, 0, s>>>(acc, max_norm, scale, status);
+  Next(ClipGlobalScaleKernel, 1, 1, 0, s)(acc, max_norm, scale, status);
 }
 
 void AdamWStep(float* p, const float* g, float* m, float* v, size_t n, const AdamScalars* a,
                const float* clip_scale, const DeviceStatus* status, int g_copies,
                size_t copy_stride, float inv_copies, cudaStream_t s) {
   if (n == 0) return;
-  AdamWKernel<<<GridFor(n), 256, 0, s>>>(p, g, m, v, n, a, clip_scale, status, g_copies,
+  Next(AdamWKernel, GridFor(n), 256, 0, s)(p, g, m, v, n, a, clip_scale, status, g_copies,
                                          copy_stride, inv_copies);
 }
 
@@ -230,7 +241,7 @@ void AdamWStepMulti(const AdamTensor* table, int count, uint64_t max_n, const Ad
   if (count <= 0 || max_n == 0) return;
   size_t bx = (max_n + 255) / 256;
   if (bx > 64) bx = 64;
-  AdamWMultiKernel<<<dim3(static_cast<unsigned>(bx), static_cast<unsigned>(count)), 256, 0, s>>>(
+  Next(AdamWMultiKernel, dim3(static_cast<unsigned>(bx), static_cast<unsigned>(count)), 256, 0, s)(
       table, a, status, inv_copies);
 }
 
@@ -238,14 +249,14 @@ void SgdStep(float* p, const float* g, size_t n, const AdamScalars* a,
              const float* clip_scale, const DeviceStatus* status, int g_copies,
              size_t copy_stride, float inv_copies, cudaStream_t s) {
   if (n == 0) return;
-  SgdKernel<<<GridFor(n), 256, 0, s>>>(p, g, n, a, clip_scale, status, g_copies,
+  Next(SgdKernel, GridFor(n), 256, 0, s)(p, g, n, a, clip_scale, status, g_copies,
                                        copy_stride, inv_copies);
 }
 
 void SumCopies(const float* g, float* out, size_t n, int g_copies, size_t copy_stride,
                float inv_copies, cudaStream_t s) {
   if (n == 0) return;
-  SumCopiesKernel<<<GridFor(n), 256, 0, s>>>(g, out, n, g_copies, copy_stride, inv_copies);
+  Next(SumCopiesKernel, GridFor(n), 256, 0, s)(g, out, n, g_copies, copy_stride, inv_copies);
 }
 
 }  // namespace see::k
