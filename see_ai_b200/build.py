@@ -35,6 +35,7 @@ CU_SOURCES = {
     "k_eval.cu": [],
     "k_host.cu": [],
     "k_attn_umma.cu": [],
+    "k_attn_slice.cu": [],
     "k_no_alloc.cu": ["-fmad=false"],
     "k_lora.cu": [],
     "k_gemm_skinny_fast.cu": [],

@@ -2561,7 +2561,9 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
       launched();
       break;
     case kAttnFwd:
-      k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
+      if (!fused || !k::AttnFwdSlices(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
+                                      Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), d_status_, s))
+        k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
                  Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
       launched();
       break;
@@ -2598,8 +2600,10 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
           break;
         }
       }
-      k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
-                 Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
+      if (!fused || !k::AttnFwdSlices(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
+                                      Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), d_status_, s))
+        k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
+                   Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
       launched();
       break;
     case kAttnFwdTiledSeg: {
@@ -2610,8 +2614,10 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
       break;
     }
     case kAttnDP:
-      k::AttnDP(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
-                Hi32(ins.out[1]), Lo32(ins.out[1]), OwnOrder(), s);
+      if (!fused || !k::AttnDPSlices(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
+                                     Hi32(ins.out[1]), Lo32(ins.out[1]), d_status_, s))
+        k::AttnDP(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
+                  Hi32(ins.out[1]), Lo32(ins.out[1]), fused, s);
       launched();
       break;
     case kAttnDV:

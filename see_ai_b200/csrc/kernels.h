@@ -176,6 +176,12 @@ void SetScalars(const AdamScalars& v, AdamScalars* dst, cudaStream_t s);
 void AttnFwd(const float* q, const float* k, const float* v, float* o, float* probs,
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,
              bool fused, cudaStream_t s);  // probs != null: cached family; stats != null: tiled family
+// The same on the tensor cores (k_attn_slice.cu), where the bits are not observed and no segment starts are given.  False: not
+// a geometry of theirs, and nothing was launched.
+bool AttnFwdSlices(const float* q, const float* k, const float* v, float* o, float* probs, float* stats, size_t B, size_t S,
+                   size_t H, size_t d, DeviceStatus* status, cudaStream_t s);
+bool AttnDPSlices(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, DeviceStatus* status,
+                  cudaStream_t s);
 void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, bool own_order,
             cudaStream_t s);
 void AttnDV(const float* probs, const float* dout, float* dv, size_t B, size_t S, size_t H,
