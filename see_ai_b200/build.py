@@ -63,6 +63,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(os.path.dirname(HERE), "include", "see_cuda.h"))
+    headers.append(os.path.join(CSRC, "k_gemm_skinny.cu"))   # (included by k_gemm_skinny_fast.cu)
     jobs = []
     objs = []
     for src, extra in CU_SOURCES.items():

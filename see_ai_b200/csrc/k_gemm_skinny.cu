@@ -459,62 +459,81 @@ namespace {
 // K floats) are staged in shared memory once and read back as broadcasts.  Rows
 // go four at a time: the four 16-byte addend loads are issued before any
 // arithmetic, so each thread keeps 64 bytes of the stream in flight.  The kernel
-// moves 32 bytes per 2K multiply-adds.
+// moves 32 bytes per 2K multiply-adds.  Of few rows it is a chain of memory round
+// trips, so all that its first rows need is asked for at once, eight rows to a
+// thread keep a thousand threads on an SM at 4096 x 768, and an activation's
+// code is there only where there is one.  Measured on a B200, us (32 rows to a
+// thread, W behind the barrier and column by column / now): 4096 x 768 of rank 16
+// 12.4 / 7.2, [N, K] 12.5 / 8.7, with an add 18.9 / 11.7; 4096 x 256 of rank 8 8.8 /
+// 3.5; 64 x 64 of rank 4 8.3 / 3.5; 32768 x 768 of rank 16 53 / 47.
 constexpr int kExpandThreads = 64;
-constexpr int kExpandRows = 32;
+constexpr int kExpandRows = 8;
 constexpr int kExpandBatch = 4;
 
-template <int K, bool kLane, bool kTail>
+template <int K, bool kLane, bool kTail, bool kPlain>
 __global__ void __launch_bounds__(kExpandThreads) ExpandKernel(Params p) {
   AwaitPrevious();
   __shared__ __align__(16) float As[kExpandRows][K];
-  const size_t r0 = static_cast<size_t>(blockIdx.y) * kExpandRows;
+  const size_t r0 = static_cast<size_t>(blockIdx.x) * kExpandRows;
   const int rows = p.M - r0 < static_cast<size_t>(kExpandRows) ? static_cast<int>(p.M - r0) : kExpandRows;
+  const size_t n = (static_cast<size_t>(blockIdx.y) * kExpandThreads + threadIdx.x) * 4;
+  const bool live = n < p.N;
+  // W, the first rows of the addends and the rows of A are all asked for before anything is waited for.
+  const float* B = static_cast<const float*>(p.B);
+  float w[K][4];
+  // W as [N, K]: the block's columns are one stretch of memory, which goes through shared memory (a thread's 4 K floats
+  // four apart from the next one's: neighbouring threads read different banks).
+  constexpr int kGroup = 4 * K + 4;
+  __shared__ __align__(16) float Ws[kLane ? kExpandThreads * kGroup : 4];
+  if (kLane) {
+    const size_t n0 = static_cast<size_t>(blockIdx.y) * (kExpandThreads * 4);
+    const int quads = static_cast<int>((p.N - n0 < kExpandThreads * 4 ? p.N - n0 : kExpandThreads * 4) * (K / 4));
+    const float4* src = reinterpret_cast<const float4*>(B + n0 * K);
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const int idx = static_cast<int>(threadIdx.x) + i * kExpandThreads;   // a quad of k of one column
+      if (idx < quads) *reinterpret_cast<float4*>(Ws + idx / K * kGroup + idx % K * 4) = src[idx];
+    }
+  } else {      // W is [K, N]
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float4 t = live ? *reinterpret_cast<const float4*>(B + static_cast<size_t>(k) * p.N + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+      w[k][0] = t.x; w[k][1] = t.y; w[k][2] = t.z; w[k][3] = t.w;
+    }
+  }
+  float4 d[kExpandBatch], tail[kTail ? kExpandBatch : 1];   // tail: the absorbed add's other operand, fetched with the addend
+  auto fetch = [&](int mb) {
+#pragma unroll
+    for (int u = 0; u < kExpandBatch; ++u) {
+      const bool there = live && mb + u < rows;
+      d[u] = p.addend && there ? *reinterpret_cast<const float4*>(p.addend + (r0 + mb + u) * p.N + n) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (kTail) tail[kTail ? u : 0] = there ? *reinterpret_cast<const float4*>(p.tail_addend + (r0 + mb + u) * p.N + n) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+  };
+  fetch(0);
   {
     const float4* src = reinterpret_cast<const float4*>(p.A + r0 * K);
     for (int idx = threadIdx.x; idx < rows * K / 4; idx += kExpandThreads)
       reinterpret_cast<float4*>(&As[0][0])[idx] = src[idx];
   }
   __syncthreads();
-  const size_t n = (static_cast<size_t>(blockIdx.x) * kExpandThreads + threadIdx.x) * 4;
-  if (n >= p.N) return;
-  const float* B = static_cast<const float*>(p.B);
-  float w[K][4];
-  if (kLane) {  // W is [N, K]
+  if (!live) return;
+  if (kLane) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int kq = 0; kq < K; kq += 4) {
-        const float4 t = *reinterpret_cast<const float4*>(B + (n + j) * K + kq);
+        const float4 t = *reinterpret_cast<const float4*>(Ws + threadIdx.x * kGroup + j * K + kq);
         w[kq][j] = t.x; w[kq + 1][j] = t.y; w[kq + 2][j] = t.z; w[kq + 3][j] = t.w;
       }
-  } else {      // W is [K, N]
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const float4 t = *reinterpret_cast<const float4*>(B + static_cast<size_t>(k) * p.N + n);
-      w[k][0] = t.x; w[k][1] = t.y; w[k][2] = t.z; w[k][3] = t.w;
-    }
   }
   float bias[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  if (p.bias) {
+  if (!kPlain && p.bias) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) bias[j] = p.bias[n + j];
   }
   for (int mb = 0; mb < rows; mb += kExpandBatch) {
-    float4 d[kExpandBatch];
-#pragma unroll
-    for (int u = 0; u < kExpandBatch; ++u)
-      d[u] = (p.addend && mb + u < rows)
-                 ? *reinterpret_cast<const float4*>(p.addend + (r0 + mb + u) * p.N + n)
-                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 tail[kTail ? kExpandBatch : 1];   // the absorbed add's other operand, fetched with the addend
-    if (kTail) {
-#pragma unroll
-      for (int u = 0; u < kExpandBatch; ++u)
-        tail[kTail ? u : 0] = mb + u < rows
-                                  ? *reinterpret_cast<const float4*>(p.tail_addend + (r0 + mb + u) * p.N + n)
-                                  : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
+    if (mb > 0) fetch(mb);
 #pragma unroll
     for (int u = 0; u < kExpandBatch; ++u) {
       if (mb + u >= rows) break;
@@ -562,7 +581,7 @@ __global__ void __launch_bounds__(kExpandThreads) ExpandKernel(Params p) {
       if (p.addend) {
         v[0] = d[u].x + v[0]; v[1] = d[u].y + v[1]; v[2] = d[u].z + v[2]; v[3] = d[u].w + v[3];
       }
-      if (!kLane) {
+      if (!kPlain) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (p.bias) v[j] = v[j] + bias[j];
@@ -582,14 +601,19 @@ __global__ void __launch_bounds__(kExpandThreads) ExpandKernel(Params p) {
 
 template <int K>
 void LaunchExpand(const Params& p, bool lane_order, cudaStream_t s) {
-  const dim3 grid(static_cast<unsigned>((p.N / 4 + kExpandThreads - 1) / kExpandThreads),
-                  static_cast<unsigned>((p.M + kExpandRows - 1) / kExpandRows));
-  if (p.tail_out) {
-    if (lane_order) Next(ExpandKernel<K, true, true>, grid, kExpandThreads, 0, s)(p);
-    else Next(ExpandKernel<K, false, true>, grid, kExpandThreads, 0, s)(p);
+  const dim3 grid(static_cast<unsigned>((p.M + kExpandRows - 1) / kExpandRows),
+                  static_cast<unsigned>((p.N / 4 + kExpandThreads - 1) / kExpandThreads));
+  auto launch = [&](auto kernel) { Next(kernel, grid, kExpandThreads, 0, s)(p); };
+  const bool plain = !p.bias && p.act == kActNone;   // (always, in the lane order)
+  if (lane_order) {
+    if (p.tail_out) launch(ExpandKernel<K, true, true, true>);
+    else launch(ExpandKernel<K, true, false, true>);
+  } else if (plain) {
+    if (p.tail_out) launch(ExpandKernel<K, false, true, true>);
+    else launch(ExpandKernel<K, false, false, true>);
   } else {
-    if (lane_order) Next(ExpandKernel<K, true, false>, grid, kExpandThreads, 0, s)(p);
-    else Next(ExpandKernel<K, false, false>, grid, kExpandThreads, 0, s)(p);
+    if (p.tail_out) launch(ExpandKernel<K, false, true, false>);
+    else launch(ExpandKernel<K, false, false, false>);
   }
 }
 
@@ -598,7 +622,7 @@ void LaunchExpand(const Params& p, bool lane_order, cudaStream_t s) {
 bool SkinnyExpand(const exact::Params& p, bool lane_order, cudaStream_t s) {
   if (p.K != 4 && p.K != 8 && p.K != 12 && p.K != 16) return false;
   if ((p.N & 3) != 0 || p.N < 64 || p.M < 64) return false;
-  if (p.M > 65535u * static_cast<size_t>(kExpandRows)) return false;
+  if (p.M > 65535u * 32u || p.N > 65535u * static_cast<size_t>(4 * kExpandThreads)) return false;
   if (p.accumulate || p.b_col_scale || p.a_k_scale || p.partials) return false;
   if (lane_order && (p.bias || p.act != kActNone)) return false;
   if (!Aligned16(p.A) || !Aligned16(p.B) || !Aligned16(p.C) || !Aligned16(p.addend)) return false;
