@@ -9,10 +9,14 @@
 // tiles anew: 6 x (16 + 32) KB per 64 k of a 128 x 256 tile.  Here 32 KB of f32 and each piece of B once: what a small
 // product (4096 x 256 x 256 of an f32 decoder, 4096 x 768 x 768 of an int8 one) waited for.
 //
-// One CTA a tile (or a cluster of `splits`, each a part of K): warp 0 brings B by TMA, warp 1 issues tcgen05.mma, and
-// sixteen working warps do the rest in turn, a block of 64 k at a time: cut block k (its f32 already in registers) into
-// the ring, ask for block k + 1, add the accumulator of block k - 1 into their registers while the tensor core
-// multiplies block k.  Then the tile goes through the ring's memory and leaves as whole rows.
+// One CTA a tile (or a cluster of `splits`, each a part of K): warp 0 brings B by TMA, warp 1 issues tcgen05.mma.  An f32
+// weight's few blocks of six products are cut and added by sixteen warps in turn, 64 k at a time: cut block k (its f32 already
+// in registers) into the ring, ask for block k + 1, add the accumulator of block k - 1 into their registers while the tensor core
+// multiplies block k.  An exact weight's blocks have three products and are many, so eight warps only cut and eight or, of wide tiles,
+// sixteen only add: of a block of 128 x 192 cutting takes 1500 cycles, adding 1250 (tensor memory is read against the products
+// that run), the products 1150; in turn that was 3000.  Then the tile goes through the ring's memory and leaves as whole rows.
+// (4096 x 768 x 768 of int8 22.4 / 19.8 us, 4096 x 768 x 3072 61.7 / 56.0, 2048 x 512 x 2048 24.1 / 21.4, 600 x 2048 x 512 14.4 / 12.9; f32
+// weights apart: 4096 x 256 x 256 9.2 / 9.0, 4096 x 256 x 1024 17.7 / 18.6, 300 x 5000 x 256 10.7 / 10.8.)
 //
 // Every wait on an mbarrier is bounded; one that runs out raises DeviceStatus::wait_timeout and the CTA stores nothing.
 #include <cuda.h>
@@ -36,7 +40,6 @@ using namespace umma_epi;
 
 constexpr uint32_t kBlockM = umma_cfg::kBlockM, kBlockK = umma_cfg::kBlockK;
 constexpr uint32_t kPieceBytes = kBlockM * kBlockK * 2;   // one bf16 piece of a block of A
-constexpr uint32_t kWorkWarps = 16, kWorkThreads = 32 * kWorkWarps, kCutThreads = 64 + kWorkThreads;
 constexpr uint32_t kMaxStages = 3;
 
 template <uint32_t kTN, uint32_t kBPieces>
@@ -46,7 +49,12 @@ struct CutShape {
   static constexpr uint32_t kFit = 216u * 1024u / kStageBytes;
   static constexpr uint32_t kStages = kFit < kMaxStages ? kFit : kMaxStages;
   static constexpr uint32_t kAccCols = kTN <= 64 ? 64 : (kTN <= 128 ? 128 : 256);
-  static constexpr uint32_t kColsPerWarp = kTN / 4;        // a warp's share of a tile: 32 rows x a quarter of the columns
+  // kApart (an exact weight: many blocks, of three products each): eight warps cut and eight or, of wide tiles, sixteen add.
+  // Otherwise (an f32 weight: a few blocks of six) sixteen warps do both in turn.
+  static constexpr bool kApart = kBPieces == 1;
+  static constexpr uint32_t kCutWarps = kApart ? 8 : 16, kAddWarps = kApart && kTN <= 128 ? 8 : 16, kFirstAdd = kApart ? 2 + kCutWarps : 2;
+  static constexpr uint32_t kColsPerWarp = kTN * 4 / kAddWarps;   // an adding warp has 32 rows of so many columns
+  static constexpr uint32_t kWorkThreads = 32 * (kApart ? kCutWarps + kAddWarps : 16), kThreads = 64 + kWorkThreads;
   static constexpr size_t kSmem = kStages * kStageBytes + 512 + 1024;
   static_assert(kStages >= 1 && kStages * kStageBytes >= kBlockM * kTN * 4, "the epilogue stages the whole tile in the ring");
 };
@@ -59,36 +67,39 @@ struct __align__(8) CutBarriers {
   volatile uint32_t nonfinite;
 };
 
-// Sixteen of the 128 x 64 f32 elements of block kb: rows r and r + 4 of the warp's eight, eight columns of each.
-struct CutRegs { float4 v[4]; };
-__device__ __forceinline__ void FetchBlock(CutRegs* f, const UmmaEpilogue& ep, uint32_t m0, uint32_t kb, bool vec) {
-  const uint32_t work = (threadIdx.x - 64) >> 5, lane = threadIdx.x & 31;
-  const uint32_t k = kb * kBlockK + (lane & 7) * 8;
+// A thread's part of the 128 x 64 f32 elements of block kb: some of the warp's rows, four apart, eight columns of each.
+template <uint32_t kWarps>
+struct CutRegs {
+  static constexpr uint32_t kRows = kBlockM / (4 * kWarps);
+  float4 v[2 * kRows];
+  static __device__ __forceinline__ uint32_t Row(uint32_t h) {
+    return ((threadIdx.x >> 5) - 2) * (4 * kRows) + h * 4 + ((threadIdx.x & 31) >> 3);
+  }
+};
+// kPlain: nothing but loads of 16 bytes (src_k % 4 == 0: four elements are all in or all out), so that the thread goes on while
+// they fly; a choice between two ways of loading would end in moves that wait for them.
+template <bool kPlain, uint32_t kWarps>
+__device__ __forceinline__ void FetchBlock(CutRegs<kWarps>* f, const UmmaEpilogue& ep, uint32_t m0, uint32_t kb) {
+  const uint32_t k = kb * kBlockK + (threadIdx.x & 7) * 8;
 #pragma unroll
-  for (uint32_t h = 0; h < 2; ++h) {
-    const uint32_t row = m0 + work * 8 + h * 4 + (lane >> 3);
+  for (uint32_t h = 0; h < CutRegs<kWarps>::kRows; ++h) {
+    const uint32_t row = m0 + CutRegs<kWarps>::Row(h);
     const float* p = ep.src_a + static_cast<size_t>(row) * ep.src_k + k;
 #pragma unroll
     for (uint32_t q = 0; q < 2; ++q) {
       const uint32_t c = k + 4 * q;
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (row < ep.M && c < ep.src_k) {
-        if (vec) {   // src_k % 4 == 0: four elements are all in or all out
-          x = __ldg(reinterpret_cast<const float4*>(p + 4 * q));
-        } else {
-          x.x = p[4 * q];
-          if (c + 1 < ep.src_k) x.y = p[4 * q + 1];
-          if (c + 2 < ep.src_k) x.z = p[4 * q + 2];
-          if (c + 3 < ep.src_k) x.w = p[4 * q + 3];
-        }
-        if (ep.src_a_scale) {
-          x.x = x.x * ep.src_a_scale[c];
-          if (c + 1 < ep.src_k) x.y = x.y * ep.src_a_scale[c + 1];
-          if (c + 2 < ep.src_k) x.z = x.z * ep.src_a_scale[c + 2];
-          if (c + 3 < ep.src_k) x.w = x.w * ep.src_a_scale[c + 3];
-        }
+      float4& x = f->v[2 * h + q];
+      x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row >= ep.M || c >= ep.src_k) continue;
+      if constexpr (kPlain) {
+        x = __ldg(reinterpret_cast<const float4*>(p + 4 * q));
+      } else {
+        auto at = [&](uint32_t e) {
+          if (c + e >= ep.src_k) return 0.0f;
+          return ep.src_a_scale ? p[4 * q + e] * ep.src_a_scale[c + e] : p[4 * q + e];
+        };
+        x = make_float4(at(0), at(1), at(2), at(3));
       }
-      f->v[2 * h + q] = x;
     }
   }
 }
@@ -101,10 +112,10 @@ __device__ __forceinline__ void CutPair(float lo, float hi, uint32_t (&p)[3]) {
     hi = hi - __uint_as_float(p[i] & 0xFFFF0000u);
   }
 }
-__device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs& f) {
-  const uint32_t work = (threadIdx.x - 64) >> 5, lane = threadIdx.x & 31;
+template <uint32_t kWarps>
+__device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs<kWarps>& f) {
 #pragma unroll
-  for (uint32_t h = 0; h < 2; ++h) {
+  for (uint32_t h = 0; h < CutRegs<kWarps>::kRows; ++h) {
     uint32_t w[3][4];
 #pragma unroll
     for (uint32_t q = 0; q < 2; ++q) {
@@ -115,7 +126,7 @@ __device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs& f) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) { w[i][2 * q] = a[i]; w[i][2 * q + 1] = b[i]; }
     }
-    const uint32_t at = Sw128Offset(work * 8 + h * 4 + (lane >> 3), lane & 7);
+    const uint32_t at = Sw128Offset(f.Row(h), threadIdx.x & 7);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
       *reinterpret_cast<uint4*>(pieces + i * kPieceBytes + at) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
@@ -124,7 +135,7 @@ __device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs& f) {
 
 // kParts: a CTA's blocks are summed in several parts.
 template <uint32_t kTN, uint32_t kBPieces, bool kParts>
-__global__ void __launch_bounds__(kCutThreads, 1)
+__global__ void __launch_bounds__((CutShape<kTN, kBPieces>::kThreads), 1)
 UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ UmmaEpilogue ep, uint32_t splits,
                   uint32_t parts) {
   using Sh = CutShape<kTN, kBPieces>;
@@ -143,13 +154,13 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < Sh::kStages; ++s) {
-      MbarInit(&bars->a_full[s], kWorkWarps);
+      MbarInit(&bars->a_full[s], Sh::kCutWarps);
       MbarInit(&bars->b_full[s], 1);
       MbarInit(&bars->empty[s], 1);
     }
     for (uint32_t b = 0; b < 2; ++b) {
       MbarInit(&bars->tmem_full[b], 1);
-      MbarInit(&bars->tmem_empty[b], kWorkWarps);
+      MbarInit(&bars->tmem_empty[b], Sh::kAddWarps);
     }
     bars->abort = 0;
     bars->nonfinite = 0;
@@ -217,94 +228,119 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
     }
     __syncwarp();
   } else {
-    // ---- cut, and add ----
-    const uint32_t quarter = warp & 3, columns = ((warp - 2) >> 2) * Sh::kColsPerWarp;
-    const uint32_t t_row = tmem_base + ((quarter * 32) << 16) + columns;
-    const bool vec = (ep.src_k & 3u) == 0 && (reinterpret_cast<uintptr_t>(ep.src_a) & 15) == 0;
-    // The blocks of a part of K are one chain of additions and the parts meet after that, as the piece form's CTAs do
-    // where it cuts K more often than this kernel: no chain is longer than there.
-    float sum[Sh::kColsPerWarp];
+    // ---- cut, and add: the roles of this warp ----
+    auto role = [&](auto cuts, auto adds) {
+      constexpr bool kCuts = decltype(cuts)::value, kAdds = decltype(adds)::value;
+      const uint32_t quarter = warp & 3, columns = kAdds ? ((warp - Sh::kFirstAdd) >> 2) * Sh::kColsPerWarp : 0;
+      const uint32_t t_row = tmem_base + ((quarter * 32) << 16) + columns;
+      // The blocks of a part of K are one chain of additions and the parts meet after that, as the piece form's CTAs do
+      // where it cuts K more often than this kernel: no chain is longer than there.
+      float sum[kAdds ? Sh::kColsPerWarp : 1];
 #pragma unroll
-    for (uint32_t j = 0; j < Sh::kColsPerWarp; ++j) sum[j] = 0.0f;
-    [[maybe_unused]] const uint32_t first_part = parts / splits * split;
-    [[maybe_unused]] uint32_t part = first_part, part_end = groups * (part + 1) / parts;
-    auto add = [&](uint32_t it) {   // the accumulator of this CTA's group number `it`
-      const uint32_t buf = it & 1;
-      bool there = MbarWait(&bars->tmem_full[buf], (it >> 1) & 1);
-      if (!there && lane == 0) give_up();
-      if (bars->abort) there = false;
-      there = __all_sync(0xFFFFFFFFu, there);
-      TcFenceAfter();
-      if (!there) return false;
+      for (uint32_t j = 0; j < (kAdds ? Sh::kColsPerWarp : 1u); ++j) sum[j] = 0.0f;
+      [[maybe_unused]] const uint32_t first_part = parts / splits * split;
+      [[maybe_unused]] uint32_t part = first_part, part_end = groups * (part + 1) / parts;
+      [[maybe_unused]] auto add = [&](uint32_t it) {   // the accumulator of this CTA's group number `it`
+        const uint32_t buf = it & 1;
+        bool there = MbarWait(&bars->tmem_full[buf], (it >> 1) & 1);
+        if (!there && lane == 0) give_up();
+        if (bars->abort) there = false;
+        there = __all_sync(0xFFFFFFFFu, there);
+        TcFenceAfter();
+        if (!there) return false;
+        constexpr uint32_t kChunk = kTN > 128 ? 8 : 16;   // (the registers of 26 warps hold 48 sums and no more than eight at once)
 #pragma unroll
-      for (uint32_t c = 0; c < Sh::kColsPerWarp; c += 16) {
-        uint32_t r[16];
-        TmemLoad16(t_row + buf * Sh::kAccCols + c, r);
-        TmemWaitLd();
+        for (uint32_t c = 0; c < Sh::kColsPerWarp; c += kChunk) {
+          uint32_t r[kChunk];
+          if constexpr (kChunk == 8) TmemLoad8(t_row + buf * Sh::kAccCols + c, r);
+          else TmemLoad16(t_row + buf * Sh::kAccCols + c, r);
+          TmemWaitLd();
 #pragma unroll
-        for (uint32_t j = 0; j < 16; ++j) sum[c + j] += __uint_as_float(r[j]);
-      }
-      TcFenceBefore();
-      __syncwarp();
-      if (lane == 0) MbarArrive(&bars->tmem_empty[buf]);
-      if constexpr (kParts) {
-        if (g0 + it + 1 == part_end) {   // the parts so far wait in tensor memory: the registers are full
-#pragma unroll
-          for (uint32_t c = 0; c < Sh::kColsPerWarp; c += 16) {
-            uint32_t r[16];
-            if (part > first_part) {
-              TmemLoad16(t_row + 2 * Sh::kAccCols + c, r);
-              TmemWaitLd();
-#pragma unroll
-              for (uint32_t j = 0; j < 16; ++j) sum[c + j] = __uint_as_float(r[j]) + sum[c + j];
-            }
-            if (part_end < g1) {
-#pragma unroll
-              for (uint32_t j = 0; j < 16; ++j) {
-                r[j] = __float_as_uint(sum[c + j]);
-                sum[c + j] = 0.0f;
-              }
-              TmemStore16(t_row + 2 * Sh::kAccCols + c, r);
-            }
-          }
-          TmemWaitSt();
-          ++part;
-          part_end = groups * (part + 1) / parts;
+          for (uint32_t j = 0; j < kChunk; ++j) sum[c + j] += __uint_as_float(r[j]);
         }
-      }
-      return true;
-    };
-    CutRegs f;
-    FetchBlock(&f, ep, m0, g0, vec);
-    for (uint32_t g = g0, it = 0; g < g1 && ok; ++g, ++it) {
-      const uint32_t s = it % Sh::kStages, round = it / Sh::kStages;
-      bool free = round == 0 || MbarWait(&bars->empty[s], (round - 1) & 1);
-      if (!free && lane == 0) give_up();
-      if (bars->abort) free = false;
-      if (!(ok = __all_sync(0xFFFFFFFFu, free))) break;
-      StoreBlock(smem + s * Sh::kStageBytes, f);
-      if (g + 1 < g1) FetchBlock(&f, ep, m0, g + 1, vec);
-      FenceProxyAsync();
-      __syncwarp();
-      if (lane == 0) MbarArrive(&bars->a_full[s]);
-      if (it > 0) ok = add(it - 1);
-    }
-    if (ok && g1 > g0) ok = add(g1 - g0 - 1);
-    if (ok) {
-      // All products are complete, so the ring is free: the tile goes there as [128][kTN] f32, 16-byte chunks XOR-ed
-      // with the row so that neither side conflicts.
-      if (!AllFinite(sum)) bars->nonfinite = 1;
-      float* dump = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kTN;
+        TcFenceBefore();
+        __syncwarp();
+        if (lane == 0) MbarArrive(&bars->tmem_empty[buf]);
+        if constexpr (kParts) {
+          if (g0 + it + 1 == part_end) {   // the parts so far wait in tensor memory: the registers are full
 #pragma unroll
-      for (uint32_t q = 0; q < Sh::kColsPerWarp / 4; ++q)
-        *reinterpret_cast<float4*>(dump + (((columns >> 2) + q) ^ (lane & 7u)) * 4) =
-            make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
+            for (uint32_t c = 0; c < Sh::kColsPerWarp; c += 16) {
+              uint32_t r[16];
+              if (part > first_part) {
+                TmemLoad16(t_row + 2 * Sh::kAccCols + c, r);
+                TmemWaitLd();
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j) sum[c + j] = __uint_as_float(r[j]) + sum[c + j];
+              }
+              if (part_end < g1) {
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j) {
+                  r[j] = __float_as_uint(sum[c + j]);
+                  sum[c + j] = 0.0f;
+                }
+                TmemStore16(t_row + 2 * Sh::kAccCols + c, r);
+              }
+            }
+            TmemWaitSt();
+            ++part;
+            part_end = groups * (part + 1) / parts;
+          }
+        }
+        return true;
+      };
+      // Cut block after block; where the same warps add, the one before while the products of this one run.
+      [[maybe_unused]] auto walk = [&](auto plain) {
+        constexpr bool kPlain = decltype(plain)::value;
+        CutRegs<Sh::kCutWarps> f;
+        FetchBlock<kPlain>(&f, ep, m0, g0);
+        for (uint32_t g = g0, it = 0; g < g1 && ok; ++g, ++it) {
+          const uint32_t s = it % Sh::kStages, round = it / Sh::kStages;
+          bool free = round == 0 || MbarWait(&bars->empty[s], (round - 1) & 1);
+          if (!free && lane == 0) give_up();
+          if (bars->abort) free = false;
+          if (!(ok = __all_sync(0xFFFFFFFFu, free))) break;
+          StoreBlock(smem + s * Sh::kStageBytes, f);
+          if (g + 1 < g1) FetchBlock<kPlain>(&f, ep, m0, g + 1);
+          FenceProxyAsync();
+          __syncwarp();
+          if (lane == 0) MbarArrive(&bars->a_full[s]);
+          if constexpr (kAdds)
+            if (it > 0) ok = add(it - 1);
+        }
+      };
+      if constexpr (kCuts) {
+        if ((ep.src_k & 3u) == 0 && (reinterpret_cast<uintptr_t>(ep.src_a) & 15) == 0 && !ep.src_a_scale) walk(std::true_type{});
+        else walk(std::false_type{});
+        if constexpr (kAdds)
+          if (ok && g1 > g0) ok = add(g1 - g0 - 1);
+      } else {
+        for (uint32_t it = 0; it < g1 - g0 && ok; ++it) ok = add(it);
+      }
+      if constexpr (kAdds) {
+        if (ok) {
+          // All products are complete, so the ring is free: the tile goes there as [128][kTN] f32, 16-byte chunks XOR-ed
+          // with the row so that neither side conflicts.
+          if (!AllFinite(sum)) bars->nonfinite = 1;
+          float* dump = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * kTN;
+#pragma unroll
+          for (uint32_t q = 0; q < Sh::kColsPerWarp / 4; ++q)
+            *reinterpret_cast<float4*>(dump + (((columns >> 2) + q) ^ (lane & 7u)) * 4) =
+                make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
+        }
+        TcFenceBefore();
+      }
+    };
+    if constexpr (!Sh::kApart) {
+      role(std::true_type{}, std::true_type{});
+    } else {
+      if (warp < Sh::kFirstAdd) role(std::true_type{}, std::false_type{});
+      else role(std::false_type{}, std::true_type{});
     }
-    TcFenceBefore();
   }
   __syncwarp();   // (one lane of the loading and of the issuing warp has walked the blocks: the barriers want whole warps)
   if (splits > 1) ClusterSync();
-  else if (work) asm volatile("bar.sync 1, %0;" ::"n"(kWorkThreads) : "memory");
+  else if (work) asm volatile("bar.sync 1, %0;" ::"n"(Sh::kWorkThreads) : "memory");
+  if (bars->abort) ok = false;
   if (work && ok) {
     const uint32_t dump = SmemAddr(smem);
     auto element = [&](uint32_t lr, uint32_t chunk) {
@@ -321,7 +357,7 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
     for (uint32_t p = 0; p < splits; ++p)
       remake = remake || (splits == 1 ? bars->nonfinite : LoadClusterU32(MapToCta(SmemAddr(const_cast<uint32_t*>(&bars->nonfinite)), p))) != 0;
     const bool ragged = (ep.N & 3u) != 0, plain = IsPlainStore(ep);
-    for (uint32_t i = wt; i < rows * kChunks; i += kWorkThreads) {
+    for (uint32_t i = wt; i < rows * kChunks; i += Sh::kWorkThreads) {
       const uint32_t lr = r0 + i / kChunks, chunk = i % kChunks, row = m0 + lr, n = n0 + chunk * 4;
       if (row >= ep.M || n >= ep.N) continue;
       const float4 acc = element(lr, chunk);
@@ -361,7 +397,7 @@ cudaError_t Launch(const UmmaCutPlan& plan, const CUtensorMap& map_b, const Umma
       return e;
     if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
   }
-  return Next(kernel, plan.grid, kCutThreads, kSmem, s, plan.splits)(map_b, ep, plan.splits, plan.parts);
+  return Next(kernel, plan.grid, CutShape<kTN, kBPieces>::kThreads, kSmem, s, plan.splits)(map_b, ep, plan.splits, plan.parts);
 }
 
 }  // namespace
@@ -373,7 +409,7 @@ UmmaCutPlan UmmaPlanCut(uint32_t M, uint32_t N, uint32_t groups, bool exact_b, u
   // us, f32 weights: 4096 x 256 x 256 14.0 (+2.8) / 9.7, 1024 x 256 x 256 8.4 (+2.0) / 8.0, 600 x 512 x 512 12.3 (+2.1) / 10.7,
   // 128 x 1024 x 1024 14.7 (+2.0) / 11.1, 300 x 5000 x 256 15.1 (+1.9) / 11.8, 4096 x 256 x 1024 21.7 (+5.9) / 18.5; past the line
   // 2048 x 512 x 2048 32.1 (+5.9) / 42.0, 4096 x 1024 x 256 18.8 (+2.7) / 22.4, 4096 x 4096 x 256 57.9 (+4.0) / 77.1; int8 weights:
-  // 4096 x 768 x 768 24.8 (+4.2) / 23.1, 4096 x 768 x 3072 69.0 (+20.9) / 67.9, 2048 x 512 x 2048 22.2 (+6.2) / 25.0; past it 4096 x
+  // 4096 x 768 x 768 24.8 (+4.2) / 19.8, 4096 x 768 x 3072 69.0 (+20.9) / 56.0, 2048 x 512 x 2048 22.2 (+6.2) / 21.4; past it 4096 x
   // 3072 x 768 67.3 (+6.1) / 87.9.
   UmmaCutPlan best;
   if (!exact_b && groups > 16) return best;
