@@ -462,6 +462,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
     PlanShadows(program, begin, std::min(end, program.size()));
     PlanBiasFusions(program, begin, std::min(end, program.size()));
     PlanActFusions(program, begin, std::min(end, program.size()));
+    PlanExactEpilogues(program, begin, std::min(end, program.size()));
     PlanAttentionPacks(program, begin, std::min(end, program.size()));
     PlanProductGroups(program, begin, std::min(end, program.size()));
   };
@@ -574,6 +575,7 @@ void CudaBackend::EndRange() {
   act_fusion_.clear();
   loss_fusion_.clear();
   add_fusion_.clear();
+  exact_fusion_.clear();
   skip_add_at_ = -1;
   attn_dv_out_.clear();
   attn_dv_shadow_.clear();
@@ -1643,6 +1645,116 @@ void CudaBackend::PlanActFusions(std::span<const Instruction> program, size_t be
   }
 }
 
+void CudaBackend::PlanExactEpilogues(std::span<const Instruction> program, size_t begin, size_t end) {
+  exact_fusion_.assign(end > begin ? end - begin : 0, ExactFusion{});
+  if (!OwnOrder() || !epilogue_fusion_ || end < begin + 2 || lora_skip_.size() != end - begin) return;
+  const bool whole = step_program_ != nullptr && program.data() == step_program_;
+  const size_t ext_base = whole ? 0 : begin, ext_end = whole ? program.size() : end;
+  std::vector<Extents> ext(ext_end - ext_base);
+  for (size_t i = ext_base; i < ext_end; ++i)
+    if (!DescribeInstruction(program[i], arena_bytes_, rodata_bytes_, source_bytes_, &ext[i - ext_base]).empty()) return;
+  auto apart = [](uint64_t alo, uint64_t ahi, uint64_t blo, uint64_t bhi) { return ahi <= blo || bhi <= alo; };
+  auto unobserved = [&](uint64_t lo, uint64_t hi) {
+    for (const auto& [off, bytes] : observed_)
+      if (!apart(lo, hi, off, off + bytes)) return false;
+    return !(gather_ranks_ > 1 && !apart(lo, hi, gather_off_, gather_off_ + gather_bytes_));
+  };
+  // Is [lo, hi), which instruction `def` defines, read by nothing after instruction `last`?
+  auto dead_after = [&](size_t last, uint64_t lo, uint64_t hi, size_t def) {
+    const DeadQuery q{lo, hi, false, ~0ull, 0, 0};
+    if (whole && !unobserved(lo, hi)) {
+      std::vector<Extents> in_range(ext.begin() + static_cast<long>(begin), ext.begin() + static_cast<long>(end));
+      return DeadFrom(program, in_range, begin, end, last + 1, false, 0, q);
+    }
+    return DeadFrom(program, ext, ext_base, end, last + 1, whole, def, q);
+  };
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  for (size_t i = begin; i + 1 < end; ++i) {
+    const Instruction& g = program[i];
+    const size_t at = i - begin;
+    switch (g.opcode) {
+      case kGemmNN: case kGemmNT: case kGemmNNQ8: case kGemmNTQ8: case kGemmNNBF16: case kGemmNTBF16: break;
+      default: continue;
+    }
+    if ((g.flags & kFlagRelaxed) && relaxed_allowed_ && RefSpace(g.in[1]) != kArena) continue;   // the relaxed products' fusions
+    if (ActOf(g.flags) != kActNone || RefSpace(g.in[2]) != kArena || lora_skip_[at] != 0 || add_fusion_[at].fuse ||
+        adapter_bwd_[at].fuse || shadow_plan_[at].want)
+      continue;
+    const k::GemmArgs a = GemmArgsOf(g);
+    const bool pieces = SplitGemmOn() && umma::SplitGemmEligible(a, SplitGemmWide());
+    if (a.b_transposed && !pieces) continue;   // (the CUDA-core kernels of that form have no bias and no activation)
+    const uint64_t bytes = a.M * a.N * 4;
+    ExactFusion best, f;                   // the longest run that may be absorbed; the one looked at
+    uint64_t z = g.in[2];                  // the value so far
+    uint64_t passed[3] = {};               // outputs of the product and of what is absorbed, but for the last
+    bool done = false;
+    for (size_t j = i + 1; j < end && f.count < 3 && !done; ++j) {
+      const Instruction& n = program[j];
+      if (lora_skip_[j - begin] != 0 || shadow_plan_[j - begin].want) break;
+      uint64_t out = kNullRef;
+      if (n.opcode == kAddBias && f.count == 0 && !a.bias && n.in[0] == z && n.out[0] == a.M && n.out[1] == a.N) {
+        f.bias_ref = n.in[1];
+        out = n.in[2];
+      } else if ((n.opcode == kReluFwd || (pieces && (n.opcode == kGeluFwd || n.opcode == kSiluFwd))) && n.in[0] == z &&
+                 n.out[0] == a.M * a.N) {
+        f.act = n.opcode == kReluFwd ? kActRelu : n.opcode == kGeluFwd ? kActGelu : kActSilu;
+        out = n.in[1];
+        done = true;
+      } else if (n.opcode == kAddEW && pieces && !a.addend && n.out[0] == a.M * a.N && (n.in[0] == z) != (n.in[1] == z)) {
+        f.x_ref = n.in[0] == z ? n.in[1] : n.in[0];
+        out = n.in[2];
+        done = true;
+      }
+      if (out == kNullRef || RefSpace(out) != kArena) break;
+      passed[f.count] = z;
+      f.out_ref = out;
+      ++f.count;
+      z = out;
+      // What the kernel reads must outlive what it now writes: the operands and the bias apart from the result, an added tensor
+      // apart from it or in its very place, and from the values that are not made.
+      const uint64_t o_lo = RefOffset(out), o_hi = o_lo + bytes;
+      bool ok = aligned(Wr(out)) && (f.bias_ref == kNullRef || aligned(Rd(f.bias_ref)));
+      auto keeps = [&](uint64_t ref, uint64_t n_bytes, bool in_place) {
+        if (ref == kNullRef || RefSpace(ref) != kArena) return true;
+        const uint64_t lo = RefOffset(ref);
+        return apart(lo, lo + n_bytes, o_lo, o_hi) || (in_place && lo == o_lo);
+      };
+      ok = ok && keeps(g.in[0], a.M * a.K * 4, false) && keeps(g.in[1], a.K * a.N * 4, false) && keeps(f.bias_ref, a.N * 4, false);
+      if (g.flags & kFlagGemmAddend) ok = ok && keeps(g.in[3], bytes, true);
+      else if (g.flags & kFlagEpilogueBias) ok = ok && keeps(g.in[3], a.N * 4, false);
+      if (f.x_ref != kNullRef) {
+        ok = ok && RefSpace(f.x_ref) == kArena && aligned(Rd(f.x_ref)) && keeps(f.x_ref, bytes, true);
+        for (uint32_t p = 0; p < f.count && ok; ++p)
+          ok = apart(RefOffset(f.x_ref), RefOffset(f.x_ref) + bytes, RefOffset(passed[p]), RefOffset(passed[p]) + bytes);
+      }
+      // Every value before the last is read by the next instruction alone; its place is the result's or apart from it.
+      for (uint32_t p = 0; p < f.count && ok; ++p) {
+        const uint64_t lo = RefOffset(passed[p]);
+        if (lo == o_lo) continue;
+        ok = apart(lo, lo + bytes, o_lo, o_hi) && dead_after(j, lo, lo + bytes, i + p);
+        // ... and nobody's bias, which a later value's place must not be either.
+        ok = ok && (f.bias_ref == kNullRef || RefSpace(f.bias_ref) != kArena ||
+                    apart(lo, lo + bytes, RefOffset(f.bias_ref), RefOffset(f.bias_ref) + a.N * 4));
+      }
+      if (!ok) continue;   // (with what follows it may be: the result then lies elsewhere)
+      for (uint32_t p = 1; p < f.count; ++p) f.unwritten[p - 1] = RefOffset(passed[p]) != o_lo;
+      f.unwritten[f.count - 1] = false;
+      f.z_lo = f.z_hi = 0;
+      if (RefOffset(passed[0]) != o_lo) { f.z_lo = RefOffset(passed[0]); f.z_hi = f.z_lo + bytes; }
+      best = f;
+    }
+    if (best.count > 0) exact_fusion_[at] = best;
+  }
+}
+
+// The product's kernel has done what follows it.
+void CudaBackend::AbsorbExact(const ExactFusion& f, uint64_t elems) {
+  for (uint32_t j = 0; j < f.count; ++j) lora_skip_[range_index_ + 1 + j] = f.unwritten[j] ? 2 : 1;
+  counters_.fused_dispatches += f.count;
+  umma::InvalidateRange(&umma_->ctx, RefOffset(f.out_ref), elems * 4);
+  if (f.z_hi > f.z_lo) pending_elided_.push_back({f.z_lo, f.z_hi});
+}
+
 void CudaBackend::PlanProductGroups(std::span<const Instruction> program, size_t begin, size_t end) {
   product_group_.assign(end > begin ? end - begin : 0, ProductGroup{});
   if (coherence_ == Coherence::kStrict || !relaxed_allowed_ || !epilogue_fusion_ || !product_groups_ || end < begin + 3) return;
@@ -2193,6 +2305,19 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     ++counters_.kernel_launches;
     return {};
   }
+  // What follows the product, in its epilogue.
+  const ExactFusion* xf = range_index_ < exact_fusion_.size() && exact_fusion_[range_index_].count > 0
+                              ? &exact_fusion_[range_index_] : nullptr;
+  const k::GemmArgs alone = a;
+  if (xf) {
+    if (xf->bias_ref != kNullRef) a.bias = Rd(xf->bias_ref);
+    a.act = xf->act;
+    if (xf->x_ref != kNullRef) {
+      a.addend = Rd(xf->x_ref);
+      a.addend_after_bias = true;
+    }
+    a.C = Wr(xf->out_ref);
+  }
   // Exact f32 products: bf16 pieces on the tensor cores where the bits are not observed.
   if (SplitGemmOn() && ins.opcode != kGemmAccNN && umma::SplitGemmEligible(a, SplitGemmWide())) {
     int launches = 0;
@@ -2203,8 +2328,14 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
     if (launches > 0) {
       counters_.kernel_launches += launches;
       ++counters_.split_executions;
+      if (xf) AbsorbExact(*xf, a.M * a.N);
       return {};
     }
+  }
+  // (The CUDA-core kernels add before the bias, and their GELU and SiLU are the CPU's, not the elementwise kernels' expressions.)
+  if (xf && (xf->x_ref != kNullRef || a.b_transposed || xf->act == kActGelu || xf->act == kActSilu)) {
+    a = alone;
+    xf = nullptr;
   }
   // Small and narrow products likewise, but for the rank-r expand product of many rows: that one is a stream, and a
   // following add may ride it.  A forward layer of short reduction takes the kernel in the reference's order of
@@ -2219,6 +2350,7 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
   if (OwnOrder() && !expand && !streamed && !short_layer && !a.accumulate &&
       k::FastGemm(a, stream_)) {
     ++counters_.kernel_launches;
+    if (xf) AbsorbExact(*xf, a.M * a.N);
     return {};
   }
   // The split-K scratch is sized per range (BeginRange); an instruction executed
@@ -2235,6 +2367,7 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
   a.contract_fma = coherence_ == Coherence::kLazy && adapter_fma_;
   const bool tail_done = k::GemmExact(a, stream_);
   ++counters_.kernel_launches;
+  if (xf) AbsorbExact(*xf, a.M * a.N);
   if (tail && tail_done) {
     ++counters_.fused_dispatches;
     skip_add_at_ = static_cast<int64_t>(tail->add_index);

@@ -373,6 +373,19 @@ class CudaBackend {
   };
   std::vector<AddFusion> add_fusion_;   // per range position (of the GEMM)
 
+  // What directly follows an exact product and its kernel's epilogue can do: a kAddBias, and after it an activation or, in the
+  // piece products, a kAddEW, each on the result of the one before, which nothing else reads.
+  struct ExactFusion {
+    uint32_t count = 0;            // instructions absorbed
+    uint64_t bias_ref = kNullRef, x_ref = kNullRef, out_ref = kNullRef;
+    Act act = kActNone;
+    bool unwritten[3] = {};        // whether absorbed instruction j's own output stays unwritten
+    uint64_t z_lo = 0, z_hi = 0;   // the product's own range where that does
+  };
+  std::vector<ExactFusion> exact_fusion_;   // per range position (of the product)
+  void PlanExactEpilogues(std::span<const Instruction> program, size_t begin, size_t end);
+  void AbsorbExact(const ExactFusion& f, uint64_t elems);
+
   // kAttnDKTiled directly followed by kAttnDVTiled on the same operands (relaxed,
   // head width 64): one kernel walks the queries once for both.  Per range
   // position of the dK instruction: the dV output reference, or kNullRef.

@@ -357,20 +357,55 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
     for (uint32_t p = 0; p < splits; ++p)
       remake = remake || (splits == 1 ? bars->nonfinite : LoadClusterU32(MapToCta(SmemAddr(const_cast<uint32_t*>(&bars->nonfinite)), p))) != 0;
     const bool ragged = (ep.N & 3u) != 0, plain = IsPlainStore(ep);
-    for (uint32_t i = wt; i < rows * kChunks; i += Sh::kWorkThreads) {
-      const uint32_t lr = r0 + i / kChunks, chunk = i % kChunks, row = m0 + lr, n = n0 + chunk * 4;
-      if (row >= ep.M || n >= ep.N) continue;
-      const float4 acc = element(lr, chunk);
-      if (remake) { StoreRemade(ep, row, n, acc); continue; }
-      if (ragged) { EpilogueStoreRagged(ep, row, n, acc, false); continue; }
-      float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
-      if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
-      const size_t at = static_cast<size_t>(row) * ep.N + n;
-      if (plain) {
-        EpilogueStorePlain(ep, at, acc, scale);
-      } else {
-        const float4 bias = ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        EpilogueStore(ep, at, n, acc, scale, bias);
+    const bool sum_only = ep.addend != nullptr && ep.act == kActNone && ep.pack_dst == nullptr && ep.fuse_mode == kFuseNone;
+    if (remake || ragged || !(plain || sum_only)) {
+#pragma unroll 1
+      for (uint32_t i = wt; i < rows * kChunks; i += Sh::kWorkThreads) {
+        const uint32_t lr = r0 + i / kChunks, chunk = i % kChunks, row = m0 + lr, n = n0 + chunk * 4;
+        if (row >= ep.M || n >= ep.N) continue;
+        const float4 acc = element(lr, chunk);
+        if (remake) { StoreRemade(ep, row, n, acc); continue; }
+        if (ragged) { EpilogueStoreRagged(ep, row, n, acc, false); continue; }
+        float4 scale = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha), bias = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ep.col_scale) scale = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n));
+        if (ep.bias) bias = __ldg(reinterpret_cast<const float4*>(ep.bias + n));
+        EpilogueStore(ep, static_cast<size_t>(row) * ep.N + n, n, acc, scale, bias);
+      }
+    } else {   // the frequent forms: a few elements per thread at a time, what they need of global memory asked for first
+      constexpr uint32_t kUnroll = kTN > 128 ? 2 : 4;
+      for (uint32_t i0 = wt; i0 < rows * kChunks; i0 += Sh::kWorkThreads * kUnroll) {
+        float4 side[kUnroll], scale[kUnroll];
+        auto there = [&](uint32_t u, uint32_t* lr, uint32_t* chunk) {
+          const uint32_t i = i0 + u * Sh::kWorkThreads;
+          *lr = r0 + i / kChunks;
+          *chunk = i % kChunks;
+          return i < rows * kChunks && m0 + *lr < ep.M && n0 + *chunk * 4 < ep.N;
+        };
+#pragma unroll
+        for (uint32_t u = 0; u < kUnroll; ++u) {
+          uint32_t lr, chunk;
+          scale[u] = make_float4(ep.alpha, ep.alpha, ep.alpha, ep.alpha);
+          if (!there(u, &lr, &chunk)) continue;
+          if (ep.col_scale) scale[u] = __ldg(reinterpret_cast<const float4*>(ep.col_scale + n0 + chunk * 4));
+          if (!plain) side[u] = __ldg(reinterpret_cast<const float4*>(ep.addend + static_cast<size_t>(m0 + lr) * ep.N + n0 + chunk * 4));
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kUnroll; ++u) {
+          uint32_t lr, chunk;
+          if (!there(u, &lr, &chunk)) continue;
+          const uint32_t n = n0 + chunk * 4;
+          const float4 acc = element(lr, chunk), d = side[u];
+          float4 v = make_float4(acc.x * scale[u].x, acc.y * scale[u].y, acc.z * scale[u].z, acc.w * scale[u].w);
+          if (!plain) {
+            if (!ep.addend_last) v = make_float4(d.x + v.x, d.y + v.y, d.z + v.z, d.w + v.w);
+            if (ep.bias) {
+              const float4 b = __ldg(reinterpret_cast<const float4*>(ep.bias + n));
+              v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+            }
+            if (ep.addend_last) v = make_float4(d.x + v.x, d.y + v.y, d.z + v.z, d.w + v.w);
+          }
+          *reinterpret_cast<float4*>(ep.C + static_cast<size_t>(m0 + lr) * ep.N + n) = v;
+        }
       }
     }
   }

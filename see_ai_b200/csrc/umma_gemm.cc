@@ -618,6 +618,7 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   ep.addend = a.addend;
   ep.bias = a.bias;
   ep.col_scale = a.b_col_scale;
+  ep.addend_last = a.addend_after_bias ? 1 : 0;
   ep.alpha = a.alpha;   // (the exact kernels fold alpha into A or the finished dot; here it scales the tile)
   ep.act = static_cast<int>(a.act);
   ep.M = static_cast<uint32_t>(a.M);
