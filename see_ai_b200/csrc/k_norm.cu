@@ -147,7 +147,7 @@ LayerNormFwdVecKernel(const float* __restrict__ x, const float* __restrict__ gam
   }
 }
 
-template <int V>
+template <int V, bool kAdd>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 LayerNormBwdVecKernel(const float* __restrict__ dy, const float* __restrict__ x,
                       const float* __restrict__ gamma, const float* __restrict__ mean,
@@ -163,12 +163,24 @@ LayerNormBwdVecKernel(const float* __restrict__ dy, const float* __restrict__ x,
   const float row_mean = mean[r], inv_sigma = rstd[r];
   float unit[V][4], g[V][4];
   double acc_g = 0.0, acc_gu = 0.0;
+  // Everything the row needs of memory is asked for at once, an absorbed add's other operand too (behind the row's sums it was
+  // a round trip of its own: 32768 x 768 83.9 / 66.9 us for 403 MB, 4096 x 768 7.5 / 5.9).
+  float4 xv[V], dv[V], av[kAdd ? V : 1];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    xv[i] = xr[lane + 32 * i];
+    dv[i] = dyr[lane + 32 * i];
+  }
+  if constexpr (kAdd) {
+    const float4* adr = reinterpret_cast<const float4*>(addend + r * cols);
+#pragma unroll
+    for (int i = 0; i < V; ++i) av[i] = adr[lane + 32 * i];
+  }
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     const int c4 = lane + 32 * i;
-    const float4 xv = xr[c4], dv = dyr[c4];
     const float4 gm = __ldg(reinterpret_cast<const float4*>(gamma) + c4);
-    const float xe[4] = {xv.x, xv.y, xv.z, xv.w}, de[4] = {dv.x, dv.y, dv.z, dv.w},
+    const float xe[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w}, de[4] = {dv[i].x, dv[i].y, dv[i].z, dv[i].w},
                 ge[4] = {gm.x, gm.y, gm.z, gm.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -183,15 +195,12 @@ LayerNormBwdVecKernel(const float* __restrict__ dy, const float* __restrict__ x,
   const float avg_g = static_cast<float>(acc_g) * per_col;
   const float avg_gu = static_cast<float>(acc_gu) * per_col;
   float4* dxr = reinterpret_cast<float4*>(dx + r * cols);
-  const float4* adr = addend ? reinterpret_cast<const float4*>(addend + r * cols) : nullptr;
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     float4 v = make_float4(inv_sigma * (g[i][0] - avg_g - unit[i][0] * avg_gu), inv_sigma * (g[i][1] - avg_g - unit[i][1] * avg_gu),
                            inv_sigma * (g[i][2] - avg_g - unit[i][2] * avg_gu), inv_sigma * (g[i][3] - avg_g - unit[i][3] * avg_gu));
-    if (adr) {   // an absorbed kAddEW: the sum it would have written (dx may alias the addend)
-      const float4 a = adr[lane + 32 * i];
-      v = make_float4(a.x + v.x, a.y + v.y, a.z + v.z, a.w + v.w);
-    }
+    // an absorbed kAddEW: the sum it would have written (dx may alias the addend)
+    if constexpr (kAdd) v = make_float4(av[i].x + v.x, av[i].y + v.y, av[i].z + v.z, av[i].w + v.w);
     dxr[lane + 32 * i] = v;
     if (sh.dst) ShadowStore4(sh, r * (cols / 4) + lane + 32 * i, static_cast<uint32_t>((lane + 32 * i) * 4), v);
   }
@@ -279,7 +288,8 @@ int LayerNormBwd(const float* dy, const float* x, const float* gamma, const floa
     const Shadow sh = fused && ShadowUsable(sum_shadow, sum_out, rows * cols) && sum_shadow->cols == cols
                           ? *sum_shadow : Shadow{};
 #define SEE_LN_BWD(V) \
-    case V: Next(LayerNormBwdVecKernel<V>, blocks, kWarpsPerBlock * 32, 0, s)(dy, x, gamma, mean, rstd, dx, rows, addend, sh); break
+    case V: Next(addend ? LayerNormBwdVecKernel<V, true> : LayerNormBwdVecKernel<V, false>, blocks, kWarpsPerBlock * 32, 0, s)( \
+        dy, x, gamma, mean, rstd, dx, rows, addend, sh); break
     switch (cols / 128) {
       SEE_LN_BWD(1); SEE_LN_BWD(2); SEE_LN_BWD(3); SEE_LN_BWD(4);
       SEE_LN_BWD(5); SEE_LN_BWD(6); SEE_LN_BWD(7); SEE_LN_BWD(8);
