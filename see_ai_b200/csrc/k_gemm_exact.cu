@@ -383,28 +383,65 @@ __global__ void __launch_bounds__(kThreads) MergeDeltasKernel(const __grid_const
 // With fewer 64 x 64 (or skinny) tiles than SMs the kernels above are a serial chain of global loads: K / 16 steps of
 // about 1.4 us in one or two blocks.  Here a block owns 16 R x 16 R outputs, R x R per thread, so that there are blocks
 // to go round, and takes K 128 at a time with the next 128 already on their way in registers while these are
-// multiplied.  The same operations per output in the same order (57 x 8 x 784: 81.5 -> 11.2 us; 57 x 128 x 784: 76 -> 12.5 us).
+// multiplied.  The same operations per output in the same order (57 x 8 x 784: 81.5 -> 9.9 us; 57 x 128 x 784: 76 -> 10.3 us).
 constexpr int kFlatK = 128;
 template <bool TA, bool TB, typename BT, int R>
 struct FlatLoader {
   static constexpr int T = 16 * R, kPer = T * kFlatK / kThreads;   // elements per thread and operand
   float a[kPer], b[kPer];
-  // Which (row, k) element i of this thread is: lanes along the operand's contiguous axis.
+  // Where an operand's first element of this thread lies, how far its elements and the blocks of K are apart: lanes along
+  // the operand's contiguous axis.  (Addresses made anew for every element, 64-bit products and two bounds each, took as long as the
+  // arithmetic: 57 x 128 x 784 11.4 / 10.3 us, transposed 15.7 / 10.8 and 15.4 / 10.2.)
+  const float* pa;
+  const BT* pb;
+  size_t a_step, b_step, a_chunk, b_chunk;
+  static constexpr int kRowStep = kThreads / kFlatK, kKStep = kThreads / T;
+  // Which (row, k) element i of this thread is.
   static __device__ __forceinline__ void At(int i, bool k_contiguous, int* row, int* k) {
-    const int idx = static_cast<int>(threadIdx.x) + i * kThreads;
-    if (k_contiguous) { *row = idx / kFlatK; *k = idx % kFlatK; }
-    else { *row = idx % T; *k = idx / T; }
+    const int t = static_cast<int>(threadIdx.x);
+    if (k_contiguous) { *row = t / kFlatK + i * kRowStep; *k = t % kFlatK; }
+    else { *row = t % T; *k = t / T + i * kKStep; }
   }
+  __device__ __forceinline__ FlatLoader(const Params& p, size_t m0, size_t n0) {
+    int r, k;
+    At(0, !TA, &r, &k);
+    pa = TA ? p.A + k * p.M + m0 + r : p.A + (m0 + r) * p.K + k;
+    a_step = TA ? kKStep * p.M : kRowStep * p.K;
+    a_chunk = TA ? kFlatK * p.M : kFlatK;
+    At(0, TB, &r, &k);
+    pb = static_cast<const BT*>(p.B) + (TB ? (n0 + r) * p.K + k : k * p.N + n0 + r);
+    b_step = TB ? kRowStep * p.K : kKStep * p.N;
+    b_chunk = TB ? kFlatK : kFlatK * p.N;
+  }
+  // The block at k0, which follows the one loaded before.
   __device__ __forceinline__ void Load(const Params& p, size_t m0, size_t n0, size_t k0) {
+    auto clamp = [](size_t left) { return left < static_cast<size_t>(kFlatK) ? static_cast<int>(left) : kFlatK; };
+    const int left = clamp(p.K - k0), rows = clamp(p.M - m0), cols = clamp(p.N - n0);
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       int r, k;
       At(i, !TA, &r, &k);
-      a[i] = LoadA<TA>(p, m0 + r, k0 + k);
-      if (p.a_k_scale && k0 + k < p.K) a[i] = a[i] * p.a_k_scale[k0 + k];
+      a[i] = r < rows && k < left ? pa[i * a_step] : 0.0f;
       At(i, TB, &r, &k);
-      b[i] = LoadB<TB, BT>(p, k0 + k, n0 + r);
-      if (p.b_col_scale && n0 + r < p.N) b[i] = b[i] * p.b_col_scale[n0 + r];
+      b[i] = r < cols && k < left ? Widen<BT>(pb[i * b_step]) : 0.0f;
+    }
+    pa += a_chunk;
+    pb += b_chunk;
+    if (p.a_k_scale) {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        int r, k;
+        At(i, !TA, &r, &k);
+        if (k < left) a[i] = a[i] * p.a_k_scale[k0 + k];
+      }
+    }
+    if (p.b_col_scale) {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        int r, k;
+        At(i, TB, &r, &k);
+        if (r < cols) b[i] = b[i] * p.b_col_scale[n0 + r];
+      }
     }
   }
   // As [row][k] (a row's quads are 16-byte reads), Bs [row][k] likewise.
@@ -440,7 +477,7 @@ __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
       if (!kLane && p.accumulate && m < p.M && n < p.N) c[i][j][0] = p.C[m * p.N + n];
     }
   const float alpha_a = kLane ? 1.0f : p.alpha;   // (x * 1 == x)
-  FlatLoader<TA, TB, BT, R> next;
+  FlatLoader<TA, TB, BT, R> next(p, m0, n0);
   next.Load(p, m0, n0, 0);
   for (size_t k0 = 0; k0 < p.K; k0 += kFlatK) {
     next.Store(As, Bs, alpha_a);
@@ -448,7 +485,7 @@ __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
     if (k0 + kFlatK < p.K) next.Load(p, m0, n0, k0 + kFlatK);
     const int kmax = p.K - k0 < static_cast<size_t>(kFlatK) ? static_cast<int>(p.K - k0) : kFlatK;
     int k = 0;
-    for (; k + 4 <= kmax; k += 4) {
+    auto quad = [&](int k) {
       float4 a[R], b[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4*>(&As[ty + 16 * i][k]);
@@ -478,6 +515,12 @@ __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
             c[i][j][0] = c[i][j][0] + t;
           }
         }
+    };
+    if (kmax == kFlatK) {   // (quads' products do not wait for one another: only the sums are a chain)
+#pragma unroll 8
+      for (; k < kFlatK; k += 4) quad(k);
+    } else {
+      for (; k + 4 <= kmax; k += 4) quad(k);
     }
     for (; k < kmax; ++k)   // the K % 4 tail, one term at a time
 #pragma unroll
