@@ -383,11 +383,13 @@ __global__ void __launch_bounds__(kThreads) MergeDeltasKernel(const __grid_const
 // With fewer 64 x 64 (or skinny) tiles than SMs the kernels above are a serial chain of global loads: K / 16 steps of
 // about 1.4 us in one or two blocks.  Here a block owns 16 R x 16 R outputs, R x R per thread, so that there are blocks
 // to go round, and takes K 128 at a time with the next 128 already on their way in registers while these are
-// multiplied.  The same operations per output in the same order (57 x 8 x 784: 81.5 -> 9.9 us; 57 x 128 x 784: 76 -> 10.3 us).
+// multiplied.  The same operations per output in the same order (57 x 8 x 784: 81.5 -> 8.1 us; 57 x 128 x 784: 76 -> 8.4 us).
 constexpr int kFlatK = 128;
-template <bool TA, bool TB, typename BT, int R>
+// T x T outputs of a block, R x R of a thread.
+template <int T> struct FlatShape { static constexpr int R = T > 16 ? 2 : 1, kSide = T / R, kThreads = kSide * kSide; };
+template <bool TA, bool TB, typename BT, int T>
 struct FlatLoader {
-  static constexpr int T = 16 * R, kPer = T * kFlatK / kThreads;   // elements per thread and operand
+  static constexpr int kThreads = FlatShape<T>::kThreads, kPer = T * kFlatK / kThreads;   // elements per thread and operand
   float a[kPer], b[kPer];
   // Where an operand's first element of this thread lies, how far its elements and the blocks of K are apart: lanes along
   // the operand's contiguous axis.  (Addresses made anew for every element, 64-bit products and two bounds each, took as long as the
@@ -395,12 +397,17 @@ struct FlatLoader {
   const float* pa;
   const BT* pb;
   size_t a_step, b_step, a_chunk, b_chunk;
-  static constexpr int kRowStep = kThreads / kFlatK, kKStep = kThreads / T;
+  static constexpr int kKStep = kThreads / T;                                   // (k apart, along rows)
+  static constexpr int kLanes = kThreads < kFlatK ? kThreads : kFlatK, kRun = kFlatK / kLanes, kRowStep = kThreads / kLanes;
   // Which (row, k) element i of this thread is.
   static __device__ __forceinline__ void At(int i, bool k_contiguous, int* row, int* k) {
     const int t = static_cast<int>(threadIdx.x);
-    if (k_contiguous) { *row = t / kFlatK + i * kRowStep; *k = t % kFlatK; }
+    if (k_contiguous) { *row = t / kLanes + i / kRun * kRowStep; *k = t % kLanes + i % kRun * kLanes; }
     else { *row = t % T; *k = t / T + i * kKStep; }
+  }
+  // ... and how far from element 0.
+  static __device__ __forceinline__ size_t Distance(int i, bool k_contiguous, size_t step) {
+    return k_contiguous ? i / kRun * step + i % kRun * kLanes : i * step;
   }
   __device__ __forceinline__ FlatLoader(const Params& p, size_t m0, size_t n0) {
     int r, k;
@@ -421,9 +428,9 @@ struct FlatLoader {
     for (int i = 0; i < kPer; ++i) {
       int r, k;
       At(i, !TA, &r, &k);
-      a[i] = r < rows && k < left ? pa[i * a_step] : 0.0f;
+      a[i] = r < rows && k < left ? pa[Distance(i, !TA, a_step)] : 0.0f;
       At(i, TB, &r, &k);
-      b[i] = r < cols && k < left ? Widen<BT>(pb[i * b_step]) : 0.0f;
+      b[i] = r < cols && k < left ? Widen<BT>(pb[Distance(i, TB, b_step)]) : 0.0f;
     }
     pa += a_chunk;
     pb += b_chunk;
@@ -458,13 +465,13 @@ struct FlatLoader {
 };
 
 // Lane order when kLane, quad order otherwise.
-template <bool kLane, bool TA, bool TB, typename BT, int R>
-__global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
+template <bool kLane, bool TA, bool TB, typename BT, int T>
+__global__ void __launch_bounds__(FlatShape<T>::kThreads) GemmFlatKernel(Params p) {
   AwaitPrevious();
-  constexpr int T = 16 * R;
+  constexpr int R = FlatShape<T>::R, kSide = FlatShape<T>::kSide;
   __shared__ __align__(16) float As[T][kFlatK + 4];
   __shared__ __align__(16) float Bs[T][kFlatK + 4];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // outputs (ty + 16 i, tx + 16 j)
+  const int tx = threadIdx.x % kSide, ty = threadIdx.x / kSide;   // outputs (ty + kSide i, tx + kSide j)
   const size_t m0 = static_cast<size_t>(blockIdx.y) * T, n0 = static_cast<size_t>(blockIdx.x) * T;
   float c[R][R][kLane ? 8 : 1];
 #pragma unroll
@@ -473,11 +480,11 @@ __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
     for (int j = 0; j < R; ++j) {
 #pragma unroll
       for (int l = 0; l < (kLane ? 8 : 1); ++l) c[i][j][l] = 0.0f;
-      const size_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      const size_t m = m0 + ty + kSide * i, n = n0 + tx + kSide * j;
       if (!kLane && p.accumulate && m < p.M && n < p.N) c[i][j][0] = p.C[m * p.N + n];
     }
   const float alpha_a = kLane ? 1.0f : p.alpha;   // (x * 1 == x)
-  FlatLoader<TA, TB, BT, R> next(p, m0, n0);
+  FlatLoader<TA, TB, BT, T> next(p, m0, n0);
   next.Load(p, m0, n0, 0);
   for (size_t k0 = 0; k0 < p.K; k0 += kFlatK) {
     next.Store(As, Bs, alpha_a);
@@ -488,9 +495,9 @@ __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
     auto quad = [&](int k) {
       float4 a[R], b[R];
 #pragma unroll
-      for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4*>(&As[ty + 16 * i][k]);
+      for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const float4*>(&As[ty + kSide * i][k]);
 #pragma unroll
-      for (int j = 0; j < R; ++j) b[j] = *reinterpret_cast<const float4*>(&Bs[tx + 16 * j][k]);
+      for (int j = 0; j < R; ++j) b[j] = *reinterpret_cast<const float4*>(&Bs[tx + kSide * j][k]);
 #pragma unroll
       for (int i = 0; i < R; ++i)
 #pragma unroll
@@ -527,7 +534,7 @@ __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
       for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < R; ++j) {
-          const float x = As[ty + 16 * i][k] * Bs[tx + 16 * j][k];
+          const float x = As[ty + kSide * i][k] * Bs[tx + kSide * j][k];
 #pragma unroll
           for (int l = 0; l < (kLane ? 8 : 1); ++l)
             if (!kLane || l == (k & 7)) c[i][j][l] = c[i][j][l] + x;
@@ -538,7 +545,7 @@ __global__ void __launch_bounds__(kThreads) GemmFlatKernel(Params p) {
   for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      const size_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      const size_t m = m0 + ty + kSide * i, n = n0 + tx + kSide * j;
       if (m >= p.M || n >= p.N) continue;
       float v = c[i][j][0];
       if (kLane) {
@@ -566,13 +573,17 @@ size_t LaneTiles(size_t M, size_t N) {
 }
 
 // The flat kernel where the tile kernels would leave SMs idle: 32 x 32 outputs per block if that still makes a block
-// per SM, else 16 x 16.
+// per SM, else 16 x 16, and 8 x 8 where those are few: a block is bound by its own shared memory and chains of sums (57 x 128 x 784
+// 10.1 / 8.4 us, 32 x 8 x 1024 12.1 / 9.5; of a transposed A, whose rows of eight are half a sector, 10.2 / 11.3: 16 x 16).
 template <bool kLane, bool TA, bool TB, typename BT>
 void LaunchFlat(const Params& p, cudaStream_t s) {
-  if (static_cast<size_t>(Blocks(p.M, 32)) * Blocks(p.N, 32) >= 148)
-    Next(GemmFlatKernel<kLane, TA, TB, BT, 2>, dim3(Blocks(p.N, 32), Blocks(p.M, 32)), kThreads, 0, s)(p);
-  else
-    Next(GemmFlatKernel<kLane, TA, TB, BT, 1>, dim3(Blocks(p.N, 16), Blocks(p.M, 16)), kThreads, 0, s)(p);
+  auto blocks = [&](size_t t) { return static_cast<size_t>(Blocks(p.M, t)) * Blocks(p.N, t); };
+  if (blocks(32) >= 148)
+    Next(GemmFlatKernel<kLane, TA, TB, BT, 32>, dim3(Blocks(p.N, 32), Blocks(p.M, 32)), FlatShape<32>::kThreads, 0, s)(p);
+  else if (TA || blocks(16) > 37)
+    Next(GemmFlatKernel<kLane, TA, TB, BT, 16>, dim3(Blocks(p.N, 16), Blocks(p.M, 16)), FlatShape<16>::kThreads, 0, s)(p);
+  else if constexpr (!TA)
+    Next(GemmFlatKernel<kLane, TA, TB, BT, 8>, dim3(Blocks(p.N, 8), Blocks(p.M, 8)), FlatShape<8>::kThreads, 0, s)(p);
 }
 
 template <bool TA, typename BT>
