@@ -357,7 +357,7 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
     for (uint32_t p = 0; p < splits; ++p)
       remake = remake || (splits == 1 ? bars->nonfinite : LoadClusterU32(MapToCta(SmemAddr(const_cast<uint32_t*>(&bars->nonfinite)), p))) != 0;
     const bool ragged = (ep.N & 3u) != 0, plain = IsPlainStore(ep);
-    const bool sum_only = ep.addend != nullptr && ep.act == kActNone && ep.pack_dst == nullptr && ep.fuse_mode == kFuseNone;
+    const bool sum_only = IsSum(ep);
     if (remake || ragged || !(plain || sum_only)) {
 #pragma unroll 1
       for (uint32_t i = wt; i < rows * kChunks; i += Sh::kWorkThreads) {

@@ -411,6 +411,18 @@ UmmaGemmTileKernel(const __grid_constant__ UmmaMaps maps, const __grid_constant_
       each(NoSide{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4&) {
         EpilogueStoreBiasGelu(ep, at, acc, scale, bias_at(n), one);
       });
+    } else if (kSeg && IsBiasStored(ep, kActNone)) {
+      each(NoSide{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4&) {
+        EpilogueStoreBias<kActNone>(ep, at, acc, scale, bias_at(n));
+      });
+    } else if (kSeg && IsBiasStored(ep, kActGelu)) {
+      each(NoSide{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4&) {
+        EpilogueStoreBias<kActGelu>(ep, at, acc, scale, bias_at(n));
+      });
+    } else if (kSeg && IsSum(ep)) {
+      each(Side{}, [&](size_t at, uint32_t, uint32_t n, const float4& acc, const float4& scale, const float4& side) {
+        EpilogueStoreSum(ep, at, acc, scale, bias_at(n), side);
+      });
     } else if (IsGeluGradOnly(ep) && !ep.shadow_k_scale) {
       each(Side{}, [&](size_t at, uint32_t, uint32_t, const float4& acc, const float4& scale, const float4& side) {
         EpilogueStoreGeluGrad(ep, at, acc, scale, one, side);
@@ -721,6 +733,8 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
       [[maybe_unused]] const bool bias_gelu_only = IsBiasGeluOnly(ep);
       [[maybe_unused]] const bool copy_only = IsCopyOnly(ep);
       [[maybe_unused]] const bool plain_store = IsPlainStore(ep);
+      [[maybe_unused]] const bool bias_stored = kSeg && IsBiasStored(ep, kActNone), bias_gelu_stored = kSeg && IsBiasStored(ep, kActGelu);
+      [[maybe_unused]] const bool sum_stored = kSeg && IsSum(ep);
       const bool side_by_side = kSeveral && ep.products > 1;
       [[maybe_unused]] const float alpha = side_by_side ? ep.product[product].alpha : ep.alpha;
       [[maybe_unused]] const float* col_scale = side_by_side ? ep.product[product].col_scale : ep.col_scale;
@@ -821,6 +835,17 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
             float4 kscale = make_float4(1.f, 1.f, 1.f, 1.f);   // the consumer's per-column factor (x * 1 == x)
             if (ep.fuse_mode != kFuseNone && ep.shadow_k_scale)
               kscale = __ldg(reinterpret_cast<const float4*>(ep.shadow_k_scale + n));
+            if (kSeg && sum_stored) {   // two addends in flight at a time: more do not fit the registers
+  #pragma unroll 1
+              for (uint32_t rr = sub; rr < rows; rr += 2 * kRowsPerInstr) {
+                const bool both = rr + kRowsPerInstr < rows;
+                const size_t at = static_cast<size_t>(row0 + rr) * ep.N + n, next = at + static_cast<size_t>(kRowsPerInstr) * ep.N;
+                const float4 d = __ldg(reinterpret_cast<const float4*>(ep.addend + at));
+                const float4 e = __ldg(reinterpret_cast<const float4*>(ep.addend + (both ? next : at)));
+                EpilogueStoreSum(ep, at, staged(rr), scale, bias, d);
+                if (both) EpilogueStoreSum(ep, next, staged(rr + kRowsPerInstr), scale, bias, e);
+              }
+            } else
   #pragma unroll 4
             for (uint32_t rr = sub; rr < rows; rr += kRowsPerInstr) {
               const float4 acc = staged(rr);
@@ -829,6 +854,10 @@ UmmaGemmPersistentKernel(const __grid_constant__ UmmaMaps maps, const __grid_con
                 EpilogueStorePlain(ep, at, acc, scale);
               else if (copy_only)
                 EpilogueStoreCopy(pack_dst, at, acc, scale);
+              else if (kSeg && bias_stored)
+                EpilogueStoreBias<kActNone>(ep, at, acc, scale, bias);
+              else if (kSeg && bias_gelu_stored)
+                EpilogueStoreBias<kActGelu>(ep, at, acc, scale, bias);
               else if (bias_gelu_only)
                 EpilogueStoreBiasGelu(ep, at, acc, scale, bias, kscale);
               else
