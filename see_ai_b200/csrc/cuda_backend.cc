@@ -454,6 +454,7 @@ void CudaBackend::BeginRange(std::span<const Instruction> program, size_t begin,
   range_index_ = 0;
   lora_rows_tag_.valid = false;
   waiting_products_.clear();   // (an earlier range that ended in an error)
+  waiting_downs_.clear();
   umma::ReleaseProducts(&umma_->ctx);
   PlanAdamGroups(program, begin, std::min(end, program.size()));
   PlanMergeRuns(program, begin, std::min(end, program.size()));
@@ -2120,6 +2121,17 @@ k::GemmArgs CudaBackend::GemmArgsOf(const Instruction& ins) const {
   return a;
 }
 
+Status CudaBackend::LaunchDowns() {
+  if (waiting_downs_.empty()) return {};
+  int launches = 0;
+  const k::GemmArgs& d = waiting_down_;
+  const bool ok = k::LoraDowns(d.A, waiting_downs_.data(), static_cast<int>(waiting_downs_.size()), d.M, d.K, d.N, stream_, &launches);
+  waiting_downs_.clear();
+  counters_.kernel_launches += launches;
+  if (!ok) return std::unexpected("cuda: low-rank fold: the down products were refused");
+  return {};
+}
+
 Status CudaBackend::DispatchGemm(const Instruction& ins) {
   k::GemmArgs a = GemmArgsOf(ins);
   // The relaxed permission: frozen-weight products may run on the bf16 tensor
@@ -2157,13 +2169,38 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
         k::GemmArgs d = GemmArgsOf(lf->down);
         d.contract_fma = adapter_fma_;
         // (the tensor-core form of it leaves t's bf16 cut in the same launch)
-        pieces_made = adapter_fma_ && lf->down.flags == 0 && d.N == lf->r && k::LoraDownSupported(d.M, d.K, d.N) &&
-                      k::LoraDown(d.A, static_cast<const float*>(d.B), d.C, d.M, d.K, d.N, d.alpha, stream_,
-                                  LoraRows());
-        if (!pieces_made && !(OwnOrder() && k::FastGemm(d, stream_))) k::GemmExact(d, stream_);
-        ++counters_.kernel_launches;
+        const bool supported = adapter_fma_ && lf->down.flags == 0 && d.N == lf->r && k::LoraDownSupported(d.M, d.K, d.N);
+        // Members of a side-by-side group have nothing between them but what they stand for: theirs leave together before the
+        // first product does.
+        const ProductGroup* g = range_index_ < product_group_.size() && product_group_[range_index_].member
+                                    ? &product_group_[range_index_] : nullptr;
+        auto apart = [](const void* p, uint64_t n, const void* q, uint64_t m) {
+          const uintptr_t a0 = reinterpret_cast<uintptr_t>(p), b0 = reinterpret_cast<uintptr_t>(q);
+          return a0 + n * 4 <= b0 || b0 + m * 4 <= a0;
+        };
+        auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+        const uint64_t t_n = d.M * d.N, w_n = d.K * d.N;
+        bool waits = g && !g->chained && supported && apart(d.C, t_n, d.A, d.M * d.K) && apart(d.C, t_n, d.B, w_n) &&
+                     aligned(d.A) && aligned(d.B) && aligned(d.C) && aligned(LoraRows());
+        const k::GemmArgs& w = waiting_down_;
+        bool together = waits && w.A == d.A && w.M == d.M && w.K == d.K && w.N == d.N;
+        for (const k::LoraDownJob& o : waiting_downs_)
+          together = together && apart(d.C, t_n, o.out, t_n) && apart(d.C, t_n, o.A, w_n) && apart(o.out, t_n, d.B, w_n);
+        if (!together)
+          if (Status st = LaunchDowns(); !st) return st;
+        if (waits) {
+          waiting_down_ = d;
+          waiting_downs_.push_back({static_cast<const float*>(d.B), d.C, LoraRows(), d.alpha});
+          pieces_made = true;
+        } else {
+          pieces_made = supported && k::LoraDown(d.A, static_cast<const float*>(d.B), d.C, d.M, d.K, d.N, d.alpha, stream_, LoraRows());
+          if (!pieces_made && !(OwnOrder() && k::FastGemm(d, stream_))) k::GemmExact(d, stream_);
+          ++counters_.kernel_launches;
+        }
         umma::InvalidateRange(&umma_->ctx, RefOffset(lf->down.in[2]), d.M * d.N * 4);
       }
+      if (lf->kind != 1)   // (its t may be one that waits)
+        if (Status st = LaunchDowns(); !st) return st;
       if (!pieces_made && lf->kind != 1 && lora_rows_tag_.valid && lora_rows_tag_.off == RefOffset(lf->t_ref) &&
           lora_rows_tag_.M == a.M && lora_rows_tag_.r == lf->r)
         pieces_made = true;   // the adapter backward left dT's cut in the scratch
@@ -2199,6 +2236,8 @@ Status CudaBackend::DispatchGemm(const Instruction& ins) {
                                     ? &product_group_[range_index_] : nullptr;
     // (without a copy buffer of its own a product leaves as f32, by itself)
     const bool joins = group && (group->chained || (pack_rows && !a.store_c));
+    if (!joins || group->last)
+      if (Status st = LaunchDowns(); !st) return st;
     umma::PreparedProduct product;
     std::string err = umma::PrepareProduct(&umma_->ctx, a, RefSpace(ins.in[1]) == kRodata ? 1 : 2, RefOffset(ins.in[1]),
                                            RefOffset(ins.in[0]),

@@ -469,6 +469,11 @@ class CudaBackend {
   void PlanProductGroups(std::span<const Instruction> program, size_t begin, size_t end);
   std::vector<ProductGroup> product_group_;              // per range position
   std::vector<umma::PreparedProduct> waiting_products_;  // prepared, not launched
+  // The down products t = x A of those that wait side by side, not launched either: from one x, none of them writing what another
+  // touches.
+  std::vector<k::LoraDownJob> waiting_downs_;
+  k::GemmArgs waiting_down_{};   // their x and shape
+  Status LaunchDowns();
   std::vector<uint8_t> lora_skip_;           // per range position: 1 done by an earlier dispatch, 2 never runs
   std::vector<k::LoraWeight> lora_weights_;  // the range's adapter matrices (host copy of the table)
   uint32_t lora_max_n_ = 0, lora_max_kx_ = 0;

@@ -166,6 +166,12 @@ constexpr int kDownAhead = 4;   // 16-wide k blocks in flight per lane and row
 // reduction axis is cut instead: `ksplit` warps (a power of two) share a tile, each over its
 // own run of k blocks, and the tile's first warp adds their sums in warp order through
 // shared memory — a fixed order, so a given row count always gives the same bits.
+//
+// Several products of one x (an attention block's Q, K and V) share a launch where the reduction is cut, that is where the
+// prologue is most of a launch: each takes its share of the SMs, cut as it is alone (the same bits), so its tiles take more
+// trips and the prologue is paid once.  Three and one of a layer at 4096 x 768, r 16: 31.8 -> 23.6 us; at 2048 rows 26.0 -> 18.1, at
+// 18432 70 -> 66; with whole tiles to a warp there is nothing left to save (24576 rows 77 us one by one).
+constexpr int kDownTogether = 2;   // `ksplit` from which they do
 template <int K, int R>
 struct DownSmem {
   static constexpr int kStride = K + 16;   // rows 16 banks apart: a quarter warp's two rows cover all 32
@@ -174,11 +180,17 @@ struct DownSmem {
   static constexpr size_t kFloats = kWeightFloats + static_cast<size_t>(kDownThreads) * kLaneFloats;
 };
 
+struct DownJobs { LoraDownJob job[kUmmaProducts]; };   // one a row of the grid
+
 template <int K, int R, bool kSplitK>
 __global__ void __launch_bounds__(kDownThreads, 1)
-LoraDownKernel(const float* __restrict__ x, const float* __restrict__ A, float* __restrict__ out,
-               uint16_t* __restrict__ pieces, uint32_t piece_cols, size_t M, float alpha, int ksplit) {
+LoraDownKernel(const float* __restrict__ x, const __grid_constant__ DownJobs jobs, uint32_t piece_cols, size_t M, int ksplit) {
   AwaitPrevious();
+  const LoraDownJob& job = jobs.job[blockIdx.y];
+  const float* __restrict__ A = job.A;
+  float* __restrict__ out = job.out;
+  uint16_t* __restrict__ pieces = job.pieces;
+  const float alpha = job.alpha;
   using S = DownSmem<K, R>;
   extern __shared__ __align__(16) float smem[];
   uint32_t* a_hi = reinterpret_cast<uint32_t*>(smem);
@@ -563,24 +575,27 @@ int SmCount() {
 }
 
 template <int K, int R>
-bool LaunchDown(const float* x, const float* A, float* out, uint16_t* pieces, uint32_t piece_cols, size_t M,
-                float alpha, cudaStream_t s) {
+bool LaunchDown(const float* x, const LoraDownJob* jobs, int count, uint32_t piece_cols, size_t M, cudaStream_t s, int* launches) {
   static std::atomic<bool> configured[64] = {};
   const size_t smem = DownSmem<K, R>::kFloats * sizeof(float);
   static std::atomic<bool> configured_split[64] = {};
   if (!Configure(LoraDownKernel<K, R, false>, smem, configured)) return false;
   if (!Configure(LoraDownKernel<K, R, true>, smem, configured_split)) return false;
-  // One block per SM as soon as there is a tile per SM: the tiles go round the blocks first.
   const size_t tiles = (M + kTileRows - 1) / kTileRows;
   const size_t sms = static_cast<size_t>(SmCount());
-  const unsigned grid = static_cast<unsigned>(tiles < sms ? tiles : sms);
   // Warps per tile: the largest power of two that still leaves every tile a group of warps.
   int ksplit = 1;
   while (ksplit < kDownWarps && (K / 16) % (2 * ksplit) == 0 && tiles * (2 * ksplit) <= sms * kDownWarps) ksplit *= 2;
-  if (ksplit > 1)
-    Next(LoraDownKernel<K, R, true>, grid, kDownThreads, smem, s)(x, A, out, pieces, piece_cols, M, alpha, ksplit);
-  else
-    Next(LoraDownKernel<K, R, false>, grid, kDownThreads, smem, s)(x, A, out, pieces, piece_cols, M, alpha, 1);
+  const int together = ksplit >= kDownTogether ? count : 1;
+  // One block per SM as soon as there is a tile per SM: the tiles go round the blocks first.
+  const size_t room = sms / together;
+  const unsigned grid = static_cast<unsigned>(tiles < room ? tiles : room);
+  for (int j = 0; j < count; j += together, ++*launches) {
+    DownJobs d;
+    for (int u = 0; u < together; ++u) d.job[u] = jobs[j + u];
+    if (ksplit > 1) Next(LoraDownKernel<K, R, true>, dim3(grid, together), kDownThreads, smem, s)(x, d, piece_cols, M, ksplit);
+    else Next(LoraDownKernel<K, R, false>, dim3(grid, together), kDownThreads, smem, s)(x, d, piece_cols, M, 1);
+  }
   return true;
 }
 
@@ -615,12 +630,20 @@ bool LoraDownSupported(size_t M, size_t K, size_t r) {
 
 bool LoraDown(const float* x, const float* A, float* out, size_t M, size_t K, size_t r, float alpha, cudaStream_t s,
               uint16_t* pieces) {
-  if (!LoraDownSupported(M, K, r) || !Aligned16(x) || !Aligned16(A) || !Aligned16(out) || !Aligned16(pieces))
-    return false;
+  const LoraDownJob job{A, out, pieces, alpha};
+  int launches = 0;
+  return LoraDowns(x, &job, 1, M, K, r, s, &launches);
+}
+
+bool LoraDowns(const float* x, const LoraDownJob* jobs, int count, size_t M, size_t K, size_t r, cudaStream_t s, int* launches) {
+  *launches = 0;
+  if (!LoraDownSupported(M, K, r) || !Aligned16(x) || count < 1 || count > static_cast<int>(kUmmaProducts)) return false;
+  for (int j = 0; j < count; ++j)
+    if (!Aligned16(jobs[j].A) || !Aligned16(jobs[j].out) || !Aligned16(jobs[j].pieces)) return false;
   const uint32_t cols = LoraSplitColumns(static_cast<uint32_t>(r));
-  if (K == 768 && r == 16) return LaunchDown<768, 16>(x, A, out, pieces, cols, M, alpha, s);
-  if (K == 768 && r == 8) return LaunchDown<768, 8>(x, A, out, pieces, cols, M, alpha, s);
-  return LaunchDown<256, 8>(x, A, out, pieces, cols, M, alpha, s);
+  if (K == 768 && r == 16) return LaunchDown<768, 16>(x, jobs, count, cols, M, s, launches);
+  if (K == 768 && r == 8) return LaunchDown<768, 8>(x, jobs, count, cols, M, s, launches);
+  return LaunchDown<256, 8>(x, jobs, count, cols, M, s, launches);
 }
 
 void LoraFoldPartials(const LoraBackwardArgs& a, int blocks, cudaStream_t s) {

@@ -248,6 +248,9 @@ void LoraSplitWeights(const LoraWeight* table, int count, uint32_t max_n_out, ui
 bool LoraDownSupported(size_t M, size_t K, size_t r);
 bool LoraDown(const float* x, const float* A, float* out, size_t M, size_t K, size_t r, float alpha, cudaStream_t s,
               uint16_t* pieces = nullptr);
+// Up to kUmmaProducts of them from one x, the same bits: one launch where that is the shorter way.  *launches = how many it took.
+struct LoraDownJob { const float* A = nullptr; float* out = nullptr; uint16_t* pieces = nullptr; float alpha = 1.0f; };
+bool LoraDowns(const float* x, const LoraDownJob* jobs, int count, size_t M, size_t K, size_t r, cudaStream_t s, int* launches);
 // The three backward products of one adapter site in one pass over dY and x:
 // dT = alpha_dt dY B^T, dB = alpha_db t^T dY, dA = alpha_da x^T dT.  `partials`
 // holds LoraBackwardPartialFloats(N, K, r) floats of scratch.
