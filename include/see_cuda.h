@@ -113,6 +113,12 @@ int see_cuda_set_adapter_fma(see_cuda_backend* h, int enabled);
  * the keys once instead of twice.  Same quantity, another rounding (tolerance class, like every relaxed
  * attention result).  Default on; 0 keeps the two-walk kernel. */
 int see_cuda_set_attention_one_walk(see_cuda_backend* h, int enabled);
+/* Lazy coherence, where the exact attention family may have its own order of sums: its forward and
+ * dP = dO V^T on the tensor cores, operands as fixed-point digits.  1 (default): where that is estimated
+ * to be the shorter way; 2: wherever the kernel takes the geometry (heads of up to 64 features, a
+ * multiple of four); 0: never.  see_cuda_attention_slices: how many instructions ran so since creation. */
+int see_cuda_set_attention_slices(see_cuda_backend* h, int use);
+uint64_t see_cuda_attention_slices(see_cuda_backend* h);
 /* Exact products (without the relaxed permission) on the tensor cores: f32 operands
  * cut into three bf16 pieces, the six largest piece products of 64 k at a time in one
  * accumulator, the blocks of 64 added in rounded f32.  The result is as close to a

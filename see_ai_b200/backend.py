@@ -33,6 +33,7 @@ EXPORTED_SYMBOLS = [
     "see_cuda_set_profiling", "see_cuda_take_profile",
     "see_cuda_xent_forward_static", "see_cuda_static_max_rows", "see_cuda_static_last_error",
     "see_cuda_quantize_columns", "see_cuda_set_lora_fold", "see_cuda_set_product_groups", "see_cuda_set_adapter_fma", "see_cuda_set_split_gemm", "see_cuda_set_cta_pairs", "see_cuda_set_adapter_tensor_backward", "see_cuda_set_attention_one_walk",
+    "see_cuda_set_attention_slices", "see_cuda_attention_slices",
 ]
 
 
@@ -111,6 +112,9 @@ def load_library() -> ctypes.CDLL:
     lib.see_cuda_set_cta_pairs.argtypes = [i32]
     lib.see_cuda_set_adapter_tensor_backward.argtypes = [i32]
     lib.see_cuda_set_attention_one_walk.argtypes = [vp, i32]
+    lib.see_cuda_set_attention_slices.argtypes = [vp, i32]
+    lib.see_cuda_attention_slices.argtypes = [vp]
+    lib.see_cuda_attention_slices.restype = u64
     lib.see_cuda_xent_forward_static.argtypes = [vp, vp, vp, vp, u64, u64, i32, vp]
     lib.see_cuda_static_max_rows.restype = u64
     lib.see_cuda_static_last_error.restype = ctypes.c_char_p
@@ -264,6 +268,14 @@ class CudaBackend:
 
     def set_attention_one_walk(self, enabled: bool):
         self._check(self.lib.see_cuda_set_attention_one_walk(self.h, int(enabled)))
+
+    def set_attention_slices(self, use: int):
+        """0: exact attention never by digits on the tensor cores; 1: where that is the shorter way; 2: wherever it can be."""
+        self._check(self.lib.see_cuda_set_attention_slices(self.h, use))
+
+    def attention_slices(self) -> int:
+        """Instructions that ran so since creation."""
+        return int(self.lib.see_cuda_attention_slices(self.h))
 
     def set_cta_pairs(self, enabled: bool):
         """Process-wide: large tensor-core products on CTA pairs (default) or one CTA per tile."""

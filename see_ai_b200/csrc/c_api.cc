@@ -131,6 +131,13 @@ int see_cuda_set_attention_one_walk(see_cuda_backend* h, int enabled) {
   return SEE_OK;
 }
 
+int see_cuda_set_attention_slices(see_cuda_backend* h, int use) {
+  h->backend->SetAttentionSlices(use);
+  return SEE_OK;
+}
+
+uint64_t see_cuda_attention_slices(see_cuda_backend* h) { return h->backend->attention_slices(); }
+
 int see_cuda_set_adapter_fma(see_cuda_backend* h, int enabled) {
   h->backend->SetAdapterFma(enabled != 0);
   return SEE_OK;

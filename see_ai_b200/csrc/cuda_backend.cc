@@ -2733,10 +2733,12 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
       launched();
       break;
     case kAttnFwd:
-      if (!fused || !k::AttnFwdSlices(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
-                                      Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), d_status_, s))
+      if (fused && k::AttnFwdSlices(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
+                                    Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), attn_slices_, d_status_, s))
+        ++slice_executions_;
+      else
         k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), Wr(ins.out[0]), nullptr,
-                 Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
+                   Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
       launched();
       break;
     case kAttnFwdSeg: {
@@ -2772,8 +2774,10 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
           break;
         }
       }
-      if (!fused || !k::AttnFwdSlices(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
-                                      Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), d_status_, s))
+      if (fused && k::AttnFwdSlices(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
+                                    Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), attn_slices_, d_status_, s))
+        ++slice_executions_;
+      else
         k::AttnFwd(Rd(ins.in[0]), Rd(ins.in[1]), Rd(ins.in[2]), Wr(ins.in[3]), nullptr, Wr(ins.out[0]),
                    Hi32(ins.out[1]), Lo32(ins.out[1]), Hi32(ins.out[2]), Lo32(ins.out[2]), nullptr, fused, s);
       launched();
@@ -2786,8 +2790,10 @@ Status CudaBackend::Dispatch(const Instruction& ins, const StepParams& params, c
       break;
     }
     case kAttnDP:
-      if (!fused || !k::AttnDPSlices(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
-                                     Hi32(ins.out[1]), Lo32(ins.out[1]), d_status_, s))
+      if (fused && k::AttnDPSlices(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
+                                   Hi32(ins.out[1]), Lo32(ins.out[1]), attn_slices_, d_status_, s))
+        ++slice_executions_;
+      else
         k::AttnDP(Rd(ins.in[0]), Rd(ins.in[1]), Wr(ins.in[2]), Hi32(ins.out[0]), Lo32(ins.out[0]),
                   Hi32(ins.out[1]), Lo32(ins.out[1]), fused, s);
       launched();

@@ -155,6 +155,9 @@ class CudaBackend {
   // Off: relaxed products are launched one by one (takes effect at the next BeginRange).
   void SetProductGroups(bool enabled) { product_groups_ = enabled; }
   void SetAttentionOneWalk(bool enabled) { attn_one_walk_ = enabled; }
+  // The exact attention family by digits on the tensor cores, in its own order (lazy coherence).
+  void SetAttentionSlices(int use) { attn_slices_ = use == 0 ? k::SliceUse::kNever : use == 2 ? k::SliceUse::kAlways : k::SliceUse::kShorter; }
+  uint64_t attention_slices() const { return slice_executions_; }
 
   // Off: the rank-r adapter products keep the CPU's one-rounding-per-operation
   // arithmetic even in lazy coherence (default on: fused multiply-adds there).
@@ -496,6 +499,8 @@ class CudaBackend {
   bool lora_fold_enabled_ = true;
   bool product_groups_ = true;
   bool attn_one_walk_ = true;
+  k::SliceUse attn_slices_ = k::SliceUse::kShorter;
+  uint64_t slice_executions_ = 0;
   bool adapter_fma_ = true;
   // The three backward products of an adapter site (dT = a dY B^T, dB = a t^T dY,
   // dA = x^T dT), which the plan spells as three instructions that each stream a

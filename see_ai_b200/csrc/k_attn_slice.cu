@@ -625,8 +625,9 @@ bool Fits(std::initializer_list<const void*> ps, size_t B, size_t S, size_t H, s
 }  // namespace
 
 bool AttnFwdSlices(const float* q, const float* k, const float* v, float* o, float* probs, float* stats, size_t B, size_t S,
-                   size_t H, size_t d, DeviceStatus* status, cudaStream_t s) {
-  if (!Fits({q, k, v, o, stats}, B, S, H, d) || !Shorter(probs ? Form::kCached : Form::kTiled, B, S, H, d)) return false;
+                   size_t H, size_t d, SliceUse use, DeviceStatus* status, cudaStream_t s) {
+  if (use == SliceUse::kNever || !Fits({q, k, v, o, stats}, B, S, H, d)) return false;
+  if (use == SliceUse::kShorter && !Shorter(probs ? Form::kCached : Form::kTiled, B, S, H, d)) return false;
   const SliceArgs a{q, k, v, o, probs, stats, static_cast<uint32_t>(B * H), static_cast<uint32_t>(S), static_cast<uint32_t>(H),
                     static_cast<uint32_t>(d), 1.0f / sqrtf(static_cast<float>(d)),
                     S % 4 == 0 && (reinterpret_cast<uintptr_t>(probs) & 15) == 0, status};
@@ -634,9 +635,10 @@ bool AttnFwdSlices(const float* q, const float* k, const float* v, float* o, flo
   return probs ? Launch<Form::kCached>(a, blocks, s) : Launch<Form::kTiled>(a, blocks, s);
 }
 
-bool AttnDPSlices(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, DeviceStatus* status,
-                  cudaStream_t s) {
-  if (!Fits({dout, v}, B, S, H, d) || !Shorter(Form::kScores, B, S, H, d)) return false;
+bool AttnDPSlices(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, SliceUse use,
+                  DeviceStatus* status, cudaStream_t s) {
+  if (use == SliceUse::kNever || !Fits({dout, v}, B, S, H, d)) return false;
+  if (use == SliceUse::kShorter && !Shorter(Form::kScores, B, S, H, d)) return false;
   const SliceArgs a{dout, v, nullptr, nullptr, dp, nullptr, static_cast<uint32_t>(B * H), static_cast<uint32_t>(S),
                     static_cast<uint32_t>(H), static_cast<uint32_t>(d), 1.0f,
                     S % 4 == 0 && (reinterpret_cast<uintptr_t>(dp) & 15) == 0, status};

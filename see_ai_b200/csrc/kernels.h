@@ -177,11 +177,12 @@ void AttnFwd(const float* q, const float* k, const float* v, float* o, float* pr
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,
              bool fused, cudaStream_t s);  // probs != null: cached family; stats != null: tiled family
 // The same on the tensor cores (k_attn_slice.cu), where the bits are not observed and no segment starts are given.  False: not
-// a geometry of theirs, and nothing was launched.
+// a geometry of theirs (or, by default, not the shorter way), and nothing was launched.
+enum class SliceUse { kNever = 0, kShorter = 1, kAlways = 2 };
 bool AttnFwdSlices(const float* q, const float* k, const float* v, float* o, float* probs, float* stats, size_t B, size_t S,
-                   size_t H, size_t d, DeviceStatus* status, cudaStream_t s);
-bool AttnDPSlices(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, DeviceStatus* status,
-                  cudaStream_t s);
+                   size_t H, size_t d, SliceUse use, DeviceStatus* status, cudaStream_t s);
+bool AttnDPSlices(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, SliceUse use,
+                  DeviceStatus* status, cudaStream_t s);
 void AttnDP(const float* dout, const float* v, float* dp, size_t B, size_t S, size_t H, size_t d, bool own_order,
             cudaStream_t s);
 void AttnDV(const float* probs, const float* dout, float* dv, size_t B, size_t S, size_t H,
