@@ -149,23 +149,24 @@ __device__ __noinline__ void RowAgain(const SliceArgs& a, uint32_t bh, uint32_t 
     for (uint32_t c = 0; c < a.d; ++c) sum += static_cast<double>(q[c]) * static_cast<double>(k[c]);
     return static_cast<float>(sum);
   };
+  auto score = [&](uint32_t j) { return __fmul_rn(dot(j), a.inv_sqrt_d); };   // (no fused difference behind it: a maximum's is 0)
   const size_t unit = static_cast<size_t>(bh) * a.S + i;
   if constexpr (kForm == Form::kScores) {
     for (uint32_t j = lane; j < a.S; j += 32) a.probs[unit * a.S + j] = j <= i ? dot(j) : 0.0f;
   } else {
     float top = -INFINITY;
-    for (uint32_t j = lane; j <= i; j += 32) top = fmaxf(top, dot(j) * a.inv_sqrt_d);
+    for (uint32_t j = lane; j <= i; j += 32) top = fmaxf(top, score(j));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
     double denom = 0.0;
-    for (uint32_t j = lane; j <= i; j += 32) denom += static_cast<double>(expf(dot(j) * a.inv_sqrt_d - top));
+    for (uint32_t j = lane; j <= i; j += 32) denom += static_cast<double>(expf(score(j) - top));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) denom += __shfl_xor_sync(0xFFFFFFFFu, denom, o);
     const float inv = 1.0f / static_cast<float>(denom);
     float acc[2] = {0.0f, 0.0f};
     for (uint32_t j0 = 0; j0 < a.S; j0 += 32) {
       const uint32_t j = j0 + lane;
-      const float p = j <= i ? expf(dot(j) * a.inv_sqrt_d - top) * inv : 0.0f;
+      const float p = j <= i ? expf(score(j) - top) * inv : 0.0f;
       if (kForm == Form::kCached && j < a.S) a.probs[unit * a.S + j] = p;
       for (uint32_t l = 0; l < 32 && j0 + l <= i; ++l) {
         const float w = __shfl_sync(0xFFFFFFFFu, p, l);

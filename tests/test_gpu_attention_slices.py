@@ -106,7 +106,7 @@ def test_what_takes_the_kernel_unasked(shape):
     assert _run(prog, arena, True, use=0)[1] == 0
 
 
-@pytest.mark.parametrize("shape", [(24, 128, 4, 64)], ids=["24x128x4x64"])
+@pytest.mark.parametrize("shape", [(24, 128, 4, 64), (2, 200, 3, 20)], ids=["24x128x4x64", "2x200x3x20"])
 @pytest.mark.parametrize("what", ["inf_q", "nan_k", "minus_inf_k", "inf_v", "nan_v", "huge_q", "tiny_k", "zero_rows"])
 def test_rows_without_digits(what, shape):
     Bq, S, H, d = shape
