@@ -21,13 +21,18 @@
 // before.  The exponents follow a row's maximum lazily (they are relative to an earlier maximum until that is exceeded by 8), so
 // one walk over the keys does; with probabilities to be stored (the cached form) a first walk takes the statistics.
 //
-// A row whose elements are not finite, or beyond 2^60 or all below 2^-60, has no such digits: its CTA then makes its rows
-// again with dots in double, one warp a row.
+// A row whose elements are not finite, or beyond 2^60 or all below 2^-60, has no such digits, and V that is not has
+// no pieces: the rows concerned (of an odd key, those that see it) are made again with dots in double, after the
+// rest, up to 65 at a time by all warps of the CTA (Again); a tile of nothing but such rows is not walked at all.  NaN needs no such
+// thing: it goes through a row's scale into its scores.  Measured on a B200, us, 8 x 512 positions of 12 heads of 64, statistics /
+// probabilities / raw scores: 71 / 115 / 57, all NaN the same, an infinite element in one query 85 / 118 / 57, every row again 325 / 394 / 140 (the
+// tile kernels, whatever the elements: 174 / 184 / 87.7; a warp a row that reads each key three times from global memory: 10100 / 10200 / 3250).
 //
 // Every wait on an mbarrier is bounded; one that runs out raises DeviceStatus::wait_timeout and the CTA stores nothing.
 #include <algorithm>
 #include <cmath>
 #include <initializer_list>
+#include <type_traits>
 
 #include "kernels.h"
 #include "launch.cuh"
@@ -40,7 +45,7 @@ namespace {
 using namespace umma_dev;
 
 constexpr uint32_t kRows = 128, kKeys = 64, kWidth = 64;   // queries of a CTA, keys of a step, widest head
-constexpr uint32_t kWorkWarps = 8, kCutWarps = 4, kThreads = 32 * (kWorkWarps + kCutWarps + 1);
+constexpr uint32_t kWorkWarps = 8, kCutWarps = 4, kWarps = kWorkWarps + kCutWarps + 1, kThreads = 32 * kWarps;
 constexpr uint32_t kQSlice = kRows * 128, kKSlice = kKeys * 128, kPPiece = kRows * 128, kVPiece = kKeys * 128;
 constexpr uint32_t kStageBytes = 3 * kPPiece + 3 * kVPiece;   // K's four digits, then P's three pieces; V's pieces behind
 static_assert(4 * kKSlice <= 3 * kPPiece, "K's digits lie where P's pieces come");
@@ -56,8 +61,14 @@ struct __align__(16) SliceCtl {
   double denom[kParts][kRows];
   uint64_t k_full[2], v_full[2], stage_empty[2], s_full, s_empty, p_full, sum_full;
   uint32_t tmem_base;
+  volatile size_t base;                      // the tile: where its (sequence, head) begins, which it is, its first query (read again
+  volatile uint32_t bh, i0;                  // where they are needed: registers are short)
   volatile uint32_t failed;
-  volatile uint32_t odd;                     // some row has no digits
+  uint32_t odd_rows[kRows / 32];             // a bit for each row of queries without digits:
+  uint32_t nan_rows[kRows / 32];             // (rows that are NaN as they are)
+  uint32_t odd_key, odd_value;               // these are made again, and all that see this key, or this row of V
+  volatile uint32_t some;                    // there are any
+  uint8_t list[kRows];                       // those rows, in order
 };
 constexpr uint32_t kSlabFloats = 32 * 8;     // a working warp's 32 x 8 f32 on their way out
 constexpr size_t kSliceSmem = 1024 + 4 * kQSlice + 2 * kStageBytes + sizeof(SliceCtl);
@@ -81,18 +92,19 @@ __device__ __forceinline__ void FetchSixteen(float (&x)[16], const float* __rest
     x[4 * q] = f.x; x[4 * q + 1] = f.y; x[4 * q + 2] = f.z; x[4 * q + 3] = f.w;
   }
 }
-// The digits of a row that four neighbouring lanes hold; the factor that undoes their scale.  *odd: it has none.
+// The digits of a row that four neighbouring lanes hold; the factor that undoes its scale, which is NaN where an element is: its
+// scores are NaN then.  *odd: it has none.
 __device__ __forceinline__ float CutDigits(float (&x)[16], uint8_t* dst, uint32_t slice_bytes, uint32_t row, uint32_t c0, bool* odd) {
   uint32_t top = 0;   // the largest magnitude's bits (a NaN's are larger than any number's)
 #pragma unroll
   for (int e = 0; e < 16; ++e) top = max(top, __float_as_uint(x[e]) & 0x7FFFFFFFu);
   top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
   top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
-  const bool none = top >= 0x5D800000u || (top != 0 && top < 0x21800000u);   // 2^60, 2^-60
-  *odd = *odd || none;
+  const bool none = top >= 0x5D800000u || (top != 0 && top < 0x21800000u), nan = top > 0x7F800000u;   // 2^60, 2^-60
+  *odd = none && !nan;
   const uint32_t ex = top >> 23;
-  const float to = none ? 0.0f : (top == 0 ? 1.0f : __uint_as_float((260u - ex) << 23));      // 2^(7 - e)
-  const float back = none || top == 0 ? 1.0f : __uint_as_float((ex - 6u) << 23);             // 2^(e - 7)
+  const float to = none ? 0.0f : (top == 0 ? 1.0f : __uint_as_float((260u - ex) << 23));                      // 2^(7 - e)
+  const float back = nan ? NAN : none || top == 0 ? 0.0f : __uint_as_float((ex - 6u) << 23);             // 2^(e - 7)
 #pragma unroll
   for (int e = 0; e < 16; ++e) x[e] = none ? 0.0f : x[e] * to;
   constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23: adding and taking it away rounds to a whole number
@@ -137,50 +149,249 @@ __device__ __forceinline__ bool SliceWait(SliceCtl* ctl, uint64_t* bar, uint32_t
   return there;
 }
 
-// One row as the tile kernels' expressions have it, by a warp, three times over the keys and without memory for scores.
+// Rows `first` to first + count of the list as the tile kernels' expressions have them, up to kSlots of each warp together: keys
+// 64 at a time as doubles in shared memory (a conversion costs four multiply-adds), the next 64 on their way in registers, each
+// dot one chain over ascending features.  Softmax forms walk the keys twice: each lane's maximum and sum, then the probabilities
+// and their products with V.
+constexpr uint32_t kAgainSlots = 5, kAgainLd = kKeys + 1;
+struct AgainSmem {
+  double k[kKeys * kAgainLd];                      // [key][feature]
+  double q[kWarps * kAgainSlots * kWidth];
+  float v[kKeys * kWidth];
+  float w[kWarps * kAgainSlots * kKeys];           // probabilities
+};
+static_assert(sizeof(AgainSmem) <= 4 * kQSlice + 2 * kStageBytes, "in the place of the digits");
+
+__device__ __noinline__ double AgainExp(double x) { return exp(x); }
 template <Form kForm>
-__device__ __noinline__ void RowAgain(const SliceArgs& a, uint32_t bh, uint32_t i) {
-  const uint32_t lane = threadIdx.x & 31, b = bh / a.H, h = bh % a.H;
-  const size_t D = static_cast<size_t>(a.H) * a.d, base = static_cast<size_t>(b) * a.S * D + static_cast<size_t>(h) * a.d;
-  const float* q = a.q + base + i * D;
-  auto dot = [&](uint32_t j) {
-    const float* k = a.k + base + j * D;
-    double sum = 0.0;
-    for (uint32_t c = 0; c < a.d; ++c) sum += static_cast<double>(q[c]) * static_cast<double>(k[c]);
-    return static_cast<float>(sum);
+__device__ __noinline__ void Again(const SliceArgs a, AgainSmem* sm, const SliceCtl* ctl, uint32_t bh, uint32_t i0, uint32_t first,
+                                   uint32_t count) {
+  constexpr uint32_t kSlots = kAgainSlots;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t D = static_cast<size_t>(a.H) * a.d;
+  const size_t base = ctl->base;
+  uint32_t row[kSlots];
+  bool mine[kSlots];
+  uint32_t nearest = a.S;
+  double* q = sm->q + warp * kSlots * kWidth;
+  float* w = sm->w + warp * kSlots * kKeys;
+#pragma unroll
+  for (uint32_t s = 0; s < kSlots; ++s) {
+    mine[s] = warp + kWarps * s < count;
+    row[s] = i0 + ctl->list[first + (mine[s] ? warp + kWarps * s : 0)];
+    nearest = min(nearest, row[s]);
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      const uint32_t c = lane + 32 * h;
+      q[s * kWidth + c] = c < a.d ? static_cast<double>(a.q[base + static_cast<size_t>(row[s]) * D + c]) : 0.0;
+    }
+  }
+  const uint32_t chunks = (i0 + ctl->list[first + count - 1]) / kKeys + 1;
+  constexpr uint32_t kQuads = kKeys * kWidth / 4, kEach = (kQuads + kThreads - 1) / kThreads;
+  float4 kf[kEach], vf[kEach];
+  auto fetch = [&](float4 (&f)[kEach], const float* src, uint32_t chunk) {
+#pragma unroll
+    for (uint32_t e = 0; e < kEach; ++e) {
+      const uint32_t idx = threadIdx.x + e * kThreads, key = chunk * kKeys + idx / (kWidth / 4), c = idx % (kWidth / 4) * 4;
+      f[e] = idx < kQuads && key < a.S && c < a.d ? __ldg(reinterpret_cast<const float4*>(src + base + static_cast<size_t>(key) * D + c))
+                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   };
-  auto score = [&](uint32_t j) { return __fmul_rn(dot(j), a.inv_sqrt_d); };   // (no fused difference behind it: a maximum's is 0)
-  const size_t unit = static_cast<size_t>(bh) * a.S + i;
-  if constexpr (kForm == Form::kScores) {
-    for (uint32_t j = lane; j < a.S; j += 32) a.probs[unit * a.S + j] = j <= i ? dot(j) : 0.0f;
-  } else {
-    float top = -INFINITY;
-    for (uint32_t j = lane; j <= i; j += 32) top = fmaxf(top, score(j));
+  // The dots of a slot's row with keys lane and lane + 32 of the chunk in shared memory, in f32.
+  float dot[kSlots][2] = {};
+  auto dots = [&] {
+    double acc[kSlots][2] = {};
+    const double *k0 = sm->k + lane * kAgainLd, *k1 = k0 + 32 * kAgainLd;
+    if (!mine[0]) return;
+#pragma unroll 2
+    for (uint32_t c = 0; c < a.d; c += 2) {   // (d is a multiple of four)
+      const double x0 = k0[c], x1 = k0[c + 1], y0 = k1[c], y1 = k1[c + 1];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-    double denom = 0.0;
-    for (uint32_t j = lane; j <= i; j += 32) denom += static_cast<double>(expf(score(j) - top));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) denom += __shfl_xor_sync(0xFFFFFFFFu, denom, o);
-    const float inv = 1.0f / static_cast<float>(denom);
-    float acc[2] = {0.0f, 0.0f};
-    for (uint32_t j0 = 0; j0 < a.S; j0 += 32) {
-      const uint32_t j = j0 + lane;
-      const float p = j <= i ? expf(score(j) - top) * inv : 0.0f;
-      if (kForm == Form::kCached && j < a.S) a.probs[unit * a.S + j] = p;
-      for (uint32_t l = 0; l < 32 && j0 + l <= i; ++l) {
-        const float w = __shfl_sync(0xFFFFFFFFu, p, l);
-        const float* v = a.v + base + static_cast<size_t>(j0 + l) * D;
-        if (lane < a.d) acc[0] = fmaf(w, v[lane], acc[0]);
-        if (lane + 32 < a.d) acc[1] = fmaf(w, v[lane + 32], acc[1]);
+      for (uint32_t s = 0; s < kSlots; ++s) {
+        if (!mine[s]) continue;
+        const double2 f = *reinterpret_cast<const double2*>(q + s * kWidth + c);
+        acc[s][0] = fma(f.x, x0, acc[s][0]);
+        acc[s][0] = fma(f.y, x1, acc[s][0]);
+        acc[s][1] = fma(f.x, y0, acc[s][1]);
+        acc[s][1] = fma(f.y, y1, acc[s][1]);
       }
     }
-    float* o = a.o + base + i * D;
-    if (lane < a.d) o[lane] = acc[0];
-    if (lane + 32 < a.d) o[lane + 32] = acc[1];
-    if (a.stats && lane == 0)
-      *reinterpret_cast<float4*>(a.stats + unit * kAttnStatsWidth) = make_float4(top, inv, 0.0f, 0.0f);
+#pragma unroll
+    for (uint32_t s = 0; s < kSlots; ++s) {
+      dot[s][0] = static_cast<float>(acc[s][0]);
+      dot[s][1] = static_cast<float>(acc[s][1]);
+    }
+  };
+  // f(chunk) with each chunk of keys (and, where wanted, of V) in shared memory.
+  auto walk = [&](bool values, auto f) {
+    fetch(kf, a.k, 0);
+    if (values) fetch(vf, a.v, 0);
+    for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
+      __syncthreads();
+#pragma unroll
+      for (uint32_t e = 0; e < kEach; ++e) {
+        const uint32_t idx = threadIdx.x + e * kThreads;
+        if (idx >= kQuads) continue;
+        double* k = sm->k + idx / (kWidth / 4) * kAgainLd + idx % (kWidth / 4) * 4;
+        k[0] = kf[e].x; k[1] = kf[e].y; k[2] = kf[e].z; k[3] = kf[e].w;
+        if (values) *reinterpret_cast<float4*>(sm->v + idx * 4) = vf[e];
+      }
+      __syncthreads();
+      if (chunk + 1 < chunks) {
+        fetch(kf, a.k, chunk + 1);
+        if (values) fetch(vf, a.v, chunk + 1);
+      }
+      f(chunk);
+    }
+  };
+  auto to_probs = [&](uint32_t s, uint32_t j, float x) {
+    if (mine[s] && j < a.S) a.probs[(static_cast<size_t>(bh) * a.S + row[s]) * a.S + j] = x;
+  };
+  if constexpr (kForm == Form::kScores) {
+    walk(false, [&](uint32_t chunk) {
+      dots();
+#pragma unroll
+      for (uint32_t s = 0; s < kSlots; ++s)
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+          const uint32_t j = chunk * kKeys + lane + 32 * h;
+          to_probs(s, j, j <= row[s] ? dot[s][h] : 0.0f);
+        }
+    });
+  } else {
+    float top[kSlots], inv[kSlots];
+    {
+      double sum[kSlots];   // of this lane's keys, relative to its maximum
+#pragma unroll
+      for (uint32_t s = 0; s < kSlots; ++s) { top[s] = -INFINITY; sum[s] = 0.0; }
+      walk(false, [&](uint32_t chunk) {
+        dots();
+#pragma unroll
+        for (uint32_t s = 0; s < kSlots; ++s)
+#pragma unroll
+          for (uint32_t h = 0; h < 2; ++h) {
+            const float x = __fmul_rn(dot[s][h], a.inv_sqrt_d);   // (and no fused difference: a maximum's is 0)
+            if (chunk * kKeys + lane + 32 * h > row[s] || x == -INFINITY) continue;
+            if (x > top[s]) {
+              sum[s] *= AgainExp(static_cast<double>(top[s]) - static_cast<double>(x));   // (0 before the first)
+              top[s] = x;
+            }
+            sum[s] += static_cast<double>(expf(x - top[s]));
+          }
+      });
+#pragma unroll
+      for (uint32_t s = 0; s < kSlots; ++s) {
+        float all = top[s];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) all = fmaxf(all, __shfl_xor_sync(0xFFFFFFFFu, all, o));
+        // (A lane of NaN alone has no maximum of its own; a row of -inf alone has no sum: NaN, as an exponential of inf - inf.)
+        double part = top[s] == all ? sum[s] : top[s] == -INFINITY ? (sum[s] == 0.0 ? 0.0 : NAN)
+                                             : sum[s] * AgainExp(static_cast<double>(top[s]) - static_cast<double>(all));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xFFFFFFFFu, part, o);
+        top[s] = all;
+        inv[s] = all == -INFINITY ? NAN : 1.0f / static_cast<float>(part);
+      }
+    }
+    float acc[kSlots][2] = {};
+    walk(true, [&](uint32_t chunk) {
+      dots();
+#pragma unroll
+      for (uint32_t s = 0; s < kSlots; ++s)
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+          const uint32_t j = chunk * kKeys + lane + 32 * h;
+          const float p = j <= row[s] ? expf(__fmul_rn(dot[s][h], a.inv_sqrt_d) - top[s]) * inv[s] : 0.0f;
+          if constexpr (kForm == Form::kCached) to_probs(s, j, p);
+          w[s * kKeys + lane + 32 * h] = p;
+        }
+      __syncwarp();
+      const bool all_seen = chunk * kKeys + kKeys - 1 <= nearest;   // (an unseen key's V may be NaN: it is passed by)
+#pragma unroll 1
+      for (uint32_t l = 0; l < kKeys; l += 4) {
+        float x[4][2];
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+          x[e][0] = sm->v[(l + e) * kWidth + lane];
+          x[e][1] = sm->v[(l + e) * kWidth + lane + 32];
+        }
+#pragma unroll
+        for (uint32_t s = 0; s < kSlots; ++s) {
+          if (!mine[s]) continue;
+          const float4 p4 = *reinterpret_cast<const float4*>(w + s * kKeys + l);
+          const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+          for (uint32_t e = 0; e < 4; ++e) {
+            if (!all_seen && chunk * kKeys + l + e > row[s]) continue;
+            acc[s][0] = fmaf(p[e], x[e][0], acc[s][0]);
+            acc[s][1] = fmaf(p[e], x[e][1], acc[s][1]);
+          }
+        }
+      }
+      __syncwarp();
+    });
+#pragma unroll
+    for (uint32_t s = 0; s < kSlots; ++s) {
+      if (!mine[s]) continue;
+      float* o = a.o + base + static_cast<size_t>(row[s]) * D;
+      if (lane < a.d) o[lane] = acc[s][0];
+      if (lane + 32 < a.d) o[lane + 32] = acc[s][1];
+      if (a.stats && lane == 0)
+        *reinterpret_cast<float4*>(a.stats + (static_cast<size_t>(bh) * a.S + row[s]) * kAttnStatsWidth) = make_float4(top[s], inv[s], 0.0f, 0.0f);
+    }
   }
+  if constexpr (kForm != Form::kTiled) {   // the keys no row of these sees
+#pragma unroll
+    for (uint32_t s = 0; s < kSlots; ++s)
+      for (uint32_t j = chunks * kKeys + lane; j < a.S; j += 32) to_probs(s, j, 0.0f);
+  }
+  __syncthreads();
+}
+
+// A CTA's tile.
+struct Place {
+  uint32_t bh, i0, live, n;   // (sequence, head); its queries; steps of a walk over the keys
+  size_t D, base;
+  __device__ __forceinline__ Place(const SliceArgs& a, const SliceCtl* ctl) {
+    bh = ctl->bh;
+    i0 = ctl->i0;
+    live = min(kRows, a.S - i0);
+    n = (min(i0 + kRows, a.S) + kKeys - 1) / kKeys;
+    D = static_cast<size_t>(a.H) * a.d;
+    base = ctl->base;
+  }
+  __device__ __forceinline__ uint32_t RowsOf(uint32_t w) const {   // the 32 rows of a word, those there are
+    return live >= 32 * w + 32 ? 0xFFFFFFFFu : live > 32 * w ? (1u << (live - 32 * w)) - 1 : 0u;
+  }
+  __device__ __forceinline__ bool Without(const SliceCtl* ctl) const {   // not one row has digits
+    bool none = true;
+#pragma unroll
+    for (uint32_t w = 0; w < kRows / 32; ++w) none = none && ctl->odd_rows[w] == RowsOf(w);
+    return none;
+  }
+};
+// Behind the tile: rows that are made again.
+template <Form kForm>
+__device__ __forceinline__ void Finish(const SliceArgs& a, AgainSmem* sm, SliceCtl* ctl) {
+  const Place at(a, ctl);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (ctl->some == 0) return;
+  uint32_t words[kRows / 32], count = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kRows / 32; ++w) {
+    auto see = [&](uint32_t key) {
+      const uint32_t r0 = at.i0 + 32 * w;
+      return key <= r0 ? 0xFFFFFFFFu : key - r0 >= 32 ? 0u : 0xFFFFFFFFu << (key - r0);
+    };
+    words[w] = (ctl->odd_rows[w] | see(ctl->odd_key) | (see(ctl->odd_value) & ~ctl->nan_rows[w])) & at.RowsOf(w);
+    count += __popc(words[w]);
+  }
+  if (count == 0) return;
+  for (uint32_t w = 0, before = 0; w < kRows / 32; before += __popc(words[w]), ++w)
+    if (warp == w && (words[w] >> lane & 1)) ctl->list[before + __popc(words[w] & ((1u << lane) - 1))] = static_cast<uint8_t>(32 * w + lane);
+  __syncthreads();
+  for (uint32_t first = 0; first < count; first += kWarps * kAgainSlots)
+    Again<kForm>(a, sm, ctl, at.bh, at.i0, first, min(kWarps * kAgainSlots, count - first));
 }
 
 template <Form kForm>
@@ -191,15 +402,6 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
   SliceCtl* ctl = reinterpret_cast<SliceCtl*>(ring + 2 * kStageBytes);
 
   const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  // Longest tiles first over the whole grid, so that the last wave is short ones.
-  const uint32_t tiles = (a.S + kRows - 1) / kRows, tile = tiles - 1 - blockIdx.x / a.BH, bh = blockIdx.x % a.BH;
-  const uint32_t i0 = tile * kRows, keys = min(i0 + kRows, a.S);
-  const uint32_t n = (keys + kKeys - 1) / kKeys;                                  // steps of a walk
-  const uint32_t ahead = kForm == Form::kTiled ? 0 : n;                           // steps that only take scores
-  const uint32_t total = kForm == Form::kCached ? 2 * n : n;
-  const size_t D = static_cast<size_t>(a.H) * a.d;
-  const size_t base = static_cast<size_t>(bh / a.H) * a.S * D + static_cast<size_t>(bh % a.H) * a.d;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       MbarInit(&ctl->k_full[s], kCutWarps);
@@ -211,8 +413,15 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
     MbarInit(&ctl->p_full, kWorkWarps);
     MbarInit(&ctl->sum_full, 1);
     ctl->failed = 0;
-    ctl->odd = 0;
+    ctl->odd_key = ctl->odd_value = 0xFFFFFFFFu;
+    ctl->some = 0;
+    for (uint32_t w = 0; w < kRows / 32; ++w) ctl->odd_rows[w] = ctl->nan_rows[w] = 0;
     MbarInitFence();
+    // Longest tiles first over the whole grid, so that the last wave is short ones.
+    ctl->i0 = ((a.S + kRows - 1) / kRows - 1 - blockIdx.x / a.BH) * kRows;
+    const uint32_t bh = blockIdx.x % a.BH;
+    ctl->bh = bh;
+    ctl->base = (static_cast<size_t>(bh / a.H) * a.S * a.H + bh % a.H) * a.d;
   }
   if (warp == kWorkWarps + kCutWarps) TmemAlloc(&ctl->tmem_base, 512);
   TcFenceBefore();
@@ -221,22 +430,55 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
   AwaitPrevious();
   constexpr uint32_t tmem = 0;   // all 512 columns are this CTA's
 
-  if (warp < kWorkWarps + kCutWarps) {   // the queries' digits
-    bool odd = false;
-    for (uint32_t t = threadIdx.x; t < 4 * kRows; t += 32 * (kWorkWarps + kCutWarps)) {   // (whole warps)
-      const uint32_t r = t >> 2, c0 = (t & 3) * 16;
-      float x[16];
-      FetchSixteen(x, a.q + base + static_cast<size_t>(i0 + r) * D, i0 + r < a.S, c0, a.d);
-      const float back = CutDigits(x, q_s, kQSlice, r, c0, &odd);
-      if (c0 == 0) ctl->q_scale[r] = back * (kForm == Form::kScores ? 1.0f : a.inv_sqrt_d);
+  const Place at(a, ctl);
+  const uint32_t i0 = at.i0, n = at.n;
+  const uint32_t ahead = kForm == Form::kTiled ? 0 : n;                           // steps that only take scores
+  const uint32_t total = kForm == Form::kCached ? 2 * n : n;
+  const size_t D = at.D, base = at.base;
+  constexpr uint32_t kEach = kKeys / (8 * kCutWarps);   // keys of a cutting thread in a step, 8 kCutWarps apart
+  const uint32_t c0 = (threadIdx.x & 3) * 16;           // sixteen features of a thread that cuts
+  auto fetch_keys = [&](float (&f)[kEach][16], const float* src, uint32_t u) {
+#pragma unroll
+    for (uint32_t h = 0; h < kEach; ++h) {
+      const uint32_t key = (u < n ? u : u - n) * kKeys + ((threadIdx.x - 32 * kWorkWarps) >> 2) + h * 8 * kCutWarps;
+      FetchSixteen(f[h], src + base + static_cast<size_t>(key) * D, u < total && key < a.S, c0, a.d);
     }
-    if (odd) ctl->odd = 1;
-    FenceProxyAsync();
+  };
+  float k_next[kEach][16];   // a step's keys, on their way since the step before
+  {   // the queries' digits, by whole warps; all that the first step needs of memory is asked for at once
+    constexpr uint32_t kLoaders = kWorkWarps + kCutWarps, kTwice = kRows / 8 - kLoaders;   // warps that have rows twice
+    static_assert(kTwice <= kWorkWarps, "not those that have keys");
+    float x[16], second[16];
+    auto fetch = [&](float (&f)[16], uint32_t r) { FetchSixteen(f, a.q + base + static_cast<size_t>(i0 + r) * D, i0 + r < a.S, c0, a.d); };
+    if (warp < kLoaders) fetch(x, threadIdx.x >> 2);
+    if (warp < kTwice) fetch(second, 8 * kLoaders + (threadIdx.x >> 2));
+    if (warp >= kWorkWarps && warp < kLoaders) fetch_keys(k_next, a.k, 0);
+    if (warp < kLoaders) {
+#pragma unroll 1
+      for (uint32_t r = threadIdx.x >> 2;;) {
+        bool odd;
+        const float back = CutDigits(x, q_s, kQSlice, r, c0, &odd);
+        if (c0 == 0) {
+          ctl->q_scale[r] = back * (kForm == Form::kScores ? 1.0f : a.inv_sqrt_d);
+          if (odd) {
+            atomicOr(&ctl->odd_rows[r / 32], 1u << (r & 31));
+            ctl->some = 1;
+          }
+        }
+        __syncwarp();
+        r += 8 * kLoaders;
+        if (r >= kRows) break;   // (whole warps)
+#pragma unroll
+        for (int e = 0; e < 16; ++e) x[e] = second[e];
+      }
+      FenceProxyAsync();
+    }
   }
   __syncthreads();
 
   bool ok = true;
-  if (warp == kWorkWarps + kCutWarps) {
+  if (at.Without(ctl)) {
+  } else if (warp == kWorkWarps + kCutWarps) {
     // ---- products (the whole warp walks and waits; one elected lane issues) ----
     const uint32_t k_steps = (a.d + 15) / 16;
     auto scores = [&](uint32_t u) {
@@ -290,43 +532,58 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
     }
   } else if (warp >= kWorkWarps) {
     // ---- K's digits, V's pieces ----
-    const uint32_t t = threadIdx.x - 32 * kWorkWarps, r0 = t >> 2, c0 = (t & 3) * 16;
-    constexpr uint32_t kEach = kKeys / (8 * kCutWarps);   // keys of a thread, 8 kCutWarps apart
-    bool odd = false;
-    float x[kEach][16], y[kEach][16];   // a step's elements, on their way since the step before
+    const uint32_t t = threadIdx.x - 32 * kWorkWarps, r0 = t >> 2;
+    float y[kEach][16];
     auto row_of = [&](uint32_t h) { return r0 + h * 8 * kCutWarps; };
     auto sums_at = [&](uint32_t u) { return kForm == Form::kTiled || (kForm == Form::kCached && u >= ahead && u < total); };
-    auto fetch = [&](float (&f)[kEach][16], const float* src, uint32_t u) {
-#pragma unroll
-      for (uint32_t h = 0; h < kEach; ++h) {
-        const uint32_t key = (u < n ? u : u - n) * kKeys + row_of(h);
-        FetchSixteen(f[h], src + base + static_cast<size_t>(key) * D, u < total && key < a.S, c0, a.d);
-      }
-    };
-    fetch(x, a.k, 0);
-    if (sums_at(0)) fetch(y, a.v, 0);
+    if (sums_at(0)) fetch_keys(y, a.v, 0);
     for (uint32_t u = 0; u < total && ok; ++u) {
       const uint32_t s = u & 1;
       uint8_t* stage = ring + s * kStageBytes;
       if (u >= 2) ok = SliceWait(ctl, &ctl->stage_empty[s], ((u >> 1) - 1) & 1);
       if (!ok) break;
+      const uint32_t key0 = (u < n ? u : u - n) * kKeys;
+      bool odd[kEach];   // (looked at behind the loop: the rows' cutting is one stream of instructions)
 #pragma unroll
       for (uint32_t h = 0; h < kEach; ++h) {
-        const float back = CutDigits(x[h], stage, kKSlice, row_of(h), c0, &odd);
+        const float back = CutDigits(k_next[h], stage, kKSlice, row_of(h), c0, &odd[h]);
         if (c0 == 0) ctl->k_scale[u & 3][row_of(h)] = back;
       }
-      if (odd) ctl->odd = 1;
+      auto least = [&] {
+        uint32_t at = 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t h = 0; h < kEach; ++h) at = min(at, odd[h] ? key0 + row_of(h) : 0xFFFFFFFFu);
+        return at;
+      };
+      if (least() != 0xFFFFFFFFu) {
+        atomicMin(&ctl->odd_key, least());
+        ctl->some = 1;
+      }
       FenceProxyAsync();
       __syncwarp();
       if (lane == 0) MbarArrive(&ctl->k_full[s]);
-      fetch(x, a.k, u + 1);
+      fetch_keys(k_next, a.k, u + 1);
       if (sums_at(u)) {   // V's pieces while the scores are formed
+        // (Rows that do not see the key see zeros.)
+#pragma unroll
+        for (uint32_t h = 0; h < kEach; ++h) {
+          odd[h] = false;
+#pragma unroll
+          for (int e = 0; e < 16; ++e) odd[h] = odd[h] || !(fabsf(y[h][e]) < 1e36f);
+        }
+        if (least() != 0xFFFFFFFFu) {
+          atomicMin(&ctl->odd_value, least());
+          ctl->some = 1;
+#pragma unroll
+          for (uint32_t h = 0; h < kEach; ++h)
+#pragma unroll
+            for (int e = 0; e < 16; ++e) y[h][e] = odd[h] ? 0.0f : y[h][e];
+        }
 #pragma unroll
         for (uint32_t h = 0; h < kEach; ++h) {
           uint32_t w[3][8];
 #pragma unroll
           for (int e = 0; e < 16; e += 2) {
-            odd = odd || !(fabsf(y[h][e]) < 1e36f) || !(fabsf(y[h][e + 1]) < 1e36f);
             uint32_t p[3];
             CutPieces(y[h][e], y[h][e + 1], p);
 #pragma unroll
@@ -339,19 +596,17 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
             *reinterpret_cast<uint4*>(at + Sw128Offset(row_of(h), c0 / 8 + 1)) = make_uint4(w[i][4], w[i][5], w[i][6], w[i][7]);
           }
         }
-        if (odd) ctl->odd = 1;
         FenceProxyAsync();
         __syncwarp();
       }
       if (lane == 0) MbarArrive(&ctl->v_full[s]);   // (every step: its phases are the stage's)
-      if (sums_at(u + 1)) fetch(y, a.v, u + 1);
+      if (sums_at(u + 1)) fetch_keys(y, a.v, u + 1);
     }
   } else {
     // ---- scores, probabilities, sums: thread (row, part of the keys) ----
     const uint32_t quarter = warp & 3, part = warp >> 2, r = quarter * 32 + lane, i = i0 + r;
     const uint32_t t_s = tmem + ((quarter * 32) << 16) + part * kOwn, t_o = t_s + kScoreCols;
     const float q_scale = ctl->q_scale[r];
-    const size_t unit = static_cast<size_t>(bh) * a.S + i;
     float s[kOwn];
     [[maybe_unused]] float sum[kOwn];
     [[maybe_unused]] float top = -INFINITY, ref = -INFINITY, inv = 0.0f;   // the row's maximum; what its exponents are relative to
@@ -431,7 +686,8 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
         d0 += Widen(s[e]);
         d1 += Widen(s[e + 1]);
       }
-      denom += d0 + d1;
+      const double d = d0 + d1;
+      denom += d < 0x1p100 ? d : NAN;   // (a NaN, widened, is 2^128)
       return factor;
     };
     // Eight columns of 32 rows of the score matrix at a time, through memory of the stage that holds neither K's digits nor,
@@ -452,7 +708,7 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
           const uint32_t lr = x * 16 + (lane >> 1), q = lane & 1, row = i0 + quarter * 32 + lr, j = key0 + c + 4 * q;
           const float4 f = *reinterpret_cast<const float4*>(slab + lr * 8 + ((q ^ ((lr >> 2) & 1)) * 4));
           if (row >= a.S || j >= a.S) continue;
-          float* to = a.probs + (static_cast<size_t>(bh) * a.S + row) * a.S + j;
+          float* to = a.probs + (static_cast<size_t>(ctl->bh) * a.S + row) * a.S + j;
           if (a.store16) {
             *reinterpret_cast<float4*>(to) = f;
           } else {
@@ -491,10 +747,15 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
       for (uint32_t p = 0; p < kParts; ++p) whole += ctl->denom[p][r];
       return whole;
     };
+    auto mark = [&](bool nan) {   // rows that nothing need be made again of
+      const uint32_t none = __ballot_sync(0xFFFFFFFFu, nan);
+      if (part == 0 && lane == 0) ctl->nan_rows[quarter] = none;
+    };
     auto put_stats = [&](double whole) {   // relative to the maximum: the rows' statistics, and their factor
       inv = 1.0f / static_cast<float>(whole * exp(static_cast<double>(ref) - static_cast<double>(top)));
-      if (a.stats && part == 0 && i < a.S && ok && ctl->odd == 0)
-        *reinterpret_cast<float4*>(a.stats + unit * kAttnStatsWidth) = make_float4(top, inv, 0.0f, 0.0f);
+      mark(isnan(inv));
+      if (a.stats && part == 0 && i < a.S && ok)
+        *reinterpret_cast<float4*>(a.stats + (static_cast<size_t>(ctl->bh) * a.S + i) * kAttnStatsWidth) = make_float4(top, inv, 0.0f, 0.0f);
     };
 
     if constexpr (kForm == Form::kScores) {
@@ -517,6 +778,10 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
         if constexpr (kForm == Form::kCached) {
 #pragma unroll
           for (int e = 0; e < kOwn; ++e) s[e] = expf(s[e] - top) * inv;
+          if (key0 + kOwn - 1 > i0 + quarter * 32) {   // (of a row that is NaN, too, the keys it does not see are 0)
+#pragma unroll
+            for (int e = 0; e < kOwn; ++e) s[e] = key0 + e <= i ? s[e] : 0.0f;
+          }
           if (ok) store_scores(u, key0);
           row_sync();   // (a quarter's pieces and slabs share memory)
         } else {
@@ -563,14 +828,15 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
             make_float4(sum[4 * q] * scale, sum[4 * q + 1] * scale, sum[4 * q + 2] * scale, sum[4 * q + 3] * scale);
       asm volatile("bar.sync 5, %0;" ::"n"(32 * kWorkWarps) : "memory");
       const uint32_t chunk = threadIdx.x & 15;
-      if (ok && ctl->odd == 0 && 4 * chunk < a.d)
+      if (ok && 4 * chunk < a.d)
         for (uint32_t row = threadIdx.x >> 4; row < kRows && i0 + row < a.S; row += 2 * kWorkWarps)
-          *reinterpret_cast<float4*>(a.o + base + static_cast<size_t>(i0 + row) * D + 4 * chunk) =
+          if ((ctl->odd_rows[row / 32] >> (row & 31) & 1) == 0 && i0 + row < ctl->odd_key &&
+              (i0 + row < ctl->odd_value || (ctl->nan_rows[row / 32] >> (row & 31) & 1) != 0)) *reinterpret_cast<float4*>(a.o + ctl->base + static_cast<size_t>(i0 + row) * a.H * a.d + 4 * chunk) =
               *reinterpret_cast<const float4*>(tile_o + row * kWidth + ((chunk ^ (row & 15)) * 4));
     }
     if constexpr (kForm != Form::kTiled) {   // the keys no walk reaches
       for (uint32_t row = warp; ok && row < kRows && i0 + row < a.S; row += kWorkWarps) {
-        float* to = a.probs + (static_cast<size_t>(bh) * a.S + i0 + row) * a.S;
+        float* to = a.probs + (static_cast<size_t>(ctl->bh) * a.S + i0 + row) * a.S;
         for (uint32_t j = n * kKeys + lane; j < a.S; j += 32) to[j] = 0.0f;
       }
     }
@@ -587,8 +853,7 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
     TcFenceAfter();
     TmemFree(ctl->tmem_base, 512);
   }
-  if (ctl->odd != 0 && ctl->failed == 0)
-    for (uint32_t row = warp; row < kRows && i0 + row < a.S; row += kThreads / 32) RowAgain<kForm>(a, bh, i0 + row);
+  if (ctl->failed == 0) Finish<kForm>(a, reinterpret_cast<AgainSmem*>(q_s), ctl);
 }
 
 // Whether the kernel is the shorter one, by estimates of both in us: 64 keys a step, the longest tile's steps or an SM's share

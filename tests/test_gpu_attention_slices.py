@@ -107,7 +107,8 @@ def test_what_takes_the_kernel_unasked(shape):
 
 
 @pytest.mark.parametrize("shape", [(24, 128, 4, 64), (2, 200, 3, 20)], ids=["24x128x4x64", "2x200x3x20"])
-@pytest.mark.parametrize("what", ["inf_q", "nan_k", "minus_inf_k", "inf_v", "nan_v", "huge_q", "tiny_k", "zero_rows"])
+@pytest.mark.parametrize("what", ["inf_q", "nan_k", "minus_inf_k", "inf_v", "nan_v", "huge_q", "tiny_k", "zero_rows", "nan_all", "inf_scores",
+                                  "nan_last_tile"])
 def test_rows_without_digits(what, shape):
     Bq, S, H, d = shape
     prog, arena, run = _three(shape)
@@ -131,6 +132,17 @@ def test_rows_without_digits(what, shape):
     elif what == "tiny_k":
         x["k"][:, 64:] *= np.float32(1e-30)
         x["v"][:, ::3] *= np.float32(1e-30)
+    elif what == "nan_all":
+        for t in x.values():
+            t[:] = np.nan
+    elif what == "inf_scores":                   # finite rows whose products are not, of both signs
+        x["q"][:, S // 2] *= np.float32(1e25)
+        x["k"][:, 3] *= np.float32(1e25)
+        x["do"][:, S // 2] *= np.float32(1e25)
+        x["v"][:, 3] *= np.float32(1e25)
+    elif what == "nan_last_tile":                # a whole tile of queries without digits, and the one before it with them
+        x["q"][:, 128:] = np.nan
+        x["do"][:, 128:] = np.nan
     else:
         x["q"][:, 3] = 0.0
         x["k"][:, 0:40] = 0.0
