@@ -1,16 +1,24 @@
-// Exact causal attention on the tensor cores, where the bits are not observed: scores as accurate as dots in double, sums
-// of probabilities times values as accurate as f32 multiply-adds.
+// Exact causal attention on the tensor cores, where the bits are not observed: scores as accurate as dots in double that are
+// rounded to f32, but for a tenth of the rounding of the row's largest score, sums of probabilities times values as accurate as
+// f32 multiply-adds.
 //
-// Scores.  A row of Q (or K) is a fixed-point number per element: scaled by a power of two to (-128, 128) and cut into four
-// signed digits of eight bits, each a whole number up to 128 and so a bf16 value exactly:
-//     x = 2^(e - 7) (s0 + s1 / 2^8 + s2 / 2^16 + s3 / 2^24) + r,  |r| <= 2^(e - 32),  2^e > max |x|.
-// Products of digits are whole numbers up to 2^14, and a sum of up to 4 x 64 of them is one below 2^24: the tensor core's
+// Scores.  A row of Q (or K) is a fixed-point number per element: scaled by a power of two to (-256, 256) and cut into four
+// signed digits of eight bits, whole numbers up to 256 (the first) and 128 and so bf16 values exactly:
+//     x = 2^(e - 8) (s0 + s1 / 2^8 + s2 / 2^16 + s3 / 2^24) + r,  |r| <= 2^(e - 33),  2^e > max |x|.
+// Products of digits are whole numbers, and a sum of those of up to 64 features with one i + j is below 2^23: the tensor core's
 // f32 accumulator holds it exactly, in whatever order and rounding it adds.  The thirteen products of digits with i + j <= 4 meet in
-// five accumulators, one for each i + j, which four multiply-adds put together.  What is left out (i + j > 4, r) is
-// 2^-32 of 2^(eq + ek) in the middle, a fiftieth of the rounding to f32 that a dot in double ends with too.
+// five accumulators, one for each i + j, which four multiply-adds put together.
 // (Fixed-point slices: Ozaki, Ogita, Oishi, Rump, "Error-free transformations of matrix multiplication by using fast
 // routines of matrix multiplication", 2012.)  The digits of K lie one under the other, so digit i of Q times all of K's
 // digits that count is one product of width 64 (4 - i): the accumulators stand side by side, each i starts one further on.
+//
+// What is left out of a score (r, i + j > 4) is about 2^-33 of 2^(eq + ek), whatever the score is, so it matters that a row's large
+// elements meet large ones.  Two things see to it.  (1) Features are balanced: each is multiplied by a power of two in Q and
+// divided by it in K, so that all features are of one size in the tile's queries (by the mean exponents of 32 of them; not where
+// all are alike anyway): gains that cancel between Q and K, or a feature that is large in one and small in the other, cost no bits.  (2) A row whose largest score is
+// still below 2^(eq + ek - 4), that is where 2^(eq + ek - 33) exceeds 2^-29 of it (of probabilities: of the larger of it and 1,
+// scaled), is made again with dots in double.  Errors against float64, by rounding to f32 alone 1: normal elements 1.000, gains of
+// 2^+-2 to 2^+-12 a feature 1.001, spread of 2^+-12 within the rows 1.001, queries orthogonal to ten times as large a mean of the keys 1.005.
 //
 // Output sums.  P and V as three bf16 pieces each, six piece products by the same scheme, 64 keys at a time: three
 // accumulators, added in f32 registers.
@@ -21,12 +29,13 @@
 // before.  The exponents follow a row's maximum lazily (they are relative to an earlier maximum until that is exceeded by 8), so
 // one walk over the keys does; with probabilities to be stored (the cached form) a first walk takes the statistics.
 //
-// A row whose elements are not finite, or beyond 2^60 or all below 2^-60, has no such digits, and V that is not has
-// no pieces: the rows concerned (of an odd key, those that see it) are made again with dots in double, after the
+// A row whose elements are not finite, or beyond 2^90 or all below 2^-90, has no such digits, and V that is not has
+// no pieces: the rows concerned (of an odd key, those that see it) are made again likewise, after the
 // rest, up to 65 at a time by all warps of the CTA (Again); a tile of nothing but such rows is not walked at all.  NaN needs no such
 // thing: it goes through a row's scale into its scores.  Measured on a B200, us, 8 x 512 positions of 12 heads of 64, statistics /
-// probabilities / raw scores: 71 / 115 / 57, all NaN the same, an infinite element in one query 85 / 118 / 57, every row again 325 / 394 / 140 (the
-// tile kernels, whatever the elements: 174 / 184 / 87.7; a warp a row that reads each key three times from global memory: 10100 / 10200 / 3250).
+// probabilities / raw scores: 72.5 / 116 / 58.4; gains of 2^+-10 a feature 74.2 / 117 / 60.7; all NaN 73.2 / 116 / 57.3; an infinite element in
+// one query 86 / 124 / 59.2; every row again 325 / 394 / 140 (the tile kernels, whatever the elements: 174 / 184 / 87.7; with neither
+// balance nor test: 70.9 / 115 / 56.7).
 //
 // Every wait on an mbarrier is bounded; one that runs out raises DeviceStatus::wait_timeout and the CTA stores nothing.
 #include <algorithm>
@@ -51,12 +60,16 @@ constexpr uint32_t kStageBytes = 3 * kPPiece + 3 * kVPiece;   // K's four digits
 static_assert(4 * kKSlice <= 3 * kPPiece, "K's digits lie where P's pieces come");
 constexpr uint32_t kParts = kWorkWarps / 4, kOwn = kKeys / kParts;   // threads to a row; keys (and features) of each
 constexpr uint32_t kScoreCols = 5 * kKeys;                    // tensor memory: five accumulators of scores, three of sums
+constexpr uint32_t kGroups = 4, kGroupRows = 8, kFirst = 8;   // rows that features are balanced by; rows of dP that are always dots in double
 constexpr float kSlack = 8.0f;                                // how far a row's maximum may exceed its reference
 
 enum class Form { kTiled, kCached, kScores };   // statistics; probabilities and statistics; raw scores (dP = dO V^T)
 
 struct __align__(16) SliceCtl {
   float q_scale[kRows], k_scale[4][kKeys];   // (a step's is read after its stage may have gone on: four in turns)
+  float gain[kWidth], ungain[kWidth];        // the features' powers of two: K's (V's) and Q's (dO's)
+  uint2 sample[kGroups][kWidth / 2];         // of a group of queries' elements, by feature: how many, and the sum of their exponents
+  double first[kFirst][kFirst];              // the first scores of a sequence
   float row_max[2][kParts][kRows];           // by parity of the step
   double denom[kParts][kRows];
   uint64_t k_full[2], v_full[2], stage_empty[2], s_full, s_empty, p_full, sum_full;
@@ -64,7 +77,9 @@ struct __align__(16) SliceCtl {
   volatile size_t base;                      // the tile: where its (sequence, head) begins, which it is, its first query (read again
   volatile uint32_t bh, i0;                  // where they are needed: registers are short)
   volatile uint32_t failed;
-  uint32_t odd_rows[kRows / 32];             // a bit for each row of queries without digits:
+  uint32_t k_top;                            // the largest scale of the keys, its bits
+  uint32_t odd_rows[kRows / 32];             // a bit for each row of queries without digits ...
+  uint32_t again[kRows / 32];                // ... and for each whose scores are too small for what the digits leave out:
   uint32_t nan_rows[kRows / 32];             // (rows that are NaN as they are)
   uint32_t odd_key, odd_value;               // these are made again, and all that see this key, or this row of V
   volatile uint32_t some;                    // there are any
@@ -92,6 +107,14 @@ __device__ __forceinline__ void FetchSixteen(float (&x)[16], const float* __rest
     x[4 * q] = f.x; x[4 * q + 1] = f.y; x[4 * q + 2] = f.z; x[4 * q + 3] = f.w;
   }
 }
+// Sixteen elements times their features' factors.
+__device__ __forceinline__ void ScaleSixteen(float (&x)[16], const float* gain, uint32_t c0) {
+#pragma unroll
+  for (int e = 0; e < 16; e += 4) {
+    const float4 g = *reinterpret_cast<const float4*>(gain + c0 + e);
+    x[e] *= g.x; x[e + 1] *= g.y; x[e + 2] *= g.z; x[e + 3] *= g.w;
+  }
+}
 // The digits of a row that four neighbouring lanes hold; the factor that undoes its scale, which is NaN where an element is: its
 // scores are NaN then.  *odd: it has none.
 __device__ __forceinline__ float CutDigits(float (&x)[16], uint8_t* dst, uint32_t slice_bytes, uint32_t row, uint32_t c0, bool* odd) {
@@ -100,11 +123,11 @@ __device__ __forceinline__ float CutDigits(float (&x)[16], uint8_t* dst, uint32_
   for (int e = 0; e < 16; ++e) top = max(top, __float_as_uint(x[e]) & 0x7FFFFFFFu);
   top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
   top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
-  const bool none = top >= 0x5D800000u || (top != 0 && top < 0x21800000u), nan = top > 0x7F800000u;   // 2^60, 2^-60
+  const bool none = top >= 0x6C800000u || (top != 0 && top < 0x12800000u), nan = top > 0x7F800000u;   // 2^90, 2^-90
   *odd = none && !nan;
   const uint32_t ex = top >> 23;
-  const float to = none ? 0.0f : (top == 0 ? 1.0f : __uint_as_float((260u - ex) << 23));                      // 2^(7 - e)
-  const float back = nan ? NAN : none || top == 0 ? 0.0f : __uint_as_float((ex - 6u) << 23);             // 2^(e - 7)
+  const float to = none ? 0.0f : (top == 0 ? 1.0f : __uint_as_float((261u - ex) << 23));                      // 2^(8 - e)
+  const float back = nan ? NAN : none || top == 0 ? 0.0f : __uint_as_float((ex - 7u) << 23);             // 2^(e - 8)
 #pragma unroll
   for (int e = 0; e < 16; ++e) x[e] = none ? 0.0f : x[e] * to;
   constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23: adding and taking it away rounds to a whole number
@@ -123,6 +146,40 @@ __device__ __forceinline__ float CutDigits(float (&x)[16], uint8_t* dst, uint32_
     *reinterpret_cast<uint4*>(at + Sw128Offset(row, c0 / 8 + 1)) = make_uint4(w[4], w[5], w[6], w[7]);
   }
   return back;
+}
+// An element of the sample: one, and its exponent; nothing of zeros and of what is not finite.
+__device__ __forceinline__ uint32_t CountExponent(float f) {
+  const uint32_t e = __float_as_uint(f) >> 23 & 0xFFu;
+  return e - 1u < 254u ? (1u << 16) + e : 0u;
+}
+// The features' powers of two, from the means of their exponents, by every warp for itself (all write the same).  False: none is
+// worth it, they are all within a factor of six of the middle, or of sixteen of one another.  (The kernel's code is cold at most of
+// its launches: as little as can be comes before the first products.)
+__device__ __forceinline__ bool BalanceFeatures(SliceCtl* ctl) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint2 v = make_uint2(0, 0);
+#pragma unroll
+  for (uint32_t g = 0; g < kGroups; ++g) {
+    const uint2 f = ctl->sample[g][lane];
+    v = make_uint2(v.x + f.x, v.y + f.y);
+  }
+  // Mostly as many of each, and no two sums more than four powers of two an element apart: nothing to divide.
+  const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, max(v.x, v.y));
+  const uint32_t least = __reduce_min_sync(0xFFFFFFFFu, min(v.x != 0 ? v.x : ~0u, v.y != 0 ? v.y : ~0u));
+  if (most - least <= 4 * kGroups * kGroupRows) return false;
+  auto mean = [](uint32_t w) {   // in eighths
+    return __float2int_rn(__fdividef(static_cast<float>((w & 0xFFFFu) * 8), fmaxf(static_cast<float>(w >> 16), 1.0f)));
+  };
+  const int m0 = mean(v.x), m1 = mean(v.y);
+  const int all = __reduce_add_sync(0xFFFFFFFFu, m0 + m1 + (v.x != 0 ? 1 << 20 : 0) + (v.y != 0 ? 1 << 20 : 0));
+  const int middle = __float2int_rn(__fdividef(static_cast<float>(all & 0xFFFFF), fmaxf(static_cast<float>(all >> 20), 1.0f)));
+  const int off0 = v.x != 0 ? m0 - middle : 0, off1 = v.y != 0 ? m1 - middle : 0;
+  if (!__any_sync(0xFFFFFFFFu, max(abs(off0), abs(off1)) > 20)) return false;
+  const int by0 = max(-64, min(64, (off0 + 4) >> 3)), by1 = max(-64, min(64, (off1 + 4) >> 3));
+  *reinterpret_cast<float2*>(ctl->gain + 2 * lane) = make_float2(__uint_as_float((127 + by0) << 23), __uint_as_float((127 + by1) << 23));
+  *reinterpret_cast<float2*>(ctl->ungain + 2 * lane) = make_float2(__uint_as_float((127 - by0) << 23), __uint_as_float((127 - by1) << 23));
+  __syncwarp();
+  return true;
 }
 // Two elements' bf16 pieces, packed.
 __device__ __forceinline__ void CutPieces(float lo, float hi, uint32_t (&p)[3]) {
@@ -370,11 +427,15 @@ struct Place {
     return none;
   }
 };
-// Behind the tile: rows that are made again.
+// Behind the tile: the first scores, and rows that are made again.
 template <Form kForm>
 __device__ __forceinline__ void Finish(const SliceArgs& a, AgainSmem* sm, SliceCtl* ctl) {
   const Place at(a, ctl);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (kForm == Form::kScores && at.i0 == 0 && !at.Without(ctl) && threadIdx.x < kFirst * kFirst) {
+    const uint32_t i = threadIdx.x / kFirst, j = threadIdx.x % kFirst;
+    if (i < a.S && j <= i) a.probs[(static_cast<size_t>(at.bh) * a.S + i) * a.S + j] = static_cast<float>(ctl->first[i][j]);
+  }
   if (ctl->some == 0) return;
   uint32_t words[kRows / 32], count = 0;
 #pragma unroll
@@ -383,7 +444,7 @@ __device__ __forceinline__ void Finish(const SliceArgs& a, AgainSmem* sm, SliceC
       const uint32_t r0 = at.i0 + 32 * w;
       return key <= r0 ? 0xFFFFFFFFu : key - r0 >= 32 ? 0u : 0xFFFFFFFFu << (key - r0);
     };
-    words[w] = (ctl->odd_rows[w] | see(ctl->odd_key) | (see(ctl->odd_value) & ~ctl->nan_rows[w])) & at.RowsOf(w);
+    words[w] = (ctl->odd_rows[w] | ctl->again[w] | see(ctl->odd_key) | (see(ctl->odd_value) & ~ctl->nan_rows[w])) & at.RowsOf(w);
     count += __popc(words[w]);
   }
   if (count == 0) return;
@@ -414,8 +475,8 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
     MbarInit(&ctl->sum_full, 1);
     ctl->failed = 0;
     ctl->odd_key = ctl->odd_value = 0xFFFFFFFFu;
-    ctl->some = 0;
-    for (uint32_t w = 0; w < kRows / 32; ++w) ctl->odd_rows[w] = ctl->nan_rows[w] = 0;
+    ctl->k_top = ctl->some = 0;
+    for (uint32_t w = 0; w < kRows / 32; ++w) ctl->odd_rows[w] = ctl->again[w] = ctl->nan_rows[w] = 0;
     MbarInitFence();
     // Longest tiles first over the whole grid, so that the last wave is short ones.
     ctl->i0 = ((a.S + kRows - 1) / kRows - 1 - blockIdx.x / a.BH) * kRows;
@@ -445,18 +506,41 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
     }
   };
   float k_next[kEach][16];   // a step's keys, on their way since the step before
+  bool balanced;
   {   // the queries' digits, by whole warps; all that the first step needs of memory is asked for at once
     constexpr uint32_t kLoaders = kWorkWarps + kCutWarps, kTwice = kRows / 8 - kLoaders;   // warps that have rows twice
     static_assert(kTwice <= kWorkWarps, "not those that have keys");
     float x[16], second[16];
     auto fetch = [&](float (&f)[16], uint32_t r) { FetchSixteen(f, a.q + base + static_cast<size_t>(i0 + r) * D, i0 + r < a.S, c0, a.d); };
+    const bool samples = warp >= kTwice && warp < kTwice + kGroups;   // a group of the sample, two features to a lane
+    static_assert(kTwice + kGroups <= kWorkWarps, "warps that have no second rows");
+    float2 f[kGroupRows];
+    if (samples && 2 * lane < a.d) {   // (first of all: everything waits for it)
+      const bool many = at.live >= kGroups * kGroupRows;   // (of few, every group has the first)
+      uint32_t row = many ? (warp - kTwice) * at.live / kGroups : 0;
+      const uint32_t step = many ? at.live / (kGroups * kGroupRows) : 1;
+#pragma unroll
+      for (uint32_t r = 0; r < kGroupRows; ++r) {
+        f[r] = __ldg(reinterpret_cast<const float2*>(a.q + base + static_cast<size_t>(i0 + row) * D + 2 * lane));
+        row = row + step < at.live ? row + step : 0;
+      }
+    }
     if (warp < kLoaders) fetch(x, threadIdx.x >> 2);
     if (warp < kTwice) fetch(second, 8 * kLoaders + (threadIdx.x >> 2));
     if (warp >= kWorkWarps && warp < kLoaders) fetch_keys(k_next, a.k, 0);
+    if (samples) {
+      uint2 v = make_uint2(0, 0);
+#pragma unroll
+      for (uint32_t r = 0; r < kGroupRows; ++r) v = make_uint2(v.x + CountExponent(f[r].x), v.y + CountExponent(f[r].y));
+      ctl->sample[warp - kTwice][lane] = 2 * lane < a.d ? v : make_uint2(0, 0);
+    }
+    __syncthreads();
+    balanced = BalanceFeatures(ctl);
     if (warp < kLoaders) {
 #pragma unroll 1
       for (uint32_t r = threadIdx.x >> 2;;) {
         bool odd;
+        if (balanced) ScaleSixteen(x, ctl->ungain, c0);
         const float back = CutDigits(x, q_s, kQSlice, r, c0, &odd);
         if (c0 == 0) {
           ctl->q_scale[r] = back * (kForm == Form::kScores ? 1.0f : a.inv_sqrt_d);
@@ -536,6 +620,7 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
     float y[kEach][16];
     auto row_of = [&](uint32_t h) { return r0 + h * 8 * kCutWarps; };
     auto sums_at = [&](uint32_t u) { return kForm == Form::kTiled || (kForm == Form::kCached && u >= ahead && u < total); };
+    float top = 0.0f;   // the largest scale of this thread's keys
     if (sums_at(0)) fetch_keys(y, a.v, 0);
     for (uint32_t u = 0; u < total && ok; ++u) {
       const uint32_t s = u & 1;
@@ -543,12 +628,18 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
       if (u >= 2) ok = SliceWait(ctl, &ctl->stage_empty[s], ((u >> 1) - 1) & 1);
       if (!ok) break;
       const uint32_t key0 = (u < n ? u : u - n) * kKeys;
+      if (balanced) {
+#pragma unroll
+        for (uint32_t h = 0; h < kEach; ++h) ScaleSixteen(k_next[h], ctl->gain, c0);
+      }
       bool odd[kEach];   // (looked at behind the loop: the rows' cutting is one stream of instructions)
 #pragma unroll
       for (uint32_t h = 0; h < kEach; ++h) {
         const float back = CutDigits(k_next[h], stage, kKSlice, row_of(h), c0, &odd[h]);
         if (c0 == 0) ctl->k_scale[u & 3][row_of(h)] = back;
+        top = fmaxf(top, back);
       }
+      if (u + 1 == n) atomicMax(&ctl->k_top, __float_as_uint(top));   // (all keys': the workers read it behind this step's scores)
       auto least = [&] {
         uint32_t at = 0xFFFFFFFFu;
 #pragma unroll
@@ -601,6 +692,19 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
       }
       if (lane == 0) MbarArrive(&ctl->v_full[s]);   // (every step: its phases are the stage's)
       if (sums_at(u + 1)) fetch_keys(y, a.v, u + 1);
+    }
+    if (kForm == Form::kScores && i0 == 0) {   // two threads to a pair of the first rows
+      const uint32_t i = t >> 4, j = t >> 1 & 7, half = t & 1;
+      static_assert(kForm != Form::kScores || kFirst * kFirst * 2 == 32 * kCutWarps, "all of them");
+      double sum = 0.0;
+      if (j <= i && i < a.S)
+        for (uint32_t c = 4 * half; c < a.d; c += 8) {
+          const float4 f = __ldg(reinterpret_cast<const float4*>(a.q + base + static_cast<size_t>(i) * D + c));
+          const float4 g = __ldg(reinterpret_cast<const float4*>(a.k + base + static_cast<size_t>(j) * D + c));
+          sum += static_cast<double>(f.x) * static_cast<double>(g.x) + static_cast<double>(f.y) * static_cast<double>(g.y) +
+                 static_cast<double>(f.z) * static_cast<double>(g.z) + static_cast<double>(f.w) * static_cast<double>(g.w);
+        }
+      ctl->first[i][j] = sum + __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
     }
   } else {
     // ---- scores, probabilities, sums: thread (row, part of the keys) ----
@@ -747,22 +851,38 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
       for (uint32_t p = 0; p < kParts; ++p) whole += ctl->denom[p][r];
       return whole;
     };
-    auto mark = [&](bool nan) {   // rows that nothing need be made again of
+    // What the digits leave out, 2^-17 of both scales, against 2^-29 of the size that matters: beyond it the row is made again,
+    // unless it is NaN.
+    auto check = [&](float size, bool nan, bool exact = false) {
+      const float k_top = __uint_as_float(ctl->k_top);
       const uint32_t none = __ballot_sync(0xFFFFFFFFu, nan);
-      if (part == 0 && lane == 0) ctl->nan_rows[quarter] = none;
+      const uint32_t rows = __ballot_sync(0xFFFFFFFFu, !(q_scale * k_top <= 0x1p-12f * size && size < INFINITY) && i < a.S && !exact);
+      if (part == 0 && lane == 0) {
+        ctl->nan_rows[quarter] = none;
+        ctl->again[quarter] = rows & ~none;
+        if ((rows & ~none) != 0) ctl->some = 1;
+      }
     };
     auto put_stats = [&](double whole) {   // relative to the maximum: the rows' statistics, and their factor
       inv = 1.0f / static_cast<float>(whole * exp(static_cast<double>(ref) - static_cast<double>(top)));
-      mark(isnan(inv));
+      check(fmaxf(1.0f, fabsf(top)), isnan(inv));
       if (a.stats && part == 0 && i < a.S && ok)
         *reinterpret_cast<float4*>(a.stats + (static_cast<size_t>(ctl->bh) * a.S + i) * kAttnStatsWidth) = make_float4(top, inv, 0.0f, 0.0f);
     };
 
     if constexpr (kForm == Form::kScores) {
+      float size = 0.0f;
       for (uint32_t u = 0; u < n; ++u) {
         const uint32_t key0 = take_scores(u);
+#pragma unroll
+        for (int e = 0; e < kOwn; ++e) size = fmaxf(size, fabsf(s[e]));
         if (ok) store_scores(u, key0);
       }
+      ctl->row_max[0][part][r] = size;
+      row_sync();
+#pragma unroll
+      for (uint32_t p = 0; p < kParts; ++p) size = fmaxf(size, ctl->row_max[0][p][r]);
+      check(size, isnan(q_scale), i < kFirst);
     } else {
       if constexpr (kForm == Form::kCached) {
         for (uint32_t u = 0; u < n; ++u) {
@@ -830,7 +950,7 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
       const uint32_t chunk = threadIdx.x & 15;
       if (ok && 4 * chunk < a.d)
         for (uint32_t row = threadIdx.x >> 4; row < kRows && i0 + row < a.S; row += 2 * kWorkWarps)
-          if ((ctl->odd_rows[row / 32] >> (row & 31) & 1) == 0 && i0 + row < ctl->odd_key &&
+          if (((ctl->odd_rows[row / 32] | ctl->again[row / 32]) >> (row & 31) & 1) == 0 && i0 + row < ctl->odd_key &&
               (i0 + row < ctl->odd_value || (ctl->nan_rows[row / 32] >> (row & 31) & 1) != 0)) *reinterpret_cast<float4*>(a.o + ctl->base + static_cast<size_t>(i0 + row) * a.H * a.d + 4 * chunk) =
               *reinterpret_cast<const float4*>(tile_o + row * kWidth + ((chunk ^ (row & 15)) * 4));
     }

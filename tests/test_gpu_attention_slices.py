@@ -1,7 +1,7 @@
 """The exact attention family on the tensor cores (lazy coherence): scores from fixed-point digits, output sums from bf16
 pieces.  Edges of 128 queries and 64 keys, heads of 4 to 64 features, one walk over the keys (statistics) and two
-(probabilities), raw scores; against float64, and no further from it than the f32 sums of the strict seam; and rows that have no
-digits, against the strict seam."""
+(probabilities), raw scores; against float64, and no further from it than the f32 sums of the strict seam, also where features
+and elements differ widely in size; and rows that have no digits, against the strict seam."""
 
 import numpy as np
 import pytest
@@ -82,9 +82,13 @@ def _check(got, strict, want, S, same=1.03, most=np.inf):
         err = np.linalg.norm(got[name] - w) / np.linalg.norm(w)
         before = np.linalg.norm(strict[name] - w) / np.linalg.norm(w)
         # A rounding to f32 is 2.5e-8 rms of the value; scores and probabilities carry one or two, sums of up to 321 f32
-        # products more.  The kernel adds 5e-10 to the scores (digits left out), i.e. nothing that 3 % would not hold.
+        # products more.  What the digits leave out is at most 2^-29 of a row's largest score, i.e. nothing that 3 % would not hold.
         # (1e-12: geometries of a few elements that the strict seam has exactly.)
         assert err <= same * before + 1e-12 and before < most, (name, err, before)
+    # Score by score: a rounding (2^-24 of it), and 128 products of a residue, uniform within 2^-33 of its row's 2^e, with an element: six
+    # standard deviations of their sum are 39 x 2^-33 of 2^(eq + ek), which is at most 2^4 of the row's largest score: 2^-23.7 of that.
+    w, g = want["dP"].reshape(-1, S), got["dP"].reshape(-1, S)
+    assert (np.abs(g - w) <= 2.0 ** -24 * np.abs(w) + 2.0 ** -23.7 * np.abs(w).max(-1, keepdims=True)).all()
     upper = ~np.tril(np.ones((S, S), dtype=bool))
     for name in ("P", "dP"):
         assert not got[name].reshape(-1, S, S)[:, upper].any(), name
@@ -104,6 +108,57 @@ def test_what_takes_the_kernel_unasked(shape):
     prog = [i for i in prog if i.opcode in OPS]
     assert _run(prog, arena, True)[1] == shape[4]
     assert _run(prog, arena, True, use=0)[1] == 0
+
+
+def _spread(x, what, rng):
+    """Features and elements of different sizes, in Q against K and in dO against V."""
+    d = x["q"].shape[-1]
+    if what.startswith("gains"):
+        gain = np.exp2(rng.uniform(-1, 1, size=(x["q"].shape[2], d)) * float(what[5:])).astype(np.float32)
+    for a, b in (("q", "k"), ("do", "v")):
+        if what.startswith("gains"):             # an ordinary reparametrisation
+            x[a] *= gain
+            x[b] /= gain
+        elif what.startswith("feature"):         # one outlier
+            x[a][..., 3] *= np.float32(what[7:])
+            x[b][..., 3] /= np.float32(what[7:])
+        elif what == "unmet":                    # a large element that meets none, in every row
+            x[a][..., 0], x[b][..., 0] = 2.0 ** 34, 0.0
+            x[a][..., 1:], x[b][..., 1:] = 1.0, 1.0
+        elif what == "unmet_rows":               # ... in some rows
+            x[a][:, ::7, :, 0] = 2.0 ** 34
+            x[b][..., 0] = 0.0
+        elif what == "within_rows":
+            x[a] *= np.exp2(rng.uniform(-12, 12, size=x[a].shape)).astype(np.float32)
+            x[b] *= np.exp2(rng.uniform(-12, 12, size=x[b].shape)).astype(np.float32)
+        elif what == "orthogonal":               # to a mean of the keys a hundred times as large as what they differ by
+            m = 100.0 * rng.standard_normal(d)
+            x[b] += m.astype(np.float32)
+            x[a] -= np.outer(x[a].reshape(-1, d).astype(np.float64) @ m, m / (m @ m)).reshape(x[a].shape).astype(np.float32)
+        elif what == "small":                    # gradients, some rows far smaller than others
+            x[a] *= np.exp2(rng.uniform(-85, -20, size=x[a].shape[:3]))[..., None].astype(np.float32)
+
+
+@pytest.mark.parametrize("what", ["gains2", "gains4", "gains8", "gains12", "gains20", "feature1e3", "feature1e4", "feature1e5",
+                                  "feature1e6", "unmet", "unmet_rows", "within_rows", "orthogonal", "small"])
+@pytest.mark.parametrize("shape", [(24, 128, 4, 64), (3, 321, 2, 36)], ids=["24x128x4x64", "3x321x2x36"])
+def test_sizes_that_differ_within_a_row(shape, what):
+    Bq, S, H, d = shape
+    prog, arena, run = _three(shape)
+    fwd, dp, _ = prog
+    x = {n: arena[off:off + 4 * Bq * S * H * d].view(np.float32).reshape(Bq, S, H, d)
+         for n, off in zip(("q", "k", "v", "do"), (*fwd.ins[:3], dp.ins[0]))}
+    v = x["v"].copy()
+    _spread(x, what, np.random.default_rng(7))
+    want, strict, got = _float64(prog, arena, *shape), run(False), run(True)
+    if what == "small":   # (scores near 0: a probability is their exponential all the same)
+        want.pop("stats")
+    if np.abs(x["v"]).max() > 1e3 * np.abs(v).max():   # one feature of O is nearly all of its norm
+        scale = np.abs(want["o"].reshape(-1, d)).max(0, keepdims=True)
+        for r in (want, strict, got):
+            for name in ("o", "o2"):
+                r[name] = (r[name].reshape(-1, d) / scale).reshape(-1)
+    _check(got, strict, want, S)
 
 
 @pytest.mark.parametrize("shape", [(24, 128, 4, 64), (2, 200, 3, 20)], ids=["24x128x4x64", "2x200x3x20"])
