@@ -29,8 +29,8 @@
 // before.  The exponents follow a row's maximum lazily (they are relative to an earlier maximum until that is exceeded by 8), so
 // one walk over the keys does; with probabilities to be stored (the cached form) a first walk takes the statistics.
 //
-// A row whose elements are not finite, or beyond 2^90 or all below 2^-90, has no such digits, and V that is not has
-// no pieces: the rows concerned (of an odd key, those that see it) are made again likewise, after the
+// A row whose elements are not finite, or beyond 2^90 or all below 2^-90, has no such digits, and V beyond 1e28 might overflow
+// in sums that are not normalised yet: the rows concerned (of an odd key, those that see it) are made again likewise, after the
 // rest, up to 65 at a time by all warps of the CTA (Again); a tile of nothing but such rows is not walked at all.  NaN needs no such
 // thing: it goes through a row's scale into its scores.  Measured on a B200, us, 8 x 512 positions of 12 heads of 64, statistics /
 // probabilities / raw scores: 72.5 / 116 / 58.4; gains of 2^+-10 a feature 74.2 / 117 / 60.7; all NaN 73.2 / 116 / 57.3; an infinite element in
@@ -655,12 +655,12 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
       if (lane == 0) MbarArrive(&ctl->k_full[s]);
       fetch_keys(k_next, a.k, u + 1);
       if (sums_at(u)) {   // V's pieces while the scores are formed
-        // (Rows that do not see the key see zeros.)
+        // (Sums of up to 2^23 weights of up to e^kSlack stay finite; rows that do not see the key see zeros.)
 #pragma unroll
         for (uint32_t h = 0; h < kEach; ++h) {
           odd[h] = false;
 #pragma unroll
-          for (int e = 0; e < 16; ++e) odd[h] = odd[h] || !(fabsf(y[h][e]) < 1e36f);
+          for (int e = 0; e < 16; ++e) odd[h] = odd[h] || !(fabsf(y[h][e]) < 1e28f);
         }
         if (least() != 0xFFFFFFFFu) {
           atomicMin(&ctl->odd_value, least());

@@ -163,7 +163,7 @@ def test_sizes_that_differ_within_a_row(shape, what):
 
 @pytest.mark.parametrize("shape", [(24, 128, 4, 64), (2, 200, 3, 20)], ids=["24x128x4x64", "2x200x3x20"])
 @pytest.mark.parametrize("what", ["inf_q", "nan_k", "minus_inf_k", "inf_v", "nan_v", "huge_q", "tiny_k", "zero_rows", "nan_all", "inf_scores",
-                                  "nan_last_tile"])
+                                  "nan_last_tile", "large_v", "large_v_rising"])
 def test_rows_without_digits(what, shape):
     Bq, S, H, d = shape
     prog, arena, run = _three(shape)
@@ -198,6 +198,10 @@ def test_rows_without_digits(what, shape):
     elif what == "nan_last_tile":                # a whole tile of queries without digits, and the one before it with them
         x["q"][:, 128:] = np.nan
         x["do"][:, 128:] = np.nan
+    elif what.startswith("large_v"):             # sums that are not normalised would overflow
+        x["q"][:] = np.float32(1.0) / np.float32(d)
+        x["k"][:] = (np.arange(S, dtype=np.float32) * np.float32(7.5 / S * np.sqrt(d)))[None, :, None, None] if what.endswith("rising") else 1.0
+        x["v"][:] = np.float32(9e35)
     else:
         x["q"][:, 3] = 0.0
         x["k"][:, 0:40] = 0.0
