@@ -1039,6 +1039,10 @@ inline dim3 TileGrid(size_t BH, size_t tiles, size_t d) {
 // exact in double and the order over c is the same), so the tiled backward may
 // take the key rows as the first operand and stream the query rows.
 
+int AttnTileRows(size_t BH, size_t S, size_t d, bool score_rows) {
+  return score_rows ? RowsPerThreadWithScores(BH, S, d, 1) : RowsPerThread(BH, S, 8);
+}
+
 void AttnFwd(const float* q, const float* k, const float* v, float* o, float* probs,
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,
              bool fused, cudaStream_t s) {

@@ -39,6 +39,7 @@
 //
 // Every wait on an mbarrier is bounded; one that runs out raises DeviceStatus::wait_timeout and the CTA stores nothing.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <initializer_list>
 #include <type_traits>
@@ -976,27 +977,54 @@ __global__ void __launch_bounds__(kThreads, 1) AttnSliceKernel(const SliceArgs a
   if (ctl->failed == 0) Finish<kForm>(a, reinterpret_cast<AgainSmem*>(q_s), ctl);
 }
 
-// Whether the kernel is the shorter one, by estimates of both in us: 64 keys a step, the longest tile's steps or an SM's share
-// of them all; and the tile kernels of k_attention.cu by the pairs they take, whatever their rows (of the raw scores, by their
-// features too).  Measured on a B200, tile kernels / this, us: statistics 8 x 512 positions of 12 heads of 64 176 / 69.7, 32 x 128 of 4 30.9 /
-// 15.1, 2 x 1030 of 3 72.9 / 61.6, 8 x 100 of 4 12.4 / 13.3, 64 x 32 of 4 17.5 / 20.2; probabilities 186 / 114, 31.0 / 19.8, 73.9 / 133, 12.5 / 17.6;
-// raw scores 90.3 / 56.0, 18.6 / 11.2, 36.0 / 64.8, 8.4 / 9.3.
+int SmCount() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  return cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0 ? sms : 148;
+}
+
+// Whether the kernel is the shorter one, by estimates of both in us.  This: a CTA takes a + b a step of 64 keys (of rows that are no
+// multiple of 16 bytes, single stores: b + 2), and the grid its longest CTA or the SMs' share of all with most of a shortest one
+// left over, a whole number of rounds where all are equally long.  The tile kernels of k_attention.cu: the pairs of their blocks, 64
+// keys at a time (by features, of which statistics and sums are half), the blocks past one to two SMs, and no less than the
+// longest block's walk.  Measured on a B200, tile kernels / this, us: statistics 8 x 512 positions of 12 heads of 64 174 /
+// 72.7, 32 x 128 of 4 29.0 / 15.4, 2 x 1030 of 3 71.6 / 63.3, 8 x 100 of 4 10.9 / 14.1, 64 x 32 of 4 15.7 / 19.6, 12 x 129 of 8 28.8 / 29.4;
+// probabilities 184 / 117, 29.9 / 21.8, 72.3 / 126, 11.1 / 19.0, 16.0 / 24.7, 29.6 / 47.5; raw scores 87.7 / 59.0, 16.2 / 12.2, 34.5 / 63.9, 5.9 /
+// 10.2, 10.7 / 15.8, 18.4 / 26.9.  Of 84 launches measured (1 x 300 to 128 x 64 positions, heads of 4 to 64) the rule takes the longer way in
+// two: probabilities of 24 x 127 of 4 heads 26.3 / 25.0, raw scores of 10 x 321 of 10 heads of 60 55.0 / 53.0.
 bool Shorter(Form form, size_t B, size_t S, size_t H, size_t d) {
-  const double tiles = static_cast<double>((S + kRows - 1) / kRows), units = static_cast<double>(B * H);
-  const double longest = static_cast<double>((S + kKeys - 1) / kKeys), steps = units * (tiles * (tiles + 1) - (2 * tiles - longest));
-  const double rounds = std::max(1.0, units * tiles / 148.0);
-  const double step = form == Form::kCached ? 7.0 : 3.3, mine = 6.0 + step * std::max(longest, steps / 148.0) + 5.0 * (rounds - 1.0);
-  double pairs = units * static_cast<double>(S) * static_cast<double>(S + 1) * 0.5e-6;
-  if (form == Form::kScores) pairs *= static_cast<double>(d) / 64.0;
-  const double first = std::min(pairs, 1.0), more = pairs - first;
-  const double theirs = form == Form::kScores ? 6.0 + 11.0 * first + 6.0 * more : 7.0 + 21.0 * first + 13.5 * more;
-  return mine < theirs;
+  const int rows = 8 * AttnTileRows(B * H, S, d, form != Form::kScores);
+  if (rows == 0) return true;   // (not even that: a warp a row)
+  const double sms = SmCount(), units = static_cast<double>(B * H);
+  const double tiles = static_cast<double>((S + kRows - 1) / kRows), chunks = static_cast<double>((S + kKeys - 1) / kKeys);
+  const double a = form == Form::kScores ? 6.4 : 7.3;
+  const double b = (form == Form::kTiled ? 3.4 : form == Form::kCached ? 5.9 : 2.2) + (form != Form::kTiled && S % 4 != 0 ? 2.0 : 0.0);
+  double mine = a + b * chunks;
+  if (tiles == 1.0) {
+    mine *= std::ceil(units / sms);
+  } else {
+    const double steps = tiles * (tiles + 1) - (2 * tiles - chunks);   // of a unit
+    mine = std::max(mine, units * (a * tiles + b * steps) / sms + (units * tiles > sms ? 0.6 * (a + 2 * b) : 0.0));
+  }
+  const double theirs_tiles = static_cast<double>((S + rows - 1) / rows), blocks = units * theirs_tiles, per = static_cast<double>(kKeys) / rows;
+  const double keys = kKeys * (per * chunks * (chunks + 1) / 2 - (per * chunks - theirs_tiles) * chunks);   // of a unit's blocks
+  const double wide = static_cast<double>(d) / 64.0, half = 0.5 + 0.5 * wide, few = rows == 8 ? 1.7 : 1.0;
+  const double pairs = units * keys * rows * 1e-6 * 148.0 / sms, more = std::max(0.0, blocks - sms / 2) * 148.0 / sms;
+  const double theirs = form == Form::kScores ? 5.0 + std::max(1.4 * chunks, 4.7 * wide * pairs + 0.011 * more)
+                                              : 4.0 + std::max(4.1 * half * few * chunks, 9.3 * half * few * pairs + 0.022 * more);
+  return mine < 0.96 * theirs;
 }
 
 template <Form kForm>
 bool Launch(const SliceArgs& a, size_t blocks, cudaStream_t s) {
-  if (cudaFuncSetAttribute(AttnSliceKernel<kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSliceSmem)) != cudaSuccess)
-    return false;
+  static std::atomic<bool> configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(AttnSliceKernel<kForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSliceSmem)) != cudaSuccess)
+      return false;
+    if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+  }
   return Next(AttnSliceKernel<kForm>, static_cast<unsigned>(blocks), kThreads, kSliceSmem, s)(a) == cudaSuccess;
 }
 

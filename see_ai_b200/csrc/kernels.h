@@ -176,6 +176,8 @@ void SetScalars(const AdamScalars& v, AdamScalars* dst, cudaStream_t s);
 void AttnFwd(const float* q, const float* k, const float* v, float* o, float* probs,
              float* stats, size_t B, size_t S, size_t H, size_t d, const int32_t* starts,
              bool fused, cudaStream_t s);  // probs != null: cached family; stats != null: tiled family
+// An eighth of the query rows of a block of AttnFwd's (with score rows in shared memory) or AttnDP's tile kernels; 0: they have none.
+int AttnTileRows(size_t BH, size_t S, size_t d, bool score_rows);
 // The same on the tensor cores (k_attn_slice.cu), where the bits are not observed and no segment starts are given.  False: not
 // a geometry of theirs (or, by default, not the shorter way), and nothing was launched.
 enum class SliceUse { kNever = 0, kShorter = 1, kAlways = 2 };
