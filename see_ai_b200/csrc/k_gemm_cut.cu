@@ -67,23 +67,34 @@ struct __align__(8) CutBarriers {
   volatile uint32_t nonfinite;
 };
 
+// How a block of A comes: loads of 16 bytes alone (src_k % 4 == 0: four elements are all in or all out), the same with a scale
+// along k, loaded likewise, or one element at a time.
+enum class Loads { kPlain, kScaled, kAny };
+
 // A thread's part of the 128 x 64 f32 elements of block kb: some of the warp's rows, four apart, eight columns of each.
-template <uint32_t kWarps>
+template <uint32_t kWarps, Loads kLoads>
 struct CutRegs {
   static constexpr uint32_t kRows = kBlockM / (4 * kWarps);
   float4 v[2 * kRows];
+  float4 scale[kLoads == Loads::kScaled ? 2 : 1];   // (the columns', for when the elements are cut)
   static __device__ __forceinline__ uint32_t Row(uint32_t h) {
     return ((threadIdx.x >> 5) - 2) * (4 * kRows) + h * 4 + ((threadIdx.x & 31) >> 3);
   }
 };
-// kPlain: nothing but loads of 16 bytes (src_k % 4 == 0: four elements are all in or all out), so that the thread goes on while
-// they fly; a choice between two ways of loading would end in moves that wait for them.
-template <bool kPlain, uint32_t kWarps>
-__device__ __forceinline__ void FetchBlock(CutRegs<kWarps>* f, const UmmaEpilogue& ep, uint32_t m0, uint32_t kb) {
+// The loads alone, so that the thread goes on while they fly; a choice between two ways of loading, or a product, would end in
+// moves that wait for them (int8 products in exact arithmetic with a scale along k, us, one element at a time / so: 4096 x 768 x 768
+// 38.8 / 21.7, 2048 x 512 x 2048 43.6 / 23.4, 4096 x 768 x 3072 126 / 62.9; without a scale 20.4, 21.5, 56.7).
+template <Loads kLoads, uint32_t kWarps>
+__device__ __forceinline__ void FetchBlock(CutRegs<kWarps, kLoads>* f, const UmmaEpilogue& ep, uint32_t m0, uint32_t kb) {
   const uint32_t k = kb * kBlockK + (threadIdx.x & 7) * 8;
+  if constexpr (kLoads == Loads::kScaled) {
 #pragma unroll
-  for (uint32_t h = 0; h < CutRegs<kWarps>::kRows; ++h) {
-    const uint32_t row = m0 + CutRegs<kWarps>::Row(h);
+    for (uint32_t q = 0; q < 2; ++q)
+      f->scale[q] = k + 4 * q < ep.src_k ? __ldg(reinterpret_cast<const float4*>(ep.src_a_scale + k + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (uint32_t h = 0; h < f->kRows; ++h) {
+    const uint32_t row = m0 + f->Row(h);
     const float* p = ep.src_a + static_cast<size_t>(row) * ep.src_k + k;
 #pragma unroll
     for (uint32_t q = 0; q < 2; ++q) {
@@ -91,7 +102,7 @@ __device__ __forceinline__ void FetchBlock(CutRegs<kWarps>* f, const UmmaEpilogu
       float4& x = f->v[2 * h + q];
       x = make_float4(0.f, 0.f, 0.f, 0.f);
       if (row >= ep.M || c >= ep.src_k) continue;
-      if constexpr (kPlain) {
+      if constexpr (kLoads != Loads::kAny) {
         x = __ldg(reinterpret_cast<const float4*>(p + 4 * q));
       } else {
         auto at = [&](uint32_t e) {
@@ -112,14 +123,15 @@ __device__ __forceinline__ void CutPair(float lo, float hi, uint32_t (&p)[3]) {
     hi = hi - __uint_as_float(p[i] & 0xFFFF0000u);
   }
 }
-template <uint32_t kWarps>
-__device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs<kWarps>& f) {
+template <uint32_t kWarps, Loads kLoads>
+__device__ __forceinline__ void StoreBlock(uint8_t* pieces, const CutRegs<kWarps, kLoads>& f) {
 #pragma unroll
-  for (uint32_t h = 0; h < CutRegs<kWarps>::kRows; ++h) {
+  for (uint32_t h = 0; h < f.kRows; ++h) {
     uint32_t w[3][4];
 #pragma unroll
     for (uint32_t q = 0; q < 2; ++q) {
-      const float4 x = f.v[2 * h + q];
+      float4 x = f.v[2 * h + q];
+      if constexpr (kLoads == Loads::kScaled) x = make_float4(x.x * f.scale[q].x, x.y * f.scale[q].y, x.z * f.scale[q].z, x.w * f.scale[q].w);
       uint32_t a[3], b[3];
       CutPair(x.x, x.y, a);
       CutPair(x.z, x.w, b);
@@ -289,10 +301,10 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
         return true;
       };
       // Cut block after block; where the same warps add, the one before while the products of this one run.
-      [[maybe_unused]] auto walk = [&](auto plain) {
-        constexpr bool kPlain = decltype(plain)::value;
-        CutRegs<Sh::kCutWarps> f;
-        FetchBlock<kPlain>(&f, ep, m0, g0);
+      [[maybe_unused]] auto walk = [&](auto loads) {
+        constexpr Loads kLoads = decltype(loads)::value;
+        CutRegs<Sh::kCutWarps, kLoads> f;
+        FetchBlock<kLoads>(&f, ep, m0, g0);
         for (uint32_t g = g0, it = 0; g < g1 && ok; ++g, ++it) {
           const uint32_t s = it % Sh::kStages, round = it / Sh::kStages;
           bool free = round == 0 || MbarWait(&bars->empty[s], (round - 1) & 1);
@@ -300,7 +312,7 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
           if (bars->abort) free = false;
           if (!(ok = __all_sync(0xFFFFFFFFu, free))) break;
           StoreBlock(smem + s * Sh::kStageBytes, f);
-          if (g + 1 < g1) FetchBlock<kPlain>(&f, ep, m0, g + 1);
+          if (g + 1 < g1) FetchBlock<kLoads>(&f, ep, m0, g + 1);
           FenceProxyAsync();
           __syncwarp();
           if (lane == 0) MbarArrive(&bars->a_full[s]);
@@ -309,8 +321,11 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
         }
       };
       if constexpr (kCuts) {
-        if ((ep.src_k & 3u) == 0 && (reinterpret_cast<uintptr_t>(ep.src_a) & 15) == 0 && !ep.src_a_scale) walk(std::true_type{});
-        else walk(std::false_type{});
+        const bool aligned = (ep.src_k & 3u) == 0 && ((reinterpret_cast<uintptr_t>(ep.src_a) | reinterpret_cast<uintptr_t>(ep.src_a_scale)) & 15) == 0;
+        constexpr Loads kWithScale = Sh::kApart ? Loads::kScaled : Loads::kAny;   // (an f32 weight has no scales)
+        if (aligned && !ep.src_a_scale) walk(std::integral_constant<Loads, Loads::kPlain>{});
+        else if (aligned && kWithScale == Loads::kScaled) walk(std::integral_constant<Loads, kWithScale>{});
+        else walk(std::integral_constant<Loads, Loads::kAny>{});
         if constexpr (kAdds)
           if (ok && g1 > g0) ok = add(g1 - g0 - 1);
       } else {

@@ -166,3 +166,28 @@ def test_pieces_that_are_there_are_used_on_a_long_walk():
         err = np.abs(got[out:out + 4 * M * N].view(np.float32).reshape(M, N) - ref)
         rms = np.sqrt(np.mean(ref ** 2))
         assert np.sqrt(np.mean(err ** 2)) <= 4e-7 * rms and err.max() <= 8e-6 * rms
+
+
+# Scales along k (they join the activation): each tile width, K that ends inside a block, a CTA's part of K that begins inside
+# the scales.
+SCALED = [(4096, 256, 256), (300, 5000, 256), (4096, 768, 768), (1000, 768, 3072), (640, 514, 328), (129, 1000, 1000), (2000, 385, 96)]
+
+
+@pytest.mark.parametrize("shape", SCALED, ids=["x".join(map(str, s)) for s in SCALED])
+def test_scales_along_k(shape):
+    M, N, K = shape
+    rng = np.random.default_rng(M + N + K)
+    a = Arena(rng)
+    x, out = a.alloc(M * K, "normal"), a.alloc(M * N)
+    q = rng.integers(-127, 128, size=(N, K), dtype=np.int8)
+    scale = np.exp2(rng.uniform(-12, -2, size=K)).astype(np.float32)
+    prog = [P.Instr(Op.GEMM_NT_Q8, P.FLAG_Q8_COL_SCALE, 0, (x, a.ro_alloc(q.reshape(-1)), out, a.ro_alloc(scale)), (M, N, K))]
+    arena, ro = a.build()
+    got, taken = _run(prog, arena, ro, -1)
+    assert taken == 1
+    A = arena[x:x + 4 * M * K].view(np.float32).reshape(M, K)
+    want = (A.astype(np.float64) * scale) @ q.T.astype(np.float64)
+    err = got[out:out + 4 * M * N].view(np.float32).reshape(M, N) - want
+    # (as above, and a rounding of every scaled element)
+    assert np.sqrt(np.mean(err ** 2)) <= 4e-7 * np.sqrt(np.mean(want ** 2))
+    assert np.abs(err).max() <= 8e-6 * np.sqrt(np.mean(want ** 2))
