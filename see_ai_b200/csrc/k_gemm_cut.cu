@@ -453,14 +453,15 @@ cudaError_t Launch(const UmmaCutPlan& plan, const CUtensorMap& map_b, const Umma
 }  // namespace
 
 UmmaCutPlan UmmaPlanCut(uint32_t M, uint32_t N, uint32_t groups, bool exact_b, uint32_t sms) {
-  // One round of CTAs only, and for an f32 weight at most sixteen blocks of 64 k: beyond that the working warps, which
-  // take about 1.2 us to cut a block and add one (1.4 at a tile width of 128 or 192), fall behind the piece form's
-  // tensor time, and every further column tile cuts A again.  Measured on a B200, the piece form's kernel (+ its cut of A) / this,
-  // us, f32 weights: 4096 x 256 x 256 14.0 (+2.8) / 9.7, 1024 x 256 x 256 8.4 (+2.0) / 8.0, 600 x 512 x 512 12.3 (+2.1) / 10.7,
-  // 128 x 1024 x 1024 14.7 (+2.0) / 11.1, 300 x 5000 x 256 15.1 (+1.9) / 11.8, 4096 x 256 x 1024 21.7 (+5.9) / 18.5; past the line
-  // 2048 x 512 x 2048 32.1 (+5.9) / 42.0, 4096 x 1024 x 256 18.8 (+2.7) / 22.4, 4096 x 4096 x 256 57.9 (+4.0) / 77.1; int8 weights:
-  // 4096 x 768 x 768 24.8 (+4.2) / 19.8, 4096 x 768 x 3072 69.0 (+20.9) / 56.0, 2048 x 512 x 2048 22.2 (+6.2) / 21.4; past it 4096 x
-  // 3072 x 768 67.3 (+6.1) / 87.9.
+  // One round of CTAs only, and for an f32 weight at most sixteen blocks of 64 k: every further column tile cuts A again, and
+  // the working warps, which take about 1 us for a block, fall behind the piece form's tensor time.  Measured on a B200, the
+  // piece form's kernel (+ its cut of A) / this, us, f32 weights: 4096 x 256 x 256 13.3 (+2.5) / 8.9, 1024 x 256 x 256 8.0 (+1.6) / 7.8,
+  // 600 x 512 x 512 11.3 (+1.8) / 10.6, 128 x 1024 x 1024 13.5 (+1.4) / 10.5, 300 x 5000 x 256 13.9 (+1.1) / 11.6, 4096 x 256 x 1024 20.3 (+5.8) /
+  // 18.0, 4096 x 512 x 256 14.1 (+2.5) / 11.7; past the line 4096 x 768 x 256 16.1 (+2.8) / 21.9, 4096 x 1024 x 256 17.3 (+2.9) / 22.2, 4096 x 4096 x
+  // 256 52.4 (+4.3) / 75.9; int8 weights: 4096 x 768 x 768 23.8 (+3.7) / 20.4, 4096 x 768 x 3072 64.5 (+20.7) / 56.6, 2048 x 512 x 2048 21.4 (+5.7) /
+  // 21.8; past it 4096 x 3072 x 768 65.6 (+4.2) / 78.4, 2048 x 2304 x 768 24.4 (+3.4) / 31.9, 4096 x 1024 x 256 14.3 (+2.5) / 18.5.  Drawn when a
+  // block took longer, the line is short of where both meet now: f32 2048 x 512 x 2048 28.9 (+6.8) / 27.4, and of exact weights in two
+  // full rounds 4096 x 1536 x 768 44.8 (+4.0) / 39.3, 8192 x 768 x 768 44.7 (+9.2) / 39.3.
   UmmaCutPlan best;
   if (!exact_b && groups > 16) return best;
   double least = 1e30;

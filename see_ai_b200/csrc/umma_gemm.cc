@@ -571,9 +571,9 @@ std::string TrySplitGemm(Context* ctx, const k::GemmArgs& a, bool wide, int a_sp
   // float64 at int8 2048 x 512 x 2048 1.03e-7 in one chain a CTA, 9.3e-8 in parts (piece form 9.4e-8), f32 4096 x 256 x 1024 1.00e-7 and
   // 9.6e-8 (9.7e-8), for 2 to 3 % of the time; up to four blocks the errors are the same.
   cut.parts = Kp / 64 > 4 * cut.splits ? plan.splits : cut.splits;
-  // (Pieces that are there already are worth it where the kernel's working warps would take a long walk alone: int8 2048 x
-  // 512 x 2048 25.0 us, 22.2 from pieces, 4096 x 512 x 2048 41.9 and 33.8; up to 16 blocks of 64 k, and with 192-wide tiles,
-  // cutting is the shorter all the same, 4096 x 768 x 3072 67.9 and 69.0.)
+  // (Pieces that are there already are worth it where the kernel's working warps would take a long walk alone: int8 4096 x
+  // 512 x 2048 34.4 us, 31.3 from pieces, 2048 x 512 x 2048 22.0 and 21.4; up to 16 blocks of 64 k, and with 192-wide tiles,
+  // cutting is the shorter all the same, 4096 x 768 x 3072 57.5 and 64.7.)
   const bool long_walk = exact_b && cut.tn <= 128 && Kp / 64 > 16 * cut.splits;
   const bool cuts = !a.a_transposed && cut.grid != 0 && !(have_pieces && long_walk);
   // No memory for a copy or for pieces: the product stays on the CUDA cores, which need neither.
