@@ -74,7 +74,7 @@ struct Impl {
   // ended by any write into that range.
   struct SplitTag { bool valid = false, transposed = false; uint64_t off = 0, M = 0, K = 0; const float* k_scale = nullptr; } split_tag;
   uint32_t sms = 148;
-  uint64_t device_bytes = 0;   // the device's memory, asked for once: the question takes the driver about 100 us
+  uint64_t device_bytes = 0;   // the device's memory, asked for by the first range that needs it: the question takes the driver about 100 us
   uint64_t moves = 0;   // device buffers of this context freed since it was made (BufferMoves)
   std::map<WeightKey, uint16_t*> split_weights;          // frozen B operands, once per binding
   std::set<WeightKey> split_refused;                     // those there was no memory for
@@ -94,8 +94,6 @@ std::string Init(Context* ctx, int device, k::DeviceStatus* status) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0)
     impl->sms = static_cast<uint32_t>(sms);
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) impl->device_bytes = total_b;
   impl->status = status;
   ctx->impl = impl;
   return {};
@@ -176,6 +174,8 @@ void PlanRange(Context* ctx, const Instruction* program, size_t begin, size_t en
     }
   }
   if (attn > 0) {
+    size_t free_b = 0, total_b = 0;
+    if (impl->device_bytes == 0 && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) impl->device_bytes = total_b;
     const uint64_t per_entry = attn * 2;   // bf16
     const uint64_t by_budget = std::max<uint64_t>(4, (impl->device_bytes / 8) / per_entry);
     const size_t want = static_cast<size_t>(
