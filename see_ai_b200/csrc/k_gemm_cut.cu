@@ -409,17 +409,14 @@ UmmaGemmCutKernel(const __grid_constant__ CUtensorMap map_b, const __grid_consta
           uint32_t lr, chunk;
           if (!there(u, &lr, &chunk)) continue;
           const uint32_t n = n0 + chunk * 4;
-          const float4 acc = element(lr, chunk), d = side[u];
-          float4 v = make_float4(acc.x * scale[u].x, acc.y * scale[u].y, acc.z * scale[u].z, acc.w * scale[u].w);
-          if (!plain) {
-            if (!ep.addend_last) v = make_float4(d.x + v.x, d.y + v.y, d.z + v.z, d.w + v.w);
-            if (ep.bias) {
-              const float4 b = __ldg(reinterpret_cast<const float4*>(ep.bias + n));
-              v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
-            }
-            if (ep.addend_last) v = make_float4(d.x + v.x, d.y + v.y, d.z + v.z, d.w + v.w);
+          const float4 acc = element(lr, chunk);
+          const size_t at = static_cast<size_t>(m0 + lr) * ep.N + n;
+          if (plain) {
+            EpilogueStorePlain(ep, at, acc, scale[u]);
+          } else {
+            const float4 bias = ep.bias ? __ldg(reinterpret_cast<const float4*>(ep.bias + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            EpilogueStoreSum(ep, at, acc, scale[u], bias, side[u]);
           }
-          *reinterpret_cast<float4*>(ep.C + static_cast<size_t>(m0 + lr) * ep.N + n) = v;
         }
       }
     }
