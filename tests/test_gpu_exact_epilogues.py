@@ -63,16 +63,18 @@ def _case(shape, kind, tail, in_place=False, read_between=False, over_operand=Fa
         prog.append(P.Instr(Op.GELU_FWD, 0, 0, (last, out), (M * N,)))
     if "r" in tail:
         prog.append(P.Instr(Op.RELU_FWD, 0, 0, (last, out), (M * N,)))
+    if "s" in tail:
+        prog.append(P.Instr(Op.SILU_FWD, 0, 0, (last, out), (M * N,)))
     if "+" in tail:
         prog.append(P.Instr(Op.ADD_EW, 0, 0, (y, last, out), (M * N,)))
     # The values in between are overwritten, as a plan's next layer overwrites them.
-    final = prog[-1].ins[1 if prog[-1].opcode in (Op.GELU_FWD, Op.RELU_FWD) else 2]
+    final = prog[-1].ins[1 if prog[-1].opcode in (Op.GELU_FWD, Op.RELU_FWD, Op.SILU_FWD) else 2]
     for r in {z, zb} - {final}:
         prog.append(P.Instr(Op.FILL, 0, 0, (r, 0), (M * N, 0, 0)))
     return prog, a.build(), final
 
 
-@pytest.mark.parametrize("tail", ["bg", "b+", "br"])
+@pytest.mark.parametrize("tail", ["bg", "b+", "br", "bs"])
 @pytest.mark.parametrize("kind", ["f32", "nt", "q8", "addend"])
 @pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
 def test_the_separate_instructions_bits(shape, kind, tail):
@@ -100,3 +102,27 @@ def test_values_that_others_read(shape, how, tail):
     both = {"in_place": 2, "read_between": 1, "over_operand": 1}[how]
     # (a GELU in place of its input, which only the piece kernels take with them, leaves the bias to the others)
     assert fused.fused_dispatches == (min(both, 1) if tail == "bg" and K == 1024 else both)
+
+
+def sums_that_are_not_finite(shape, kind, tail):
+    """An infinity, a NaN, and an overflow of finite operands in the activation: what is remade carries the absorbed bias,
+    activation and add.  Returns the counters, absorbed and separate."""
+    M, N, K = shape
+    prog, (arena, ro), final = _case(shape, kind, tail)
+    x = prog[0].ins[0]
+    A = arena[x:x + 4 * M * K].view(np.float32).reshape(M, K)
+    A[M // 2, K // 3], A[M // 3, K - 1], A[M - 1] = np.inf, np.nan, 3e38
+    got, fused = _run(prog, arena, ro, True)
+    want, single = _run(prog, arena, ro, False)
+    g, w = (a[final:final + 4 * M * N].view(np.float32) for a in (got, want))
+    assert not np.isfinite(w).all()
+    np.testing.assert_array_equal(g, w)   # (any NaN is as good as another)
+    return fused, single
+
+
+@pytest.mark.parametrize("tail", ["bs", "bg", "b+"])
+@pytest.mark.parametrize("kind", ["f32", "q8"])
+@pytest.mark.parametrize("shape", [(600, 512, 512), (1023, 768, 768), (200, 514, 304)], ids=["cut", "cut192", "ragged"])
+def test_sums_that_are_not_finite(shape, kind, tail):
+    fused, single = sums_that_are_not_finite(shape, kind, tail)
+    assert fused.fused_dispatches == len(tail) == single.kernel_launches - fused.kernel_launches
